@@ -883,3 +883,14 @@ def test_product_kernels_on_random_shapes():
         assert int(err) == 0, what
         ran[kind] = ran.get(kind, 0) + 1
     assert len(ran) == 9 and min(ran.values()) >= 5, ran
+
+
+@pytest.mark.parametrize("m, n, k", [(1, 33, 4), (16, 48, 20), (40, 130, 64), (200, 1000, 100), (700, 2100, 36), (130, 4100, 2052)])
+def test_aligned_fp32_product_has_the_plain_kernels_bits(m, n, k):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    x, w = dev(rnd(m, k, scale=2)), dev(rnd(n, k, seed=3))
+    wide = torch.empty(m, k + 1, device="cuda")[:, :k]      # (rows off their 16-byte boundaries: the plain kernel)
+    wide.copy_(x)
+    plain = ops.gemm_f32(wide, w, torch.empty(m, n, device="cuda"))
+    assert torch.equal(ops.gemm_f32(x, w, torch.empty(m, n, device="cuda")), plain)
