@@ -894,3 +894,46 @@ def test_aligned_fp32_product_has_the_plain_kernels_bits(m, n, k):
     wide.copy_(x)
     plain = ops.gemm_f32(wide, w, torch.empty(m, n, device="cuda"))
     assert torch.equal(ops.gemm_f32(x, w, torch.empty(m, n, device="cuda")), plain)
+
+
+# ------------------------------------------------- linear attention in runs and token by token
+@pytest.mark.parametrize("lens, heads, key_dim, value_dim", [
+    ([1, 1, 1], 3, 128, 128), ([32, 5, 9], 2, 64, 96),                        # token by token, to its longest portion
+    ([33, 1, 64], 2, 128, 64), ([65, 128, 127, 2], 2, 64, 128), ([200, 63], 3, 128, 128)])      # runs and their edges
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_linear_attention_forms_agree_with_the_recurrence(lens, heads, key_dim, value_dim, dtype):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    n, entries = sum(lens), len(lens)
+    rows = rnd(n, heads * (2 * key_dim + value_dim) + 8, dtype=dtype)
+    decay = torch.tensor([1 - 2.0 ** -(3 + i) for i in range(heads)], dtype=torch.float64)
+    state = rnd(entries + 1, heads, key_dim, value_dim, seed=5)
+    slots = [entries - i for i in range(entries)]
+
+    def powers(most):
+        return dev((decay[:, None] ** torch.arange(most + 1, dtype=torch.float64)).float().contiguous())
+
+    starts = torch.tensor([sum(lens[:i]) for i in range(entries + 1)], dtype=torch.int32)
+    proj, got_state = dev(rows), dev(state.clone())
+    qk = heads * key_dim
+    out = ops.linear_attention(proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + heads * value_dim],
+                               torch.empty(n, heads * value_dim, device="cuda"), got_state,
+                               powers(ops.linear_attention_chunk(key_dim, value_dim)), dev(starts),
+                               dev(torch.tensor(slots, dtype=torch.int32)), entries, heads, key_dim, value_dim, silu=True,
+                               max_q_len=max(lens), run_powers=powers(ops.linear_attention_run()))
+    x = rows.double()
+    act = x * torch.sigmoid(x)
+    q, k = act[:, :qk].view(n, heads, key_dim), act[:, qk:2 * qk].view(n, heads, key_dim)
+    v = act[:, 2 * qk:2 * qk + heads * value_dim].view(n, heads, value_dim)
+    want, want_state = torch.empty(n, heads, value_dim, dtype=torch.float64), state.double().clone()
+    for e, length in enumerate(lens):
+        s = want_state[slots[e]].clone()
+        for t in range(int(starts[e]), int(starts[e]) + length):
+            s = decay[:, None, None] * s + k[t][:, :, None] * v[t][:, None, :]
+            want[t] = torch.einsum("hkv,hk->hv", s, q[t])
+        want_state[slots[e]] = s
+    # fp32 throughout: every output is a sum of at most key_dim + 64 products a run, each rounded once (2^-24), and the
+    # sums' magnitude is at most about sqrt(terms) times the outputs'; 2e-6 is 32 roundings of the largest value
+    assert (as_ref(out) - want.reshape(n, -1)).abs().max() <= 2e-6 * want.abs().max()
+    assert (as_ref(got_state) - want_state).abs().max() <= 2e-6 * want_state.abs().max()
+

@@ -14,6 +14,13 @@
 // which is the recurrence written out.  Scores, decay powers, state and sums are fp32; the powers
 // lambda^0 .. lambda^C come from the host as a table (made in double precision).  A single token is a chunk
 // of one.  State is read from and written back to the request's slot; a new request's slot is zero.
+//
+// Three ways to run that, chosen by sizes alone (tib_linear_attention):
+//   runs   (portions above 32 tokens, head sizes of 64 or 128) every run of 64 tokens makes its own sum L of decayed k v^T
+//          side by side, one thread per state element then folds S <- lambda^n S + L over a request's runs, and every run
+//          makes its outputs from its starting state: the serial chain is one fused multiply-add a run
+//   walk   (steps whose portions have at most 32 tokens) S in registers, token by token
+//   chunks (everything else) the block walk described above
 #include "common.cuh"
 
 namespace tib {
@@ -206,6 +213,396 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   for (int e = threadIdx.x; e < D * V; e += blockDim.x) state[(size_t)(e / V) * a.value_dim + e % V] = S[e];
 }
 
+// ---------------------------------------------------------------------------------------------------------- runs
+// The walk above is one serial chain of 64 chunks for 2,048 tokens, each with four barriers, on 512 blocks that each see 32 of a
+// run's 128 columns: 980 us for two portions of 1,366 and 682 tokens, 16 heads of 128 x 128, of which the fp32 arithmetic
+// (3.3 GFLOP here) is some 50 us.  In runs the three launches below take 144 us.  What bounds them is the fp32 pipe: register
+// tiles of 8 x 8 (sums) and 4 x 8 (outputs) per thread, products in pairs of neighbouring columns (fma.rn.f32x2, each
+// half rounded as the scalar instruction rounds it), operands from shared memory in 16-byte loads without bank conflicts.
+// Everything stays fp32: activations, decay powers, scores, states and sums.
+constexpr int kLinRun = 64;
+constexpr int kLinPad = kLinRun + 4;       // row stride of the transposed q, k and scores
+
+struct LinRunArgs {
+  const int* q_start;
+  const int* slots;
+  const float* powers;    // [heads, kLinRun + 1]
+  float* state;           // [slots, heads, D, value_dim]
+  float* run_state;       // [runs, heads, D, value_dim]: L of a run, then the state at its start
+  float* out;
+  int64_t ldq, ldk, ldv;
+  int heads, value_dim, activation;
+};
+
+// An entry's first run: entries' runs never overlap, since an entry of len tokens has at most len / kLinRun + 1 runs and the
+// next entry starts len rows and one entry later.
+__device__ __forceinline__ size_t lin_first_run(int row0, int entry) { return (size_t)(row0 / kLinRun) + entry; }
+
+// eight elements of a row, activated, in fp32
+__device__ __forceinline__ void lin_load8(const __nv_bfloat16* p, int activation, float (&v)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+    v[2 * i] = lin_act(f.x, activation);
+    v[2 * i + 1] = lin_act(f.y, activation);
+  }
+}
+__device__ __forceinline__ void lin_load8(const float* p, int activation, float (&v)[8]) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = lin_act(v[i], activation);
+}
+
+// grid (heads * column tiles, runs, entries): L[d][c] = sum_j lambda^(n-1-j) k_j[d] v_j[c] of the run's n tokens
+template <typename T, int D, int TV>
+__global__ void __launch_bounds__(256, 2) lin_run_sums_kernel(const T* __restrict__ k, const T* __restrict__ v, LinRunArgs a) {
+  extern __shared__ __align__(16) float lin_smem[];
+  float* ks = lin_smem;                 // [64][D]
+  float* vs = ks + kLinRun * D;         // [64][TV]
+  __shared__ float pw[kLinRun + 1];
+  pdl_wait();
+  pdl_trigger();
+  const int tiles = a.value_dim / TV, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * TV;
+  const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
+  const int t0 = blockIdx.y * kLinRun;
+  if (t0 >= len) return;
+  const int n = min(kLinRun, len - t0), tid = threadIdx.x;
+  if (tid <= kLinRun) pw[tid] = a.powers[head * (kLinRun + 1) + tid];
+  __syncthreads();
+  float x[8];
+#pragma unroll
+  for (int it = 0; it < kLinRun * D / 8 / 256; ++it) {
+    const int p = tid + it * 256, j = p / (D / 8), c = (p % (D / 8)) * 8;
+    if (j < n) {
+      lin_load8(k + (size_t)(row0 + t0 + j) * a.ldk + head * D + c, a.activation, x);
+      const float f = pw[n - 1 - j];
+      reinterpret_cast<float4*>(ks + j * D + c)[0] = make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f);
+      reinterpret_cast<float4*>(ks + j * D + c)[1] = make_float4(x[4] * f, x[5] * f, x[6] * f, x[7] * f);
+    }
+  }
+#pragma unroll
+  for (int it = 0; it < kLinRun * TV / 8 / 256; ++it) {
+    const int p = tid + it * 256, j = p / (TV / 8), c = (p % (TV / 8)) * 8;
+    if (j < n) {
+      lin_load8(v + (size_t)(row0 + t0 + j) * a.ldv + head * a.value_dim + col0 + c, a.activation, x);
+      reinterpret_cast<float4*>(vs + j * TV + c)[0] = make_float4(x[0], x[1], x[2], x[3]);
+      reinterpret_cast<float4*>(vs + j * TV + c)[1] = make_float4(x[4], x[5], x[6], x[7]);
+    }
+  }
+  __syncthreads();
+  // rows ty * 4 + 64 r + i, columns tx * 4 + 64 g + c
+  constexpr int R = D / 64, G = TV / 64;
+  const int tx = tid & 15, ty = tid >> 4;
+  f32x2 acc[R * 4][G * 2];
+#pragma unroll
+  for (int i = 0; i < R * 4; ++i)
+#pragma unroll
+    for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_pack(0.f, 0.f);
+#pragma unroll 2
+  for (int j = 0; j < n; ++j) {
+    ulonglong2 b[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) b[g] = *reinterpret_cast<const ulonglong2*>(vs + j * TV + g * 64 + tx * 4);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 av = *reinterpret_cast<const float4*>(ks + j * D + r * 64 + ty * 4);
+      const float ai[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const f32x2 aa = f2_pack(ai[i], ai[i]);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          acc[r * 4 + i][2 * g] = f2_fma(aa, b[g].x, acc[r * 4 + i][2 * g]);
+          acc[r * 4 + i][2 * g + 1] = f2_fma(aa, b[g].y, acc[r * 4 + i][2 * g + 1]);
+        }
+      }
+    }
+  }
+  float* dst = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.heads + head) * (size_t)D * a.value_dim + col0;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        ulonglong2 o;
+        o.x = acc[r * 4 + i][2 * g];
+        o.y = acc[r * 4 + i][2 * g + 1];
+        *reinterpret_cast<ulonglong2*>(dst + (size_t)(r * 64 + ty * 4 + i) * a.value_dim + g * 64 + tx * 4) = o;
+      }
+}
+
+// grid (state elements / 1024, entries): S <- lambda^n S + L over the entry's runs, four elements a thread; run_state turns from
+// a run's sum into the state at its start, the last state goes to the slot.
+__global__ void __launch_bounds__(256) lin_fold_kernel(LinRunArgs a, int key_dim) {
+  pdl_wait();
+  pdl_trigger();
+  const int entry = blockIdx.y, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
+  const size_t per_head = (size_t)key_dim * a.value_dim, width = per_head * a.heads;
+  const size_t e = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
+  if (len <= 0 || e >= width) return;
+  const float* pw = a.powers + (e / per_head) * (kLinRun + 1);
+  const int runs = (len + kLinRun - 1) / kLinRun, last = len - (runs - 1) * kLinRun;
+  const float whole = pw[kLinRun], part = pw[last];
+  float* run = a.run_state + lin_first_run(row0, entry) * width + e;
+  float4* slot = reinterpret_cast<float4*>(a.state + (size_t)a.slots[entry] * width + e);
+  float4 st = *slot;
+  constexpr int AHEAD = 8;      // (loads in flight a thread: the fold is a chain of memory latencies)
+  for (int r = 0; r < runs; r += AHEAD) {
+    float4 sum[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+      if (r + u < runs) sum[u] = *reinterpret_cast<const float4*>(run + (size_t)(r + u) * width);
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      if (r + u >= runs) break;
+      *reinterpret_cast<float4*>(run + (size_t)(r + u) * width) = st;
+      const float f = r + u == runs - 1 ? part : whole;
+      st = make_float4(fmaf(f, st.x, sum[u].x), fmaf(f, st.y, sum[u].y), fmaf(f, st.z, sum[u].z), fmaf(f, st.w, sum[u].w));
+    }
+  }
+  *slot = st;
+}
+
+// grid (heads * column tiles, runs, entries): o_i = lambda^(i+1) S^T q_i + sum_(j<=i) (q_i . k_j) lambda^(i-j) v_j, S the state at the
+// run's start.  q and k lie transposed in shared memory ([d][token]); the scores (also transposed) and the tiles of 32 rows
+// of S take k's place once the scores are made.
+template <typename T, int D, int TV>
+__global__ void __launch_bounds__(256, 2)
+lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, LinRunArgs a) {
+  constexpr int SR = 32;                                     // rows of S a tile
+  constexpr int kRegion = D * kLinPad > kLinRun * kLinPad + SR * TV ? D * kLinPad : kLinRun * kLinPad + SR * TV;
+  extern __shared__ __align__(16) float lin_smem[];
+  float* qt = lin_smem;                   // [D][kLinPad]
+  float* kt = qt + D * kLinPad;           // [D][kLinPad], then:
+  float* at = kt;                         // [64][kLinPad]: at[j][i] = (q_i . k_j) lambda^(i-j), 0 above the diagonal
+  float* ss = kt + kLinRun * kLinPad;     // [SR][TV]
+  float* vs = kt + kRegion;               // [64][TV]
+  __shared__ float pw[kLinRun + 1];
+  pdl_wait();
+  pdl_trigger();
+  const int tiles = a.value_dim / TV, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * TV;
+  const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
+  const int t0 = blockIdx.y * kLinRun;
+  if (t0 >= len) return;
+  const int n = min(kLinRun, len - t0), tid = threadIdx.x;
+  const float* S = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.heads + head) * (size_t)D * a.value_dim + col0;
+  constexpr int SV = SR * TV / 4 / 256;                      // 16-byte pieces of a tile of S a thread fetches
+  float4 sp[SV];
+  auto ask = [&](int d0) {
+#pragma unroll
+    for (int it = 0; it < SV; ++it) {
+      const int p = tid + it * 256;
+      sp[it] = *reinterpret_cast<const float4*>(S + (size_t)(d0 + p / (TV / 4)) * a.value_dim + (p % (TV / 4)) * 4);
+    }
+  };
+  ask(0);
+  if (tid <= kLinRun) pw[tid] = a.powers[head * (kLinRun + 1) + tid];
+  float x[8];
+#pragma unroll
+  for (int it = 0; it < kLinRun * D / 8 / 256; ++it) {       // (neighbouring lanes take neighbouring tokens: no bank conflicts in the transposed stores)
+    const int p = tid + it * 256, j = p % kLinRun, c = (p / kLinRun) * 8;
+    const size_t row = (size_t)(row0 + t0 + min(j, n - 1));
+    lin_load8(q + row * a.ldq + head * D + c, a.activation, x);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) qt[(c + e) * kLinPad + j] = x[e];
+    lin_load8(k + row * a.ldk + head * D + c, a.activation, x);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) kt[(c + e) * kLinPad + j] = x[e];
+  }
+#pragma unroll
+  for (int it = 0; it < kLinRun * TV / 8 / 256; ++it) {
+    const int p = tid + it * 256, j = p / (TV / 8), c = (p % (TV / 8)) * 8;
+    if (j < n) {
+      lin_load8(v + (size_t)(row0 + t0 + j) * a.ldv + head * a.value_dim + col0 + c, a.activation, x);
+      reinterpret_cast<float4*>(vs + j * TV + c)[0] = make_float4(x[0], x[1], x[2], x[3]);
+      reinterpret_cast<float4*>(vs + j * TV + c)[1] = make_float4(x[4], x[5], x[6], x[7]);
+    }
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  {
+    float s[4][4];                                           // s[j][i]: keys tx * 4 + j, tokens ty * 4 + i
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[j][i] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < D; ++d) {
+      const float4 qv = *reinterpret_cast<const float4*>(qt + d * kLinPad + ty * 4);
+      const float4 kv = *reinterpret_cast<const float4*>(kt + d * kLinPad + tx * 4);
+      const float qi[4] = {qv.x, qv.y, qv.z, qv.w}, kj[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[j][i] = fmaf(qi[i], kj[j], s[j][i]);
+    }
+    __syncthreads();                                         // k is no longer needed: the scores take its place
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int kj = tx * 4 + j;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int back = ty * 4 + i - kj;
+        s[j][i] = back >= 0 ? s[j][i] * pw[back] : 0.f;
+      }
+      *reinterpret_cast<float4*>(at + kj * kLinPad + ty * 4) = make_float4(s[j][0], s[j][1], s[j][2], s[j][3]);
+    }
+  }
+  constexpr int G = TV / 64;
+  f32x2 acc[4][G * 2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_pack(0.f, 0.f);
+  auto add = [&](const float4& av, const float* brow) {      // acc[i][.] += a[i] * b[.]
+    ulonglong2 b[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) b[g] = *reinterpret_cast<const ulonglong2*>(brow + g * 64 + tx * 4);
+    const float ai[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const f32x2 aa = f2_pack(ai[i], ai[i]);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        acc[i][2 * g] = f2_fma(aa, b[g].x, acc[i][2 * g]);
+        acc[i][2 * g + 1] = f2_fma(aa, b[g].y, acc[i][2 * g + 1]);
+      }
+    }
+  };
+  for (int d0 = 0; d0 < D; d0 += SR) {
+#pragma unroll
+    for (int it = 0; it < SV; ++it) reinterpret_cast<float4*>(ss)[tid + it * 256] = sp[it];
+    __syncthreads();
+    if (d0 + SR < D) ask(d0 + SR);
+#pragma unroll 4
+    for (int d = 0; d < SR; ++d) add(*reinterpret_cast<const float4*>(qt + (d0 + d) * kLinPad + ty * 4), ss + d * TV);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float f = pw[ty * 4 + i + 1];
+    const f32x2 ff = f2_pack(f, f);
+#pragma unroll
+    for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_mul(ff, acc[i][g]);
+  }
+  const int keys = min(n, (tid >> 5) * 8 + 8);               // (a warp holds eight tokens: later keys weigh nothing)
+#pragma unroll 4
+  for (int j = 0; j < keys; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (ty * 4 + i >= n) break;
+    float* dst = a.out + (size_t)(row0 + t0 + ty * 4 + i) * a.heads * a.value_dim + head * a.value_dim + col0;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      ulonglong2 o;
+      o.x = acc[i][2 * g];
+      o.y = acc[i][2 * g + 1];
+      *reinterpret_cast<ulonglong2*>(dst + g * 64 + tx * 4) = o;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------- walk
+// Single tokens and portions of a few: a block holds 32 columns of one head's S in registers (a thread four neighbouring columns
+// of every 32nd row), so a step reads and writes the state once, 16 bytes a load with all of a thread's loads in flight.
+// What bounds it is the launch and one trip to memory: eight tokens of 16 heads of 128 x 128 12 us, 41 in the chunk kernel,
+// whose score is one thread's chain of 128 products for a single token.
+constexpr int kLinWalk = 32;            // the longest portion it takes
+constexpr int kLinWalkStage = 8;        // tokens it holds in shared memory at a time
+
+template <typename T, int ROWS>         // ROWS: key_dim / 32
+__global__ void __launch_bounds__(256)
+lin_walk_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, LinRunArgs a) {
+  constexpr int D = ROWS * 32;
+  constexpr int C = kLinWalkStage;
+  __shared__ float qs[C][D], ks[C][D];
+  __shared__ __align__(16) float vs[C][32];
+  __shared__ float4 red[C][8][8];
+  pdl_wait();
+  pdl_trigger();
+  const int tiles = a.value_dim / 32, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * 32;
+  const int entry = blockIdx.y, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
+  if (len <= 0) return;
+  const int tid = threadIdx.x, cg = tid & 7, rt = tid >> 3;
+  float* S = a.state + ((size_t)a.slots[entry] * a.heads + head) * (size_t)D * a.value_dim + col0 + cg * 4;
+  float4 s[ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) s[i] = *reinterpret_cast<const float4*>(S + (size_t)(rt + 32 * i) * a.value_dim);
+  const float lambda = a.powers[head * (kLinRun + 1) + 1];
+  for (int t0 = 0; t0 < len; t0 += C) {
+    const int n = min(C, len - t0);
+    const size_t first = row0 + t0;
+    for (int e = tid; e < n * D; e += 256) {
+      const int t = e / D, d = e % D;
+      qs[t][d] = lin_act(to_f32(q[(first + t) * a.ldq + head * D + d]), a.activation);
+      ks[t][d] = lin_act(to_f32(k[(first + t) * a.ldk + head * D + d]), a.activation);
+    }
+    if (tid < n * 32)
+      vs[tid >> 5][tid & 31] = lin_act(to_f32(v[(first + (tid >> 5)) * a.ldv + head * a.value_dim + col0 + (tid & 31)]), a.activation);
+    __syncthreads();
+    for (int t = 0; t < n; ++t) {
+      const float4 vv = *reinterpret_cast<const float4*>(&vs[t][cg * 4]);
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const float kk = ks[t][rt + 32 * i], qq = qs[t][rt + 32 * i];
+        s[i] = make_float4(fmaf(lambda, s[i].x, kk * vv.x), fmaf(lambda, s[i].y, kk * vv.y), fmaf(lambda, s[i].z, kk * vv.z),
+                           fmaf(lambda, s[i].w, kk * vv.w));
+        o.x = fmaf(qq, s[i].x, o.x); o.y = fmaf(qq, s[i].y, o.y); o.z = fmaf(qq, s[i].z, o.z); o.w = fmaf(qq, s[i].w, o.w);
+      }
+#pragma unroll
+      for (int m = 8; m < 32; m <<= 1) {
+        o.x += __shfl_xor_sync(0xffffffffu, o.x, m); o.y += __shfl_xor_sync(0xffffffffu, o.y, m);
+        o.z += __shfl_xor_sync(0xffffffffu, o.z, m); o.w += __shfl_xor_sync(0xffffffffu, o.w, m);
+      }
+      if ((tid & 31) < 8) red[t][tid >> 5][cg] = o;
+    }
+    __syncthreads();               // the partial sums are in place, and q, k, v of these tokens no longer needed
+    if (tid < n * 8) {
+      const int t = tid >> 3;
+      float4 o = red[t][0][cg];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) {
+        const float4 p = red[t][w][cg];
+        o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
+      }
+      *reinterpret_cast<float4*>(a.out + (first + t) * a.heads * a.value_dim + head * a.value_dim + col0 + cg * 4) = o;
+    }
+    // (the next tokens' partial sums are written only after the barrier behind their loads, which the threads above reach last)
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) *reinterpret_cast<float4*>(S + (size_t)(rt + 32 * i) * a.value_dim) = s[i];
+}
+
+template <typename T, int D, int TV>
+static int launch_lin_runs(const void* q, const void* k, const void* v, const LinRunArgs& a, int n_entries, int max_q_len, cudaStream_t stream) {
+  constexpr size_t sums = sizeof(float) * kLinRun * (D + TV);
+  constexpr int region = D * kLinPad > kLinRun * kLinPad + 32 * TV ? D * kLinPad : kLinRun * kLinPad + 32 * TV;
+  constexpr size_t outs = sizeof(float) * (D * kLinPad + region + kLinRun * TV);
+  auto ks = lin_run_sums_kernel<T, D, TV>;
+  auto ko = lin_run_out_kernel<T, D, TV>;
+  cudaError_t e = cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outs);
+  if (e != cudaSuccess) return (int)e;
+  const dim3 grid(a.heads * (a.value_dim / TV), ceil_div(max_q_len, kLinRun), n_entries);
+  TIB_LAUNCH_DEPENDENT(ks, grid, 256, sums, stream, (const T*)k, (const T*)v, a);
+  TIB_LAUNCH_DEPENDENT(lin_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.heads * D * a.value_dim, 1024), n_entries), 256, 0, stream, a, D);
+  TIB_LAUNCH_DEPENDENT(ko, grid, 256, outs, stream, (const T*)q, (const T*)k, (const T*)v, a);
+  return TIB_OK;
+}
+
+template <typename T>
+static int launch_lin_walk(const void* q, const void* k, const void* v, const LinRunArgs& a, int key_dim, int n_entries, cudaStream_t stream) {
+  const dim3 grid(a.heads * (a.value_dim / 32), n_entries);
+  if (key_dim == 64) TIB_LAUNCH_DEPENDENT((lin_walk_kernel<T, 2>), grid, 256, 0, stream, (const T*)q, (const T*)k, (const T*)v, a);
+  else TIB_LAUNCH_DEPENDENT((lin_walk_kernel<T, 4>), grid, 256, 0, stream, (const T*)q, (const T*)k, (const T*)v, a);
+  return TIB_OK;
+}
+
 static inline size_t lin_attn_smem(int D, int V, int C) {
   return sizeof(float) * ((size_t)D * V + 2 * (size_t)C * (D + 1) + 3 + (size_t)C * V + (size_t)C * C + C + 1);
 }
@@ -221,16 +618,48 @@ TIB_API int tib_linear_attention_chunk(int key_dim, int value_dim) {
   return 0;
 }
 
+// Tokens of a run, and the longest portion the walk takes.
+TIB_API int tib_linear_attention_run() { return kLinRun; }
+TIB_API int tib_linear_attention_walk() { return kLinWalk; }
+
 // q, k: [tokens, >= heads * key_dim] and v: [tokens, >= heads * value_dim] with row strides ldq, ldk, ldv (they may be
 // slices of one wider row); out: [tokens, heads * value_dim] fp32; state: [slots, heads, key_dim, value_dim] fp32;
 // powers: [heads, chunk + 1] fp32, powers[h][m] = lambda_h^m; activation: 0 none, 1 silu on q, k and v.
+// max_q_len: the longest entry of the step, 0 where it is not known (then, or without run_powers, the chunk kernel runs).
+// run_powers: [heads, run + 1] fp32 likewise, or null.  run_state: scratch of run_capacity >= tokens / run + n_entries times
+// heads * key_dim * value_dim floats for portions of more than tib_linear_attention_walk() tokens, or null.
 TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, int64_t ldq, int64_t ldk, int64_t ldv,
                                  float* out, float* state, const float* powers, const int* q_start, const int* slots,
                                  int n_entries, int heads, int key_dim, int value_dim, int chunk, int activation, int dtype,
+                                 int tokens, int max_q_len, const float* run_powers, float* run_state, int64_t run_capacity,
                                  cudaStream_t stream) {
   if (n_entries == 0) return TIB_OK;
   if (!q || !k || !v || !out || !state || !powers || !q_start || !slots) return TIB_E_ARG;
   if (heads < 1 || key_dim < 1 || value_dim < 1 || chunk < 1 || chunk > 32 || n_entries > 65535) return TIB_E_SIZE;
+  // The newer kernels take heads of 64 or 128 keys whose values come in whole tiles, rows and state on 16-byte boundaries.
+  // The line between walk and runs: at 32 tokens a portion both take some 40 us (four portions of 16 heads of 128 x 128: the walk
+  // 14, 16 and 23 us at 8, 9 and 16 tokens, the runs' three launches 52 at 9, 54 at 16 and 71 at 64; the chunk kernel 33, 35, 78).
+  const int64_t size = dtype == TIB_F32 ? 4 : 2;
+  const bool aligned = (ldq * size) % 16 == 0 && (ldk * size) % 16 == 0 && (ldv * size) % 16 == 0 &&
+                       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)run_state) & 15) == 0;
+  if (run_powers && max_q_len > 0 && (key_dim == 64 || key_dim == 128) && value_dim % 32 == 0 && aligned &&
+      (dtype == TIB_F32 || dtype == TIB_BF16)) {
+    LinRunArgs r;
+    r.q_start = q_start; r.slots = slots; r.powers = run_powers; r.state = state; r.run_state = run_state; r.out = out;
+    r.ldq = ldq; r.ldk = ldk; r.ldv = ldv; r.heads = heads; r.value_dim = value_dim; r.activation = activation;
+    if (max_q_len <= kLinWalk)
+      return dtype == TIB_F32 ? launch_lin_walk<float>(q, k, v, r, key_dim, n_entries, stream)
+                              : launch_lin_walk<__nv_bfloat16>(q, k, v, r, key_dim, n_entries, stream);
+    if (run_state && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535) {
+#define TIB_LIN_GO(T)                                                                                             \
+  (key_dim == 64 ? (value_dim % 128 == 0 ? launch_lin_runs<T, 64, 128>(q, k, v, r, n_entries, max_q_len, stream)    \
+                                         : launch_lin_runs<T, 64, 64>(q, k, v, r, n_entries, max_q_len, stream))    \
+                 : (value_dim % 128 == 0 ? launch_lin_runs<T, 128, 128>(q, k, v, r, n_entries, max_q_len, stream)   \
+                                         : launch_lin_runs<T, 128, 64>(q, k, v, r, n_entries, max_q_len, stream)))
+      return dtype == TIB_F32 ? TIB_LIN_GO(float) : TIB_LIN_GO(__nv_bfloat16);
+#undef TIB_LIN_GO
+    }
+  }
   LinAttnArgs a;
   a.q_start = q_start; a.slots = slots; a.powers = powers; a.state = state; a.out = out;
   a.ldq = ldq; a.ldk = ldk; a.ldv = ldv;

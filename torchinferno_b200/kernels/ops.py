@@ -121,7 +121,7 @@ def lib() -> ctypes.CDLL:
                    "tib_gemm_tcgen05_swapab", "tib_gemm_tcgen05_swapab_supports", "tib_gemm_decode", "tib_gemm_decode_supports",
                    "tib_plan_attention", "tib_plan_product", "tib_blas_gemm_batched",
                    "tib_add_pair", "tib_unit_norm_add", "tib_sigmoid_gate", "tib_gelu_gate_table", "tib_relu_squared", "tib_gelu",
-                   "tib_scale_f32", "tib_pair_rows", "tib_add_vector", "tib_linear_attention", "tib_linear_attention_chunk",
+                   "tib_scale_f32", "tib_pair_rows", "tib_add_vector", "tib_linear_attention", "tib_linear_attention_chunk", "tib_linear_attention_run", "tib_linear_attention_walk",
                    "tib_latent_append", "tib_latent_attention", "tib_latent_attention_splits", "tib_moe_route", "tib_moe_group", "tib_router_logits",
                    "tib_moe_expert_product", "tib_moe_combine", "tib_glu_clamp", "tib_layernorm", "tib_layernorm_tail",
                    "tib_qk_norm_append", "tib_sigmoid_attention", "tib_sigmoid_attention_takes_mma", "tib_gated_recurrence",
@@ -887,11 +887,22 @@ def linear_attention_chunk(key_dim: int, value_dim: int) -> int:
     return int(lib().tib_linear_attention_chunk(c_int(key_dim), c_int(value_dim)))
 
 
+def linear_attention_run() -> int:
+    """Tokens of a run of the decayed linear attention (long portions are cut into runs that go side by side)."""
+    return int(lib().tib_linear_attention_run())
+
+
+LINEAR_ATTENTION_SCRATCH = 1 << 30      # bytes of run states a call may take (2,048 tokens of 16 heads of 128 x 128: 34 MB)
+
+
 def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
                      powers: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, n_entries: int, heads: int,
-                     key_dim: int, value_dim: int, *, silu: bool) -> torch.Tensor:
+                     key_dim: int, value_dim: int, *, silu: bool, max_q_len: int = 0,
+                     run_powers: torch.Tensor | None = None) -> torch.Tensor:
     """o_t = S_t^T q_t with S_t = decay * S_(t-1) + k_t v_t^T per head, over the ragged batch; ``state``
-    [slots, heads, key_dim, value_dim] (fp32) is read and left updated; ``powers`` [heads, chunk + 1] holds decay^m."""
+    [slots, heads, key_dim, value_dim] (fp32) is read and left updated; ``powers`` [heads, chunk + 1] holds decay^m.
+    With the step's longest entry and ``run_powers`` [heads, linear_attention_run() + 1] (decay^m again) long portions run in
+    pieces side by side and single tokens by a kernel of their own, where those kernels take the head sizes."""
     for name, t, width in (("q", q, heads * key_dim), ("k", k, heads * key_dim), ("v", v, heads * value_dim)):
         _rows_of(t, name, width)
         if t.dtype != q.dtype:
@@ -903,10 +914,21 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
         raise KernelError("linear_attention: out, state or powers do not fit the head sizes")
     if q_start.numel() < n_entries + 1 or slots.numel() < n_entries:
         raise KernelError("linear_attention: entry arrays are shorter than n_entries")
+    run_state, capacity = None, 0
+    if run_powers is not None:
+        run = linear_attention_run()
+        _need(run_powers, "run_powers", torch.float32)
+        if run_powers.shape != (heads, run + 1):
+            raise KernelError("linear_attention: run_powers has the wrong shape")
+        if max_q_len > int(lib().tib_linear_attention_walk()) and key_dim in (64, 128) and value_dim % 64 == 0:
+            capacity = q.shape[0] // run + n_entries
+            if capacity * heads * key_dim * value_dim * 4 <= LINEAR_ATTENTION_SCRATCH:
+                run_state = torch.empty(capacity * heads * key_dim * value_dim, dtype=torch.float32, device=q.device)
     _check("linear_attention", lib().tib_linear_attention(
         _ptr(q), _ptr(k), _ptr(v), c_int64(q.stride(0)), c_int64(k.stride(0)), c_int64(v.stride(0)), _ptr(out), _ptr(state),
         _ptr(powers), _ptr(q_start), _ptr(slots), c_int(n_entries), c_int(heads), c_int(key_dim), c_int(value_dim),
-        c_int(chunk), c_int(1 if silu else 0), c_int(_code(q.dtype)), _stream()))
+        c_int(chunk), c_int(1 if silu else 0), c_int(_code(q.dtype)), c_int(q.shape[0]), c_int(max_q_len), _ptr(run_powers),
+        _ptr(run_state), c_int64(capacity), _stream()))
     return out
 
 

@@ -39,6 +39,7 @@ class DecayLinearAttention(Mixer):
         self.o_weight: LinearWeight | None = None
         self.norm_weight: torch.Tensor | None = None
         self.powers: torch.Tensor | None = None
+        self.run_powers: torch.Tensor | None = None
 
     def weight_specs(self) -> list[WeightSpec]:
         n, qk, vv = self.names, self.heads * self.key_dim, self.heads * self.value_dim
@@ -62,9 +63,13 @@ class DecayLinearAttention(Mixer):
         chunk = ops.linear_attention_chunk(self.key_dim, self.value_dim) if device.type == "cuda" else 1
         if chunk < 1:
             raise ValueError(f"heads of {self.key_dim} x {self.value_dim} do not fit the linear attention kernel")
-        # decay^m for m = 0 .. chunk, made in double precision
-        table = torch.tensor(self.decay, dtype=torch.float64)[:, None] ** torch.arange(chunk + 1, dtype=torch.float64)[None, :]
-        self.powers = table.to(torch.float32).contiguous().to(device)
+        # decay^m for m = 0 .. chunk (and up to the length of a run), made in double precision
+        def powers(most: int) -> torch.Tensor:
+            table = torch.tensor(self.decay, dtype=torch.float64)[:, None] ** torch.arange(most + 1, dtype=torch.float64)[None, :]
+            return table.to(torch.float32).contiguous().to(device)
+
+        self.powers = powers(chunk)
+        self.run_powers = powers(ops.linear_attention_run()) if device.type == "cuda" else None
 
     def state_spec(self) -> StateSpec:
         return StateSpec((self.heads, self.key_dim, self.value_dim), torch.float32)
@@ -78,7 +83,7 @@ class DecayLinearAttention(Mixer):
         q, k, v = proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + vv]
         mixed = torch.empty((n, vv), dtype=torch.float32, device=x.device)
         ops.linear_attention(q, k, v, mixed, ctx.state, self.powers, batch.q_start, batch.slots, batch.n_entries, self.heads,
-                             self.key_dim, self.value_dim, silu=self.activation == "silu")
+                             self.key_dim, self.value_dim, silu=self.activation == "silu", max_q_len=batch.max_q_len, run_powers=self.run_powers)
         if self.gate:
             rows = torch.empty((n, vv), dtype=x.dtype, device=x.device)
             ops.sigmoid_gate(mixed, proj[:, 2 * qk + vv:], rows, self.norm_weight, self.eps)
