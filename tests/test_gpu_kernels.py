@@ -937,3 +937,47 @@ def test_linear_attention_forms_agree_with_the_recurrence(lens, heads, key_dim, 
     assert (as_ref(out) - want.reshape(n, -1)).abs().max() <= 2e-6 * want.abs().max()
     assert (as_ref(got_state) - want_state).abs().max() <= 2e-6 * want_state.abs().max()
 
+
+
+# ------------------------------------------------------------------------------------------------- the experts' products
+@pytest.mark.parametrize("tokens, experts, top, k, n, act, by_pair, out_dtype", [
+    (1, 1, 1, 8, 16, "none", True, torch.float32), (5, 4, 2, 72, 130, "relu2", True, torch.bfloat16),      # tails of k and of the features
+    (40, 3, 2, 128, 96, "silu", True, torch.bfloat16), (90, 3, 2, 200, 136, "gelu", True, torch.float32),   # tiles of 64 and 96 rows
+    (400, 5, 2, 192, 192, "swiglu", True, torch.bfloat16), (330, 2, 1, 64, 258, "glu_clamp", True, torch.bfloat16),      # 160, several a expert
+    (64, 16, 1, 64, 128, "none", False, torch.float32), (700, 3, 2, 136, 260, "none", False, torch.float32)])            # rows already sorted
+def test_expert_product_on_uneven_experts(tokens, experts, top, k, n, act, by_pair, out_dtype):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    pairs, gated = tokens * top, act in ("swiglu", "glu_clamp")
+    scores = rnd(tokens, experts, seed=2)
+    scores[:, 0] += 1.5                                   # (one expert gets many rows, some perhaps none)
+    ids = scores.topk(top, -1).indices.int().contiguous()
+    offsets, order, place = (torch.empty(m, dtype=torch.int32, device="cuda") for m in (experts + 1, pairs, pairs))
+    ops.moe_group(dev(ids), experts, offsets, order, place)
+    x, w = rnd(tokens if by_pair else pairs, k, dtype=torch.bfloat16), rnd(experts, n, k, dtype=torch.bfloat16, scale=k ** -0.5, seed=3)
+    factor = rnd(pairs, seed=4).abs() if gated else None
+    y = torch.full((pairs, n // 2 if gated else n), float("nan"), dtype=out_dtype, device="cuda")
+    error = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.moe_expert_product(dev(x), dev(w), y, offsets, order, top, x_by_pair=by_pair, act=act, limit=2.0, alpha=1.702,
+                           row_scale=None if factor is None else dev(factor), error_word=error)
+    assert int(error) == 0
+    order, expert_of = order.cpu().long(), ids.flatten().long()
+    assert torch.equal(expert_of[order], expert_of.sort()[0])
+    rows = x.double()[order // top] if by_pair else x.double()
+    v = torch.einsum("sk,snk->sn", rows, w.double()[expert_of[order]])
+    if factor is not None:
+        v = v * factor.double()[order][:, None]
+    if act == "relu2":
+        v = v.clamp(min=0) ** 2
+    elif act == "silu":
+        v = v * torch.sigmoid(v)
+    elif act == "gelu":
+        v = 0.5 * v * (1 + torch.erf(v * 0.5 ** 0.5))
+    elif act == "swiglu":
+        v = v[:, 0::2] * torch.sigmoid(v[:, 0::2]) * v[:, 1::2]
+    elif act == "glu_clamp":
+        g = v[:, 0::2].clamp(max=2.0)
+        v = g * torch.sigmoid(1.702 * g) * (v[:, 1::2].clamp(-2.0, 2.0) + 1)
+    # exact bf16 products, fp32 sums of k of them (2^-23 of the largest partial sum each), then one rounding to the output type
+    bound = (2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0) * v.abs() + 4 * k * 2.0 ** -23
+    assert ((as_ref(y) - v).abs() <= bound).all()

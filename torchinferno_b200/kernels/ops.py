@@ -1055,7 +1055,7 @@ def moe_group(ids: torch.Tensor, experts: int, offsets: torch.Tensor, order: tor
 
 def moe_expert_product(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, offsets: torch.Tensor, order: torch.Tensor, top: int,
                        *, x_by_pair: bool, act: str = "none", limit: float = 0.0, alpha: float = 1.0,
-                       row_scale: torch.Tensor | None = None) -> torch.Tensor:
+                       row_scale: torch.Tensor | None = None, error_word: torch.Tensor | None = None) -> torch.Tensor:
     """y[s] = act(row_scale[pair of s] * (x[source of s] . w[expert of s]^T)) for the sorted rows s; ``w``: [experts, N, K];
     ``x_by_pair``: the source of sorted row s is token order[s] // top, else row s itself.  ``act="glu_clamp"``: the rows
     of ``w`` are (gate i, up i) pairs and y has N / 2 columns: g * sigmoid(alpha g) * (u + 1) with g = min(g, limit),
@@ -1073,7 +1073,7 @@ def moe_expert_product(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, offset
     _check("moe_expert_product", lib().tib_moe_expert_product(
         _ptr(x), c_int(_code(x.dtype)), c_int64(x.stride(0)), _ptr(w), c_int(_code(w.dtype)), _ptr(y), c_int(_code(y.dtype)),
         c_int64(y.stride(0)), _ptr(offsets), _ptr(order), c_int(pairs), c_int(experts), c_int(top), c_int(int(x_by_pair)),
-        c_int(n), c_int(k), c_int(MOE_ACT[act]), c_float(limit), c_float(alpha), _ptr(row_scale), _stream()))
+        c_int(n), c_int(k), c_int(MOE_ACT[act]), c_float(limit), c_float(alpha), _ptr(row_scale), _ptr(error_word), _stream()))
     return y
 
 

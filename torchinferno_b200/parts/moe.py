@@ -125,6 +125,7 @@ class RoutedExperts(FeedForward):
 
     def forward(self, x: torch.Tensor, ctx: LayerContext) -> torch.Tensor:
         n, dev, top = x.shape[0], x.device, self.top
+        error_word = None if ctx is None else ctx.error_word
         logits = torch.empty((n, self.router_weight.shape[0]), dtype=torch.float32, device=dev)
         ops.router_logits(x, self.router_weight, logits, self.router_bias)
         ids = torch.empty((n, top), dtype=torch.int32, device=dev)
@@ -138,9 +139,10 @@ class RoutedExperts(FeedForward):
         ops.moe_group(ids, self.experts, offsets, order, place)
         inner = torch.empty((n * top, self.expert_size), dtype=x.dtype, device=dev)
         ops.moe_expert_product(x, self.up_weight, inner, offsets, order, top, x_by_pair=True, act=self.activation,
-                               limit=self.limit, alpha=self.alpha, row_scale=weights.view(-1) if self.weight_on_input else None)
+                               limit=self.limit, alpha=self.alpha, row_scale=weights.view(-1) if self.weight_on_input else None,
+                               error_word=error_word)
         outer = torch.empty((n * top, self.hidden_size), dtype=torch.float32, device=dev)
-        ops.moe_expert_product(inner, self.down_weight, outer, offsets, order, top, x_by_pair=False)
+        ops.moe_expert_product(inner, self.down_weight, outer, offsets, order, top, x_by_pair=False, error_word=error_word)
         shared_rows = None
         if self.shared_size:
             hidden = linear(x, self.shared_up_weight)
