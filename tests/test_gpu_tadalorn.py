@@ -848,3 +848,35 @@ def test_sizes_drawn_at_random(draw, tmp_path):
             runner = make_runner(tmp_path, dtype, replay_util.peak_tokens(steps), page_size=rng.choice([4, 16]))
             rows = replay_util.gather(run_steps(runner, steps), index)
             compare(rows, tmp_path, requests, dtype, f"draw {draw} {kind}")
+
+
+@pytest.mark.parametrize("heads,dim,rot,vdim,rank,gate,q_rank", [(2, 128, 64, 128, 512, True, None), (3, 64, 32, 128, 72, "head", 24),
+                                                                 (1, 128, 8, 64, 64, False, None), (2, 64, 64, 64, 128, True, 40)])
+def test_prompts_on_keys_and_values_made_for_the_step(heads, dim, rot, vdim, rank, gate, q_rank):
+    """Portions that end at, before and behind the edges of tiles of 128 tokens and keys, behind cached context and beside other
+    requests, against the folded form of the same layer (which the plain implementations check) in 32 bits."""
+    need_gpu()
+    from torchinferno_b200.parts.base import PartSpec, build_part
+    from torchinferno_b200.weights.random_init import random_tensor
+    W = 64
+    params = {"hidden_size": W, "heads": heads, "dim": dim, "rot_dim": rot, "value_dim": vdim, "kv_rank": rank, "scale": 0.7 / math.sqrt(dim + rot),
+              "rot_base": 3000.0, "eps": 1e-5, "sink": True, "gate": gate, "q_rank": q_rank, "pairing": "half" if q_rank else "interleaved"}
+    outs = {}
+    x = {r: torch.randn(n, W, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16) for i, (r, n) in enumerate((("a", 401), ("b", 256), ("c", 30)))}
+    steps = [[("a", 127), ("b", 20)], [("b", 109), ("a", 1), ("c", 30)], [("a", 129)], [("a", 144), ("b", 127)]]
+    for dtype in (torch.float32, torch.bfloat16):
+        mixer = build_part("mixer", PartSpec("latent_attention", params), dtype=dtype, device=CUDA)
+        _bind(mixer, {ws.name: random_tensor(ws, 4, dtype=torch.bfloat16) for ws in mixer.weight_specs()}, dtype, "mix.")
+        rows = []
+        if dtype == torch.bfloat16:
+            assert mixer.unfold is not None
+            plan = mixer._unfolded_rows
+            mixer._unfolded_rows = lambda batch: rows.append(plan(batch)) or rows[-1]
+        cache = _cache_for(mixer, dtype, 16, 64, 4, 416)
+        for r in x:
+            cache.open(r)
+        outs[dtype] = _run_steps(mixer, cache, steps, {r: t.to(dtype) for r, t in x.items()})
+        assert dtype == torch.float32 or rows == [256, 512, 384, 768]      # (the layer took the path, with padded rows)
+    for r in x:
+        err = _row_error(outs[torch.bfloat16][r].double(), outs[torch.float32][r].double())
+        assert err.max() <= 0.03, (r, int(err.argmax()), float(err.max()))      # (the bound of the layer's other tests in bfloat16)

@@ -41,14 +41,19 @@ struct LatentAppendArgs {
   float eps;
   int* error_word;
   int half_pairs;             // 0: rotary pairs are (2i, 2i + 1); 1: (i, i + n_freq)
+  int in_place;               // the rotated query parts replace the unrotated ones in q instead of going to the folded rows
 };
+constexpr int kAppendFreq = 256;      // frequencies whose cosine and sine a block keeps for all its heads
 
+// A block per token.  Cosine and sine of the token's angles are made once for all heads (at positions of thousands they take the
+// functions' slow path).
 template <typename T>
-__global__ void latent_append_kernel(const T* __restrict__ dkv, const T* __restrict__ q, T* __restrict__ pool,
+__global__ void latent_append_kernel(const T* __restrict__ dkv, T* __restrict__ q, T* __restrict__ pool,
                                      float* __restrict__ folded, LatentAppendArgs a) {
   pdl_wait();
   pdl_trigger();
   __shared__ float scratch[33];
+  __shared__ float cos_s[kAppendFreq], sin_s[kAppendFreq];
   const size_t t = blockIdx.x;
   const int pos = a.positions[t];
   const int width = a.rank + a.rot;
@@ -62,32 +67,46 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, const T* __restr
       atomicExch(a.error_word, 0x20000 + (int)(t & 0xffff));
     }
   }
+  for (int i = threadIdx.x; i < min(a.n_freq, kAppendFreq); i += blockDim.x) {
+    const float angle = (float)pos * a.inv_freq[i];
+    cos_s[i] = cosf(angle);
+    sin_s[i] = sinf(angle);
+  }
   float ss = 0.f;
   for (int c = threadIdx.x; c < a.rank; c += blockDim.x) {
     const float v = to_f32(src[c]);
     ss += v * v;
   }
-  const float inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)a.rank + a.eps);
+  const float inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)a.rank + a.eps);      // (its barriers publish the table too)
   if (dst)
     for (int c = threadIdx.x; c < a.rank; c += blockDim.x) dst[c] = from_f32<T>(to_f32(src[c]) * inv * a.norm_weight[c]);
-  // the shared key part (job 0) and every head's rotated query part (jobs 1 .. heads)
+  auto turn = [&](int i, float& c, float& sn) {
+    if (i < kAppendFreq) { c = cos_s[i]; sn = sin_s[i]; return; }
+    const float angle = (float)pos * a.inv_freq[i];
+    c = cosf(angle);
+    sn = sinf(angle);
+  };
+  // job 0: the shared key part; jobs 1 .. heads: every head's rotated query part
+  auto from_of = [&](int job) { return job == 0 ? src + a.rank : q + t * a.ld_q + (size_t)(job - 1) * (a.dim + a.rot) + a.dim; };
+  auto put = [&](int job, int i, float v) {
+    if (job == 0) { if (dst) dst[a.rank + i] = from_f32<T>(v); }
+    else if (a.in_place) q[t * a.ld_q + (size_t)(job - 1) * (a.dim + a.rot) + a.dim + i] = from_f32<T>(v);
+    else folded[(t * a.heads + (job - 1)) * (size_t)width + a.rank + i] = v;
+  };
   if (a.half_pairs) {
     // pairs (i, i + n_freq) over the first 2 * n_freq elements; the rest pass unchanged
     for (int e = threadIdx.x; e < (a.heads + 1) * a.rot; e += blockDim.x) {
       const int job = e / a.rot, i = e - job * a.rot;
       if (i >= a.n_freq && i < 2 * a.n_freq) continue;       // (written with its partner)
-      const T* from = job == 0 ? src + a.rank : q + t * a.ld_q + (size_t)(job - 1) * (a.dim + a.rot) + a.dim;
-      float* f = job == 0 ? nullptr : folded + (t * a.heads + (job - 1)) * (size_t)width + a.rank;
+      const T* from = from_of(job);
       if (i < a.n_freq) {
         const float lo = to_f32(from[i]), hi = to_f32(from[i + a.n_freq]);
-        const float angle = (float)pos * a.inv_freq[i];
-        const float c = cosf(angle), sn = sinf(angle);
-        const float l2 = rope_lo(lo, hi, c, sn), h2 = rope_hi(lo, hi, c, sn);
-        if (f) { f[i] = l2; f[i + a.n_freq] = h2; }
-        else if (dst) { dst[a.rank + i] = from_f32<T>(l2); dst[a.rank + i + a.n_freq] = from_f32<T>(h2); }
-      } else {
-        if (f) f[i] = to_f32(from[i]);
-        else if (dst) dst[a.rank + i] = from[i];
+        float c, sn;
+        turn(i, c, sn);
+        put(job, i, rope_lo(lo, hi, c, sn));
+        put(job, i + a.n_freq, rope_hi(lo, hi, c, sn));
+      } else if (job == 0 || !a.in_place) {
+        put(job, i, to_f32(from[i]));
       }
     }
     return;
@@ -96,24 +115,21 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, const T* __restr
   const int half = a.rot / 2;      // an odd last element, if any, passes unchanged below
   for (int e = threadIdx.x; e < (a.heads + 1) * half; e += blockDim.x) {
     const int job = e / half, i = e - job * half;
-    const T* from = job == 0 ? src + a.rank : q + t * a.ld_q + (size_t)(job - 1) * (a.dim + a.rot) + a.dim;
-    float lo = to_f32(from[2 * i]), hi = to_f32(from[2 * i + 1]);
+    const T* from = from_of(job);
+    const float lo = to_f32(from[2 * i]), hi = to_f32(from[2 * i + 1]);
     if (i < a.n_freq) {
-      const float angle = (float)pos * a.inv_freq[i];
-      const float c = cosf(angle), s = sinf(angle);
-      const float l2 = rope_lo(lo, hi, c, s), h2 = rope_hi(lo, hi, c, s);
-      lo = l2; hi = h2;
-    }
-    if (job == 0) {
-      if (dst) { dst[a.rank + 2 * i] = from_f32<T>(lo); dst[a.rank + 2 * i + 1] = from_f32<T>(hi); }
-    } else {
-      float* f = folded + (t * a.heads + (job - 1)) * (size_t)width + a.rank;
-      f[2 * i] = lo; f[2 * i + 1] = hi;
+      float c, sn;
+      turn(i, c, sn);
+      put(job, 2 * i, rope_lo(lo, hi, c, sn));
+      put(job, 2 * i + 1, rope_hi(lo, hi, c, sn));
+    } else if (job == 0 || !a.in_place) {
+      put(job, 2 * i, lo);
+      put(job, 2 * i + 1, hi);
     }
   }
   if ((a.rot & 1) && threadIdx.x == 0) {
     if (dst) dst[width - 1] = src[width - 1];
-    for (int h = 0; h < a.heads; ++h)
+    for (int h = 0; h < a.heads && !a.in_place; ++h)
       folded[(t * a.heads + h) * (size_t)width + width - 1] = to_f32(q[t * a.ld_q + (size_t)h * (a.dim + a.rot) + a.dim + a.rot - 1]);
   }
 }
@@ -592,15 +608,15 @@ using namespace tib;
 
 // dkv: [tokens, rank + rot] (row stride ld_dkv); q: [tokens, heads * (dim + rot)] (row stride ld_q); pool: this layer's
 // pages, each [page_size][rank + rot] (null: nothing is stored); folded: [tokens, heads, rank + rot] fp32, of which
-// this call writes the last `rot` elements of every head.  half_pairs: the rotary pairs are (i, i + n_freq) instead of
+// this call writes the last `rot` elements of every head, or null: then the rotated query parts replace those in q.  half_pairs: the rotary pairs are (i, i + n_freq) instead of
 // (2i, 2i + 1).
-TIB_API int tib_latent_append(const void* dkv, int64_t ld_dkv, const void* q, int64_t ld_q, void* pool, float* folded,
+TIB_API int tib_latent_append(const void* dkv, int64_t ld_dkv, void* q, int64_t ld_q, void* pool, float* folded,
                               const int* positions, const int* token_slot, const int* block_table, int table_stride,
                               const float* norm_weight, float eps, const float* inv_freq, int n_freq, int n_tokens, int heads,
                               int dim, int rank, int rot, int page_size, int64_t page_stride, int num_pages,
                               int half_pairs, int* error_word, int dtype, cudaStream_t stream) {
   if (n_tokens == 0) return TIB_OK;
-  if (!dkv || !q || !folded || !positions || !norm_weight || (n_freq > 0 && !inv_freq)) return TIB_E_ARG;
+  if (!dkv || !q || !positions || !norm_weight || (n_freq > 0 && !inv_freq)) return TIB_E_ARG;
   if (pool && (!token_slot || !block_table || page_size < 1)) return TIB_E_ARG;
   if (heads < 1 || dim < 0 || rank < 1 || rot < 0 || 2 * n_freq > rot) return TIB_E_SIZE;
   LatentAppendArgs a;
@@ -608,12 +624,13 @@ TIB_API int tib_latent_append(const void* dkv, int64_t ld_dkv, const void* q, in
   a.norm_weight = norm_weight; a.inv_freq = inv_freq; a.n_freq = n_freq; a.rank = rank; a.rot = rot; a.heads = heads;
   a.dim = dim; a.ld_dkv = ld_dkv; a.ld_q = ld_q; a.page_size = page_size; a.num_pages = num_pages;
   a.page_stride = page_stride; a.eps = eps; a.error_word = error_word; a.half_pairs = half_pairs;
+  a.in_place = folded == nullptr;
   if (dtype == TIB_F32)
-    TIB_LAUNCH_DEPENDENT(latent_append_kernel<float>, n_tokens, 128, 0, stream, (const float*)dkv, (const float*)q,
+    TIB_LAUNCH_DEPENDENT(latent_append_kernel<float>, n_tokens, 128, 0, stream, (const float*)dkv, (float*)q,
                          (float*)pool, folded, a);
   else if (dtype == TIB_BF16)
     TIB_LAUNCH_DEPENDENT(latent_append_kernel<__nv_bfloat16>, n_tokens, 128, 0, stream, (const __nv_bfloat16*)dkv,
-                         (const __nv_bfloat16*)q, (__nv_bfloat16*)pool, folded, a);
+                         (__nv_bfloat16*)q, (__nv_bfloat16*)pool, folded, a);
   else
     return TIB_E_DTYPE;
   return TIB_OK;

@@ -122,7 +122,7 @@ def lib() -> ctypes.CDLL:
                    "tib_plan_attention", "tib_plan_product", "tib_blas_gemm_batched",
                    "tib_add_pair", "tib_unit_norm_add", "tib_sigmoid_gate", "tib_gelu_gate_table", "tib_relu_squared", "tib_gelu",
                    "tib_scale_f32", "tib_pair_rows", "tib_add_vector", "tib_linear_attention", "tib_linear_attention_chunk", "tib_linear_attention_run", "tib_linear_attention_walk",
-                   "tib_latent_append", "tib_latent_attention", "tib_latent_attention_splits", "tib_moe_route", "tib_moe_group", "tib_router_logits",
+                   "tib_latent_append", "tib_latent_prefill_supports", "tib_latent_gather", "tib_latent_prefill", "tib_latent_attention", "tib_latent_attention_splits", "tib_moe_route", "tib_moe_group", "tib_router_logits",
                    "tib_moe_expert_product", "tib_moe_combine", "tib_glu_clamp", "tib_layernorm", "tib_layernorm_tail",
                    "tib_qk_norm_append", "tib_sigmoid_attention", "tib_sigmoid_attention_takes_mma", "tib_gated_recurrence",
                    "tib_softcap_f32", "tib_short_conv", "tib_ssd_scan", "tib_ssd_scan_max_state", "tib_ssd_scan_run", "tib_gated_group_norm",
@@ -933,18 +933,21 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
 
 
 # ---------------------------------------------------------------------------
-def latent_append(dkv: torch.Tensor, q: torch.Tensor, folded: torch.Tensor, keys: torch.Tensor | None,
+def latent_append(dkv: torch.Tensor, q: torch.Tensor, folded: torch.Tensor | None, keys: torch.Tensor | None,
                   positions: torch.Tensor, token_slot: torch.Tensor | None, block_table: torch.Tensor | None,
                   norm_weight: torch.Tensor, eps: float, inv_freq: torch.Tensor, heads: int, dim: int, rank: int, rot: int,
                   error_word: torch.Tensor | None = None, half_pairs: bool = False) -> None:
     """Norm the latent, rotate the shared key part and store both in the tokens' pages (``keys``: [pages, 1, page_size,
-    rank + rot], or None to store nothing); rotate every head's query part into ``folded[..., rank:]``.  The rotary pairs
+    rank + rot], or None to store nothing); rotate every head's query part into ``folded[..., rank:]`` (None: in place, in ``q``).  The rotary pairs
     are (2i, 2i + 1), or with ``half_pairs`` (i, i + len(inv_freq)), over the first 2 * len(inv_freq) rotated elements."""
     _rows_of(dkv, "dkv", rank + rot), _rows_of(q, "q", heads * (dim + rot))
-    _need(folded, "folded", torch.float32), _need(positions, "positions", torch.int32)
+    if folded is not None:
+        _need(folded, "folded", torch.float32)
+    _need(positions, "positions", torch.int32)
     _need(norm_weight, "norm_weight", torch.float32), _need(inv_freq, "inv_freq", torch.float32)
     n = dkv.shape[0]
-    if q.dtype != dkv.dtype or q.shape[0] != n or folded.shape != (n, heads, rank + rot) or norm_weight.numel() != rank:
+    if q.dtype != dkv.dtype or q.shape[0] != n or norm_weight.numel() != rank \
+            or (folded is not None and folded.shape != (n, heads, rank + rot)):
         raise KernelError("latent_append: shapes or types do not fit")
     page_size = page_stride = num_pages = table_stride = 0
     if keys is not None:
@@ -996,6 +999,63 @@ def latent_attention(folded: torch.Tensor, keys: torch.Tensor, out: torch.Tensor
         c_int(max_kv_len), c_int(int(force_simt)), _ptr(error_word), c_int(_code(keys.dtype)), _stream()))
     if partial is not None:
         count_launches(1)
+    return out
+
+
+LATENT_TILE = 128      # an entry's keys made for the step are padded to a multiple of this many rows
+
+
+def latent_prefill_supports(dim: int, value_dim: int, rank: int, rot: int) -> bool:
+    """Whether prompt portions of these head sizes may run on keys and values made for the step (bfloat16)."""
+    return bool(lib().tib_latent_prefill_supports(c_int(dim), c_int(value_dim), c_int(rank), c_int(rot)))
+
+
+def latent_gather(keys: torch.Tensor, block_table: torch.Tensor, q_start: torch.Tensor, kv_start: torch.Tensor, slots: torch.Tensor,
+                  n_entries: int, max_kv_len: int, latent: torch.Tensor, rotated: torch.Tensor,
+                  error_word: torch.Tensor | None = None) -> None:
+    """The cached rows of every entry (its earlier tokens and this step's), dense: ``latent`` [rows, rank] and ``rotated``
+    [rows, rot]; an entry takes its length rounded up to LATENT_TILE rows, the last of them zeros."""
+    _need(latent, "latent", torch.bfloat16), _need(rotated, "rotated", torch.bfloat16)
+    rank, rot = latent.shape[1], rotated.shape[1]
+    for name, t in (("q_start", q_start), ("kv_start", kv_start), ("slots", slots), ("block_table", block_table)):
+        _need(t, name, torch.int32)
+    if keys.dtype != torch.bfloat16 or keys.dim() != 4 or keys.shape[1] != 1 or keys.shape[3] != rank + rot or keys.stride(3) != 1 \
+            or keys.stride(2) != rank + rot or latent.shape[0] != rotated.shape[0]:
+        raise KernelError("latent_gather: pages or rows do not fit")
+    if q_start.numel() < n_entries + 1 or kv_start.numel() < n_entries or slots.numel() < n_entries:
+        raise KernelError("latent_gather: entry arrays are shorter than n_entries")
+    _check("latent_gather", lib().tib_latent_gather(
+        _ptr(keys), c_int64(keys.stride(0)), c_int(keys.shape[2]), c_int(keys.shape[0]), _ptr(block_table), c_int(block_table.stride(0)),
+        _ptr(q_start), _ptr(kv_start), _ptr(slots), c_int(n_entries), c_int(max_kv_len), _ptr(latent), _ptr(rotated), c_int(rank),
+        c_int(rot), _ptr(error_word), _stream()))
+
+
+def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
+                   kv_start: torch.Tensor, n_entries: int, max_q_len: int, heads: int, dim: int, value_dim: int, scale: float,
+                   gate: torch.Tensor | None = None, gate_per_head: bool = False, sink: torch.Tensor | None = None,
+                   error_word: torch.Tensor | None = None) -> torch.Tensor:
+    """Causal attention of rotated queries [tokens, heads * (dim + rot)] over the rows :func:`latent_gather` laid out: ``kv`` [rows,
+    heads * (dim + value_dim)] holds all heads' keys and then all heads' values, ``rotated`` the key part the heads share.
+    ``out`` [tokens, heads, value_dim] is multiplied by sigmoid(gate) when one is given, element by element or head by head."""
+    rot = rotated.shape[1]
+    _rows_of(q, "q", heads * (dim + rot)), _need(kv, "kv", torch.bfloat16), _need(rotated, "rotated", torch.bfloat16), _need(out, "out", torch.bfloat16)
+    for name, t in (("q_start", q_start), ("kv_start", kv_start)):
+        _need(t, name, torch.int32)
+    n = q.shape[0]
+    if q.dtype != torch.bfloat16 or out.numel() != n * heads * value_dim or kv.shape != (rotated.shape[0], heads * (dim + value_dim)):
+        raise KernelError("latent_prefill: shapes or types do not fit")
+    if gate is not None:
+        _rows_of(gate, "gate", heads if gate_per_head else heads * value_dim)
+        if gate.dtype != torch.bfloat16 or gate.shape[0] != n:
+            raise KernelError("latent_prefill: the gate's rows do not fit")
+    if sink is not None:
+        _need(sink, "sink", torch.float32)
+        if sink.numel() != heads:
+            raise KernelError("latent_prefill: sink holds one number per head")
+    _check("latent_prefill", lib().tib_latent_prefill(
+        _ptr(q), c_int64(q.stride(0)), _ptr(kv), _ptr(rotated), c_int(kv.shape[0]), _ptr(q_start), _ptr(kv_start), c_int(n_entries),
+        c_int(max_q_len), c_int(n), c_int(heads), c_int(dim), c_int(value_dim), c_int(rot), c_float(scale), _ptr(sink), _ptr(gate),
+        c_int64(gate.stride(0) if gate is not None else 0), c_int(int(gate_per_head)), _ptr(out), _ptr(error_word), _stream()))
     return out
 
 

@@ -12,7 +12,8 @@ Only c and r are cached (one row of kv_rank + rot_dim elements per token: a cach
 values).  The queries are folded through W_uk (a_j = W_uk_j^T q_j, one batched product), attention runs over the
 latent rows with their first kv_rank elements as values, and W_uv is applied to the result (another batched
 product): the same arithmetic regrouped, in which no per-head key or value is ever made.  Scores, softmax
-weights, their sums and the folded queries are fp32.  Rotary pairs are (2i, 2i + 1) (``pairing="interleaved"``) or
+weights, their sums and the folded queries are fp32.  In bfloat16, prompt portions of some length run the other way round:
+the step's per-head keys and values are made from the cached rows by one product and used once (:meth:`_unfolded_rows`).  Rotary pairs are (2i, 2i + 1) (``pairing="interleaved"``) or
 (i, i + rot_dims / 2) (``pairing="half"``) over the first ``rot_dims`` elements of the rotated part, angle = position *
 rot_base^(-2i / rot_dims).
 """
@@ -54,6 +55,7 @@ class LatentAttention(Mixer):
         self.in_weight: LinearWeight | None = None
         self.uq_weight: LinearWeight | None = None
         self.o_weight: LinearWeight | None = None
+        self.unfold: LinearWeight | None = None
 
     def weight_specs(self) -> list[WeightSpec]:
         n, h, w = self.names, self.heads, self.hidden_size
@@ -96,8 +98,45 @@ class LatentAttention(Mixer):
         else:
             self.uk_weight = uk.contiguous()
 
+        # (all heads' W_uk, then all heads' W_uv: the step's keys and values for prompts)
+        self.unfold = None
+        if uk.dtype == torch.bfloat16 and uk.is_cuda and self.scale > 0 \
+                and ops.latent_prefill_supports(self.dim, self.value_dim, self.kv_rank, self.rot_dim):
+            self.unfold = LinearWeight(torch.cat([weights[n["uk"]], weights[n["uv"]]], dim=0))
+
     def cache_spec(self) -> CacheSpec:
         return CacheSpec(1, self.kv_rank + self.rot_dim, None, value_dim=0)
+
+    # The unfolded form multiplies 2 (dim + value_dim) rank numbers a head and key once, and saves some two thirds of the folded
+    # kernel's products on every (query, key) pair, which run at a tenth of the library's rate: it wins from about six
+    # queries a key on average, and is taken from sixteen (the layer on two prompts of 1,667 and 833 tokens, 16 heads: 1,226 us
+    # folded, 165 unfolded; error against 64 bits 0.0048 and 0.0045).
+    UNFOLD_QUERIES = 16
+    UNFOLD_BYTES = 1 << 30      # the most that a step's keys and values may take
+
+    def _unfolded_rows(self, batch) -> int:
+        """Rows of keys and values to make for this step, 0 where the folded form is to run."""
+        if self.unfold is None or batch.n_multi == 0 or len(batch.entries) != batch.n_entries:
+            return 0
+        keys = sum(e.kv_start + e.q_len for e in batch.entries)
+        pairs = sum(e.q_len * (e.kv_start + e.q_len) for e in batch.entries)
+        rows = sum(-(-(e.kv_start + e.q_len) // ops.LATENT_TILE) * ops.LATENT_TILE for e in batch.entries)
+        size = 2 * rows * (self.heads * (self.dim + self.value_dim) + self.kv_rank + self.rot_dim)
+        return rows if pairs >= self.UNFOLD_QUERIES * keys and size <= self.UNFOLD_BYTES else 0
+
+    def _forward_unfolded(self, rows: int, q: torch.Tensor, dkv: torch.Tensor, gate: torch.Tensor | None, ctx: LayerContext) -> torch.Tensor:
+        kv, batch, n, h = ctx.kv, ctx.batch, q.shape[0], self.heads
+        ops.latent_append(dkv, q, None, kv.keys if kv.writes else None, batch.positions, batch.token_slot, kv.block_table,
+                          self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, self.kv_rank, self.rot_dim, ctx.error_word,
+                          half_pairs=self.half_pairs)
+        latent = torch.empty((rows, self.kv_rank), dtype=q.dtype, device=q.device)
+        rotated = torch.empty((rows, self.rot_dim), dtype=q.dtype, device=q.device)
+        ops.latent_gather(kv.keys, kv.block_table, batch.q_start, batch.kv_start, batch.slots, batch.n_entries, batch.max_kv_len, latent,
+                          rotated, ctx.error_word)
+        out = torch.empty((n, h, self.value_dim), dtype=q.dtype, device=q.device)
+        ops.latent_prefill(q, linear(latent, self.unfold), rotated, out, batch.q_start, batch.kv_start, batch.n_entries, batch.max_q_len,
+                           h, self.dim, self.value_dim, self.scale, gate, self.gate_per_head, self.sink, ctx.error_word)
+        return linear(out.view(n, h * self.value_dim), self.o_weight)
 
     def forward(self, x: torch.Tensor, ctx: LayerContext) -> torch.Tensor:
         kv, batch = ctx.kv, ctx.batch
@@ -111,6 +150,13 @@ class LatentAttention(Mixer):
         if self.q_rank:
             latent_q = ops.rmsnorm(q, self.q_norm_weight, self.eps, torch.empty((n, self.q_rank), dtype=x.dtype, device=x.device))
             q = linear(latent_q, self.uq_weight)
+        gates = (h if self.gate_per_head else h * self.value_dim) if self.gate else 0
+        gate = proj[:, q_width + width:q_width + width + gates] if self.gate else None
+        rows = self._unfolded_rows(batch) if x.dtype == torch.bfloat16 else 0
+        # (the kernels copy rows from 16-byte boundaries; a projection of an odd width leaves the gate's rows off them)
+        if rows and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and kv.keys.stride(0) % 8 == 0 and kv.keys.data_ptr() % 16 == 0 \
+                and (gate is None or self.gate_per_head or gate.data_ptr() % 16 == 0):
+            return self._forward_unfolded(rows, q, dkv, gate, ctx)
         folded = torch.empty((n, h, width), dtype=torch.float32, device=x.device)
         ops.latent_append(dkv, q, folded, kv.keys if kv.writes else None, batch.positions, batch.token_slot, kv.block_table,
                           self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, c, r, ctx.error_word,
@@ -134,9 +180,7 @@ class LatentAttention(Mixer):
             ops.library_gemm_batched(rows, self.uv_weight, heads_out, w_kn=False)
         heads_out = heads_out.view(n, h * self.value_dim)
         if self.gate:
-            gates = h if self.gate_per_head else h * self.value_dim
-            ops.sigmoid_gate(heads_out, proj[:, q_width + width:q_width + width + gates], heads_out,
-                             group=self.value_dim if self.gate_per_head else 1)
+            ops.sigmoid_gate(heads_out, gate, heads_out, group=self.value_dim if self.gate_per_head else 1)
         return linear(heads_out, self.o_weight)
 
 
