@@ -981,3 +981,35 @@ def test_expert_product_on_uneven_experts(tokens, experts, top, k, n, act, by_pa
     # exact bf16 products, fp32 sums of k of them (2^-23 of the largest partial sum each), then one rounding to the output type
     bound = (2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0) * v.abs() + 4 * k * 2.0 ** -23
     assert ((as_ref(y) - v).abs() <= bound).all()
+
+
+# ------------------------------------------------------------- the state-space scan in chunks, convolutions and gated norms by eight
+@pytest.mark.parametrize("lens, heads, head_dim, state, groups, shift", [
+    ([65, 1, 128], 4, 64, 128, 2, 0.0), ([129, 64, 256], 2, 128, 64, 1, 0.0), ([300], 4, 32, 64, 4, 0.0), ([127, 130], 2, 32, 128, 1, -6.0),
+    ([200, 70], 2, 64, 128, 1, 8.0)])      # (steps near zero: nothing decays; steps of eight: everything does)
+def test_scan_in_chunks_agrees_with_the_recurrence(lens, heads, head_dim, state, groups, shift):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    n, inner, entries = sum(lens), heads * head_dim, len(lens)
+    xbc, dt = rnd(n, inner + 2 * groups * state, dtype=torch.bfloat16), rnd(n, heads, dtype=torch.bfloat16, seed=1)
+    bias, a_log, skip = rnd(heads, seed=2) + shift, 0.5 * rnd(heads, seed=3), rnd(heads, seed=4)
+    held, slots = rnd(entries + 1, heads * state * head_dim + 8, seed=5), [entries - i for i in range(entries)]
+    starts = torch.tensor([sum(lens[:i]) for i in range(entries + 1)], dtype=torch.int32)
+    y, got = torch.empty(n, inner, device="cuda"), dev(held.clone())
+    ops.ssd_scan(dev(xbc), dev(dt), 0, dev(bias), dev(a_log), dev(skip), got, dev(starts), dev(torch.tensor(slots, dtype=torch.int32)), y, entries,
+                 heads=heads, groups=groups, state_dim=state, head_dim=head_dim, max_q_len=max(lens))
+    x = xbc[:, :inner].double().view(n, heads, head_dim)
+    b, c = (xbc[:, inner + i * groups * state:inner + (i + 1) * groups * state].double().view(n, groups, state).repeat_interleave(heads // groups, 1)
+            for i in range(2))
+    step = torch.nn.functional.softplus(dt.double() + bias.double(), threshold=1e9)
+    decay = (-a_log.double().exp() * step).exp()
+    want, want_state = torch.empty(n, heads, head_dim, dtype=torch.float64), held.double().clone()
+    for e, length in enumerate(lens):
+        s = want_state[slots[e], :heads * state * head_dim].view(heads, state, head_dim).clone()
+        for t in range(int(starts[e]), int(starts[e]) + length):
+            s = decay[t][:, None, None] * s + (step[t][:, None] * b[t])[:, :, None] * x[t][:, None, :]
+            want[t] = torch.einsum("hsp,hs->hp", s, c[t]) + skip.double()[:, None] * x[t]
+        want_state[slots[e], :heads * state * head_dim] = s.reshape(-1)
+    # everything 32-bit enters its products with 24 bits: sums of up to `state` + 128 such terms, 2^-23 of the largest value each
+    for out, ref in ((y, want.reshape(n, inner)), (got, want_state)):
+        assert (as_ref(out) - ref).abs().max() <= 32 * 2.0 ** -23 * ref.abs().max()

@@ -12,19 +12,15 @@
 // accumulates in fp32 and leaves its rows in the activation type.  Every kernel takes the step's ragged batch
 // through its device arrays (q_start, slots), so prompt portions and single tokens run in one launch and a decode
 // step can be captured.
-#include "common.cuh"
+#include "state_space.cuh"
 
 namespace tib {
 
-__device__ __forceinline__ float ss_load(const void* p, int dtype, size_t i) {
-  return dtype == TIB_F32 ? reinterpret_cast<const float*>(p)[i] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
-}
 __device__ __forceinline__ void ss_store(void* p, int dtype, size_t i, float v) {
   if (dtype == TIB_F32) reinterpret_cast<float*>(p)[i] = v;
   else reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
 }
 __device__ __forceinline__ float ss_silu(float v) { return v / (1.f + expf(-v)); }
-__device__ __forceinline__ float ss_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // ------------------------------------------------------------------------------------------- short convolution
 constexpr int kConvMaxTaps = 8;
@@ -117,7 +113,8 @@ __global__ void __launch_bounds__(kConvChannels) short_conv_kernel(ConvArgs a) {
 // kScanRun tokens that are walked side by side: first every run from a zero state (its own sum L_r and the product of its
 // decays A_r), then one thread per state element folds S_(r+1) = A_r S_r + L_r over the request's runs, leaving each run's
 // starting state in the place of its sum and the last state in the slot, then every run again from its starting state,
-// now with the outputs.  Cutting changes only the order of fp32 sums.
+// now with the outputs.  Cutting changes only the order of fp32 sums.  (bf16 rows of the usual head and state sizes take
+// ssd_chunks.cu there instead.)
 //
 // Tokens are staged in shared memory a chunk at a time, in two stages: while the block walks token t of one chunk, its
 // threads fetch row t of the next chunk into registers (as raw bits, so that nothing waits on the loads) and leave it in
@@ -127,17 +124,6 @@ constexpr int kScanGroups = 16;        // column groups of a block
 constexpr int kScanRun = 64;           // tokens of a run
 constexpr int kScanThreads = 128;
 enum { kScanWhole = 0, kScanLocal = 1, kScanFrom = 2 };
-
-struct ScanArgs {
-  const void* xbc; int xbc_dtype; int64_t ld_xbc;        // rows [x: heads * P | B: groups * N | C: groups * N]
-  const void* dt; int dt_dtype; int64_t ld_dt; int dt_col;   // raw step sizes: column dt_col + h of a row
-  const float* dt_bias; const float* a_log; const float* d_skip;   // [heads] each
-  float* state; int64_t state_stride;                      // per slot: S [heads][N][P] at offset 0
-  const int* q_start; const int* slots;
-  float* y;                                                // [tokens, heads * P] fp32
-  float* run_state; float* run_decay;                      // [runs][heads * N * P], [runs][heads]
-  int heads, groups, N, P;
-};
 
 // The first run of an entry in the run arrays: entries' runs never overlap, since an entry of len tokens has at most
 // len / kScanRun + 1 runs and the next entry starts len rows and one entry later.
@@ -464,6 +450,7 @@ TIB_API int tib_ssd_scan(const void* xbc, int xbc_dtype, int64_t ld_xbc, const v
   a.dt_bias = dt_bias; a.a_log = a_log; a.d_skip = d_skip; a.state = state; a.state_stride = state_stride;
   a.q_start = q_start; a.slots = slots; a.y = y; a.run_state = run_state; a.run_decay = run_decay;
   a.heads = heads; a.groups = groups; a.N = N; a.P = P;
+  if (runs && ssd_chunks_takes(a)) return ssd_chunks(a, n_entries, max_q_len, stream);
   const int npt = ceil_div(N, kScanLanesN);
   const bool wide = P > kScanGroups;        // four columns a thread where a head has more columns than a block has groups
 #define TIB_SCAN_CASE(NPT) \
