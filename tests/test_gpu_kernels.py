@@ -1013,3 +1013,22 @@ def test_scan_in_chunks_agrees_with_the_recurrence(lens, heads, head_dim, state,
     # everything 32-bit enters its products with 24 bits: sums of up to `state` + 128 such terms, 2^-23 of the largest value each
     for out, ref in ((y, want.reshape(n, inner)), (got, want_state)):
         assert (as_ref(out) - ref).abs().max() <= 32 * 2.0 ** -23 * ref.abs().max()
+
+
+@pytest.mark.parametrize("lens, channels, taps", [([1, 2, 3], 8, 4), ([16, 17, 1], 1032, 3), ([50, 2], 520, 2), ([40], 16, 4)])
+def test_short_convolution_by_eight_channels_has_the_plain_kernels_bits(lens, channels, taps):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    n, entries = sum(lens), len(lens)
+    rows = rnd(n, channels + 24, dtype=torch.bfloat16)
+    weight, bias, state = rnd(channels, taps, seed=1), rnd(channels, seed=2), rnd(entries, (taps - 1) * channels, seed=3)
+    starts = torch.tensor([sum(lens[:i]) for i in range(entries + 1)], dtype=torch.int32)
+    results = []
+    for shift in (8, 9):      # (columns off their 16-byte boundaries take the plain kernel)
+        wide = torch.zeros(n, channels + 24, dtype=torch.bfloat16)
+        wide[:, shift:shift + channels] = rows[:, 8:8 + channels]
+        out, held = torch.empty(n, channels, dtype=torch.bfloat16, device="cuda"), dev(state.clone())
+        ops.short_conv(dev(wide), shift, dev(weight), dev(bias), held, 0, dev(starts), dev(torch.arange(entries, dtype=torch.int32)), out,
+                       entries, max(lens), silu=True)
+        results.append((out, held))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])

@@ -106,6 +106,106 @@ __global__ void __launch_bounds__(kConvChannels) short_conv_kernel(ConvArgs a) {
   }
 }
 
+// The same for bf16 rows on 16-byte boundaries: a thread takes eight neighbouring channels and walks 16 tokens (the taps - 1 before
+// them read again), so a warp reads 512 bytes of a row at a time.  Same sums in the same order.  2,048 tokens x 4,352
+// channels: 58 us with a channel a thread, 34 here (cold); what bounds it is the taps' arithmetic with the silu, and memory.
+constexpr int kConvVecSegment = 16;
+
+template <int TAPS>
+__global__ void __launch_bounds__(128) short_conv_vec_kernel(ConvArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  constexpr int CARRIED = TAPS - 1;
+  const int entry = blockIdx.z, seg = blockIdx.y;
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
+  const int row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
+  const int t0 = seg * kConvVecSegment;
+  if (c >= a.channels || t0 >= len) return;
+  float* st = a.state + (size_t)a.slots[entry] * a.state_stride + a.state_off;
+  const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(a.in) + (size_t)row0 * a.ld + a.col + c;
+  auto load = [&](int r, float (&v)[8]) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(in + (size_t)r * a.ld);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+      v[2 * i] = f.x;
+      v[2 * i + 1] = f.y;
+    }
+  };
+  float prev[CARRIED][8];      // the inputs before the one at hand, oldest first
+  if (seg == 0) {
+    float old[CARRIED][8];
+#pragma unroll
+    for (int k = 0; k < CARRIED; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) prev[k][j] = old[k][j] = st[(size_t)k * a.channels + c + j];
+#pragma unroll
+    for (int k = 0; k < CARRIED; ++k) {      // what the next step finds: the last inputs
+      const int r = len - CARRIED + k;
+      float v[8];
+      if (r >= 0) load(r, v);
+      else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[j] = 0.f;
+#pragma unroll
+          for (int u = 0; u < CARRIED; ++u) if (u == k + len) v[j] = old[u][j];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) st[(size_t)k * a.channels + c + j] = v[j];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < CARRIED; ++k) load(t0 - CARRIED + k, prev[k]);      // (a segment is longer than what it looks back)
+  }
+  float w[TAPS][8], b[8];
+  {
+    const float4* wp = reinterpret_cast<const float4*>(a.weight + (size_t)c * TAPS);      // (8 TAPS numbers in a row)
+    float raw[8 * TAPS];
+#pragma unroll
+    for (int i = 0; i < 2 * TAPS; ++i) reinterpret_cast<float4*>(raw)[i] = wp[i];
+    float4 bias[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    if (a.bias) { bias[0] = reinterpret_cast<const float4*>(a.bias + c)[0]; bias[1] = reinterpret_cast<const float4*>(a.bias + c)[1]; }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      b[j] = reinterpret_cast<const float*>(bias)[j];
+#pragma unroll
+      for (int k = 0; k < TAPS; ++k) w[k][j] = raw[j * TAPS + k];
+    }
+  }
+  const int t1 = min(len, t0 + kConvVecSegment);
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)row0 * a.channels + c;
+  constexpr int AHEAD = 4;
+  for (int t = t0; t < t1; t += AHEAD) {
+    float x[AHEAD][8];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) load(min(t + i, t1 - 1), x[i]);
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      if (t + i >= t1) break;
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float acc = b[j];
+#pragma unroll
+        for (int k = 0; k < CARRIED; ++k) acc = fmaf(w[k][j], prev[k][j], acc);
+        acc = fmaf(w[CARRIED][j], x[i][j], acc);
+#pragma unroll
+        for (int k = 0; k + 1 < CARRIED; ++k) prev[k][j] = prev[k + 1][j];
+        prev[CARRIED - 1][j] = x[i][j];
+        o[j] = a.silu ? ss_silu(acc) : acc;
+      }
+      uint4 packed;
+      __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p2[j] = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
+      *reinterpret_cast<uint4*>(out + (size_t)(t + i) * a.channels) = packed;
+    }
+  }
+}
+
 // --------------------------------------------------------------------------------------------------- the scan
 // A block of 128 threads owns 16 * CP columns of one head's state: 8 lanes share a group of CP columns along N (lane l holds
 // the pairs n = 2 l, 2 l + 1, then 16 further on and so on, two values to a 64-bit register for fma.rn.f32x2), so a token's B and C are read once from shared memory for CP columns.  A step whose longest portion
@@ -405,6 +505,15 @@ TIB_API int tib_short_conv(const void* in, int in_dtype, int64_t ld, int col, co
   a.in = in; a.in_dtype = in_dtype; a.ld = ld; a.col = col; a.weight = weight; a.bias = bias; a.state = state;
   a.state_stride = state_stride; a.state_off = state_off; a.q_start = q_start; a.slots = slots; a.out = out;
   a.out_dtype = out_dtype; a.channels = channels; a.taps = taps; a.silu = silu;
+  const int vec_segments = ceil_div(max_q_len, kConvVecSegment);
+  if (in_dtype == TIB_BF16 && out_dtype == TIB_BF16 && taps >= 2 && taps <= 4 && channels % 8 == 0 && ld % 8 == 0 && col % 8 == 0 &&
+      (((uintptr_t)in | (uintptr_t)out | (uintptr_t)weight | (uintptr_t)bias) & 15) == 0 && vec_segments <= 65535) {
+    const dim3 grid(ceil_div(channels, 1024), vec_segments, n_entries);
+    if (taps == 4) TIB_LAUNCH_DEPENDENT(short_conv_vec_kernel<4>, grid, 128, 0, stream, a);
+    else if (taps == 3) TIB_LAUNCH_DEPENDENT(short_conv_vec_kernel<3>, grid, 128, 0, stream, a);
+    else TIB_LAUNCH_DEPENDENT(short_conv_vec_kernel<2>, grid, 128, 0, stream, a);
+    return TIB_OK;
+  }
   const int segments = ceil_div(max_q_len, kConvSegment);
   if (segments > 65535) return TIB_E_SIZE;
   TIB_LAUNCH_DEPENDENT(short_conv_kernel, dim3(ceil_div(channels, kConvChannels), segments, n_entries), kConvChannels, 0, stream, a);
