@@ -1032,3 +1032,28 @@ def test_short_convolution_by_eight_channels_has_the_plain_kernels_bits(lens, ch
                        entries, max(lens), silu=True)
         results.append((out, held))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("rows, width, parts", [(1, 8, 1), (3, 264, 1), (5, 2056, 1), (2, 4104, 1), (3, 8192, 4), (2, 8200, 1)])
+@pytest.mark.parametrize("mode", ["gate last", "gate first", "norm and gate", "gate", "head gate"])
+def test_gated_rows_by_eight_columns(rows, width, parts, mode):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    y, z, weight = rnd(rows, width), rnd(rows, width + 16, dtype=torch.bfloat16, seed=1), rnd(width, seed=2)
+    out = torch.empty(rows, width, dtype=torch.bfloat16, device="cuda")
+    v, gate = y.double(), z[:, 8:8 + width].double()
+    if mode in ("gate last", "gate first"):
+        ops.gated_group_norm(dev(y), dev(z), 8, dev(weight), 1e-6, out, parts, gate_last=mode == "gate last")
+        v = v * gate * torch.sigmoid(gate) if mode == "gate first" else v
+        v = v.view(rows, parts, -1)
+        v = (v / (v.pow(2).mean(-1, keepdim=True) + 1e-6).sqrt()).reshape(rows, width) * weight.double()
+        want = v * torch.sigmoid(gate) if mode == "gate last" else v
+    elif mode == "norm and gate":
+        ops.sigmoid_gate(dev(y), dev(z)[:, 8:8 + width], out, dev(weight), 1e-6)
+        want = v / (v.pow(2).mean(-1, keepdim=True) + 1e-6).sqrt() * weight.double() * torch.sigmoid(gate)
+    else:
+        group = 8 if mode == "head gate" else 1
+        ops.sigmoid_gate(dev(y).bfloat16(), dev(z)[:, 8:8 + width // group], out, group=group)
+        want = y.bfloat16().double() * torch.sigmoid(z[:, 8:8 + width // group].double()).repeat_interleave(group, 1)
+    # fp32 arithmetic (a few roundings of 2^-24), then one rounding to the eight significant bits of bfloat16 (2^-8 at most)
+    assert ((as_ref(out) - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 1e-6 * want.abs().max()).all()

@@ -5,7 +5,7 @@
 //
 // In every kernel x / y / g may be float or bf16 in memory (a dtype code each) and may be slices of a wider
 // row (a row stride each), so the output of one fused projection can be taken apart without a copy.
-#include "common.cuh"
+#include "row_gate.cuh"
 
 namespace tib {
 
@@ -258,6 +258,11 @@ TIB_API int tib_sigmoid_gate(const void* x, int x_dtype, int64_t ldx, const void
   if (rows == 0 || width == 0) return TIB_OK;
   if (!x || !g || !out || rows < 0 || width < 0 || group < 1) return TIB_E_ARG;
   if (!known(x_dtype) || !known(g_dtype) || !known(out_dtype)) return TIB_E_DTYPE;
+  RowGateArgs r;
+  r.x = x; r.x_dtype = x_dtype; r.ldx = ldx; r.z = g; r.z_dtype = g_dtype; r.ldz = ldg; r.weight = weight; r.eps = eps; r.out = out;
+  r.out_dtype = out_dtype; r.rows = rows; r.width = r.part = width; r.group = group;
+  const int mode = weight ? ROW_GATE_LAST : ROW_GATE_ONLY;
+  if (row_gate_takes(r, mode)) return row_gate(r, mode, stream);
   TIB_LAUNCH_DEPENDENT(sigmoid_gate_kernel, rows, row_threads(width), 0, stream, x, x_dtype, ldx, g, g_dtype, ldg, weight, eps,
                        out, out_dtype, width, group);
   return TIB_OK;

@@ -13,6 +13,7 @@
 // through its device arrays (q_start, slots), so prompt portions and single tokens run in one launch and a decode
 // step can be captured.
 #include "state_space.cuh"
+#include "row_gate.cuh"
 
 namespace tib {
 
@@ -582,6 +583,12 @@ TIB_API int tib_gated_group_norm(const float* y, const void* z, int z_dtype, int
   if (parts < 1 || width % parts || parts > 65535) return TIB_E_SIZE;
   if (!ss_known(z_dtype) || !ss_known(out_dtype)) return TIB_E_DTYPE;
   const int part = width / parts;
+  const int64_t zsize = z_dtype == TIB_F32 ? 4 : 2;
+  RowGateArgs r;
+  r.x = y; r.x_dtype = TIB_F32; r.ldx = width; r.z = (const char*)z + z_col * zsize; r.z_dtype = z_dtype; r.ldz = ldz; r.weight = weight;
+  r.eps = eps; r.out = out; r.out_dtype = out_dtype; r.rows = rows; r.width = width; r.part = part; r.group = 1;
+  const int mode = gate_last ? ROW_GATE_LAST : ROW_GATE_FIRST;
+  if (row_gate_takes(r, mode)) return row_gate(r, mode, stream);
   const int threads = part >= 1024 ? 256 : part >= 256 ? 128 : 64;
   if (gate_last)
     TIB_LAUNCH_DEPENDENT(gated_group_norm_kernel<true>, dim3(rows, parts), threads, 0, stream, y, z, z_dtype, ldz, z_col, weight,
