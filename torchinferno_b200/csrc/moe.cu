@@ -28,9 +28,9 @@ namespace tib {
 // token: the order of every sum is fixed by k and the alignment alone, so a token's logits do not depend on what else is
 // in the step.  (The general fp32 product gives a product
 // this narrow to a single block.)
-// A block takes kRouterTokens tokens, so that a row of w read from the L2 serves several of them.  With 16-byte aligned
+// A block takes TOK tokens, so that a row of w read from the L2 serves several of them.  With 16-byte aligned
 // rows (VEC) a lane takes eight consecutive k at a time: 16 bytes of a bf16 token row, 32 bytes of w.
-constexpr int kRouterTokens = 4;
+constexpr int kRouterTokens = 4, kRouterMany = 8;      // tokens of a block: of a small step or odd rows, of a large one
 
 __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
   const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
@@ -43,45 +43,58 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
 }
 
-template <typename TX, bool VEC>
+// In a large step a warp works R rows of w at a time (rows e, e + all the warps of the token group, ...), whose pieces stay in
+// registers while the group's tokens pass by, so a token's elements are widened once for R rows: 2,048 tokens, 33 rows of 2,048
+// 36 us with one row and four tokens, 28 with five and eight.  With few tokens one row and four tokens stay ahead (8 tokens:
+// 15 against 21), since there the number of warps counts.
+template <typename TX, bool VEC, int TOK, int R>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ out, int64_t ldo, int tokens, int rows, int K) {
   pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int t0 = blockIdx.x * kRouterTokens;
-  const int nt = min(kRouterTokens, tokens - t0);
+  const int t0 = blockIdx.x * TOK;
+  const int nt = min(TOK, tokens - t0);
   const int K8 = VEC ? (K / 8) * 8 : 0;
-  for (int e = warp + blockIdx.y * nwarps; e < rows; e += nwarps * gridDim.y) {
-    const float* wr = w + (size_t)e * K;
-    float acc[kRouterTokens];
+  const int stride = nwarps * gridDim.y;
+  for (int e0 = warp + blockIdx.y * nwarps; e0 < rows; e0 += stride * R) {
+    float acc[R][TOK];
 #pragma unroll
-    for (int i = 0; i < kRouterTokens; ++i) acc[i] = 0.f;
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int i = 0; i < TOK; ++i) acc[r][i] = 0.f;
     if (VEC) {
       for (int k = lane * 8; k < K8; k += 256) {
-        float wv[8];
-        load8(wr + k, wv);
+        float wv[R][8];
 #pragma unroll
-        for (int i = 0; i < kRouterTokens; ++i) {
-          if (i >= nt) continue;
+        for (int r = 0; r < R; ++r) load8(w + (size_t)min(e0 + r * stride, rows - 1) * K + k, wv[r]);      // (a row too many is not stored)
+#pragma unroll
+        for (int i = 0; i < TOK; ++i) {
           float xv[8];
-          load8(x + (size_t)(t0 + i) * ldx + k, xv);
+          load8(x + (size_t)(t0 + min(i, nt - 1)) * ldx + k, xv);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i] = fmaf(xv[j], wv[j], acc[i]);
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[r][i] = fmaf(xv[j], wv[r][j], acc[r][i]);
         }
       }
     }
-    for (int k = K8 + lane; k < K; k += 32) {
-      const float wv = wr[k];
 #pragma unroll
-      for (int i = 0; i < kRouterTokens; ++i)
-        if (i < nt) acc[i] = fmaf(to_f32(x[(size_t)(t0 + i) * ldx + k]), wv, acc[i]);
-    }
+    for (int r = 0; r < R; ++r) {
+      const int e = e0 + r * stride;
+      if (e >= rows) break;
+      for (int k = K8 + lane; k < K; k += 32) {
+        const float wv = w[(size_t)e * K + k];
 #pragma unroll
-    for (int i = 0; i < kRouterTokens; ++i) {
-      const float v = warp_sum(acc[i]);
-      if (lane == 0 && i < nt) out[(size_t)(t0 + i) * ldo + e] = bias ? v + bias[e] : v;
+        for (int i = 0; i < TOK; ++i)
+          if (i < nt) acc[r][i] = fmaf(to_f32(x[(size_t)(t0 + i) * ldx + k]), wv, acc[r][i]);
+      }
+#pragma unroll
+      for (int i = 0; i < TOK; ++i) {
+        const float v = warp_sum(acc[r][i]);
+        if (lane == 0 && i < nt) out[(size_t)(t0 + i) * ldo + e] = bias ? v + bias[e] : v;
+      }
     }
   }
 }
@@ -319,6 +332,63 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
   }
 }
 
+// The same with rows on 16-byte boundaries: a thread takes eight neighbouring columns, and all choices' rows are asked for before the
+// first is used (four at a time).  Same sums in the same order.  What bounds it is reading top x 4 bytes a column: 2,048 tokens x
+// 2,048 columns with four choices and a shared expert 19 us cold, 46 element by element.
+template <typename TS, typename TO>
+__global__ void __launch_bounds__(256)
+moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights,
+                       int top, const TS* __restrict__ shared, const float* __restrict__ gate, int64_t ld_gate,
+                       TO* __restrict__ out, int width, const int* __restrict__ ids, int identity_from,
+                       const TO* __restrict__ x, int64_t ldx) {
+  pdl_wait();
+  pdl_trigger();
+  const size_t t = blockIdx.x;
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (c >= width) return;
+  float own[8], v[8];
+  if (shared) load8(shared + t * width + c, own);
+  const float g = (shared && gate) ? 1.f / (1.f + expf(-gate[t * ld_gate])) : 1.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = 0.f;
+  for (int k0 = 0; k0 < top; k0 += 4) {
+    float row[4][8], f[4];
+    bool add[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      add[u] = false;
+      if (k0 + u >= top) continue;
+      const int s = place[t * top + k0 + u];
+      f[u] = weights ? weights[t * top + k0 + u] : 1.f;
+      if (s >= 0) { load8(y + (size_t)s * width + c, row[u]); add[u] = true; }
+      else if (ids && ids[t * top + k0 + u] >= identity_from) { load8(x + t * ldx + c, row[u]); add[u] = true; }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (add[u]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = fmaf(f[u], row[u][j], v[j]);
+      }
+  }
+  if (shared) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = fmaf(g, own[j], v[j]);
+  }
+  if constexpr (sizeof(TO) == 2) {
+    uint4 packed;
+    uint32_t* p = reinterpret_cast<uint32_t*>(&packed);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+      p[j] = *reinterpret_cast<const uint32_t*>(&pair);
+    }
+    *reinterpret_cast<uint4*>(out + t * width + c) = packed;
+  } else {
+    reinterpret_cast<float4*>(out + t * width + c)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(out + t * width + c)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  }
+}
+
 }  // namespace tib
 
 using namespace tib;
@@ -330,17 +400,28 @@ TIB_API int tib_router_logits(const void* x, int x_dtype, int64_t ldx, const flo
   if (tokens == 0 || rows == 0) return TIB_OK;
   if (!x || !w || !out || tokens < 0 || rows < 0 || K < 1) return TIB_E_ARG;
   if (tokens > 0x7fffffff / 2) return TIB_E_SIZE;
-  int slices = 1;      // few tokens: the rows of w are spread over several blocks a token
-  const int groups = ceil_div(tokens, kRouterTokens);
-  while (groups * slices < 2 * 148 && slices * 8 < rows) slices *= 2;
-  dim3 grid(groups, slices);
   const int64_t xbytes = x_dtype == TIB_F32 ? 4 : 2;
   const bool vec = K % 4 == 0 && (ldx * xbytes) % 16 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-#define TIB_ROUTER_GO(TX, VEC) \
-  TIB_LAUNCH_DEPENDENT((router_logits_kernel<TX, VEC>), grid, 256, 0, stream, (const TX*)x, ldx, w, bias, out, ldo, tokens, rows, K)
+  const bool many = vec && tokens >= kRouterMany * 148;      // (a block an SM at least)
+  int slices = 1;      // few tokens: the rows of w are spread over several blocks a token
+  const int groups = ceil_div(tokens, many ? kRouterMany : kRouterTokens);
+  while (groups * slices < 2 * 148 && slices * 8 < rows && !many) slices *= 2;
+  dim3 grid(groups, slices);
+  // rows a warp works at a time in a large step: as few passes over the rows as five at a time need, shared out evenly
+  const int passes = ceil_div(rows, 8 * 5), together = ceil_div(rows, 8 * passes);
+#define TIB_ROUTER_R(TX, VEC, TOK, R) \
+  TIB_LAUNCH_DEPENDENT((router_logits_kernel<TX, VEC, TOK, R>), grid, 256, 0, stream, (const TX*)x, ldx, w, bias, out, ldo, tokens, rows, K)
+#define TIB_ROUTER_GO(TX, VEC)                                                    \
+  do {                                                                            \
+    if (!many) TIB_ROUTER_R(TX, VEC, kRouterTokens, 1);                           \
+    else if (together <= 1) TIB_ROUTER_R(TX, true, kRouterMany, 1);               \
+    else if (together <= 3) TIB_ROUTER_R(TX, true, kRouterMany, 3);               \
+    else TIB_ROUTER_R(TX, true, kRouterMany, 5);                                  \
+  } while (0)
   if (x_dtype == TIB_F32) { if (vec) TIB_ROUTER_GO(float, true); else TIB_ROUTER_GO(float, false); }
   else if (x_dtype == TIB_BF16) { if (vec) TIB_ROUTER_GO(__nv_bfloat16, true); else TIB_ROUTER_GO(__nv_bfloat16, false); }
 #undef TIB_ROUTER_GO
+#undef TIB_ROUTER_R
   else
     return TIB_E_DTYPE;
   return TIB_OK;
@@ -409,9 +490,20 @@ TIB_API int tib_moe_combine(const float* y, const int* place, const float* weigh
   const int threads = width >= 1024 ? 256 : 128;
   // (few tokens: a row's columns are spread over several blocks)
   const dim3 grid(tokens, tokens < 2 * 148 ? ceil_div(width, threads) : 1);
+  const int64_t xsize = out_dtype == TIB_F32 ? 4 : 2;
+  const bool vec = width % 8 == 0 && (((uintptr_t)y | (uintptr_t)shared | (uintptr_t)out) & 15) == 0 &&
+                   (!ids || (((uintptr_t)x & 15) == 0 && (ldx * xsize) % 16 == 0));
+  const int vec_threads = tokens < 2 * 148 ? 64 : 256;
+  const dim3 vec_grid(tokens, ceil_div(width / 8, vec_threads));
 #define TIB_COMBINE_GO(TS, TO)                                                                                       \
-  TIB_LAUNCH_DEPENDENT((moe_combine_kernel<TS, TO>), grid, threads, 0, stream, y, place, weights, top, (const TS*)shared, gate, \
-                       ld_gate, (TO*)out, width, ids, identity_from, (const TO*)x, ldx)
+  do {                                                                                                               \
+    if (vec)                                                                                                         \
+      TIB_LAUNCH_DEPENDENT((moe_combine_vec_kernel<TS, TO>), vec_grid, vec_threads, 0, stream, y, place, weights, top, (const TS*)shared, \
+                           gate, ld_gate, (TO*)out, width, ids, identity_from, (const TO*)x, ldx);                    \
+    else                                                                                                             \
+      TIB_LAUNCH_DEPENDENT((moe_combine_kernel<TS, TO>), grid, threads, 0, stream, y, place, weights, top, (const TS*)shared, gate, \
+                           ld_gate, (TO*)out, width, ids, identity_from, (const TO*)x, ldx);                         \
+  } while (0)
   const int sd = shared ? shared_dtype : out_dtype;
   if (sd == TIB_F32 && out_dtype == TIB_F32) TIB_COMBINE_GO(float, float);
   else if (sd == TIB_BF16 && out_dtype == TIB_BF16) TIB_COMBINE_GO(__nv_bfloat16, __nv_bfloat16);
