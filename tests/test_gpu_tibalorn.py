@@ -626,3 +626,47 @@ def test_sizes_drawn_at_random(draw, tmp_path):
             runner = make_runner(tmp_path, dtype, replay_util.peak_tokens(steps), page_size=rng.choice([4, 16]))
             rows = replay_util.gather(run_steps(runner, steps), index)
             compare(rows, tmp_path, requests, dtype, f"draw {draw} {kind}")
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,window,pool,keep,page,vfreq", [
+    (4, 2, 128, 100, 16, 0, 16, True), (3, 1, 64, 70, 8, 0, 8, False), (2, 2, 128, 300, 0, 20, 32, False), (5, 1, 64, 1, 4, 0, 16, True),
+    (64, 1, 64, 130, 0, 0, 128, False), (2, 1, 128, 64, 1, 0, 64, True)])
+def test_prompt_portions_of_window_attention_on_both_tensor_core_forms(heads, kv_heads, dim, window, pool, keep, page, vfreq):
+    """Portions around the edges of tiles (128 keys, 128 rows of tokens x heads), behind cached context, against the CUDA-core kernel
+    on the same pages; entries that no query may see hold NaN.  Turned values, temperature (one of them negative), sink and gate."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    g = torch.Generator().manual_seed(heads * dim + window)
+    rnd = lambda *shape: torch.randn(*shape, generator=g)
+    lens, pasts = [1, 130, 257, 66], [300, 0, 127, 511]
+    n, per = sum(lens), max(a + b for a, b in zip(lens, pasts)) // page + 1
+    pages = torch.full((len(lens) * per, 2, kv_heads, page, dim), float("nan"))
+    table = torch.randperm(len(lens) * per, generator=g).view(len(lens), per)
+    blocks, btable = None, None
+    if pool:
+        bper = max(a + b for a, b in zip(lens, pasts)) // pool // page + 1
+        blocks = torch.full((len(lens) * bper, 2, kv_heads, page, dim), float("nan"))
+        btable = torch.randperm(len(lens) * bper, generator=g).view(len(lens), bper)
+    for e, (new, past) in enumerate(zip(lens, pasts)):
+        for p in range(past + new):
+            pages[table[e, p // page], :, :, p % page] = rnd(2, kv_heads, dim)
+        for b in range((past + new) // pool if pool else 0):
+            blocks[btable[e, b // page], :, :, b % page] = rnd(2, kv_heads, dim)
+    cuda = lambda t: None if t is None else t.to(torch.bfloat16).cuda()
+    ints = lambda t: None if t is None else torch.as_tensor(t).to(torch.int32).cuda()
+    pages, blocks, table, btable = cuda(pages), cuda(blocks), ints(table), ints(btable)
+    q, gate = cuda(rnd(n, heads * dim)), cuda(rnd(n, heads * dim))
+    temp = (1 + 0.2 * rnd(heads))
+    temp[0] = -temp[0]
+    starts = ints([sum(lens[:i]) for i in range(len(lens) + 1)])
+    sink, freq, outs = rnd(heads).cuda(), torch.linspace(1.0, 0.01, dim // 2, device="cuda") if vfreq else None, []
+    for simt in (False, True):
+        out, error = torch.empty(n, heads * dim, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        ops.pooled_window_attention(q, out, starts, ints(pasts), ints(range(len(lens))), pages[:, 0], pages[:, 1], table,
+                                    blocks[:, 0] if pool else None, blocks[:, 1] if pool else None, btable, len(lens), max(lens), heads, kv_heads,
+                                    window=window, pool=pool, keep=keep, scale=dim ** -0.5, temp=temp.cuda(), sink=sink, value_freq=freq,
+                                    gate=gate, error_word=error, force_simt=simt)
+        assert int(error) == 0
+        outs.append(out.double().cpu())
+    # the weights' 16 bits (2^-16 of values of unit size, over a sum of weights of one), then a rounding to bfloat16 (2^-8) on either side
+    assert ((outs[0] - outs[1]).abs() <= 2.0 ** -7 * outs[1].abs() + 2.0 ** -12 * outs[1].abs().max()).all()

@@ -24,21 +24,9 @@
 // several blocks, whose sums a small second kernel adds in the order of the parts.
 #include "mma.cuh"
 #include <math_constants.h>
+#include "window_attention.cuh"
 
 namespace tib {
-
-struct PwaCache {
-  void* keys; void* values;          // first key / value of the layer's first page
-  const int* block_table; int table_stride;
-  int page_size; int64_t page_stride; int num_pages;
-};
-
-__device__ __forceinline__ int pwa_page(const PwaCache& c, const int* table, int index, int* error_word, int code) {
-  const int page = table[index / c.page_size];
-  if (page >= 0 && page < c.num_pages) return page;
-  if (error_word) atomicExch(error_word, code);
-  return -1;
-}
 
 // ---------------------------------------------------------------------------------------------------- append
 struct PwaAppendArgs {
@@ -267,22 +255,6 @@ constexpr int kPwaWarps = 4;
 constexpr int kPwaRowsPerWarp = 4;
 constexpr int kPwaRows = kPwaWarps * kPwaRowsPerWarp;      // rows (token, head) per block
 constexpr int kPwaKeys = 32;                               // keys per step = lanes
-
-struct PwaArgs {
-  const int* q_start; const int* kv_start; const int* slots;
-  int heads, kv_heads, dim, vdim;
-  int window, pool;                  // pool 0: no blocks, only the window
-  int keep;                          // tokens 0 .. keep - 1 are seen from behind the window too (pool 0 only)
-  float scale;
-  const float* temp; const float* sink;                    // [heads] or null
-  const float* vfreq;                                      // [vdim / 2] or null (values were not turned)
-  const void* gate; int gate_dtype; int64_t ld_gate;       // [tokens, heads * vdim] logits or null
-  const float* rel_bias; int rel_span;                     // [heads, rel_span] or null: added to a token's score by distance
-  PwaCache tokens, blocks;
-  int group_chunk, q_tile;
-  int* error_word;
-  float* partial; int n_splits; int n_tokens;              // a step of single tokens whose contexts are shared out over blocks
-};
 
 template <typename T, int DPL>
 __global__ void __launch_bounds__(kPwaWarps * 32)
@@ -1164,6 +1136,8 @@ TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_s
   if ((int64_t)kv_heads * chunks > 65535) return TIB_E_SIZE;
   // bf16 steps run on the tensor cores, single tokens too (their tiles come in by cp.async, 16 bytes a piece, where the
   // other kernel waits for one element at a time); 32-bit and head sizes that are no multiples of 8 run on the CUDA cores.
+  // Portions of prompts that fill the rows of a tile take tcgen05 products where pages and head sizes suit the copies.
+  if (dtype == TIB_BF16 && !force_simt && window_tcgen05_takes(a, q, out, max_q_len)) return window_tcgen05(q, out, a, n_entries, max_q_len, stream);
   if (dtype == TIB_BF16 && !force_simt && pwa_mma_takes(a, q)) {
     if (dim <= 64 && vdim <= 64) return pwa_launch_mma<64, 64>(q, out, a, n_entries, max_q_len, stream);
     if (dim <= 64) return pwa_launch_mma<64, 128>(q, out, a, n_entries, max_q_len, stream);
