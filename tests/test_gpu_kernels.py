@@ -899,7 +899,8 @@ def test_aligned_fp32_product_has_the_plain_kernels_bits(m, n, k):
 # ------------------------------------------------- linear attention in runs and token by token
 @pytest.mark.parametrize("lens, heads, key_dim, value_dim", [
     ([1, 1, 1], 3, 128, 128), ([32, 5, 9], 2, 64, 96),                        # token by token, to its longest portion
-    ([33, 1, 64], 2, 128, 64), ([65, 128, 127, 2], 2, 64, 128), ([200, 63], 3, 128, 128)])      # runs and their edges
+    ([33, 1, 64], 2, 128, 64), ([192, 7], 2, 64, 64),                                           # in chunks, to their longest portion
+    ([193, 1, 64], 2, 128, 64), ([257, 128, 127, 2], 2, 64, 128), ([200, 63], 3, 128, 128)])    # in runs and at their edges
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_linear_attention_forms_agree_with_the_recurrence(lens, heads, key_dim, value_dim, dtype):
     need_gpu()

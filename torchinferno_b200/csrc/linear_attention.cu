@@ -16,7 +16,7 @@
 // of one.  State is read from and written back to the request's slot; a new request's slot is zero.
 //
 // Three ways to run that, chosen by sizes alone (tib_linear_attention):
-//   runs   (portions above 32 tokens, head sizes of 64 or 128) every run of 64 tokens makes its own sum L of decayed k v^T
+//   runs   (portions above 192 tokens, head sizes of 64 or 128) every run of 64 tokens makes its own sum L of decayed k v^T
 //          side by side, one thread per state element then folds S <- lambda^n S + L over a request's runs, and every run
 //          makes its outputs from its starting state: the serial chain is one fused multiply-add a run
 //   walk   (steps whose portions have at most 32 tokens) S in registers, token by token
@@ -221,6 +221,7 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 // half rounded as the scalar instruction rounds it), operands from shared memory in 16-byte loads without bank conflicts.
 // Everything stays fp32: activations, decay powers, scores, states and sums.
 constexpr int kLinRun = 64;
+constexpr int kLinRunsFrom = 193;          // the shortest longest portion that is cut into runs
 constexpr int kLinPad = kLinRun + 4;       // row stride of the transposed q, k and scores
 
 struct LinRunArgs {
@@ -618,16 +619,17 @@ TIB_API int tib_linear_attention_chunk(int key_dim, int value_dim) {
   return 0;
 }
 
-// Tokens of a run, and the longest portion the walk takes.
+// Tokens of a run, the longest portion the walk takes, and the shortest longest portion that is cut into runs.
 TIB_API int tib_linear_attention_run() { return kLinRun; }
 TIB_API int tib_linear_attention_walk() { return kLinWalk; }
+TIB_API int tib_linear_attention_runs_from() { return kLinRunsFrom; }
 
 // q, k: [tokens, >= heads * key_dim] and v: [tokens, >= heads * value_dim] with row strides ldq, ldk, ldv (they may be
 // slices of one wider row); out: [tokens, heads * value_dim] fp32; state: [slots, heads, key_dim, value_dim] fp32;
 // powers: [heads, chunk + 1] fp32, powers[h][m] = lambda_h^m; activation: 0 none, 1 silu on q, k and v.
 // max_q_len: the longest entry of the step, 0 where it is not known (then, or without run_powers, the chunk kernel runs).
 // run_powers: [heads, run + 1] fp32 likewise, or null.  run_state: scratch of run_capacity >= tokens / run + n_entries times
-// heads * key_dim * value_dim floats for portions of more than tib_linear_attention_walk() tokens, or null.
+// heads * key_dim * value_dim floats for portions of tib_linear_attention_runs_from() tokens and more, or null.
 TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, int64_t ldq, int64_t ldk, int64_t ldv,
                                  float* out, float* state, const float* powers, const int* q_start, const int* slots,
                                  int n_entries, int heads, int key_dim, int value_dim, int chunk, int activation, int dtype,
@@ -637,8 +639,10 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   if (!q || !k || !v || !out || !state || !powers || !q_start || !slots) return TIB_E_ARG;
   if (heads < 1 || key_dim < 1 || value_dim < 1 || chunk < 1 || chunk > 32 || n_entries > 65535) return TIB_E_SIZE;
   // The newer kernels take heads of 64 or 128 keys whose values come in whole tiles, rows and state on 16-byte boundaries.
-  // The line between walk and runs: at 32 tokens a portion both take some 40 us (four portions of 16 heads of 128 x 128: the walk
-  // 14, 16 and 23 us at 8, 9 and 16 tokens, the runs' three launches 52 at 9, 54 at 16 and 71 at 64; the chunk kernel 33, 35, 78).
+  // The lines between the three: four portions of 16 heads of 128 x 128 take the walk 14, 16 and 23 us at 8, 9 and 16 tokens and the chunk
+  // kernel 33, 33 and 35; at 64 tokens the chunk kernel takes 78 and the runs 71.  The runs are two launches and an allocation
+  // more, which a step of a few hundred tokens waits for on the host: the layer on 158 and 78 tokens of 12 heads of 64 takes 89 us
+  // in chunks and 98 in runs, so chunks keep portions up to 192.
   const int64_t size = dtype == TIB_F32 ? 4 : 2;
   const bool aligned = (ldq * size) % 16 == 0 && (ldk * size) % 16 == 0 && (ldv * size) % 16 == 0 &&
                        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)run_state) & 15) == 0;
@@ -650,7 +654,7 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
     if (max_q_len <= kLinWalk)
       return dtype == TIB_F32 ? launch_lin_walk<float>(q, k, v, r, key_dim, n_entries, stream)
                               : launch_lin_walk<__nv_bfloat16>(q, k, v, r, key_dim, n_entries, stream);
-    if (run_state && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535) {
+    if (max_q_len >= kLinRunsFrom && run_state && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535) {
 #define TIB_LIN_GO(T)                                                                                             \
   (key_dim == 64 ? (value_dim % 128 == 0 ? launch_lin_runs<T, 64, 128>(q, k, v, r, n_entries, max_q_len, stream)    \
                                          : launch_lin_runs<T, 64, 64>(q, k, v, r, n_entries, max_q_len, stream))    \

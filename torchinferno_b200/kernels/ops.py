@@ -121,7 +121,7 @@ def lib() -> ctypes.CDLL:
                    "tib_gemm_tcgen05_swapab", "tib_gemm_tcgen05_swapab_supports", "tib_gemm_decode", "tib_gemm_decode_supports",
                    "tib_plan_attention", "tib_plan_product", "tib_blas_gemm_batched",
                    "tib_add_pair", "tib_unit_norm_add", "tib_sigmoid_gate", "tib_gelu_gate_table", "tib_relu_squared", "tib_gelu",
-                   "tib_scale_f32", "tib_pair_rows", "tib_add_vector", "tib_linear_attention", "tib_linear_attention_chunk", "tib_linear_attention_run", "tib_linear_attention_walk",
+                   "tib_scale_f32", "tib_pair_rows", "tib_add_vector", "tib_linear_attention", "tib_linear_attention_chunk", "tib_linear_attention_run", "tib_linear_attention_walk", "tib_linear_attention_runs_from",
                    "tib_latent_append", "tib_latent_prefill_supports", "tib_latent_gather", "tib_latent_prefill", "tib_latent_attention", "tib_latent_attention_splits", "tib_moe_route", "tib_moe_group", "tib_router_logits",
                    "tib_moe_expert_product", "tib_moe_combine", "tib_glu_clamp", "tib_layernorm", "tib_layernorm_tail",
                    "tib_qk_norm_append", "tib_sigmoid_attention", "tib_sigmoid_attention_takes_mma", "tib_gated_recurrence",
@@ -887,9 +887,20 @@ def linear_attention_chunk(key_dim: int, value_dim: int) -> int:
     return int(lib().tib_linear_attention_chunk(c_int(key_dim), c_int(value_dim)))
 
 
+_linear_sizes: tuple[int, int] | None = None
+
+
+def _linear_attention_sizes() -> tuple[int, int]:
+    """(tokens of a run, the shortest longest portion of a step that is cut into runs); asked of the library once."""
+    global _linear_sizes
+    if _linear_sizes is None:
+        _linear_sizes = int(lib().tib_linear_attention_run()), int(lib().tib_linear_attention_runs_from())
+    return _linear_sizes
+
+
 def linear_attention_run() -> int:
     """Tokens of a run of the decayed linear attention (long portions are cut into runs that go side by side)."""
-    return int(lib().tib_linear_attention_run())
+    return _linear_attention_sizes()[0]
 
 
 LINEAR_ATTENTION_SCRATCH = 1 << 30      # bytes of run states a call may take (2,048 tokens of 16 heads of 128 x 128: 34 MB)
@@ -916,11 +927,11 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
         raise KernelError("linear_attention: entry arrays are shorter than n_entries")
     run_state, capacity = None, 0
     if run_powers is not None:
-        run = linear_attention_run()
+        run, runs_from = _linear_attention_sizes()
         _need(run_powers, "run_powers", torch.float32)
         if run_powers.shape != (heads, run + 1):
             raise KernelError("linear_attention: run_powers has the wrong shape")
-        if max_q_len > int(lib().tib_linear_attention_walk()) and key_dim in (64, 128) and value_dim % 64 == 0:
+        if max_q_len >= runs_from and key_dim in (64, 128) and value_dim % 64 == 0:
             capacity = q.shape[0] // run + n_entries
             if capacity * heads * key_dim * value_dim * 4 <= LINEAR_ATTENTION_SCRATCH:
                 run_state = torch.empty(capacity * heads * key_dim * value_dim, dtype=torch.float32, device=q.device)
