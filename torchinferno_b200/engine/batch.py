@@ -63,43 +63,50 @@ def build_batch(placements: list[EntryPlacement], tokens: list[Sequence[int]], w
                 table_updates: list[tuple[list[int], list[int]]], device: torch.device
                 ) -> tuple[StepBatch, list[tuple[torch.Tensor, torch.Tensor]]]:
     """Pack the step's integers into one host buffer, upload it once, and slice it."""
-    token_ids: list[int] = []
-    positions: list[int] = []
-    token_slot: list[int] = []
-    q_start = [0]
-    kv_start: list[int] = []
-    slots: list[int] = []
+    n = sum(place.q_len for place in placements)
+    entries = len(placements)
+    q_start, kv_start, slots = [0], [], []
     logit_rows: list[int] = []
     logit_slots: list[int] = []
-    for place, toks, want in zip(placements, tokens, wants):
-        token_ids.extend(int(t) for t in toks)
-        positions.extend(range(place.kv_start, place.kv_start + place.q_len))
-        token_slot.extend([place.slot] * place.q_len)
+    for place, want in zip(placements, wants):
         q_start.append(place.q_start + place.q_len)
         kv_start.append(place.kv_start)
         slots.append(place.slot)
         logit_rows.extend(place.q_start + int(w) for w in want)
         logit_slots.extend([place.slot] * len(want))
-    sections = [token_ids, positions, token_slot, q_start, kv_start, slots, logit_rows, logit_slots]
+    small = [q_start, kv_start, slots, logit_rows, logit_slots]
     for index, value in table_updates:
-        sections.extend((index, value))
-    total = sum(len(s) for s in sections)
+        small.extend((index, value))
+    lengths = [n, n, n] + [len(section) for section in small]
+    total = sum(lengths)
     use_cuda = device.type == "cuda"
     host = torch.empty(max(total, 1), dtype=torch.int32, pin_memory=use_cuda)
+    # the three arrays of one number per token are filled entry by entry where they lie (a Python list of a prompt's numbers
+    # three times over took most of the time before the step's first launch); the short ones go in as one list
+    if entries and entries == n:      # single tokens
+        host[:3 * n] = torch.tensor([int(toks[0]) for toks in tokens] + kv_start + slots, dtype=torch.int32)
+    else:
+        row = 0
+        for place, toks in zip(placements, tokens):
+            end = row + place.q_len
+            host[row:end] = torch.tensor(toks if isinstance(toks, list) else [int(t) for t in toks], dtype=torch.int32)
+            torch.arange(place.kv_start, place.kv_start + place.q_len, dtype=torch.int32, out=host[n + row:n + end])
+            host[2 * n + row:2 * n + end].fill_(place.slot)
+            row = end
     flat: list[int] = []
-    for section in sections:
+    for section in small:
         flat.extend(section)
     if flat:
-        host[:total] = torch.tensor(flat, dtype=torch.int32)
+        host[3 * n:total] = torch.tensor(flat, dtype=torch.int32)
     dev = host.to(device, non_blocking=use_cuda)
     views: list[torch.Tensor] = []
     offset = 0
-    for section in sections:
-        views.append(dev[offset: offset + len(section)])
-        offset += len(section)
+    for length in lengths:
+        views.append(dev[offset: offset + length])
+        offset += length
     batch = StepBatch(
         token_ids=views[0], positions=views[1], token_slot=views[2], q_start=views[3], kv_start=views[4],
-        slots=views[5], logit_rows=views[6], logit_slots=views[7], n_tokens=len(token_ids), n_entries=len(placements),
+        slots=views[5], logit_rows=views[6], logit_slots=views[7], n_tokens=n, n_entries=entries,
         n_logits=len(logit_rows), max_q_len=max((p.q_len for p in placements), default=0),
         max_kv_len=max((p.kv_start + p.q_len for p in placements), default=0),
         n_single=sum(1 for p in placements if p.q_len == 1), n_multi=sum(1 for p in placements if p.q_len > 1),

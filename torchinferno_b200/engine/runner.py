@@ -86,7 +86,10 @@ class ModelRunner:
             seen.add(entry.request_id)
             if len(entry.tokens) < 1:
                 raise StepError(f"request {entry.request_id!r} brings no tokens")
-            for token in entry.tokens:
+            # (a list of whole numbers within the vocabulary needs no look at its tokens one by one)
+            plain = isinstance(entry.tokens, list) and set(map(type, entry.tokens)) == {int}
+            within = plain and min(entry.tokens) >= 0 and max(entry.tokens) < spec.vocab_size
+            for token in () if within else entry.tokens:
                 if not 0 <= int(token) < spec.vocab_size:
                     raise StepError(f"token id {token} of request {entry.request_id!r} is outside the vocabulary "
                                     f"(size {spec.vocab_size})")
