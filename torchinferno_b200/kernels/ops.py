@@ -979,12 +979,18 @@ def latent_append(dkv: torch.Tensor, q: torch.Tensor, folded: torch.Tensor | Non
 def latent_attention(folded: torch.Tensor, keys: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor, kv_start: torch.Tensor,
                      slots: torch.Tensor, block_table: torch.Tensor, n_entries: int, max_q_len: int, heads: int, rank: int,
                      rot: int, scale: float, error_word: torch.Tensor | None = None, max_kv_len: int = 0,
-                     force_simt: bool = False, sink: torch.Tensor | None = None) -> torch.Tensor:
+                     force_simt: bool = False, sink: torch.Tensor | None = None, merged: torch.Tensor | None = None) -> torch.Tensor:
     """Causal attention of folded queries [tokens, heads, rank + rot] (fp32) over paged latent rows; the value of a
     key is its first ``rank`` elements.  ``out``: [tokens, heads, rank] fp32.  A step of single tokens only
     (``max_q_len`` 1) that names the longest context (``max_kv_len``) cuts every context into runs that go to blocks of
-    their own and are merged by a second kernel.  ``sink`` [heads] fp32: exp(sink) is added to the softmax's denominator."""
+    their own and are merged by a second kernel.  ``sink`` [heads] fp32: exp(sink) is added to the softmax's denominator.
+    ``merged``: a bfloat16 tensor of ``out``'s shape that takes the rows, rounded once, when contexts were cut (``out`` is then left
+    as it is); the tensor that holds the rows is returned."""
     _need(folded, "folded", torch.float32), _need(out, "out", torch.float32)
+    if merged is not None:
+        _need(merged, "merged", torch.bfloat16)
+        if merged.shape != out.shape:
+            raise KernelError("latent_attention: merged does not fit")
     for name, t in (("q_start", q_start), ("kv_start", kv_start), ("slots", slots), ("block_table", block_table)):
         _need(t, name, torch.int32)
     n = folded.shape[0]
@@ -1007,10 +1013,11 @@ def latent_attention(folded: torch.Tensor, keys: torch.Tensor, out: torch.Tensor
         _ptr(folded), _ptr(keys), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(block_table),
         c_int(block_table.stride(0)), c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(rank), c_int(rot),
         c_int(keys.shape[2]), c_int64(keys.stride(0)), c_int(keys.shape[0]), c_float(scale), _ptr(sink), _ptr(partial), c_int(splits),
-        c_int(max_kv_len), c_int(int(force_simt)), _ptr(error_word), c_int(_code(keys.dtype)), _stream()))
+        c_int(max_kv_len), c_int(int(force_simt)), _ptr(error_word), c_int(_code(keys.dtype)),
+        _ptr(merged if splits > 1 else None), _stream()))
     if partial is not None:
         count_launches(1)
-    return out
+    return out if merged is None or splits == 1 else merged
 
 
 LATENT_TILE = 128      # an entry's keys made for the step are padded to a multiple of this many rows

@@ -168,15 +168,17 @@ class LatentAttention(Mixer):
         else:
             ops.library_gemm_batched(q_plain, self.uk_weight, folded[:, :, :c], w_kn=True)
         latent_out = torch.empty((n, h, c), dtype=torch.float32, device=x.device)
-        ops.latent_attention(folded, kv.keys, latent_out, batch.q_start, batch.kv_start, batch.slots, kv.block_table,
-                             batch.n_entries, batch.max_q_len, h, c, r, self.scale, ctx.error_word, max_kv_len=batch.max_kv_len,
-                             sink=self.sink)
+        rows = torch.empty((n, h, c), dtype=x.dtype, device=x.device) if x.dtype != torch.float32 else None
+        mixed = ops.latent_attention(folded, kv.keys, latent_out, batch.q_start, batch.kv_start, batch.slots, kv.block_table,
+                                     batch.n_entries, batch.max_q_len, h, c, r, self.scale, ctx.error_word, max_kv_len=batch.max_kv_len,
+                                     sink=self.sink, merged=rows)
         heads_out = torch.empty((n, h, self.value_dim), dtype=x.dtype, device=x.device)
         if x.dtype == torch.float32:
             for j in range(h):
                 ops.gemm_f32(latent_out[:, j], self.uv_weight[j], heads_out[:, j])
         else:
-            rows = ops.cast(latent_out, torch.empty((n, h, c), dtype=x.dtype, device=x.device))
+            if mixed is not rows:
+                ops.cast(mixed, rows)
             ops.library_gemm_batched(rows, self.uv_weight, heads_out, w_kn=False)
         heads_out = heads_out.view(n, h * self.value_dim)
         if self.gate:
