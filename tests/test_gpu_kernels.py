@@ -1058,3 +1058,119 @@ def test_gated_rows_by_eight_columns(rows, width, parts, mode):
         want = y.bfloat16().double() * torch.sigmoid(z[:, 8:8 + width // group].double()).repeat_interleave(group, 1)
     # fp32 arithmetic (a few roundings of 2^-24), then one rounding to the eight significant bits of bfloat16 (2^-8 at most)
     assert ((as_ref(out) - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 1e-6 * want.abs().max()).all()
+
+
+# ------------------------------------------------- routers, weighted sums, appends and block means of large steps
+@pytest.mark.parametrize("rows, k", [(1, 64), (8, 72), (9, 520), (33, 1020), (128, 256)])      # one, three and five rows a warp
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_router_logits_of_large_steps_have_the_bits_of_small_ones(rows, k, dtype):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    tokens = 8 * 148 + 5
+    x, w, bias = dev(rnd(tokens, (k + 7) // 8 * 8, dtype=dtype))[:, :k], dev(rnd(rows, k, seed=1)), dev(rnd(rows, seed=2))
+    out = ops.router_logits(x, w, torch.empty(tokens, rows, device="cuda"), bias)
+    parts = [ops.router_logits(x[i:i + 400], w, torch.empty(len(x[i:i + 400]), rows, device="cuda"), bias) for i in range(0, tokens, 400)]
+    assert torch.equal(out, torch.cat(parts))
+    want = as_ref(x) @ as_ref(w).T + as_ref(bias)
+    assert (as_ref(out) - want).abs().max() <= k * 2.0 ** -23 * want.abs().max()      # fp32 sums of k products
+
+
+@pytest.mark.parametrize("tokens, width, top", [(1, 8, 1), (7, 520, 3), (300, 2056, 2)])
+@pytest.mark.parametrize("shared, handed_on", [(False, False), (True, False), (True, True)])
+def test_weighted_sums_by_eight_columns_have_the_plain_kernels_bits(tokens, width, top, shared, handed_on):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    y, weights = rnd(tokens * top, width), rnd(tokens, top, seed=1).abs()
+    place = dev(torch.randperm(tokens * top, generator=torch.Generator().manual_seed(2)).int().view(tokens, top))
+    options = {}
+    if shared:
+        options = dict(shared=dev(rnd(tokens, width, dtype=torch.bfloat16, seed=3)), gate=dev(rnd(tokens, 1, seed=4))[:, 0])
+    if handed_on:
+        ids = torch.arange(tokens * top, dtype=torch.int32).view(tokens, top) % 5
+        options.update(ids=dev(ids), identity_from=3, x=dev(rnd(tokens, width, dtype=torch.bfloat16, seed=5)))
+    results = []
+    for shift in (0, 1):      # (rows off their 16-byte boundaries take the plain kernel)
+        rows = torch.empty(y.numel() + shift, device="cuda")[shift:].view(y.shape).copy_(dev(y))
+        results.append(ops.moe_combine(rows, place, dev(weights), torch.empty(tokens, width, dtype=torch.bfloat16, device="cuda"), **options))
+    assert torch.equal(*results)
+
+
+def page_views(pages, kv_heads, page, dim, vdim, dtype):
+    """One layer's key and value pages side by side in one buffer, zeroed."""
+    both = torch.zeros(pages, kv_heads * page * (dim + vdim), dtype=dtype, device="cuda")
+    cut = kv_heads * page * dim
+    return both[:, :cut].view(pages, kv_heads, page, dim), both[:, cut:].view(pages, kv_heads, page, vdim)
+
+
+@pytest.mark.parametrize("tokens, heads, kv_heads, dim, vdim, rot, turned", [
+    (3, 2, 1, 64, 32, 64, True), (70, 5, 2, 36, 20, 12, True), (33, 4, 4, 256, 256, 128, True), (9, 3, 1, 8, 6, 4, False)])
+def test_append_with_one_table_of_angles_agrees_with_the_plain_kernel(tokens, heads, kv_heads, dim, vdim, rot, turned):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    total, page = heads * dim + kv_heads * (dim + vdim), 8
+    pages = -(-tokens // page) + 1
+    rows, q_bias = rnd(tokens, total, dtype=torch.bfloat16), dev(rnd(heads * dim, seed=1))
+    freq = dev(1e4 ** (-torch.arange(rot // 2) / (rot // 2)))
+    vfreq = dev(1e4 ** (-torch.arange(vdim // 2) / (vdim // 2))) if turned else None
+    table = dev(torch.randperm(pages, generator=torch.Generator().manual_seed(3)).int().view(1, pages))
+    results = []
+    for shift in (2, 1):      # (columns off their 4-byte boundaries take the plain kernel)
+        wide = torch.zeros(tokens, total + 2, dtype=torch.bfloat16)
+        wide[:, shift:shift + total] = rows
+        keys, values = page_views(pages, kv_heads, page, dim, vdim, torch.bfloat16)
+        q = torch.empty(tokens, heads * dim, dtype=torch.bfloat16, device="cuda")
+        ops.rotary_kv_append(dev(wide), shift, shift + heads * dim,
+                             shift + (heads + kv_heads) * dim, q, keys, values, dev(torch.arange(tokens, dtype=torch.int32)),
+                             torch.zeros(tokens, dtype=torch.int32, device="cuda"), table, freq, vfreq, heads, kv_heads, dim, vdim,
+                             rot_dim=rot, amplitude=1.25, q_bias=q_bias)
+        results.append((q, keys, values))
+    for got, plain in zip(*results):
+        # the same fp32 turns (their sums differ by 2^-22 of a pair at most), each side rounded once to bfloat16
+        assert ((as_ref(got) - as_ref(plain)).abs() <= 2.0 ** -8 * as_ref(plain).abs() + 2.0 ** -22 * as_ref(plain).abs().max()).all()
+
+
+@pytest.mark.parametrize("tokens, kv_heads, dim, vdim, pool", [(65, 1, 64, 64, 4), (97, 2, 40, 24, 8), (300, 2, 128, 96, 32), (130, 1, 16, 8, 1)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_block_means_of_large_steps_have_the_bits_of_small_ones(tokens, kv_heads, dim, vdim, pool, dtype):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    page, pages = 16, -(-tokens // 16)
+    count = tokens // pool
+    keys, values = page_views(pages, kv_heads, page, dim, vdim, dtype)
+    keys.copy_(rnd(*keys.shape)), values.copy_(rnd(*values.shape, seed=1))
+    table, b_pages = dev(torch.arange(pages, dtype=torch.int32).flip(0).contiguous().view(1, pages)), -(-count // page) + 1
+    b_table = dev(torch.arange(b_pages, dtype=torch.int32).view(1, b_pages))
+    positions, slots = dev(torch.arange(tokens, dtype=torch.int32)), torch.zeros(tokens, dtype=torch.int32, device="cuda")
+    results = []
+    for run in (tokens, 50):
+        b_keys, b_values = page_views(b_pages, kv_heads, page, dim, vdim, dtype)
+        for i in range(0, tokens, run):
+            ops.pool_blocks(keys, values, table, b_keys, b_values, b_table, positions[i:i + run], slots[i:i + run], pool)
+        results.append((b_keys, b_values))
+    for large, small, rows in zip(*results, (keys, values)):
+        assert torch.equal(large, small)
+        flat = as_ref(rows).flip(0).transpose(1, 2).reshape(pages * page, kv_heads, -1)[:count * pool]
+        want = flat.view(count, pool, kv_heads, -1).mean(1)
+        got = as_ref(large).transpose(1, 2).reshape(b_pages * page, kv_heads, -1)[:count]
+        # fp32 sums of `pool` numbers, then one rounding to the element type
+        assert (got - want).abs().max() <= ((2.0 ** -8 if dtype == torch.bfloat16 else 0.0) + (pool + 1) * 2.0 ** -23) * want.abs().max() + pool * 2.0 ** -23
+
+
+@pytest.mark.parametrize("contexts, heads, rank", [([1, 64, 65, 1000], 3, 64), ([4000], 16, 512), ([129, 700], 20, 200)])
+@pytest.mark.parametrize("sink", [False, True])
+def test_merged_latent_rows_in_bfloat16_are_the_fp32_rows_rounded_once(contexts, heads, rank, sink):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    n, page, rot = len(contexts), 16, 16
+    per = -(-max(contexts) // page)
+    keys = dev(rnd(n * per, 1, page, rank + rot, dtype=torch.bfloat16, scale=0.7))
+    table = dev(torch.randperm(n * per, generator=torch.Generator().manual_seed(4)).int().view(n, per))
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    args = (ints(range(n + 1)), ints(c - 1 for c in contexts), ints(range(n)), table, n, 1, heads, rank, rot, 0.11)
+    options = dict(max_kv_len=max(contexts), sink=dev(rnd(heads, seed=2)) if sink else None)
+    folded = dev(rnd(n, heads, rank + rot, scale=0.3, seed=1))
+    out = ops.latent_attention(folded, keys, torch.empty(n, heads, rank, device="cuda"), *args, **options)
+    merged = torch.empty(n, heads, rank, dtype=torch.bfloat16, device="cuda")
+    rows = ops.latent_attention(folded, keys, torch.zeros_like(out), *args, merged=merged, **options)
+    assert torch.equal(rows.bfloat16(), out.bfloat16())
+    assert rows is merged
