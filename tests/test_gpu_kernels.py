@@ -1174,3 +1174,23 @@ def test_merged_latent_rows_in_bfloat16_are_the_fp32_rows_rounded_once(contexts,
     rows = ops.latent_attention(folded, keys, torch.zeros_like(out), *args, merged=merged, **options)
     assert torch.equal(rows.bfloat16(), out.bfloat16())
     assert rows is merged
+
+
+@pytest.mark.parametrize("tokens, experts, kept, top, groups, keep", [(1, 1, 1, 1, 1, 1), (31, 40, 33, 3, 4, 2), (64, 300, 300, 8, 1, 1), (65, 64, 64, 2, 8, 3)])
+def test_choices_and_sorting_in_one_launch(tokens, experts, kept, top, groups, keep):
+    """Some choices name no expert (``kept`` of ``experts`` are ones): their place is -1."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    logits, results = dev(rnd(tokens, experts)), []
+    for together in (True, False):
+        ids, weights = torch.empty(tokens, top, dtype=torch.int32, device="cuda"), torch.empty(tokens, top, device="cuda")
+        offsets, order, place = (torch.full((m,), -7, dtype=torch.int32, device="cuda") for m in (kept + 1, tokens * top, tokens * top))
+        ops.moe_route(logits, experts, top, ids, weights, groups=groups, keep=keep, sort=(kept, offsets, order, place) if together else None)
+        if not together:
+            ops.moe_group(ids, kept, offsets, order, place)
+        results.append((ids, weights, offsets))
+        flat, total = ids.flatten().cpu(), int((ids < kept).sum())
+        assert torch.equal(offsets.cpu().long(), torch.cat([torch.zeros(1, dtype=torch.long), torch.bincount(flat[flat < kept].long(), minlength=kept).cumsum(0)]))
+        assert torch.equal(flat[order[:total].cpu().long()], flat[flat < kept].sort()[0])
+        assert torch.equal(place[order[:total].long()].cpu(), torch.arange(total, dtype=torch.int32)) and (place.cpu()[flat >= kept] == -1).all()
+    assert all(torch.equal(a, b) for a, b in zip(*results))

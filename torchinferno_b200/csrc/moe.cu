@@ -65,6 +65,8 @@ router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restr
 #pragma unroll
       for (int i = 0; i < TOK; ++i) acc[r][i] = 0.f;
     if (VEC) {
+      // (small steps wait for loads: 12 us for eight tokens of 2,048 with one round's in flight, 7.4 with four rounds')
+#pragma unroll(R == 1 && TOK == kRouterTokens ? 4 : 1)
       for (int k = lane * 8; k < K8; k += 256) {
         float wv[R][8];
 #pragma unroll
@@ -106,16 +108,26 @@ router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restr
 // scores without the correction.  Lowest index first among equals, for groups and for experts.
 constexpr int kRouteMaxGroups = 64;      // (two groups a lane)
 
-__global__ void __launch_bounds__(128)
-moe_route_kernel(const float* __restrict__ logits, int64_t ld, int experts, int top, int sigmoid_scores,
-                 int normalize, float norm_eps, const float* __restrict__ correction, int groups, int keep,
-                 int* __restrict__ ids, float* __restrict__ weights, int tokens) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ unsigned char kept_s[4][kRouteMaxGroups];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (t >= tokens) return;
+struct MoeRouteArgs {
+  const float* logits; int64_t ld;
+  int experts, top, sigmoid_scores, normalize;
+  float norm_eps;
+  const float* correction;
+  int groups, keep;
+  int* ids; float* weights;
+  int tokens;
+};
+
+// One token, by a whole warp; kept: this warp's place for the kept groups.
+__device__ __forceinline__ void moe_route_token(const MoeRouteArgs& r, int t, unsigned char* kept) {
+  const float* __restrict__ logits = r.logits;
+  const float* __restrict__ correction = r.correction;
+  const int64_t ld = r.ld;
+  const int experts = r.experts, top = r.top, sigmoid_scores = r.sigmoid_scores, normalize = r.normalize, groups = r.groups, keep = r.keep;
+  const float norm_eps = r.norm_eps;
+  int* __restrict__ ids = r.ids;
+  float* __restrict__ weights = r.weights;
+  const int lane = threadIdx.x & 31;
   const float* z = logits + (size_t)t * ld;
   float mx = -CUDART_INF_F;
   for (int e = lane; e < experts; e += 32) mx = fmaxf(mx, z[e]);
@@ -133,7 +145,7 @@ moe_route_kernel(const float* __restrict__ logits, int64_t ld, int experts, int 
       const int g = lane + 32 * i;
       gscore[i] = -CUDART_INF_F;
       if (g < groups) {
-        kept_s[warp][g] = 0;
+        kept[g] = 0;
         for (int e = g * per_group; e < (g + 1) * per_group; ++e)
           gscore[i] = fmaxf(gscore[i], score(e) + (correction ? correction[e] : 0.f));
       }
@@ -155,7 +167,7 @@ moe_route_kernel(const float* __restrict__ logits, int64_t ld, int experts, int 
         if (og != 0x7fffffff && (best_g == 0x7fffffff || ob > best || (ob == best && og < best_g))) { best = ob; best_g = og; }
       }
       if (best_g < groups) {
-        if ((best_g & 31) == lane) { taken |= 1u << (best_g >> 5); kept_s[warp][best_g] = 1; }
+        if ((best_g & 31) == lane) { taken |= 1u << (best_g >> 5); kept[best_g] = 1; }
       }
     }
     __syncwarp();
@@ -167,7 +179,7 @@ moe_route_kernel(const float* __restrict__ logits, int64_t ld, int experts, int 
     int best_e = 0x7fffffff;
     for (int e = lane, i = 0; e < experts; e += 32, ++i) {
       if ((taken_lo >> i) & 1ull) continue;
-      if (grouped && !kept_s[warp][e / per_group]) continue;
+      if (grouped && !kept[e / per_group]) continue;
       const float s = score(e);
       const float c = s + (correction ? correction[e] : 0.f);
       if (c > best || best_e == 0x7fffffff) { best = c; best_s = s; best_e = e; }     // (rising e: the lowest index wins among equals)
@@ -188,13 +200,18 @@ moe_route_kernel(const float* __restrict__ logits, int64_t ld, int experts, int 
   if (normalize) for (int k = lane + 32; k < top; k += 32) weights[(size_t)t * top + k] /= (chosen_sum + norm_eps);
 }
 
-// ------------------------------------------------------------------- group
-// One block.  counts in shared memory (experts <= 1024), exclusive scan by one warp, then placement with atomics.
-__global__ void __launch_bounds__(1024)
-moe_group_kernel(const int* __restrict__ ids, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ order,
-                 int* __restrict__ place) {
+__global__ void __launch_bounds__(128) moe_route_kernel(MoeRouteArgs r) {
   pdl_wait();
   pdl_trigger();
+  __shared__ unsigned char kept_s[4][kRouteMaxGroups];
+  const int warp = threadIdx.x >> 5, t = blockIdx.x * (blockDim.x >> 5) + warp;
+  if (t < r.tokens) moe_route_token(r, t, kept_s[warp]);
+}
+
+// ------------------------------------------------------------------- group
+// One block.  counts in shared memory (experts <= 1024), exclusive scan by one warp, then placement with atomics.
+__device__ __forceinline__ void moe_group_pairs(const int* ids, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ order,
+                                               int* __restrict__ place) {
   __shared__ int count[1024];
   __shared__ int cursor[1024];
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
@@ -204,10 +221,20 @@ moe_group_kernel(const int* __restrict__ ids, int pairs, int experts, int* __res
     if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {      // a warp's running sums, 32 experts at a time
     int run = 0;
-    for (int e = 0; e < experts; ++e) { offsets[e] = run; cursor[e] = run; run += count[e]; }
-    offsets[experts] = run;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + (int)threadIdx.x, own = e < experts ? count[e] : 0;
+      int upto = own;
+#pragma unroll
+      for (int step = 1; step < 32; step *= 2) {
+        const int below = __shfl_up_sync(0xffffffffu, upto, step);
+        if ((int)threadIdx.x >= step) upto += below;
+      }
+      if (e < experts) { offsets[e] = run + upto - own; cursor[e] = run + upto - own; }
+      run += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (threadIdx.x == 0) offsets[experts] = run;
   }
   __syncthreads();
   for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
@@ -220,6 +247,29 @@ moe_group_kernel(const int* __restrict__ ids, int pairs, int experts, int* __res
       place[p] = -1;
     }
   }
+}
+
+__global__ void __launch_bounds__(1024)
+moe_group_kernel(const int* __restrict__ ids, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ order,
+                 int* __restrict__ place) {
+  pdl_wait();
+  pdl_trigger();
+  moe_group_pairs(ids, pairs, experts, offsets, order, place);
+}
+
+// Both for a step of few tokens, in one launch: a warp per token makes its choices, then the block sorts the pairs.  (Eight tokens x 4
+// of 32: 7.4 us cold, where the two kernels took 5.0 and 3.5 and the second's launch; beyond 64 tokens, two rounds of the block's
+// warps, one block's arithmetic is slower than the grid's.)
+constexpr int kRouteGroupTokens = 64;
+__global__ void __launch_bounds__(1024)
+moe_route_group_kernel(MoeRouteArgs r, int kept_experts, int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ place) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ unsigned char kept_s[32][kRouteMaxGroups];
+  const int warp = threadIdx.x >> 5;
+  for (int t = warp; t < r.tokens; t += 32) moe_route_token(r, t, kept_s[warp]);
+  __syncthreads();
+  moe_group_pairs(r.ids, r.tokens * r.top, kept_experts, offsets, order, place);
 }
 
 // ---------------------------------------------------------------- products
@@ -429,16 +479,26 @@ TIB_API int tib_router_logits(const void* x, int x_dtype, int64_t ldx, const flo
 
 // correction: [experts] fp32 added to the scores for the choice only, or null; groups > 1 with keep < groups: the experts
 // are cut into `groups` equal runs of adjacent ones and only members of the best `keep` runs are eligible.
+// offsets, order, place (or null): with at most 64 tokens the pairs are sorted by expert in the same launch, as
+// tib_moe_group does for `sorted_experts` experts.
 TIB_API int tib_moe_route(const float* logits, int64_t ld, int tokens, int experts, int top, int sigmoid_scores, int normalize,
                           float norm_eps, const float* correction, int groups, int keep, int* ids, float* weights,
-                          cudaStream_t stream) {
+                          int sorted_experts, int* offsets, int* order, int* place, cudaStream_t stream) {
   if (tokens == 0) return TIB_OK;
   if (!logits || !ids || !weights) return TIB_E_ARG;
   if (experts < 1 || experts > 2048 || top < 1 || top > experts) return TIB_E_SIZE;
   if (groups < 1 || keep < 1 || keep > groups || groups > kRouteMaxGroups || experts % groups) return TIB_E_SIZE;
   if (groups > 1 && keep < groups && top > keep * (experts / groups)) return TIB_E_SIZE;
-  TIB_LAUNCH_DEPENDENT(moe_route_kernel, ceil_div(tokens, 4), 128, 0, stream, logits, ld, experts, top, sigmoid_scores, normalize,
-                       norm_eps, correction, groups, keep, ids, weights, tokens);
+  MoeRouteArgs r;
+  r.logits = logits; r.ld = ld; r.experts = experts; r.top = top; r.sigmoid_scores = sigmoid_scores; r.normalize = normalize; r.norm_eps = norm_eps;
+  r.correction = correction; r.groups = groups; r.keep = keep; r.ids = ids; r.weights = weights; r.tokens = tokens;
+  if (offsets) {      // choices and sorting in one launch
+    if (!order || !place) return TIB_E_ARG;
+    if (tokens > kRouteGroupTokens || sorted_experts < 1 || sorted_experts > 1024) return TIB_E_SIZE;
+    TIB_LAUNCH_DEPENDENT(moe_route_group_kernel, 1, 1024, 0, stream, r, sorted_experts, offsets, order, place);
+    return TIB_OK;
+  }
+  TIB_LAUNCH_DEPENDENT(moe_route_kernel, ceil_div(tokens, 4), 128, 0, stream, r);
   return TIB_OK;
 }
 

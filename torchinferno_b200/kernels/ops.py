@@ -1097,13 +1097,18 @@ def router_logits(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: tor
     return out
 
 
+MOE_SORT_TOKENS = 64      # steps of at most this many tokens choose and sort in one launch (tib_moe_route)
+
+
 def moe_route(logits: torch.Tensor, experts: int, top: int, ids: torch.Tensor, weights: torch.Tensor, *,
               sigmoid_scores: bool = False, normalize: bool = True, norm_eps: float = 0.0,
-              correction: torch.Tensor | None = None, groups: int = 1, keep: int = 1) -> None:
+              correction: torch.Tensor | None = None, groups: int = 1, keep: int = 1,
+              sort: tuple[int, torch.Tensor, torch.Tensor, torch.Tensor] | None = None) -> None:
     """From fp32 router logits (the first ``experts`` columns of ``logits``): the ``top`` best experts of every token and
     their weights.  ``correction`` [experts] is added to the scores for the choice only (the weights are made from the
     scores themselves); with ``groups`` > 1 the outputs are cut into that many equal runs of adjacent ones, every run is
-    ranked by the best corrected score in it, and only members of the ``keep`` best runs are eligible."""
+    ranked by the best corrected score in it, and only members of the ``keep`` best runs are eligible.  ``sort`` (experts,
+    offsets, order, place): the pairs are sorted too, as ``moe_group`` does, for a step of few tokens in the same launch."""
     if not logits.is_cuda or logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1 or logits.shape[1] < experts:
         raise KernelError("moe_route: logits must be 2-D fp32 with unit inner stride and at least `experts` columns")
     _need(ids, "ids", torch.int32), _need(weights, "weights", torch.float32)
@@ -1116,18 +1121,31 @@ def moe_route(logits: torch.Tensor, experts: int, top: int, ids: torch.Tensor, w
             raise KernelError("moe_route: correction must hold one number per expert")
     if groups <= 1:
         groups = keep = 1
+    together = sort is not None and 0 < n <= MOE_SORT_TOKENS
+    if together:
+        _moe_sorted_arrays(ids, *sort)
+    kept, offsets, order, place = sort if together else (0, None, None, None)
     _check("moe_route", lib().tib_moe_route(_ptr(logits), c_int64(logits.stride(0)), c_int(n), c_int(experts), c_int(top),
                                             c_int(int(sigmoid_scores)), c_int(int(normalize)), c_float(norm_eps),
-                                            _ptr(correction), c_int(groups), c_int(keep), _ptr(ids), _ptr(weights), _stream()))
+                                            _ptr(correction), c_int(groups), c_int(keep), _ptr(ids), _ptr(weights),
+                                            c_int(kept), _ptr(offsets), _ptr(order), _ptr(place), _stream()))
+    if sort is not None and not together:
+        moe_group(ids, *sort)
 
 
-def moe_group(ids: torch.Tensor, experts: int, offsets: torch.Tensor, order: torch.Tensor, place: torch.Tensor) -> None:
-    """Sort the (token, choice) pairs by expert on the device: offsets [experts + 1], order[sorted] = pair, place[pair] = sorted."""
+def _moe_sorted_arrays(ids: torch.Tensor, experts: int, offsets: torch.Tensor, order: torch.Tensor, place: torch.Tensor) -> int:
+    """The number of pairs, when the arrays fit."""
     for name, t in (("ids", ids), ("offsets", offsets), ("order", order), ("place", place)):
         _need(t, name, torch.int32)
     pairs = ids.numel()
     if offsets.numel() != experts + 1 or order.numel() != pairs or place.numel() != pairs:
         raise KernelError("moe_group: array lengths do not fit")
+    return pairs
+
+
+def moe_group(ids: torch.Tensor, experts: int, offsets: torch.Tensor, order: torch.Tensor, place: torch.Tensor) -> None:
+    """Sort the (token, choice) pairs by expert on the device: offsets [experts + 1], order[sorted] = pair, place[pair] = sorted."""
+    pairs = _moe_sorted_arrays(ids, experts, offsets, order, place)
     _check("moe_group", lib().tib_moe_group(_ptr(ids), c_int(pairs), c_int(experts), _ptr(offsets), _ptr(order), _ptr(place), _stream()))
 
 

@@ -131,12 +131,12 @@ class RoutedExperts(FeedForward):
         ids = torch.empty((n, top), dtype=torch.int32, device=dev)
         weights = torch.empty((n, top), dtype=torch.float32, device=dev)
         count, keep = self.groups if self.groups is not None else (1, 1)
-        ops.moe_route(logits, self.routed, top, ids, weights, sigmoid_scores=self.scores == "sigmoid",
-                      normalize=self.normalize, norm_eps=self.norm_eps, correction=self.correction, groups=count, keep=keep)
         offsets = torch.empty(self.experts + 1, dtype=torch.int32, device=dev)
         order = torch.empty(n * top, dtype=torch.int32, device=dev)
         place = torch.empty(n * top, dtype=torch.int32, device=dev)
-        ops.moe_group(ids, self.experts, offsets, order, place)
+        ops.moe_route(logits, self.routed, top, ids, weights, sigmoid_scores=self.scores == "sigmoid",
+                      normalize=self.normalize, norm_eps=self.norm_eps, correction=self.correction, groups=count, keep=keep,
+                      sort=(self.experts, offsets, order, place))
         inner = torch.empty((n * top, self.expert_size), dtype=x.dtype, device=dev)
         ops.moe_expert_product(x, self.up_weight, inner, offsets, order, top, x_by_pair=True, act=self.activation,
                                limit=self.limit, alpha=self.alpha, row_scale=weights.view(-1) if self.weight_on_input else None,
