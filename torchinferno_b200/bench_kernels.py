@@ -265,7 +265,7 @@ def run_step_timeline(args) -> None:
 
 
 def run_latent_attention(args) -> None:
-    """The latent attention kernel on a prompt of --tokens (flops: folded scores over rank + rot and values over rank, causal)
+    """The latent attention kernel over folded queries on a prompt of --tokens (flops: folded scores over rank + rot and values over rank, causal)
     and on --batch single tokens at --context (bytes: the latent rows of every context once)."""
     h, c, r, page = args.heads, args.rank, args.rot, args.page_size
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
@@ -286,16 +286,18 @@ def run_latent_attention(args) -> None:
             flops, moved = None, n * ctx * (c + r) * 2
         fn = lambda: ops.latent_attention(folded, keys, out, q_start, kv_start, slots, table, n_entries, max_q, h, c, r, 0.07,
                                           max_kv_len=ctx)
-        report(f"latent_attention[{mode}]", timer(fn), flops=flops, bytes_moved=moved, entries=n_entries, context=ctx, heads=h,
+        report(f"latent_attention[{mode}, folded]", timer(fn), flops=flops, bytes_moved=moved, entries=n_entries, context=ctx, heads=h,
                rank=c, rot=r)
 
 
 def run_linear_attention(args) -> None:
-    """The decayed linear attention kernel on a prompt of --tokens (flops of the chunked form) and on --batch single
+    """The decayed linear attention on a prompt of --tokens (flops of runs of its length), in the form the layer takes, and on --batch single
     tokens (bytes: every head's state read and written once)."""
     h, d, v = args.heads, args.key_dim, args.value_dim
     chunk = ops.linear_attention_chunk(d, v)
-    powers = (torch.full((h, 1), 0.99, dtype=torch.float64) ** torch.arange(chunk + 1, dtype=torch.float64)[None]).float().cuda()
+    run = ops.linear_attention_run()
+    powers, run_powers = ((torch.full((h, 1), 0.99, dtype=torch.float64) ** torch.arange(most + 1, dtype=torch.float64)[None]).float().cuda()
+                          for most in (chunk, run))
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
     timer = Timer(args.iters)
     for mode in ("prompt", "single tokens"):
@@ -306,10 +308,11 @@ def run_linear_attention(args) -> None:
         state = torch.zeros(n_entries, h, d, v, device="cuda")
         q_start = i32([0, n]) if mode == "prompt" else i32(list(range(n + 1)))
         slots = i32(list(range(n_entries)))
-        fn = lambda: ops.linear_attention(q, k, val, out, state, powers, q_start, slots, n_entries, h, d, v, silu=True)
+        fn = lambda: ops.linear_attention(q, k, val, out, state, powers, q_start, slots, n_entries, h, d, v, silu=True,
+                                          max_q_len=n // n_entries, run_powers=run_powers)
         if mode == "prompt":
-            flops = 2 * h * n * (chunk * (d + v) / 2 + 2 * d * v)
-            report("linear_attention[prompt]", timer(fn), flops=flops, tokens=n, heads=h, key_dim=d, value_dim=v, chunk=chunk)
+            flops = 2 * h * n * (run * (d + v) / 2 + 2 * d * v)
+            report("linear_attention[prompt]", timer(fn), flops=flops, tokens=n, heads=h, key_dim=d, value_dim=v, run=run)
         else:
             report("linear_attention[single tokens]", timer(fn), bytes_moved=2 * n * h * d * v * 4, batch=n, heads=h, key_dim=d,
                    value_dim=v)
@@ -379,7 +382,7 @@ def run_sigmoid_attention(args) -> None:
             fn = lambda: ops.sigmoid_attention(q, keys, values, out, q_start, kv_start, slots, table, n_entries, max_q, h, k,
                                                scale=0.1, chunk=chunk, head_bias=bias, gate=gate, force_simt=simt)
             report(f"sigmoid_attention[{'cuda cores' if simt else 'mma.sync'}, {mode}]", timer(fn), flops=flops, bytes_moved=moved,
-                   entries=n_entries, context=ctx, heads=h, kv_heads=k, head_dim=d, value_dim=v, chunk=chunk)
+                   entries=n_entries, context=ctx, heads=h, kv_heads=k, head_dim=d, value_dim=v, run=run)
 
 
 def run_gated_recurrence(args) -> None:
