@@ -110,10 +110,10 @@ __global__ void __launch_bounds__(512) pwa_append_kernel(const T* __restrict__ p
 
 // The same for bf16 rows whose pairs lie on 4-byte boundaries: the token's cosines and sines are made once for all heads, and a
 // thread moves two neighbouring elements (with their partners) at a time.  Same bits.  2,048 tokens of 16 + 8 + 8 heads of 128:
-// 28 us with angles made per head, 21 here (both cold).
+// 28 us with angles made per head, 21 here; three tokens of 12 + 12 + 12: 7.4 and 6.2 (all cold).
 constexpr int kPwaTurns = 128;       // pairs of a table
 
-__global__ void __launch_bounds__(256) pwa_append_pairs_kernel(const __nv_bfloat16* __restrict__ proj, __nv_bfloat16* __restrict__ q_out,
+__global__ void __launch_bounds__(1024) pwa_append_pairs_kernel(const __nv_bfloat16* __restrict__ proj, __nv_bfloat16* __restrict__ q_out,
                                                                PwaAppendArgs a) {
   pdl_wait();
   pdl_trigger();
@@ -185,7 +185,7 @@ struct PwaPoolArgs {
   int* error_word;
 };
 
-// grid (runs of `per` tokens, kv_heads, tiles of kPoolTile elements); a block has work only where one of its tokens completes a block
+// grid (runs of `per` tokens, kv_heads, tiles of kPoolTile elements, or 1); a block has work only where one of its tokens completes a block
 // of `pool` positions.  The positions of such a block are dealt to kPoolLanes lanes (lane l sums l, l + lanes, ... in
 // rising order, every load of a thread in flight at once); then one thread per element adds the lanes' sums in the order of
 // the lanes.  The order is the same wherever the block is completed, in a prompt's portion or by a single token.
@@ -206,12 +206,8 @@ __global__ void __launch_bounds__(kPoolLanes * kPoolTile) pwa_pool_kernel(PwaPoo
   // (every warp looks at the same tokens, so all agree on what there is to do)
   const int my_pos = wl < a.per && t0 + wl < a.n_tokens ? a.positions[t0 + wl] : 0;
   unsigned todo = __ballot_sync(0xffffffffu, wl < a.per && t0 + wl < a.n_tokens && my_pos % a.pool == a.pool - 1);
-  const int e = blockIdx.z * kPoolTile + col;
   const int width = a.dim + a.vdim;
   const float inv = 1.f / (float)a.pool;
-  const bool live = e < width, is_k = e < a.dim;
-  const int dd = is_k ? e : e - a.dim, w = is_k ? a.dim : a.vdim;
-  const T* base = reinterpret_cast<const T*>(is_k ? a.tokens.keys : a.tokens.values);
   for (; todo; todo &= todo - 1) {
     const int bit = __ffs(todo) - 1, t = t0 + bit;
     const int pos = __shfl_sync(0xffffffffu, my_pos, bit);
@@ -221,30 +217,36 @@ __global__ void __launch_bounds__(kPoolLanes * kPoolTile) pwa_pool_kernel(PwaPoo
     const int bpage = pwa_page(a.blocks, btable, b, a.error_word, 0x40000 + (t & 0xffff));
     if (bpage < 0) continue;
     bool bad = false;
-    float sum = 0.f;
-    for (int j0 = lane; j0 < a.pool; j0 += kPoolLanes * kPoolAhead) {
-      float got[kPoolAhead];
+    for (int e0 = blockIdx.z * kPoolTile; e0 < width; e0 += gridDim.z * kPoolTile) {
+      const int e = e0 + col;
+      const bool live = e < width, is_k = e < a.dim;
+      const int dd = is_k ? e : e - a.dim, w = is_k ? a.dim : a.vdim;
+      const T* base = reinterpret_cast<const T*>(is_k ? a.tokens.keys : a.tokens.values);
+      float sum = 0.f;
+      for (int j0 = lane; j0 < a.pool; j0 += kPoolLanes * kPoolAhead) {
+        float got[kPoolAhead];
 #pragma unroll
-      for (int u = 0; u < kPoolAhead; ++u) {
-        const int j = j0 + u * kPoolLanes;
-        got[u] = 0.f;
-        if (!live || j >= a.pool) continue;
-        const int page = ttable[(first + j) / a.tokens.page_size];
-        if (page < 0 || page >= a.tokens.num_pages) { bad = true; continue; }
-        got[u] = to_f32(base[(size_t)page * a.tokens.page_stride + ((size_t)kvh * a.tokens.page_size + (first + j) % a.tokens.page_size) * w + dd]);
+        for (int u = 0; u < kPoolAhead; ++u) {
+          const int j = j0 + u * kPoolLanes;
+          got[u] = 0.f;
+          if (!live || j >= a.pool) continue;
+          const int page = ttable[(first + j) / a.tokens.page_size];
+          if (page < 0 || page >= a.tokens.num_pages) { bad = true; continue; }
+          got[u] = to_f32(base[(size_t)page * a.tokens.page_stride + ((size_t)kvh * a.tokens.page_size + (first + j) % a.tokens.page_size) * w + dd]);
+        }
+#pragma unroll
+        for (int u = 0; u < kPoolAhead; ++u) sum += got[u];
       }
+      __syncthreads();
+      part_s[lane][col] = sum;
+      __syncthreads();
+      if (lane == 0 && live) {
+        float total = 0.f;
 #pragma unroll
-      for (int u = 0; u < kPoolAhead; ++u) sum += got[u];
-    }
-    __syncthreads();
-    part_s[lane][col] = sum;
-    __syncthreads();
-    if (lane == 0 && live) {
-      float total = 0.f;
-#pragma unroll
-      for (int l = 0; l < kPoolLanes; ++l) total += part_s[l][col];
-      T* out = reinterpret_cast<T*>(is_k ? a.blocks.keys : a.blocks.values);
-      out[(size_t)bpage * a.blocks.page_stride + ((size_t)kvh * a.blocks.page_size + b % a.blocks.page_size) * w + dd] = from_f32<T>(total * inv);
+        for (int l = 0; l < kPoolLanes; ++l) total += part_s[l][col];
+        T* out = reinterpret_cast<T*>(is_k ? a.blocks.keys : a.blocks.values);
+        out[(size_t)bpage * a.blocks.page_stride + ((size_t)kvh * a.blocks.page_size + b % a.blocks.page_size) * w + dd] = from_f32<T>(total * inv);
+      }
     }
     if (bad && a.error_word) atomicExch(a.error_word, 0x50000 + (t & 0xffff));
   }
@@ -1060,7 +1062,10 @@ TIB_API int tib_rotary_kv_append(const void* proj, int64_t ld, int q_off, int k_
   if (dtype == TIB_BF16 && dim % 2 == 0 && vdim % 2 == 0 && rot_dim % 4 == 0 && vhalf % 2 == 0 && rot_dim / 2 <= kPwaTurns && vhalf <= kPwaTurns &&
       ld % 2 == 0 && q_off % 2 == 0 && k_off % 2 == 0 && v_off % 2 == 0 && page_stride % 2 == 0 &&
       (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages) & 3) == 0) {
-    TIB_LAUNCH_DEPENDENT(pwa_append_pairs_kernel, n_tokens, 256, 0, stream, (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a);
+    // few tokens: a thread for every two elements, so that a token is one round of loads and not five or six one after the other
+    const int units = ((heads + kv_heads) * dim + kv_heads * vdim) / 4;
+    const int wide = units > 1024 ? 1024 : units < 256 ? 256 : (units + 31) / 32 * 32;
+    TIB_LAUNCH_DEPENDENT(pwa_append_pairs_kernel, n_tokens, n_tokens <= 2 * 148 ? wide : 256, 0, stream, (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a);
     return TIB_OK;
   }
   if (dtype == TIB_F32)
@@ -1089,7 +1094,7 @@ TIB_API int tib_pool_blocks(const void* k_pages, const void* v_pages, const int*
   a.blocks = pwa_cache(bk_pages, bv_pages, b_table, b_table_stride, b_page_size, b_page_stride, b_num_pages);
   a.error_word = error_word;
   a.n_tokens = n_tokens; a.per = n_tokens > 2 * kPoolRun ? kPoolRun : 1;
-  const dim3 grid(ceil_div(n_tokens, a.per), kv_heads, ceil_div(dim + vdim, kPoolTile));
+  const dim3 grid(ceil_div(n_tokens, a.per), kv_heads, a.per > 1 ? ceil_div(dim + vdim, kPoolTile) : 1);      // (few tokens: most complete nothing)
   if (dtype == TIB_F32) TIB_LAUNCH_DEPENDENT(pwa_pool_kernel<float>, grid, kPoolLanes * kPoolTile, 0, stream, a);
   else if (dtype == TIB_BF16) TIB_LAUNCH_DEPENDENT(pwa_pool_kernel<__nv_bfloat16>, grid, kPoolLanes * kPoolTile, 0, stream, a);
   else return TIB_E_DTYPE;
