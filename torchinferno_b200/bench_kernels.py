@@ -382,7 +382,7 @@ def run_sigmoid_attention(args) -> None:
             fn = lambda: ops.sigmoid_attention(q, keys, values, out, q_start, kv_start, slots, table, n_entries, max_q, h, k,
                                                scale=0.1, chunk=chunk, head_bias=bias, gate=gate, force_simt=simt)
             report(f"sigmoid_attention[{'cuda cores' if simt else 'mma.sync'}, {mode}]", timer(fn), flops=flops, bytes_moved=moved,
-                   entries=n_entries, context=ctx, heads=h, kv_heads=k, head_dim=d, value_dim=v, run=run)
+                   entries=n_entries, context=ctx, heads=h, kv_heads=k, head_dim=d, value_dim=v, chunk=chunk)
 
 
 def run_gated_recurrence(args) -> None:
