@@ -83,7 +83,7 @@ def build_batch(placements: list[EntryPlacement], tokens: list[Sequence[int]], w
     host = torch.empty(max(total, 1), dtype=torch.int32, pin_memory=use_cuda)
     # the three arrays of one number per token are filled entry by entry where they lie (a Python list of a prompt's numbers
     # three times over took most of the time before the step's first launch); the short ones go in as one list
-    if entries and entries == n:      # single tokens
+    if entries and all(place.q_len == 1 for place in placements):      # single tokens
         host[:3 * n] = torch.tensor([int(toks[0]) for toks in tokens] + kv_start + slots, dtype=torch.int32)
     else:
         row = 0
