@@ -89,7 +89,8 @@ def build_batch(placements: list[EntryPlacement], tokens: list[Sequence[int]], w
         row = 0
         for place, toks in zip(placements, tokens):
             end = row + place.q_len
-            host[row:end] = torch.tensor(toks if isinstance(toks, list) else [int(t) for t in toks], dtype=torch.int32)
+            plain = isinstance(toks, list) and set(map(type, toks)) == {int}
+            host[row:end] = torch.tensor(toks if plain else [int(t) for t in toks], dtype=torch.int32)
             torch.arange(place.kv_start, place.kv_start + place.q_len, dtype=torch.int32, out=host[n + row:n + end])
             host[2 * n + row:2 * n + end].fill_(place.slot)
             row = end
