@@ -1194,3 +1194,23 @@ def test_choices_and_sorting_in_one_launch(tokens, experts, kept, top, groups, k
         assert torch.equal(flat[order[:total].cpu().long()], flat[flat < kept].sort()[0])
         assert torch.equal(place[order[:total].long()].cpu(), torch.arange(total, dtype=torch.int32)) and (place.cpu()[flat >= kept] == -1).all()
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("missing", [0, 128, 256])
+def test_gathered_latent_rows_stay_within_their_buffer(missing):
+    """Two entries of 200 and 129 keys need 512 rows; with fewer, what is missing is reported and nothing is written behind the last."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    rank, rot, page, lens = 16, 8, 16, (200, 129)
+    pool = dev(rnd(32, 1, page, rank + rot, dtype=torch.bfloat16))
+    table = dev(torch.arange(32, dtype=torch.int32).view(2, 16))
+    latent_room, rotated_room = (torch.full((512 + 8, w), 7.0, dtype=torch.bfloat16, device="cuda") for w in (rank, rot))
+    rows, error = 512 - missing, torch.zeros(1, dtype=torch.int32, device="cuda")
+    ints = lambda v: dev(torch.tensor(v, dtype=torch.int32))
+    ops.latent_gather(pool, table, ints([0, 50, 51]), ints([150, 128]), ints([0, 1]), 2, 200, latent_room[:rows], rotated_room[:rows], error)
+    want = torch.zeros(512, rank + rot, dtype=torch.bfloat16)
+    for first, n, at in ((0, lens[0], 0), (256, lens[1], 16)):
+        want[first:first + n] = pool[at:at + 16].cpu().view(256, rank + rot)[:n]
+    got = torch.cat([latent_room, rotated_room], 1).cpu()
+    assert torch.equal(got[:rows], want[:rows]) and (got[rows:] == 7.0).all()
+    assert int(error) == (0x60001 if missing else 0)

@@ -56,7 +56,7 @@ __device__ __forceinline__ int lp_first_row(const int* q_start, const int* kv_st
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const uint4* __restrict__ pool, int64_t page_stride, int page_size, int num_pages, const int* __restrict__ block_table,
                      int table_stride, const int* __restrict__ q_start, const int* __restrict__ kv_start, const int* __restrict__ slots,
-                     uint4* __restrict__ latent, uint4* __restrict__ rotated, int rank8, int rot8, int* __restrict__ error_word) {
+                     uint4* __restrict__ latent, uint4* __restrict__ rotated, int rows, int rank8, int rot8, int* __restrict__ error_word) {
   pdl_wait();
   pdl_trigger();
   const int entry = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -75,6 +75,10 @@ latent_gather_kernel(const uint4* __restrict__ pool, int64_t page_stride, int pa
     const int r = r0 + i;
     const bool have = page[i] >= 0 && page[i] < num_pages;
     if (r < keys && !have && error_word && lane == 0) atomicExch(error_word, 0x30000 + entry);
+    if (first + r >= rows) {      // (the entries need more rows than there are: reported, nothing is written behind the last one)
+      if (error_word && lane == 0) atomicExch(error_word, 0x60000 + entry);
+      continue;
+    }
     const uint4* src = pool + (size_t)(have ? page[i] : 0) * page_stride + (size_t)(r % page_size) * pieces;
     for (int c = lane; c < pieces; c += 32) {
       const uint4 v = have ? src[c] : make_uint4(0u, 0u, 0u, 0u);
@@ -427,17 +431,18 @@ TIB_API int tib_latent_prefill_supports(int dim, int value_dim, int rank, int ro
 }
 
 // pool: this layer's pages of [page_size][rank + rot] bf16; latent [rows, rank] and rotated [rows, rot]: every entry's keys padded to a
-// multiple of 128 rows (zeros), entry after entry; rows: their sum, which must not be less than the entries need.
+// multiple of 128 rows (zeros), entry after entry; rows: how many there are.  What the entries need beyond that is reported in
+// error_word (0x60000 + entry) and not written.
 TIB_API int tib_latent_gather(const void* pool, int64_t page_stride, int page_size, int num_pages, const int* block_table, int table_stride,
                               const int* q_start, const int* kv_start, const int* slots, int n_entries, int max_kv_len, void* latent,
-                              void* rotated, int rank, int rot, int* error_word, cudaStream_t stream) {
+                              void* rotated, int rows, int rank, int rot, int* error_word, cudaStream_t stream) {
   if (n_entries == 0 || max_kv_len == 0) return TIB_OK;
-  if (!pool || !block_table || !q_start || !kv_start || !slots || !latent || !rotated || page_size < 1) return TIB_E_ARG;
+  if (!pool || !block_table || !q_start || !kv_start || !slots || !latent || !rotated || page_size < 1 || rows < 0) return TIB_E_ARG;
   if (rank % 8 || rot % 8 || page_stride % 8 || (((uintptr_t)pool | (uintptr_t)latent | (uintptr_t)rotated) & 15)) return TIB_E_ALIGN;
   if (n_entries > 65535) return TIB_E_SIZE;
   TIB_LAUNCH_DEPENDENT(latent_gather_kernel, dim3(ceil_div(max_kv_len, kLpTile) * (kLpTile / 32), n_entries), 256, 0, stream, (const uint4*)pool,
                        page_stride / 8, page_size, num_pages, block_table, table_stride, q_start, kv_start, slots, (uint4*)latent,
-                       (uint4*)rotated, rank / 8, rot / 8, error_word);
+                       (uint4*)rotated, rows, rank / 8, rot / 8, error_word);
   return TIB_OK;
 }
 

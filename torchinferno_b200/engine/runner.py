@@ -306,4 +306,4 @@ class ModelRunner:
         if word:
             self.cache.error_word.zero_()
             raise StepError(f"a kernel reported an error (code {word:#x}: 0x7c.... a bounded wait of a tcgen05 kernel ran out, "
-                            f"else a page id outside its pool); the step's result is invalid")
+                            f"else a page id outside its pool or a row outside its buffer); the step's result is invalid")

@@ -1032,20 +1032,21 @@ def latent_gather(keys: torch.Tensor, block_table: torch.Tensor, q_start: torch.
                   n_entries: int, max_kv_len: int, latent: torch.Tensor, rotated: torch.Tensor,
                   error_word: torch.Tensor | None = None) -> None:
     """The cached rows of every entry (its earlier tokens and this step's), dense: ``latent`` [rows, rank] and ``rotated``
-    [rows, rot]; an entry takes its length rounded up to LATENT_TILE rows, the last of them zeros."""
+    [rows, rot]; an entry takes its length rounded up to LATENT_TILE rows, the last of them zeros.
+    Entries that need more rows than there are get what is there, and an error is reported."""
     _need(latent, "latent", torch.bfloat16), _need(rotated, "rotated", torch.bfloat16)
     rank, rot = latent.shape[1], rotated.shape[1]
     for name, t in (("q_start", q_start), ("kv_start", kv_start), ("slots", slots), ("block_table", block_table)):
         _need(t, name, torch.int32)
     if keys.dtype != torch.bfloat16 or keys.dim() != 4 or keys.shape[1] != 1 or keys.shape[3] != rank + rot or keys.stride(3) != 1 \
-            or keys.stride(2) != rank + rot or latent.shape[0] != rotated.shape[0]:
+            or keys.stride(2) != rank + rot or latent.shape[0] != rotated.shape[0] or latent.shape[0] % LATENT_TILE:
         raise KernelError("latent_gather: pages or rows do not fit")
     if q_start.numel() < n_entries + 1 or kv_start.numel() < n_entries or slots.numel() < n_entries:
         raise KernelError("latent_gather: entry arrays are shorter than n_entries")
     _check("latent_gather", lib().tib_latent_gather(
         _ptr(keys), c_int64(keys.stride(0)), c_int(keys.shape[2]), c_int(keys.shape[0]), _ptr(block_table), c_int(block_table.stride(0)),
-        _ptr(q_start), _ptr(kv_start), _ptr(slots), c_int(n_entries), c_int(max_kv_len), _ptr(latent), _ptr(rotated), c_int(rank),
-        c_int(rot), _ptr(error_word), _stream()))
+        _ptr(q_start), _ptr(kv_start), _ptr(slots), c_int(n_entries), c_int(max_kv_len), _ptr(latent), _ptr(rotated), c_int(latent.shape[0]),
+        c_int(rank), c_int(rot), _ptr(error_word), _stream()))
 
 
 def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
