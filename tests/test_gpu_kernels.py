@@ -939,6 +939,38 @@ def test_linear_attention_forms_agree_with_the_recurrence(lens, heads, key_dim, 
     assert (as_ref(got_state) - want_state).abs().max() <= 2e-6 * want_state.abs().max()
 
 
+@pytest.mark.parametrize("lens, dim", [([300, 7, 193], 64), ([200, 450], 128), ([100, 20], 64)])      # (in runs, and in chunks)
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_linear_attention_keeps_what_is_not_finite_from_earlier_tokens(lens, dim, bad):
+    """One value of one request: only its own column of its head changes, from its own token on.  One key: only its head."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    n, heads, entries = sum(lens), 2, len(lens)
+    width = heads * dim
+    starts = [sum(lens[:i]) for i in range(entries + 1)]
+    decay = torch.tensor([0.9, 0.99], dtype=torch.float64)
+    powers = [dev((decay[:, None] ** torch.arange(most + 1, dtype=torch.float64)).float().contiguous())
+              for most in (ops.linear_attention_chunk(dim, dim), ops.linear_attention_run())]
+    rows, held = rnd(n, 3 * width, dtype=torch.bfloat16), rnd(entries, heads, dim, dim, seed=5)
+
+    def run(rows):
+        proj, state = dev(rows), dev(held.clone())
+        out = ops.linear_attention(proj[:, :width], proj[:, width:2 * width], proj[:, 2 * width:], torch.empty(n, width, device="cuda"), state,
+                                   powers[0], dev(torch.tensor(starts, dtype=torch.int32)), dev(torch.arange(entries, dtype=torch.int32)), entries, heads,
+                                   dim, dim, silu=False, max_q_len=max(lens), run_powers=powers[1])
+        return out.cpu(), state.cpu()
+
+    clean, clean_state = run(rows)
+    for t in (0, 5, lens[0] - 1, 66):
+        for column, hit in ((2 * width + dim + 3, slice(dim + 3, dim + 4)), (width + 7, slice(0, dim))):
+            broken = rows.clone()
+            broken[t, column] = bad
+            out, state = run(broken)
+            changed = torch.zeros(n, width, dtype=torch.bool)
+            changed[t:lens[0], hit] = True
+            assert torch.equal(out[~changed], clean[~changed]) and not torch.isfinite(out[changed]).any(), (t, column)
+            assert torch.equal(state[1:], clean_state[1:])
+
 
 # ------------------------------------------------------------------------------------------------- the experts' products
 @pytest.mark.parametrize("tokens, experts, top, k, n, act, by_pair, out_dtype", [

@@ -459,13 +459,14 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_pack(0.f, 0.f);
-  auto add = [&](const float4& av, const float* brow) {      // acc[i][.] += a[i] * b[.]
+  auto add = [&](const float4& av, const float* brow, int from) {      // acc[i][.] += a[i] * b[.] for i >= from
     ulonglong2 b[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) b[g] = *reinterpret_cast<const ulonglong2*>(brow + g * 64 + tx * 4);
     const float ai[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+      if (i < from) continue;
       const f32x2 aa = f2_pack(ai[i], ai[i]);
 #pragma unroll
       for (int g = 0; g < G; ++g) {
@@ -480,7 +481,7 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
     __syncthreads();
     if (d0 + SR < D) ask(d0 + SR);
 #pragma unroll 4
-    for (int d = 0; d < SR; ++d) add(*reinterpret_cast<const float4*>(qt + (d0 + d) * kLinPad + ty * 4), ss + d * TV);
+    for (int d = 0; d < SR; ++d) add(*reinterpret_cast<const float4*>(qt + (d0 + d) * kLinPad + ty * 4), ss + d * TV, 0);
     __syncthreads();
   }
 #pragma unroll
@@ -490,9 +491,13 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
 #pragma unroll
     for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_mul(ff, acc[i][g]);
   }
-  const int keys = min(n, (tid >> 5) * 8 + 8);               // (a warp holds eight tokens: later keys weigh nothing)
+  // a warp holds eight tokens: those before them count for all eight, those among them only for the tokens they come before (left
+  // out, not weighed with 0: an infinity or NaN must not reach an earlier token)
+  const int own = (tid >> 5) * 8, keys = min(n, own);
 #pragma unroll 4
-  for (int j = 0; j < keys; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV);
+  for (int j = 0; j < keys; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV, 0);
+  const int last = min(n, own + 8);
+  for (int j = own; j < last; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV, j - ty * 4);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     if (ty * 4 + i >= n) break;
