@@ -1048,6 +1048,39 @@ def test_scan_in_chunks_agrees_with_the_recurrence(lens, heads, head_dim, state,
         assert (as_ref(out) - ref).abs().max() <= 32 * 2.0 ** -23 * ref.abs().max()
 
 
+@pytest.mark.parametrize("lens, head_dim, state", [([300, 7, 129], 64, 128), ([140, 70], 32, 64)])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_scan_in_chunks_keeps_what_is_not_finite_from_earlier_tokens(lens, head_dim, state, bad):
+    """One number of x of one request: only its own column changes, from its own token on.  One of B: the tokens from its own on;
+    one of C: its own token alone."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, n, entries = 2, sum(lens), len(lens)
+    inner = heads * head_dim
+    xbc, dt = rnd(n, inner + 2 * state, dtype=torch.bfloat16), dev(rnd(n, heads, dtype=torch.bfloat16, seed=1))
+    bias, a_log, skip = dev(rnd(heads, seed=2) - 3.0), dev(rnd(heads, seed=3)), dev(rnd(heads, seed=4))
+    held, starts = rnd(entries, heads * state * head_dim, seed=5), [sum(lens[:i]) for i in range(entries + 1)]
+
+    def run(rows):
+        y, carried = torch.empty(n, inner, device="cuda"), dev(held.clone())
+        ops.ssd_scan(dev(rows), dt, 0, bias, a_log, skip, carried, dev(torch.tensor(starts, dtype=torch.int32)),
+                     dev(torch.arange(entries, dtype=torch.int32)), y, entries, heads=heads, groups=1, state_dim=state, head_dim=head_dim,
+                     max_q_len=max(lens))
+        return y.cpu(), carried.cpu()
+
+    clean, clean_state = run(xbc)
+    for t in (0, 5, 15, 16, 127, 128, lens[0] - 1):
+        for column, last, hit in ((head_dim + 3, lens[0], slice(head_dim + 3, head_dim + 4)), (inner + 9, lens[0], slice(0, inner)),
+                                  (inner + state + 9, t + 1, slice(0, inner))):
+            broken = xbc.clone()
+            broken[t, column] = bad
+            y, carried = run(broken)
+            changed = torch.zeros(n, inner, dtype=torch.bool)
+            changed[t:last, hit] = True
+            assert torch.equal(y[~changed], clean[~changed]) and not torch.isfinite(y[changed]).any(), (t, column)
+            assert torch.equal(carried[1:], clean_state[1:])
+
+
 @pytest.mark.parametrize("lens, channels, taps", [([1, 2, 3], 8, 4), ([16, 17, 1], 1032, 3), ([50, 2], 520, 2), ([40], 16, 4)])
 def test_short_convolution_by_eight_channels_has_the_plain_kernels_bits(lens, channels, taps):
     need_gpu()

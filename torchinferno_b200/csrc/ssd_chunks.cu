@@ -29,14 +29,7 @@ constexpr int kSsdRows = 32;            // rows of the state staged at a time
 
 __device__ __forceinline__ size_t ssd_first_chunk(int row0, int entry) { return (size_t)(row0 / kQ) + entry; }
 
-// v as three bf16 terms
-__device__ __forceinline__ void ssd_split(float v, __nv_bfloat16& hi, __nv_bfloat16& mid, __nv_bfloat16& lo) {
-  hi = __float2bfloat16_rn(v);
-  const float r = v - __bfloat162float(hi);
-  mid = __float2bfloat16_rn(r);
-  lo = __float2bfloat16_rn(r - __bfloat162float(mid));
-}
-// the same for a pair, packed (a in the low half)
+// a and b as three bf16 terms each, packed (a in the low half)
 __device__ __forceinline__ void ssd_split2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   const float2 hf = bf16x2_floats(h);
@@ -58,6 +51,13 @@ __device__ __forceinline__ void ssd_mma8(float (&d)[4], const uint32_t (&a)[4], 
 __device__ __forceinline__ void ssd_add(float (&sum)[4], const float (&step)[4]) {
 #pragma unroll
   for (int c = 0; c < 4; ++c) sum[c] += step[c];
+}
+
+// A packed pair without what is not finite (zeros in its place; odd says that there was some).
+__device__ __forceinline__ uint32_t ssd_finite2(uint32_t v, bool& odd) {
+  const uint32_t keep = ((v & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
+  odd |= keep != 0xffffffffu;
+  return v & keep;
 }
 
 // Step sizes and sums of log decays of a chunk's n tokens (tokens behind it: no step, the sum stays).  Called by the whole block;
@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
       ssd_add(s[1], step[2]);
     }
     uint32_t w[3][4];
+    bool odd = false;
 #pragma unroll
     for (int half = 0; half < 2; ++half)        // (tokens j0 + 8 half + 2 t4 and the next one)
 #pragma unroll
@@ -345,6 +346,10 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
     for (int j = 0; j < NT / 2; ++j) {
       uint32_t b[4];
       ldmatrix_x4_trans(b, xs + (j0 + ((lane >> 3) & 1) * 8 + (lane & 7)) * PS + j * 16 + ((lane >> 4) << 3));
+      if (j0 == m0) {      // (the tile of the warp's own tokens: a later one weighs 0, which must not meet an infinity or NaN)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) b[q] = ssd_finite2(b[q], odd);
+      }
       float step[2][4] = {};
 #pragma unroll
       for (int u = 2; u >= 0; --u) {
@@ -353,6 +358,29 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
       }
       ssd_add(acc[2 * j], step[0]);
       ssd_add(acc[2 * j + 1], step[1]);
+    }
+    if (__any_sync(0xffffffffu, odd)) {         // what was left out, for the tokens it does not come after
+#pragma unroll 1
+      for (int jj = 0; jj < 16; ++jj) {
+        const int from = (lane & ~3) | ((jj & 7) >> 1);      // (the lane that holds this token's weights)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          float weight = 0.f;
+#pragma unroll
+          for (int u = 2; u >= 0; --u) {
+            const uint32_t pair = __shfl_sync(0xffffffffu, jj < 8 ? w[u][r] : w[u][2 + r], from);
+            const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&pair));
+            weight += jj & 1 ? f.y : f.x;
+          }
+          if (j0 + jj > (r == 0 ? i0 : i1)) continue;
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            const float2 x = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(xs + (j0 + jj) * PS + t * 8 + 2 * t4));
+            if (!isfinite(x.x)) acc[t][2 * r] = fmaf(weight, x.x, acc[t][2 * r]);
+            if (!isfinite(x.y)) acc[t][2 * r + 1] = fmaf(weight, x.y, acc[t][2 * r + 1]);
+          }
+        }
+      }
     }
   }
   const float skip = a.d_skip[h];
