@@ -1081,6 +1081,28 @@ def test_scan_in_chunks_keeps_what_is_not_finite_from_earlier_tokens(lens, head_
             assert torch.equal(carried[1:], clean_state[1:])
 
 
+def test_scan_in_chunks_of_an_infinite_state():
+    """One infinite element of a request's state: its column is infinite from then on, as in the token-by-token walk."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, head_dim, state, n = 2, 64, 128, 200
+    inner = heads * head_dim
+    xbc, dt = dev(rnd(n, inner + 2 * state, dtype=torch.bfloat16)), dev(rnd(n, heads, dtype=torch.bfloat16, seed=1))
+    bias, a_log, skip = dev(rnd(heads, seed=2) - 6.0), dev(0.2 * rnd(heads, seed=3)), dev(rnd(heads, seed=4))
+    held = rnd(1, heads, state, head_dim, seed=5)
+    held[0, 1, 17, 5] = float("inf")
+    results = []
+    for longest in (n, None):      # (in chunks; token by token)
+        y, carried = torch.empty(n, inner, device="cuda"), dev(held.view(1, -1).clone())
+        ops.ssd_scan(xbc, dt, 0, bias, a_log, skip, carried, dev(torch.tensor([0, n], dtype=torch.int32)), dev(torch.zeros(1, dtype=torch.int32)), y, 1,
+                     heads=heads, groups=1, state_dim=state, head_dim=head_dim, max_q_len=longest)
+        results.append((y.cpu(), carried.cpu()))
+    for chunks, walk in zip(*results):
+        assert torch.isinf(walk).any() and torch.equal(torch.where(torch.isinf(walk), walk, 0.0), torch.where(torch.isfinite(chunks), 0.0, chunks))
+        fine = torch.isfinite(walk)
+        assert (chunks[fine] - walk[fine]).abs().max() <= 32 * 2.0 ** -23 * walk[fine].abs().max()      # (the bound of the finite states' test)
+
+
 @pytest.mark.parametrize("lens, channels, taps", [([1, 2, 3], 8, 4), ([16, 17, 1], 1032, 3), ([50, 2], 520, 2), ([40], 16, 4)])
 def test_short_convolution_by_eight_channels_has_the_plain_kernels_bits(lens, channels, taps):
     need_gpu()

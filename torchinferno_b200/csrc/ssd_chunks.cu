@@ -11,7 +11,8 @@
 // (the state, the weighted scores, the weighted x) enters its product as three bf16 terms, which hold all 24 bits of an fp32
 // number; F is summed in double precision and kept as two floats, so that differences of long sums keep their last bits.  The
 // tensor core's own sums are cut off rather than rounded, so only the 16 terms of a step (small ones first) are left to it, and
-// the steps are added as ordinary fp32 numbers.
+// the steps are added as ordinary fp32 numbers.  What is not finite stays with the tokens it concerns, as in the walk, though an
+// infinity may come out as NaN (where it meets a term or a decay of zero).
 //
 // The walk of ssd_scan_kernel spends five fp32 operations per state element and token twice over (two prompts of 1,366 and 682
 // tokens, 64 heads of 64 with a state of 128: 182 + 32 + 264 us, the fp32 pipe at 40 %).  Here a token costs its share of the
@@ -29,11 +30,14 @@ constexpr int kSsdRows = 32;            // rows of the state staged at a time
 
 __device__ __forceinline__ size_t ssd_first_chunk(int row0, int entry) { return (size_t)(row0 / kQ) + entry; }
 
-// a and b as three bf16 terms each, packed (a in the low half)
+// a and b as three bf16 terms each, packed (a in the low half).  What the first term cannot hold (an infinity; anything above
+// 3.39e38) is an infinity there, with nothing left for the others.
 __device__ __forceinline__ void ssd_split2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   const float2 hf = bf16x2_floats(h);
-  const float ra = a - hf.x, rb = b - hf.y;
+  float ra = a - hf.x, rb = b - hf.y;
+  ra = isfinite(hf.x) ? ra : 0.f;
+  rb = isfinite(hf.y) ? rb : 0.f;
   const __nv_bfloat162 m = __floats2bfloat162_rn(ra, rb);
   const float2 mf = bf16x2_floats(m);
   const __nv_bfloat162 l = __floats2bfloat162_rn(ra - mf.x, rb - mf.y);
