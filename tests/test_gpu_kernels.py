@@ -939,6 +939,40 @@ def test_linear_attention_forms_agree_with_the_recurrence(lens, heads, key_dim, 
     assert (as_ref(got_state) - want_state).abs().max() <= 2e-6 * want_state.abs().max()
 
 
+@pytest.mark.parametrize("dim, value_dim", [(64, 64), (128, 128), (128, 32), (64, 40)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_linear_attention_of_a_request_does_not_depend_on_its_neighbours(dim, value_dim, dtype):
+    """Portions of every form, alone and in one step, bit for bit; and the launches counted are those of the forms that occur."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    lens, heads = [1, 300, 40, 1, 192, 32, 193, 2], 2
+    n, entries, widths = sum(lens), len(lens), [heads * dim, heads * dim, heads * value_dim]
+    decay = torch.tensor([0.9, 0.99], dtype=torch.float64)
+    powers = [dev((decay[:, None] ** torch.arange(most + 1, dtype=torch.float64)).float().contiguous())
+              for most in (ops.linear_attention_chunk(dim, value_dim), ops.linear_attention_run())]
+    q, k, v = (dev(rnd(n, w, dtype=dtype, seed=i)) for i, w in enumerate(widths))
+    held, slots = dev(rnd(entries, heads, dim, value_dim, seed=5)), dev(torch.arange(entries, dtype=torch.int32))
+
+    def run(first, count, portions):
+        rows, part = slice(sum(lens[:first]), sum(lens[:first + count])), lens[first:first + count]
+        state, before = held.clone(), ops.launch_count()
+        starts = dev(torch.tensor([sum(part[:i]) for i in range(count + 1)], dtype=torch.int32))
+        out = ops.linear_attention(q[rows], k[rows], v[rows], torch.empty(sum(part), widths[2], device="cuda"), state, powers[0], starts,
+                                   slots[first:first + count].contiguous(), count, heads, dim, value_dim, silu=True, max_q_len=max(part),
+                                   run_powers=powers[1], portions={m: part.count(m) for m in part} if portions else None)
+        return out, state, ops.launch_count() - before
+
+    out, state, launches = run(0, entries, True)
+    out_unnamed, state_unnamed, _ = run(0, entries, False)
+    assert torch.equal(out, out_unnamed) and torch.equal(state, state_unnamed)
+    new_forms = value_dim % 32 == 0
+    assert launches == (1 if not new_forms else 5 if value_dim % 64 == 0 else 2)
+    for i, m in enumerate(lens):
+        alone, alone_state, launches = run(i, 1, True)
+        assert torch.equal(alone, out[sum(lens[:i]):sum(lens[:i + 1])]) and torch.equal(alone_state[i], state[i]), (i, m)
+        assert launches == (3 if m >= 193 and value_dim % 64 == 0 else 1)
+
+
 @pytest.mark.parametrize("lens, dim", [([300, 7, 193], 64), ([200, 450], 128), ([100, 20], 64)])      # (in runs, and in chunks)
 @pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
 def test_linear_attention_keeps_what_is_not_finite_from_earlier_tokens(lens, dim, bad):

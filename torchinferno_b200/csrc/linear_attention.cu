@@ -15,11 +15,13 @@
 // lambda^0 .. lambda^C come from the host as a table (made in double precision).  A single token is a chunk
 // of one.  State is read from and written back to the request's slot; a new request's slot is zero.
 //
-// Three ways to run that, chosen by sizes alone (tib_linear_attention):
+// Three ways to run that.  Every portion takes the one its own length and the layer's sizes name, whatever else is in the step
+// (tib_linear_attention launches each form that occurs over the whole batch, and a form's blocks leave the others' portions alone), so a
+// request's numbers do not depend on its neighbours:
 //   runs   (portions above 192 tokens, head sizes of 64 or 128) every run of 64 tokens makes its own sum L of decayed k v^T
 //          side by side, one thread per state element then folds S <- lambda^n S + L over a request's runs, and every run
 //          makes its outputs from its starting state: the serial chain is one fused multiply-add a run
-//   walk   (steps whose portions have at most 32 tokens) S in registers, token by token
+//   walk   (portions of at most 32 tokens) S in registers, token by token
 //   chunks (everything else) the block walk described above
 #include "common.cuh"
 
@@ -34,6 +36,7 @@ struct LinAttnArgs {
   int64_t ldq, ldk, ldv;  // row strides of q, k, v (elements)
   int heads, key_dim, value_dim, chunk, activation;
   int cols;               // value columns per block
+  int shortest, longest;  // the portions this launch takes (the others are another form's)
 };
 
 __device__ __forceinline__ float lin_act(float z, int activation) { return activation ? z / (1.f + expf(-z)) : z; }
@@ -56,7 +59,7 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   pdl_wait();
   pdl_trigger();
   const int row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
-  if (len <= 0) return;
+  if (len < a.shortest || len > a.longest) return;
   float* state = a.state + ((size_t)a.slots[entry] * a.heads + head) * D * a.value_dim + col0;      // row stride value_dim
   for (int e = threadIdx.x; e < D * V; e += blockDim.x) S[e] = state[(size_t)(e / V) * a.value_dim + e % V];
   for (int e = threadIdx.x; e <= C; e += blockDim.x) pw[e] = a.powers[head * (C + 1) + e];
@@ -221,7 +224,7 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 // half rounded as the scalar instruction rounds it), operands from shared memory in 16-byte loads without bank conflicts.
 // Everything stays fp32: activations, decay powers, scores, states and sums.
 constexpr int kLinRun = 64;
-constexpr int kLinRunsFrom = 193;          // the shortest longest portion that is cut into runs
+constexpr int kLinRunsFrom = 193;          // the shortest portion that is cut into runs
 constexpr int kLinPad = kLinRun + 4;       // row stride of the transposed q, k and scores
 
 struct LinRunArgs {
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(256, 2) lin_run_sums_kernel(const T* __restric
   const int tiles = a.value_dim / TV, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * TV;
   const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const int t0 = blockIdx.y * kLinRun;
-  if (t0 >= len) return;
+  if (t0 >= len || len < kLinRunsFrom) return;
   const int n = min(kLinRun, len - t0), tid = threadIdx.x;
   if (tid <= kLinRun) pw[tid] = a.powers[head * (kLinRun + 1) + tid];
   __syncthreads();
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(256) lin_fold_kernel(LinRunArgs a, int key_dim
   const int entry = blockIdx.y, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const size_t per_head = (size_t)key_dim * a.value_dim, width = per_head * a.heads;
   const size_t e = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
-  if (len <= 0 || e >= width) return;
+  if (len < kLinRunsFrom || e >= width) return;
   const float* pw = a.powers + (e / per_head) * (kLinRun + 1);
   const int runs = (len + kLinRun - 1) / kLinRun, last = len - (runs - 1) * kLinRun;
   const float whole = pw[kLinRun], part = pw[last];
@@ -388,7 +391,7 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   const int tiles = a.value_dim / TV, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * TV;
   const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const int t0 = blockIdx.y * kLinRun;
-  if (t0 >= len) return;
+  if (t0 >= len || len < kLinRunsFrom) return;
   const int n = min(kLinRun, len - t0), tid = threadIdx.x;
   const float* S = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.heads + head) * (size_t)D * a.value_dim + col0;
   constexpr int SV = SR * TV / 4 / 256;                      // 16-byte pieces of a tile of S a thread fetches
@@ -532,7 +535,7 @@ lin_walk_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
   pdl_trigger();
   const int tiles = a.value_dim / 32, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * 32;
   const int entry = blockIdx.y, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
-  if (len <= 0) return;
+  if (len <= 0 || len > kLinWalk) return;
   const int tid = threadIdx.x, cg = tid & 7, rt = tid >> 3;
   float* S = a.state + ((size_t)a.slots[entry] * a.heads + head) * (size_t)D * a.value_dim + col0 + cg * 4;
   float4 s[ROWS];
@@ -624,7 +627,7 @@ TIB_API int tib_linear_attention_chunk(int key_dim, int value_dim) {
   return 0;
 }
 
-// Tokens of a run, the longest portion the walk takes, and the shortest longest portion that is cut into runs.
+// Tokens of a run, the longest portion the walk takes, and the shortest that is cut into runs.
 TIB_API int tib_linear_attention_run() { return kLinRun; }
 TIB_API int tib_linear_attention_walk() { return kLinWalk; }
 TIB_API int tib_linear_attention_runs_from() { return kLinRunsFrom; }
@@ -632,14 +635,18 @@ TIB_API int tib_linear_attention_runs_from() { return kLinRunsFrom; }
 // q, k: [tokens, >= heads * key_dim] and v: [tokens, >= heads * value_dim] with row strides ldq, ldk, ldv (they may be
 // slices of one wider row); out: [tokens, heads * value_dim] fp32; state: [slots, heads, key_dim, value_dim] fp32;
 // powers: [heads, chunk + 1] fp32, powers[h][m] = lambda_h^m; activation: 0 none, 1 silu on q, k and v.
-// max_q_len: the longest entry of the step, 0 where it is not known (then, or without run_powers, the chunk kernel runs).
+// forms: which portions occur, 1: of at most tib_linear_attention_walk() tokens, 4: of tib_linear_attention_runs_from() and more, 2:
+// between them; 0 where it is not known (then, or without run_powers, the chunk kernel runs them all).  n_chunked: how many portions lie
+// between them (at most; the chunk kernel shares a head's columns out by it).  max_q_len: the longest portion.
 // run_powers: [heads, run + 1] fp32 likewise, or null.  run_state: scratch of run_capacity >= tokens / run + n_entries times
-// heads * key_dim * value_dim floats for portions of tib_linear_attention_runs_from() tokens and more, or null.
+// heads * key_dim * value_dim floats for portions of tib_linear_attention_runs_from() tokens and more, or null (they run in chunks then).
+// launches: takes the number of kernels launched.
 TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, int64_t ldq, int64_t ldk, int64_t ldv,
                                  float* out, float* state, const float* powers, const int* q_start, const int* slots,
                                  int n_entries, int heads, int key_dim, int value_dim, int chunk, int activation, int dtype,
-                                 int tokens, int max_q_len, const float* run_powers, float* run_state, int64_t run_capacity,
-                                 cudaStream_t stream) {
+                                 int tokens, int max_q_len, int forms, int n_chunked, const float* run_powers, float* run_state, int64_t run_capacity,
+                                 int* launches, cudaStream_t stream) {
+  *launches = 0;
   if (n_entries == 0) return TIB_OK;
   if (!q || !k || !v || !out || !state || !powers || !q_start || !slots) return TIB_E_ARG;
   if (heads < 1 || key_dim < 1 || value_dim < 1 || chunk < 1 || chunk > 32 || n_entries > 65535) return TIB_E_SIZE;
@@ -651,31 +658,45 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   const int64_t size = dtype == TIB_F32 ? 4 : 2;
   const bool aligned = (ldq * size) % 16 == 0 && (ldk * size) % 16 == 0 && (ldv * size) % 16 == 0 &&
                        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)run_state) & 15) == 0;
-  if (run_powers && max_q_len > 0 && (key_dim == 64 || key_dim == 128) && value_dim % 32 == 0 && aligned &&
-      (dtype == TIB_F32 || dtype == TIB_BF16)) {
+  int shortest = 1;      // what is left for the chunk kernel
+  int longest = 0x7fffffff, chunked = n_entries;
+  if (run_powers && forms && (key_dim == 64 || key_dim == 128) && value_dim % 32 == 0 && aligned && (dtype == TIB_F32 || dtype == TIB_BF16)) {
     LinRunArgs r;
     r.q_start = q_start; r.slots = slots; r.powers = run_powers; r.state = state; r.run_state = run_state; r.out = out;
     r.ldq = ldq; r.ldk = ldk; r.ldv = ldv; r.heads = heads; r.value_dim = value_dim; r.activation = activation;
-    if (max_q_len <= kLinWalk)
-      return dtype == TIB_F32 ? launch_lin_walk<float>(q, k, v, r, key_dim, n_entries, stream)
-                              : launch_lin_walk<__nv_bfloat16>(q, k, v, r, key_dim, n_entries, stream);
-    if (max_q_len >= kLinRunsFrom && run_state && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535) {
+    if (forms & 1) {
+      const int status = dtype == TIB_F32 ? launch_lin_walk<float>(q, k, v, r, key_dim, n_entries, stream)
+                                          : launch_lin_walk<__nv_bfloat16>(q, k, v, r, key_dim, n_entries, stream);
+      if (status != TIB_OK) return status;
+      *launches += 1;
+    }
+    shortest = kLinWalk + 1;
+    const bool runs = run_state && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535;
+    if ((forms & 4) && runs) {
 #define TIB_LIN_GO(T)                                                                                             \
   (key_dim == 64 ? (value_dim % 128 == 0 ? launch_lin_runs<T, 64, 128>(q, k, v, r, n_entries, max_q_len, stream)    \
                                          : launch_lin_runs<T, 64, 64>(q, k, v, r, n_entries, max_q_len, stream))    \
                  : (value_dim % 128 == 0 ? launch_lin_runs<T, 128, 128>(q, k, v, r, n_entries, max_q_len, stream)   \
                                          : launch_lin_runs<T, 128, 64>(q, k, v, r, n_entries, max_q_len, stream)))
-      return dtype == TIB_F32 ? TIB_LIN_GO(float) : TIB_LIN_GO(__nv_bfloat16);
+      const int status = dtype == TIB_F32 ? TIB_LIN_GO(float) : TIB_LIN_GO(__nv_bfloat16);
 #undef TIB_LIN_GO
+      if (status != TIB_OK) return status;
+      *launches += 3;
+    }
+    if (runs) longest = kLinRunsFrom - 1;
+    if (runs || !(forms & 4)) {
+      if (!(forms & 2)) return TIB_OK;
+      chunked = n_chunked > 0 && n_chunked < n_entries ? n_chunked : n_entries;
     }
   }
   LinAttnArgs a;
+  a.shortest = shortest; a.longest = longest;
   a.q_start = q_start; a.slots = slots; a.powers = powers; a.state = state; a.out = out;
   a.ldq = ldq; a.ldk = ldk; a.ldv = ldv;
   a.heads = heads; a.key_dim = key_dim; a.value_dim = value_dim; a.chunk = chunk; a.activation = activation;
   // runs of value columns: halve them (down to 8) while the grid has fewer than two blocks per SM
   int cols = value_dim;
-  while (cols >= 16 && cols % 2 == 0 && (int64_t)heads * n_entries * (value_dim / cols) < 2 * 148) cols /= 2;
+  while (cols >= 16 && cols % 2 == 0 && (int64_t)heads * chunked * (value_dim / cols) < 2 * 148) cols /= 2;
   a.cols = cols;
   const size_t smem = lin_attn_smem(key_dim, cols, chunk);
   if (smem > 227 * 1024) return TIB_E_SMEM;
@@ -698,5 +719,6 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   } else {
     return TIB_E_DTYPE;
   }
+  *launches += 1;
   return TIB_OK;
 }

@@ -13,6 +13,7 @@ Device arrays (int32, views into one uploaded buffer):
 """
 from __future__ import annotations
 
+from collections import Counter
 from dataclasses import dataclass, field
 from typing import Hashable, Sequence
 
@@ -56,6 +57,7 @@ class StepBatch:
     n_single: int = 0             # entries that bring one token
     n_multi: int = 0              # entries that bring more
     entries: list[EntryPlacement] = field(default_factory=list)
+    portions: dict[int, int] = field(default_factory=dict)      # how many entries bring that many tokens (empty: not known)
     h2d_bytes: int = 0
 
 
@@ -111,6 +113,6 @@ def build_batch(placements: list[EntryPlacement], tokens: list[Sequence[int]], w
         n_logits=len(logit_rows), max_q_len=max((p.q_len for p in placements), default=0),
         max_kv_len=max((p.kv_start + p.q_len for p in placements), default=0),
         n_single=sum(1 for p in placements if p.q_len == 1), n_multi=sum(1 for p in placements if p.q_len > 1),
-        entries=placements, h2d_bytes=total * 4)
+        entries=placements, portions=dict(Counter(p.q_len for p in placements)), h2d_bytes=total * 4)
     updates = [(views[8 + 2 * i], views[9 + 2 * i]) for i in range(len(table_updates))]
     return batch, updates

@@ -47,7 +47,7 @@ class _DecodeGraph:
         self.batch = StepBatch(
             token_ids=self.token_ids, positions=self.positions, token_slot=self.slots, q_start=self.q_start,
             kv_start=self.positions, slots=self.slots, logit_rows=self.logit_rows, logit_slots=self.slots, n_tokens=n, n_entries=n,
-            n_logits=n, max_q_len=1, max_kv_len=max_kv_len, n_single=n, n_multi=0, entries=[])
+            n_logits=n, max_q_len=1, max_kv_len=max_kv_len, n_single=n, n_multi=0, entries=[], portions={1: n})
         self.graph: torch.cuda.CUDAGraph | None = None
         self.logits: torch.Tensor | None = None
         self.launches = 0          # kernels of this library inside the graph

@@ -7,6 +7,7 @@ not take) raises :class:`KernelError`; nothing falls back to another path.
 from __future__ import annotations
 
 import ctypes
+from collections.abc import Mapping
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
@@ -887,14 +888,16 @@ def linear_attention_chunk(key_dim: int, value_dim: int) -> int:
     return int(lib().tib_linear_attention_chunk(c_int(key_dim), c_int(value_dim)))
 
 
-_linear_sizes: tuple[int, int] | None = None
+_linear_sizes: tuple[int, int, int] | None = None
 
 
-def _linear_attention_sizes() -> tuple[int, int]:
-    """(tokens of a run, the shortest longest portion of a step that is cut into runs); asked of the library once."""
+def _linear_attention_sizes() -> tuple[int, int, int]:
+    """(tokens of a run, the longest portion that is walked token by token, the shortest that is cut into runs); asked of the
+    library once."""
     global _linear_sizes
     if _linear_sizes is None:
-        _linear_sizes = int(lib().tib_linear_attention_run()), int(lib().tib_linear_attention_runs_from())
+        _linear_sizes = (int(lib().tib_linear_attention_run()), int(lib().tib_linear_attention_walk()),
+                         int(lib().tib_linear_attention_runs_from()))
     return _linear_sizes
 
 
@@ -909,11 +912,12 @@ LINEAR_ATTENTION_SCRATCH = 1 << 30      # bytes of run states a call may take (2
 def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
                      powers: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, n_entries: int, heads: int,
                      key_dim: int, value_dim: int, *, silu: bool, max_q_len: int = 0,
-                     run_powers: torch.Tensor | None = None) -> torch.Tensor:
+                     run_powers: torch.Tensor | None = None, portions: Mapping[int, int] | None = None) -> torch.Tensor:
     """o_t = S_t^T q_t with S_t = decay * S_(t-1) + k_t v_t^T per head, over the ragged batch; ``state``
     [slots, heads, key_dim, value_dim] (fp32) is read and left updated; ``powers`` [heads, chunk + 1] holds decay^m.
     With the step's longest entry and ``run_powers`` [heads, linear_attention_run() + 1] (decay^m again) long portions run in
-    pieces side by side and single tokens by a kernel of their own, where those kernels take the head sizes."""
+    pieces side by side and single tokens by a kernel of their own, where those kernels take the head sizes; which kernel takes an
+    entry depends on its own length alone.  ``portions`` (length: how many entries have it) spares launches over nothing."""
     for name, t, width in (("q", q, heads * key_dim), ("k", k, heads * key_dim), ("v", v, heads * value_dim)):
         _rows_of(t, name, width)
         if t.dtype != q.dtype:
@@ -925,21 +929,28 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
         raise KernelError("linear_attention: out, state or powers do not fit the head sizes")
     if q_start.numel() < n_entries + 1 or slots.numel() < n_entries:
         raise KernelError("linear_attention: entry arrays are shorter than n_entries")
-    run_state, capacity = None, 0
+    run_state, capacity, forms, chunked = None, 0, 0, 0
     if run_powers is not None:
-        run, runs_from = _linear_attention_sizes()
+        run, walk, runs_from = _linear_attention_sizes()
         _need(run_powers, "run_powers", torch.float32)
         if run_powers.shape != (heads, run + 1):
             raise KernelError("linear_attention: run_powers has the wrong shape")
-        if max_q_len >= runs_from and key_dim in (64, 128) and value_dim % 64 == 0:
+        if max_q_len > 0:
+            for length in portions or {1: 1, min(max_q_len, walk + 1): 1, max_q_len: 1}:
+                forms |= 1 if length <= walk else 2 if length < runs_from else 4
+        if portions:
+            chunked = sum(count for length, count in portions.items() if walk < length < runs_from)
+        if forms & 4 and key_dim in (64, 128) and value_dim % 64 == 0:
             capacity = q.shape[0] // run + n_entries
             if capacity * heads * key_dim * value_dim * 4 <= LINEAR_ATTENTION_SCRATCH:
                 run_state = torch.empty(capacity * heads * key_dim * value_dim, dtype=torch.float32, device=q.device)
+    launches = c_int(0)
     _check("linear_attention", lib().tib_linear_attention(
         _ptr(q), _ptr(k), _ptr(v), c_int64(q.stride(0)), c_int64(k.stride(0)), c_int64(v.stride(0)), _ptr(out), _ptr(state),
         _ptr(powers), _ptr(q_start), _ptr(slots), c_int(n_entries), c_int(heads), c_int(key_dim), c_int(value_dim),
-        c_int(chunk), c_int(1 if silu else 0), c_int(_code(q.dtype)), c_int(q.shape[0]), c_int(max_q_len), _ptr(run_powers),
-        _ptr(run_state), c_int64(capacity), _stream()))
+        c_int(chunk), c_int(1 if silu else 0), c_int(_code(q.dtype)), c_int(q.shape[0]), c_int(max_q_len), c_int(forms),
+        c_int(chunked), _ptr(run_powers), _ptr(run_state), c_int64(capacity), ctypes.byref(launches), _stream()))
+    count_launches(launches.value - 1)      # (_check counted one)
     return out
 
 

@@ -83,7 +83,8 @@ class DecayLinearAttention(Mixer):
         q, k, v = proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + vv]
         mixed = torch.empty((n, vv), dtype=torch.float32, device=x.device)
         ops.linear_attention(q, k, v, mixed, ctx.state, self.powers, batch.q_start, batch.slots, batch.n_entries, self.heads,
-                             self.key_dim, self.value_dim, silu=self.activation == "silu", max_q_len=batch.max_q_len, run_powers=self.run_powers)
+                             self.key_dim, self.value_dim, silu=self.activation == "silu", max_q_len=batch.max_q_len,
+                             run_powers=self.run_powers, portions=batch.portions)
         if self.gate:
             rows = torch.empty((n, vv), dtype=x.dtype, device=x.device)
             ops.sigmoid_gate(mixed, proj[:, 2 * qk + vv:], rows, self.norm_weight, self.eps)
