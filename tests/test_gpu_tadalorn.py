@@ -880,3 +880,38 @@ def test_prompts_on_keys_and_values_made_for_the_step(heads, dim, rot, vdim, ran
     for r in x:
         err = _row_error(outs[torch.bfloat16][r].double(), outs[torch.float32][r].double())
         assert err.max() <= 0.03, (r, int(err.argmax()), float(err.max()))      # (the bound of the layer's other tests in bfloat16)
+
+
+@pytest.mark.parametrize("order", ["abcd", "cadb", "acbd", "dcba"])
+def test_a_latent_portion_takes_its_own_form_beside_any_others(order, monkeypatch):
+    """A prompt of 300 tokens (a) and one of 20 (b) run on keys and values made for the step, a single token (c) and a portion of three
+    (d) folded, whatever lies before, between and behind them; all against the same layer in 32 bits."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    from torchinferno_b200.parts.base import PartSpec, build_part
+    from torchinferno_b200.weights.random_init import random_tensor
+    params = {"hidden_size": 64, "heads": 2, "dim": 64, "rot_dim": 32, "value_dim": 64, "kv_rank": 64, "scale": 0.07, "rot_base": 3000.0, "eps": 1e-5,
+              "gate": True, "sink": False}
+    lens = {"a": 300, "b": 20, "c": 1, "d": 3}
+    x = {r: torch.randn(n, 64, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16) for i, (r, n) in enumerate((("a", 300), ("b", 220), ("c", 202), ("d", 204)))}
+    steps = [[(r, 200) for r in "bcd"], [(r, lens[r]) for r in order], [("c", 1), ("d", 1)]]
+    outs, calls = {}, []
+    for name in ("latent_attention", "latent_prefill"):
+        inner = getattr(ops, name)
+        monkeypatch.setattr(ops, name, lambda *a, inner=inner, name=name, **k: calls.append((name, a)) or inner(*a, **k))
+    for dtype in (torch.float32, torch.bfloat16):
+        mixer = build_part("mixer", PartSpec("latent_attention", params), dtype=dtype, device=CUDA)
+        _bind(mixer, {ws.name: random_tensor(ws, 4, dtype=torch.bfloat16) for ws in mixer.weight_specs()}, dtype, "mix.")
+        cache = _cache_for(mixer, dtype, 16, 64, 4, 600)
+        for r in "bcda":
+            cache.open(r)
+        calls.clear()
+        outs[dtype] = _run_steps(mixer, cache, steps, {r: t.to(dtype) for r, t in x.items()})
+    forms = [name for name, _ in calls]
+    assert forms[0] == "latent_prefill" and forms[-1] == "latent_attention"
+    mixed = calls[1:-1]
+    assert [name for name, _ in mixed].count("latent_attention") == 1
+    assert next(a for name, a in mixed if name == "latent_attention")[8] == 3      # (its longest portion is d)
+    for r in lens:
+        err = _row_error(outs[torch.bfloat16][r].double(), outs[torch.float32][r].double())
+        assert err.max() <= 0.03, (r, int(err.argmax()), float(err.max()))      # (the bound of the layer's other tests in bfloat16)

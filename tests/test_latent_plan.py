@@ -1,0 +1,37 @@
+"""How a step is shared out between the two forms of the latent attention."""
+import pytest
+
+from torchinferno_b200.engine.batch import EntryPlacement
+from torchinferno_b200.parts.latent_attention import _plan
+
+
+def _entries(pairs):
+    row, out = 0, []
+    for i, (new, past) in enumerate(pairs):
+        out.append(EntryPlacement(i, i, row, new, past))
+        row += new
+    return out
+
+
+@pytest.mark.parametrize("pairs, groups, short", [
+    ([(1, 4000)] * 3, None, None),
+    ([(15, 0), (16, 0)], ((1, 2, 128),), (0, 1)),
+    ([(1, 4000)] * 8 + [(2048, 0)], ((8, 9, 2048),), (0, 8)),                          # (decoding contexts are not unfolded)
+    ([(512, 0)] + [(1, 4000)] * 64, ((0, 1, 512),), (1, 65)),                          # (many of them do not fold the prompt)
+    ([(109, 20), (1, 127), (30, 0)], ((0, 3, 512),), (1, 2)),                          # (a small one between is carried along)
+    ([(109, 20), (1, 1000), (30, 0)], ((0, 1, 256), (2, 3, 128)), (1, 2)),
+    ([(900, 0), (900, 0), (900, 0)], ((0, 2, 2048), (2, 3, 1024)), None),              # (as many together as there is room for)
+    ([(64, 3000), (64, 100)], ((1, 2, 256),), (0, 1))])                                # (one that needs more room than there is)
+def test_portions_by_their_own_length(pairs, groups, short):
+    entries = _entries(pairs)
+    plan = _plan(entries, 16, 2048)
+    if groups is None:
+        assert plan is None
+        return
+    assert plan.groups == groups and plan.short == short
+    first, last = entries[groups[0][0]], entries[groups[-1][1] - 1]
+    assert plan.long_tokens == (first.q_start, last.q_start + last.q_len)
+    if short:
+        inside = [e for i, e in enumerate(entries) if short[0] <= i < short[1] and not any(a <= i < b and e.q_len >= 16 for a, b, _ in groups)]
+        assert plan.short_tokens == (entries[short[0]].q_start, entries[short[1] - 1].q_start + entries[short[1] - 1].q_len)
+        assert (plan.short_q_len, plan.short_kv_len) == (max(e.q_len for e in inside), max(e.q_len + e.kv_start for e in inside))

@@ -153,6 +153,7 @@ struct LatentAttnArgs {
   const float* sink;          // [heads] or null: exp(sink[h]) is added to the softmax's denominator
   int head_chunk, q_tile;
   __nv_bfloat16* merged;      // where the merged rows of split contexts go in bf16, or null (then to `out`)
+  int row_base, longest;      // the step's token whose row comes first in `folded` and `out`; longer portions are left alone
   int* error_word;
   // a step of single tokens may cut every context into `n_splits` runs of `blocks_per_split` key blocks, one block
   // each: they leave their running maximum, sum and unnormalised output in `partial` [tokens, heads, n_splits,
@@ -182,11 +183,11 @@ latent_attention_kernel(const float* __restrict__ folded, const T* __restrict__ 
   const int entry = blockIdx.y;
   const int h0 = blockIdx.z * a.head_chunk;
   const int hc = min(a.head_chunk, a.heads - h0);
-  const int row0 = a.q_start[entry];
-  const int q_len = a.q_start[entry + 1] - row0;
+  const int row0 = a.q_start[entry] - a.row_base;
+  const int q_len = a.q_start[entry + 1] - a.row_base - row0;
   const int split = a.partial ? blockIdx.x : 0;
   const int t0 = a.partial ? 0 : blockIdx.x * a.q_tile;
-  if (t0 >= q_len) return;
+  if (t0 >= q_len || q_len > a.longest) return;
   const int nt = min(a.q_tile, q_len - t0);
   const int nrows = nt * hc;
   const int pos0 = a.kv_start[entry] + t0;
@@ -363,12 +364,12 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
   pdl_wait();
   pdl_trigger();
   const int entry = blockIdx.y;
-  const int row0 = a.q_start[entry];
-  const int q_len = a.q_start[entry + 1] - row0;
+  const int row0 = a.q_start[entry] - a.row_base;
+  const int q_len = a.q_start[entry + 1] - a.row_base - row0;
   const int total_rows = q_len * a.heads;
   const int split = a.partial ? blockIdx.x : 0;
   const int r0 = a.partial ? blockIdx.z * RB : blockIdx.x * RB;           // first (token, head) row of the block
-  if (r0 >= total_rows) return;
+  if (r0 >= total_rows || q_len > a.longest) return;
   const int nrows = min(RB, total_rows - r0);
   const int kv0 = a.kv_start[entry];
   const int last_pos = kv0 + (r0 + nrows - 1) / a.heads;                  // highest key any row of the block reads
@@ -676,11 +677,13 @@ TIB_API int tib_latent_attention_splits(int n_entries, int heads, int max_kv_len
 // n_splits > 1 (a step of single tokens only, contexts of at most max_kv_len keys): partial [tokens, heads, n_splits, 2 + rank].
 // merged: with n_splits > 1, [tokens, heads, rank] bf16 that takes the rows instead of out, or null.
 // sink: [heads] fp32 or null.  force_simt: the CUDA-core kernel also where the tensor-core one takes the shape.
+// row_base: the token (as q_start counts them) that folded's and out's first row belongs to.  Portions of more than max_q_len tokens
+// are left alone: their rows of out keep what they hold.
 TIB_API int tib_latent_attention(const float* folded, const void* pool, float* out, const int* q_start, const int* kv_start,
                                  const int* slots, const int* block_table, int table_stride, int n_entries, int max_q_len,
                                  int heads, int rank, int rot, int page_size, int64_t page_stride, int num_pages, float scale,
                                  const float* sink, float* partial, int n_splits, int max_kv_len, int force_simt, int* error_word, int dtype,
-                                 void* merged, cudaStream_t stream) {
+                                 void* merged, int row_base, cudaStream_t stream) {
   if (n_entries == 0 || max_q_len == 0) return TIB_OK;
   if (!folded || !pool || (!out && !(merged && n_splits > 1)) || !q_start || !kv_start || !slots || !block_table) return TIB_E_ARG;
   if (heads < 1 || rank < 1 || rot < 0 || page_size < 1 || rank > 512 || n_entries > 65535) return TIB_E_SIZE;
@@ -689,6 +692,7 @@ TIB_API int tib_latent_attention(const float* folded, const void* pool, float* o
   a.heads = heads; a.rank = rank; a.width = rank + rot; a.page_size = page_size; a.num_pages = num_pages;
   a.page_stride = page_stride; a.scale = scale; a.sink = sink; a.error_word = error_word;
   a.partial = nullptr; a.n_splits = 1; a.blocks_per_split = 0; a.merged = (__nv_bfloat16*)merged;
+  a.row_base = row_base; a.longest = max_q_len;
   if (n_splits > 1) {
     if (!partial || max_q_len != 1 || max_kv_len < 1) return TIB_E_ARG;
     a.partial = partial; a.n_splits = n_splits;

@@ -39,6 +39,7 @@ struct LpArgs {
   int gate_per_head;
   __nv_bfloat16* out;              // [tokens, heads, value_dim]
   int heads, dim;
+  int shortest;                    // shorter portions are left alone
   float scale_log2;
   int* error_word;
 };
@@ -129,7 +130,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int row0 = a.q_start[entry];
   const int q_len = a.q_start[entry + 1] - row0;
   const int t0 = (gridDim.z - 1 - blockIdx.z) * kLpTile;      // longest first
-  if (t0 >= q_len) return;
+  if (t0 >= q_len || q_len < a.shortest) return;
   const int nt = min(kLpTile, q_len - t0);
   const int pos0 = a.kv_start[entry] + t0, last_pos = pos0 + nt - 1;
   const int n_tiles = last_pos / kLpTile + 1;
@@ -448,9 +449,10 @@ TIB_API int tib_latent_gather(const void* pool, int64_t page_stride, int page_si
 
 // q: [tokens, heads, dim + rot] (row stride ldq) with the rotation applied; kv: [rows, heads * (dim + value_dim)], the heads' keys, then
 // their values; rotated: [rows, rot]; gate: rows of heads (per head) or heads * value_dim numbers (row stride ld_gate) or null;
-// out: [tokens, heads, value_dim].  All bf16; sink: [heads] fp32 or null; scale > 0.
+// out: [tokens, heads, value_dim].  All bf16; sink: [heads] fp32 or null; scale > 0.  Portions of fewer than `shortest` tokens are left
+// alone (their keys have their rows all the same).
 TIB_API int tib_latent_prefill(const void* q, int64_t ldq, const void* kv, const void* rotated, int rows, const int* q_start,
-                               const int* kv_start, int n_entries, int max_q_len, int n_tokens, int heads, int dim, int value_dim, int rot,
+                               const int* kv_start, int n_entries, int max_q_len, int shortest, int n_tokens, int heads, int dim, int value_dim, int rot,
                                float scale, const float* sink, const void* gate, int64_t ld_gate, int gate_per_head, void* out,
                                int* error_word, cudaStream_t stream) {
   if (n_entries == 0 || max_q_len == 0) return TIB_OK;
@@ -468,7 +470,7 @@ TIB_API int tib_latent_prefill(const void* q, int64_t ldq, const void* kv, const
   if (rc != TIB_OK) return rc;
   LpArgs a;
   a.q_start = q_start; a.kv_start = kv_start; a.sink = sink; a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate;
-  a.gate_per_head = gate_per_head; a.out = (__nv_bfloat16*)out; a.heads = heads; a.dim = dim; a.scale_log2 = scale * 1.4426950408889634f;
+  a.gate_per_head = gate_per_head; a.out = (__nv_bfloat16*)out; a.heads = heads; a.dim = dim; a.shortest = shortest; a.scale_log2 = scale * 1.4426950408889634f;
   a.error_word = error_word;
   if (dim == 128)
     return value_dim == 128 ? launch_lp<2, 2>(map_q, map_kv, map_r, a, n_entries, max_q_len, stream)

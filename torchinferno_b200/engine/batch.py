@@ -59,6 +59,7 @@ class StepBatch:
     entries: list[EntryPlacement] = field(default_factory=list)
     portions: dict[int, int] = field(default_factory=dict)      # how many entries bring that many tokens (empty: not known)
     h2d_bytes: int = 0
+    plans: dict = field(default_factory=dict)      # what the parts worked out from the entries, for their other layers
 
 
 def build_batch(placements: list[EntryPlacement], tokens: list[Sequence[int]], wants: list[Sequence[int]],

@@ -990,13 +990,14 @@ def latent_append(dkv: torch.Tensor, q: torch.Tensor, folded: torch.Tensor | Non
 def latent_attention(folded: torch.Tensor, keys: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor, kv_start: torch.Tensor,
                      slots: torch.Tensor, block_table: torch.Tensor, n_entries: int, max_q_len: int, heads: int, rank: int,
                      rot: int, scale: float, error_word: torch.Tensor | None = None, max_kv_len: int = 0,
-                     force_simt: bool = False, sink: torch.Tensor | None = None, merged: torch.Tensor | None = None) -> torch.Tensor:
+                     force_simt: bool = False, sink: torch.Tensor | None = None, merged: torch.Tensor | None = None, first_row: int = 0) -> torch.Tensor:
     """Causal attention of folded queries [tokens, heads, rank + rot] (fp32) over paged latent rows; the value of a
     key is its first ``rank`` elements.  ``out``: [tokens, heads, rank] fp32.  A step of single tokens only
     (``max_q_len`` 1) that names the longest context (``max_kv_len``) cuts every context into runs that go to blocks of
     their own and are merged by a second kernel.  ``sink`` [heads] fp32: exp(sink) is added to the softmax's denominator.
     ``merged``: a bfloat16 tensor of ``out``'s shape that takes the rows, rounded once, when contexts were cut (``out`` is then left
-    as it is); the tensor that holds the rows is returned."""
+    as it is); the tensor that holds the rows is returned.  ``first_row``: the step's token that row 0 of ``folded`` and ``out`` belongs
+    to, where they hold a part of the step's.  Portions longer than ``max_q_len`` are left alone."""
     _need(folded, "folded", torch.float32), _need(out, "out", torch.float32)
     if merged is not None:
         _need(merged, "merged", torch.bfloat16)
@@ -1025,7 +1026,7 @@ def latent_attention(folded: torch.Tensor, keys: torch.Tensor, out: torch.Tensor
         c_int(block_table.stride(0)), c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(rank), c_int(rot),
         c_int(keys.shape[2]), c_int64(keys.stride(0)), c_int(keys.shape[0]), c_float(scale), _ptr(sink), _ptr(partial), c_int(splits),
         c_int(max_kv_len), c_int(int(force_simt)), _ptr(error_word), c_int(_code(keys.dtype)),
-        _ptr(merged if splits > 1 else None), _stream()))
+        _ptr(merged if splits > 1 else None), c_int(first_row), _stream()))
     if partial is not None:
         count_launches(1)
     return out if merged is None or splits == 1 else merged
@@ -1061,12 +1062,13 @@ def latent_gather(keys: torch.Tensor, block_table: torch.Tensor, q_start: torch.
 
 
 def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
-                   kv_start: torch.Tensor, n_entries: int, max_q_len: int, heads: int, dim: int, value_dim: int, scale: float,
+                   kv_start: torch.Tensor, n_entries: int, max_q_len: int, heads: int, dim: int, value_dim: int, scale: float, shortest: int = 1,
                    gate: torch.Tensor | None = None, gate_per_head: bool = False, sink: torch.Tensor | None = None,
                    error_word: torch.Tensor | None = None) -> torch.Tensor:
     """Causal attention of rotated queries [tokens, heads * (dim + rot)] over the rows :func:`latent_gather` laid out: ``kv`` [rows,
     heads * (dim + value_dim)] holds all heads' keys and then all heads' values, ``rotated`` the key part the heads share.
-    ``out`` [tokens, heads, value_dim] is multiplied by sigmoid(gate) when one is given, element by element or head by head."""
+    ``out`` [tokens, heads, value_dim] is multiplied by sigmoid(gate) when one is given, element by element or head by head.
+    Portions of fewer than ``shortest`` tokens are left alone."""
     rot = rotated.shape[1]
     _rows_of(q, "q", heads * (dim + rot)), _need(kv, "kv", torch.bfloat16), _need(rotated, "rotated", torch.bfloat16), _need(out, "out", torch.bfloat16)
     for name, t in (("q_start", q_start), ("kv_start", kv_start)):
@@ -1084,7 +1086,7 @@ def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out
             raise KernelError("latent_prefill: sink holds one number per head")
     _check("latent_prefill", lib().tib_latent_prefill(
         _ptr(q), c_int64(q.stride(0)), _ptr(kv), _ptr(rotated), c_int(kv.shape[0]), _ptr(q_start), _ptr(kv_start), c_int(n_entries),
-        c_int(max_q_len), c_int(n), c_int(heads), c_int(dim), c_int(value_dim), c_int(rot), c_float(scale), _ptr(sink), _ptr(gate),
+        c_int(max_q_len), c_int(shortest), c_int(n), c_int(heads), c_int(dim), c_int(value_dim), c_int(rot), c_float(scale), _ptr(sink), _ptr(gate),
         c_int64(gate.stride(0) if gate is not None else 0), c_int(int(gate_per_head)), _ptr(out), _ptr(error_word), _stream()))
     return out
 

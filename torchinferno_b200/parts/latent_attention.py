@@ -13,16 +13,18 @@ values).  The queries are folded through W_uk (a_j = W_uk_j^T q_j, one batched p
 latent rows with their first kv_rank elements as values, and W_uv is applied to the result (another batched
 product): the same arithmetic regrouped, in which no per-head key or value is ever made.  Scores, softmax
 weights, their sums and the folded queries are fp32.  In bfloat16, prompt portions of some length run the other way round:
-the step's per-head keys and values are made from the cached rows by one product and used once (:meth:`_unfolded_rows`).  Rotary pairs are (2i, 2i + 1) (``pairing="interleaved"``) or
+their per-head keys and values are made from the cached rows by one product and used once (:class:`_Plan`).  Rotary pairs are (2i, 2i + 1) (``pairing="interleaved"``) or
 (i, i + rot_dims / 2) (``pairing="half"``) over the first ``rot_dims`` elements of the rotated part, angle = position *
 rot_base^(-2i / rot_dims).
 """
 from __future__ import annotations
 
-from typing import Mapping
+from dataclasses import dataclass
+from typing import Mapping, Sequence
 
 import torch
 
+from torchinferno_b200.engine.batch import EntryPlacement
 from torchinferno_b200.kernels import ops
 from torchinferno_b200.kernels.gemm import LinearWeight, linear
 from torchinferno_b200.parts.base import CacheSpec, LayerContext, Mixer, WeightSpec, register_part
@@ -109,34 +111,75 @@ class LatentAttention(Mixer):
 
     # The unfolded form multiplies 2 (dim + value_dim) rank numbers a head and key once, and saves some two thirds of the folded
     # kernel's products on every (query, key) pair, which run at a tenth of the library's rate: it wins from about six
-    # queries a key on average, and is taken from sixteen (the layer on two prompts of 1,667 and 833 tokens, 16 heads: 1,226 us
-    # folded, 165 unfolded; error against 64 bits 0.0048 and 0.0045).
+    # queries a key, and is taken from sixteen (the layer on two prompts of 1,667 and 833 tokens, 16 heads: 1,226 us
+    # folded, 165 unfolded; error against 64 bits 0.0048 and 0.0045).  A portion's own length decides, whatever else is in the step.
     UNFOLD_QUERIES = 16
-    UNFOLD_BYTES = 1 << 30      # the most that a step's keys and values may take
+    UNFOLD_BYTES = 1 << 30      # the most that keys and values made at a time may take
+
+    def _plan(self, batch) -> "_Plan | None":
+        """Which entries of the step run on keys and values made for it; None: none, or the entries are not known."""
+        if self.unfold is None or batch.n_multi == 0 or len(batch.entries) != batch.n_entries:
+            return None
+        row_bytes = 2 * (self.heads * (self.dim + self.value_dim) + self.kv_rank + self.rot_dim)
+        key = ("latent", self.UNFOLD_QUERIES, self.UNFOLD_BYTES // row_bytes)
+        if key not in batch.plans:
+            batch.plans[key] = _plan(batch.entries, *key[1:])
+        return batch.plans[key]
 
     def _unfolded_rows(self, batch) -> int:
-        """Rows of keys and values to make for this step, 0 where the folded form is to run."""
-        if self.unfold is None or batch.n_multi == 0 or len(batch.entries) != batch.n_entries:
-            return 0
-        keys = sum(e.kv_start + e.q_len for e in batch.entries)
-        pairs = sum(e.q_len * (e.kv_start + e.q_len) for e in batch.entries)
-        rows = sum(-(-(e.kv_start + e.q_len) // ops.LATENT_TILE) * ops.LATENT_TILE for e in batch.entries)
-        size = 2 * rows * (self.heads * (self.dim + self.value_dim) + self.kv_rank + self.rot_dim)
-        return rows if pairs >= self.UNFOLD_QUERIES * keys and size <= self.UNFOLD_BYTES else 0
+        """Rows of keys and values to make for this step, 0 where the folded form is to run throughout."""
+        plan = self._plan(batch)
+        return sum(rows for _, _, rows in plan.groups) if plan else 0
 
-    def _forward_unfolded(self, rows: int, q: torch.Tensor, dkv: torch.Tensor, gate: torch.Tensor | None, ctx: LayerContext) -> torch.Tensor:
-        kv, batch, n, h = ctx.kv, ctx.batch, q.shape[0], self.heads
-        ops.latent_append(dkv, q, None, kv.keys if kv.writes else None, batch.positions, batch.token_slot, kv.block_table,
-                          self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, self.kv_rank, self.rot_dim, ctx.error_word,
+    def _unfolded(self, plan: "_Plan", q: torch.Tensor, dkv: torch.Tensor, gate: torch.Tensor | None, out: torch.Tensor, ctx: LayerContext) -> None:
+        """The portions of the plan's groups, on keys and values made for them."""
+        kv, batch, h = ctx.kv, ctx.batch, self.heads
+        tokens = slice(*plan.long_tokens)
+        ops.latent_append(dkv[tokens], q[tokens], None, kv.keys if kv.writes else None, batch.positions[tokens], batch.token_slot[tokens],
+                          kv.block_table, self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, self.kv_rank, self.rot_dim,
+                          ctx.error_word, half_pairs=self.half_pairs)
+        for first, end, rows in plan.groups:
+            latent = torch.empty((rows, self.kv_rank), dtype=q.dtype, device=q.device)
+            rotated = torch.empty((rows, self.rot_dim), dtype=q.dtype, device=q.device)
+            q_start, kv_start, slots = batch.q_start[first:end + 1], batch.kv_start[first:end], batch.slots[first:end]
+            entries = batch.entries[first:end]
+            ops.latent_gather(kv.keys, kv.block_table, q_start, kv_start, slots, end - first, max(e.kv_start + e.q_len for e in entries),
+                              latent, rotated, ctx.error_word)
+            ops.latent_prefill(q, linear(latent, self.unfold), rotated, out, q_start, kv_start, end - first, max(e.q_len for e in entries),
+                               h, self.dim, self.value_dim, self.scale, self.UNFOLD_QUERIES, gate, self.gate_per_head, self.sink, ctx.error_word)
+
+    def _folded(self, q: torch.Tensor, dkv: torch.Tensor, gate: torch.Tensor | None, heads_out: torch.Tensor, ctx: LayerContext,
+                entries: slice, first_row: int, max_q_len: int, max_kv_len: int) -> None:
+        """Portions of at most ``max_q_len`` tokens among these entries, whose tokens the rows given are, from the step's
+        ``first_row`` on."""
+        kv, batch, n, h, c, r = ctx.kv, ctx.batch, q.shape[0], self.heads, self.kv_rank, self.rot_dim
+        width, tokens = c + r, slice(first_row, first_row + n)
+        q_start, kv_start, slots = batch.q_start[entries.start:entries.stop + 1], batch.kv_start[entries], batch.slots[entries]
+        folded = torch.empty((n, h, width), dtype=torch.float32, device=q.device)
+        ops.latent_append(dkv, q, folded, kv.keys if kv.writes else None, batch.positions[tokens], batch.token_slot[tokens], kv.block_table,
+                          self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, c, r, ctx.error_word,
                           half_pairs=self.half_pairs)
-        latent = torch.empty((rows, self.kv_rank), dtype=q.dtype, device=q.device)
-        rotated = torch.empty((rows, self.rot_dim), dtype=q.dtype, device=q.device)
-        ops.latent_gather(kv.keys, kv.block_table, batch.q_start, batch.kv_start, batch.slots, batch.n_entries, batch.max_kv_len, latent,
-                          rotated, ctx.error_word)
-        out = torch.empty((n, h, self.value_dim), dtype=q.dtype, device=q.device)
-        ops.latent_prefill(q, linear(latent, self.unfold), rotated, out, batch.q_start, batch.kv_start, batch.n_entries, batch.max_q_len,
-                           h, self.dim, self.value_dim, self.scale, gate, self.gate_per_head, self.sink, ctx.error_word)
-        return linear(out.view(n, h * self.value_dim), self.o_weight)
+        q_plain = q.as_strided((n, h, self.dim), (q.stride(0), self.dim + r, 1))
+        if q.dtype == torch.float32:
+            for j in range(h):
+                ops.gemm_f32(q_plain[:, j], self.uk_weight[j], folded[:, j, :c])
+        else:
+            ops.library_gemm_batched(q_plain, self.uk_weight, folded[:, :, :c], w_kn=True)
+        latent_out = torch.empty((n, h, c), dtype=torch.float32, device=q.device)
+        rows = torch.empty((n, h, c), dtype=q.dtype, device=q.device) if q.dtype != torch.float32 else None
+        mixed = ops.latent_attention(folded, kv.keys, latent_out, q_start, kv_start, slots, kv.block_table,
+                                     slots.shape[0], max_q_len, h, c, r, self.scale, ctx.error_word, max_kv_len=max_kv_len,
+                                     sink=self.sink, merged=rows, first_row=first_row)
+        if q.dtype == torch.float32:
+            for j in range(h):
+                ops.gemm_f32(latent_out[:, j], self.uv_weight[j], heads_out[:, j])
+        else:
+            if mixed is not rows:
+                ops.cast(mixed, rows)
+            ops.library_gemm_batched(rows, self.uv_weight, heads_out, w_kn=False)
+        if gate is not None:
+            flat = heads_out.view(n, h * self.value_dim)
+            ops.sigmoid_gate(flat, gate, flat, group=self.value_dim if self.gate_per_head else 1)
 
     def forward(self, x: torch.Tensor, ctx: LayerContext) -> torch.Tensor:
         kv, batch = ctx.kv, ctx.batch
@@ -152,38 +195,52 @@ class LatentAttention(Mixer):
             q = linear(latent_q, self.uq_weight)
         gates = (h if self.gate_per_head else h * self.value_dim) if self.gate else 0
         gate = proj[:, q_width + width:q_width + width + gates] if self.gate else None
-        rows = self._unfolded_rows(batch) if x.dtype == torch.bfloat16 else 0
-        # (the kernels copy rows from 16-byte boundaries; a projection of an odd width leaves the gate's rows off them)
-        if rows and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and kv.keys.stride(0) % 8 == 0 and kv.keys.data_ptr() % 16 == 0 \
-                and (gate is None or self.gate_per_head or gate.data_ptr() % 16 == 0):
-            return self._forward_unfolded(rows, q, dkv, gate, ctx)
-        folded = torch.empty((n, h, width), dtype=torch.float32, device=x.device)
-        ops.latent_append(dkv, q, folded, kv.keys if kv.writes else None, batch.positions, batch.token_slot, kv.block_table,
-                          self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, c, r, ctx.error_word,
-                          half_pairs=self.half_pairs)
-        q_plain = q.as_strided((n, h, self.dim), (q.stride(0), self.dim + r, 1))
-        if x.dtype == torch.float32:
-            for j in range(h):
-                ops.gemm_f32(q_plain[:, j], self.uk_weight[j], folded[:, j, :c])
-        else:
-            ops.library_gemm_batched(q_plain, self.uk_weight, folded[:, :, :c], w_kn=True)
-        latent_out = torch.empty((n, h, c), dtype=torch.float32, device=x.device)
-        rows = torch.empty((n, h, c), dtype=x.dtype, device=x.device) if x.dtype != torch.float32 else None
-        mixed = ops.latent_attention(folded, kv.keys, latent_out, batch.q_start, batch.kv_start, batch.slots, kv.block_table,
-                                     batch.n_entries, batch.max_q_len, h, c, r, self.scale, ctx.error_word, max_kv_len=batch.max_kv_len,
-                                     sink=self.sink, merged=rows)
         heads_out = torch.empty((n, h, self.value_dim), dtype=x.dtype, device=x.device)
-        if x.dtype == torch.float32:
-            for j in range(h):
-                ops.gemm_f32(latent_out[:, j], self.uv_weight[j], heads_out[:, j])
+        # (the kernels copy rows from 16-byte boundaries; a projection of an odd width leaves the gate's rows off them)
+        plan = self._plan(batch) if x.dtype == torch.bfloat16 and self._unfolded_rows(batch) else None
+        if plan and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and kv.keys.stride(0) % 8 == 0 and kv.keys.data_ptr() % 16 == 0 \
+                and (gate is None or self.gate_per_head or gate.data_ptr() % 16 == 0):
+            if plan.short:      # (first: where long portions lie between, their rows are written here too, and again below)
+                rows = slice(*plan.short_tokens)
+                self._folded(q[rows], dkv[rows], None if gate is None else gate[rows], heads_out[rows], ctx, slice(*plan.short), rows.start,
+                             plan.short_q_len, plan.short_kv_len)
+            self._unfolded(plan, q, dkv, gate, heads_out, ctx)
         else:
-            if mixed is not rows:
-                ops.cast(mixed, rows)
-            ops.library_gemm_batched(rows, self.uv_weight, heads_out, w_kn=False)
-        heads_out = heads_out.view(n, h * self.value_dim)
-        if self.gate:
-            ops.sigmoid_gate(heads_out, gate, heads_out, group=self.value_dim if self.gate_per_head else 1)
-        return linear(heads_out, self.o_weight)
+            self._folded(q, dkv, gate, heads_out, ctx, slice(0, batch.n_entries), 0, batch.max_q_len, batch.max_kv_len)
+        return linear(heads_out.view(n, h * self.value_dim), self.o_weight)
+
+
+@dataclass(frozen=True)
+class _Plan:
+    """How a step is shared out between the two forms."""
+    groups: tuple[tuple[int, int, int], ...]      # entries first .. end - 1 whose keys and values are made together, and their rows
+    long_tokens: tuple[int, int]                  # the tokens from the first to the last of the groups' entries
+    short: tuple[int, int] | None                 # the entries from the first to the last that stay folded, and their tokens
+    short_tokens: tuple[int, int]
+    short_q_len: int                              # their longest portion and context
+    short_kv_len: int
+
+
+def _plan(entries: Sequence[EntryPlacement], queries: int, most_rows: int) -> _Plan | None:
+    """Portions of at least ``queries`` tokens run on keys and values made for the step, unless their own keys alone need more than
+    ``most_rows`` rows.  Neighbours share a product, across short portions too where these add no more rows than there are."""
+    padded = [-(-(e.kv_start + e.q_len) // ops.LATENT_TILE) * ops.LATENT_TILE for e in entries]
+    long = [i for i, e in enumerate(entries) if e.q_len >= queries and padded[i] <= most_rows]
+    if not long:
+        return None
+    groups = []
+    for i in long:
+        between = sum(padded[groups[-1][1]:i]) if groups else 0
+        if groups and between <= groups[-1][2] and groups[-1][2] + between + padded[i] <= most_rows:
+            groups[-1] = (groups[-1][0], i + 1, groups[-1][2] + between + padded[i])
+        else:
+            groups.append((i, i + 1, padded[i]))
+    taken = set(long)
+    short = [i for i in range(len(entries)) if i not in taken]
+    tokens = lambda first, last: (entries[first].q_start, entries[last].q_start + entries[last].q_len)
+    return _Plan(tuple(groups), tokens(long[0], long[-1]), (short[0], short[-1] + 1) if short else None,
+                 tokens(short[0], short[-1]) if short else (0, 0), max((entries[i].q_len for i in short), default=0),
+                 max((entries[i].kv_start + entries[i].q_len for i in short), default=0))
 
 
 register_part("mixer", "latent_attention", LatentAttention)
