@@ -915,3 +915,37 @@ def test_a_latent_portion_takes_its_own_form_beside_any_others(order, monkeypatc
     for r in lens:
         err = _row_error(outs[torch.bfloat16][r].double(), outs[torch.float32][r].double())
         assert err.max() <= 0.03, (r, int(err.argmax()), float(err.max()))      # (the bound of the layer's other tests in bfloat16)
+
+
+@pytest.mark.parametrize("room", [1, 700_000, 1_200_000])
+def test_latent_prompts_in_little_room(room, monkeypatch):
+    """Keys and values made for one entry and some heads at a time: as with room for all, to the last bit of the products' sums."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    from torchinferno_b200.parts.base import PartSpec, build_part
+    from torchinferno_b200.parts.latent_attention import LatentAttention
+    from torchinferno_b200.weights.random_init import random_tensor
+    params = {"hidden_size": 64, "heads": 5, "dim": 64, "rot_dim": 32, "value_dim": 128, "kv_rank": 64, "scale": 0.07, "rot_base": 3000.0, "eps": 1e-5,
+              "gate": "head", "sink": True}
+    mixer = build_part("mixer", PartSpec("latent_attention", params), dtype=torch.bfloat16, device=CUDA)
+    _bind(mixer, {ws.name: random_tensor(ws, 4, dtype=torch.bfloat16) for ws in mixer.weight_specs()}, torch.bfloat16, "mix.")
+    x = {r: torch.randn(n, 64, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16) for i, (r, n) in enumerate((("a", 590), ("b", 41), ("c", 130)))}
+    outs, sizes = [], []
+    inner = ops.latent_prefill
+    monkeypatch.setattr(ops, "latent_prefill", lambda *a, **k: sizes.append(a[1].shape) or inner(*a, **k))
+    for _ in range(2):
+        cache = _cache_for(mixer, torch.bfloat16, 16, 128, 4, 600)
+        for r in x:
+            cache.open(r)
+        outs.append(_run_steps(mixer, cache, [[("a", 300), ("b", 1), ("c", 130)], [("b", 40), ("a", 290)]], x))
+        if len(outs) == 1:
+            assert [s for s in sizes] == [(768, 960), (768, 960)]
+            sizes.clear()
+            monkeypatch.setattr(LatentAttention, "UNFOLD_BYTES", room)
+    for rows, width in sizes:
+        assert width == 192 or 2 * rows * (width + 96) <= room
+    assert len(sizes) > 2
+    for r in x:
+        # (the library may cut its sums otherwise for another number of features or rows: a last bit of a key, value or row)
+        err = _row_error(outs[1][r].double(), outs[0][r].double())
+        assert err.max() <= 0.01, (r, int(err.argmax()), float(err.max()))

@@ -21,7 +21,7 @@ def _entries(pairs):
     ([(109, 20), (1, 127), (30, 0)], ((0, 3, 512),), (1, 2)),                          # (a small one between is carried along)
     ([(109, 20), (1, 1000), (30, 0)], ((0, 1, 256), (2, 3, 128)), (1, 2)),
     ([(900, 0), (900, 0), (900, 0)], ((0, 2, 2048), (2, 3, 1024)), None),              # (as many together as there is room for)
-    ([(64, 3000), (64, 100)], ((1, 2, 256),), (0, 1))])                                # (one that needs more room than there is)
+    ([(64, 3000), (64, 100)], ((0, 1, 3072), (1, 2, 256)), None)])                     # (one that needs more room than there is)
 def test_portions_by_their_own_length(pairs, groups, short):
     entries = _entries(pairs)
     plan = _plan(entries, 16, 2048)

@@ -3,7 +3,7 @@
 // The cache holds one row per token: the normed latent c (rank wide) and the rotated key part r all heads share.  For single tokens
 // the folded form (latent_attention.cu) reads that row once for all heads.  A prompt pays for it: every head multiplies keys of
 // rank + rot and values of rank numbers.  Here the step's keys and values are made once from the cached rows,
-//     K_j = W_uk_j c,   V_j = W_uv_j c        (one library product over all heads, [keys, heads * (dim + value_dim)])
+//     K_j = W_uk_j c,   V_j = W_uv_j c        (one library product over some or all heads, [keys, heads * (dim + value_dim)])
 // and attention runs at its own head sizes, a quarter of the products at rank 512, heads of 128 and 64 rotated.
 //
 //   latent_gather    the cached rows of every entry, dense: latents [rows, rank] and rotated parts [rows, rot]; an entry's rows
@@ -38,7 +38,7 @@ struct LpArgs {
   int64_t ld_gate;
   int gate_per_head;
   __nv_bfloat16* out;              // [tokens, heads, value_dim]
-  int heads, dim;
+  int heads, dim, head0;           // head0: the first of the launch's heads
   int shortest;                    // shorter portions are left alone
   float scale_log2;
   int* error_word;
@@ -124,7 +124,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - base));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.x, entry = blockIdx.y;
+  const int own = blockIdx.x, head = a.head0 + own, entry = blockIdx.y;      // own: among the heads that kv holds
   // (the first block may be placed while the kernel before drains: the entries' arrays were uploaded before the step began,
   // what the step's kernels write is only touched behind pdl_wait below)
   const int row0 = a.q_start[entry];
@@ -183,11 +183,11 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (values) {
           mbar_expect_tx(v_full(s), L::kV);
 #pragma unroll
-          for (int i = 0; i < DV; ++i) tma_load_2d(v_s(s) + i * kLpSub, &map_kv, a.heads * a.dim + head * D + i * 64, row, v_full(s));
+          for (int i = 0; i < DV; ++i) tma_load_2d(v_s(s) + i * kLpSub, &map_kv, own * (a.dim + D) + a.dim + i * 64, row, v_full(s));
         } else {
           mbar_expect_tx(k_full(s), L::kK);
 #pragma unroll
-          for (int i = 0; i < DQ; ++i) tma_load_2d(k_s(s) + i * kLpSub, &map_kv, head * a.dim + i * 64, row, k_full(s));
+          for (int i = 0; i < DQ; ++i) tma_load_2d(k_s(s) + i * kLpSub, &map_kv, own * (a.dim + D) + i * 64, row, k_full(s));
           tma_load_2d(k_s(s) + DQ * kLpSub, &map_r, 0, row, k_full(s));      // (rot below 64: the box's last columns are zeros, as Q's are)
         }
       }
@@ -412,12 +412,12 @@ static int lp_map(CUtensorMap* map, const void* ptr, int rank, const cuuint64_t*
 }
 
 template <int DQ, int DV>
-static int launch_lp(const CUtensorMap& map_q, const CUtensorMap& map_kv, const CUtensorMap& map_r, const LpArgs& a, int n_entries,
+static int launch_lp(const CUtensorMap& map_q, const CUtensorMap& map_kv, const CUtensorMap& map_r, const LpArgs& a, int n_heads, int n_entries,
                      int max_q_len, cudaStream_t stream) {
   auto kern = latent_prefill_kernel<DQ, DV>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LpSmem<DQ, DV>::kTotal);
   if (e != cudaSuccess) return (int)e;
-  TIB_LAUNCH_DEPENDENT(kern, dim3(a.heads, n_entries, ceil_div(max_q_len, kLpTile)), kLpThreads, (LpSmem<DQ, DV>::kTotal), stream, map_q, map_kv,
+  TIB_LAUNCH_DEPENDENT(kern, dim3(n_heads, n_entries, ceil_div(max_q_len, kLpTile)), kLpThreads, (LpSmem<DQ, DV>::kTotal), stream, map_q, map_kv,
                        map_r, a);
   return TIB_OK;
 }
@@ -447,22 +447,22 @@ TIB_API int tib_latent_gather(const void* pool, int64_t page_stride, int page_si
   return TIB_OK;
 }
 
-// q: [tokens, heads, dim + rot] (row stride ldq) with the rotation applied; kv: [rows, heads * (dim + value_dim)], the heads' keys, then
-// their values; rotated: [rows, rot]; gate: rows of heads (per head) or heads * value_dim numbers (row stride ld_gate) or null;
+// q: [tokens, heads, dim + rot] (row stride ldq) with the rotation applied; kv: [rows, n_heads * (dim + value_dim)], key and value of the
+// heads head0 .. head0 + n_heads - 1, head by head, which are the ones this call works; rotated: [rows, rot]; gate: rows of heads (per head) or heads * value_dim numbers (row stride ld_gate) or null;
 // out: [tokens, heads, value_dim].  All bf16; sink: [heads] fp32 or null; scale > 0.  Portions of fewer than `shortest` tokens are left
 // alone (their keys have their rows all the same).
 TIB_API int tib_latent_prefill(const void* q, int64_t ldq, const void* kv, const void* rotated, int rows, const int* q_start,
-                               const int* kv_start, int n_entries, int max_q_len, int shortest, int n_tokens, int heads, int dim, int value_dim, int rot,
+                               const int* kv_start, int n_entries, int max_q_len, int shortest, int n_tokens, int heads, int head0, int n_heads, int dim, int value_dim, int rot,
                                float scale, const float* sink, const void* gate, int64_t ld_gate, int gate_per_head, void* out,
                                int* error_word, cudaStream_t stream) {
   if (n_entries == 0 || max_q_len == 0) return TIB_OK;
   if (!q || !kv || !rotated || !q_start || !kv_start || !out || rows < 1 || !(scale > 0.f)) return TIB_E_ARG;
-  if (!tib_latent_prefill_supports(dim, value_dim, 8, rot) || heads < 1 || n_entries > 65535 || ceil_div(max_q_len, kLpTile) > 65535) return TIB_E_SIZE;
+  if (!tib_latent_prefill_supports(dim, value_dim, 8, rot) || heads < 1 || head0 < 0 || n_heads < 1 || head0 > heads - n_heads || n_entries > 65535 || ceil_div(max_q_len, kLpTile) > 65535) return TIB_E_SIZE;
   if (ldq % 8 || (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)rotated | (uintptr_t)out) & 15)) return TIB_E_ALIGN;
   if (gate && !gate_per_head && (ld_gate % 8 || ((uintptr_t)gate & 15))) return TIB_E_ALIGN;
   CUtensorMap map_q, map_kv, map_r;
   const cuuint64_t qd[3] = {(cuuint64_t)(dim + rot), (cuuint64_t)heads, (cuuint64_t)n_tokens}, qs[2] = {(cuuint64_t)(dim + rot) * 2, (cuuint64_t)ldq * 2};
-  const cuuint64_t width = (cuuint64_t)heads * (dim + value_dim);
+  const cuuint64_t width = (cuuint64_t)n_heads * (dim + value_dim);
   const cuuint64_t kd[2] = {width, (cuuint64_t)rows}, ks[1] = {width * 2}, rd[2] = {(cuuint64_t)rot, (cuuint64_t)rows}, rs[1] = {(cuuint64_t)rot * 2};
   int rc = lp_map(&map_q, q, 3, qd, qs);
   if (rc == TIB_OK) rc = lp_map(&map_kv, kv, 2, kd, ks);
@@ -470,11 +470,11 @@ TIB_API int tib_latent_prefill(const void* q, int64_t ldq, const void* kv, const
   if (rc != TIB_OK) return rc;
   LpArgs a;
   a.q_start = q_start; a.kv_start = kv_start; a.sink = sink; a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate;
-  a.gate_per_head = gate_per_head; a.out = (__nv_bfloat16*)out; a.heads = heads; a.dim = dim; a.shortest = shortest; a.scale_log2 = scale * 1.4426950408889634f;
+  a.gate_per_head = gate_per_head; a.out = (__nv_bfloat16*)out; a.heads = heads; a.dim = dim; a.head0 = head0; a.shortest = shortest; a.scale_log2 = scale * 1.4426950408889634f;
   a.error_word = error_word;
   if (dim == 128)
-    return value_dim == 128 ? launch_lp<2, 2>(map_q, map_kv, map_r, a, n_entries, max_q_len, stream)
-                            : launch_lp<2, 1>(map_q, map_kv, map_r, a, n_entries, max_q_len, stream);
-  return value_dim == 128 ? launch_lp<1, 2>(map_q, map_kv, map_r, a, n_entries, max_q_len, stream)
-                          : launch_lp<1, 1>(map_q, map_kv, map_r, a, n_entries, max_q_len, stream);
+    return value_dim == 128 ? launch_lp<2, 2>(map_q, map_kv, map_r, a, n_heads, n_entries, max_q_len, stream)
+                            : launch_lp<2, 1>(map_q, map_kv, map_r, a, n_heads, n_entries, max_q_len, stream);
+  return value_dim == 128 ? launch_lp<1, 2>(map_q, map_kv, map_r, a, n_heads, n_entries, max_q_len, stream)
+                          : launch_lp<1, 1>(map_q, map_kv, map_r, a, n_heads, n_entries, max_q_len, stream);
 }

@@ -1063,10 +1063,11 @@ def latent_gather(keys: torch.Tensor, block_table: torch.Tensor, q_start: torch.
 
 def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
                    kv_start: torch.Tensor, n_entries: int, max_q_len: int, heads: int, dim: int, value_dim: int, scale: float, shortest: int = 1,
-                   gate: torch.Tensor | None = None, gate_per_head: bool = False, sink: torch.Tensor | None = None,
+                   first_head: int = 0, gate: torch.Tensor | None = None, gate_per_head: bool = False, sink: torch.Tensor | None = None,
                    error_word: torch.Tensor | None = None) -> torch.Tensor:
     """Causal attention of rotated queries [tokens, heads * (dim + rot)] over the rows :func:`latent_gather` laid out: ``kv`` [rows,
-    heads * (dim + value_dim)] holds all heads' keys and then all heads' values, ``rotated`` the key part the heads share.
+    n * (dim + value_dim)] holds key and value of the n heads from ``first_head`` on, head by head, which are the ones worked here, and
+    ``rotated`` the key part the heads share.
     ``out`` [tokens, heads, value_dim] is multiplied by sigmoid(gate) when one is given, element by element or head by head.
     Portions of fewer than ``shortest`` tokens are left alone."""
     rot = rotated.shape[1]
@@ -1074,7 +1075,8 @@ def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out
     for name, t in (("q_start", q_start), ("kv_start", kv_start)):
         _need(t, name, torch.int32)
     n = q.shape[0]
-    if q.dtype != torch.bfloat16 or out.numel() != n * heads * value_dim or kv.shape != (rotated.shape[0], heads * (dim + value_dim)):
+    if q.dtype != torch.bfloat16 or out.numel() != n * heads * value_dim or kv.dim() != 2 or kv.shape[0] != rotated.shape[0] or kv.shape[1] % (dim + value_dim) \
+            or first_head + kv.shape[1] // (dim + value_dim) > heads:
         raise KernelError("latent_prefill: shapes or types do not fit")
     if gate is not None:
         _rows_of(gate, "gate", heads if gate_per_head else heads * value_dim)
@@ -1086,7 +1088,8 @@ def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out
             raise KernelError("latent_prefill: sink holds one number per head")
     _check("latent_prefill", lib().tib_latent_prefill(
         _ptr(q), c_int64(q.stride(0)), _ptr(kv), _ptr(rotated), c_int(kv.shape[0]), _ptr(q_start), _ptr(kv_start), c_int(n_entries),
-        c_int(max_q_len), c_int(shortest), c_int(n), c_int(heads), c_int(dim), c_int(value_dim), c_int(rot), c_float(scale), _ptr(sink), _ptr(gate),
+        c_int(max_q_len), c_int(shortest), c_int(n), c_int(heads), c_int(first_head), c_int(kv.shape[1] // (dim + value_dim)),
+        c_int(dim), c_int(value_dim), c_int(rot), c_float(scale), _ptr(sink), _ptr(gate),
         c_int64(gate.stride(0) if gate is not None else 0), c_int(int(gate_per_head)), _ptr(out), _ptr(error_word), _stream()))
     return out
 

@@ -100,11 +100,11 @@ class LatentAttention(Mixer):
         else:
             self.uk_weight = uk.contiguous()
 
-        # (all heads' W_uk, then all heads' W_uv: the step's keys and values for prompts)
+        # (W_uk and W_uv head by head: the step's keys and values for prompts, of all heads or a run of them)
         self.unfold = None
         if uk.dtype == torch.bfloat16 and uk.is_cuda and self.scale > 0 \
                 and ops.latent_prefill_supports(self.dim, self.value_dim, self.kv_rank, self.rot_dim):
-            self.unfold = LinearWeight(torch.cat([weights[n["uk"]], weights[n["uv"]]], dim=0))
+            self.unfold = LinearWeight(torch.cat([self.uk_weight, self.uv_weight], dim=1).flatten(0, 1))
 
     def cache_spec(self) -> CacheSpec:
         return CacheSpec(1, self.kv_rank + self.rot_dim, None, value_dim=0)
@@ -114,13 +114,15 @@ class LatentAttention(Mixer):
     # queries a key, and is taken from sixteen (the layer on two prompts of 1,667 and 833 tokens, 16 heads: 1,226 us
     # folded, 165 unfolded; error against 64 bits 0.0048 and 0.0045).  A portion's own length decides, whatever else is in the step.
     UNFOLD_QUERIES = 16
-    UNFOLD_BYTES = 1 << 30      # the most that keys and values made at a time may take
+    # Room for the rows, keys and values made at a time (two prompts of 1,667 and 833 tokens take 24 MB at 16 heads of 128 + 128): what
+    # is above the bound goes entry by entry, and some heads at a time.
+    UNFOLD_BYTES = 256 << 20
 
     def _plan(self, batch) -> "_Plan | None":
         """Which entries of the step run on keys and values made for it; None: none, or the entries are not known."""
         if self.unfold is None or batch.n_multi == 0 or len(batch.entries) != batch.n_entries:
             return None
-        row_bytes = 2 * (self.heads * (self.dim + self.value_dim) + self.kv_rank + self.rot_dim)
+        row_bytes = 2 * (self.dim + self.value_dim + self.kv_rank + self.rot_dim)      # (with one head's key and value)
         key = ("latent", self.UNFOLD_QUERIES, self.UNFOLD_BYTES // row_bytes)
         if key not in batch.plans:
             batch.plans[key] = _plan(batch.entries, *key[1:])
@@ -142,11 +144,15 @@ class LatentAttention(Mixer):
             latent = torch.empty((rows, self.kv_rank), dtype=q.dtype, device=q.device)
             rotated = torch.empty((rows, self.rot_dim), dtype=q.dtype, device=q.device)
             q_start, kv_start, slots = batch.q_start[first:end + 1], batch.kv_start[first:end], batch.slots[first:end]
-            entries = batch.entries[first:end]
+            entries, width = batch.entries[first:end], self.dim + self.value_dim
+            at_a_time = min(h, max(1, (self.UNFOLD_BYTES - 2 * rows * (self.kv_rank + self.rot_dim)) // (2 * rows * width)))
             ops.latent_gather(kv.keys, kv.block_table, q_start, kv_start, slots, end - first, max(e.kv_start + e.q_len for e in entries),
                               latent, rotated, ctx.error_word)
-            ops.latent_prefill(q, linear(latent, self.unfold), rotated, out, q_start, kv_start, end - first, max(e.q_len for e in entries),
-                               h, self.dim, self.value_dim, self.scale, self.UNFOLD_QUERIES, gate, self.gate_per_head, self.sink, ctx.error_word)
+            for head in range(0, h, at_a_time):
+                heads = self.unfold if at_a_time == h else self.unfold.rows(head * width, min(h, head + at_a_time) * width)
+                ops.latent_prefill(q, linear(latent, heads), rotated, out, q_start, kv_start, end - first, max(e.q_len for e in entries),
+                                   h, self.dim, self.value_dim, self.scale, self.UNFOLD_QUERIES, head, gate, self.gate_per_head, self.sink,
+                                   ctx.error_word)
 
     def _folded(self, q: torch.Tensor, dkv: torch.Tensor, gate: torch.Tensor | None, heads_out: torch.Tensor, ctx: LayerContext,
                 entries: slice, first_row: int, max_q_len: int, max_kv_len: int) -> None:
@@ -222,10 +228,10 @@ class _Plan:
 
 
 def _plan(entries: Sequence[EntryPlacement], queries: int, most_rows: int) -> _Plan | None:
-    """Portions of at least ``queries`` tokens run on keys and values made for the step, unless their own keys alone need more than
-    ``most_rows`` rows.  Neighbours share a product, across short portions too where these add no more rows than there are."""
+    """Portions of at least ``queries`` tokens run on keys and values made for the step.  Neighbours share a product up to ``most_rows``
+    rows, across short portions too where these add no more rows than there are."""
     padded = [-(-(e.kv_start + e.q_len) // ops.LATENT_TILE) * ops.LATENT_TILE for e in entries]
-    long = [i for i, e in enumerate(entries) if e.q_len >= queries and padded[i] <= most_rows]
+    long = [i for i, e in enumerate(entries) if e.q_len >= queries]
     if not long:
         return None
     groups = []
