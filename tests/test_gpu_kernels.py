@@ -973,6 +973,36 @@ def test_linear_attention_of_a_request_does_not_depend_on_its_neighbours(dim, va
         assert launches == (3 if m >= 193 and value_dim % 64 == 0 else 1)
 
 
+@pytest.mark.parametrize("at_a_time", [1, 2, 3])
+def test_linear_attention_in_runs_some_heads_at_a_time(at_a_time, monkeypatch):
+    """With less room for the runs' states than all heads take, the same bits and no more room than that."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    lens, heads, dim = [300, 1, 200], 5, 128
+    n, entries, width = sum(lens), len(lens), heads * dim
+    decay = torch.tensor([1 - 2.0 ** -(3 + i) for i in range(heads)], dtype=torch.float64)
+    powers = [dev((decay[:, None] ** torch.arange(most + 1, dtype=torch.float64)).float().contiguous())
+              for most in (ops.linear_attention_chunk(dim, dim), ops.linear_attention_run())]
+    rows, held = dev(rnd(n, 3 * width, dtype=torch.bfloat16)), dev(rnd(entries, heads, dim, dim, seed=5))
+    starts, slots = dev(torch.tensor([0, 300, 301, 501], dtype=torch.int32)), dev(torch.arange(entries, dtype=torch.int32))
+
+    def run():
+        out, state = torch.empty(n, width, device="cuda"), held.clone()
+        torch.cuda.reset_peak_memory_stats()
+        before, launches = torch.cuda.memory_allocated(), ops.launch_count()
+        ops.linear_attention(rows[:, :width], rows[:, width:2 * width], rows[:, 2 * width:], out, state, powers[0], starts, slots, entries, heads, dim,
+                             dim, silu=True, max_q_len=max(lens), run_powers=powers[1], portions={300: 1, 1: 1, 200: 1})
+        return out, state, torch.cuda.max_memory_allocated() - before, ops.launch_count() - launches
+
+    out, state, _, launches = run()
+    assert launches == 1 + 3
+    per_head = (n // ops.linear_attention_run() + entries) * dim * dim * 4
+    monkeypatch.setattr(ops, "LINEAR_ATTENTION_SCRATCH", at_a_time * per_head + 5)
+    parts, parts_state, room, launches = run()
+    assert torch.equal(parts, out) and torch.equal(parts_state, state)
+    assert room <= at_a_time * per_head + 2 ** 20 and launches == 1 + 3 * -(-heads // at_a_time)      # (the allocator's granularity)
+
+
 @pytest.mark.parametrize("lens, dim", [([300, 7, 193], 64), ([200, 450], 128), ([100, 20], 64)])      # (in runs, and in chunks)
 @pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
 def test_linear_attention_keeps_what_is_not_finite_from_earlier_tokens(lens, dim, bad):

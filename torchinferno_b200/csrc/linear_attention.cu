@@ -232,10 +232,11 @@ struct LinRunArgs {
   const int* slots;
   const float* powers;    // [heads, kLinRun + 1]
   float* state;           // [slots, heads, D, value_dim]
-  float* run_state;       // [runs, heads, D, value_dim]: L of a run, then the state at its start
+  float* run_state;       // [runs, n_heads, D, value_dim]: L of a run, then the state at its start
   float* out;
   int64_t ldq, ldk, ldv;
   int heads, value_dim, activation;
+  int head0, n_heads;     // the heads of these launches (the runs' states are made for some heads at a time)
 };
 
 // An entry's first run: entries' runs never overlap, since an entry of len tokens has at most len / kLinRun + 1 runs and the
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(256, 2) lin_run_sums_kernel(const T* __restric
   __shared__ float pw[kLinRun + 1];
   pdl_wait();
   pdl_trigger();
-  const int tiles = a.value_dim / TV, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * TV;
+  const int tiles = a.value_dim / TV, own = blockIdx.x / tiles, head = a.head0 + own, col0 = (blockIdx.x - own * tiles) * TV;
   const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const int t0 = blockIdx.y * kLinRun;
   if (t0 >= len || len < kLinRunsFrom) return;
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(256, 2) lin_run_sums_kernel(const T* __restric
       }
     }
   }
-  float* dst = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.heads + head) * (size_t)D * a.value_dim + col0;
+  float* dst = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.n_heads + own) * (size_t)D * a.value_dim + col0;
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -345,14 +346,14 @@ __global__ void __launch_bounds__(256) lin_fold_kernel(LinRunArgs a, int key_dim
   pdl_wait();
   pdl_trigger();
   const int entry = blockIdx.y, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
-  const size_t per_head = (size_t)key_dim * a.value_dim, width = per_head * a.heads;
+  const size_t per_head = (size_t)key_dim * a.value_dim, width = per_head * a.n_heads;
   const size_t e = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
   if (len < kLinRunsFrom || e >= width) return;
-  const float* pw = a.powers + (e / per_head) * (kLinRun + 1);
+  const float* pw = a.powers + (a.head0 + e / per_head) * (kLinRun + 1);
   const int runs = (len + kLinRun - 1) / kLinRun, last = len - (runs - 1) * kLinRun;
   const float whole = pw[kLinRun], part = pw[last];
   float* run = a.run_state + lin_first_run(row0, entry) * width + e;
-  float4* slot = reinterpret_cast<float4*>(a.state + (size_t)a.slots[entry] * width + e);
+  float4* slot = reinterpret_cast<float4*>(a.state + ((size_t)a.slots[entry] * a.heads + a.head0) * per_head + e);
   float4 st = *slot;
   constexpr int AHEAD = 8;      // (loads in flight a thread: the fold is a chain of memory latencies)
   for (int r = 0; r < runs; r += AHEAD) {
@@ -388,12 +389,12 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   __shared__ float pw[kLinRun + 1];
   pdl_wait();
   pdl_trigger();
-  const int tiles = a.value_dim / TV, head = blockIdx.x / tiles, col0 = (blockIdx.x - head * tiles) * TV;
+  const int tiles = a.value_dim / TV, own = blockIdx.x / tiles, head = a.head0 + own, col0 = (blockIdx.x - own * tiles) * TV;
   const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const int t0 = blockIdx.y * kLinRun;
   if (t0 >= len || len < kLinRunsFrom) return;
   const int n = min(kLinRun, len - t0), tid = threadIdx.x;
-  const float* S = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.heads + head) * (size_t)D * a.value_dim + col0;
+  const float* S = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.n_heads + own) * (size_t)D * a.value_dim + col0;
   constexpr int SV = SR * TV / 4 / 256;                      // 16-byte pieces of a tile of S a thread fetches
   float4 sp[SV];
   auto ask = [&](int d0) {
@@ -496,11 +497,11 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   }
   // a warp holds eight tokens: those before them count for all eight, those among them only for the tokens they come before (left
   // out, not weighed with 0: an infinity or NaN must not reach an earlier token)
-  const int own = (tid >> 5) * 8, keys = min(n, own);
+  const int mine = (tid >> 5) * 8, keys = min(n, mine);
 #pragma unroll 4
   for (int j = 0; j < keys; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV, 0);
-  const int last = min(n, own + 8);
-  for (int j = own; j < last; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV, j - ty * 4);
+  const int last = min(n, mine + 8);
+  for (int j = mine; j < last; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV, j - ty * 4);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     if (ty * 4 + i >= n) break;
@@ -597,9 +598,9 @@ static int launch_lin_runs(const void* q, const void* k, const void* v, const Li
   cudaError_t e = cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outs);
   if (e != cudaSuccess) return (int)e;
-  const dim3 grid(a.heads * (a.value_dim / TV), ceil_div(max_q_len, kLinRun), n_entries);
+  const dim3 grid(a.n_heads * (a.value_dim / TV), ceil_div(max_q_len, kLinRun), n_entries);
   TIB_LAUNCH_DEPENDENT(ks, grid, 256, sums, stream, (const T*)k, (const T*)v, a);
-  TIB_LAUNCH_DEPENDENT(lin_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.heads * D * a.value_dim, 1024), n_entries), 256, 0, stream, a, D);
+  TIB_LAUNCH_DEPENDENT(lin_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.n_heads * D * a.value_dim, 1024), n_entries), 256, 0, stream, a, D);
   TIB_LAUNCH_DEPENDENT(ko, grid, 256, outs, stream, (const T*)q, (const T*)k, (const T*)v, a);
   return TIB_OK;
 }
@@ -639,12 +640,13 @@ TIB_API int tib_linear_attention_runs_from() { return kLinRunsFrom; }
 // between them; 0 where it is not known (then, or without run_powers, the chunk kernel runs them all).  n_chunked: how many portions lie
 // between them (at most; the chunk kernel shares a head's columns out by it).  max_q_len: the longest portion.
 // run_powers: [heads, run + 1] fp32 likewise, or null.  run_state: scratch of run_capacity >= tokens / run + n_entries times
-// heads * key_dim * value_dim floats for portions of tib_linear_attention_runs_from() tokens and more, or null (they run in chunks then).
+// run_heads * key_dim * value_dim floats for portions of tib_linear_attention_runs_from() tokens and more, which are worked run_heads heads
+// at a time, or null (they run in chunks then).
 // launches: takes the number of kernels launched.
 TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, int64_t ldq, int64_t ldk, int64_t ldv,
                                  float* out, float* state, const float* powers, const int* q_start, const int* slots,
                                  int n_entries, int heads, int key_dim, int value_dim, int chunk, int activation, int dtype,
-                                 int tokens, int max_q_len, int forms, int n_chunked, const float* run_powers, float* run_state, int64_t run_capacity,
+                                 int tokens, int max_q_len, int forms, int n_chunked, const float* run_powers, float* run_state, int64_t run_capacity, int run_heads,
                                  int* launches, cudaStream_t stream) {
   *launches = 0;
   if (n_entries == 0) return TIB_OK;
@@ -663,7 +665,7 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   if (run_powers && forms && (key_dim == 64 || key_dim == 128) && value_dim % 32 == 0 && aligned && (dtype == TIB_F32 || dtype == TIB_BF16)) {
     LinRunArgs r;
     r.q_start = q_start; r.slots = slots; r.powers = run_powers; r.state = state; r.run_state = run_state; r.out = out;
-    r.ldq = ldq; r.ldk = ldk; r.ldv = ldv; r.heads = heads; r.value_dim = value_dim; r.activation = activation;
+    r.ldq = ldq; r.ldk = ldk; r.ldv = ldv; r.heads = heads; r.head0 = 0; r.n_heads = heads; r.value_dim = value_dim; r.activation = activation;
     if (forms & 1) {
       const int status = dtype == TIB_F32 ? launch_lin_walk<float>(q, k, v, r, key_dim, n_entries, stream)
                                           : launch_lin_walk<__nv_bfloat16>(q, k, v, r, key_dim, n_entries, stream);
@@ -671,17 +673,20 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
       *launches += 1;
     }
     shortest = kLinWalk + 1;
-    const bool runs = run_state && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535;
+    const bool runs = run_state && run_heads > 0 && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535;
     if ((forms & 4) && runs) {
 #define TIB_LIN_GO(T)                                                                                             \
   (key_dim == 64 ? (value_dim % 128 == 0 ? launch_lin_runs<T, 64, 128>(q, k, v, r, n_entries, max_q_len, stream)    \
                                          : launch_lin_runs<T, 64, 64>(q, k, v, r, n_entries, max_q_len, stream))    \
                  : (value_dim % 128 == 0 ? launch_lin_runs<T, 128, 128>(q, k, v, r, n_entries, max_q_len, stream)   \
                                          : launch_lin_runs<T, 128, 64>(q, k, v, r, n_entries, max_q_len, stream)))
-      const int status = dtype == TIB_F32 ? TIB_LIN_GO(float) : TIB_LIN_GO(__nv_bfloat16);
+      for (; r.head0 < heads; r.head0 += run_heads) {
+        r.n_heads = run_heads < heads - r.head0 ? run_heads : heads - r.head0;
+        const int status = dtype == TIB_F32 ? TIB_LIN_GO(float) : TIB_LIN_GO(__nv_bfloat16);
+        if (status != TIB_OK) return status;
+        *launches += 3;
+      }
 #undef TIB_LIN_GO
-      if (status != TIB_OK) return status;
-      *launches += 3;
     }
     if (runs) longest = kLinRunsFrom - 1;
     if (runs || !(forms & 4)) {

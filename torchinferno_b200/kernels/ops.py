@@ -906,7 +906,9 @@ def linear_attention_run() -> int:
     return _linear_attention_sizes()[0]
 
 
-LINEAR_ATTENTION_SCRATCH = 1 << 30      # bytes of run states a call may take (2,048 tokens of 16 heads of 128 x 128: 34 MB)
+# Bytes of run states that a call makes room for at a time: 2,048 tokens of 16 heads of 128 x 128 take 34 MB, and what is above the
+# bound goes some heads at a time (of one head, whatever it takes: 1 KB a token at 128 x 128).
+LINEAR_ATTENTION_SCRATCH = 128 << 20
 
 
 def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
@@ -929,7 +931,7 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
         raise KernelError("linear_attention: out, state or powers do not fit the head sizes")
     if q_start.numel() < n_entries + 1 or slots.numel() < n_entries:
         raise KernelError("linear_attention: entry arrays are shorter than n_entries")
-    run_state, capacity, forms, chunked = None, 0, 0, 0
+    run_state, capacity, run_heads, forms, chunked = None, 0, 0, 0, 0
     if run_powers is not None:
         run, walk, runs_from = _linear_attention_sizes()
         _need(run_powers, "run_powers", torch.float32)
@@ -942,14 +944,14 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
             chunked = sum(count for length, count in portions.items() if walk < length < runs_from)
         if forms & 4 and key_dim in (64, 128) and value_dim % 64 == 0:
             capacity = q.shape[0] // run + n_entries
-            if capacity * heads * key_dim * value_dim * 4 <= LINEAR_ATTENTION_SCRATCH:
-                run_state = torch.empty(capacity * heads * key_dim * value_dim, dtype=torch.float32, device=q.device)
+            run_heads = min(heads, max(1, LINEAR_ATTENTION_SCRATCH // (capacity * key_dim * value_dim * 4)))
+            run_state = torch.empty(capacity * run_heads * key_dim * value_dim, dtype=torch.float32, device=q.device)
     launches = c_int(0)
     _check("linear_attention", lib().tib_linear_attention(
         _ptr(q), _ptr(k), _ptr(v), c_int64(q.stride(0)), c_int64(k.stride(0)), c_int64(v.stride(0)), _ptr(out), _ptr(state),
         _ptr(powers), _ptr(q_start), _ptr(slots), c_int(n_entries), c_int(heads), c_int(key_dim), c_int(value_dim),
         c_int(chunk), c_int(1 if silu else 0), c_int(_code(q.dtype)), c_int(q.shape[0]), c_int(max_q_len), c_int(forms),
-        c_int(chunked), _ptr(run_powers), _ptr(run_state), c_int64(capacity), ctypes.byref(launches), _stream()))
+        c_int(chunked), _ptr(run_powers), _ptr(run_state), c_int64(capacity), c_int(run_heads), ctypes.byref(launches), _stream()))
     count_launches(launches.value - 1)      # (_check counted one)
     return out
 
