@@ -949,3 +949,17 @@ def test_latent_prompts_in_little_room(room, monkeypatch):
         # (the library may cut its sums otherwise for another number of features or rows: a last bit of a key, value or row)
         err = _row_error(outs[1][r].double(), outs[0][r].double())
         assert err.max() <= 0.01, (r, int(err.argmax()), float(err.max()))
+
+
+def test_latent_weights_are_held_once():
+    need_gpu()
+    from torchinferno_b200.parts.base import PartSpec, build_part
+    from torchinferno_b200.weights.random_init import random_tensor
+    params = {"hidden_size": 64, "heads": 5, "dim": 64, "rot_dim": 32, "value_dim": 128, "kv_rank": 64, "scale": 0.07, "rot_base": 3000.0, "gate": False}
+    mixer = build_part("mixer", PartSpec("latent_attention", params), dtype=torch.bfloat16, device=CUDA)
+    stored = {ws.name: random_tensor(ws, 4, dtype=torch.bfloat16).cuda() for ws in mixer.weight_specs()}
+    mixer.bind(stored)
+    places = {t.untyped_storage().data_ptr() for t in (mixer.unfold.tensor, mixer.uk_weight, mixer.uv_weight)}
+    assert len(places) == 1 and not places & {t.untyped_storage().data_ptr() for t in stored.values()}
+    assert mixer.unfold.tensor.untyped_storage().nbytes() == 2 * 5 * (64 + 128) * 64
+    assert torch.equal(mixer.uk_weight, stored["uk"].view(5, 64, 64)) and torch.equal(mixer.uv_weight, stored["uv"].view(5, 128, 64))

@@ -100,11 +100,14 @@ class LatentAttention(Mixer):
         else:
             self.uk_weight = uk.contiguous()
 
-        # (W_uk and W_uv head by head: the step's keys and values for prompts, of all heads or a run of them)
+        # W_uk and W_uv head by head: the step's keys and values for prompts, of all heads or a run of them.  The folded form's two weights
+        # are views of it.
         self.unfold = None
         if uk.dtype == torch.bfloat16 and uk.is_cuda and self.scale > 0 \
                 and ops.latent_prefill_supports(self.dim, self.value_dim, self.kv_rank, self.rot_dim):
-            self.unfold = LinearWeight(torch.cat([self.uk_weight, self.uv_weight], dim=1).flatten(0, 1))
+            both = torch.cat([self.uk_weight, self.uv_weight], dim=1)
+            self.unfold = LinearWeight(both.flatten(0, 1), allow_transpose=False)
+            self.uk_weight, self.uv_weight = both[:, :self.dim], both[:, self.dim:]
 
     def cache_spec(self) -> CacheSpec:
         return CacheSpec(1, self.kv_rank + self.rot_dim, None, value_dim=0)
