@@ -670,3 +670,41 @@ def test_prompt_portions_of_window_attention_on_both_tensor_core_forms(heads, kv
         outs.append(out.double().cpu())
     # the weights' 16 bits (2^-16 of values of unit size, over a sum of weights of one), then a rounding to bfloat16 (2^-8) on either side
     assert ((outs[0] - outs[1]).abs() <= 2.0 ** -7 * outs[1].abs() + 2.0 ** -12 * outs[1].abs().max()).all()
+
+
+@pytest.mark.parametrize("keep", [0, 20])
+def test_window_attention_of_a_request_does_not_depend_on_its_neighbours(keep):
+    """Single tokens beside prompt portions, alone and in one step: prompts bit for bit, single tokens but for the order of their sums (a
+    step of single tokens has a form of its own); a launch for each of the two kernels that occur."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, kv_heads, dim, window, page = 4, 2, 64, 100, 16
+    lens, pasts = [1, 150, 1, 33, 70], [300, 20, 0, 127, 64]
+    g = torch.Generator().manual_seed(keep)
+    per = max(a + b for a, b in zip(lens, pasts)) // page + 1
+    pages = torch.randn(len(lens) * per, 2, kv_heads, page, dim, generator=g).to(torch.bfloat16).cuda()
+    table = torch.randperm(len(lens) * per, generator=g).view(len(lens), per).to(torch.int32).cuda()
+    q = torch.randn(sum(lens), heads * dim, generator=g).to(torch.bfloat16).cuda()
+    ints = lambda t: torch.as_tensor(list(t)).to(torch.int32).cuda()
+
+    def run(first, count):
+        part = lens[first:first + count]
+        rows = q[sum(lens[:first]):sum(lens[:first + count])].contiguous()
+        out, error, before = torch.empty_like(rows), ints([0]), ops.launch_count()
+        ops.pooled_window_attention(rows, out, ints(sum(part[:i]) for i in range(count + 1)), ints(pasts[first:first + count]),
+                                    ints(range(first, first + count)), pages[:, 0], pages[:, 1], table, None, None, None, count, max(part), heads,
+                                    kv_heads, window=window, pool=0, keep=keep, scale=dim ** -0.5, error_word=error,
+                                    portions={m: part.count(m) for m in part})
+        assert int(error) == 0
+        return out, ops.launch_count() - before
+
+    together, launches = run(0, len(lens))
+    assert launches == 2
+    for i in range(len(lens)):
+        alone, launches = run(i, 1)
+        beside = together[sum(lens[:i]):sum(lens[:i + 1])]
+        assert launches == 1
+        if lens[i] > 1:
+            assert torch.equal(alone, beside), i
+        else:      # (the bound of the two tensor-core forms above)
+            assert ((alone - beside).abs().double() <= 2.0 ** -7 * beside.abs().double() + 2.0 ** -12 * beside.abs().max().double()).all(), i

@@ -458,7 +458,9 @@ static int pwa_launch(const void* q, void* out, const PwaArgs& a, int n_entries,
 // ------------------------------------------------------------ tensor cores
 // 64 rows (tokens x the query heads of one kv head) against tiles of 64 keys, four warps of 16 rows: first the tiles of
 // block means (aligned to absolute block numbers), then the tiles of tokens (aligned to absolute positions), both in
-// rising order, so a row's sums do not depend on how the prompt was cut or on what else the step holds.  Keys and values
+// rising order, so a row's sums do not depend on how the prompt was cut.  (The form for few rows below adds them in another
+// order; it is taken where all portions of the step are that short.  Portions of more than a tile's rows go to
+// window_tcgen05.cu where it takes them, whatever else is in the step.)  Keys and values
 // of a tile come in by cp.async, row by row from their pages, two stages; rows the tile's queries cannot see are
 // zero-filled (unwritten cache may hold anything) and masked.  Scores accumulate in fp32; the softmax runs in fp32 on
 // scores in units of ln 2; the weights enter the second product as a high bf16 part plus the remainder, so that they
@@ -501,7 +503,7 @@ pwa_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __r
   // (with the contexts shared out, blockIdx.x counts the parts of a context, and the block's rows are the entry's only ones)
   const bool shared_out = SHARES && WT && a.n_splits > 1;
   const int t0 = shared_out ? 0 : blockIdx.x * a.q_tile;
-  if (t0 >= q_len) return;
+  if (t0 >= q_len || q_len > a.longest) return;
   const int nt = min(a.q_tile, q_len - t0);
   const int nrows = nt * gc;
   const int pos0 = a.kv_start[entry] + t0;
@@ -972,14 +974,14 @@ static int pwa_launch_mma_staged(const void* q, void* out, const PwaArgs& a, dim
 // sums are added afterwards in a fixed order.  A row's result then differs from the other form's in the order of fp32
 // sums only.
 template <int DK, int DV>
-static int pwa_launch_mma(const void* q, void* out, PwaArgs a, int n_entries, int max_q_len, cudaStream_t stream) {
+static int pwa_launch_mma(const void* q, void* out, PwaArgs a, int n_entries, int max_q_len, bool whole_step, cudaStream_t stream) {
   const int group = a.heads / a.kv_heads;
   a.group_chunk = group < kPmRows ? group : kPmRows;
   a.q_tile = kPmRows / a.group_chunk;
   const int chunks = (group + a.group_chunk - 1) / a.group_chunk;
   if ((int64_t)a.kv_heads * chunks > 65535) return TIB_E_SIZE;
   dim3 grid(ceil_div(max_q_len, a.q_tile), n_entries, a.kv_heads * chunks);
-  if ((int64_t)max_q_len * a.group_chunk <= 16) {
+  if (whole_step && (int64_t)max_q_len * a.group_chunk <= 16) {
     if (a.n_splits > 1) {
       // single tokens whose contexts are shared out over n_splits blocks each; a second kernel adds the parts
       if (max_q_len != 1 || !a.partial || a.vfreq) return TIB_E_ARG;
@@ -1013,6 +1015,8 @@ TIB_API int tib_pooled_window_attention_splits(int n_entries, int heads, int kv_
   if (splits > 32) splits = 32;
   return splits < 1 ? 1 : splits;
 }
+// Rows (tokens x query heads of a key head) of a portion up to which the mma.sync kernel keeps it.
+TIB_API int tib_pooled_window_attention_few_rows() { return kWtFewRows; }
 TIB_API int tib_pooled_window_attention_part_floats(int vdim) { return (vdim <= 64 ? 64 : 128) + 2; }
 
 // Whether the tensor-core kernel takes these shapes (bf16; rows of 16-byte pieces in every array it copies from).
@@ -1108,6 +1112,8 @@ TIB_API int tib_pool_blocks(const void* k_pages, const void* v_pages, const int*
 // turned values): every context is shared out over n_splits blocks, whose sums go through `partial`
 // [n_splits, n_tokens, heads, part floats] to a second kernel; n_tokens: rows of q.
 // keep > 0: the first `keep` tokens are seen from behind the window too (no blocks and no rel_bias then).
+// few_rows: the longest portion of at most tib_pooled_window_attention_few_rows() rows, 0: there is none, -1: not known.
+// launches: takes the number of kernels launched.
 // force_simt: the CUDA-core kernel also where the tensor-core kernel would take the step.
 TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_start, const int* kv_start, const int* slots,
                                         const void* k_pages, const void* v_pages, const int* block_table, int table_stride,
@@ -1117,8 +1123,10 @@ TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_s
                                         int kv_heads, int dim, int vdim, int window, int keep, int pool, float scale, const float* temp,
                                         const float* sink, const float* vfreq, const void* gate, int gate_dtype, int64_t ld_gate,
                                         const float* rel_bias, int rel_span, float* partial, int n_splits, int n_tokens,
-                                        int* error_word, int dtype, int force_simt, cudaStream_t stream) {
+                                        int few_rows, int* launches, int* error_word, int dtype, int force_simt, cudaStream_t stream) {
+  *launches = 0;
   if (n_entries == 0 || max_q_len == 0) return TIB_OK;
+  *launches = n_splits > 1 ? 2 : 1;
   if (!q || !out || !q_start || !kv_start || !slots || !k_pages || !v_pages || !block_table) return TIB_E_ARG;
   if (pool > 0 && (!bk_pages || !bv_pages || !b_table || b_page_size < 1)) return TIB_E_ARG;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || dim < 1 || vdim < 1 || page_size < 1 || window < 1 || pool < 0) return TIB_E_SIZE;
@@ -1135,19 +1143,31 @@ TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_s
   a.error_word = error_word;
   a.partial = partial; a.n_splits = n_splits > 1 ? n_splits : 1; a.n_tokens = n_tokens;
   const int group = heads / kv_heads;
+  a.shortest = kWtFewRows / group + 1; a.longest = 0x7fffffff;
   a.group_chunk = group < kPwaRows ? group : kPwaRows;
   a.q_tile = kPwaRows / a.group_chunk;
   const int chunks = (group + a.group_chunk - 1) / a.group_chunk;
   if ((int64_t)kv_heads * chunks > 65535) return TIB_E_SIZE;
   // bf16 steps run on the tensor cores, single tokens too (their tiles come in by cp.async, 16 bytes a piece, where the
   // other kernel waits for one element at a time); 32-bit and head sizes that are no multiples of 8 run on the CUDA cores.
-  // Portions of prompts that fill the rows of a tile take tcgen05 products where pages and head sizes suit the copies.
-  if (dtype == TIB_BF16 && !force_simt && window_tcgen05_takes(a, q, out, max_q_len)) return window_tcgen05(q, out, a, n_entries, max_q_len, stream);
+  // Portions of prompts that fill the rows of a tile take tcgen05 products where pages and head sizes suit the copies; each portion by its
+  // own length, so that a single token beside a prompt is not given a block of 128 rows (64 single tokens at 4,000 beside eight
+  // portions of 33, 16 / 8 heads of 128: the layer took 163 us when the step's longest portion chose for all, 132 without tcgen05).
+  bool whole_step = true;
+  if (dtype == TIB_BF16 && !force_simt && window_tcgen05_takes(a, q, out, max_q_len)) {
+    const int status = window_tcgen05(q, out, a, n_entries, max_q_len, stream);
+    if (few_rows < 0 || few_rows > kWtFewRows / group) few_rows = kWtFewRows / group;
+    if (status != TIB_OK || few_rows == 0) return status;
+    max_q_len = few_rows;
+    whole_step = false;
+    a.longest = kWtFewRows / group;
+    *launches = 2;
+  }
   if (dtype == TIB_BF16 && !force_simt && pwa_mma_takes(a, q)) {
-    if (dim <= 64 && vdim <= 64) return pwa_launch_mma<64, 64>(q, out, a, n_entries, max_q_len, stream);
-    if (dim <= 64) return pwa_launch_mma<64, 128>(q, out, a, n_entries, max_q_len, stream);
-    if (vdim <= 64) return pwa_launch_mma<128, 64>(q, out, a, n_entries, max_q_len, stream);
-    return pwa_launch_mma<128, 128>(q, out, a, n_entries, max_q_len, stream);
+    if (dim <= 64 && vdim <= 64) return pwa_launch_mma<64, 64>(q, out, a, n_entries, max_q_len, whole_step, stream);
+    if (dim <= 64) return pwa_launch_mma<64, 128>(q, out, a, n_entries, max_q_len, whole_step, stream);
+    if (vdim <= 64) return pwa_launch_mma<128, 64>(q, out, a, n_entries, max_q_len, whole_step, stream);
+    return pwa_launch_mma<128, 128>(q, out, a, n_entries, max_q_len, whole_step, stream);
   }
   const int dpl = (vdim + 31) / 32;
 #define TIB_PWA_DISPATCH(T)                                                              \

@@ -31,10 +31,14 @@ struct PwaArgs {
   PwaCache tokens, blocks;
   int group_chunk, q_tile;
   int* error_word;
+  int shortest, longest;                                   // portions this launch takes (window_tcgen05 / the mma.sync kernel)
   float* partial; int n_splits; int n_tokens;              // a step of single tokens whose contexts are shared out over blocks
 };
 
-// Prompt portions on the 5th-generation tensor cores (window_tcgen05.cu), where window_tcgen05_takes them.
+// Prompt portions on the 5th-generation tensor cores (window_tcgen05.cu), where window_tcgen05_takes them: those of `shortest` tokens
+// and more, which is more rows (tokens x query heads of a key head) than kWtFewRows, a tile of the mma.sync kernel, which keeps
+// the others.
+constexpr int kWtFewRows = 64;
 bool window_tcgen05_takes(const PwaArgs& a, const void* q, const void* out, int max_q_len);
 int window_tcgen05(const void* q, void* out, const PwaArgs& a, int n_entries, int max_q_len, cudaStream_t stream);
 

@@ -80,7 +80,7 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int q_len = a.q_start[entry + 1] - row0;
   const int q_tile = kWtTile / group;
   const int t0 = (gridDim.z - 1 - blockIdx.z) * q_tile;
-  if (t0 >= q_len) return;
+  if (t0 >= q_len || q_len < a.shortest) return;
   const int nt = min(q_tile, q_len - t0), nrows = nt * group;
   const int pos0 = a.kv_start[entry] + t0, last_pos = pos0 + nt - 1;
   // block means any row sees, kept tokens' tiles ahead of the window's first, the window's tiles
@@ -432,11 +432,11 @@ static bool wt_pages_suit(const PwaCache& c) {
 }
 
 // Heads of 64 or 128, keys and values alike, groups of up to 64, pages of 8 .. 128 tokens, no distance bias; and portions with more
-// rows (tokens x query heads of a key head) than one warp-tile of the other kernel, which single tokens and short portions keep.
+// than kWtFewRows rows in the step.
 bool window_tcgen05_takes(const PwaArgs& a, const void* q, const void* out, int max_q_len) {
   const int group = a.heads / a.kv_heads;
   if (a.dim != a.vdim || (a.dim != 64 && a.dim != 128) || group > 64 || a.rel_bias || a.n_splits > 1) return false;
-  if ((int64_t)max_q_len * group <= 64 || !wt_pages_suit(a.tokens) || (a.pool > 0 && !wt_pages_suit(a.blocks))) return false;
+  if ((int64_t)max_q_len * group <= kWtFewRows || !wt_pages_suit(a.tokens) || (a.pool > 0 && !wt_pages_suit(a.blocks))) return false;
   if (a.gate && (a.gate_dtype != TIB_BF16 || a.ld_gate % 8 || ((uintptr_t)a.gate & 15))) return false;
   return (((uintptr_t)q | (uintptr_t)out) & 15) == 0 && ceil_div(max_q_len, kWtTile / group) <= 65535;
 }

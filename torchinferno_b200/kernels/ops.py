@@ -128,7 +128,7 @@ def lib() -> ctypes.CDLL:
                    "tib_qk_norm_append", "tib_sigmoid_attention", "tib_sigmoid_attention_takes_mma", "tib_gated_recurrence",
                    "tib_softcap_f32", "tib_short_conv", "tib_ssd_scan", "tib_ssd_scan_max_state", "tib_ssd_scan_run", "tib_gated_group_norm",
                    "tib_rotary_kv_append", "tib_pool_blocks", "tib_pooled_window_attention", "tib_hyper_step",
-                   "tib_pooled_window_attention_splits", "tib_pooled_window_attention_part_floats",
+                   "tib_pooled_window_attention_splits", "tib_pooled_window_attention_part_floats", "tib_pooled_window_attention_few_rows",
                    "tib_input_conv", "tib_norm_conv_step", "tib_row_norm_append", "tib_talking_heads_attention",
                    "tib_talking_heads_takes_mma", "tib_talking_heads_takes_step", "tib_talking_heads_key_span",
                    "tib_talking_heads_tiles_per_part", "tib_conv_norm_append", "tib_matrix_memory", "tib_matrix_memory_tile",
@@ -1569,7 +1569,8 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
                             temp: torch.Tensor | None = None, sink: torch.Tensor | None = None,
                             value_freq: torch.Tensor | None = None, gate: torch.Tensor | None = None,
                             error_word: torch.Tensor | None = None, force_simt: bool = False,
-                            rel_bias: torch.Tensor | None = None, max_kv_len: int = 0, splits: int | None = None) -> torch.Tensor:
+                            rel_bias: torch.Tensor | None = None, max_kv_len: int = 0, splits: int | None = None,
+                            portions: Mapping[int, int] | None = None) -> torch.Tensor:
     """Per head, out[i] = sigmoid(gate[i]) * turn_back_i(sum_j w_ij v_j + sum_b w_ib V_b): softmax weights over the tokens j
     with 0 <= i - j < window and the blocks b of ``pool`` positions with b * pool + pool - 1 <= i - window (their means K_b,
     V_b from the strided pages), scores q . k * scale * temp[h], exp(sink[h]) added to the denominator; turn_back undoes at
@@ -1579,7 +1580,8 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
     ``scale`` nor ``temp`` multiplies it).  A step of single tokens only on the tensor cores (no turned values) that
     names the longest context (``max_kv_len``) shares every context's visible keys out over ``splits`` blocks (None: enough
     to fill the GPU) whose sums a second small kernel adds in a fixed order.
-    bfloat16 steps run on the tensor cores when the head sizes are multiples of 8 up to 128, unless ``force_simt``."""
+    bfloat16 steps run on the tensor cores when the head sizes are multiples of 8 up to 128, unless ``force_simt``; long portions
+    and short ones then by kernels of their own.  ``portions`` (length: how many entries have it) spares a launch over nothing."""
     _need(q, "q"), _need(out, "out", q.dtype)
     dim, vdim = keys.shape[3], values.shape[3]
     n = q.shape[0]
@@ -1614,9 +1616,13 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
         if n_splits > 1:
             floats = int(lib().tib_pooled_window_attention_part_floats(c_int(vdim)))
             partial = torch.empty((n_splits, n, heads, floats), dtype=torch.float32, device=q.device)
-            count_launches(1)
         else:
             n_splits = 1
+    few_rows = -1
+    if portions:
+        most = int(lib().tib_pooled_window_attention_few_rows()) * kv_heads // heads
+        few_rows = max((length for length in portions if length <= most), default=0)
+    launches = c_int(0)
     _check("pooled_window_attention", lib().tib_pooled_window_attention(
         _ptr(q), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(keys), _ptr(values), _ptr(block_table),
         c_int(block_table.stride(0)), c_int(page_size), c_int64(page_stride), c_int(num_pages),
@@ -1625,7 +1631,9 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
         c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim), c_int(window), c_int(keep), c_int(pool),
         c_float(scale), _ptr(temp), _ptr(sink), _ptr(value_freq), _ptr(gate), c_int(_code(gate.dtype) if gate is not None else 0),
         c_int64(ld_gate), _ptr(rel_bias), c_int(rel_bias.shape[1] if rel_bias is not None else 0), _ptr(partial),
-        c_int(n_splits), c_int(n), _ptr(error_word), c_int(_code(q.dtype)), c_int(int(force_simt)), _stream()))
+        c_int(n_splits), c_int(n), c_int(few_rows), ctypes.byref(launches), _ptr(error_word), c_int(_code(q.dtype)), c_int(int(force_simt)),
+        _stream()))
+    count_launches(launches.value - 1)      # (_check counted one)
     return out
 
 

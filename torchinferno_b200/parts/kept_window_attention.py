@@ -123,7 +123,7 @@ class KeptWindowAttention(Mixer):
             q, out, batch.q_start, batch.kv_start, batch.slots, kv.keys, kv.values, kv.block_table, None, None, None, batch.n_entries,
             batch.max_q_len, h, g, window=self.window or NO_WINDOW, keep=self.keep_first, pool=0, scale=self.scale, sink=self.sink,
             gate=proj[:, self.g_off:self.g_off + h * d] if self.has_gate else None, error_word=ctx.error_word,
-            max_kv_len=batch.max_kv_len)
+            max_kv_len=batch.max_kv_len, portions=batch.portions)
         return linear(out, self.o_weight)
 
 

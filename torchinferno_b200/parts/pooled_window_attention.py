@@ -133,7 +133,8 @@ class PooledWindowAttention(Mixer):
             side.keys if self.pool else None, side.values if self.pool else None, side.block_table if self.pool else None,
             batch.n_entries, batch.max_q_len, h, g, window=self.window, pool=self.pool, scale=self.scale, temp=self.temp,
             sink=self.sink, value_freq=self.value_freq,
-            gate=proj[:, self.g_off:self.g_off + h * self.value_dim] if self.has_gate else None, error_word=ctx.error_word)
+            gate=proj[:, self.g_off:self.g_off + h * self.value_dim] if self.has_gate else None, error_word=ctx.error_word,
+            portions=batch.portions)
         return linear(out, self.o_weight)
 
 
