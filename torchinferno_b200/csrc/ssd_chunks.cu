@@ -21,6 +21,7 @@
 // states' way through the L2 (one of 32 KB a head and chunk, written twice and read twice).
 #include "state_space.cuh"
 #include "mma.cuh"
+#include <type_traits>
 
 namespace tib {
 
@@ -57,11 +58,9 @@ __device__ __forceinline__ void ssd_add(float (&sum)[4], const float (&step)[4])
   for (int c = 0; c < 4; ++c) sum[c] += step[c];
 }
 
-// A packed pair without what is not finite (zeros in its place; odd says that there was some).
-__device__ __forceinline__ uint32_t ssd_finite2(uint32_t v, bool& odd) {
-  const uint32_t keep = ((v & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
-  odd |= keep != 0xffffffffu;
-  return v & keep;
+// The bits of a packed pair that belong to finite numbers.
+__device__ __forceinline__ uint32_t ssd_finite2(uint32_t v) {
+  return ((v & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
 }
 
 // Step sizes and sums of log decays of a chunk's n tokens (tokens behind it: no step, the sum stays).  Called by the whole block;
@@ -315,77 +314,86 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
       acc[i][2] *= f1; acc[i][3] *= f1;
     }
   }
-  for (int j0 = 0; j0 <= m0; j0 += 16) {        // 16 tokens before (or among) the warp's own
-    float s[2][4];
+  // Among the warp's own tokens a later one weighs 0, which must not meet an infinity or NaN: what is not finite there stays out of the
+  // product and is added below, to the tokens it does not come after.  (A prompt of 2,048 tokens, 64 heads of 64: the layer takes 254 us
+  // without any look, 263 with the check and the repair in the loop, 258 so.)
+  bool odd = false;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+  for (int p = lane; p < 16 * PT / 8; p += 32) {
+    const uint4 v = *reinterpret_cast<const uint4*>(xs + (m0 + p / (PT / 8)) * PS + (p % (PT / 8)) * 8);
+    odd |= (ssd_finite2(v.x) & ssd_finite2(v.y) & ssd_finite2(v.z) & ssd_finite2(v.w)) != 0xffffffffu;
+  }
+  odd = __any_sync(0xffffffffu, odd);
+  const auto within = [&](auto checked) {         // (the common case without the check)
+    constexpr bool CHECKED = decltype(checked)::value;
+    for (int j0 = 0; j0 <= m0; j0 += 16) {        // 16 tokens before (or among) the warp's own
+      float s[2][4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) s[i][c] = 0.f;
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int k = 0; k < N / 16; ++k) {
-      uint32_t b[4];
-      ldmatrix_x4(b, bs + (j0 + ((lane >> 4) << 3) + (lane & 7)) * NS + k * 16 + ((lane >> 3) & 1) * 8);
-      float step[4][4] = {};
-      ssd_mma8(step[0], cv[k], b[0], 0);
-      ssd_mma8(step[1], cv[k], b[1], 1);
-      ssd_mma8(step[2], cv[k], b[2], 0);
-      ssd_mma8(step[3], cv[k], b[3], 1);
-      ssd_add(step[0], step[1]);
-      ssd_add(step[2], step[3]);
-      ssd_add(s[0], step[0]);
-      ssd_add(s[1], step[2]);
+        for (int c = 0; c < 4; ++c) s[i][c] = 0.f;
+#pragma unroll
+      for (int k = 0; k < N / 16; ++k) {
+        uint32_t b[4];
+        ldmatrix_x4(b, bs + (j0 + ((lane >> 4) << 3) + (lane & 7)) * NS + k * 16 + ((lane >> 3) & 1) * 8);
+        float step[4][4] = {};
+        ssd_mma8(step[0], cv[k], b[0], 0);
+        ssd_mma8(step[1], cv[k], b[1], 1);
+        ssd_mma8(step[2], cv[k], b[2], 0);
+        ssd_mma8(step[3], cv[k], b[3], 1);
+        ssd_add(step[0], step[1]);
+        ssd_add(step[2], step[3]);
+        ssd_add(s[0], step[0]);
+        ssd_add(s[1], step[2]);
+      }
+      uint32_t w[3][4];
+#pragma unroll
+      for (int half = 0; half < 2; ++half)        // (tokens j0 + 8 half + 2 t4 and the next one)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {             // (rows i0, i1)
+          const int i = r == 0 ? i0 : i1, j = j0 + half * 8 + 2 * t4;
+          const float v0 = j <= i ? s[half][2 * r] * (ssd_decay(st, i, j) * st.dt[j]) : 0.f;
+          const float v1 = j + 1 <= i ? s[half][2 * r + 1] * (ssd_decay(st, i, j + 1) * st.dt[j + 1]) : 0.f;
+          ssd_split2(v0, v1, w[0][half * 2 + r], w[1][half * 2 + r], w[2][half * 2 + r]);
+        }
+#pragma unroll
+      for (int j = 0; j < NT / 2; ++j) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, xs + (j0 + ((lane >> 3) & 1) * 8 + (lane & 7)) * PS + j * 16 + ((lane >> 4) << 3));
+        if (CHECKED && j0 == m0) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) b[q] &= ssd_finite2(b[q]);
+        }
+        float step[2][4] = {};
+#pragma unroll
+        for (int u = 2; u >= 0; --u) {
+          mma_bf16(step[0], w[u], b[0], b[1]);
+          mma_bf16(step[1], w[u], b[2], b[3]);
+        }
+        ssd_add(acc[2 * j], step[0]);
+        ssd_add(acc[2 * j + 1], step[1]);
+      }
     }
-    uint32_t w[3][4];
-    bool odd = false;
-#pragma unroll
-    for (int half = 0; half < 2; ++half)        // (tokens j0 + 8 half + 2 t4 and the next one)
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {             // (rows i0, i1)
-        const int i = r == 0 ? i0 : i1, j = j0 + half * 8 + 2 * t4;
-        const float v0 = j <= i ? s[half][2 * r] * (ssd_decay(st, i, j) * st.dt[j]) : 0.f;
-        const float v1 = j + 1 <= i ? s[half][2 * r + 1] * (ssd_decay(st, i, j + 1) * st.dt[j + 1]) : 0.f;
-        ssd_split2(v0, v1, w[0][half * 2 + r], w[1][half * 2 + r], w[2][half * 2 + r]);
-      }
-#pragma unroll
-    for (int j = 0; j < NT / 2; ++j) {
-      uint32_t b[4];
-      ldmatrix_x4_trans(b, xs + (j0 + ((lane >> 3) & 1) * 8 + (lane & 7)) * PS + j * 16 + ((lane >> 4) << 3));
-      if (j0 == m0) {      // (the tile of the warp's own tokens: a later one weighs 0, which must not meet an infinity or NaN)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) b[q] = ssd_finite2(b[q], odd);
-      }
-      float step[2][4] = {};
-#pragma unroll
-      for (int u = 2; u >= 0; --u) {
-        mma_bf16(step[0], w[u], b[0], b[1]);
-        mma_bf16(step[1], w[u], b[2], b[3]);
-      }
-      ssd_add(acc[2 * j], step[0]);
-      ssd_add(acc[2 * j + 1], step[1]);
-    }
-    if (__any_sync(0xffffffffu, odd)) {         // what was left out, for the tokens it does not come after
+  };
+  if (odd) within(std::true_type{});
+  else within(std::false_type{});
+  if (odd) {
 #pragma unroll 1
-      for (int jj = 0; jj < 16; ++jj) {
-        const int from = (lane & ~3) | ((jj & 7) >> 1);      // (the lane that holds this token's weights)
+    for (int j = m0; j < m0 + 16; ++j)
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          float weight = 0.f;
+      for (int r = 0; r < 2; ++r) {
+        const int i = r == 0 ? i0 : i1;
+        if (j > i) continue;
+        float weight = 0.f;
+        for (int k = 0; k < N; ++k) weight = fmaf(__bfloat162float(cs[i * NS + k]), __bfloat162float(bs[j * NS + k]), weight);
+        weight *= ssd_decay(st, i, j) * st.dt[j];
 #pragma unroll
-          for (int u = 2; u >= 0; --u) {
-            const uint32_t pair = __shfl_sync(0xffffffffu, jj < 8 ? w[u][r] : w[u][2 + r], from);
-            const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&pair));
-            weight += jj & 1 ? f.y : f.x;
-          }
-          if (j0 + jj > (r == 0 ? i0 : i1)) continue;
-#pragma unroll
-          for (int t = 0; t < NT; ++t) {
-            const float2 x = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(xs + (j0 + jj) * PS + t * 8 + 2 * t4));
-            if (!isfinite(x.x)) acc[t][2 * r] = fmaf(weight, x.x, acc[t][2 * r]);
-            if (!isfinite(x.y)) acc[t][2 * r + 1] = fmaf(weight, x.y, acc[t][2 * r + 1]);
-          }
+        for (int t = 0; t < NT; ++t) {
+          const float2 x = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(xs + j * PS + t * 8 + 2 * t4));
+          if (!isfinite(x.x)) acc[t][2 * r] = fmaf(weight, x.x, acc[t][2 * r]);
+          if (!isfinite(x.y)) acc[t][2 * r + 1] = fmaf(weight, x.y, acc[t][2 * r + 1]);
         }
       }
-    }
   }
   const float skip = a.d_skip[h];
 #pragma unroll
