@@ -963,3 +963,25 @@ def test_latent_weights_are_held_once():
     assert len(places) == 1 and not places & {t.untyped_storage().data_ptr() for t in stored.values()}
     assert mixer.unfold.tensor.untyped_storage().nbytes() == 2 * 5 * (64 + 128) * 64
     assert torch.equal(mixer.uk_weight, stored["uk"].view(5, 64, 64)) and torch.equal(mixer.uv_weight, stored["uv"].view(5, 128, 64))
+
+
+def test_latent_rows_off_their_boundaries_stay_folded(monkeypatch):
+    """A query latent of 20 leaves the gate's rows off their 16-byte boundaries: the kernels on keys made for the step cannot read
+    them, and the folded form takes the prompt."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    from torchinferno_b200.parts.base import PartSpec, build_part
+    from torchinferno_b200.weights.random_init import random_tensor
+    params = {"hidden_size": 64, "heads": 2, "dim": 64, "rot_dim": 32, "value_dim": 64, "kv_rank": 64, "scale": 0.07, "rot_base": 3000.0, "eps": 1e-5,
+              "gate": True, "sink": False, "q_rank": 20}
+    monkeypatch.setattr(ops, "latent_prefill", lambda *a, **k: pytest.fail("took rows it cannot read"))
+    x, outs = {"a": torch.randn(200, 64, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)}, {}
+    for dtype in (torch.float32, torch.bfloat16):
+        mixer = build_part("mixer", PartSpec("latent_attention", params), dtype=dtype, device=CUDA)
+        _bind(mixer, {ws.name: random_tensor(ws, 4, dtype=torch.bfloat16) for ws in mixer.weight_specs()}, dtype, "mix.")
+        assert dtype == torch.float32 or mixer.unfold is not None
+        cache = _cache_for(mixer, dtype, 16, 32, 2, 300)
+        cache.open("a")
+        outs[dtype] = _run_steps(mixer, cache, [[("a", 150)], [("a", 50)]], {"a": x["a"].to(dtype)})["a"]
+    err = _row_error(outs[torch.bfloat16], outs[torch.float32])
+    assert err.max() <= 0.03, (int(err.argmax()), float(err.max()))      # (the bound of the layer's other tests in bfloat16)
