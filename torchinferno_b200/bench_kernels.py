@@ -309,7 +309,7 @@ def run_linear_attention(args) -> None:
         q_start = i32([0, n]) if mode == "prompt" else i32(list(range(n + 1)))
         slots = i32(list(range(n_entries)))
         fn = lambda: ops.linear_attention(q, k, val, out, state, powers, q_start, slots, n_entries, h, d, v, silu=True,
-                                          max_q_len=n // n_entries, run_powers=run_powers)
+                                          max_q_len=n // n_entries, run_powers=run_powers, portions={n // n_entries: n_entries})
         if mode == "prompt":
             flops = 2 * h * n * (run * (d + v) / 2 + 2 * d * v)
             report("linear_attention[prompt]", timer(fn), flops=flops, tokens=n, heads=h, key_dim=d, value_dim=v, run=run)
@@ -457,7 +457,7 @@ def run_pooled_window_attention(args) -> None:
             flops, moved = None, n * seen(ctx - 1) * k * (d + v) * 2
         fn = lambda: ops.pooled_window_attention(q, out, q_start, kv_start, slots, keys, values, table, bkeys, bvalues, btable, n_entries,
                                                  max_q, h, k, window=window, pool=pool, scale=0.09, temp=temp, sink=sink,
-                                                 value_freq=vfreq, gate=gate)
+                                                 value_freq=vfreq, gate=gate, portions={max_q: n_entries})
         report(f"pooled_window_attention[{mode}]", timer(fn), flops=flops, bytes_moved=moved, entries=n_entries, context=ctx, heads=h,
                kv_heads=k, head_dim=d, value_dim=v, window=window, pool=pool)
     # the launch ahead of it: biases, the two rotations, the store into the pages; then the means of completed blocks
@@ -506,7 +506,8 @@ def run_biased_attention(args) -> None:
             flops, moved = None, n * ctx * k * (d + v) * 2
         for name, bias in (("biased_attention", rel), ("the same without the bias", None)):
             fn = lambda: ops.pooled_window_attention(q, out, q_start, kv_start, slots, keys, values, table, None, None, None, n_entries,
-                                                     max_q, h, k, window=1 << 30, pool=0, scale=0.09, rel_bias=bias, max_kv_len=ctx)
+                                                     max_q, h, k, window=1 << 30, pool=0, scale=0.09, rel_bias=bias, max_kv_len=ctx,
+                                                     portions={max_q: n_entries})
             report(f"{name}[{mode}]", timer(fn), flops=flops, bytes_moved=moved, entries=n_entries, context=ctx, heads=h, kv_heads=k,
                    head_dim=d, value_dim=v, bias_max=args.bias_max)
     n = args.tokens
@@ -635,7 +636,7 @@ def run_kept_window_attention(args) -> None:
         for splits in tried:
             fn = lambda: ops.pooled_window_attention(q, out, q_start, kv_start, slots, keys, values, table, None, None, None, n_entries, max_q,
                                                      h, k, window=window, keep=keep, pool=0, scale=0.09, sink=sink, gate=gate,
-                                                     max_kv_len=ctx if max_q == 1 else 0, splits=splits)
+                                                     max_kv_len=ctx if max_q == 1 else 0, splits=splits, portions={max_q: n_entries})
             extra = {} if splits is None else {"splits": splits}
             report(f"kept_window_attention[{mode}]", timer(fn), flops=flops, bytes_moved=moved, entries=n_entries, context=ctx, heads=h,
                    kv_heads=k, head_dim=d, window=window, keep=keep, **extra)
