@@ -18,7 +18,7 @@
 // Three ways to run that.  Every portion takes the one its own length and the layer's sizes name, whatever else is in the step
 // (tib_linear_attention launches each form that occurs over the whole batch, and a form's blocks leave the others' portions alone), so a
 // request's numbers do not depend on its neighbours:
-//   runs   (portions above 192 tokens, head sizes of 64 or 128) every run of 64 tokens makes its own sum L of decayed k v^T
+//   runs   (portions above 192 tokens, or 384 in heads of 64 x 64; head sizes of 64 or 128) every run of 64 tokens makes its own sum L of decayed k v^T
 //          side by side, one thread per state element then folds S <- lambda^n S + L over a request's runs, and every run
 //          makes its outputs from its starting state: the serial chain is one fused multiply-add a run
 //   walk   (portions of at most 32 tokens) S in registers, token by token
@@ -224,7 +224,8 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 // half rounded as the scalar instruction rounds it), operands from shared memory in 16-byte loads without bank conflicts.
 // Everything stays fp32: activations, decay powers, scores, states and sums.
 constexpr int kLinRun = 64;
-constexpr int kLinRunsFrom = 193;          // the shortest portion that is cut into runs
+// The shortest portion that is cut into runs (why: tib_linear_attention).
+static int lin_runs_from(int key_dim, int value_dim) { return key_dim * value_dim <= 64 * 64 ? 385 : 193; }
 constexpr int kLinPad = kLinRun + 4;       // row stride of the transposed q, k and scores
 
 struct LinRunArgs {
@@ -237,6 +238,7 @@ struct LinRunArgs {
   int64_t ldq, ldk, ldv;
   int heads, value_dim, activation;
   int head0, n_heads;     // the heads of these launches (the runs' states are made for some heads at a time)
+  int shortest;           // portion that is cut into runs
 };
 
 // An entry's first run: entries' runs never overlap, since an entry of len tokens has at most len / kLinRun + 1 runs and the
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(256, 2) lin_run_sums_kernel(const T* __restric
   const int tiles = a.value_dim / TV, own = blockIdx.x / tiles, head = a.head0 + own, col0 = (blockIdx.x - own * tiles) * TV;
   const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const int t0 = blockIdx.y * kLinRun;
-  if (t0 >= len || len < kLinRunsFrom) return;
+  if (t0 >= len || len < a.shortest) return;
   const int n = min(kLinRun, len - t0), tid = threadIdx.x;
   if (tid <= kLinRun) pw[tid] = a.powers[head * (kLinRun + 1) + tid];
   __syncthreads();
@@ -348,7 +350,7 @@ __global__ void __launch_bounds__(256) lin_fold_kernel(LinRunArgs a, int key_dim
   const int entry = blockIdx.y, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const size_t per_head = (size_t)key_dim * a.value_dim, width = per_head * a.n_heads;
   const size_t e = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
-  if (len < kLinRunsFrom || e >= width) return;
+  if (len < a.shortest || e >= width) return;
   const float* pw = a.powers + (a.head0 + e / per_head) * (kLinRun + 1);
   const int runs = (len + kLinRun - 1) / kLinRun, last = len - (runs - 1) * kLinRun;
   const float whole = pw[kLinRun], part = pw[last];
@@ -392,7 +394,7 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   const int tiles = a.value_dim / TV, own = blockIdx.x / tiles, head = a.head0 + own, col0 = (blockIdx.x - own * tiles) * TV;
   const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const int t0 = blockIdx.y * kLinRun;
-  if (t0 >= len || len < kLinRunsFrom) return;
+  if (t0 >= len || len < a.shortest) return;
   const int n = min(kLinRun, len - t0), tid = threadIdx.x;
   const float* S = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.n_heads + own) * (size_t)D * a.value_dim + col0;
   constexpr int SV = SR * TV / 4 / 256;                      // 16-byte pieces of a tile of S a thread fetches
@@ -628,10 +630,10 @@ TIB_API int tib_linear_attention_chunk(int key_dim, int value_dim) {
   return 0;
 }
 
-// Tokens of a run, the longest portion the walk takes, and the shortest that is cut into runs.
+// Tokens of a run, the longest portion the walk takes, and the shortest that is cut into runs in heads of these sizes.
 TIB_API int tib_linear_attention_run() { return kLinRun; }
 TIB_API int tib_linear_attention_walk() { return kLinWalk; }
-TIB_API int tib_linear_attention_runs_from() { return kLinRunsFrom; }
+TIB_API int tib_linear_attention_runs_from(int key_dim, int value_dim) { return lin_runs_from(key_dim, value_dim); }
 
 // q, k: [tokens, >= heads * key_dim] and v: [tokens, >= heads * value_dim] with row strides ldq, ldk, ldv (they may be
 // slices of one wider row); out: [tokens, heads * value_dim] fp32; state: [slots, heads, key_dim, value_dim] fp32;
@@ -653,10 +655,12 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   if (!q || !k || !v || !out || !state || !powers || !q_start || !slots) return TIB_E_ARG;
   if (heads < 1 || key_dim < 1 || value_dim < 1 || chunk < 1 || chunk > 32 || n_entries > 65535) return TIB_E_SIZE;
   // The newer kernels take heads of 64 or 128 keys whose values come in whole tiles, rows and state on 16-byte boundaries.
-  // The lines between the three: four portions of 16 heads of 128 x 128 take the walk 14, 16 and 23 us at 8, 9 and 16 tokens and the chunk
-  // kernel 33, 33 and 35; at 64 tokens the chunk kernel takes 78 and the runs 71.  The runs are two launches and an allocation
-  // more, which a step of a few hundred tokens waits for on the host: the layer on 158 and 78 tokens of 12 heads of 64 takes 89 us
-  // in chunks and 98 in runs, so chunks keep portions up to 192.
+  // The lines between the three.  Walk and chunks (four portions of 16 heads of 128 x 128): 14, 16 and 23 us at 8, 9 and 16 tokens
+  // against 33, 33 and 35.  Chunks and runs, the whole layer's device time at 64 / 128 / 192 tokens: one portion of 16 heads of 128 x 128
+  // 43 / 68 / 92 us against 57 / 70 / 72, four of them 87 / 148 / 213 against 76 / 83 / 94; one portion of 12 heads of 64 x 64 27 / 41 /
+  // 53 against 32 / 33 / 33.  On the device alone the lines would lie near 100 tokens.  But a prompt's layer is issued call by call, which
+  // takes some 87 us of the host in chunks and 97 in runs (two launches and an allocation more), and what is shorter on the device
+  // than that waits for the host: runs pay a lone portion from some 200 tokens at 128 x 128 and some 400 at 64 x 64.
   const int64_t size = dtype == TIB_F32 ? 4 : 2;
   const bool aligned = (ldq * size) % 16 == 0 && (ldk * size) % 16 == 0 && (ldv * size) % 16 == 0 &&
                        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)run_state) & 15) == 0;
@@ -665,7 +669,7 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   if (run_powers && forms && (key_dim == 64 || key_dim == 128) && value_dim % 32 == 0 && aligned && (dtype == TIB_F32 || dtype == TIB_BF16)) {
     LinRunArgs r;
     r.q_start = q_start; r.slots = slots; r.powers = run_powers; r.state = state; r.run_state = run_state; r.out = out;
-    r.ldq = ldq; r.ldk = ldk; r.ldv = ldv; r.heads = heads; r.head0 = 0; r.n_heads = heads; r.value_dim = value_dim; r.activation = activation;
+    r.ldq = ldq; r.ldk = ldk; r.ldv = ldv; r.heads = heads; r.head0 = 0; r.n_heads = heads; r.shortest = lin_runs_from(key_dim, value_dim); r.value_dim = value_dim; r.activation = activation;
     if (forms & 1) {
       const int status = dtype == TIB_F32 ? launch_lin_walk<float>(q, k, v, r, key_dim, n_entries, stream)
                                           : launch_lin_walk<__nv_bfloat16>(q, k, v, r, key_dim, n_entries, stream);
@@ -688,7 +692,7 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
       }
 #undef TIB_LIN_GO
     }
-    if (runs) longest = kLinRunsFrom - 1;
+    if (runs) longest = r.shortest - 1;
     if (runs || !(forms & 4)) {
       if (!(forms & 2)) return TIB_OK;
       chunked = n_chunked > 0 && n_chunked < n_entries ? n_chunked : n_entries;

@@ -7,6 +7,7 @@ not take) raises :class:`KernelError`; nothing falls back to another path.
 from __future__ import annotations
 
 import ctypes
+import functools
 from collections.abc import Mapping
 from ctypes import c_float, c_int, c_int64, c_void_p
 
@@ -888,22 +889,16 @@ def linear_attention_chunk(key_dim: int, value_dim: int) -> int:
     return int(lib().tib_linear_attention_chunk(c_int(key_dim), c_int(value_dim)))
 
 
-_linear_sizes: tuple[int, int, int] | None = None
-
-
-def _linear_attention_sizes() -> tuple[int, int, int]:
-    """(tokens of a run, the longest portion that is walked token by token, the shortest that is cut into runs); asked of the
-    library once."""
-    global _linear_sizes
-    if _linear_sizes is None:
-        _linear_sizes = (int(lib().tib_linear_attention_run()), int(lib().tib_linear_attention_walk()),
-                         int(lib().tib_linear_attention_runs_from()))
-    return _linear_sizes
-
-
+@functools.lru_cache(maxsize=None)
 def linear_attention_run() -> int:
     """Tokens of a run of the decayed linear attention (long portions are cut into runs that go side by side)."""
-    return _linear_attention_sizes()[0]
+    return int(lib().tib_linear_attention_run())
+
+
+@functools.lru_cache(maxsize=None)
+def linear_attention_forms(key_dim: int, value_dim: int) -> tuple[int, int]:
+    """(the longest portion that is walked token by token, the shortest that is cut into runs) in heads of these sizes."""
+    return int(lib().tib_linear_attention_walk()), int(lib().tib_linear_attention_runs_from(c_int(key_dim), c_int(value_dim)))
 
 
 # Bytes of run states that a call makes room for at a time: 2,048 tokens of 16 heads of 128 x 128 take 34 MB, and what is above the
@@ -933,15 +928,18 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
         raise KernelError("linear_attention: entry arrays are shorter than n_entries")
     run_state, capacity, run_heads, forms, chunked = None, 0, 0, 0, 0
     if run_powers is not None:
-        run, walk, runs_from = _linear_attention_sizes()
+        run, (walk, runs_from) = linear_attention_run(), linear_attention_forms(key_dim, value_dim)
         _need(run_powers, "run_powers", torch.float32)
         if run_powers.shape != (heads, run + 1):
             raise KernelError("linear_attention: run_powers has the wrong shape")
         if max_q_len > 0:
-            for length in portions or {1: 1, min(max_q_len, walk + 1): 1, max_q_len: 1}:
-                forms |= 1 if length <= walk else 2 if length < runs_from else 4
-        if portions:
-            chunked = sum(count for length, count in portions.items() if walk < length < runs_from)
+            for length, count in (portions or {1: n_entries, min(max_q_len, walk + 1): n_entries, max_q_len: n_entries}).items():
+                if length <= walk:
+                    forms |= 1
+                elif length < runs_from:
+                    forms, chunked = forms | 2, chunked + count
+                else:
+                    forms |= 4
         if forms & 4 and key_dim in (64, 128) and value_dim % 64 == 0:
             capacity = q.shape[0] // run + n_entries
             run_heads = min(heads, max(1, LINEAR_ATTENTION_SCRATCH // (capacity * key_dim * value_dim * 4)))
@@ -1562,6 +1560,12 @@ def pool_blocks(keys: torch.Tensor, values: torch.Tensor, block_table: torch.Ten
         c_int(kv_heads), c_int(dim), c_int(vdim), c_int(pool), _ptr(error_word), c_int(_code(keys.dtype)), _stream()))
 
 
+@functools.lru_cache(maxsize=None)
+def _window_few_rows() -> int:
+    """Rows (tokens x query heads of a key head) of a portion up to which the windowed attention's first tensor-core kernel keeps it."""
+    return int(lib().tib_pooled_window_attention_few_rows())
+
+
 def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor, kv_start: torch.Tensor, slots: torch.Tensor,
                             keys: torch.Tensor, values: torch.Tensor, block_table: torch.Tensor, block_keys: torch.Tensor | None,
                             block_values: torch.Tensor | None, block_block_table: torch.Tensor | None, n_entries: int,
@@ -1620,7 +1624,7 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
             n_splits = 1
     few_rows = -1
     if portions:
-        most = int(lib().tib_pooled_window_attention_few_rows()) * kv_heads // heads
+        most = _window_few_rows() * kv_heads // heads
         few_rows = max((length for length in portions if length <= most), default=0)
     launches = c_int(0)
     _check("pooled_window_attention", lib().tib_pooled_window_attention(
