@@ -885,9 +885,11 @@ def test_prompts_on_keys_and_values_made_for_the_step(heads, dim, rot, vdim, ran
 @pytest.mark.parametrize("order", ["abcd", "cadb", "acbd", "dcba"])
 def test_a_latent_portion_takes_its_own_form_beside_any_others(order, monkeypatch):
     """A prompt of 300 tokens (a) and one of 20 (b) run on keys and values made for the step, a single token (c) and a portion of three
-    (d) folded, whatever lies before, between and behind them; all against the same layer in 32 bits."""
+    (d) folded (told that both forms cost nothing), whatever lies before, between and behind them; all against the same layer in 32 bits."""
     need_gpu()
     from torchinferno_b200.kernels import ops
+    from torchinferno_b200.parts import latent_attention
+    monkeypatch.setattr(latent_attention, "BOTH_FORMS_US", -1e9)
     from torchinferno_b200.parts.base import PartSpec, build_part
     from torchinferno_b200.weights.random_init import random_tensor
     params = {"hidden_size": 64, "heads": 2, "dim": 64, "rot_dim": 32, "value_dim": 64, "kv_rank": 64, "scale": 0.07, "rot_base": 3000.0, "eps": 1e-5,
@@ -985,3 +987,25 @@ def test_latent_rows_off_their_boundaries_stay_folded(monkeypatch):
         outs[dtype] = _run_steps(mixer, cache, [[("a", 150)], [("a", 50)]], {"a": x["a"].to(dtype)})["a"]
     err = _row_error(outs[torch.bfloat16], outs[torch.float32])
     assert err.max() <= 0.03, (int(err.argmax()), float(err.max()))      # (the bound of the layer's other tests in bfloat16)
+
+
+def test_latent_tokens_beside_a_prompt_and_alone():
+    """Single tokens whose few keys are made with a prompt's, against the same tokens folded in a step of their own: either form rounds
+    to bfloat16 (keys, values and a part of the queries; the folded queries), so they differ by no more than twice a form's bound."""
+    need_gpu()
+    from torchinferno_b200.parts.base import PartSpec, build_part
+    from torchinferno_b200.weights.random_init import random_tensor
+    params = {"hidden_size": 64, "heads": 3, "dim": 64, "rot_dim": 32, "value_dim": 128, "kv_rank": 64, "scale": 0.07, "rot_base": 3000.0, "eps": 1e-5,
+              "gate": True, "sink": True}
+    mixer = build_part("mixer", PartSpec("latent_attention", params), dtype=torch.bfloat16, device=CUDA)
+    _bind(mixer, {ws.name: random_tensor(ws, 4, dtype=torch.bfloat16) for ws in mixer.weight_specs()}, torch.bfloat16, "mix.")
+    x = {r: torch.randn(n, 64, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16) for i, (r, n) in enumerate((("a", 200), ("b", 144), ("c", 31)))}
+    outs = []
+    for steps in ([[("b", 140), ("c", 30)], [("b", 1), ("a", 200), ("c", 1)], [("b", 3)]], [[("b", 140), ("c", 30)], [("b", 1), ("c", 1)], [("a", 200)], [("b", 3)]]):
+        cache = _cache_for(mixer, torch.bfloat16, 16, 64, 4, 300)
+        for r in x:
+            cache.open(r)
+        outs.append(_run_steps(mixer, cache, steps, x))
+    assert _row_error(outs[0]["a"], outs[1]["a"]).max() <= 0.01      # (the same form: a last bit of the products)
+    for r in "bc":
+        assert _row_error(outs[0][r], outs[1][r]).max() <= 0.06

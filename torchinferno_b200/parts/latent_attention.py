@@ -115,7 +115,8 @@ class LatentAttention(Mixer):
     # The unfolded form multiplies 2 (dim + value_dim) rank numbers a head and key once, and saves some two thirds of the folded
     # kernel's products on every (query, key) pair, which run at a tenth of the library's rate: it wins from about six
     # queries a key, and is taken from sixteen (the layer on two prompts of 1,667 and 833 tokens, 16 heads: 1,226 us
-    # folded, 165 unfolded; error against 64 bits 0.0048 and 0.0045).  A portion's own length decides, whatever else is in the step.
+    # folded, 165 unfolded; error against 64 bits 0.0048 and 0.0045).  A step of prompts alone unfolds them all, a step of shorter
+    # portions none; a step that mixes them takes what :func:`_plan` finds cheapest.
     UNFOLD_QUERIES = 16
     # Room for the rows, keys and values made at a time (two prompts of 1,667 and 833 tokens take 24 MB at 16 heads of 128 + 128): what
     # is above the bound goes entry by entry, and some heads at a time.
@@ -126,46 +127,54 @@ class LatentAttention(Mixer):
         if self.unfold is None or batch.n_multi == 0 or len(batch.entries) != batch.n_entries:
             return None
         row_bytes = 2 * (self.dim + self.value_dim + self.kv_rank + self.rot_dim)      # (with one head's key and value)
-        key = ("latent", self.UNFOLD_QUERIES, self.UNFOLD_BYTES // row_bytes)
+        key = (self.UNFOLD_QUERIES, self.UNFOLD_BYTES // row_bytes, self.heads, self.dim + self.value_dim, self.kv_rank, self.rot_dim)
         if key not in batch.plans:
-            batch.plans[key] = _plan(batch.entries, *key[1:])
+            batch.plans[key] = _plan(batch.entries, *key)
         return batch.plans[key]
 
     def _unfolded_rows(self, batch) -> int:
         """Rows of keys and values to make for this step, 0 where the folded form is to run throughout."""
         plan = self._plan(batch)
-        return sum(rows for _, _, rows in plan.groups) if plan else 0
+        return plan.rows if plan else 0
 
     def _unfolded(self, plan: "_Plan", q: torch.Tensor, dkv: torch.Tensor, gate: torch.Tensor | None, out: torch.Tensor, ctx: LayerContext) -> None:
         """The portions of the plan's groups, on keys and values made for them."""
-        kv, batch, h = ctx.kv, ctx.batch, self.heads
-        tokens = slice(*plan.long_tokens)
-        ops.latent_append(dkv[tokens], q[tokens], None, kv.keys if kv.writes else None, batch.positions[tokens], batch.token_slot[tokens],
-                          kv.block_table, self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, self.kv_rank, self.rot_dim,
+        kv, batch, h, width = ctx.kv, ctx.batch, self.heads, self.dim + self.value_dim
+        rows_dkv, rows_q, positions, token_slot = dkv, q, batch.positions, batch.token_slot
+        if not plan.whole:
+            tokens = slice(*plan.long_tokens)
+            rows_dkv, rows_q, positions, token_slot = dkv[tokens], q[tokens], positions[tokens], token_slot[tokens]
+        ops.latent_append(rows_dkv, rows_q, None, kv.keys if kv.writes else None, positions, token_slot, kv.block_table,
+                          self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, self.kv_rank, self.rot_dim,
                           ctx.error_word, half_pairs=self.half_pairs)
-        for first, end, rows in plan.groups:
+        for first, end, rows, longest, longest_kv in plan.groups:
+            q_start, kv_start, slots = batch.q_start, batch.kv_start, batch.slots
+            if not plan.whole:
+                q_start, kv_start, slots = q_start[first:end + 1], kv_start[first:end], slots[first:end]
+            at_a_time = min(h, max(1, (self.UNFOLD_BYTES - 2 * rows * (self.kv_rank + self.rot_dim)) // (2 * rows * width)))
             latent = torch.empty((rows, self.kv_rank), dtype=q.dtype, device=q.device)
             rotated = torch.empty((rows, self.rot_dim), dtype=q.dtype, device=q.device)
-            q_start, kv_start, slots = batch.q_start[first:end + 1], batch.kv_start[first:end], batch.slots[first:end]
-            entries, width = batch.entries[first:end], self.dim + self.value_dim
-            at_a_time = min(h, max(1, (self.UNFOLD_BYTES - 2 * rows * (self.kv_rank + self.rot_dim)) // (2 * rows * width)))
-            ops.latent_gather(kv.keys, kv.block_table, q_start, kv_start, slots, end - first, max(e.kv_start + e.q_len for e in entries),
-                              latent, rotated, ctx.error_word)
+            ops.latent_gather(kv.keys, kv.block_table, q_start, kv_start, slots, end - first, longest_kv, latent, rotated, ctx.error_word)
             for head in range(0, h, at_a_time):
                 heads = self.unfold if at_a_time == h else self.unfold.rows(head * width, min(h, head + at_a_time) * width)
-                ops.latent_prefill(q, linear(latent, heads), rotated, out, q_start, kv_start, end - first, max(e.q_len for e in entries),
-                                   h, self.dim, self.value_dim, self.scale, self.UNFOLD_QUERIES, head, gate, self.gate_per_head, self.sink,
-                                   ctx.error_word)
+                ops.latent_prefill(q, linear(latent, heads), rotated, out, q_start, kv_start, end - first, longest, h, self.dim, self.value_dim,
+                                   self.scale, plan.shortest, head, gate, self.gate_per_head, self.sink, ctx.error_word)
 
     def _folded(self, q: torch.Tensor, dkv: torch.Tensor, gate: torch.Tensor | None, heads_out: torch.Tensor, ctx: LayerContext,
-                entries: slice, first_row: int, max_q_len: int, max_kv_len: int) -> None:
-        """Portions of at most ``max_q_len`` tokens among these entries, whose tokens the rows given are, from the step's
-        ``first_row`` on."""
-        kv, batch, n, h, c, r = ctx.kv, ctx.batch, q.shape[0], self.heads, self.kv_rank, self.rot_dim
-        width, tokens = c + r, slice(first_row, first_row + n)
-        q_start, kv_start, slots = batch.q_start[entries.start:entries.stop + 1], batch.kv_start[entries], batch.slots[entries]
+                plan: "_Plan | None") -> None:
+        """The whole step folded, or the short portions of the plan."""
+        kv, batch, h, c, r = ctx.kv, ctx.batch, self.heads, self.kv_rank, self.rot_dim
+        positions, token_slot, q_start, kv_start, slots = batch.positions, batch.token_slot, batch.q_start, batch.kv_start, batch.slots
+        first_row, entries, max_q_len, max_kv_len = 0, batch.n_entries, batch.max_q_len, batch.max_kv_len
+        if plan is not None:
+            tokens, (first, end) = slice(*plan.short_tokens), plan.short
+            q, dkv, heads_out, gate = q[tokens], dkv[tokens], heads_out[tokens], None if gate is None else gate[tokens]
+            positions, token_slot = positions[tokens], token_slot[tokens]
+            q_start, kv_start, slots = q_start[first:end + 1], kv_start[first:end], slots[first:end]
+            first_row, entries, max_q_len, max_kv_len = tokens.start, end - first, plan.short_q_len, plan.short_kv_len
+        n, width = q.shape[0], c + r
         folded = torch.empty((n, h, width), dtype=torch.float32, device=q.device)
-        ops.latent_append(dkv, q, folded, kv.keys if kv.writes else None, batch.positions[tokens], batch.token_slot[tokens], kv.block_table,
+        ops.latent_append(dkv, q, folded, kv.keys if kv.writes else None, positions, token_slot, kv.block_table,
                           self.latent_norm_weight, self.eps, self.inv_freq, h, self.dim, c, r, ctx.error_word,
                           half_pairs=self.half_pairs)
         q_plain = q.as_strided((n, h, self.dim), (q.stride(0), self.dim + r, 1))
@@ -176,9 +185,8 @@ class LatentAttention(Mixer):
             ops.library_gemm_batched(q_plain, self.uk_weight, folded[:, :, :c], w_kn=True)
         latent_out = torch.empty((n, h, c), dtype=torch.float32, device=q.device)
         rows = torch.empty((n, h, c), dtype=q.dtype, device=q.device) if q.dtype != torch.float32 else None
-        mixed = ops.latent_attention(folded, kv.keys, latent_out, q_start, kv_start, slots, kv.block_table,
-                                     slots.shape[0], max_q_len, h, c, r, self.scale, ctx.error_word, max_kv_len=max_kv_len,
-                                     sink=self.sink, merged=rows, first_row=first_row)
+        mixed = ops.latent_attention(folded, kv.keys, latent_out, q_start, kv_start, slots, kv.block_table, entries, max_q_len, h, c, r,
+                                     self.scale, ctx.error_word, max_kv_len=max_kv_len, sink=self.sink, merged=rows, first_row=first_row)
         if q.dtype == torch.float32:
             for j in range(h):
                 ops.gemm_f32(latent_out[:, j], self.uv_weight[j], heads_out[:, j])
@@ -210,19 +218,21 @@ class LatentAttention(Mixer):
         if plan and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and kv.keys.stride(0) % 8 == 0 and kv.keys.data_ptr() % 16 == 0 \
                 and (gate is None or self.gate_per_head or gate.data_ptr() % 16 == 0):
             if plan.short:      # (first: where long portions lie between, their rows are written here too, and again below)
-                rows = slice(*plan.short_tokens)
-                self._folded(q[rows], dkv[rows], None if gate is None else gate[rows], heads_out[rows], ctx, slice(*plan.short), rows.start,
-                             plan.short_q_len, plan.short_kv_len)
+                self._folded(q, dkv, gate, heads_out, ctx, plan)
             self._unfolded(plan, q, dkv, gate, heads_out, ctx)
         else:
-            self._folded(q, dkv, gate, heads_out, ctx, slice(0, batch.n_entries), 0, batch.max_q_len, batch.max_kv_len)
+            self._folded(q, dkv, gate, heads_out, ctx, None)
         return linear(heads_out.view(n, h * self.value_dim), self.o_weight)
 
 
 @dataclass(frozen=True)
 class _Plan:
     """How a step is shared out between the two forms."""
-    groups: tuple[tuple[int, int, int], ...]      # entries first .. end - 1 whose keys and values are made together, and their rows
+    # entries first .. end - 1 whose keys and values are made together, their rows, their longest portion and context
+    groups: tuple[tuple[int, int, int, int, int], ...]
+    rows: int                                     # of all groups
+    whole: bool                                   # one group holds the step
+    shortest: int                                 # portion among them that runs on these
     long_tokens: tuple[int, int]                  # the tokens from the first to the last of the groups' entries
     short: tuple[int, int] | None                 # the entries from the first to the last that stay folded, and their tokens
     short_tokens: tuple[int, int]
@@ -230,13 +240,45 @@ class _Plan:
     short_kv_len: int
 
 
-def _plan(entries: Sequence[EntryPlacement], queries: int, most_rows: int) -> _Plan | None:
-    """Portions of at least ``queries`` tokens run on keys and values made for the step.  Neighbours share a product up to ``most_rows``
-    rows, across short portions too where these add no more rows than there are."""
+# What the folded form's launches, and those of both forms in one step, take the host that issues a prompt's layer call by call beyond
+# the unfolded form's, in us (130 a layer unfolded, 145 folded, some 240 with both).
+FOLDED_HOST_US, BOTH_FORMS_US = 15.0, 110.0
+
+
+def _folded_us(entries: Sequence[EntryPlacement], heads: int, rank: int, rot: int) -> float:
+    """Roughly what the folded form takes the device: products at 45 TFLOP/s, but a block walks its context 64 keys in 8 us, unless the
+    step has single tokens only, whose contexts are shared out."""
+    pairs = sum(e.q_len * (e.kv_start + (e.q_len + 1) / 2) for e in entries)
+    chain = 0.0 if all(e.q_len == 1 for e in entries) else max(8.0 * (e.kv_start + e.q_len) / 64 for e in entries)
+    return max(pairs * heads * 2 * (2 * rank + rot) / 45e6, chain)
+
+
+def _unfolded_us(entries: Sequence[EntryPlacement], heads: int, width: int, rank: int) -> float:
+    """The same of the unfolded form: keys and values at 1,100 TFLOP/s, then a block per head and 128 tokens (8 us, and 2 for every 128
+    keys), 148 of them side by side."""
+    rows = sum(e.kv_start + e.q_len + 64 for e in entries)
+    each = [8.0 + 2.0 * (e.kv_start + e.q_len) / 128 for e in entries]
+    blocks = sum(us * -(-e.q_len // 128) for us, e in zip(each, entries))
+    return rows * heads * width * rank * 2 / 1.1e9 + max(blocks * heads / 148, max(each))
+
+
+def _plan(entries: Sequence[EntryPlacement], queries: int, most_rows: int, heads: int, width: int, rank: int, rot: int) -> _Plan | None:
+    """Portions of at least ``queries`` tokens run on keys and values made for the step, shorter ones folded.  Where a step has both,
+    they run in one form, or each in its own, by what that takes (64 single tokens at 4,000 beside a prompt of 512: 673 us folded, 352 apart;
+    eight at 1,000 beside it: 122 unfolded and 89 apart, which the second set of launches costs the host).  Neighbours share a product
+    up to ``most_rows`` rows, across folded portions too where these add no more rows than there are."""
     padded = [-(-(e.kv_start + e.q_len) // ops.LATENT_TILE) * ops.LATENT_TILE for e in entries]
     long = [i for i, e in enumerate(entries) if e.q_len >= queries]
     if not long:
         return None
+    if len(long) < len(entries):
+        folded, unfolded = _folded_us(entries, heads, rank, rot) + FOLDED_HOST_US, _unfolded_us(entries, heads, width, rank)
+        apart = _unfolded_us([e for e in entries if e.q_len >= queries], heads, width, rank) + BOTH_FORMS_US \
+            + _folded_us([e for e in entries if e.q_len < queries], heads, rank, rot)
+        if folded < min(unfolded, apart):
+            return None
+        if unfolded <= apart:
+            long, queries = list(range(len(entries))), 1
     groups = []
     for i in long:
         between = sum(padded[groups[-1][1]:i]) if groups else 0
@@ -245,11 +287,13 @@ def _plan(entries: Sequence[EntryPlacement], queries: int, most_rows: int) -> _P
         else:
             groups.append((i, i + 1, padded[i]))
     taken = set(long)
+    longest = lambda part: (max(e.q_len for e in part), max(e.kv_start + e.q_len for e in part))
+    groups = tuple((first, end, rows, *longest(entries[first:end])) for first, end, rows in groups)
     short = [i for i in range(len(entries)) if i not in taken]
     tokens = lambda first, last: (entries[first].q_start, entries[last].q_start + entries[last].q_len)
-    return _Plan(tuple(groups), tokens(long[0], long[-1]), (short[0], short[-1] + 1) if short else None,
-                 tokens(short[0], short[-1]) if short else (0, 0), max((entries[i].q_len for i in short), default=0),
-                 max((entries[i].kv_start + entries[i].q_len for i in short), default=0))
+    return _Plan(groups, sum(g[2] for g in groups), groups[0][:2] == (0, len(entries)), queries, tokens(long[0], long[-1]),
+                 (short[0], short[-1] + 1) if short else None, tokens(short[0], short[-1]) if short else (0, 0),
+                 *(longest([entries[i] for i in short]) if short else (0, 0)))
 
 
 register_part("mixer", "latent_attention", LatentAttention)
