@@ -15,7 +15,7 @@
 //                    the columns of S they come from.  A head's sink and the output gate are applied at the end.
 //
 // What bounds it: the tensor core (two products, the second twice) at two stages of 80 KB of keys and values.  Two prompts of 1,667
-// and 833 tokens, 16 heads of 128 + 64 over a rank of 512: gather 11 us, product 15, attention 67, where the folded form took 20 for
+// and 833 tokens, 16 heads of 128 + 64 over a rank of 512: gather 12 us, product 15, attention 68 (cold), where the folded form took 20 for
 // folding, 1,094 for the attention, 21 for a cast, 12 for unfolding and 20 for the gate.
 #include "tcgen05.cuh"
 #include <math_constants.h>

@@ -219,7 +219,7 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 // ---------------------------------------------------------------------------------------------------------- runs
 // The walk above is one serial chain of 64 chunks for 2,048 tokens, each with four barriers, on 512 blocks that each see 32 of a
 // run's 128 columns: 980 us for two portions of 1,366 and 682 tokens, 16 heads of 128 x 128, of which the fp32 arithmetic
-// (3.3 GFLOP here) is some 50 us.  In runs the three launches below take 144 us.  What bounds them is the fp32 pipe: register
+// (3.3 GFLOP here) is some 50 us.  In runs the three launches below take 49 + 27 + 82 us (cold).  What bounds them is the fp32 pipe: register
 // tiles of 8 x 8 (sums) and 4 x 8 (outputs) per thread, products in pairs of neighbouring columns (fma.rn.f32x2, each
 // half rounded as the scalar instruction rounds it), operands from shared memory in 16-byte loads without bank conflicts.
 // Everything stays fp32: activations, decay powers, scores, states and sums.
@@ -521,7 +521,7 @@ lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
 // ---------------------------------------------------------------------------------------------------------- walk
 // Single tokens and portions of a few: a block holds 32 columns of one head's S in registers (a thread four neighbouring columns
 // of every 32nd row), so a step reads and writes the state once, 16 bytes a load with all of a thread's loads in flight.
-// What bounds it is the launch and one trip to memory: eight tokens of 16 heads of 128 x 128 12 us, 41 in the chunk kernel,
+// What bounds it is the launch and one trip to memory: eight tokens of 16 heads of 128 x 128 8 us (cold), 42 in the chunk kernel,
 // whose score is one thread's chain of 128 products for a single token.
 constexpr int kLinWalk = 32;            // the longest portion it takes
 constexpr int kLinWalkStage = 8;        // tokens it holds in shared memory at a time

@@ -16,9 +16,9 @@
 // cost 12 in the pass.)
 //
 // What bounds it: a prompt reads every expert's weights once (134 MB a product at 32 experts of 1024 on rows of 2048: 21 us) and
-// multiplies at the rate shared memory feeds 128 x 128 x 16 products; 2,048 tokens x 4 choices take 62 us a product where the
-// mma.sync kernel before took 199 and 207.  A decode step streams the chosen experts' weights with 180 KB of them on their way
-// per SM: eight tokens x 4, gate and up of 1024 on 2048: 47 us for 176 MB (68 before), down 24 (38 before).
+// multiplies at the rate shared memory feeds 128 x 128 x 16 products; 2,048 tokens x 4 choices take 68 us gathered and 62 sorted where
+// the mma.sync kernel before took 199 and 207 (cold).  A decode step streams the chosen experts' weights with 144 KB of them on their
+// way per SM (180 with the token rows): eight tokens x 4, gate and up of 1024 on 2048: 42 us for 176 MB (68 before), down 24 (38).
 // Every wait is bounded and reports in error_word, as in gemm_tcgen05.cu.
 #include "moe.cuh"
 #include "mma.cuh"

@@ -1151,8 +1151,9 @@ TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_s
   // bf16 steps run on the tensor cores, single tokens too (their tiles come in by cp.async, 16 bytes a piece, where the
   // other kernel waits for one element at a time); 32-bit and head sizes that are no multiples of 8 run on the CUDA cores.
   // Portions of prompts that fill the rows of a tile take tcgen05 products where pages and head sizes suit the copies; each portion by its
-  // own length, so that a single token beside a prompt is not given a block of 128 rows (64 single tokens at 4,000 beside eight
-  // portions of 33, 16 / 8 heads of 128: the layer took 163 us when the step's longest portion chose for all, 132 without tcgen05).
+  // own length, so that a single token beside a prompt is not given a block of 128 rows and keeps its bits.  (64 single tokens at 4,000
+  // beside a prompt of 512, 16 / 8 heads of 128: the layer takes 176 us, 189 when the step's longest portion chose for all, 216 on
+  // mma.sync alone; beside eight portions of 33 it takes 146, 156 and 126, since there one launch held them all.)
   bool whole_step = true;
   if (dtype == TIB_BF16 && !force_simt && window_tcgen05_takes(a, q, out, max_q_len)) {
     const int status = window_tcgen05(q, out, a, n_entries, max_q_len, stream);

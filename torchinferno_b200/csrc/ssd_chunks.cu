@@ -16,7 +16,7 @@
 //
 // The walk of ssd_scan_kernel spends five fp32 operations per state element and token twice over (two prompts of 1,366 and 682
 // tokens, 64 heads of 64 with a state of 128: 182 + 32 + 264 us, the fp32 pipe at 40 %).  Here a token costs its share of the
-// products above on mma.sync: 40 + 35 + 95 us cold.  Error against 64 bits there: y 9.8e-8, the walk 8.5e-8; with steps of e^-8 and
+// products above on mma.sync: 39 + 32 + 98 us cold.  Error against 64 bits there: y 9.8e-8, the walk 8.5e-8; with steps of e^-8 and
 // less, where the walk adds a thousand small terms one by one, 1e-7 against 6e-6.  What bounds it: the legacy tensor path with operands from shared memory, and the
 // states' way through the L2 (one of 32 KB a head and chunk, written twice and read twice).
 #include "state_space.cuh"

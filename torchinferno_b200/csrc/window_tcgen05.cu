@@ -12,7 +12,7 @@
 //
 // What bounds it: a block's chain of some six tiles (two products, the second twice, with the softmax's eight warps between them: a
 // third of the issue slots, two warps a scheduler) and its start and end, two blocks an SM one after the other: two portions
-// of 1,366 and 682 tokens, 16 / 8 heads of 128, window 512, blocks of 64: 84 us cold, where the mma.sync kernel (64 x 64 tiles)
+// of 1,366 and 682 tokens, 16 / 8 heads of 128, window 512, blocks of 64: 83 us cold, where the mma.sync kernel (64 x 64 tiles)
 // takes 173.
 // Every wait is bounded and reports in error_word.
 #include "tcgen05.cuh"
