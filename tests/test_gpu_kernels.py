@@ -896,6 +896,33 @@ def test_aligned_fp32_product_has_the_plain_kernels_bits(m, n, k):
     assert torch.equal(ops.gemm_f32(x, w, torch.empty(m, n, device="cuda")), plain)
 
 
+# (edges of the tiles: 128 features, 16 to 80 rows, 64 k a step and 128 a sum)
+@pytest.mark.parametrize("m, n, k", [(1, 8192, 512), (16, 7297, 576), (17, 512, 8192), (80, 6560, 640), (81, 2000, 2112), (161, 4100, 1024), (330, 7400, 576)])
+def test_fp32_product_in_three_terms(m, n, k, monkeypatch):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    x, w = dev(rnd(m, k, scale=2)), dev(rnd(n, k, seed=3))
+    error = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = ops.gemm_f32(x, w, torch.empty(m, n, device="cuda"), error)
+    # The tensor core cuts off at most 2^-23 of a sum at each of the eight instructions over 128 k, the sums of those are added in
+    # fp32, and the terms left out are below 2 * 2^-24 of a product: 2^-23 (8 + k / 256 + 1) of the products' magnitudes, and one for the small terms.
+    bound = 2.0 ** -23 * (10 + k / 256) * (x.double().abs() @ w.double().abs().T)
+    assert ((out.double() - x.double() @ w.double().T).abs() <= bound).all() and int(error) == 0
+    for rows in (slice(m // 2, m // 2 + 1), slice(0, max(1, m - 3))):      # a row does not depend on the rows beside it
+        few = x[rows].contiguous()
+        assert torch.equal(ops.gemm_f32(few, w, torch.empty(len(few), n, device="cuda")), out[rows])
+    monkeypatch.setattr(ops, "F32_TERMS_BYTES", 1)                         # 128 rows at a time, into a wider matrix
+    wide = torch.zeros(m, n + 3, device="cuda")
+    ops.gemm_f32(x, w, wide[:, :n])
+    assert torch.equal(wide[:, :n], out) and not wide[:, n:].any()
+    # infinities, NaN and numbers that no bf16 number reaches come out as in multiply-adds
+    x[0, 5], w[3, 9], w[7, 100], x[m - 1, k - 1] = math.inf, math.nan, -math.inf, 3.4e38
+    odd = torch.empty(m, k + 1, device="cuda")[:, :k]                      # (rows off their 16-byte boundaries: the plain kernel)
+    odd.copy_(x)
+    out, plain = (ops.gemm_f32(t, w, torch.empty(m, n, device="cuda")) for t in (x, odd))
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf()) and not torch.isfinite(out[:, 7]).any()
+
+
 # ------------------------------------------------- linear attention in runs and token by token
 @pytest.mark.parametrize("lens, heads, key_dim, value_dim", [
     ([1, 1, 1], 3, 128, 128), ([32, 5, 9], 2, 64, 96),                        # token by token, to its longest portion

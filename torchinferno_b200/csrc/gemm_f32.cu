@@ -7,6 +7,8 @@
 // `F.linear` calls: src/torchinferno/models/llama3/pipeline.py:206-208,245,248-250,400).
 // Optionally w and/or x may be bf16 in memory; they are widened on load.
 //
+// Weights that gemm_f32_tcgen05.cu takes (by their sizes) run there; this file has the products of small, odd or bf16 weights.
+//
 // Two kernels with the same sums, bit for bit.  32-bit operands whose rows are 16-byte aligned run through a ring of four
 // shared-memory stages (cp.async, 16 k each) with up to 8 x 8 outputs a thread; everything else (bf16 in memory, odd
 // strides) runs the plain kernel.

@@ -1,0 +1,416 @@
+// The 32-bit matrix product out[M, N] = x[M, K] . w[N, K]^T on the tensor cores, with 32-bit operands and sums.
+//
+// A float is the sum of three bf16 numbers (8 bits of its 24 each, rounded to nearest): a = a0 + a1 + a2.  The product of two
+// floats is then nine products of bf16 numbers, each exact in fp32; the six of them that are above 2^-24 of the whole are made,
+//     a0 b0   |   a0 b1 + a1 b0   |   a0 b2 + a1 b1 + a2 b0
+// each group in an accumulator of its own, for the tensor core cuts sums off where an fp32 addition rounds: the small terms lose
+// nothing that way, and a0 b0 is only summed over 128 k there (eight instructions), then added to the output's sum in registers as an
+// ordinary fp32 number.  The terms of the rows lie behind one another in shared memory, so that four instructions make the six products: a0 with
+// b0, a0 with b1 and b2 side by side, a1 with b0 and b1, a2 with b0.  Every output is summed over k in the same order whatever the number of rows, so a row's bits do not depend on its
+// neighbours or on the tile's width.
+//
+// The weights are the 128-row operand, from tensor memory; rows of x are the other (a tile takes up to 80 of them, in sixteens):
+//   warps 0..15   turn the step's 128 x 64 weights, as they came into shared memory, into three terms in tensor memory
+//   warp 16       one lane: TMA of the weights and of the rows' three terms (made by split_rows_kernel once a call: every tile of features
+//                 reads them)
+//   warp 17       issues the MMAs (the whole warp walks the loop, one lane issues: descriptors then stay in uniform registers); owns tensor
+//                 memory, all of it: a step's terms of the weights twice, the accumulator of a0 b0 twice, the small ones once
+//   warps 18..25  add the accumulators of 128 k up in registers while the next ones are made, and store the rows
+//
+// What bounds it: the warp that issues the MMAs, which waits once and issues 16 instructions a step of 64 k (0.95 us at 80 rows, of which 0.5 are
+// products), and for the last round of tiles the SMs that have none.  A wait for the rows, one for each half of the weights' terms and one
+// commit each made it 1.15 us; a lane issuing alone takes 45 cycles an instruction instead of 8.  301 rows, us, against gemm_f32.cu's fused
+// multiply-adds: 16,384 x 2,048 123 (536), 2,048 x 8,192 98 (431), 2,048 x 2,048 33 (111); 8 rows: 31 (68), 84 (146), 26 (39).
+// Error against 64 bits (2-norm): 1.4e-7 at 2,048 k and 2.0e-7 at 8,192, where multiply-adds in order have 8.1e-7 and 1.6e-6; numbers of one
+// sign 1.6e-7 (6.3e-7); sums over 256 k 2.4e-7, for a tenth off the time.
+// An output that is not finite is worked out again with fused multiply-adds in order (an infinity's terms make NaN of it).
+#include "mma.cuh"
+#include "cluster.cuh"
+
+namespace tib {
+
+constexpr int kFtM = 128, kFtK = 64, kFtRows = 80, kFtThreads = 832, kFtChunk = 2;      // (steps of 64 k in a chunk)
+constexpr int kFtGroups = (kFtRows / 16 + 1) / 2;               // groups of 16 rows a warp adds up
+constexpr uint32_t kFtW = kFtM * kFtK * 4;                      // a step's weights in shared memory
+constexpr uint32_t kFtTermCols = 3 * kFtK / 2;                  // in tensor memory: a step's terms of the weights, twice
+constexpr uint32_t kFtSums = 2 * kFtTermCols;                   // a0 b0 twice, then the two small groups
+
+__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// The three terms of two floats, packed.
+__device__ __forceinline__ void ft_split2(float a, float b, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
+  t0 = pack_bf16(a, b);
+  f2_unpack(f2_sub(f2_pack(a, b), f2_pack(__uint_as_float(t0 << 16), __uint_as_float(t0 & 0xffff0000u))), a, b);
+  t1 = pack_bf16(a, b);
+  f2_unpack(f2_sub(f2_pack(a, b), f2_pack(__uint_as_float(t1 << 16), __uint_as_float(t1 & 0xffff0000u))), a, b);
+  t2 = pack_bf16(a, b);
+}
+
+// The three terms of x, [3][rows][K]; grid-stride, four elements a thread.
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, int64_t ldx, int rows, int K, __nv_bfloat16* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t quarters = (int64_t)rows * (K / 4), plane = (int64_t)rows * K;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < quarters; e += (int64_t)gridDim.x * 256) {
+    const int64_t r = e / (K / 4);
+    const int c = (int)(e - r * (K / 4)) * 4;
+    const float4 v = *reinterpret_cast<const float4*>(x + r * ldx + c);
+    uint2 t[3];
+    ft_split2(v.x, v.y, t[0].x, t[1].x, t[2].x);
+    ft_split2(v.z, v.w, t[0].y, t[1].y, t[2].y);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(out + i * plane + r * K + c) = t[i];
+  }
+}
+
+// An output whose terms did not add up to a finite number.
+__device__ __noinline__ float ft_plain_sum(const float* __restrict__ x, const float* __restrict__ w, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K && s == s; ++k) s = fmaf(x[k], w[k], s);
+  return s;
+}
+
+// One lane of the warp.
+__device__ __forceinline__ uint32_t ft_elect() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one;
+}
+// The product with the weights in tensor memory, issued by the leader of a warp that is together.
+__device__ __forceinline__ void ft_mma(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+
+__device__ __forceinline__ void ft_tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void ft_tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+
+struct FtArgs {
+  const float* x;
+  const float* w;
+  float* out;
+  int64_t ldx, ldw, ldo;
+  int M, N, K;
+  int rows;               // rows of a tile (a multiple of 16, at most kFtRows)
+  int w_stages, x_stages;
+  int* error_word;
+};
+
+__global__ void __launch_bounds__(kFtThreads, 1)
+gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, FtArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  unsigned char* smem_gen = smem_raw + (base - smem_u32(smem_raw));
+  // Two rings: the weights' places are free again once they are converted, the rows' once they are multiplied.
+  const uint32_t xplane = (uint32_t)a.rows * kFtK * 2, xring = base + a.w_stages * kFtW;
+  const uint32_t bars = xring + a.x_stages * 3 * xplane;
+  auto w_full_bar = [&](int s) { return bars + 8u * s; };
+  auto w_empty_bar = [&](int s) { return bars + 8u * (8 + s); };
+  auto x_full_bar = [&](int s) { return bars + 8u * (16 + s); };
+  auto x_empty_bar = [&](int s) { return bars + 8u * (24 + s); };
+  auto acc_full_bar = [&](int b) { return bars + 8u * (32 + b); };
+  auto acc_empty_bar = [&](int b) { return bars + 8u * (34 + b); };
+  const uint32_t small_empty_bar = bars + 8u * 36, tmem_slot = bars + 8u * 37;
+  volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - base));
+
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 8; ++s) {
+      mbar_init(w_full_bar(s), 1);
+      mbar_init(w_empty_bar(s), 16);
+      mbar_init(x_full_bar(s), 1 + 16);      // (the rows' copies, and the weights' terms)
+      mbar_init(x_empty_bar(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full_bar(b), 1);
+      mbar_init(acc_empty_bar(b), 8);
+    }
+    mbar_init(small_empty_bar, 8);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 17) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tmem_slot), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  pdl_wait();
+  pdl_trigger();
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot_ptr;
+
+  const int m_tiles = (a.M + a.rows - 1) / a.rows, f_tiles = (a.N + kFtM - 1) / kFtM, num_tiles = m_tiles * f_tiles;
+  const int k_steps = a.K / kFtK;
+  const int own = (int)blockIdx.x < num_tiles ? (num_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;      // tiles of this block
+  const int total = own * k_steps;
+
+  if (warp < 16) {
+    // lane: a feature; the warp's 16 of the step's 64 k (which come as two copies of 32 k: rows of 128 bytes, swizzled)
+    const int quarter = warp & 3, part = warp >> 2, r = quarter * 32 + lane;
+    int ws = 0, xs = 0, before = 0;      // (places of this step, and of the one that used these terms' columns before)
+    uint32_t wphase = 0, bphase = 0;
+    const uint32_t dst = tmem_base + ((uint32_t)(quarter * 32) << 16) + part * 8;
+    for (int it = 0; it < total; ++it) {
+      if (!mbar_wait(w_full_bar(ws), wphase)) {
+        if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0071);
+        break;
+      }
+      const unsigned char* src = smem_gen + (size_t)ws * kFtW + (part >> 1) * (kFtW / 2) + r * 128;
+      uint32_t t[3][8];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float4 v = *reinterpret_cast<const float4*>(src + ((((part & 1) * 4 + c) ^ (r & 7)) << 4));
+        ft_split2(v.x, v.y, t[0][2 * c], t[1][2 * c], t[2][2 * c]);
+        ft_split2(v.z, v.w, t[0][2 * c + 1], t[1][2 * c + 1], t[2][2 * c + 1]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(w_empty_bar(ws));
+      if (it >= 2) {      // (the products of two steps ago are done)
+        if (!mbar_wait(x_empty_bar(before), bphase)) {
+          if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0076);
+          break;
+        }
+        if (++before == a.x_stages) {
+          before = 0;
+          bphase ^= 1;
+        }
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+      for (int p = 0; p < 3; ++p) ft_tmem_st8(dst + (it & 1) * kFtTermCols + p * (kFtK / 2), t[p]);
+      asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x_full_bar(xs));
+      if (++ws == a.w_stages) {
+        ws = 0;
+        wphase ^= 1;
+      }
+      if (++xs == a.x_stages) xs = 0;
+    }
+  } else if (warp == 16) {
+    if (lane == 0) {
+      int ws = 0, xs = 0;
+      uint32_t wphase = 1, xphase = 1;
+      bool ok = true;
+      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+        const int m0 = t % m_tiles * a.rows, f0 = t / m_tiles * kFtM;
+        for (int ks = 0; ks < k_steps; ++ks) {
+          ok = mbar_wait(w_empty_bar(ws), wphase);
+          if (ok) {
+            mbar_expect_tx(w_full_bar(ws), kFtW);
+            for (int half = 0; half < 2; ++half)      // (features behind the last one: zeros)
+              tma_load_2d(base + ws * kFtW + half * (kFtW / 2), &map_w, ks * kFtK + half * 32, f0, w_full_bar(ws));
+            ok = mbar_wait(x_empty_bar(xs), xphase);
+          }
+          if (!ok) {
+            if (a.error_word) atomicExch(a.error_word, 0x7C0072);
+            break;
+          }
+          mbar_expect_tx(x_full_bar(xs), 3 * xplane);
+          for (int p = 0; p < 3; ++p)      // (rows behind the last one: another term's, or zeros; never stored)
+            tma_load_2d(xring + (xs * 3 + p) * xplane, &map_x, ks * kFtK, p * a.M + m0, x_full_bar(xs));
+          if (++ws == a.w_stages) {
+            ws = 0;
+            wphase ^= 1;
+          }
+          if (++xs == a.x_stages) {
+            xs = 0;
+            xphase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp == 17) {
+    const uint32_t leader = ft_elect(), idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFtM >> 4) << 24);
+    const uint32_t n1 = (uint32_t)(a.rows >> 4) << 18;      // (an instruction's columns, in sixteens)
+    int s = 0;
+    uint32_t phase = 0, chunk = 0, it = 0, tile = 0;
+    bool ok = true;
+    const uint32_t small = tmem_base + kFtSums + 2 * kFtRows;      // (behind each other: a.rows columns a group)
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile) {
+      for (int ks = 0; ks < k_steps && ok; ks += kFtChunk, ++chunk) {
+        const int ab = chunk & 1;
+        const bool free = mbar_wait(acc_empty_bar(ab), ((chunk >> 1) & 1) ^ 1) && (ks > 0 || mbar_wait(small_empty_bar, (tile & 1) ^ 1));
+        if (!__all_sync(0xffffffffu, free)) {
+          if (a.error_word && leader) atomicExch(a.error_word, 0x7C0074);
+          ok = false;
+          break;
+        }
+        const uint32_t large = tmem_base + kFtSums + ab * kFtRows;
+        for (int kc = 0; kc < kFtChunk && ks + kc < k_steps && ok; ++kc, ++it) {
+          const uint32_t xs = xring + s * 3 * xplane, wt = tmem_base + (it & 1) * kFtTermCols;
+          if (!__all_sync(0xffffffffu, mbar_wait(x_full_bar(s), phase))) {
+            if (a.error_word && leader) atomicExch(a.error_word, 0x7C0073);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+          for (int k = 0; k < kFtK / 16; ++k) {
+            const uint64_t x0 = umma_desc_k128(xs + k * 32), x1 = umma_desc_k128(xs + xplane + k * 32);
+            const uint32_t w0 = wt + k * 8, w1 = w0 + kFtK / 2, w2 = w1 + kFtK / 2;
+            ft_mma(leader, small, w0, x1, idesc0 | 2 * n1, (ks | kc | k) != 0);
+            ft_mma(leader, small, w1, x0, idesc0 | 2 * n1, 1);
+            ft_mma(leader, small + a.rows, w2, x0, idesc0 | n1, 1);
+            ft_mma(leader, large, w0, x0, idesc0 | n1, (kc | k) != 0);
+          }
+          if (leader) umma_commit(x_empty_bar(s));
+          if (++s == a.x_stages) {
+            s = 0;
+            phase ^= 1;
+          }
+        }
+        if (leader) umma_commit(acc_full_bar(ab));      // (also on failure, so that the sums' warps do not wait in vain)
+      }
+    }
+  } else {
+    const int quarter = warp & 3, half = (warp - 18) >> 2;      // 32 features; groups of 16 rows half, half + 2, ...
+    uint32_t chunk = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      float sum[kFtGroups][16];
+#pragma unroll
+      for (int g = 0; g < kFtGroups; ++g)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) sum[g][c] = 0.f;
+      for (int ks = 0; ks < k_steps; ks += kFtChunk, ++chunk) {
+        const int b = chunk & 1;
+        if (!mbar_wait(acc_full_bar(b), (chunk >> 1) & 1)) {
+          if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0075);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const bool last = ks + kFtChunk >= k_steps;
+        const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + kFtSums;
+#pragma unroll
+        for (int g = 0; g < kFtGroups; ++g) {
+          const int c0 = (2 * g + half) * 16;
+          if (c0 >= a.rows) break;
+          uint32_t v[16];
+          tmem_ld16(at + b * kFtRows + c0, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < 16; ++c) sum[g][c] += __uint_as_float(v[c]);
+        }
+        if (last) {
+#pragma unroll
+          for (int e = 0; e < 2 * kFtGroups; ++e) {
+            const int c0 = (2 * (e >> 1) + half) * 16 + (e & 1) * 8;
+            if (c0 >= a.rows) break;
+            uint32_t m[8], n[8];
+            ft_tmem_ld8(at + 2 * kFtRows + c0, m);
+            ft_tmem_ld8(at + 2 * kFtRows + a.rows + c0, n);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 8; ++c) sum[e >> 1][(e & 1) * 8 + c] += __uint_as_float(m[c]) + __uint_as_float(n[c]);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(acc_empty_bar(b));
+          if (last) mbar_arrive(small_empty_bar);
+        }
+      }
+      if (!ok) break;
+      const int m0 = t % m_tiles * a.rows, feature = t / m_tiles * kFtM + quarter * 32 + lane;
+#pragma unroll
+      for (int g = 0; g < kFtGroups; ++g)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int j = (2 * g + half) * 16 + c;
+          if (j >= a.rows || m0 + j >= a.M || feature >= a.N) continue;
+          float v = sum[g][c];
+          if (!isfinite(v)) v = ft_plain_sum(a.x + (size_t)(m0 + j) * a.ldx, a.w + (size_t)feature * a.ldw, a.K);
+          a.out[(size_t)(m0 + j) * a.ldo + feature] = v;
+        }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 17) {
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+// Rows of 32-bit weights in boxes of 128 x 32.
+static int ft_weight_map(CUtensorMap* map, const float* w, int N, int K, int64_t ldw) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return TIB_E_ARG;
+  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N}, strides[1] = {(cuuint64_t)ldw * 4};
+  const cuuint32_t box[2] = {32u, (cuuint32_t)kFtM}, elem[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(w), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? TIB_OK : TIB_E_ARG;
+}
+
+}  // namespace tib
+
+using namespace tib;
+
+// Whether a weight's product runs here.  By the weight's sizes and the alignment alone, not by the number of rows: a request's
+// numbers do not depend on what else is in the step.  Four million weights are where the two launches and the scratch, some 8 us of the host more
+// than the other kernel's one, are paid back on few rows too: a block of 512 x 512 weights on 20
+// tokens took 143 us there and 182 here, one of 1,024 x 1,024 and 1,024 x 2,112 on 40 139 and 150, one of 1,536 x 1,536 and 1,536 x 6,400 on
+// 100 503 and 299.
+TIB_API int tib_gemm_f32_tcgen05_takes(const void* x, const void* w, int N, int K, int64_t ldx, int64_t ldw) {
+  return N >= 512 && K >= 512 && (int64_t)N * K >= (1 << 22) && K % kFtK == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+}
+
+// x: [M, K] (row stride ldx), w: [N, K] (row stride ldw), out: [M, N] (row stride ldo), all fp32.  scratch: bf16, 3 K numbers for each
+// of scratch_rows rows, on a 16-byte boundary; the product is made for that many rows at a time.  launches: takes the number of kernels launched.
+TIB_API int tib_gemm_f32_tcgen05(const float* x, const float* w, float* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
+                                 void* scratch, int scratch_rows, int* error_word, int* launches, cudaStream_t stream) {
+  *launches = 0;
+  if (M == 0) return TIB_OK;
+  if (!x || !w || !out || !scratch || M < 0 || scratch_rows < 1 || ((uintptr_t)scratch & 15)) return TIB_E_ARG;
+  if (!tib_gemm_f32_tcgen05_takes(x, w, N, K, ldx, ldw) || (int64_t)scratch_rows * 3 > 0x7fffffff - 256) return TIB_E_SIZE;
+  for (int first = 0; first < M; first += scratch_rows) {
+    const int rows = M - first < scratch_rows ? M - first : scratch_rows;
+    // Rows of a tile: whole rounds of tiles over the SMs times a step's cost (0.65 us with 16 rows, 0.76 with 48, 0.95 with 80).
+    int best = kFtRows;
+    double least = 1e30;
+    for (int tiles = ceil_div(rows, kFtRows); tiles <= ceil_div(rows, 16); ++tiles) {
+      const int r = ceil_div(ceil_div(rows, tiles), 16) * 16;
+      const double step = 120 + r;
+      const double cost = (double)ceil_div64((int64_t)ceil_div(rows, r) * ceil_div(N, kFtM), 148) * step;
+      if (cost < least) {
+        least = cost;
+        best = r;
+      }
+    }
+    FtArgs a;
+    a.x = x + (size_t)first * ldx; a.w = w; a.out = out + (size_t)first * ldo;
+    a.ldx = ldx; a.ldw = ldw; a.ldo = ldo; a.M = rows; a.N = N; a.K = K; a.rows = best; a.error_word = error_word;
+    const int x_stage = 3 * best * kFtK * 2;
+    a.x_stages = best > 48 ? 4 : 6;
+    a.w_stages = (220 * 1024 - a.x_stages * x_stage) / (int)kFtW < 6 ? (220 * 1024 - a.x_stages * x_stage) / (int)kFtW : 6;
+    const int smem = 1024 + a.w_stages * (int)kFtW + a.x_stages * x_stage + 512;
+    CUtensorMap map_w, map;
+    int rc = ft_weight_map(&map_w, w, N, K, ldw);
+    if (rc == TIB_OK) rc = make_map(&map, scratch, 3 * rows, K, K, best);
+    if (rc != TIB_OK) return rc;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    const int64_t blocks = ceil_div64((int64_t)rows * K / 4, 256);
+    TIB_LAUNCH_DEPENDENT(split_rows_kernel, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, a.x, ldx, rows, K, (__nv_bfloat16*)scratch);
+    const int64_t tiles = (int64_t)ceil_div(rows, best) * ceil_div(N, kFtM);
+    TIB_LAUNCH_DEPENDENT(gemm_f32_tcgen05_kernel, (int)(tiles < 148 ? tiles : 148), kFtThreads, smem, stream, map_w, map, a);
+    *launches += 2;
+  }
+  return TIB_OK;
+}

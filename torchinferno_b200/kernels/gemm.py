@@ -148,7 +148,7 @@ def linear(x: torch.Tensor, weight: "torch.Tensor | LinearWeight", *, out_dtype:
     if x.dtype == torch.float32 or weight.dtype == torch.float32:
         target = out if (out is not None and out.dtype == torch.float32) else \
             torch.empty((m, n), dtype=torch.float32, device=x.device)
-        ops.gemm_f32(x, weight, target)
+        ops.gemm_f32(x, weight, target, _error_word)
         if out_dtype == torch.float32:
             return target
         result = out if out is not None else torch.empty((m, n), dtype=out_dtype, device=x.device)

@@ -113,7 +113,7 @@ def lib() -> ctypes.CDLL:
     library = load_library()
     if not _signatures_set:
         for fn in ("tib_embedding", "tib_add_rmsnorm", "tib_rmsnorm", "tib_swiglu", "tib_cast",
-                   "tib_scatter_i32", "tib_decode_inputs", "tib_sample_records", "tib_rope_append", "tib_paged_attention_simt", "tib_gemm_f32", "tib_sample",
+                   "tib_scatter_i32", "tib_decode_inputs", "tib_sample_records", "tib_rope_append", "tib_paged_attention_simt", "tib_gemm_f32", "tib_gemm_f32_tcgen05", "tib_gemm_f32_tcgen05_takes", "tib_sample",
                    "tib_attention_mma_supports", "tib_prefill_attention", "tib_decode_attention",
                    "tib_prefill_attention_tcgen05", "tib_prefill_attention_tcgen05_supports",
                    "tib_decode_attention_tma", "tib_decode_attention_tma_rope", "tib_decode_attention_tma_supports", "tib_set_dependent_launch",
@@ -283,8 +283,14 @@ def paged_attention_simt(q: torch.Tensor, pool: torch.Tensor, out: torch.Tensor,
     return out
 
 
-def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """out[M, N] (fp32) = x[M, K] . w[N, K]^T with fp32 FMAs in fixed k order (rows of all three at any stride)."""
+# Room for the rows' terms in a 32-bit product on the tensor cores (6 bytes a number); more rows run so many at a time.
+F32_TERMS_BYTES = 64 << 20
+F32_TERMS_WEIGHTS = 1 << 22      # (asked here first: smaller weights never run there)
+
+
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error_word: torch.Tensor | None = None) -> torch.Tensor:
+    """out[M, N] (fp32) = x[M, K] . w[N, K]^T in 32 bits, summed over k in an order that N, K and the alignment fix (rows of all
+    three at any stride)."""
     if out.dtype != torch.float32:
         raise KernelError(f"out must be float32, got {out.dtype}")
     for name, t in (("x", x), ("w", w), ("out", out)):
@@ -293,6 +299,16 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tenso
     (m, k), (n, k2) = x.shape, w.shape
     if k != k2 or out.shape != (m, n):
         raise KernelError(f"gemm_f32: shapes {tuple(x.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
+    if x.dtype == w.dtype == torch.float32 and n * k >= F32_TERMS_WEIGHTS and m and lib().tib_gemm_f32_tcgen05_takes(
+            _ptr(x), _ptr(w), c_int(n), c_int(k), c_int64(x.stride(0)), c_int64(w.stride(0))):
+        rows = min(m, max(128, F32_TERMS_BYTES // (6 * k)))
+        scratch = torch.empty(3 * rows * k, dtype=torch.bfloat16, device=x.device)
+        launches = c_int(0)
+        _check("gemm_f32", lib().tib_gemm_f32_tcgen05(_ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k), c_int64(x.stride(0)),
+                                                      c_int64(w.stride(0)), c_int64(out.stride(0)), _ptr(scratch), c_int(rows),
+                                                      _ptr(error_word), ctypes.byref(launches), _stream()))
+        count_launches(launches.value - 1)
+        return out
     _check("gemm_f32", lib().tib_gemm_f32(_ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k),
                                           c_int64(x.stride(0)), c_int64(w.stride(0)), c_int64(out.stride(0)),
                                           c_int(_code(x.dtype)), c_int(_code(w.dtype)), _stream()))
