@@ -1000,6 +1000,32 @@ def test_linear_attention_of_a_request_does_not_depend_on_its_neighbours(dim, va
         assert launches == (3 if m >= runs_from and value_dim % 64 == 0 else 1)
 
 
+def test_linear_attention_in_runs_has_the_same_bits_in_tiles_of_either_width():
+    """Few runs go in tiles of 64 value columns, many in tiles of 128: a request alone and among others that make the step choose the other."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, dim, lens = 8, 128, [385, 200, 900, 700]
+    n, width, entries = sum(lens), heads * dim, len(lens)
+    decay = torch.tensor([1 - 2.0 ** -(3 + i % 6) for i in range(heads)], dtype=torch.float64)
+    powers = [dev((decay[:, None] ** torch.arange(most + 1, dtype=torch.float64)).float().contiguous())
+              for most in (ops.linear_attention_chunk(dim, dim), ops.linear_attention_run())]
+    rows, held = dev(rnd(n, 3 * width, dtype=torch.bfloat16)), dev(rnd(entries, heads, dim, dim, seed=5))
+
+    def run(first, count):
+        part = lens[first:first + count]
+        own, state = rows[sum(lens[:first]):sum(lens[:first + count])], held[first:first + count].clone()
+        starts = dev(torch.tensor([sum(part[:i]) for i in range(count + 1)], dtype=torch.int32))
+        out = ops.linear_attention(own[:, :width], own[:, width:2 * width], own[:, 2 * width:], torch.empty(len(own), width, device="cuda"), state, powers[0],
+                                   starts, dev(torch.arange(count, dtype=torch.int32)), count, heads, dim, dim, silu=True, max_q_len=max(part),
+                                   run_powers=powers[1], portions={m: 1 for m in part})
+        return out, state
+
+    out, state = run(0, entries)
+    for i in range(entries):
+        alone, alone_state = run(i, 1)
+        assert torch.equal(alone, out[sum(lens[:i]):sum(lens[:i + 1])]) and torch.equal(alone_state[0], state[i])
+
+
 @pytest.mark.parametrize("at_a_time", [1, 2, 3])
 def test_linear_attention_in_runs_some_heads_at_a_time(at_a_time, monkeypatch):
     """With less room for the runs' states than all heads take, the same bits and no more room than that."""

@@ -24,7 +24,7 @@
 // Error against 64 bits (2-norm): 1.4e-7 at 2,048 k and 2.0e-7 at 8,192, where multiply-adds in order have 8.1e-7 and 1.6e-6; numbers of one
 // sign 1.6e-7 (6.3e-7); sums over 256 k 2.4e-7, for a tenth off the time.
 // An output that is not finite is worked out again with fused multiply-adds in order (an infinity's terms make NaN of it).
-#include "mma.cuh"
+#include "split_terms.cuh"
 #include "cluster.cuh"
 
 namespace tib {
@@ -34,21 +34,6 @@ constexpr int kFtGroups = (kFtRows / 16 + 1) / 2;               // groups of 16 
 constexpr uint32_t kFtW = kFtM * kFtK * 4;                      // a step's weights in shared memory
 constexpr uint32_t kFtTermCols = 3 * kFtK / 2;                  // in tensor memory: a step's terms of the weights, twice
 constexpr uint32_t kFtSums = 2 * kFtTermCols;                   // a0 b0 twice, then the two small groups
-
-__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
-// The three terms of two floats, packed.
-__device__ __forceinline__ void ft_split2(float a, float b, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
-  t0 = pack_bf16(a, b);
-  f2_unpack(f2_sub(f2_pack(a, b), f2_pack(__uint_as_float(t0 << 16), __uint_as_float(t0 & 0xffff0000u))), a, b);
-  t1 = pack_bf16(a, b);
-  f2_unpack(f2_sub(f2_pack(a, b), f2_pack(__uint_as_float(t1 << 16), __uint_as_float(t1 & 0xffff0000u))), a, b);
-  t2 = pack_bf16(a, b);
-}
 
 // The three terms of x, [3][rows][K]; grid-stride, four elements a thread.
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, int64_t ldx, int rows, int K, __nv_bfloat16* __restrict__ out) {
@@ -72,28 +57,6 @@ __device__ __noinline__ float ft_plain_sum(const float* __restrict__ x, const fl
   float s = 0.f;
   for (int k = 0; k < K && s == s; ++k) s = fmaf(x[k], w[k], s);
   return s;
-}
-
-// One lane of the warp.
-__device__ __forceinline__ uint32_t ft_elect() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one;
-}
-// The product with the weights in tensor memory, issued by the leader of a warp that is together.
-__device__ __forceinline__ void ft_mma(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
-}
-
-__device__ __forceinline__ void ft_tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-__device__ __forceinline__ void ft_tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
 
 struct FtArgs {

@@ -18,12 +18,12 @@
 // Three ways to run that.  Every portion takes the one its own length and the layer's sizes name, whatever else is in the step
 // (tib_linear_attention launches each form that occurs over the whole batch, and a form's blocks leave the others' portions alone), so a
 // request's numbers do not depend on its neighbours:
-//   runs   (portions above 192 tokens, or 384 in heads of 64 x 64; head sizes of 64 or 128) every run of 64 tokens makes its own sum L of decayed k v^T
+//   runs   (portions above 192 tokens, or 384 in heads of 64 x 64; head sizes of 64 or 128) every run of 128 tokens makes its own sum L of decayed k v^T
 //          side by side, one thread per state element then folds S <- lambda^n S + L over a request's runs, and every run
 //          makes its outputs from its starting state: the serial chain is one fused multiply-add a run
 //   walk   (portions of at most 32 tokens) S in registers, token by token
 //   chunks (everything else) the block walk described above
-#include "common.cuh"
+#include "linear_attention.cuh"
 
 namespace tib {
 
@@ -38,8 +38,6 @@ struct LinAttnArgs {
   int cols;               // value columns per block
   int shortest, longest;  // the portions this launch takes (the others are another form's)
 };
-
-__device__ __forceinline__ float lin_act(float z, int activation) { return activation ? z / (1.f + expf(-z)) : z; }
 
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -219,129 +217,13 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 // ---------------------------------------------------------------------------------------------------------- runs
 // The walk above is one serial chain of 64 chunks for 2,048 tokens, each with four barriers, on 512 blocks that each see 32 of a
 // run's 128 columns: 980 us for two portions of 1,366 and 682 tokens, 16 heads of 128 x 128, of which the fp32 arithmetic
-// (3.3 GFLOP here) is some 50 us.  In runs the three launches below take 49 + 27 + 82 us (cold).  What bounds them is the fp32 pipe: register
-// tiles of 8 x 8 (sums) and 4 x 8 (outputs) per thread, products in pairs of neighbouring columns (fma.rn.f32x2, each
-// half rounded as the scalar instruction rounds it), operands from shared memory in 16-byte loads without bank conflicts.
-// Everything stays fp32: activations, decay powers, scores, states and sums.
-constexpr int kLinRun = 64;
+// (3.3 GFLOP here) is some 50 us.  In runs of 64 on the fp32 pipe the three launches took 131 us (49 + 27 + 82 cold); in runs of 128 on the
+// tensor cores (linear_tcgen05.cu) they take 68 (26 + 18 + 52), half of the states' traffic with it.  Of 2,048 tokens of 24 heads of 64 x 64
+// 57 us (74), of 600 of 8 heads of 128 x 64 27 (33).
+// Everything stays fp32 or three bf16 terms of it: activations, decay powers, scores, states and sums.  Error against 64 bits (2-norm, those
+// four cases with one of 4 heads of 64 x 128): outputs 1.0 to 1.3e-7 (1.4 to 1.9 on the fp32 pipe), states 7 to 8.7e-8 (8.6e-8 to 1.0e-7).
 // The shortest portion that is cut into runs (why: tib_linear_attention).
 static int lin_runs_from(int key_dim, int value_dim) { return key_dim * value_dim <= 64 * 64 ? 385 : 193; }
-constexpr int kLinPad = kLinRun + 4;       // row stride of the transposed q, k and scores
-
-struct LinRunArgs {
-  const int* q_start;
-  const int* slots;
-  const float* powers;    // [heads, kLinRun + 1]
-  float* state;           // [slots, heads, D, value_dim]
-  float* run_state;       // [runs, n_heads, D, value_dim]: L of a run, then the state at its start
-  float* out;
-  int64_t ldq, ldk, ldv;
-  int heads, value_dim, activation;
-  int head0, n_heads;     // the heads of these launches (the runs' states are made for some heads at a time)
-  int shortest;           // portion that is cut into runs
-};
-
-// An entry's first run: entries' runs never overlap, since an entry of len tokens has at most len / kLinRun + 1 runs and the
-// next entry starts len rows and one entry later.
-__device__ __forceinline__ size_t lin_first_run(int row0, int entry) { return (size_t)(row0 / kLinRun) + entry; }
-
-// eight elements of a row, activated, in fp32
-__device__ __forceinline__ void lin_load8(const __nv_bfloat16* p, int activation, float (&v)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
-    v[2 * i] = lin_act(f.x, activation);
-    v[2 * i + 1] = lin_act(f.y, activation);
-  }
-}
-__device__ __forceinline__ void lin_load8(const float* p, int activation, float (&v)[8]) {
-  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = lin_act(v[i], activation);
-}
-
-// grid (heads * column tiles, runs, entries): L[d][c] = sum_j lambda^(n-1-j) k_j[d] v_j[c] of the run's n tokens
-template <typename T, int D, int TV>
-__global__ void __launch_bounds__(256, 2) lin_run_sums_kernel(const T* __restrict__ k, const T* __restrict__ v, LinRunArgs a) {
-  extern __shared__ __align__(16) float lin_smem[];
-  float* ks = lin_smem;                 // [64][D]
-  float* vs = ks + kLinRun * D;         // [64][TV]
-  __shared__ float pw[kLinRun + 1];
-  pdl_wait();
-  pdl_trigger();
-  const int tiles = a.value_dim / TV, own = blockIdx.x / tiles, head = a.head0 + own, col0 = (blockIdx.x - own * tiles) * TV;
-  const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
-  const int t0 = blockIdx.y * kLinRun;
-  if (t0 >= len || len < a.shortest) return;
-  const int n = min(kLinRun, len - t0), tid = threadIdx.x;
-  if (tid <= kLinRun) pw[tid] = a.powers[head * (kLinRun + 1) + tid];
-  __syncthreads();
-  float x[8];
-#pragma unroll
-  for (int it = 0; it < kLinRun * D / 8 / 256; ++it) {
-    const int p = tid + it * 256, j = p / (D / 8), c = (p % (D / 8)) * 8;
-    if (j < n) {
-      lin_load8(k + (size_t)(row0 + t0 + j) * a.ldk + head * D + c, a.activation, x);
-      const float f = pw[n - 1 - j];
-      reinterpret_cast<float4*>(ks + j * D + c)[0] = make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f);
-      reinterpret_cast<float4*>(ks + j * D + c)[1] = make_float4(x[4] * f, x[5] * f, x[6] * f, x[7] * f);
-    }
-  }
-#pragma unroll
-  for (int it = 0; it < kLinRun * TV / 8 / 256; ++it) {
-    const int p = tid + it * 256, j = p / (TV / 8), c = (p % (TV / 8)) * 8;
-    if (j < n) {
-      lin_load8(v + (size_t)(row0 + t0 + j) * a.ldv + head * a.value_dim + col0 + c, a.activation, x);
-      reinterpret_cast<float4*>(vs + j * TV + c)[0] = make_float4(x[0], x[1], x[2], x[3]);
-      reinterpret_cast<float4*>(vs + j * TV + c)[1] = make_float4(x[4], x[5], x[6], x[7]);
-    }
-  }
-  __syncthreads();
-  // rows ty * 4 + 64 r + i, columns tx * 4 + 64 g + c
-  constexpr int R = D / 64, G = TV / 64;
-  const int tx = tid & 15, ty = tid >> 4;
-  f32x2 acc[R * 4][G * 2];
-#pragma unroll
-  for (int i = 0; i < R * 4; ++i)
-#pragma unroll
-    for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_pack(0.f, 0.f);
-#pragma unroll 2
-  for (int j = 0; j < n; ++j) {
-    ulonglong2 b[G];
-#pragma unroll
-    for (int g = 0; g < G; ++g) b[g] = *reinterpret_cast<const ulonglong2*>(vs + j * TV + g * 64 + tx * 4);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const float4 av = *reinterpret_cast<const float4*>(ks + j * D + r * 64 + ty * 4);
-      const float ai[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const f32x2 aa = f2_pack(ai[i], ai[i]);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          acc[r * 4 + i][2 * g] = f2_fma(aa, b[g].x, acc[r * 4 + i][2 * g]);
-          acc[r * 4 + i][2 * g + 1] = f2_fma(aa, b[g].y, acc[r * 4 + i][2 * g + 1]);
-        }
-      }
-    }
-  }
-  float* dst = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.n_heads + own) * (size_t)D * a.value_dim + col0;
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        ulonglong2 o;
-        o.x = acc[r * 4 + i][2 * g];
-        o.y = acc[r * 4 + i][2 * g + 1];
-        *reinterpret_cast<ulonglong2*>(dst + (size_t)(r * 64 + ty * 4 + i) * a.value_dim + g * 64 + tx * 4) = o;
-      }
-}
-
 // grid (state elements / 1024, entries): S <- lambda^n S + L over the entry's runs, four elements a thread; run_state turns from
 // a run's sum into the state at its start, the last state goes to the slot.
 __global__ void __launch_bounds__(256) lin_fold_kernel(LinRunArgs a, int key_dim) {
@@ -372,150 +254,6 @@ __global__ void __launch_bounds__(256) lin_fold_kernel(LinRunArgs a, int key_dim
     }
   }
   *slot = st;
-}
-
-// grid (heads * column tiles, runs, entries): o_i = lambda^(i+1) S^T q_i + sum_(j<=i) (q_i . k_j) lambda^(i-j) v_j, S the state at the
-// run's start.  q and k lie transposed in shared memory ([d][token]); the scores (also transposed) and the tiles of 32 rows
-// of S take k's place once the scores are made.
-template <typename T, int D, int TV>
-__global__ void __launch_bounds__(256, 2)
-lin_run_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, LinRunArgs a) {
-  constexpr int SR = 32;                                     // rows of S a tile
-  constexpr int kRegion = D * kLinPad > kLinRun * kLinPad + SR * TV ? D * kLinPad : kLinRun * kLinPad + SR * TV;
-  extern __shared__ __align__(16) float lin_smem[];
-  float* qt = lin_smem;                   // [D][kLinPad]
-  float* kt = qt + D * kLinPad;           // [D][kLinPad], then:
-  float* at = kt;                         // [64][kLinPad]: at[j][i] = (q_i . k_j) lambda^(i-j), 0 above the diagonal
-  float* ss = kt + kLinRun * kLinPad;     // [SR][TV]
-  float* vs = kt + kRegion;               // [64][TV]
-  __shared__ float pw[kLinRun + 1];
-  pdl_wait();
-  pdl_trigger();
-  const int tiles = a.value_dim / TV, own = blockIdx.x / tiles, head = a.head0 + own, col0 = (blockIdx.x - own * tiles) * TV;
-  const int entry = blockIdx.z, row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
-  const int t0 = blockIdx.y * kLinRun;
-  if (t0 >= len || len < a.shortest) return;
-  const int n = min(kLinRun, len - t0), tid = threadIdx.x;
-  const float* S = a.run_state + ((lin_first_run(row0, entry) + blockIdx.y) * a.n_heads + own) * (size_t)D * a.value_dim + col0;
-  constexpr int SV = SR * TV / 4 / 256;                      // 16-byte pieces of a tile of S a thread fetches
-  float4 sp[SV];
-  auto ask = [&](int d0) {
-#pragma unroll
-    for (int it = 0; it < SV; ++it) {
-      const int p = tid + it * 256;
-      sp[it] = *reinterpret_cast<const float4*>(S + (size_t)(d0 + p / (TV / 4)) * a.value_dim + (p % (TV / 4)) * 4);
-    }
-  };
-  ask(0);
-  if (tid <= kLinRun) pw[tid] = a.powers[head * (kLinRun + 1) + tid];
-  float x[8];
-#pragma unroll
-  for (int it = 0; it < kLinRun * D / 8 / 256; ++it) {       // (neighbouring lanes take neighbouring tokens: no bank conflicts in the transposed stores)
-    const int p = tid + it * 256, j = p % kLinRun, c = (p / kLinRun) * 8;
-    const size_t row = (size_t)(row0 + t0 + min(j, n - 1));
-    lin_load8(q + row * a.ldq + head * D + c, a.activation, x);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) qt[(c + e) * kLinPad + j] = x[e];
-    lin_load8(k + row * a.ldk + head * D + c, a.activation, x);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) kt[(c + e) * kLinPad + j] = x[e];
-  }
-#pragma unroll
-  for (int it = 0; it < kLinRun * TV / 8 / 256; ++it) {
-    const int p = tid + it * 256, j = p / (TV / 8), c = (p % (TV / 8)) * 8;
-    if (j < n) {
-      lin_load8(v + (size_t)(row0 + t0 + j) * a.ldv + head * a.value_dim + col0 + c, a.activation, x);
-      reinterpret_cast<float4*>(vs + j * TV + c)[0] = make_float4(x[0], x[1], x[2], x[3]);
-      reinterpret_cast<float4*>(vs + j * TV + c)[1] = make_float4(x[4], x[5], x[6], x[7]);
-    }
-  }
-  __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
-  {
-    float s[4][4];                                           // s[j][i]: keys tx * 4 + j, tokens ty * 4 + i
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) s[j][i] = 0.f;
-#pragma unroll 4
-    for (int d = 0; d < D; ++d) {
-      const float4 qv = *reinterpret_cast<const float4*>(qt + d * kLinPad + ty * 4);
-      const float4 kv = *reinterpret_cast<const float4*>(kt + d * kLinPad + tx * 4);
-      const float qi[4] = {qv.x, qv.y, qv.z, qv.w}, kj[4] = {kv.x, kv.y, kv.z, kv.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s[j][i] = fmaf(qi[i], kj[j], s[j][i]);
-    }
-    __syncthreads();                                         // k is no longer needed: the scores take its place
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int kj = tx * 4 + j;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int back = ty * 4 + i - kj;
-        s[j][i] = back >= 0 ? s[j][i] * pw[back] : 0.f;
-      }
-      *reinterpret_cast<float4*>(at + kj * kLinPad + ty * 4) = make_float4(s[j][0], s[j][1], s[j][2], s[j][3]);
-    }
-  }
-  constexpr int G = TV / 64;
-  f32x2 acc[4][G * 2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_pack(0.f, 0.f);
-  auto add = [&](const float4& av, const float* brow, int from) {      // acc[i][.] += a[i] * b[.] for i >= from
-    ulonglong2 b[G];
-#pragma unroll
-    for (int g = 0; g < G; ++g) b[g] = *reinterpret_cast<const ulonglong2*>(brow + g * 64 + tx * 4);
-    const float ai[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (i < from) continue;
-      const f32x2 aa = f2_pack(ai[i], ai[i]);
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        acc[i][2 * g] = f2_fma(aa, b[g].x, acc[i][2 * g]);
-        acc[i][2 * g + 1] = f2_fma(aa, b[g].y, acc[i][2 * g + 1]);
-      }
-    }
-  };
-  for (int d0 = 0; d0 < D; d0 += SR) {
-#pragma unroll
-    for (int it = 0; it < SV; ++it) reinterpret_cast<float4*>(ss)[tid + it * 256] = sp[it];
-    __syncthreads();
-    if (d0 + SR < D) ask(d0 + SR);
-#pragma unroll 4
-    for (int d = 0; d < SR; ++d) add(*reinterpret_cast<const float4*>(qt + (d0 + d) * kLinPad + ty * 4), ss + d * TV, 0);
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float f = pw[ty * 4 + i + 1];
-    const f32x2 ff = f2_pack(f, f);
-#pragma unroll
-    for (int g = 0; g < G * 2; ++g) acc[i][g] = f2_mul(ff, acc[i][g]);
-  }
-  // a warp holds eight tokens: those before them count for all eight, those among them only for the tokens they come before (left
-  // out, not weighed with 0: an infinity or NaN must not reach an earlier token)
-  const int mine = (tid >> 5) * 8, keys = min(n, mine);
-#pragma unroll 4
-  for (int j = 0; j < keys; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV, 0);
-  const int last = min(n, mine + 8);
-  for (int j = mine; j < last; ++j) add(*reinterpret_cast<const float4*>(at + j * kLinPad + ty * 4), vs + j * TV, j - ty * 4);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (ty * 4 + i >= n) break;
-    float* dst = a.out + (size_t)(row0 + t0 + ty * 4 + i) * a.heads * a.value_dim + head * a.value_dim + col0;
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      ulonglong2 o;
-      o.x = acc[i][2 * g];
-      o.y = acc[i][2 * g + 1];
-      *reinterpret_cast<ulonglong2*>(dst + g * 64 + tx * 4) = o;
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------------------------------------- walk
@@ -590,21 +328,16 @@ lin_walk_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
   for (int i = 0; i < ROWS; ++i) *reinterpret_cast<float4*>(S + (size_t)(rt + 32 * i) * a.value_dim) = s[i];
 }
 
-template <typename T, int D, int TV>
-static int launch_lin_runs(const void* q, const void* k, const void* v, const LinRunArgs& a, int n_entries, int max_q_len, cudaStream_t stream) {
-  constexpr size_t sums = sizeof(float) * kLinRun * (D + TV);
-  constexpr int region = D * kLinPad > kLinRun * kLinPad + 32 * TV ? D * kLinPad : kLinRun * kLinPad + 32 * TV;
-  constexpr size_t outs = sizeof(float) * (D * kLinPad + region + kLinRun * TV);
-  auto ks = lin_run_sums_kernel<T, D, TV>;
-  auto ko = lin_run_out_kernel<T, D, TV>;
-  cudaError_t e = cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outs);
-  if (e != cudaSuccess) return (int)e;
-  const dim3 grid(a.n_heads * (a.value_dim / TV), ceil_div(max_q_len, kLinRun), n_entries);
-  TIB_LAUNCH_DEPENDENT(ks, grid, 256, sums, stream, (const T*)k, (const T*)v, a);
-  TIB_LAUNCH_DEPENDENT(lin_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.n_heads * D * a.value_dim, 1024), n_entries), 256, 0, stream, a, D);
-  TIB_LAUNCH_DEPENDENT(ko, grid, 256, outs, stream, (const T*)q, (const T*)k, (const T*)v, a);
-  return TIB_OK;
+static int launch_lin_runs(const void* q, const void* k, const void* v, const LinRunArgs& a, int dtype, int key_dim, int n_entries, int max_q_len,
+                           cudaStream_t stream) {
+  const int runs = ceil_div(max_q_len, kLinRun);
+  // Tiles of 128 value columns, or of 64 where those leave half of the SMs without one.
+  const int tile = a.value_dim % 128 == 0 && (int64_t)a.n_heads * (a.value_dim / 128) * runs * n_entries > 74 ? 128 : 64;
+  const dim3 grid(a.n_heads * (a.value_dim / tile), runs, n_entries);
+  int status = launch_lin_run_sums(k, v, a, dtype, key_dim, tile, grid, stream);
+  if (status != TIB_OK) return status;
+  TIB_LAUNCH_DEPENDENT(lin_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.n_heads * key_dim * a.value_dim, 1024), n_entries), 256, 0, stream, a, key_dim);
+  return launch_lin_run_outs(q, k, v, a, dtype, key_dim, tile, grid, stream);
 }
 
 template <typename T>
@@ -649,7 +382,7 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
                                  float* out, float* state, const float* powers, const int* q_start, const int* slots,
                                  int n_entries, int heads, int key_dim, int value_dim, int chunk, int activation, int dtype,
                                  int tokens, int max_q_len, int forms, int n_chunked, const float* run_powers, float* run_state, int64_t run_capacity, int run_heads,
-                                 int* launches, cudaStream_t stream) {
+                                 int* launches, int* error_word, cudaStream_t stream) {
   *launches = 0;
   if (n_entries == 0) return TIB_OK;
   if (!q || !k || !v || !out || !state || !powers || !q_start || !slots) return TIB_E_ARG;
@@ -670,6 +403,7 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
     LinRunArgs r;
     r.q_start = q_start; r.slots = slots; r.powers = run_powers; r.state = state; r.run_state = run_state; r.out = out;
     r.ldq = ldq; r.ldk = ldk; r.ldv = ldv; r.heads = heads; r.head0 = 0; r.n_heads = heads; r.shortest = lin_runs_from(key_dim, value_dim); r.value_dim = value_dim; r.activation = activation;
+    r.error_word = error_word;
     if (forms & 1) {
       const int status = dtype == TIB_F32 ? launch_lin_walk<float>(q, k, v, r, key_dim, n_entries, stream)
                                           : launch_lin_walk<__nv_bfloat16>(q, k, v, r, key_dim, n_entries, stream);
@@ -679,18 +413,12 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
     shortest = kLinWalk + 1;
     const bool runs = run_state && run_heads > 0 && value_dim % 64 == 0 && run_capacity >= tokens / kLinRun + n_entries && ceil_div(max_q_len, kLinRun) <= 65535;
     if ((forms & 4) && runs) {
-#define TIB_LIN_GO(T)                                                                                             \
-  (key_dim == 64 ? (value_dim % 128 == 0 ? launch_lin_runs<T, 64, 128>(q, k, v, r, n_entries, max_q_len, stream)    \
-                                         : launch_lin_runs<T, 64, 64>(q, k, v, r, n_entries, max_q_len, stream))    \
-                 : (value_dim % 128 == 0 ? launch_lin_runs<T, 128, 128>(q, k, v, r, n_entries, max_q_len, stream)   \
-                                         : launch_lin_runs<T, 128, 64>(q, k, v, r, n_entries, max_q_len, stream)))
       for (; r.head0 < heads; r.head0 += run_heads) {
         r.n_heads = run_heads < heads - r.head0 ? run_heads : heads - r.head0;
-        const int status = dtype == TIB_F32 ? TIB_LIN_GO(float) : TIB_LIN_GO(__nv_bfloat16);
+        const int status = launch_lin_runs(q, k, v, r, dtype, key_dim, n_entries, max_q_len, stream);
         if (status != TIB_OK) return status;
         *launches += 3;
       }
-#undef TIB_LIN_GO
     }
     if (runs) longest = r.shortest - 1;
     if (runs || !(forms & 4)) {

@@ -925,7 +925,8 @@ LINEAR_ATTENTION_SCRATCH = 128 << 20
 def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
                      powers: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, n_entries: int, heads: int,
                      key_dim: int, value_dim: int, *, silu: bool, max_q_len: int = 0,
-                     run_powers: torch.Tensor | None = None, portions: Mapping[int, int] | None = None) -> torch.Tensor:
+                     run_powers: torch.Tensor | None = None, portions: Mapping[int, int] | None = None,
+                     error_word: torch.Tensor | None = None) -> torch.Tensor:
     """o_t = S_t^T q_t with S_t = decay * S_(t-1) + k_t v_t^T per head, over the ragged batch; ``state``
     [slots, heads, key_dim, value_dim] (fp32) is read and left updated; ``powers`` [heads, chunk + 1] holds decay^m.
     With the step's longest entry and ``run_powers`` [heads, linear_attention_run() + 1] (decay^m again) long portions run in
@@ -965,7 +966,7 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
         _ptr(q), _ptr(k), _ptr(v), c_int64(q.stride(0)), c_int64(k.stride(0)), c_int64(v.stride(0)), _ptr(out), _ptr(state),
         _ptr(powers), _ptr(q_start), _ptr(slots), c_int(n_entries), c_int(heads), c_int(key_dim), c_int(value_dim),
         c_int(chunk), c_int(1 if silu else 0), c_int(_code(q.dtype)), c_int(q.shape[0]), c_int(max_q_len), c_int(forms),
-        c_int(chunked), _ptr(run_powers), _ptr(run_state), c_int64(capacity), c_int(run_heads), ctypes.byref(launches), _stream()))
+        c_int(chunked), _ptr(run_powers), _ptr(run_state), c_int64(capacity), c_int(run_heads), ctypes.byref(launches), _ptr(error_word), _stream()))
     count_launches(launches.value - 1)      # (_check counted one)
     return out
 

@@ -84,7 +84,7 @@ class DecayLinearAttention(Mixer):
         mixed = torch.empty((n, vv), dtype=torch.float32, device=x.device)
         ops.linear_attention(q, k, v, mixed, ctx.state, self.powers, batch.q_start, batch.slots, batch.n_entries, self.heads,
                              self.key_dim, self.value_dim, silu=self.activation == "silu", max_q_len=batch.max_q_len,
-                             run_powers=self.run_powers, portions=batch.portions)
+                             run_powers=self.run_powers, portions=batch.portions, error_word=ctx.error_word)
         if self.gate:
             rows = torch.empty((n, vv), dtype=x.dtype, device=x.device)
             ops.sigmoid_gate(mixed, proj[:, 2 * qk + vv:], rows, self.norm_weight, self.eps)
