@@ -22,8 +22,7 @@ namespace tib {
 constexpr int kLtThreads = 512;
 constexpr uint32_t kLtSub = kLinRun * 128;      // 128 rows of 64 bf16, 128-byte swizzle
 
-// A tile's terms: [3][width / 64][rows][64]; eight elements of row r from column 8 c8.
-__device__ __forceinline__ uint32_t lt_place(int r, int c8, int rows) { return (uint32_t)((c8 >> 3) * rows * 128 + r * 128 + (((c8 & 7) ^ (r & 7)) << 4)); }
+// A tile's terms: [3][width / 64][rows][64].
 __device__ __forceinline__ void lt_put(unsigned char* tile, uint32_t term_bytes, uint32_t at, const float (&x)[8]) {
   uint32_t t[3][4];
 #pragma unroll
@@ -88,7 +87,7 @@ template <typename T, int WIDTH> struct LtRows {
       float x[8];
       raw[i].activated(activation, x);
       f(r, x);
-      lt_put(tile, WIDTH / 64 * kLtSub, lt_place(r, c8, kLinRun), x);
+      lt_put(tile, WIDTH / 64 * kLtSub, ft_place(r, c8, kLinRun), x);
     }
   }
 };
@@ -116,16 +115,6 @@ __device__ __forceinline__ void lt_products(uint32_t leader, uint32_t d, uint32_
   }
 }
 
-__device__ __forceinline__ void lt_store8(float* dst, const float (&v)[8]) {      // (on a 16-byte boundary)
-  if ((uintptr_t)dst & 16) {
-    reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-    return;
-  }
-  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
-               ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
-}
-
 // What the two kernels' blocks begin with; false: the block has no run.
 struct LtBlock {
   int head, own, col0, row0, t0, n;
@@ -144,40 +133,6 @@ __device__ __forceinline__ bool lt_block(const LinRunArgs& a, LtBlock& b) {
   b.run = lin_first_run(b.row0, entry) + blockIdx.y;
   return b.t0 < len && len >= a.shortest;
 }
-__device__ __forceinline__ uint32_t lt_setup(uint32_t bar0, int bars, uint32_t slot, volatile uint32_t* slot_ptr, int warp, uint32_t columns) {
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < bars; ++i) mbar_init(bar0 + 8 * i, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(slot), "r"(columns) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  return *slot_ptr;
-}
-// What the threads left in shared and tensor memory becomes the tensor cores' (called by the whole block).
-__device__ __forceinline__ void lt_hand_over() {
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-}
-__device__ __forceinline__ void lt_wait(uint32_t bar, int* error_word, int code) {
-  if (!mbar_wait(bar, 0) && error_word && (threadIdx.x & 31) == 0) atomicExch(error_word, code);
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-}
-__device__ __forceinline__ void lt_release(int warp, uint32_t tmem, uint32_t columns) {
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(columns) : "memory");
-  }
-}
-
 template <int D, int TV, int ACC> struct LtSums {
   static constexpr uint32_t kKeyTerm = D / 64 * kLtSub, kValueTerm = TV / 64 * kLtSub;
   static constexpr uint32_t kSmem = 1024 + 3 * (kKeyTerm + kValueTerm) + 64;
@@ -200,7 +155,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
   if (!lt_block<TV>(a, b)) return;
   const uint32_t bar = base + 3 * (S::kKeyTerm + S::kValueTerm);
   if (threadIdx.x <= kLinRun) pw[threadIdx.x] = a.powers[b.head * (kLinRun + 1) + threadIdx.x];
-  const uint32_t tmem = lt_setup(bar, 1, bar + 8, reinterpret_cast<volatile uint32_t*>(smem + (bar + 8 - base)), warp, S::kColumns);
+  const uint32_t tmem = ft_setup(bar, 1, bar + 8, reinterpret_cast<volatile uint32_t*>(smem + (bar + 8 - base)), warp, S::kColumns);
   const size_t first = (size_t)(b.row0 + b.t0);
   LtRows<T, D> keys_of;
   LtRows<T, TV> values_of;
@@ -212,7 +167,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
     for (int e = 0; e < 8; ++e) x[e] *= w;
   });
   values_of.put(smem + 3 * S::kKeyTerm, a.activation, [](int, float (&)[8]) {});
-  lt_hand_over();
+  ft_hand_over();
   if (warp == 0) {
     const uint32_t leader = ft_elect();
     // both operands have the tokens as rows (of heads of 64 the upper half of the 128 rows is the next tile's, and never stored)
@@ -223,7 +178,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
     if (leader) umma_commit(bar);
     __syncwarp();
   }
-  lt_wait(bar, a.error_word, 0x7C0081);
+  ft_wait(bar, 0, a.error_word, 0x7C0081);
   const int quarter = warp & 3, d = quarter * 32 + lane;
   const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16);
   float* dst = a.run_state + (b.run * a.n_heads + b.own) * (size_t)D * a.value_dim + (size_t)d * a.value_dim + b.col0;
@@ -246,10 +201,10 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
 #pragma unroll
     for (int e = 0; e < 16; e += 8) {
       const float o[8] = {sum[e], sum[e + 1], sum[e + 2], sum[e + 3], sum[e + 4], sum[e + 5], sum[e + 6], sum[e + 7]};
-      lt_store8(dst + c0 + e, o);
+      ft_store8(dst + c0 + e, o);
     }
   }
-  lt_release(warp, tmem, S::kColumns);
+  ft_release(warp, tmem, S::kColumns);
 }
 
 template <int D, int TV> struct LtOuts {
@@ -276,7 +231,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
   if (tid <= kLinRun) pw[tid] = a.powers[b.head * (kLinRun + 1) + tid];
   if (tid == 0) odd = 0;
   // tensor memory: scores (two accumulators), later their three terms; carried, later inside
-  const uint32_t tmem = lt_setup(bar, 3, bar + 24, reinterpret_cast<volatile uint32_t*>(smem + (bar + 24 - base)), warp, 512);
+  const uint32_t tmem = ft_setup(bar, 3, bar + 24, reinterpret_cast<volatile uint32_t*>(smem + (bar + 24 - base)), warp, 512);
   const size_t first = (size_t)(b.row0 + b.t0);
   const uint32_t one = base, two = base + S::kFirst;
   {
@@ -286,7 +241,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     rows_q.put(smem, a.activation, [](int, float (&)[8]) {});
     rows_k.put(smem + S::kFirst, a.activation, [](int, float (&)[8]) {});
   }
-  lt_hand_over();
+  ft_hand_over();
   const uint32_t leader = warp == 0 ? ft_elect() : 0;
   if (warp == 0) {
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kLinRun >> 3) << 17) | (8u << 24);
@@ -305,14 +260,14 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     held[i][0] = src[0];
     held[i][1] = src[1];
   }
-  lt_wait(bar, a.error_word, 0x7C0082);
+  ft_wait(bar, 0, a.error_word, 0x7C0082);
 #pragma unroll
   for (int i = 0; i < SV; ++i) {
     const int p = tid + i * kLtThreads;
     const float x[8] = {held[i][0].x, held[i][0].y, held[i][0].z, held[i][0].w, held[i][1].x, held[i][1].y, held[i][1].z, held[i][1].w};
-    lt_put(smem + S::kFirst, S::kStateTerm, lt_place(p / (TV / 8), p % (TV / 8), D), x);
+    lt_put(smem + S::kFirst, S::kStateTerm, ft_place(p / (TV / 8), p % (TV / 8), D), x);
   }
-  lt_hand_over();
+  ft_hand_over();
   const uint32_t carried = tmem + 256;
   constexpr uint32_t idesc_v = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(TV >> 3) << 17) | (8u << 24);
   if (warp == 0) {
@@ -356,7 +311,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     }
     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
   }
-  lt_wait(bar + 8, a.error_word, 0x7C0083);
+  ft_wait(bar + 8, 0, a.error_word, 0x7C0083);
   float sum[TV / 4];
   const float decay = pw[i + 1];
 #pragma unroll
@@ -376,7 +331,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
         x[e] = 0.f;
       }
   });
-  lt_hand_over();
+  ft_hand_over();
   if (warp == 0) {
     // (the weighted scores: tensor memory, 64 columns a term)
     const auto b_at = [&](int p, int s) { return umma_desc_mn128(one + p * S::kValueTerm + s * 2048, kLtSub); };
@@ -397,7 +352,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     if (leader) umma_commit(bar + 16);
     __syncwarp();
   }
-  lt_wait(bar + 16, a.error_word, 0x7C0084);
+  ft_wait(bar + 16, 0, a.error_word, 0x7C0084);
 #pragma unroll
   for (int c0 = 0; c0 < TV / 4; c0 += 16) {
     uint32_t x[16], y[16];
@@ -412,7 +367,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
 #pragma unroll
     for (int c0 = 0; c0 < TV / 4; c0 += 8) {
       const float o[8] = {sum[c0], sum[c0 + 1], sum[c0 + 2], sum[c0 + 3], sum[c0 + 4], sum[c0 + 5], sum[c0 + 6], sum[c0 + 7]};
-      lt_store8(dst + c0, o);
+      ft_store8(dst + c0, o);
     }
   }
   __syncwarp();
@@ -435,7 +390,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
       __syncwarp();
     }
   }
-  lt_release(warp, tmem, 512);
+  ft_release(warp, tmem, 512);
 }
 
 template <typename T, int D, int TV, int ACC>

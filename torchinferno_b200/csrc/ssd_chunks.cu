@@ -14,38 +14,24 @@
 // the steps are added as ordinary fp32 numbers.  What is not finite stays with the tokens it concerns, as in the walk, though an
 // infinity may come out as NaN (where it meets a term or a decay of zero).
 //
-// The walk of ssd_scan_kernel spends five fp32 operations per state element and token twice over (two prompts of 1,366 and 682
-// tokens, 64 heads of 64 with a state of 128: 182 + 32 + 264 us, the fp32 pipe at 40 %).  Here a token costs its share of the
-// products above on mma.sync: 39 + 32 + 98 us cold.  Error against 64 bits there: y 9.8e-8, the walk 8.5e-8; with steps of e^-8 and
-// less, where the walk adds a thousand small terms one by one, 1e-7 against 6e-6.  What bounds it: the legacy tensor path with operands from shared memory, and the
-// states' way through the L2 (one of 32 KB a head and chunk, written twice and read twice).
+// Heads in whole tiles of 64 columns run the first and the last on tcgen05 (ssd_tcgen05.cu); the kernels here, on mma.sync, take tiles of 32 (heads
+// of 32 or 96 columns).  The walk of ssd_scan_kernel spends five fp32 operations per state element and token twice over (two prompts of 1,366
+// and 682 tokens, 64 heads of 64 with a state of 128: 182 + 32 + 264 us, the fp32 pipe at 40 %), the products took 39 + 32 + 98 us
+// cold here and take 29 + 33 + 65 there.  Error against 64 bits of such a scan: y 9.8e-8 in both, the walk 8.5e-8; with steps of e^-8 and less, where
+// the walk adds a thousand small terms one by one, 1e-7 against 6e-6.  What bounds it: the legacy tensor path with operands from shared memory,
+// and the states' way through the L2 (one of 32 KB a head of 64 and chunk, written twice and read twice).
 #include "state_space.cuh"
-#include "mma.cuh"
+#include "split_terms.cuh"
 #include <type_traits>
 
 namespace tib {
 
 constexpr int kQ = kSsdChunk;
 constexpr int kSsdThreads = 256;
+constexpr int kSsdTile = 32;            // columns of a head a block takes
 constexpr int kSsdRows = 32;            // rows of the state staged at a time
 
 __device__ __forceinline__ size_t ssd_first_chunk(int row0, int entry) { return (size_t)(row0 / kQ) + entry; }
-
-// a and b as three bf16 terms each, packed (a in the low half).  What the first term cannot hold (an infinity; anything above
-// 3.39e38) is an infinity there, with nothing left for the others.
-__device__ __forceinline__ void ssd_split2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  const float2 hf = bf16x2_floats(h);
-  float ra = a - hf.x, rb = b - hf.y;
-  ra = isfinite(hf.x) ? ra : 0.f;
-  rb = isfinite(hf.y) ? rb : 0.f;
-  const __nv_bfloat162 m = __floats2bfloat162_rn(ra, rb);
-  const float2 mf = bf16x2_floats(m);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(ra - mf.x, rb - mf.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  mid = *reinterpret_cast<const uint32_t*>(&m);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
 
 // d = a . b over eight of the sixteen k of a fragment (halves 0 and 1)
 __device__ __forceinline__ void ssd_mma8(float (&d)[4], const uint32_t (&a)[4], uint32_t b, int half) {
@@ -56,11 +42,6 @@ __device__ __forceinline__ void ssd_mma8(float (&d)[4], const uint32_t (&a)[4], 
 __device__ __forceinline__ void ssd_add(float (&sum)[4], const float (&step)[4]) {
 #pragma unroll
   for (int c = 0; c < 4; ++c) sum[c] += step[c];
-}
-
-// The bits of a packed pair that belong to finite numbers.
-__device__ __forceinline__ uint32_t ssd_finite2(uint32_t v) {
-  return ((v & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
 }
 
 // Step sizes and sums of log decays of a chunk's n tokens (tokens behind it: no step, the sum stays).  Called by the whole block;
@@ -145,7 +126,7 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_sums_kernel(ScanArgs a) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float2 v = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&raw[q]));
-      ssd_split2(v.x * w, v.y * w, term[0][q], term[1][q], term[2][q]);
+      ft_split2_finite(v.x * w, v.y * w, term[0][q], term[1][q], term[2][q]);
     }
 #pragma unroll
     for (int u = 0; u < 3; ++u) *reinterpret_cast<uint4*>(wx + (u * kQ + r) * PS + c) = make_uint4(term[u][0], term[u][1], term[u][2], term[u][3]);
@@ -276,8 +257,8 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
     for (int i = 0; i < SV; ++i) {
       const int p = threadIdx.x + i * kSsdThreads, r = p / (PT / 4), c = (p % (PT / 4)) * 4;
       uint32_t lo[3], hi[3];
-      ssd_split2(sv[i].x, sv[i].y, lo[0], lo[1], lo[2]);
-      ssd_split2(sv[i].z, sv[i].w, hi[0], hi[1], hi[2]);
+      ft_split2_finite(sv[i].x, sv[i].y, lo[0], lo[1], lo[2]);
+      ft_split2_finite(sv[i].z, sv[i].w, hi[0], hi[1], hi[2]);
 #pragma unroll
       for (int u = 0; u < 3; ++u) *reinterpret_cast<uint2*>(ss + (u * kSsdRows + r) * PS + c) = make_uint2(lo[u], hi[u]);
     }
@@ -321,7 +302,7 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
 #pragma unroll
   for (int p = lane; p < 16 * PT / 8; p += 32) {
     const uint4 v = *reinterpret_cast<const uint4*>(xs + (m0 + p / (PT / 8)) * PS + (p % (PT / 8)) * 8);
-    odd |= (ssd_finite2(v.x) & ssd_finite2(v.y) & ssd_finite2(v.z) & ssd_finite2(v.w)) != 0xffffffffu;
+    odd |= (ft_finite2(v.x) & ft_finite2(v.y) & ft_finite2(v.z) & ft_finite2(v.w)) != 0xffffffffu;
   }
   odd = __any_sync(0xffffffffu, odd);
   const auto within = [&](auto checked) {         // (the common case without the check)
@@ -354,7 +335,7 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
           const int i = r == 0 ? i0 : i1, j = j0 + half * 8 + 2 * t4;
           const float v0 = j <= i ? s[half][2 * r] * (ssd_decay(st, i, j) * st.dt[j]) : 0.f;
           const float v1 = j + 1 <= i ? s[half][2 * r + 1] * (ssd_decay(st, i, j + 1) * st.dt[j + 1]) : 0.f;
-          ssd_split2(v0, v1, w[0][half * 2 + r], w[1][half * 2 + r], w[2][half * 2 + r]);
+          ft_split2_finite(v0, v1, w[0][half * 2 + r], w[1][half * 2 + r], w[2][half * 2 + r]);
         }
 #pragma unroll
       for (int j = 0; j < NT / 2; ++j) {
@@ -362,7 +343,7 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
         ldmatrix_x4_trans(b, xs + (j0 + ((lane >> 3) & 1) * 8 + (lane & 7)) * PS + j * 16 + ((lane >> 4) << 3));
         if (CHECKED && j0 == m0) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) b[q] &= ssd_finite2(b[q]);
+          for (int q = 0; q < 4; ++q) b[q] &= ft_finite2(b[q]);
         }
         float step[2][4] = {};
 #pragma unroll
@@ -409,30 +390,35 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
   }
 }
 
-template <int N, int PT>
+int ssd_fold(const ScanArgs& a, int n_entries, cudaStream_t stream) {
+  TIB_LAUNCH_DEPENDENT(ssd_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.heads * a.N * a.P, 1024), n_entries), 256, 0, stream, a);
+  return TIB_OK;
+}
+
+template <int N>
 static int launch_ssd_chunks(const ScanArgs& a, int n_entries, int max_q_len, cudaStream_t stream) {
-  constexpr int sums = 2 * (kQ * (N + 8) + 3 * kQ * (PT + 8)), outs = 2 * (2 * kQ * (N + 8) + kQ * (PT + 8) + 3 * kSsdRows * (PT + 8));
+  constexpr int PT = kSsdTile, sums = 2 * (kQ * (N + 8) + 3 * kQ * (PT + 8)), outs = 2 * (2 * kQ * (N + 8) + kQ * (PT + 8) + 3 * kSsdRows * (PT + 8));
   cudaError_t e = cudaFuncSetAttribute(ssd_sums_kernel<N, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sums);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_outs_kernel<N, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, outs);
   if (e != cudaSuccess) return (int)e;
   const dim3 grid(a.heads * (a.P / PT), ceil_div(max_q_len, kQ), n_entries);
   TIB_LAUNCH_DEPENDENT((ssd_sums_kernel<N, PT>), grid, kSsdThreads, sums, stream, a);
-  TIB_LAUNCH_DEPENDENT(ssd_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.heads * N * a.P, 1024), n_entries), 256, 0, stream, a);
+  const int status = ssd_fold(a, n_entries, stream);
+  if (status != TIB_OK) return status;
   TIB_LAUNCH_DEPENDENT((ssd_outs_kernel<N, PT>), grid, kSsdThreads, outs, stream, a);
   return TIB_OK;
 }
 
-// bf16 rows on 16-byte boundaries, a state of 64 or 128, heads in whole tiles of 32 or 64 columns, states on 16-byte boundaries.
+// bf16 rows on 16-byte boundaries, a state of 64 or 128, heads in whole tiles of 32 columns, states on 16-byte boundaries.
 bool ssd_chunks_takes(const ScanArgs& a) {
   const int64_t inner = (int64_t)a.heads * a.P;
   return a.xbc_dtype == TIB_BF16 && (a.N == 64 || a.N == 128) && a.P % 32 == 0 && a.ld_xbc % 8 == 0 && inner % 8 == 0 && a.state_stride % 4 == 0 &&
          (((uintptr_t)a.xbc | (uintptr_t)a.state | (uintptr_t)a.run_state | (uintptr_t)a.y) & 15) == 0;
 }
 
-int ssd_chunks(const ScanArgs& a, int n_entries, int max_q_len, cudaStream_t stream) {
-  if (a.P % 64 == 0)
-    return a.N == 128 ? launch_ssd_chunks<128, 64>(a, n_entries, max_q_len, stream) : launch_ssd_chunks<64, 64>(a, n_entries, max_q_len, stream);
-  return a.N == 128 ? launch_ssd_chunks<128, 32>(a, n_entries, max_q_len, stream) : launch_ssd_chunks<64, 32>(a, n_entries, max_q_len, stream);
+int ssd_chunks(const ScanArgs& a, int n_entries, int n_tokens, int max_q_len, cudaStream_t stream) {
+  if (a.P % 64 == 0) return ssd_tcgen05(a, n_entries, n_tokens, max_q_len, stream);
+  return a.N == 128 ? launch_ssd_chunks<128>(a, n_entries, max_q_len, stream) : launch_ssd_chunks<64>(a, n_entries, max_q_len, stream);
 }
 
 }  // namespace tib

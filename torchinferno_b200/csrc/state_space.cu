@@ -547,7 +547,7 @@ TIB_API int tib_ssd_scan(const void* xbc, int xbc_dtype, int64_t ld_xbc, const v
                          const float* dt_bias, const float* a_log, const float* d_skip, float* state, int64_t state_stride,
                          const int* q_start, const int* slots, float* y, int heads, int groups, int N, int P, int n_entries,
                          int n_tokens, int max_q_len, float* run_state, float* run_decay, int64_t run_capacity,
-                         cudaStream_t stream) {
+                         int* error_word, cudaStream_t stream) {
   if (n_entries == 0 || max_q_len == 0) return TIB_OK;
   if (!xbc || !dt || !dt_bias || !a_log || !d_skip || !state || !q_start || !slots || !y) return TIB_E_ARG;
   if (heads < 1 || groups < 1 || heads % groups || N < 1 || P < 1 || N > 32 * kScanLanesN) return TIB_E_SIZE;
@@ -559,8 +559,8 @@ TIB_API int tib_ssd_scan(const void* xbc, int xbc_dtype, int64_t ld_xbc, const v
   a.xbc = xbc; a.xbc_dtype = xbc_dtype; a.ld_xbc = ld_xbc; a.dt = dt; a.dt_dtype = dt_dtype; a.ld_dt = ld_dt; a.dt_col = dt_col;
   a.dt_bias = dt_bias; a.a_log = a_log; a.d_skip = d_skip; a.state = state; a.state_stride = state_stride;
   a.q_start = q_start; a.slots = slots; a.y = y; a.run_state = run_state; a.run_decay = run_decay;
-  a.heads = heads; a.groups = groups; a.N = N; a.P = P;
-  if (runs && ssd_chunks_takes(a)) return ssd_chunks(a, n_entries, max_q_len, stream);
+  a.heads = heads; a.groups = groups; a.N = N; a.P = P; a.error_word = error_word;
+  if (runs && ssd_chunks_takes(a)) return ssd_chunks(a, n_entries, n_tokens, max_q_len, stream);
   const int npt = ceil_div(N, kScanLanesN);
   const bool wide = P > kScanGroups;        // four columns a thread where a head has more columns than a block has groups
 #define TIB_SCAN_CASE(NPT) \

@@ -19,12 +19,16 @@ struct ScanArgs {
   float* y;                                                // [tokens, heads * P] fp32
   float* run_state; float* run_decay;                      // [runs][heads * N * P], [runs][heads]
   int heads, groups, N, P;
+  int* error_word;
 };
 
 // Long portions of bf16 rows on the tensor cores (ssd_chunks.cu), where ssd_chunks_takes them: run_state [runs][heads * N * P] and
 // run_decay [runs][heads] with n_tokens / kSsdChunk + n_entries runs.
 constexpr int kSsdChunk = 128;
 bool ssd_chunks_takes(const ScanArgs& a);
-int ssd_chunks(const ScanArgs& a, int n_entries, int max_q_len, cudaStream_t stream);
+int ssd_chunks(const ScanArgs& a, int n_entries, int n_tokens, int max_q_len, cudaStream_t stream);
+// The same for heads in whole tiles of 64 columns (ssd_tcgen05.cu), and what both run between sums and outputs.
+int ssd_tcgen05(const ScanArgs& a, int n_entries, int n_tokens, int max_q_len, cudaStream_t stream);
+int ssd_fold(const ScanArgs& a, int n_entries, cudaStream_t stream);
 
 }  // namespace tib

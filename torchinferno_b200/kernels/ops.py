@@ -1475,7 +1475,8 @@ def ssd_scan_run() -> int:
 
 def ssd_scan(xbc: torch.Tensor, dt_rows: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, y: torch.Tensor, n_entries: int, *, heads: int,
-             groups: int, state_dim: int, head_dim: int, max_q_len: int | None = None) -> torch.Tensor:
+             groups: int, state_dim: int, head_dim: int, max_q_len: int | None = None,
+             error_word: torch.Tensor | None = None) -> torch.Tensor:
     """The recurrence S_t = a_t S_(t-1) + dt_t B_t x_t^T, y_t = S_t^T C_t + D x_t per head over the ragged batch;
     ``xbc`` rows hold [x | B | C]; ``dt_rows[:, dt_col + h]`` the raw step size of head h; S is the first
     heads * state_dim * head_dim floats of ``state[slot]`` (fp32), read at the start and left at the end.
@@ -1502,7 +1503,7 @@ def ssd_scan(xbc: torch.Tensor, dt_rows: torch.Tensor, dt_col: int, dt_bias: tor
         c_int64(dt_rows.stride(0)), c_int(dt_col), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), c_int64(state.stride(0)),
         _ptr(q_start), _ptr(slots), _ptr(y), c_int(heads), c_int(groups), c_int(state_dim), c_int(head_dim), c_int(n_entries),
         c_int(n_tokens), c_int(n_tokens if max_q_len is None else max_q_len), _ptr(run_state), _ptr(run_decay), c_int64(capacity),
-        _stream()))
+        _ptr(error_word), _stream()))
     return y
 
 
