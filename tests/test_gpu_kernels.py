@@ -1379,6 +1379,27 @@ def test_merged_latent_rows_in_bfloat16_are_the_fp32_rows_rounded_once(contexts,
     assert rows is merged
 
 
+# (rows wider than the queries' registers hold, in whole and odd steps; heads beyond a block's 16; contexts split and, with many entries, whole)
+@pytest.mark.parametrize("heads, rank, rot, entries", [(17, 512, 128, 3), (5, 512, 80, 150), (16, 384, 16, 2), (33, 64, 16, 160), (4, 192, 112, 1)])
+@pytest.mark.parametrize("sink", [False, True])
+def test_latent_single_tokens_on_tensor_cores(heads, rank, rot, entries, sink):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    page, width = 16, rank + rot
+    contexts = [(1, 64, 65, 127, 200, 129)[i % 6] + 64 * (i % 2) for i in range(entries)]
+    per = -(-max(contexts) // page)
+    keys = dev(rnd(entries * per, 1, page, width, dtype=torch.bfloat16, scale=0.7))
+    table = dev(torch.randperm(entries * per, generator=torch.Generator().manual_seed(4)).int().view(entries, per))
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    folded = dev(rnd(entries, heads, width, scale=0.3, seed=1).bfloat16().float())      # (no rounding of the queries between the two kernels)
+    error = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, plain = (ops.latent_attention(folded, keys, torch.empty(entries, heads, rank, device="cuda"), ints(range(entries + 1)), ints(c - 1 for c in contexts),
+                                       ints(range(entries)), table, entries, 1, heads, rank, rot, 0.11, error, max_kv_len=max(contexts),
+                                       sink=dev(rnd(heads, seed=2)) if sink else None, force_simt=simt) for simt in (False, True))
+    # the weights enter as two bf16 terms (2^-17 of each), everything else is fp32 sums of at most `width` or 264 numbers
+    assert (out - plain).abs().max() <= (2.0 ** -16 + 640 * 2.0 ** -23) * plain.abs().max() and int(error) == 0
+
+
 @pytest.mark.parametrize("tokens, experts, kept, top, groups, keep", [(1, 1, 1, 1, 1, 1), (31, 40, 33, 3, 4, 2), (64, 300, 300, 8, 1, 1), (65, 64, 64, 2, 8, 3)])
 def test_choices_and_sorting_in_one_launch(tokens, experts, kept, top, groups, keep):
     """Some choices name no expert (``kept`` of ``experts`` are ones): their place is -1."""

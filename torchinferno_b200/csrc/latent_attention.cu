@@ -18,8 +18,8 @@
 //                       (token, head) row and walks the keys in blocks of 32 aligned to absolute positions, so a
 //                       row's arithmetic does not depend on how the batch was cut;
 //                     - tensor cores (mma.sync m16n8k16) for bf16 latent rows with rank a multiple of 64: tiles of
-//                       64 keys aligned to absolute positions through two cp.async stages; the four warps of a
-//                       block split a tile's keys for the scores and the value columns for the output; scores,
+//                       64 keys aligned to absolute positions through two cp.async stages; the warps of a
+//                       block (four; single tokens: sixteen) split a tile's keys for the scores and the value columns for the output; scores,
 //                       maxima, sums and the accumulator are fp32, and the softmax weights enter the second
 //                       product as TWO bf16 terms (p = hi + lo, 16 bits of mantissa), so they are not cut to 8.
 #include "mma.cuh"
@@ -346,14 +346,15 @@ static inline size_t latent_mma_smem(int width, int mt) {
          + 4 * ((size_t)2 * kMmaWarps * mt * 16);                                                          // fp32: maxima and sums per warp
 }
 
-// MT: m-tiles of 16 rows a block owns (rows are (token, head) pairs of one entry, heads fastest);
+constexpr int kMmaTiles = 2;        // m-tiles of 16 rows a block owns (rows are (token, head) pairs of one entry, heads fastest)
+
 // R64 = rank / 64: every warp owns 16 * R64 value columns.
-template <int MT, int R64>
+template <int R64>
 __global__ void __launch_bounds__(kMmaWarps * 32)
 latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat16* __restrict__ pool, float* __restrict__ out,
                             LatentAttnArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int RB = MT * 16;
+  constexpr int MT = kMmaTiles, RB = MT * 16;
   const int w = a.width, wp = w + 8, pp = kMmaKeys + 8;
   __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);       // [RB][wp]
   __nv_bfloat16* k_s = q_s + RB * wp;                                     // [2][64][wp]
@@ -367,8 +368,7 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
   const int row0 = a.q_start[entry] - a.row_base;
   const int q_len = a.q_start[entry + 1] - a.row_base - row0;
   const int total_rows = q_len * a.heads;
-  const int split = a.partial ? blockIdx.x : 0;
-  const int r0 = a.partial ? blockIdx.z * RB : blockIdx.x * RB;           // first (token, head) row of the block
+  const int r0 = blockIdx.x * RB;                                         // first (token, head) row of the block
   if (r0 >= total_rows || q_len > a.longest) return;
   const int nrows = min(RB, total_rows - r0);
   const int kv0 = a.kv_start[entry];
@@ -376,12 +376,7 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
   const int* table = a.block_table + (size_t)a.slots[entry] * a.table_stride;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
 
-  int tile_lo = 0, tile_hi = last_pos / kMmaKeys;
-  if (a.partial) {      // (blocks_per_split counts runs of 32 keys; a tile is two of them)
-    const int tiles_per_split = (a.blocks_per_split + 1) / 2;
-    tile_lo = split * tiles_per_split;
-    tile_hi = min(tile_hi, tile_lo + tiles_per_split - 1);
-  }
+  const int tile_lo = 0, tile_hi = last_pos / kMmaKeys;
   const int pieces_per_key = w / 8;
   auto fetch = [&](int stage, int tile) {      // a warp takes every fourth key, its lanes the 16-byte pieces of the row
     __nv_bfloat16* dst = k_s + (size_t)stage * kMmaKeys * wp;
@@ -566,24 +561,219 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
     for (int h = 0; h < 2; ++h) {
       const int r = mt * 16 + g + h * 8;
       if (r >= nrows) continue;
-      if (a.partial) {      // (one token per entry: the block's rows are heads)
-        float* p = a.partial + (((size_t)row0 * a.heads + r0 + r) * a.n_splits + split) * (2 + a.rank);
-        if (warp == 0 && t4 == 0) { p[0] = m_run[mt][h]; p[1] = l_run[mt][h]; }
+      float* dst = out + ((size_t)row0 * a.heads + r0 + r) * a.rank;
+      const float inv = latent_inverse(m_run[mt][h], l_run[mt][h], a.sink, (r0 + r) % a.heads);
 #pragma unroll
-        for (int n = 0; n < 2 * R64; ++n) {
-          p[2 + col0 + n * 8 + 2 * t4] = o[mt][n][2 * h];
-          p[2 + col0 + n * 8 + 2 * t4 + 1] = o[mt][n][2 * h + 1];
-        }
-      } else {
-        float* dst = out + ((size_t)row0 * a.heads + r0 + r) * a.rank;
-        const float inv = latent_inverse(m_run[mt][h], l_run[mt][h], a.sink, (r0 + r) % a.heads);
-#pragma unroll
-        for (int n = 0; n < 2 * R64; ++n) {
-          dst[col0 + n * 8 + 2 * t4] = o[mt][n][2 * h] * inv;
-          dst[col0 + n * 8 + 2 * t4 + 1] = o[mt][n][2 * h + 1] * inv;
-        }
+      for (int n = 0; n < 2 * R64; ++n) {
+        dst[col0 + n * 8 + 2 * t4] = o[mt][n][2 * h] * inv;
+        dst[col0 + n * 8 + 2 * t4 + 1] = o[mt][n][2 * h + 1] * inv;
       }
     }
+}
+
+// ------------------------------------------------------- single tokens on the tensor cores
+// One token an entry: a block of 16 warps owns 16 heads of an entry, or of one run of its keys.  Per tile of 64 keys a warp makes the scores of
+// 16 keys over a fourth of the row's width, then the softmax of one head, then 16 or 32 value columns: the chain of one tile is some
+// 20 products and four barriers long.  What bounds it is that chain, the lookups before the first tile and, cold, the rows: eight tokens of 16
+// heads over 3,000 cached rows of 576 take 14 us, and took 33 in blocks of four warps that looked every key's page up by itself (16 with
+// queries read from shared memory for every tile).  The layer: 50 us (66); 12 tokens of 32 heads over 2,000 rows of 320: 54 (84).
+constexpr int kLdThreads = 512;
+constexpr int kLdScores = kMmaKeys + 4;      // row stride of the scores
+constexpr int kLdSteps = 9;                  // steps of 16 of a fourth of the row's width whose queries a warp keeps
+
+static inline size_t latent_decode_smem(int width) {
+  const size_t wp = width + 8;
+  return 2 * (16 * wp + 2 * (size_t)kMmaKeys * wp + 2 * 16 * (kMmaKeys + 8)) + 4 * ((size_t)4 * 16 * kLdScores + 16);
+}
+
+template <int R64>
+__global__ void __launch_bounds__(kLdThreads)
+latent_decode_kernel(const float* __restrict__ folded, const __nv_bfloat16* __restrict__ pool, float* __restrict__ out, LatentAttnArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int PAIRS = (R64 * 4 + 15) / 16;      // pairs of eight value columns a warp makes at most
+  const int w = a.width, wp = w + 8, pp = kMmaKeys + 8;
+  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);       // [16][wp]
+  __nv_bfloat16* k_s = q_s + 16 * wp;                                     // [2][64][wp]
+  __nv_bfloat16* p_hi = k_s + 2 * kMmaKeys * wp;                          // [16][pp]
+  __nv_bfloat16* p_lo = p_hi + 16 * pp;                                   // [16][pp]
+  float* sc = reinterpret_cast<float*>(p_lo + 16 * pp);                   // [4][16][kLdScores]
+  float* alpha_s = sc + 4 * 16 * kLdScores;                               // [16]
+  pdl_wait();
+  pdl_trigger();
+  const int entry = blockIdx.y;
+  const int row0 = a.q_start[entry] - a.row_base;
+  if (a.q_start[entry + 1] - a.row_base - row0 != 1) return;
+  const int h0 = blockIdx.z * 16, nrows = min(16, a.heads - h0);
+  const int last_pos = a.kv_start[entry];                                 // the token's own position: the last key
+  const int* table = a.block_table + (size_t)a.slots[entry] * a.table_stride;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const int split = a.partial ? blockIdx.x : 0;
+  int tile_lo = 0, tile_hi = last_pos / kMmaKeys;
+  if (a.partial) {      // (blocks_per_split counts runs of 32 keys; a tile is two of them)
+    const int tiles_per_split = (a.blocks_per_split + 1) / 2;
+    tile_lo = split * tiles_per_split;
+    tile_hi = min(tile_hi, tile_lo + tiles_per_split - 1);
+  }
+  const int pieces = w / 8;
+  // A warp takes four keys of a tile: a lane finds each one's row (a tile's lookups are under way two tiles ahead), all lanes copy it.
+  auto find = [&](int tile) -> long long {
+    const int kp = tile * kMmaKeys + warp * 4 + (lane & 3);
+    long long at = -1;
+    if (kp <= last_pos && tile <= tile_hi) {
+      const int page = table[kp / a.page_size];
+      if (page >= 0 && page < a.num_pages) at = (long long)page * a.page_stride + (long long)(kp % a.page_size) * w;
+      else if (a.error_word && lane < 4) atomicExch(a.error_word, 0x30000 + entry);
+    }
+    return at;
+  };
+  auto fetch = [&](int stage, long long at) {
+    __nv_bfloat16* dst = k_s + ((size_t)stage * kMmaKeys + warp * 4) * wp;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long from = __shfl_sync(0xffffffffu, at, j);
+      for (int c = lane; c < pieces; c += 32)      // (not valid: zeros; such keys are always masked)
+        cp_async16(dst + j * wp + c * 8, from >= 0 ? pool + from + c * 8 : pool, from >= 0);
+    }
+    cp_async_commit();
+  };
+  const long long rows0 = find(tile_lo), rows1 = find(tile_lo + 1);
+  long long rows2 = find(tile_lo + 2);
+  if (tile_lo <= tile_hi) fetch(0, rows0);        // (the first two tiles are on their way while the queries are read)
+  if (tile_lo + 1 <= tile_hi) fetch(1, rows1);
+  {
+    const float4* src = reinterpret_cast<const float4*>(folded + ((size_t)row0 * a.heads + h0 + warp) * w);
+    for (int c = lane; c < w / 4; c += 32) {
+      const float4 v = warp < nrows ? src[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<uint2*>(q_s + warp * wp + c * 4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    }
+  }
+  float m_run = -CUDART_INF_F, l_run = 0.f;      // of head h0 + warp
+  float o[PAIRS][2][4];
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[i][n][c] = 0.f;
+  // scores: the warp's fourth of the row's width and its 16 keys; the queries' fragments stay in registers (eight warps that read them from
+  // shared memory again for every tile were bound by that)
+  const int steps = w / 16, fourth = warp >> 2, each = (steps + 3) / 4, first_step = fourth * each, own = max(0, min(each, steps - first_step));
+  const __nv_bfloat16* qrow = q_s + (lane & 15) * wp + (lane >> 4) * 8 + first_step * 16;
+  uint32_t qa[kLdSteps][4];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kLdSteps; ++k)
+    if (k < own) ldmatrix_x4(qa[k], qrow + k * 16);
+  for (int tile = tile_lo; tile <= tile_hi; ++tile) {
+    const int stage = (tile - tile_lo) & 1;
+    if (tile + 1 <= tile_hi) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();                                   // the tile (and, the first time, q_s) is in shared memory
+    const __nv_bfloat16* kt = k_s + (size_t)stage * kMmaKeys * wp;
+    {
+      float s[2][4] = {};
+      const __nv_bfloat16* krow = kt + ((warp & 3) * 16 + ((lane >> 4) << 3) + (lane & 7)) * wp + ((lane >> 3) & 1) * 8 + first_step * 16;
+#pragma unroll
+      for (int k = 0; k < kLdSteps; ++k)
+        if (k < own) {
+          uint32_t b[4];
+          ldmatrix_x4(b, krow + k * 16);
+          mma_bf16(s[0], qa[k], b[0], b[1]);
+          mma_bf16(s[1], qa[k], b[2], b[3]);
+        }
+      for (int k = kLdSteps; k < own; ++k) {      // (rows wider than 576)
+        uint32_t b[4], q[4];
+        ldmatrix_x4(q, qrow + k * 16);
+        ldmatrix_x4(b, krow + k * 16);
+        mma_bf16(s[0], q, b[0], b[1]);
+        mma_bf16(s[1], q, b[2], b[3]);
+      }
+      float* to = sc + (fourth * 16 + g) * kLdScores + (warp & 3) * 16 + 2 * t4;
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        *reinterpret_cast<float2*>(to + n * 8) = make_float2(s[n][0], s[n][1]);
+        *reinterpret_cast<float2*>(to + n * 8 + 8 * kLdScores) = make_float2(s[n][2], s[n][3]);
+      }
+    }
+    __syncthreads();
+    {
+      float s[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int key = lane + 32 * i;
+        const float* of = sc + warp * kLdScores + key;
+        const float sum = (of[0] + of[16 * kLdScores]) + (of[32 * kLdScores] + of[48 * kLdScores]);
+        s[i] = tile * kMmaKeys + key <= last_pos ? sum * a.scale : -CUDART_INF_F;
+      }
+      const float m_new = fmaxf(m_run, warp_max(fmaxf(s[0], s[1])));
+      const float base = m_new == -CUDART_INF_F ? 0.f : m_new;
+      const float alpha = m_run == -CUDART_INF_F ? 0.f : expf(m_run - base);
+      m_run = m_new;
+      const float p0 = expf(s[0] - base), p1 = expf(s[1] - base);
+      l_run = l_run * alpha + warp_sum(p0 + p1);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float p = i ? p1 : p0;
+        const __nv_bfloat16 hi = __float2bfloat16_rn(p);
+        p_hi[warp * pp + lane + 32 * i] = hi;
+        p_lo[warp * pp + lane + 32 * i] = __float2bfloat16_rn(p - __bfloat162float(hi));
+      }
+      if (lane == 0) alpha_s[warp] = alpha;
+    }
+    __syncthreads();
+    const float up = alpha_s[g], down = alpha_s[g + 8];
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        o[i][n][0] *= up; o[i][n][1] *= up;
+        o[i][n][2] *= down; o[i][n][3] *= down;
+      }
+#pragma unroll
+    for (int ks = 0; ks < kMmaKeys / 16; ++ks) {
+      uint32_t ph[4], pl[4];
+      ldmatrix_x4(ph, p_hi + (lane & 15) * pp + ks * 16 + (lane >> 4) * 8);
+      ldmatrix_x4(pl, p_lo + (lane & 15) * pp + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int i = 0; i < PAIRS; ++i) {
+        const int pair = warp + 16 * i;
+        if (R64 * 4 % 16 != 0 && pair >= R64 * 4) break;
+        uint32_t v[4];     // (k lo, n 0-7), (k hi, n 0-7), (k lo, n 8-15), (k hi, n 8-15), transposed on the way in
+        ldmatrix_x4_trans(v, kt + (ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * wp + pair * 16 + ((lane >> 4) << 3));
+        mma_bf16(o[i][0], ph, v[0], v[1]);
+        mma_bf16(o[i][1], ph, v[2], v[3]);
+        mma_bf16(o[i][0], pl, v[0], v[1]);
+        mma_bf16(o[i][1], pl, v[2], v[3]);
+      }
+    }
+    __syncthreads();      // the stage, the scores and the weights are free again
+    if (tile + 2 <= tile_hi) {
+      fetch(stage, rows2);
+      rows2 = find(tile + 3);
+    }
+  }
+  float* part = a.partial ? a.partial + (((size_t)row0 * a.heads + h0) * a.n_splits + split) * (2 + a.rank) : nullptr;
+  if (a.partial) {
+    if (lane == 0 && warp < nrows) *reinterpret_cast<float2*>(part + (size_t)warp * a.n_splits * (2 + a.rank)) = make_float2(m_run, l_run);
+  } else {
+    if (lane == 0) alpha_s[warp] = warp < nrows ? latent_inverse(m_run, l_run, a.sink, h0 + warp) : 0.f;
+    __syncthreads();
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = g + 8 * h;
+    if (r >= nrows) continue;
+    const float inv = a.partial ? 1.f : alpha_s[r];
+    float* dst = a.partial ? part + (size_t)r * a.n_splits * (2 + a.rank) + 2 : out + ((size_t)row0 * a.heads + h0 + r) * a.rank;
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+      const int pair = warp + 16 * i;
+      if (R64 * 4 % 16 != 0 && pair >= R64 * 4) break;
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+        *reinterpret_cast<float2*>(dst + pair * 16 + n * 8 + 2 * t4) = make_float2(o[i][n][2 * h] * inv, o[i][n][2 * h + 1] * inv);
+    }
+  }
 }
 
 static int launch_latent_merge(float* out, const LatentAttnArgs& a, int n_entries, cudaStream_t stream) {
@@ -596,18 +786,22 @@ static int launch_latent_merge(float* out, const LatentAttnArgs& a, int n_entrie
   return TIB_OK;
 }
 
-template <int MT, int R64>
-static int launch_latent_mma(const float* folded, const void* pool, float* out, const LatentAttnArgs& a, int n_entries,
-                             int max_q_len, cudaStream_t stream) {
-  const size_t smem = latent_mma_smem(a.width, MT);
-  if (smem > 227 * 1024) return TIB_E_SMEM;
-  auto kern = latent_attention_mma_kernel<MT, R64>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int R64>
+static int launch_latent_mma(const float* folded, const void* pool, float* out, const LatentAttnArgs& a, int n_entries, int max_q_len,
+                             cudaStream_t stream) {
+  if (max_q_len == 1) {
+    const size_t smem = latent_decode_smem(a.width);
+    const cudaError_t e = cudaFuncSetAttribute(latent_decode_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    TIB_LAUNCH_DEPENDENT(latent_decode_kernel<R64>, dim3(a.partial ? a.n_splits : 1, n_entries, ceil_div(a.heads, 16)), kLdThreads, smem, stream,
+                         folded, (const __nv_bfloat16*)pool, out, a);
+    return a.partial ? launch_latent_merge(out, a, n_entries, stream) : TIB_OK;
+  }
+  const size_t smem = latent_mma_smem(a.width, kMmaTiles);
+  const cudaError_t e = cudaFuncSetAttribute(latent_attention_mma_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const int rb = MT * 16;
-  dim3 grid(a.partial ? a.n_splits : ceil_div(max_q_len * a.heads, rb), n_entries, a.partial ? ceil_div(a.heads, rb) : 1);
-  TIB_LAUNCH_DEPENDENT(kern, grid, kMmaWarps * 32, smem, stream, folded, (const __nv_bfloat16*)pool, out, a);
-  if (a.partial) return launch_latent_merge(out, a, n_entries, stream);
+  TIB_LAUNCH_DEPENDENT(latent_attention_mma_kernel<R64>, dim3(ceil_div(max_q_len * a.heads, kMmaTiles * 16), n_entries), kMmaWarps * 32, smem, stream,
+                       folded, (const __nv_bfloat16*)pool, out, a);
   return TIB_OK;
 }
 
@@ -704,17 +898,16 @@ TIB_API int tib_latent_attention(const float* folded, const void* pool, float* o
   const int width = rank + rot;
   if (dtype == TIB_BF16 && !force_simt && width % 16 == 0 && rank % 64 == 0 && (page_stride % 8) == 0 && ((uintptr_t)pool & 15) == 0) {
     const int r64 = rank / 64;
-    const bool single = max_q_len == 1;
-    if (latent_mma_smem(width, single ? 1 : 2) <= 227 * 1024 && (r64 <= 4 || r64 == 6 || r64 == 8)) {
-#define TIB_LAT_MMA(MT)                                                                                         \
-  (r64 == 1 ? launch_latent_mma<MT, 1>(folded, pool, out, a, n_entries, max_q_len, stream)                     \
-   : r64 == 2 ? launch_latent_mma<MT, 2>(folded, pool, out, a, n_entries, max_q_len, stream)                   \
-   : r64 == 3 ? launch_latent_mma<MT, 3>(folded, pool, out, a, n_entries, max_q_len, stream)                   \
-   : r64 == 4 ? launch_latent_mma<MT, 4>(folded, pool, out, a, n_entries, max_q_len, stream)                   \
-   : r64 == 6 ? launch_latent_mma<MT, 6>(folded, pool, out, a, n_entries, max_q_len, stream)                   \
-              : launch_latent_mma<MT, 8>(folded, pool, out, a, n_entries, max_q_len, stream))
-      return single ? TIB_LAT_MMA(1) : TIB_LAT_MMA(2);
-#undef TIB_LAT_MMA
+    const size_t smem = max_q_len == 1 ? latent_decode_smem(width) : latent_mma_smem(width, kMmaTiles);
+    if (smem <= 227 * 1024 && (r64 <= 4 || r64 == 6 || r64 == 8) && (((uintptr_t)folded | (uintptr_t)out) & 15) == 0 && ((uintptr_t)partial & 7) == 0) {
+      switch (r64) {
+        case 1: return launch_latent_mma<1>(folded, pool, out, a, n_entries, max_q_len, stream);
+        case 2: return launch_latent_mma<2>(folded, pool, out, a, n_entries, max_q_len, stream);
+        case 3: return launch_latent_mma<3>(folded, pool, out, a, n_entries, max_q_len, stream);
+        case 4: return launch_latent_mma<4>(folded, pool, out, a, n_entries, max_q_len, stream);
+        case 6: return launch_latent_mma<6>(folded, pool, out, a, n_entries, max_q_len, stream);
+        default: return launch_latent_mma<8>(folded, pool, out, a, n_entries, max_q_len, stream);
+      }
     }
   }
   const int dpl = (rank + 31) / 32;
