@@ -1332,6 +1332,62 @@ def test_append_with_one_table_of_angles_agrees_with_the_plain_kernel(tokens, he
         assert torch.equal(got, plain)      # (the same turns and sums in fp32, each rounded once to bfloat16)
 
 
+# (297 tokens are the fewest that go in pieces of 16 bytes; halves of eight elements, heads that are turned whole or not at all, more pieces than threads)
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim, rot, turned, bias", [
+    (3, 1, 64, 64, 64, True, True), (5, 2, 32, 16, 16, True, False), (24, 8, 128, 128, 32, True, True), (2, 2, 48, 80, 0, False, True), (4, 4, 256, 256, 128, True, False)])
+def test_append_in_pieces_agrees_with_the_plain_kernel(heads, kv_heads, dim, vdim, rot, turned, bias):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    tokens, page = 297, 8
+    total, pages = heads * dim + kv_heads * (dim + vdim), -(-tokens // page) + 1
+    rows, biases = rnd(tokens, total, dtype=torch.bfloat16), [dev(rnd(w, seed=i)) if bias else None for i, w in enumerate((heads * dim, kv_heads * dim, kv_heads * vdim))]
+    freq = dev(1e4 ** (-torch.arange(rot // 2) / max(rot // 2, 1)))
+    vfreq = dev(1e4 ** (-torch.arange(vdim // 2) / (vdim // 2))) if turned else None
+    table = dev(torch.randperm(pages, generator=torch.Generator().manual_seed(3)).int().view(1, pages))
+    results = []
+    for shift in (8, 1):      # (columns off their boundaries take the plain kernel)
+        wide = torch.zeros(tokens, total + 8, dtype=torch.bfloat16)
+        wide[:, shift:shift + total] = rows
+        keys, values = page_views(pages, kv_heads, page, dim, vdim, torch.bfloat16)
+        q = torch.empty(tokens, heads * dim, dtype=torch.bfloat16, device="cuda")
+        turns = torch.empty(tokens, vdim // 2, 2, device="cuda") if turned else None
+        ops.rotary_kv_append(dev(wide), shift, shift + heads * dim, shift + (heads + kv_heads) * dim, q, keys, values,
+                             dev(torch.arange(tokens, dtype=torch.int32)), torch.zeros(tokens, dtype=torch.int32, device="cuda"), table, freq, vfreq, heads,
+                             kv_heads, dim, vdim, rot_dim=rot, amplitude=1.25, q_bias=biases[0], k_bias=biases[1], v_bias=biases[2], turns=turns)
+        results.append((q, keys, values) + ((turns,) if turned else ()))
+    for got, plain in zip(*results):
+        assert torch.equal(got, plain)      # (the same turns and sums in fp32, each rounded once to bfloat16)
+
+
+@pytest.mark.parametrize("dim, keep, pool", [(64, 0, 16), (128, 0, 64), (128, 40, 0)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_window_attention_with_the_appends_turns_has_the_bits_of_its_own(dim, keep, pool, gated):
+    """Two portions whose tiles begin and end off the window's, the blocks' and the kept tokens' edges."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, kv_heads, page, window, lens, pasts = 4, 2, 16, 150, [130, 260], [333, 0]
+    n, per = sum(lens), 32
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    keys, values = (dev(rnd(2 * per, kv_heads, page, dim, dtype=torch.bfloat16, seed=i)) for i in range(2))
+    means = [dev(rnd(4, kv_heads, page, dim, dtype=torch.bfloat16, seed=5 + i)) for i in range(2)] if pool else [None, None]
+    table, blocks = ints(range(2 * per)).view(2, per), ints(range(4)).view(2, 2)
+    q, gate = dev(rnd(n, heads * dim, dtype=torch.bfloat16)), dev(rnd(n, heads * dim, dtype=torch.bfloat16, seed=9)) if gated else None
+    freq = dev(5e5 ** (-torch.arange(dim // 2) / (dim // 2)))
+    positions = torch.cat([p + torch.arange(m) for m, p in zip(lens, pasts)])
+    angle = dev(positions.float())[:, None] * freq
+    turns = torch.stack([angle.cos(), angle.sin()], -1).contiguous()
+    own = torch.empty_like(turns)
+    pool_keys, pool_values = page_views(60, kv_heads, page, dim, dim, torch.bfloat16)
+    ops.rotary_kv_append(q[:, :2 * kv_heads * dim].repeat(1, 2).contiguous(), 0, 0, 0, torch.empty(n, kv_heads * dim, dtype=torch.bfloat16, device="cuda"), pool_keys, pool_values,
+                         dev(positions.int()), torch.zeros(n, dtype=torch.int32, device="cuda"), ints(range(60)).view(1, 60), freq, freq, kv_heads, kv_heads, dim, dim,
+                         rot_dim=dim, turns=own)
+    assert (own - turns).abs().max() <= 2.0 ** -22      # (cosines and sines to an ulp or two of one)
+    run = lambda turns: ops.pooled_window_attention(q, torch.empty_like(q), ints([0, lens[0], n]), ints(pasts), ints(range(2)), keys, values, table, *means,
+                                                    blocks if pool else None, 2, max(lens), heads, kv_heads, window=window, pool=pool, scale=dim ** -0.5, keep=keep,
+                                                    value_freq=freq, gate=gate, turns=turns)
+    assert torch.equal(run(own), run(None))
+
+
 @pytest.mark.parametrize("tokens, kv_heads, dim, vdim, pool", [(65, 1, 64, 64, 4), (97, 2, 40, 24, 8), (300, 2, 128, 96, 32), (130, 1, 16, 8, 1)])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_block_means_of_large_steps_have_the_bits_of_small_ones(tokens, kv_heads, dim, vdim, pool, dtype):

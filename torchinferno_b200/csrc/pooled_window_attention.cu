@@ -35,6 +35,7 @@ struct PwaAppendArgs {
   const int* positions; const int* token_slot;
   const float* freq; const float* vfreq;                             // [rot_dim / 2], [vdim / 2] (null: values are not turned)
   float amplitude;
+  float2* turns;                                                     // [tokens, vdim / 2] (cosine, sine) of the values' turns, or null
   int heads, kv_heads, dim, vdim, rot_dim;
   PwaCache cache;
   int* error_word;
@@ -56,6 +57,10 @@ __global__ void __launch_bounds__(512) pwa_append_kernel(const T* __restrict__ p
     in_page = pos % a.cache.page_size;
   }
   const int total = a.heads + 2 * a.kv_heads;
+  for (int i = threadIdx.x; a.turns && i < a.vdim / 2; i += blockDim.x) {
+    const float angle = fpos * a.vfreq[i];
+    a.turns[(size_t)t * (a.vdim / 2) + i] = make_float2(cosf(angle), sinf(angle));
+  }
   for (int head = warp; head < total; head += nwarps) {
     if (head < a.heads + a.kv_heads) {       // a query or key head: partial rotary, pairs (i, i + rot/2)
       const bool is_q = head < a.heads;
@@ -126,7 +131,11 @@ __global__ void __launch_bounds__(1024) pwa_append_pairs_kernel(const __nv_bfloa
     const bool key = i < half;
     const float angle = fpos * (key ? a.freq[i] : a.vfreq[i - half]);
     if (key) turn_s[i] = make_float2(cosf(angle) * a.amplitude, sinf(angle) * a.amplitude);
-    else vturn_s[i - half] = make_float2(cosf(angle), sinf(angle));
+    else {
+      const float2 turn = make_float2(cosf(angle), sinf(angle));
+      vturn_s[i - half] = turn;
+      if (a.turns) a.turns[(size_t)t * vhalf + i - half] = turn;
+    }
   }
   int page = -1, in_page = 0;
   if (a.cache.keys) {
@@ -173,6 +182,123 @@ __global__ void __launch_bounds__(1024) pwa_append_pairs_kernel(const __nv_bfloa
            reinterpret_cast<__nv_bfloat16*>(a.cache.values) + (size_t)page * a.cache.page_stride + ((size_t)hh * a.cache.page_size + in_page) * a.vdim,
            a.v_bias ? a.v_bias + hh * a.vdim : nullptr, vturn_s, vhalf, u);
     }
+  }
+}
+
+// The same bits again for large steps whose heads come in whole pieces of 16 bytes: a thread owns 16 elements of a head (eight and their
+// eight partners, or 16 neighbours that are not turned) and asks for them before the token's angles are worked out and its page is
+// found, so that a token is two trips to memory long.  2,048 tokens of 16 + 8 + 8 heads of 128: 14 us, 20 with two elements a thread at a time.
+__global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloat16* __restrict__ proj, __nv_bfloat16* __restrict__ q_out, PwaAppendArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ float2 turn_s[kPwaTurns], vturn_s[kPwaTurns];      // (cosine, sine)
+  const int t = blockIdx.x, pos = a.positions[t], slot = a.cache.keys ? a.token_slot[t] : 0;
+  const __nv_bfloat16* row = proj + (size_t)t * a.ld;
+  const int half = a.rot_dim / 2, vhalf = a.vfreq ? a.vdim / 2 : 0;
+  const int units = a.dim / 16, vunits = a.vdim / 16, qk = (a.heads + a.kv_heads) * units, total = qk + a.kv_heads * vunits;
+  struct Unit { const __nv_bfloat16* src; const float* bias; int head, i, k; bool value; };      // elements i .. i + 7 and k .. k + 7 of a head
+  auto unit_of = [&](int e) {
+    Unit u;
+    u.value = e >= qk;
+    const int per = u.value ? vunits : units, n_half = u.value ? vhalf : half, at = u.value ? e - qk : e;
+    u.head = at / per;
+    const int j = at - u.head * per;
+    u.i = j < n_half / 8 ? j * 8 : 2 * n_half + (j - n_half / 8) * 16;
+    u.k = j < n_half / 8 ? u.i + n_half : u.i + 8;
+    if (u.value) {
+      u.src = row + a.v_off + u.head * a.vdim;
+      u.bias = a.v_bias ? a.v_bias + u.head * a.vdim : nullptr;
+    } else if (u.head < a.heads) {
+      u.src = row + a.q_off + u.head * a.dim;
+      u.bias = a.q_bias ? a.q_bias + u.head * a.dim : nullptr;
+    } else {
+      u.src = row + a.k_off + (u.head - a.heads) * a.dim;
+      u.bias = a.k_bias ? a.k_bias + (u.head - a.heads) * a.dim : nullptr;
+    }
+    return u;
+  };
+  struct Pieces { uint4 lo, hi; float4 bias[4]; };
+  auto ask = [&](const Unit& u) {
+    Pieces p;
+    p.lo = *reinterpret_cast<const uint4*>(u.src + u.i);
+    p.hi = *reinterpret_cast<const uint4*>(u.src + u.k);
+    if (u.bias) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        p.bias[j] = *reinterpret_cast<const float4*>(u.bias + u.i + 4 * j);
+        p.bias[2 + j] = *reinterpret_cast<const float4*>(u.bias + u.k + 4 * j);
+      }
+    }
+    return p;
+  };
+  int page = -1, in_page = 0;
+  auto put = [&](const Unit& u, const Pieces& p) {
+    __nv_bfloat16* dst;
+    if (!u.value && u.head < a.heads) dst = q_out + ((size_t)t * a.heads + u.head) * a.dim;
+    else if (page < 0) return;
+    else if (u.value) dst = reinterpret_cast<__nv_bfloat16*>(a.cache.values) + (size_t)page * a.cache.page_stride + ((size_t)u.head * a.cache.page_size + in_page) * a.vdim;
+    else dst = reinterpret_cast<__nv_bfloat16*>(a.cache.keys) + (size_t)page * a.cache.page_stride + ((size_t)(u.head - a.heads) * a.cache.page_size + in_page) * a.dim;
+    const uint32_t l[4] = {p.lo.x, p.lo.y, p.lo.z, p.lo.w}, h[4] = {p.hi.x, p.hi.y, p.hi.z, p.hi.w};
+    float lo[8], hi[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      lo[2 * j] = __uint_as_float(l[j] << 16); lo[2 * j + 1] = __uint_as_float(l[j] & 0xffff0000u);
+      hi[2 * j] = __uint_as_float(h[j] << 16); hi[2 * j + 1] = __uint_as_float(h[j] & 0xffff0000u);
+    }
+    if (u.bias) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        lo[4 * j] += p.bias[j].x; lo[4 * j + 1] += p.bias[j].y; lo[4 * j + 2] += p.bias[j].z; lo[4 * j + 3] += p.bias[j].w;
+        hi[4 * j] += p.bias[2 + j].x; hi[4 * j + 1] += p.bias[2 + j].y; hi[4 * j + 2] += p.bias[2 + j].z; hi[4 * j + 3] += p.bias[2 + j].w;
+      }
+    }
+    if (u.k - u.i != 8 || u.i < (u.value ? vhalf : half)) {      // turned (partners eight apart: a half of eight, which its index tells apart)
+      const float2* turns = (u.value ? vturn_s : turn_s) + u.i;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 turn = turns[j];
+        const float x = rope_lo(lo[j], hi[j], turn.x, turn.y), y = rope_hi(lo[j], hi[j], turn.x, turn.y);
+        lo[j] = x;
+        hi[j] = y;
+      }
+    }
+    uint4 out[2];
+    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      o[j] = __floats2bfloat162_rn(lo[2 * j], lo[2 * j + 1]);
+      o[4 + j] = __floats2bfloat162_rn(hi[2 * j], hi[2 * j + 1]);
+    }
+    *reinterpret_cast<uint4*>(dst + u.i) = out[0];
+    *reinterpret_cast<uint4*>(dst + u.k) = out[1];
+  };
+  Unit mine;
+  Pieces held;
+  const bool any = (int)threadIdx.x < total;
+  if (any) {
+    mine = unit_of(threadIdx.x);
+    held = ask(mine);
+  }
+  if (a.cache.keys) {
+    const int* table = a.cache.block_table + (size_t)slot * a.cache.table_stride;
+    page = pwa_page(a.cache, table, pos, a.error_word, 0x30000 + (t & 0xffff));
+    in_page = pos % a.cache.page_size;
+  }
+  for (int i = threadIdx.x; i < half + vhalf; i += blockDim.x) {
+    const bool key = i < half;
+    const float angle = (float)pos * (key ? a.freq[i] : a.vfreq[i - half]);
+    const float c = cosf(angle), sn = sinf(angle);
+    if (key) turn_s[i] = make_float2(c * a.amplitude, sn * a.amplitude);
+    else {
+      vturn_s[i - half] = make_float2(c, sn);
+      if (a.turns) a.turns[(size_t)t * vhalf + i - half] = make_float2(c, sn);
+    }
+  }
+  __syncthreads();
+  if (any) put(mine, held);
+  for (int e = threadIdx.x + blockDim.x; e < total; e += blockDim.x) {
+    const Unit u = unit_of(e);
+    put(u, ask(u));
   }
 }
 
@@ -247,6 +373,71 @@ __global__ void __launch_bounds__(kPoolLanes * kPoolTile) pwa_pool_kernel(PwaPoo
         T* out = reinterpret_cast<T*>(is_k ? a.blocks.keys : a.blocks.values);
         out[(size_t)bpage * a.blocks.page_stride + ((size_t)kvh * a.blocks.page_size + b % a.blocks.page_size) * w + dd] = from_f32<T>(total * inv);
       }
+    }
+    if (bad && a.error_word) atomicExch(a.error_word, 0x50000 + (t & 0xffff));
+  }
+}
+
+// The same sums, in the same order, for large steps of bf16 rows in pieces of 16 bytes: a thread sums eight elements of a lane's positions, a
+// block all elements of a key head.  grid (runs of `per` tokens, kv_heads), dim + vdim threads: whole warps, for each looks at all tokens itself.
+// 2,048 tokens of 8 heads of 128 + 128, blocks of 64: 8.5 us, 23 with an element a thread and a tile of 64 a block.
+__global__ void __launch_bounds__(512) pwa_pool_pieces_kernel(PwaPoolArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) float pool_s[];      // [kPoolLanes][dim + vdim]
+  const int t0 = blockIdx.x * a.per, kvh = blockIdx.y, width = a.dim + a.vdim, pieces = width / 8;
+  const int lane = threadIdx.x / pieces, e = (threadIdx.x - lane * pieces) * 8, wl = threadIdx.x & 31;
+  const int my_pos = wl < a.per && t0 + wl < a.n_tokens ? a.positions[t0 + wl] : 0;
+  const int my_slot = wl < a.per && t0 + wl < a.n_tokens ? a.token_slot[t0 + wl] : 0;
+  unsigned todo = __ballot_sync(0xffffffffu, wl < a.per && t0 + wl < a.n_tokens && my_pos % a.pool == a.pool - 1);
+  const float inv = 1.f / (float)a.pool;
+  const bool is_k = e < a.dim;
+  const int dd = is_k ? e : e - a.dim, w = is_k ? a.dim : a.vdim;
+  const __nv_bfloat16* base = reinterpret_cast<const __nv_bfloat16*>(is_k ? a.tokens.keys : a.tokens.values);
+  for (; todo; todo &= todo - 1) {
+    const int bit = __ffs(todo) - 1, t = t0 + bit;
+    const int pos = __shfl_sync(0xffffffffu, my_pos, bit), slot = __shfl_sync(0xffffffffu, my_slot, bit);
+    const int b = pos / a.pool, first = b * a.pool;
+    const int* ttable = a.tokens.block_table + (size_t)slot * a.tokens.table_stride;
+    const int bpage = pwa_page(a.blocks, a.blocks.block_table + (size_t)slot * a.blocks.table_stride, b, a.error_word, 0x40000 + (t & 0xffff));
+    if (bpage < 0) continue;
+    bool bad = false;
+    float sum[8] = {};
+    for (int j0 = lane; j0 < a.pool; j0 += kPoolLanes * kPoolAhead) {
+      uint4 got[kPoolAhead];
+      int page[kPoolAhead];
+#pragma unroll
+      for (int u = 0; u < kPoolAhead; ++u) page[u] = j0 + u * kPoolLanes < a.pool ? ttable[(first + j0 + u * kPoolLanes) / a.tokens.page_size] : 0;
+#pragma unroll
+      for (int u = 0; u < kPoolAhead; ++u) {
+        const int j = first + j0 + u * kPoolLanes;
+        got[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (j0 + u * kPoolLanes >= a.pool) continue;
+        if (page[u] < 0 || page[u] >= a.tokens.num_pages) { bad = true; continue; }
+        got[u] = *reinterpret_cast<const uint4*>(base + (size_t)page[u] * a.tokens.page_stride + ((size_t)kvh * a.tokens.page_size + j % a.tokens.page_size) * w + dd);
+      }
+#pragma unroll
+      for (int u = 0; u < kPoolAhead; ++u) {
+        const uint32_t v[4] = {got[u].x, got[u].y, got[u].z, got[u].w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          sum[2 * c] += __uint_as_float(v[c] << 16);
+          sum[2 * c + 1] += __uint_as_float(v[c] & 0xffff0000u);
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 8; c += 4) *reinterpret_cast<float4*>(pool_s + lane * width + e + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+    __syncthreads();
+    for (int x = threadIdx.x; x < width; x += blockDim.x) {
+      float total = 0.f;
+#pragma unroll
+      for (int l = 0; l < kPoolLanes; ++l) total += pool_s[l * width + x];
+      const bool key = x < a.dim;
+      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(key ? a.blocks.keys : a.blocks.values);
+      const int ow = key ? a.dim : a.vdim;
+      out[(size_t)bpage * a.blocks.page_stride + ((size_t)kvh * a.blocks.page_size + b % a.blocks.page_size) * ow + (key ? x : x - a.dim)] = __float2bfloat16_rn(total * inv);
     }
     if (bad && a.error_word) atomicExch(a.error_word, 0x50000 + (t & 0xffff));
   }
@@ -1043,20 +1234,23 @@ static PwaCache pwa_cache(void* keys, void* values, const int* table, int table_
 using namespace tib;
 
 // proj: [n_tokens, ld] rows holding q at q_off, k at k_off, v at v_off; q_out: [n_tokens, heads * dim]; k_pages / v_pages:
-// first key / value of this layer's first page (null: only q is made).  Biases, freq and vfreq are fp32.
+// first key / value of this layer's first page (null: only q is made).  Biases, freq and vfreq are fp32.  turns: [n_tokens, vdim / 2] pairs that
+// take the cosine and sine the values are turned by (with vfreq), or null.
 TIB_API int tib_rotary_kv_append(const void* proj, int64_t ld, int q_off, int k_off, int v_off, const float* q_bias,
                                  const float* k_bias, const float* v_bias, void* q_out, void* k_pages, void* v_pages,
                                  const int* positions, const int* token_slot, const int* block_table, int table_stride,
                                  const float* freq, const float* vfreq, float amplitude, int n_tokens, int heads, int kv_heads,
-                                 int dim, int vdim, int rot_dim, int page_size, int64_t page_stride, int num_pages, int* error_word,
-                                 int dtype, cudaStream_t stream) {
+                                 int dim, int vdim, int rot_dim, int page_size, int64_t page_stride, int num_pages, float* turns,
+                                 int* error_word, int dtype, cudaStream_t stream) {
   if (n_tokens == 0) return TIB_OK;
+  if ((uintptr_t)turns & 7) return TIB_E_ALIGN;
   if (!proj || !q_out || !positions || n_tokens < 0 || heads < 1 || kv_heads < 1 || dim < 1 || vdim < 1) return TIB_E_ARG;
   if (rot_dim < 0 || rot_dim % 2 || rot_dim > dim || (rot_dim > 0 && !freq) || (vfreq && vdim % 2)) return TIB_E_SIZE;
   if (k_pages && (!v_pages || !token_slot || !block_table || page_size < 1)) return TIB_E_ARG;
   PwaAppendArgs a;
   a.ld = ld; a.q_off = q_off; a.k_off = k_off; a.v_off = v_off; a.q_bias = q_bias; a.k_bias = k_bias; a.v_bias = v_bias;
   a.positions = positions; a.token_slot = token_slot; a.freq = freq; a.vfreq = vfreq; a.amplitude = amplitude;
+  a.turns = vfreq ? reinterpret_cast<float2*>(turns) : nullptr;
   a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim; a.rot_dim = rot_dim;
   a.cache = pwa_cache(k_pages, v_pages, block_table, table_stride, page_size, page_stride, num_pages);
   a.error_word = error_word;
@@ -1066,6 +1260,14 @@ TIB_API int tib_rotary_kv_append(const void* proj, int64_t ld, int q_off, int k_
   if (dtype == TIB_BF16 && dim % 2 == 0 && vdim % 2 == 0 && rot_dim % 4 == 0 && vhalf % 2 == 0 && rot_dim / 2 <= kPwaTurns && vhalf <= kPwaTurns &&
       ld % 2 == 0 && q_off % 2 == 0 && k_off % 2 == 0 && v_off % 2 == 0 && page_stride % 2 == 0 &&
       (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages) & 3) == 0) {
+    const uintptr_t bits = (uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)q_bias | (uintptr_t)k_bias | (uintptr_t)v_bias;
+    if (n_tokens > 2 * 148 && dim % 16 == 0 && vdim % 16 == 0 && rot_dim % 16 == 0 && vhalf % 8 == 0 && ld % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 &&
+        v_off % 8 == 0 && page_stride % 8 == 0 && (bits & 15) == 0) {
+      const int pieces = ((heads + kv_heads) * dim + kv_heads * vdim) / 16;
+      TIB_LAUNCH_DEPENDENT(pwa_append_pieces_kernel, n_tokens, pieces >= 256 ? 256 : pieces <= 128 ? 128 : (pieces + 31) / 32 * 32, 0, stream,
+                           (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a);
+      return TIB_OK;
+    }
     // few tokens: a thread for every two elements, so that a token is one round of loads and not five or six one after the other
     const int units = ((heads + kv_heads) * dim + kv_heads * vdim) / 4;
     const int wide = units > 1024 ? 1024 : units < 256 ? 256 : (units + 31) / 32 * 32;
@@ -1098,6 +1300,11 @@ TIB_API int tib_pool_blocks(const void* k_pages, const void* v_pages, const int*
   a.blocks = pwa_cache(bk_pages, bv_pages, b_table, b_table_stride, b_page_size, b_page_stride, b_num_pages);
   a.error_word = error_word;
   a.n_tokens = n_tokens; a.per = n_tokens > 2 * kPoolRun ? kPoolRun : 1;
+  const uintptr_t bits = (uintptr_t)k_pages | (uintptr_t)v_pages;
+  if (dtype == TIB_BF16 && a.per > 1 && dim % 8 == 0 && vdim % 8 == 0 && (dim + vdim) % 32 == 0 && dim + vdim <= 512 && page_stride % 8 == 0 && (bits & 15) == 0) {
+    TIB_LAUNCH_DEPENDENT(pwa_pool_pieces_kernel, dim3(ceil_div(n_tokens, a.per), kv_heads), dim + vdim, kPoolLanes * (dim + vdim) * 4, stream, a);
+    return TIB_OK;
+  }
   const dim3 grid(ceil_div(n_tokens, a.per), kv_heads, a.per > 1 ? ceil_div(dim + vdim, kPoolTile) : 1);      // (few tokens: most complete nothing)
   if (dtype == TIB_F32) TIB_LAUNCH_DEPENDENT(pwa_pool_kernel<float>, grid, kPoolLanes * kPoolTile, 0, stream, a);
   else if (dtype == TIB_BF16) TIB_LAUNCH_DEPENDENT(pwa_pool_kernel<__nv_bfloat16>, grid, kPoolLanes * kPoolTile, 0, stream, a);
@@ -1121,7 +1328,7 @@ TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_s
                                         const void* bv_pages, const int* b_table, int b_table_stride, int b_page_size,
                                         int64_t b_page_stride, int b_num_pages, int n_entries, int max_q_len, int heads,
                                         int kv_heads, int dim, int vdim, int window, int keep, int pool, float scale, const float* temp,
-                                        const float* sink, const float* vfreq, const void* gate, int gate_dtype, int64_t ld_gate,
+                                        const float* sink, const float* vfreq, const float* turns, const void* gate, int gate_dtype, int64_t ld_gate,
                                         const float* rel_bias, int rel_span, float* partial, int n_splits, int n_tokens,
                                         int few_rows, int* launches, int* error_word, int dtype, int force_simt, cudaStream_t stream) {
   *launches = 0;
@@ -1137,6 +1344,7 @@ TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_s
   PwaArgs a;
   a.q_start = q_start; a.kv_start = kv_start; a.slots = slots; a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim;
   a.window = window; a.keep = keep; a.pool = pool; a.scale = scale; a.temp = temp; a.sink = sink; a.vfreq = vfreq; a.gate = gate;
+  a.turns = vfreq && ((uintptr_t)turns & 15) == 0 ? turns : nullptr;
   a.gate_dtype = gate_dtype; a.ld_gate = ld_gate; a.rel_bias = rel_bias; a.rel_span = rel_span;
   a.tokens = pwa_cache(const_cast<void*>(k_pages), const_cast<void*>(v_pages), block_table, table_stride, page_size, page_stride, num_pages);
   a.blocks = pwa_cache(const_cast<void*>(bk_pages), const_cast<void*>(bv_pages), b_table, b_table_stride, b_page_size, b_page_stride, b_num_pages);

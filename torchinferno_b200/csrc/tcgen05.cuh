@@ -120,6 +120,35 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
 
+// ----- products issued by a whole warp.  The warp walks its loop together and one lane, elected once, issues: operands then stay in uniform
+// registers.  (Measured, cycles an instruction while the tensor core is not the limit: 37 to 46, a lone lane 52 to 55; a phase that is over costs
+// the lone lane's wait 233, this one some 60.)
+__device__ __forceinline__ uint32_t umma_leader() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one;
+}
+// Bounded wait of a whole warp: a test first, for a phase that is over already.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+}
+// Shared-memory descriptors by their lower halves (the upper one is the same for all tiles with rows of 128 bytes, 128-byte swizzle).
+constexpr uint32_t kUmmaDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t umma_low_k128(uint32_t smem_addr) { return ((smem_addr & 0x3FFFF) >> 4) | (1u << 16); }
+__device__ __forceinline__ uint32_t umma_low_mn128(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16); }
+__device__ __forceinline__ void umma_warp(uint32_t leader, uint32_t tmem_d, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p, q;\n.reg .b64 a, b;\nmov.b64 a, {%1, %6};\nmov.b64 b, {%2, %6};\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
+               ::"r"(tmem_d), "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(leader), "r"(kUmmaDescHigh) : "memory");
+}
+// The same with the A operand in tensor memory.
+__device__ __forceinline__ void umma_warp_tmem(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p, q;\n.reg .b64 b;\nmov.b64 b, {%2, %6};\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n"
+               ::"r"(tmem_d), "r"(tmem_a), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(leader), "r"(kUmmaDescHigh) : "memory");
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

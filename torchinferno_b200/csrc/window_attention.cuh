@@ -26,6 +26,7 @@ struct PwaArgs {
   float scale;
   const float* temp; const float* sink;                    // [heads] or null
   const float* vfreq;                                      // [vdim / 2] or null (values were not turned)
+  const float* turns;                                      // [tokens, vdim / 2, 2] cosine and sine of vfreq's angles at the tokens, or null
   const void* gate; int gate_dtype; int64_t ld_gate;       // [tokens, heads * vdim] logits or null
   const float* rel_bias; int rel_span;                     // [heads, rel_span] or null: added to a token's score by distance
   PwaCache tokens, blocks;

@@ -1,6 +1,6 @@
 // Prompt portions of the attention in a sliding window (with averaged blocks behind it, or with the first tokens kept in sight) on the
 // 5th-generation tensor cores.  Contract and exactness as pooled_window_attention.cu; the structure is attention_tcgen05.cu's:
-// a block owns 128 rows (tokens x query heads of a key head), one warp copies queries and keys, one the values, one lane
+// a block owns 128 rows (tokens x query heads of a key head), one warp copies queries and keys, one the values, one
 // issues the products, eight warps do the softmax with two threads a row, whose halves merge exactly at the end.
 //
 //   tiles      first the 128-entry tiles of block means any row sees, then those of kept tokens, then the window's 128-key
@@ -10,10 +10,10 @@
 //              columns of S they come from
 //   the end    sink, division, the turn of the sum back by the query's position, the gate
 //
-// What bounds it: a block's chain of some six tiles (two products, the second twice, with the softmax's eight warps between them: a
-// third of the issue slots, two warps a scheduler) and its start and end, two blocks an SM one after the other: two portions
-// of 1,366 and 682 tokens, 16 / 8 heads of 128, window 512, blocks of 64: 83 us cold, where the mma.sync kernel (64 x 64 tiles)
-// takes 173.
+// What bounds it: a block's chain of some six tiles of 1.4 us (the softmax's eight warps, one behind the other's products), 3 us before the first and 6
+// behind the last (the division, turns and gates, whose code each block fetches anew), two blocks an SM one after the other: two portions
+// of 1,366 and 682 tokens, 16 / 8 heads of 128, window 512, blocks of 64: 44 us, where it took 81 with cosines and sines made here, masks compared
+// key by key and a lone lane issuing (mma.sync kernel, 64 x 64 tiles: 173).
 // Every wait is bounded and reports in error_word.
 #include "tcgen05.cuh"
 #include "window_attention.cuh"
@@ -40,6 +40,15 @@ __device__ __forceinline__ float wt_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// (the reciprocal by a Newton step from the approximate one, within 0.51 units in the last place: an IEEE division is half of the instructions
+// around it, which each block fetches anew; below -88 a gate is 6e-39 instead of less)
+__device__ __forceinline__ float wt_sigmoid(float x) {
+  const float d = 1.f + expf(fminf(-x, 88.f));
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return fmaf(y, fmaf(-d, y, 1.f), y);
 }
 
 __device__ __forceinline__ void wt_ld8(uint32_t taddr, uint32_t (&r)[8]) {
@@ -74,7 +83,7 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   unsigned char* smem_gen = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - base));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int entry = blockIdx.y, kvh = blockIdx.x, group = a.heads / a.kv_heads;
   const int row0 = a.q_start[entry];
   const int q_len = a.q_start[entry + 1] - row0;
@@ -169,65 +178,71 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kWtTile >> 3) << 17) | ((uint32_t)(kWtTile >> 4) << 24);
-      constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) /* B is MN-major */ | ((uint32_t)(D >> 3) << 17) |
-                                   ((uint32_t)(kWtTile >> 4) << 24);
-      bool ok = mbar_wait(q_full, 0);
-      if (!ok && a.error_word) atomicExch(a.error_word, 0x7C0082);
-      // O_half += P . V of tile j: of each half's 64 columns of S, the first 32 hold the high terms, the others the remainders
-      auto issue_pv = [&](int j) {
-        const int s = j % kWtStages;
-        if (!mbar_wait(v_full(s), (j / kWtStages) & 1)) {
-          if (a.error_word) atomicExch(a.error_word, 0x7C0089);
-          return;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kWtTile >> 3) << 17) | ((uint32_t)(kWtTile >> 4) << 24);
+    constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) /* B is MN-major */ | ((uint32_t)(D >> 3) << 17) |
+                                 ((uint32_t)(kWtTile >> 4) << 24);
+    const uint32_t leader = umma_leader();
+    auto note = [&](int code) {
+      if (a.error_word && leader) atomicExch(a.error_word, code);
+      return false;
+    };
+    bool ok = mbar_wait_warp(q_full, 0) || note(0x7C0082);
+    // O_half += P . V of tile j: of each half's 64 columns of S, the first 32 hold the high terms, the others the remainders
+    auto issue_pv = [&](int j) {
+      const int s = j % kWtStages;
+      if (!mbar_wait_warp(v_full(s), (j / kWtStages) & 1)) {
+        note(0x7C0089);
+        return;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t values = umma_low_mn128(v_s(s), kWtSub), p = tmem_s + (j & 1) * kWtTile;
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-          const int half = kk >> 3, term = (kk >> 2) & 1, k = kk & 3;
-          umma_f16_tmem_a(tmem_o + half * D, tmem_s + (j & 1) * kWtTile + half * 64 + term * 32 + k * 8,
-                          umma_desc_mn128(v_s(s) + (half * 64 + k * 16) * 128, kWtSub), idesc_o, (j | (kk & 7)) != 0);
-        }
+      for (int kk = 0; kk < 16; ++kk) {
+        const int half = kk >> 3, term = (kk >> 2) & 1, k = kk & 3;
+        umma_warp_tmem(leader, tmem_o + half * D, p + half * 64 + term * 32 + k * 8, values + (half * 64 + k * 16) * 8, idesc_o, (j | (kk & 7)) != 0);
+      }
+      if (leader) {
         umma_commit(v_empty(s));
         umma_commit(pv_done);
-      };
-      for (int it = 0; it < n_tiles && ok; ++it) {
-        const int s = it % kWtStages;
-        if (!mbar_wait(k_full(s), (it / kWtStages) & 1)) {
-          if (a.error_word) atomicExch(a.error_word, 0x7C0083);
-          ok = false;
+      }
+    };
+    const uint32_t queries = umma_low_k128(q_s);
+    for (int it = 0; it < n_tiles && ok; ++it) {
+      const int s = it % kWtStages;
+      if (!mbar_wait_warp(k_full(s), (it / kWtStages) & 1)) {
+        ok = note(0x7C0083);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t keys = umma_low_k128(k_s(s));
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        const uint32_t off = ((kk >> 2) * kWtSub + (kk & 3) * 32) >> 4;
+        umma_warp(leader, tmem_s + (it & 1) * kWtTile, queries + off, keys + off, idesc_s, kk != 0);
+      }
+      if (leader) {
+        umma_commit(k_empty(s));
+        umma_commit(s_full(it & 1));
+      }
+      if (it > 0) {
+        if (!mbar_wait_warp(p_full((it - 1) & 1), ((it - 1) >> 1) & 1)) {
+          ok = note(0x7C0084);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kWtSub + (kk & 3) * 32;
-          umma_f16_idesc(tmem_s + (it & 1) * kWtTile, umma_desc_k128(q_s + off), umma_desc_k128(k_s(s) + off), idesc_s, kk != 0);
-        }
-        umma_commit(k_empty(s));
-        umma_commit(s_full(it & 1));
-        if (it > 0) {
-          if (!mbar_wait(p_full((it - 1) & 1), ((it - 1) >> 1) & 1)) {
-            if (a.error_word) atomicExch(a.error_word, 0x7C0084);
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          issue_pv(it - 1);
-        }
+        issue_pv(it - 1);
       }
-      if (ok) {
-        const int last = n_tiles - 1;
-        if (mbar_wait(p_full(last & 1), (last >> 1) & 1)) {
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          issue_pv(last);
-        } else if (a.error_word) {
-          atomicExch(a.error_word, 0x7C0084);
-        }
-      }
-      umma_commit(o_final);
     }
+    if (ok) {
+      const int last = n_tiles - 1;
+      if (mbar_wait_warp(p_full(last & 1), (last >> 1) & 1)) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        issue_pv(last);
+      } else {
+        note(0x7C0084);
+      }
+    }
+    if (leader) umma_commit(o_final);
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;
@@ -258,7 +273,7 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           tmem_ld32(mine + 32, s_hi32);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
         }
-        // what this row sees of the tile: indices from .. from + span - 1 (and the kept tokens)
+        // what this row sees of the tile, a bit a key: indices from .. from + span - 1, and the kept tokens up to its own
         const int from = pooled ? 0 : lo, span = pooled ? seen : qpos - lo + 1;
         float mx = -CUDART_INF_F;
         if (__all_sync(0xffffffffu, key_base >= from && key_base + HC <= from + span)) {
@@ -269,12 +284,15 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             mx = fmaxf(mx, v);
           }
         } else {
-          const int keep = pooled ? 0 : a.keep;
+          auto bits = [&](int first, int end) -> unsigned long long {      // of indices first .. end - 1
+            const int b0 = min(max(first - key_base, 0), HC), b1 = min(max(end - key_base, 0), HC);
+            return b1 > b0 ? (~0ull >> (64 - (b1 - b0))) << b0 : 0ull;
+          };
+          const unsigned long long allowed = bits(from, from + span) | (pooled ? 0ull : bits(0, min(a.keep, qpos + 1)));
+          const uint32_t allow[2] = {(uint32_t)allowed, (uint32_t)(allowed >> 32)};
 #pragma unroll
           for (int j = 0; j < HC; ++j) {
-            const int idx = key_base + j;
-            const bool allowed = (unsigned)(idx - from) < (unsigned)span || (idx < keep && idx <= qpos);
-            const float v = allowed ? __uint_as_float(sv[j]) * factor : -CUDART_INF_F;
+            const float v = allow[j >> 5] & (1u << (j & 31)) ? __uint_as_float(sv[j]) * factor : -CUDART_INF_F;
             sv[j] = __float_as_uint(v);
             mx = fmaxf(mx, v);
           }
@@ -338,6 +356,26 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       mbar_arrive(p_full(it & 1));
     }
+    // A thread's columns: a quarter of the row's first half and the same quarter of its second, so that the pairs a value's turn goes over
+    // lie in one thread; eight of each at a time, the next ones' gates and turns on their way (the first while the last products run).
+    // The turns come from the table that the append made of them: cosines and sines worked out here took 18 us of a block's 39.  The loop
+    // is not unrolled: its code runs four times a block, and four copies of it, fetched once each, take 16 us where it takes 5.
+    constexpr int W = D / 4;
+    const bool store = r < nrows;
+    const size_t token = (size_t)(row0 + t0 + t);
+    const __nv_bfloat16* gates = a.gate ? reinterpret_cast<const __nv_bfloat16*>(a.gate) + token * a.ld_gate + head * D + half * W : nullptr;
+    const float4* turns = a.turns ? reinterpret_cast<const float4*>(a.turns + token * D) + half * (W / 2) : nullptr;      // (two pairs each)
+    uint4 gate[2];
+    float4 turn[4];
+    auto ask = [&](int c) {
+#pragma unroll
+      for (int part = 0; part < 2; ++part)
+        if (gates) gate[part] = *reinterpret_cast<const uint4*>(gates + part * (D / 2) + c * 8);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (turns) turn[j] = turns[4 * c + j];
+    };
+    ask(0);
     if (ok && !mbar_wait(o_final, 0)) {
       if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0086);
       ok = false;
@@ -353,21 +391,18 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const float w_mine = exp2f(m - mm), w_other = exp2f(other.x - mm);
       const float inv = 1.f / (l * w_mine + other.y * w_other + (a.sink ? exp2f(sink2 - mm) : 0.f));
       const float w0 = (half == 0 ? w_mine : w_other) * inv, w1 = (half == 0 ? w_other : w_mine) * inv;
-      const bool store = r < nrows;
-      const size_t token = (size_t)(row0 + t0 + t);
-      __nv_bfloat16* dst = out + token * a.heads * D + (size_t)head * D;
-      const __nv_bfloat16* gates = a.gate ? reinterpret_cast<const __nv_bfloat16*>(a.gate) + token * a.ld_gate + head * D : nullptr;
-      // a thread's columns: a quarter of the row's first half and the same quarter of its second, so that the pairs a value's
-      // turn goes over lie in one thread; eight of each at a time, in a loop that is not unrolled (thirty-two copies of sine and
-      // cosine would be fetched once each: the kernel took 103 us with them)
-      constexpr int W = D / 4;
+      __nv_bfloat16* dst = out + token * a.heads * D + (size_t)head * D + half * W;
 #pragma unroll 1
-      for (int c0 = half * W; c0 < half * W + W; c0 += 8) {
+      for (int c = 0; c < W / 8; ++c) {
+        const uint4 g0 = gate[0], g1 = gate[1];
+        const float4 turn_now[4] = {turn[0], turn[1], turn[2], turn[3]};
+        if (c + 1 < W / 8) ask(c + 1);
         uint32_t u0[8], u1[8], v0[8], v1[8];
-        wt_ld8(tmem_o + lane_sel + c0, u0);
-        wt_ld8(tmem_o + D + lane_sel + c0, u1);
-        wt_ld8(tmem_o + lane_sel + D / 2 + c0, v0);
-        wt_ld8(tmem_o + D + lane_sel + D / 2 + c0, v1);
+        const uint32_t at = tmem_o + lane_sel + half * W + c * 8;
+        wt_ld8(at, u0);
+        wt_ld8(at + D, u1);
+        wt_ld8(at + D / 2, v0);
+        wt_ld8(at + D + D / 2, v1);
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
         float w[2][8];
 #pragma unroll
@@ -375,37 +410,41 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           w[0][j] = __uint_as_float(u0[j]) * w0 + __uint_as_float(u1[j]) * w1;
           w[1][j] = __uint_as_float(v0[j]) * w0 + __uint_as_float(v1[j]) * w1;
         }
-        if (a.vfreq) {
-          // turned back by the query's position: (u, v) -> (u cos + v sin, v cos - u sin)
+        // turned back by the query's position: (u, v) -> (u cos + v sin, v cos - u sin)
+        auto turn_back = [&](int j, float cs, float sn) {
+          const float x = rope_lo(w[0][j], w[1][j], cs, -sn), y = rope_hi(w[0][j], w[1][j], cs, -sn);
+          w[0][j] = x;
+          w[1][j] = y;
+        };
+        if (turns) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            turn_back(2 * j, turn_now[j].x, turn_now[j].y);
+            turn_back(2 * j + 1, turn_now[j].z, turn_now[j].w);
+          }
+        } else if (a.vfreq) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float angle = (float)qpos * a.vfreq[c0 + j];
-            const float cs = cosf(angle), sn = sinf(angle);
-            const float x = rope_lo(w[0][j], w[1][j], cs, -sn), y = rope_hi(w[0][j], w[1][j], cs, -sn);
-            w[0][j] = x;
-            w[1][j] = y;
+            const float angle = (float)qpos * a.vfreq[half * W + c * 8 + j];
+            turn_back(j, cosf(angle), sinf(angle));
           }
         }
-        if (store) {
 #pragma unroll
-          for (int part = 0; part < 2; ++part) {
-            const int col = part * (D / 2) + c0;
-            if (gates) {
-              const uint4 raw = *reinterpret_cast<const uint4*>(gates + col);
-              const uint32_t g[4] = {raw.x, raw.y, raw.z, raw.w};
+        for (int part = 0; part < 2; ++part) {
+          if (gates) {
+            const uint32_t g[4] = {part ? g1.x : g0.x, part ? g1.y : g0.y, part ? g1.z : g0.z, part ? g1.w : g0.w};
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&g[j]));
-                w[part][2 * j] *= 1.f / (1.f + expf(-f.x));
-                w[part][2 * j + 1] *= 1.f / (1.f + expf(-f.y));
-              }
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&g[j]));
+              w[part][2 * j] *= wt_sigmoid(f.x);
+              w[part][2 * j + 1] *= wt_sigmoid(f.y);
             }
-            uint4 packed;
-            __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&packed);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) p2[j] = __floats2bfloat162_rn(w[part][2 * j], w[part][2 * j + 1]);
-            *reinterpret_cast<uint4*>(dst + col) = packed;
           }
+          uint4 packed;
+          __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) p2[j] = __floats2bfloat162_rn(w[part][2 * j], w[part][2 * j + 1]);
+          if (store) *reinterpret_cast<uint4*>(dst + part * (D / 2) + c * 8) = packed;
         }
       }
     }

@@ -1537,10 +1537,11 @@ def rotary_kv_append(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_o
                      values: torch.Tensor, positions: torch.Tensor, token_slot: torch.Tensor, block_table: torch.Tensor,
                      freq: torch.Tensor, value_freq: torch.Tensor | None, heads: int, kv_heads: int, dim: int, vdim: int, *,
                      rot_dim: int, amplitude: float = 1.0, q_bias: torch.Tensor | None = None, k_bias: torch.Tensor | None = None,
-                     v_bias: torch.Tensor | None = None, error_word: torch.Tensor | None = None) -> torch.Tensor:
+                     v_bias: torch.Tensor | None = None, error_word: torch.Tensor | None = None,
+                     turns: torch.Tensor | None = None) -> torch.Tensor:
     """Add the biases, rotate the first ``rot_dim`` elements of every q and k head of the fused projection ``proj`` (pairs i,
     i + rot_dim / 2, cos and sin times ``amplitude``), turn every v head over its whole width by ``value_freq`` (None: not),
-    write q to ``q_out`` and k, v into their pages."""
+    write q to ``q_out`` and k, v into their pages.  ``turns`` [tokens, vdim / 2, 2] (fp32) takes the cosines and sines of ``value_freq``."""
     _rows_of(proj, "proj"), _need(q_out, "q_out", proj.dtype), _need(positions, "positions", torch.int32)
     _need(token_slot, "token_slot", torch.int32), _need(block_table, "block_table", torch.int32), _need(freq, "freq", torch.float32)
     n = proj.shape[0]
@@ -1551,12 +1552,16 @@ def rotary_kv_append(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_o
             raise KernelError("rotary_kv_append: a bias does not fit")
     if value_freq is not None and (value_freq.dtype != torch.float32 or value_freq.numel() * 2 != vdim):
         raise KernelError("rotary_kv_append: value_freq does not fit")
+    if turns is not None:
+        _need(turns, "turns", torch.float32)
+        if value_freq is None or turns.numel() != n * vdim:
+            raise KernelError("rotary_kv_append: turns do not fit")
     num_pages, page_size, page_stride = _pages(keys, values, kv_heads, dim, vdim, "rotary_kv_append")
     _check("rotary_kv_append", lib().tib_rotary_kv_append(
         _ptr(proj), c_int64(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off), _ptr(q_bias), _ptr(k_bias), _ptr(v_bias),
         _ptr(q_out), _ptr(keys), _ptr(values), _ptr(positions), _ptr(token_slot), _ptr(block_table), c_int(block_table.stride(0)),
         _ptr(freq), _ptr(value_freq), c_float(amplitude), c_int(n), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim),
-        c_int(rot_dim), c_int(page_size), c_int64(page_stride), c_int(num_pages), _ptr(error_word), c_int(_code(proj.dtype)), _stream()))
+        c_int(rot_dim), c_int(page_size), c_int64(page_stride), c_int(num_pages), _ptr(turns), _ptr(error_word), c_int(_code(proj.dtype)), _stream()))
     return q_out
 
 
@@ -1584,6 +1589,11 @@ def _window_few_rows() -> int:
     return int(lib().tib_pooled_window_attention_few_rows())
 
 
+def pooled_window_uses_turns(dtype: torch.dtype, max_q_len: int, heads: int, kv_heads: int, dim: int, vdim: int) -> bool:
+    """Whether the windowed attention has portions for the kernel that reads the values' cosines and sines from a table."""
+    return dtype == torch.bfloat16 and dim == vdim and dim in (64, 128) and max_q_len * (heads // kv_heads) > _window_few_rows()
+
+
 def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor, kv_start: torch.Tensor, slots: torch.Tensor,
                             keys: torch.Tensor, values: torch.Tensor, block_table: torch.Tensor, block_keys: torch.Tensor | None,
                             block_values: torch.Tensor | None, block_block_table: torch.Tensor | None, n_entries: int,
@@ -1592,7 +1602,7 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
                             value_freq: torch.Tensor | None = None, gate: torch.Tensor | None = None,
                             error_word: torch.Tensor | None = None, force_simt: bool = False,
                             rel_bias: torch.Tensor | None = None, max_kv_len: int = 0, splits: int | None = None,
-                            portions: Mapping[int, int] | None = None) -> torch.Tensor:
+                            portions: Mapping[int, int] | None = None, turns: torch.Tensor | None = None) -> torch.Tensor:
     """Per head, out[i] = sigmoid(gate[i]) * turn_back_i(sum_j w_ij v_j + sum_b w_ib V_b): softmax weights over the tokens j
     with 0 <= i - j < window and the blocks b of ``pool`` positions with b * pool + pool - 1 <= i - window (their means K_b,
     V_b from the strided pages), scores q . k * scale * temp[h], exp(sink[h]) added to the denominator; turn_back undoes at
@@ -1603,7 +1613,8 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
     names the longest context (``max_kv_len``) shares every context's visible keys out over ``splits`` blocks (None: enough
     to fill the GPU) whose sums a second small kernel adds in a fixed order.
     bfloat16 steps run on the tensor cores when the head sizes are multiples of 8 up to 128, unless ``force_simt``; long portions
-    and short ones then by kernels of their own.  ``portions`` (length: how many entries have it) spares a launch over nothing."""
+    and short ones then by kernels of their own.  ``portions`` (length: how many entries have it) spares a launch over nothing.
+    ``turns``: the cosines and sines of ``value_freq`` at the step's tokens, as :func:`rotary_kv_append` leaves them (None: worked out again)."""
     _need(q, "q"), _need(out, "out", q.dtype)
     dim, vdim = keys.shape[3], values.shape[3]
     n = q.shape[0]
@@ -1621,6 +1632,10 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
             raise KernelError(f"pooled_window_attention: {name} does not fit")
     if value_freq is not None and (value_freq.dtype != torch.float32 or value_freq.numel() * 2 != vdim):
         raise KernelError("pooled_window_attention: value_freq does not fit")
+    if turns is not None:
+        _need(turns, "turns", torch.float32)
+        if turns.numel() != n * vdim:
+            raise KernelError("pooled_window_attention: turns do not fit")
     ld_gate = 0
     if gate is not None:
         _rows_of(gate, "gate", heads * vdim)
@@ -1651,7 +1666,7 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
         _ptr(block_keys if pool > 0 else None), _ptr(block_values if pool > 0 else None),
         _ptr(block_block_table if pool > 0 else None), c_int(b_table_stride), c_int(b_page_size), c_int64(b_stride), c_int(b_pages),
         c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim), c_int(window), c_int(keep), c_int(pool),
-        c_float(scale), _ptr(temp), _ptr(sink), _ptr(value_freq), _ptr(gate), c_int(_code(gate.dtype) if gate is not None else 0),
+        c_float(scale), _ptr(temp), _ptr(sink), _ptr(value_freq), _ptr(turns), _ptr(gate), c_int(_code(gate.dtype) if gate is not None else 0),
         c_int64(ld_gate), _ptr(rel_bias), c_int(rel_bias.shape[1] if rel_bias is not None else 0), _ptr(partial),
         c_int(n_splits), c_int(n), c_int(few_rows), ctypes.byref(launches), _ptr(error_word), c_int(_code(q.dtype)), c_int(int(force_simt)),
         _stream()))

@@ -120,10 +120,13 @@ class PooledWindowAttention(Mixer):
         freq, rot_dim, interleaved = self.position.rotary_table()
         if interleaved:
             raise RuntimeError("this attention's kernels pair element i with i + rot_dim / 2")
+        turns = None
+        if self.value_freq is not None and ops.pooled_window_uses_turns(x.dtype, batch.max_q_len, h, g, self.dim, self.value_dim):
+            turns = torch.empty((n, self.value_dim // 2, 2), dtype=torch.float32, device=x.device)
         ops.rotary_kv_append(proj, 0, self.k_off, self.v_off, q, kv.keys, kv.values, batch.positions, batch.token_slot,
                              kv.block_table, freq, self.value_freq, h, g, self.dim, self.value_dim, rot_dim=rot_dim,
                              amplitude=getattr(self.position, "amplitude", 1.0), q_bias=self.q_bias, k_bias=self.k_bias,
-                             v_bias=self.v_bias, error_word=ctx.error_word)
+                             v_bias=self.v_bias, error_word=ctx.error_word, turns=turns)
         if self.pool:
             ops.pool_blocks(kv.keys, kv.values, kv.block_table, side.keys, side.values, side.block_table, batch.positions,
                             batch.token_slot, self.pool, error_word=ctx.error_word)
@@ -134,7 +137,7 @@ class PooledWindowAttention(Mixer):
             batch.n_entries, batch.max_q_len, h, g, window=self.window, pool=self.pool, scale=self.scale, temp=self.temp,
             sink=self.sink, value_freq=self.value_freq,
             gate=proj[:, self.g_off:self.g_off + h * self.value_dim] if self.has_gate else None, error_word=ctx.error_word,
-            portions=batch.portions)
+            portions=batch.portions, turns=turns)
         return linear(out, self.o_weight)
 
 
