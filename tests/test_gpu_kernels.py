@@ -487,6 +487,32 @@ def test_paged_attention_ragged_batch(dtype, heads, kv_heads, d, page):
     assert torch.allclose(out.double(), ref, **(dict(atol=3e-6, rtol=1e-5) if dtype == torch.float32 else dict(atol=2e-2, rtol=2e-2)))
 
 
+# (a portion in four rows a warp, single tokens in one row and, of groups above four, in four; heads of one, two, three and eight columns a lane)
+@pytest.mark.parametrize("heads, kv_heads, d", [(4, 4, 32), (8, 2, 64), (10, 2, 72), (6, 1, 256)])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("window", [0, 40])
+def test_paged_attention_by_four_numbers_has_the_bits_of_single_ones(heads, kv_heads, d, dtype, window):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    i32 = lambda xs: dev(torch.tensor(xs, dtype=torch.int32))
+    page, pages, contexts = 8, 40, [33, 64, 100]
+    pool, table = dev(rnd(pages, 2, kv_heads, page, d, dtype=dtype)), i32(list(range(39))).view(3, 13)
+    q = rnd(sum(contexts), heads * d, dtype=dtype, seed=3)
+
+    def run(rows, starts, past, longest, shift):
+        moved = torch.empty(rows.numel() + shift, dtype=dtype, device="cuda")[shift:].view(rows.shape)      # (rows off their boundaries: one number at a time)
+        moved.copy_(rows)
+        return ops.paged_attention_simt(moved, pool, torch.empty(rows.shape, dtype=dtype, device="cuda"), i32(starts), i32(past), i32([0, 1, 2]), table, 3, longest,
+                                        heads, kv_heads, d, d ** -0.5, window=window)
+
+    starts = [0] + [sum(contexts[:i + 1]) for i in range(3)]
+    whole = run(dev(q), starts, [0, 0, 0], max(contexts), 0)
+    assert torch.equal(whole, run(dev(q), starts, [0, 0, 0], max(contexts), 1))
+    last = torch.tensor([e - 1 for e in starts[1:]])
+    for shift in (0, 1):      # the last token of each alone: the bits it has in its portion
+        assert torch.equal(run(dev(q[last]), [0, 1, 2, 3], [c - 1 for c in contexts], 1, shift), whole[last.cuda()])
+
+
 @pytest.mark.parametrize("window", [1, 5, 32, 33, 100])
 def test_paged_attention_window_edges(window):
     need_gpu()
