@@ -274,8 +274,8 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             const int c0 = (2 * (e >> 1) + half) * 16 + (e & 1) * 8;
             if (c0 >= a.rows) break;
             uint32_t m[8], n[8];
-            ft_tmem_ld8(at + 2 * kFtRows + c0, m);
-            ft_tmem_ld8(at + 2 * kFtRows + a.rows + c0, n);
+            tmem_ld8(at + 2 * kFtRows + c0, m);
+            tmem_ld8(at + 2 * kFtRows + a.rows + c0, n);
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
             for (int c = 0; c < 8; ++c) sum[e >> 1][(e & 1) * 8 + c] += __uint_as_float(m[c]) + __uint_as_float(n[c]);

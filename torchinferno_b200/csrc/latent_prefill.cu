@@ -123,7 +123,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   unsigned char* smem_gen = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - base));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int own = blockIdx.x, head = a.head0 + own, entry = blockIdx.y;      // own: among the heads that kv holds
   // (the first block may be placed while the kernel before drains: the entries' arrays were uploaded before the step began,
   // what the step's kernels write is only touched behind pdl_wait below)
@@ -193,65 +193,71 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kLpTile >> 3) << 17) | ((uint32_t)(kLpTile >> 4) << 24);
-      constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) /* B is MN-major */ | ((uint32_t)(D >> 3) << 17) |
-                                   ((uint32_t)(kLpTile >> 4) << 24);
-      bool ok = mbar_wait(q_full, 0);
-      if (!ok && a.error_word) atomicExch(a.error_word, 0x7C0072);
-      // O_half += P . V of tile j: of each half's 64 columns of S, the first 32 hold the high terms, the others the remainders
-      auto issue_pv = [&](int j) {
-        const int s = j % kLpStages;
-        if (!mbar_wait(v_full(s), (j / kLpStages) & 1)) {
-          if (a.error_word) atomicExch(a.error_word, 0x7C0079);
-          return;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kLpTile >> 3) << 17) | ((uint32_t)(kLpTile >> 4) << 24);
+    constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) /* B is MN-major */ | ((uint32_t)(D >> 3) << 17) |
+                                 ((uint32_t)(kLpTile >> 4) << 24);
+    const uint32_t leader = umma_leader();
+    auto note = [&](int code) {
+      if (a.error_word && leader) atomicExch(a.error_word, code);
+      return false;
+    };
+    bool ok = mbar_wait_warp(q_full, 0) || note(0x7C0072);
+    // O_half += P . V of tile j: of each half's 64 columns of S, the first 32 hold the high terms, the others the remainders
+    auto issue_pv = [&](int j) {
+      const int s = j % kLpStages;
+      if (!mbar_wait_warp(v_full(s), (j / kLpStages) & 1)) {
+        note(0x7C0079);
+        return;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t values = umma_low_mn128(v_s(s), kLpSub), p = tmem_s + (j & 1) * kLpTile;
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-          const int half = kk >> 3, term = (kk >> 2) & 1, k = kk & 3;
-          umma_f16_tmem_a(tmem_o + half * D, tmem_s + (j & 1) * kLpTile + half * 64 + term * 32 + k * 8,
-                          umma_desc_mn128(v_s(s) + (half * 64 + k * 16) * 128, kLpSub), idesc_o, (j | (kk & 7)) != 0);
-        }
+      for (int kk = 0; kk < 16; ++kk) {
+        const int half = kk >> 3, term = (kk >> 2) & 1, k = kk & 3;
+        umma_warp_tmem(leader, tmem_o + half * D, p + half * 64 + term * 32 + k * 8, values + (half * 64 + k * 16) * 8, idesc_o, (j | (kk & 7)) != 0);
+      }
+      if (leader) {
         umma_commit(v_empty(s));
         umma_commit(pv_done);
-      };
-      for (int it = 0; it < n_tiles && ok; ++it) {
-        const int s = it % kLpStages;
-        if (!mbar_wait(k_full(s), (it / kLpStages) & 1)) {
-          if (a.error_word) atomicExch(a.error_word, 0x7C0073);
-          ok = false;
+      }
+    };
+    const uint32_t queries = umma_low_k128(q_s);
+    for (int it = 0; it < n_tiles && ok; ++it) {
+      const int s = it % kLpStages;
+      if (!mbar_wait_warp(k_full(s), (it / kLpStages) & 1)) {
+        ok = note(0x7C0073);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t keys = umma_low_k128(k_s(s));
+#pragma unroll
+      for (int kk = 0; kk < (DQ + 1) * 4; ++kk) {
+        const uint32_t off = ((kk >> 2) * kLpSub + (kk & 3) * 32) >> 4;
+        umma_warp(leader, tmem_s + (it & 1) * kLpTile, queries + off, keys + off, idesc_s, kk != 0);
+      }
+      if (leader) {
+        umma_commit(k_empty(s));
+        umma_commit(s_full(it & 1));
+      }
+      if (it > 0) {
+        if (!mbar_wait_warp(p_full((it - 1) & 1), ((it - 1) >> 1) & 1)) {
+          ok = note(0x7C0074);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll
-        for (int kk = 0; kk < (DQ + 1) * 4; ++kk) {
-          const uint32_t off = (kk >> 2) * kLpSub + (kk & 3) * 32;
-          umma_f16_idesc(tmem_s + (it & 1) * kLpTile, umma_desc_k128(q_s + off), umma_desc_k128(k_s(s) + off), idesc_s, kk != 0);
-        }
-        umma_commit(k_empty(s));
-        umma_commit(s_full(it & 1));
-        if (it > 0) {
-          if (!mbar_wait(p_full((it - 1) & 1), ((it - 1) >> 1) & 1)) {
-            if (a.error_word) atomicExch(a.error_word, 0x7C0074);
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          issue_pv(it - 1);
-        }
+        issue_pv(it - 1);
       }
-      if (ok) {
-        const int last = n_tiles - 1;
-        if (mbar_wait(p_full(last & 1), (last >> 1) & 1)) {
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          issue_pv(last);
-        } else if (a.error_word) {
-          atomicExch(a.error_word, 0x7C0074);
-        }
-      }
-      umma_commit(o_final);
     }
+    if (ok) {
+      const int last = n_tiles - 1;
+      if (mbar_wait_warp(p_full(last & 1), (last >> 1) & 1)) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        issue_pv(last);
+      } else {
+        note(0x7C0074);
+      }
+    }
+    if (leader) umma_commit(o_final);
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;
@@ -340,6 +346,13 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       mbar_arrive(p_full(it & 1));
     }
+    // Eight columns of the row at a time, the next ones' gates on their way (the first while the last products run).  The loop is not
+    // unrolled: its code runs once a block and waits for its own fetch.
+    const bool store = r < nt;
+    const size_t row = (size_t)(row0 + t0 + (store ? r : 0));
+    const __nv_bfloat16* gates = a.gate && !a.gate_per_head ? a.gate + row * a.ld_gate + head * D + half * OC : nullptr;
+    uint4 gate = make_uint4(0u, 0u, 0u, 0u);
+    if (gates) gate = *reinterpret_cast<const uint4*>(gates);
     if (ok && !mbar_wait(o_final, 0)) {
       if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0076);
       ok = false;
@@ -356,40 +369,32 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const float w_mine = exp2f(m - mm), w_other = exp2f(other.x - mm);
       const float inv = 1.f / (l * w_mine + other.y * w_other + (a.sink ? exp2f(sink2 - mm) : 0.f));
       const float w0 = (half == 0 ? w_mine : w_other) * inv, w1 = (half == 0 ? w_other : w_mine) * inv;
-      const bool store = r < nt;
-      const size_t row = (size_t)(row0 + t0 + (store ? r : 0));
       __nv_bfloat16* dst = a.out + (row * a.heads + head) * D + half * OC;
-      const float head_gate = a.gate && a.gate_per_head ? 1.f / (1.f + expf(-__bfloat162float(a.gate[row * a.ld_gate + head]))) : 1.f;
-      const __nv_bfloat16* gates = a.gate && !a.gate_per_head ? a.gate + row * a.ld_gate + head * D + half * OC : nullptr;
-#pragma unroll
-      for (int c = 0; c < OC / 32; ++c) {
-        uint32_t v0[32], v1[32];
-        tmem_ld32(tmem_o + lane_sel + half * OC + c * 32, v0);          // O_0
-        tmem_ld32(tmem_o + D + lane_sel + half * OC + c * 32, v1);      // O_1
+      const float head_gate = a.gate && a.gate_per_head ? sigmoid_newton(__bfloat162float(a.gate[row * a.ld_gate + head])) : 1.f;
+#pragma unroll 1
+      for (int c = 0; c < OC; c += 8) {
+        const uint32_t g[4] = {gate.x, gate.y, gate.z, gate.w};
+        if (gates && c + 8 < OC) gate = *reinterpret_cast<const uint4*>(gates + c + 8);
+        uint32_t v0[8], v1[8];
+        tmem_ld8(tmem_o + lane_sel + half * OC + c, v0);          // O_0
+        tmem_ld8(tmem_o + D + lane_sel + half * OC + c, v1);      // O_1
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (store) {
+        float o[8];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            float o[8];
+        for (int j = 0; j < 8; ++j) o[j] = (__uint_as_float(v0[j]) * w0 + __uint_as_float(v1[j]) * w1) * head_gate;
+        if (gates) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = (__uint_as_float(v0[q * 8 + j]) * w0 + __uint_as_float(v1[q * 8 + j]) * w1) * head_gate;
-            if (gates) {
-              const uint4 raw = *reinterpret_cast<const uint4*>(gates + c * 32 + q * 8);
-              const uint32_t g[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&g[j]));
-                o[2 * j] *= 1.f / (1.f + expf(-f.x));
-                o[2 * j + 1] *= 1.f / (1.f + expf(-f.y));
-              }
-            }
-            uint4 packed;
-            __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&packed);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) p2[j] = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
-            *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = packed;
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&g[j]));
+            o[2 * j] *= sigmoid_newton(f.x);
+            o[2 * j + 1] *= sigmoid_newton(f.y);
           }
         }
+        uint4 packed;
+        __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p2[j] = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
+        if (store) *reinterpret_cast<uint4*>(dst + c) = packed;
       }
     }
   }

@@ -411,9 +411,9 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
 #pragma unroll
       for (int e = 0; e < 16; e += 8) {
         uint32_t v[5][8];
-        ft_tmem_ld8(small + lanes + part * 16 + e, v[0]);
+        tmem_ld8(small + lanes + part * 16 + e, v[0]);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) ft_tmem_ld8(wide + q * 64 + lanes + part * 16 + e, v[q + 1]);
+        for (int q = 0; q < 4; ++q) tmem_ld8(wide + q * 64 + lanes + part * 16 + e, v[q + 1]);
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
         for (int c = 0; c < 8; c += 2) {

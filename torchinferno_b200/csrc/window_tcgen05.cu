@@ -42,21 +42,6 @@ __device__ __forceinline__ float wt_exp2(float x) {
   return y;
 }
 
-// (the reciprocal by a Newton step from the approximate one, within 0.51 units in the last place: an IEEE division is half of the instructions
-// around it, which each block fetches anew; below -88 a gate is 6e-39 instead of less)
-__device__ __forceinline__ float wt_sigmoid(float x) {
-  const float d = 1.f + expf(fminf(-x, 88.f));
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-  return fmaf(y, fmaf(-d, y, 1.f), y);
-}
-
-__device__ __forceinline__ void wt_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-
 template <int D>
 __global__ void __launch_bounds__(kWtThreads, 1)
 window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -399,10 +384,10 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (c + 1 < W / 8) ask(c + 1);
         uint32_t u0[8], u1[8], v0[8], v1[8];
         const uint32_t at = tmem_o + lane_sel + half * W + c * 8;
-        wt_ld8(at, u0);
-        wt_ld8(at + D, u1);
-        wt_ld8(at + D / 2, v0);
-        wt_ld8(at + D + D / 2, v1);
+        tmem_ld8(at, u0);
+        tmem_ld8(at + D, u1);
+        tmem_ld8(at + D / 2, v0);
+        tmem_ld8(at + D + D / 2, v1);
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
         float w[2][8];
 #pragma unroll
@@ -436,8 +421,8 @@ window_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float2 f = bf16x2_floats(*reinterpret_cast<const __nv_bfloat162*>(&g[j]));
-              w[part][2 * j] *= wt_sigmoid(f.x);
-              w[part][2 * j + 1] *= wt_sigmoid(f.y);
+              w[part][2 * j] *= sigmoid_newton(f.x);
+              w[part][2 * j + 1] *= sigmoid_newton(f.y);
             }
           }
           uint4 packed;
