@@ -13,7 +13,8 @@
 // Warp 0 is the TMA producer of Q (one 3-D tile copy; dims: head_dim, head, token) and of K, the last
 // warp that of V, page by page through a 2-D view of the layer's pages ([page rows, head_dim]), each
 // into a ring of its own; pages past the block's last query are fetched from an out-of-range
-// coordinate, which fills zeros.  Warp 1 (one lane) issues the MMAs.  Every mbarrier wait is bounded; on a timeout a code goes to `error_word`
+// coordinate, which fills zeros.  Warp 1 issues the MMAs (the whole warp walks the loop, one lane issues: three portions of 2,048 tokens behind
+// 512, 32 / 8 heads of 128, take 59 us and took 61).  Every mbarrier wait is bounded; on a timeout a code goes to `error_word`
 // and all roles fall through to the common exit.
 //
 // Formula as in attention_mma.cu / attention_simt.cu (src/torchinferno/models/llama3/raw_ops.py:44-51).
@@ -81,7 +82,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   unsigned char* smem_gen = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - base));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int entry = blockIdx.y, kvh = blockIdx.x;
   const int row0 = a.q_start[entry];
   const int q_len = a.q_start[entry + 1] - row0;
@@ -178,71 +179,75 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFaBN >> 3) << 17) | ((uint32_t)(kFaBM >> 4) << 24);
-      constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) /* B is MN-major */ |
-                                   ((uint32_t)(D >> 3) << 17) | ((uint32_t)(kFaBM >> 4) << 24);
-      bool ok = mbar_wait(q_full, 0);
-      if (!ok && a.error_word) atomicExch(a.error_word, 0x7C0022);
-      // O += P . V of tile `j` (its V in stage j % stages, its P in buffer j & 1)
-      auto issue_pv = [&](int j) {
-        const int s = j % kFaStages;
-        if (!mbar_wait(v_full(s), (j / kFaStages) & 1)) {
-          if (a.error_word) atomicExch(a.error_word, 0x7C0029);
-          return;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFaBN >> 3) << 17) | ((uint32_t)(kFaBM >> 4) << 24);
+    constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) /* B is MN-major */ |
+                                 ((uint32_t)(D >> 3) << 17) | ((uint32_t)(kFaBM >> 4) << 24);
+    const uint32_t leader = umma_leader();
+    auto note = [&](int code) {
+      if (a.error_word && leader) atomicExch(a.error_word, code);
+      return false;
+    };
+    bool ok = mbar_wait_warp(q_full, 0) || note(0x7C0022);
+    // O += P . V of tile `j` (its V in stage j % stages, its P in buffer j & 1)
+    auto issue_pv = [&](int j) {
+      const int s = j % kFaStages;
+      if (!mbar_wait_warp(v_full(s), (j / kFaStages) & 1)) {
+        note(0x7C0029);
+        return;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t values = umma_low_mn128(v_s(s), kSub), p = tmem_s + (j & 1) * kFaBN;
 #pragma unroll
-        for (int kk = 0; kk < kFaBN / 16; ++kk) {
-          // keys 0..63 of the tile go to O_0, keys 64..127 to O_1 (the two halves of a row keep apart); P is
-          // read from tensor memory, where each half left it in the first 32 columns of its part of S
-          umma_f16_tmem_a(tmem_o + (kk >> 2) * D, tmem_s + (j & 1) * kFaBN + (kk >> 2) * (kFaBN / 2) + (kk & 3) * 8,
-                          umma_desc_mn128(v_s(s) + kk * 16 * 128, kSub), idesc_o, (j | (kk & 3)) != 0);
-        }
+      for (int kk = 0; kk < kFaBN / 16; ++kk) {
+        // keys 0..63 of the tile go to O_0, keys 64..127 to O_1 (the two halves of a row keep apart); P is
+        // read from tensor memory, where each half left it in the first 32 columns of its part of S
+        umma_warp_tmem(leader, tmem_o + (kk >> 2) * D, p + (kk >> 2) * (kFaBN / 2) + (kk & 3) * 8, values + kk * 128, idesc_o, (j | (kk & 3)) != 0);
+      }
+      if (leader) {
         umma_commit(v_empty(s));    // the value stage goes back to the producer
         umma_commit(pv_done);       // O is at rest again
-      };
-      for (int it = 0; it < n_tiles && ok; ++it) {
-        const int s = it % kFaStages;
-        const uint32_t phase = (it / kFaStages) & 1;
-        if (!mbar_wait(k_full(s), phase)) {
-          if (a.error_word) atomicExch(a.error_word, 0x7C0023);
-          ok = false;
+      }
+    };
+    const uint32_t queries = umma_low_k128(q_s);
+    for (int it = 0; it < n_tiles && ok; ++it) {
+      const int s = it % kFaStages;
+      if (!mbar_wait_warp(k_full(s), (it / kFaStages) & 1)) {
+        ok = note(0x7C0023);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      // S = Q . K^T over head_dim in steps of 16, into S buffer it & 1: it runs while the softmax warps
+      // are still busy with the tile before
+      const uint32_t keys = umma_low_k128(k_s(s));
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        const uint32_t off = ((kk >> 2) * kSub + (kk & 3) * 32) >> 4;
+        umma_warp(leader, tmem_s + (it & 1) * kFaBN, queries + off, keys + off, idesc_s, kk != 0);
+      }
+      if (leader) {
+        umma_commit(k_empty(s));    // the key stage goes back to the producer
+        umma_commit(s_full(it & 1));
+      }
+      if (it > 0) {
+        // P of the tile before (and the rescaled O) are ready: O += P . V
+        if (!mbar_wait_warp(p_full((it - 1) & 1), ((it - 1) >> 1) & 1)) {
+          ok = note(0x7C0024);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        // S = Q . K^T over head_dim in steps of 16, into S buffer it & 1: it runs while the softmax warps
-        // are still busy with the tile before
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t sub = (kk >> 2) * kSub, inner = (kk & 3) * 32;
-          umma_f16_idesc(tmem_s + (it & 1) * kFaBN, umma_desc_k128(q_s + sub + inner), umma_desc_k128(k_s(s) + sub + inner),
-                         idesc_s, kk != 0);
-        }
-        umma_commit(k_empty(s));    // the key stage goes back to the producer
-        umma_commit(s_full(it & 1));
-        if (it > 0) {
-          // P of the tile before (and the rescaled O) are ready: O += P . V
-          if (!mbar_wait(p_full((it - 1) & 1), ((it - 1) >> 1) & 1)) {
-            if (a.error_word) atomicExch(a.error_word, 0x7C0024);
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          issue_pv(it - 1);
-        }
+        issue_pv(it - 1);
       }
-      if (ok) {
-        const int last = n_tiles - 1;
-        if (mbar_wait(p_full(last & 1), (last >> 1) & 1)) {
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          issue_pv(last);
-        } else if (a.error_word) {
-          atomicExch(a.error_word, 0x7C0024);
-        }
-      }
-      umma_commit(o_final);
     }
+    if (ok) {
+      const int last = n_tiles - 1;
+      if (mbar_wait_warp(p_full(last & 1), (last >> 1) & 1)) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        issue_pv(last);
+      } else {
+        note(0x7C0024);
+      }
+    }
+    if (leader) umma_commit(o_final);
   } else {
     // softmax and epilogue: two threads per row.  `half` 0 takes keys 0..63 of every tile, half 1 keys
     // 64..127, each with a running maximum, a sum and an output accumulator (O_half in TMEM) of its own, as
