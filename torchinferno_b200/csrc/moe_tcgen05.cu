@@ -6,19 +6,23 @@
 // output (TMEM lane = feature, column = row).  An expert's rows are cut into equal tiles (170 rows are two tiles of 96 and
 // 74, not 160 and 10).  Which tiles there are is known on the device only: every block sums the experts' tiles once and walks
 // the tiles t = blockIdx.x, + gridDim.x, ...; feature tiles run fastest, so blocks that run together read the same rows of x.
-//   warp 0, one lane   TMA producer of the weights: 128 x 64 slices, 128-byte swizzle
-//   warp 1, one lane   issues tcgen05.mma (M 128, N = the tile's rows, K 16); owns the TMEM allocation
-//   warps 2..5         epilogue: tcgen05.ld, activation, stores; two accumulators alternate, so it runs under the next tile
-//   warps 6..9         producers of the rows where these are gathered (GATHER): cp.async, 16 bytes each, by source row straight
-//                      into the swizzled stage; a stage is announced two stages later, when its copies have landed.
-//                      Rows that lie sorted in memory are copied by warp 0 as well, in TMA boxes of 32 rows
+//   warp 0             TMA producer of the weights: 128 x 64 slices, 128-byte swizzle
+//   warp 1             issues tcgen05.mma (M 128, N = the tile's rows, K 16); owns the TMEM allocation
+//   the next 4 or 8    epilogue: tcgen05.ld, activation, stores; two accumulators alternate, so it runs under the next tile.  Eight
+//                      warps for tiles of 96 rows and more, four for each half of the columns
+//   the last 4 or 8    producers of the rows where these are gathered (GATHER): cp.async, 16 bytes each, by source row straight
+//                      into the swizzled stage; a stage is announced kLag stages later, when its copies have landed.
+//                      Rows that lie sorted in memory are copied by warp 0 as well, in TMA boxes of half a tile (32 rows in small ones)
+// Producer and issuer walk their loops as whole warps and one elected lane issues: a lone lane took 520 cycles to wait for a stage and
+// issue its four products (N 128 takes the tensor core 256), and 590 to issue a sorted stage's copies.
 // (Sorting the rows of the first product in a pass of its own, so that TMA could copy them too, gained 12 us in the product and
 // cost 12 in the pass.)
 //
 // What bounds it: a prompt reads every expert's weights once (134 MB a product at 32 experts of 1024 on rows of 2048: 21 us) and
-// multiplies at the rate shared memory feeds 128 x 128 x 16 products; 2,048 tokens x 4 choices take 68 us gathered and 62 sorted where
-// the mma.sync kernel before took 199 and 207 (cold).  A decode step streams the chosen experts' weights with 144 KB of them on their
-// way per SM (180 with the token rows): eight tokens x 4, gate and up of 1024 on 2048: 42 us for 176 MB (68 before), down 24 (38).
+// then brings 32 KB of weights and rows to an SM for every 128 x 128 x 64 product (256 cycles of the tensor core): 2,048 tokens x 4
+// choices, 2048 -> 1024, gathered: 57 us warm (69 with a lone lane's loops and the unrolled epilogue).  A decode step streams the chosen
+// experts' weights with 144 KB of them on their way per SM (180 with the token rows): eight tokens x 4, gate and up of 1024 on 2048:
+// 36 us for 176 MB (42 before), down 19 (24).
 // Every wait is bounded and reports in error_word, as in gemm_tcgen05.cu.
 #include "moe.cuh"
 #include "mma.cuh"
@@ -26,13 +30,17 @@
 
 namespace tib {
 
-constexpr int kMpM = 128, kMpK = 64, kMpThreads = 192, kMpGather = 128, kMpLag = 2, kMpBox = 32;
+constexpr int kMpM = 128, kMpK = 64;
 constexpr int kMpMaxExperts = 1024;
 constexpr uint32_t kMpWBytes = kMpM * kMpK * 2;
 template <int NT> struct MpShape {
   static constexpr uint32_t kXBytes = NT * kMpK * 2;
   static constexpr uint32_t kStage = kMpWBytes + kXBytes;
   static constexpr int kStages = 200 * 1024 / kStage < 9 ? 200 * 1024 / kStage : 9;
+  static constexpr int kLag = NT >= 96 ? 3 : 2;      // stages after which a gathered one is announced
+  static constexpr int kStorers = NT >= 96 ? 8 : 4, kThreads = 64 + 32 * kStorers;      // warps of the epilogue; threads without the gather's
+  static constexpr int kGather = NT >= 96 ? 256 : 128, kGatherRows = kGather / 8;       // threads of the gather, rows they copy at a time
+  static constexpr int kBox = NT >= 96 ? NT / 2 : 32;       // rows of one TMA copy of x
   static constexpr uint32_t kTmemCols = NT <= 32 ? 64 : NT <= 64 ? 128 : NT <= 128 ? 256 : 512;      // two accumulators of NT columns
   static constexpr uint32_t kSmem = 1024 + kStages * kStage + 256 + (kMpMaxExperts + 1) * 4;
 };
@@ -42,37 +50,48 @@ __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy
 
 struct MpTile { int expert, first, rows, feature; };
 
-// Stores columns c0 .. c0 + 31 (rows of the tile) of one warp's 32 features.
+// One warp's 32 features of the tile's columns c0 .. c1 - 1 (c0 a multiple of eight), from tensor memory through the activation to y.
+// A loop of eight columns: unrolled over 32, the code was fetched anew for every tile (3,000 cycles for 32 columns; rolled 1,250).
 template <int ACT, typename TO>
-__device__ __forceinline__ void mp_store(const uint32_t (&v)[32], TO* __restrict__ y, int64_t ldy, const MpTile& t, int c0, int feature, int N,
-                                         int lane, float scale_lane, const MoeEpilogue& ep) {
-  if constexpr (moe_act_gated(ACT)) {
-    // a lane pair holds (gate, up) of one output for every column: of two columns the even lane finishes the first, the odd
-    // lane the second
-    const bool odd = lane & 1;
-    const bool in = (feature | 1) < N;
+__device__ __forceinline__ void mp_store(uint32_t tmem, TO* __restrict__ y, int64_t ldy, const MpTile& t, int c0, int c1, int feature, int N, int lane,
+                                         const int* __restrict__ order, const MoeEpilogue& ep) {
+  constexpr bool kGated = moe_act_gated(ACT);
+  // (gated: a lane pair holds (gate, up) of one output for every column; of two columns the even lane finishes the first, the odd lane
+  // the second)
+  const bool odd = lane & 1;
+  const bool in = kGated ? (feature | 1) < N : feature < N;
+  TO* dst = y + (size_t)(t.first + c0 + (kGated && odd)) * ldy + (kGated ? feature >> 1 : feature);
+  float scale = 1.f;
+#pragma unroll 1
+  for (int c = c0; c < c1; c += 8) {
+    if (ep.row_scale && ((c - c0) & 31) == 0) scale = c + lane < c1 ? ep.row_scale[order[t.first + c + lane]] : 1.f;
+    uint32_t raw[8];
+    tmem_ld8(tmem + c, raw);
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+    float v[8];
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-      const float send = __uint_as_float(odd ? v[j] : v[j + 1]);
-      const float got = __shfl_xor_sync(0xffffffffu, send, 1);
-      const float rs = __shfl_sync(0xffffffffu, scale_lane, j + (odd ? 1 : 0));
-      const float g = odd ? got : __uint_as_float(v[j]), u = odd ? __uint_as_float(v[j + 1]) : got;
-      const int col = c0 + j + (odd ? 1 : 0);
-      if (in && col < t.rows)
-        y[(size_t)(t.first + col) * ldy + (feature >> 1)] = from_f32<TO>(moe_gated(g * rs, u * rs, ACT, ep.limit, ep.alpha));
+    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(raw[j]);
+    if (ep.row_scale) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] *= __shfl_sync(0xffffffffu, scale, ((c - c0) & 31) + j);
     }
-  } else {
-    const bool in = feature < N;
+    if constexpr (kGated) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float rs = __shfl_sync(0xffffffffu, scale_lane, j);
-      if (in && c0 + j < t.rows) y[(size_t)(t.first + c0 + j) * ldy + feature] = from_f32<TO>(moe_act(__uint_as_float(v[j]) * rs, ACT));
+      for (int j = 0; j < 8; j += 2, dst += 2 * ldy) {
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+        const float g = odd ? got : v[j], u = odd ? v[j + 1] : got;
+        if (in && c + j + odd < c1) *dst = from_f32<TO>(moe_gated(g, u, ACT, ep.limit, ep.alpha));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j, dst += ldy)
+        if (in && c + j < c1) *dst = from_f32<TO>(moe_act(v[j], ACT));
     }
   }
 }
 
 template <int NT, bool GATHER, typename TO>
-__global__ void __launch_bounds__(kMpThreads + (GATHER ? kMpGather : 0), 1)
+__global__ void __launch_bounds__(MpShape<NT>::kThreads + (GATHER ? MpShape<NT>::kGather : 0), 1)
 moe_product_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                            const __nv_bfloat16* __restrict__ x, int64_t ldx, TO* __restrict__ y, int64_t ldy,
                            const int* __restrict__ offsets, const int* __restrict__ order, int experts, int top, int x_by_pair, int N,
@@ -91,15 +110,15 @@ moe_product_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - base));
   int* tiles_before = reinterpret_cast<int*>(smem_gen + (bars - base) + 256);      // [experts + 1]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::kStages; ++s) {
-      mbar_init(full_bar(s), GATHER ? 1 + kMpGather : 1);
+      mbar_init(full_bar(s), GATHER ? 1 + S::kGather / 32 : 1);
       mbar_init(empty_bar(s), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full_bar(b), 1);
-      mbar_init(acc_empty_bar(b), 4);
+      mbar_init(acc_empty_bar(b), S::kStorers);
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -151,82 +170,82 @@ moe_product_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const MpTile m = tile_of(t);
-        const int row = m.expert * N + m.feature;      // (a tile may reach into the next expert's features: such lanes are never stored)
-        const int boxes = GATHER ? 0 : (m.rows + kMpBox - 1) / kMpBox;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % S::kStages;
-          if (!mbar_wait(empty_bar(s), ((it / S::kStages) & 1) ^ 1)) {
-            if (error_word) atomicExch(error_word, 0x7C0061);
-            ok = false;
-            break;
-          }
-          mbar_expect_tx(full_bar(s), kMpWBytes + boxes * kMpBox * kMpK * 2);
-          tma_load_2d(base + s * S::kStage, &map_w, kb * kMpK, row, full_bar(s));
-          for (int i = 0; i < boxes; ++i)      // (likewise a last box into the next tile's rows, or past the matrix)
-            tma_load_2d(base + s * S::kStage + kMpWBytes + i * kMpBox * kMpK * 2, &map_x, kb * kMpK, m.first + i * kMpBox, full_bar(s));
+    const uint32_t leader = umma_leader();
+    uint32_t s = 0, phase = 1;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const MpTile m = tile_of(t);
+      const int row = m.expert * N + m.feature;      // (a tile may reach into the next expert's features: such lanes are never stored)
+      const int boxes = GATHER ? 0 : (m.rows + S::kBox - 1) / S::kBox;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_warp(empty_bar(s), phase)) {
+          if (error_word && leader) atomicExch(error_word, 0x7C0061);
+          ok = false;
+          break;
         }
+        if (leader) {
+          const uint32_t stage = base + s * S::kStage;
+          mbar_expect_tx(full_bar(s), kMpWBytes + boxes * S::kBox * kMpK * 2);
+          tma_load_2d(stage, &map_w, kb * kMpK, row, full_bar(s));
+#pragma unroll
+          for (int i = 0; i < NT / S::kBox; ++i)      // (likewise a last box into the next tile's rows, or past the matrix)
+            if (i < boxes) tma_load_2d(stage + kMpWBytes + i * S::kBox * kMpK * 2, &map_x, kb * kMpK, m.first + i * S::kBox, full_bar(s));
+        }
+        if (++s == S::kStages) { s = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      int j = 0;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++j) {
-        const MpTile m = tile_of(t);
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((m.rows + 15) >> 4) << 18) | ((uint32_t)(kMpM >> 4) << 24);
-        const int b = j & 1;
-        if (!mbar_wait(acc_empty_bar(b), ((j >> 1) & 1) ^ 1)) {
-          if (error_word) atomicExch(error_word, 0x7C0064);
+    const uint32_t leader = umma_leader();
+    uint32_t s = 0, phase = 0;
+    bool ok = true;
+    int j = 0;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++j) {
+      const MpTile m = tile_of(t);
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((m.rows + 15) >> 4) << 18) | ((uint32_t)(kMpM >> 4) << 24);
+      const int b = j & 1;
+      if (!mbar_wait_warp(acc_empty_bar(b), ((j >> 1) & 1) ^ 1)) {
+        if (error_word && leader) atomicExch(error_word, 0x7C0064);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_warp(full_bar(s), phase)) {
+          if (error_word && leader) atomicExch(error_word, 0x7C0062);
+          ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % S::kStages;
-          if (!mbar_wait(full_bar(s), (it / S::kStages) & 1)) {
-            if (error_word) atomicExch(error_word, 0x7C0062);
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          const uint32_t w_src = base + s * S::kStage, x_src = w_src + kMpWBytes;
+        const uint32_t w_src = umma_low_k128(base + s * S::kStage), x_src = w_src + (kMpWBytes >> 4);
 #pragma unroll
-          for (int k = 0; k < kMpK / 16; ++k)
-            umma_f16_idesc(tmem_base + b * NT, umma_desc_k128(w_src + k * 32), umma_desc_k128(x_src + k * 32), idesc, (kb | k) != 0);
-          umma_commit(empty_bar(s));
-        }
-        umma_commit(acc_full_bar(b));      // (also on failure, so that the epilogue does not wait in vain)
+        for (int k = 0; k < kMpK / 16; ++k) umma_warp(leader, tmem_base + b * NT, w_src + k * 2, x_src + k * 2, idesc, (kb | k) != 0);
+        if (leader) umma_commit(empty_bar(s));
+        if (++s == S::kStages) { s = 0; phase ^= 1; }
       }
+      if (leader) umma_commit(acc_full_bar(b));      // (also on failure, so that the epilogue does not wait in vain)
     }
-  } else if (warp < 6) {
-    const int quarter = warp & 3;
+  } else if (warp < 2 + S::kStorers) {
+    // (with eight warps, four take the tile's first columns and four the others)
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     int j = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++j) {
       const MpTile m = tile_of(t);
       const int b = j & 1, feature = m.feature + quarter * 32 + lane;
-      if (!mbar_wait(acc_full_bar(b), (j >> 1) & 1)) {
+      const int middle = S::kStorers == 8 ? ((m.rows >> 1) + 7) & ~7 : m.rows;
+      const int c0 = half ? middle : 0, c1 = half ? m.rows : min(middle, m.rows);
+      if (!mbar_wait_warp(acc_full_bar(b), (j >> 1) & 1)) {
         if (error_word && lane == 0) atomicExch(error_word, 0x7C0063);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll 1
-      for (int c0 = 0; c0 < m.rows; c0 += 32) {
-        uint32_t v[32];
-        tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + b * NT + c0, v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        const float scale = ep.row_scale && c0 + lane < m.rows ? ep.row_scale[order[m.first + c0 + lane]] : 1.f;
+      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + b * NT;
+      if (c0 < c1) {
         switch (ep.act) {
-          case MOE_ACT_NONE: mp_store<MOE_ACT_NONE>(v, y, ldy, m, c0, feature, N, lane, scale, ep); break;
-          case MOE_ACT_RELU2: mp_store<MOE_ACT_RELU2>(v, y, ldy, m, c0, feature, N, lane, scale, ep); break;
-          case MOE_ACT_SILU: mp_store<MOE_ACT_SILU>(v, y, ldy, m, c0, feature, N, lane, scale, ep); break;
-          case MOE_ACT_GELU: mp_store<MOE_ACT_GELU>(v, y, ldy, m, c0, feature, N, lane, scale, ep); break;
-          case MOE_ACT_GLU_CLAMP: mp_store<MOE_ACT_GLU_CLAMP>(v, y, ldy, m, c0, feature, N, lane, scale, ep); break;
-          default: mp_store<MOE_ACT_SWIGLU>(v, y, ldy, m, c0, feature, N, lane, scale, ep); break;
+          case MOE_ACT_NONE: mp_store<MOE_ACT_NONE>(acc, y, ldy, m, c0, c1, feature, N, lane, order, ep); break;
+          case MOE_ACT_RELU2: mp_store<MOE_ACT_RELU2>(acc, y, ldy, m, c0, c1, feature, N, lane, order, ep); break;
+          case MOE_ACT_SILU: mp_store<MOE_ACT_SILU>(acc, y, ldy, m, c0, c1, feature, N, lane, order, ep); break;
+          case MOE_ACT_GELU: mp_store<MOE_ACT_GELU>(acc, y, ldy, m, c0, c1, feature, N, lane, order, ep); break;
+          case MOE_ACT_GLU_CLAMP: mp_store<MOE_ACT_GLU_CLAMP>(acc, y, ldy, m, c0, c1, feature, N, lane, order, ep); break;
+          default: mp_store<MOE_ACT_SWIGLU>(acc, y, ldy, m, c0, c1, feature, N, lane, order, ep); break;
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -234,22 +253,21 @@ moe_product_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       if (lane == 0) mbar_arrive(acc_empty_bar(b));
     }
   } else if constexpr (GATHER) {
-    // row r = r0 + 16 i of the tile, 16-byte piece c of its 128 bytes; the swizzle of a row depends on r % 8 = r0 % 8
-    const int g = threadIdx.x - kMpThreads, r0 = g >> 3, c = g & 7;
+    // row r = r0 + kGatherRows i of the tile, 16-byte piece c of its 128 bytes; the swizzle of a row depends on r % 8 = r0 % 8
+    const int g = threadIdx.x - S::kThreads, r0 = g >> 3, c = g & 7;
     const uint32_t dst0 = kMpWBytes + r0 * 128 + ((c ^ (r0 & 7)) << 4);
-    uint32_t it = 0;
+    uint32_t it = 0, s = 0, phase = 1, ready = 0;      // (ready: the next stage to announce)
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       const MpTile m = tile_of(t);
-      const __nv_bfloat16* src[NT / 16];
+      const __nv_bfloat16* src[NT / S::kGatherRows];
 #pragma unroll
-      for (int i = 0; i < NT / 16; ++i) {
-        const int s = m.first + min(r0 + 16 * i, m.rows - 1);
-        src[i] = x + (size_t)(x_by_pair ? order[s] / top : s) * ldx + c * 8;
+      for (int i = 0; i < NT / S::kGatherRows; ++i) {
+        const int r = m.first + min(r0 + S::kGatherRows * i, m.rows - 1);
+        src[i] = x + (size_t)(x_by_pair ? order[r] / top : r) * ldx + c * 8;
       }
       for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-        const int s = it % S::kStages;
-        if (!mbar_wait(empty_bar(s), ((it / S::kStages) & 1) ^ 1)) {
+        if (!mbar_wait_warp(empty_bar(s), phase)) {
           if (error_word) atomicExch(error_word, 0x7C0065);
           ok = false;
           break;
@@ -257,19 +275,26 @@ moe_product_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         const bool in = kb * kMpK + c * 8 < K;      // (k beyond the rows: zeros, as the weights' copies have there)
         unsigned char* dst = smem_gen + s * S::kStage + dst0;
 #pragma unroll
-        for (int i = 0; i < NT / 16; ++i)
-          if (r0 + 16 * i < m.rows) cp_async16(dst + i * 2048, in ? src[i] + kb * kMpK : x, in);      // (columns behind the rows are never stored)
+        for (int i = 0; i < NT / S::kGatherRows; ++i)
+          if (r0 + S::kGatherRows * i < m.rows) cp_async16(dst + i * S::kGatherRows * 128, in ? src[i] + kb * kMpK : x, in);      // (columns behind the rows are never stored)
         cp_async_commit();
-        if (it >= kMpLag) {
-          cp_async_wait<kMpLag>();
+        if (++s == S::kStages) { s = 0; phase ^= 1; }
+        if (it >= S::kLag) {
+          cp_async_wait<S::kLag>();
           fence_async_shared();
-          mbar_arrive(full_bar((it - kMpLag) % S::kStages));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(full_bar(ready));
+          if (++ready == S::kStages) ready = 0;
         }
       }
     }
     cp_async_wait<0>();
     fence_async_shared();
-    for (uint32_t late = it >= kMpLag ? it - kMpLag : 0; late < it; ++late) mbar_arrive(full_bar(late % S::kStages));
+    __syncwarp();
+    for (uint32_t late = it >= S::kLag ? it - S::kLag : 0; late < it; ++late) {
+      if (lane == 0) mbar_arrive(full_bar(ready));
+      if (++ready == S::kStages) ready = 0;
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
@@ -293,12 +318,17 @@ struct MpArgs {
 };
 
 template <int NT, bool GATHER, typename TO>
-static int launch_moe_product(const MpArgs& a, cudaStream_t stream) {
+static int launch_moe_product(MpArgs& a, cudaStream_t stream) {
   auto kern = moe_product_tcgen05_kernel<NT, GATHER, TO>;
+  a.map_x = a.map_w;      // (unused when gathered)
+  if (!GATHER) {
+    const int rc = make_map(&a.map_x, a.x, a.pairs, a.K, a.ldx, MpShape<NT>::kBox);
+    if (rc != TIB_OK) return rc;
+  }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MpShape<NT>::kSmem);
   if (e != cudaSuccess) return (int)e;
   const int64_t most = ((int64_t)a.pairs / NT + (a.pairs < a.experts ? a.pairs : a.experts)) * ceil_div(a.N, kMpM);
-  TIB_LAUNCH_DEPENDENT(kern, (int)(most < 148 ? most : 148), kMpThreads + (GATHER ? kMpGather : 0), MpShape<NT>::kSmem, stream, a.map_w, a.map_x,
+  TIB_LAUNCH_DEPENDENT(kern, (int)(most < 148 ? most : 148), MpShape<NT>::kThreads + (GATHER ? MpShape<NT>::kGather : 0), MpShape<NT>::kSmem, stream, a.map_w, a.map_x,
                        a.x, a.ldx, (TO*)a.y, a.ldy, a.offsets, a.order, a.experts, a.top, a.x_by_pair, a.N, a.K, a.ep, a.error_word);
   return TIB_OK;
 }
@@ -313,7 +343,6 @@ int moe_product_tcgen05(const void* x, int64_t ldx, const void* w, void* y, int 
                         cudaStream_t stream) {
   MpArgs a;
   int rc = make_map(&a.map_w, w, experts * N, K, K, kMpM);
-  if (rc == TIB_OK) rc = x_by_pair ? make_map(&a.map_x, w, experts * N, K, K, kMpBox) : make_map(&a.map_x, x, pairs, K, ldx, kMpBox);      // (unused when gathered)
   if (rc != TIB_OK) return rc;
   a.x = (const __nv_bfloat16*)x; a.ldx = ldx; a.y = y; a.ldy = ldy; a.offsets = offsets; a.order = order; a.pairs = pairs;
   a.experts = experts; a.top = top; a.x_by_pair = x_by_pair; a.N = N; a.K = K; a.ep = ep; a.error_word = error_word;
