@@ -1520,3 +1520,22 @@ def test_gathered_latent_rows_stay_within_their_buffer(missing):
     got = torch.cat([latent_room, rotated_room], 1).cpu()
     assert torch.equal(got[:rows], want[:rows]) and (got[rows:] == 7.0).all()
     assert int(error) == (0x60001 if missing else 0)
+
+
+@pytest.mark.parametrize("rows, width, wide, dtypes, shift", [
+    (1, 8, 8, (torch.bfloat16, torch.bfloat16, torch.bfloat16), 0), (7, 520, 1040, (torch.float32, torch.bfloat16, None), 8),
+    (296, 2056, 2056, (torch.bfloat16, None, torch.float32), 0), (5, 516, 520, (torch.bfloat16, torch.float32, torch.bfloat16), 0),
+    (3, 64, 96, (torch.bfloat16, torch.bfloat16, torch.bfloat16), 1)])      # (the last two: not by eight)
+def test_sums_of_two_outputs(rows, width, wide, dtypes, shift):
+    """residual += a + b, every sum in 32 bits: the same numbers as torch's, bit for bit."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    a, b = (rnd(rows, wide + shift, dtype=t, seed=s)[:, shift:shift + width] if t else None for s, t in enumerate(dtypes[:2]))
+    residual = rnd(rows, width, seed=5)
+    copy = torch.empty(rows, width, dtype=dtypes[2], device="cuda") if dtypes[2] else None
+    got = dev(residual)
+    on = [t if t is None else dev(t._base if t._base is not None else t)[:, shift:shift + width] for t in (a, b)]
+    ops.add_pair(got, on[0], on[1], copy)
+    want = residual + (a.float() if b is None else a.float() + b.float())
+    assert torch.equal(got.cpu(), want)
+    assert copy is None or torch.equal(copy.cpu(), want.to(copy.dtype))
