@@ -1224,6 +1224,36 @@ def test_scan_in_chunks_keeps_what_is_not_finite_from_earlier_tokens(lens, head_
             assert torch.equal(carried[1:], clean_state[1:])
 
 
+@pytest.mark.parametrize("head_dim, state", [(64, 128), (32, 64)])      # (on tcgen05; on mma.sync)
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_scan_in_chunks_keeps_a_step_size_that_is_not_finite_from_earlier_tokens(head_dim, state, bad):
+    """One step size of one head of one request: that head's rows from the token on, whichever of its four neighbours in the scan it is."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, lens = 3, [300, 129]
+    n, inner = sum(lens), heads * head_dim
+    xbc, steps = dev(rnd(n, inner + 2 * state, dtype=torch.bfloat16)), rnd(n, heads, dtype=torch.bfloat16, seed=1)
+    bias, a_log, skip = dev(rnd(heads, seed=2) - 3.0), dev(rnd(heads, seed=3)), dev(rnd(heads, seed=4))
+    held, starts = rnd(2, heads * state * head_dim, seed=5), dev(torch.tensor([0, lens[0], n], dtype=torch.int32))
+
+    def run(dt):
+        y, carried = torch.empty(n, inner, device="cuda"), dev(held.clone())
+        ops.ssd_scan(xbc, dev(dt), 0, bias, a_log, skip, carried, starts, dev(torch.arange(2, dtype=torch.int32)), y, 2, heads=heads, groups=1,
+                     state_dim=state, head_dim=head_dim, max_q_len=max(lens))
+        return y.cpu(), carried.cpu()
+
+    clean, clean_state = run(steps)
+    for t in (0, 1, 2, 3, 5, 30, 31, 126, 127, 128, 130, lens[0] - 1):
+        broken = steps.clone()
+        broken[t, 1] = bad
+        y, carried = run(broken)
+        changed = torch.zeros(n, inner, dtype=torch.bool)
+        changed[t:lens[0], head_dim:2 * head_dim] = True
+        assert torch.equal(y[~changed], clean[~changed]) and torch.equal(carried[1:], clean_state[1:]), t
+        if bad != bad:
+            assert y[changed].isnan().all(), t
+
+
 def test_scan_in_chunks_of_an_infinite_state():
     """One infinite element of a request's state: its column is infinite from then on, as in the token-by-token walk."""
     need_gpu()

@@ -82,7 +82,7 @@ __device__ __forceinline__ void st_steps(StSteps& s, const ScanArgs& a, const St
     const double from = __shfl_up_sync(0xffffffffu, up, o);
     if (lane >= o) up += from;
   }
-  const double before = up - f[3];
+  const double below = __shfl_up_sync(0xffffffffu, up, 1), before = lane ? below : 0.0;      // (not up - f[3]: a NaN step is not its earlier neighbours')
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const double sum = before + f[k];
