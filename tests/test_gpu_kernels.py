@@ -1444,6 +1444,51 @@ def test_window_attention_with_the_appends_turns_has_the_bits_of_its_own(dim, ke
     assert torch.equal(run(own), run(None))
 
 
+GATES = [float("nan"), float("inf"), float("-inf"), 0.0, -20.0, 60.0, -86.0, -87.5, -88.5]      # (the last: a sigmoid below the normal numbers)
+
+
+def test_gates_of_window_attention_on_prompts():
+    """A prompt's gates against those of the kernel for few tokens: NaN stays NaN, the smallest ones do not become zero."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, kv_heads, page, dim, n = 2, 1, 16, 64, 140
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    per = -(-n // page)
+    keys, values = (dev(rnd(per, kv_heads, page, dim, dtype=torch.bfloat16, seed=i)) for i in range(2))
+    q, gate = dev(rnd(n, heads * dim, dtype=torch.bfloat16)), rnd(n, heads * dim, seed=9)
+    for i, g in enumerate(GATES):
+        gate[3 + 13 * i, 5 * i:5 * i + 60] = g
+    gate = dev(gate, torch.bfloat16)
+    run = lambda gate: ops.pooled_window_attention(q, torch.empty_like(q), ints([0, n]), ints([0]), ints([0]), keys, values, ints(range(per)).view(1, per), None, None,
+                                                   None, 1, n, heads, kv_heads, window=100, pool=0, scale=dim ** -0.5, gate=gate).cpu()
+    plain, got = run(None).double(), run(gate)
+    want = plain * torch.sigmoid(gate.cpu().double())
+    assert torch.equal(got.isnan(), want.isnan()) and not got.isinf().any()
+    # a rounding to bf16 is off by at most 2^-8 of the value (eight significant bits), and the rows without gates are rounded and these again
+    assert ((got.double() - want).abs() <= 2.0 ** -6.9 * want.abs() + 2.0 ** -133)[~want.isnan()].all()
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+def test_gates_of_latent_attention_on_prompts(per_head):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, dim, rot, n = 4, 64, 64, 140
+    rows = 256
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    q = dev(rnd(n, heads * (dim + rot), dtype=torch.bfloat16))
+    kv, rotated = dev(rnd(rows, heads * 2 * dim, dtype=torch.bfloat16, seed=1)), dev(rnd(rows, rot, dtype=torch.bfloat16, seed=2))
+    gate = rnd(n, heads * (1 if per_head else dim), seed=9)
+    for i, g in enumerate(GATES):
+        gate[3 + 13 * i, i % 4 if per_head else slice(20 * i, 20 * i + 60)] = g
+    gate = dev(gate, torch.bfloat16)
+    run = lambda gate: ops.latent_prefill(q, kv, rotated, torch.empty(n, heads, dim, dtype=torch.bfloat16, device="cuda"), ints([0, n]), ints([0]), 1, n, heads, dim, dim,
+                                          (dim + rot) ** -0.5, gate=gate, gate_per_head=per_head).cpu()
+    plain, got = run(None).double(), run(gate)
+    want = plain * torch.sigmoid(gate.cpu().double()).view(n, heads, -1)
+    assert torch.equal(got.isnan(), want.isnan()) and not got.isinf().any()
+    assert ((got.double() - want).abs() <= 2.0 ** -6.9 * want.abs() + 2.0 ** -133)[~want.isnan()].all()
+
+
 @pytest.mark.parametrize("tokens, kv_heads, dim, vdim, pool", [(65, 1, 64, 64, 4), (97, 2, 40, 24, 8), (300, 2, 128, 96, 32), (130, 1, 16, 8, 1)])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_block_means_of_large_steps_have_the_bits_of_small_ones(tokens, kv_heads, dim, vdim, pool, dtype):

@@ -97,12 +97,13 @@ __device__ __forceinline__ float rope_lo(float lo, float hi, float c, float s) {
 __device__ __forceinline__ float rope_hi(float lo, float hi, float c, float s) { return __fmaf_rn(hi, c, __fmul_rn(lo, s)); }
 
 // 1 / (1 + e^-x), the reciprocal by a Newton step from the approximate one, within 0.51 units in the last place.  For code that runs once a block: an
-// IEEE division is half of the instructions around it, and these wait for their own fetch.  (Below -88 it is 6e-39 instead of less.)
+// IEEE division is half of the instructions around it, and these wait for their own fetch.  Below -80, where the approximate reciprocal would
+// soon flush to zero and its Newton step meet an infinity, the value is e^x to the last bit; a NaN stays one.
 __device__ __forceinline__ float sigmoid_newton(float x) {
-  const float d = 1.f + expf(fminf(-x, 88.f));
+  const float d = 1.f + expf(-x);
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-  return fmaf(y, fmaf(-d, y, 1.f), y);
+  return x < -80.f ? expf(x) : fmaf(y, fmaf(-d, y, 1.f), y);
 }
 
 // x times the normal distribution's cumulative function at x (the exact form of the Gaussian error linear unit)
