@@ -1115,6 +1115,52 @@ def test_linear_attention_keeps_what_is_not_finite_from_earlier_tokens(lens, dim
             assert torch.equal(state[1:], clean_state[1:])
 
 
+@pytest.mark.parametrize("key_dim, value_dim", [(64, 64), (128, 128)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_linear_attention_in_runs_keeps_infinities_and_the_largest_numbers(key_dim, value_dim, dtype):
+    """One infinite (or, in 32 bits, very large) number of q, k, v or the state: what the formula of the runs gives in 64 bits, infinities with their signs."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, n, run = 2, 400, ops.linear_attention_run()
+    qk, vv = heads * key_dim, heads * value_dim
+    decay = torch.tensor([0.99, 0.9], dtype=torch.float64)
+    powers = [dev((decay[:, None] ** torch.arange(most + 1, dtype=torch.float64)).float().contiguous()) for most in (ops.linear_attention_chunk(key_dim, value_dim), run)]
+    rows, held = rnd(n, 2 * qk + vv, dtype=dtype, scale=0.05), rnd(1, heads, key_dim, value_dim, seed=5, scale=0.05)
+    held, large = held + 0.01 * held.sign(), 3.395e38      # (above the largest bf16 number)
+
+    def reference(rows, held):
+        x, s = rows.double(), held[0].double().clone()
+        q, k, v = x[:, :qk].view(n, heads, -1), x[:, qk:2 * qk].view(n, heads, -1), x[:, 2 * qk:].view(n, heads, -1)
+        out = torch.empty(n, heads, value_dim, dtype=torch.float64)
+        for t0 in range(0, n, run):
+            m = min(run, n - t0)
+            for h in range(heads):
+                back = decay[h] ** torch.arange(m, dtype=torch.float64)
+                scores = q[t0:t0 + m, h] @ k[t0:t0 + m, h].T
+                for i in range(m):
+                    out[t0 + i, h] = decay[h] ** (i + 1) * (q[t0 + i, h] @ s[h]) + (scores[i, :i + 1] * back[:i + 1].flip(0)) @ v[t0:t0 + i + 1, h]
+                s[h] = decay[h] ** m * s[h] + (k[t0:t0 + m, h] * back.flip(0)[:, None]).T @ v[t0:t0 + m, h]
+        return out.view(n, -1).float(), s.float()
+
+    places = [("state", (0, 1, 17, 5)), ("q", (200, key_dim + 3)), ("k", (130, qk + 7)), ("v", (255, 2 * qk + value_dim + 9)), ("k", (399, qk + key_dim + 1))]
+    for what, place in places:
+        for bad in (float("inf"), float("-inf"), float("nan")) + ((large,) if dtype == torch.float32 or what == "state" else ()):
+            broken, state = rows.clone(), held.clone()
+            (state if what == "state" else broken)[place] = bad
+            want, want_state = reference(broken, state)
+            proj, got_state = dev(broken), dev(state)
+            out = ops.linear_attention(proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:], torch.empty(n, vv, device="cuda"), got_state, powers[0],
+                                       dev(torch.tensor([0, n], dtype=torch.int32)), dev(torch.zeros(1, dtype=torch.int32)), 1, heads, key_dim, value_dim, silu=False,
+                                       max_q_len=n, run_powers=powers[1], portions={n: 1})
+            for got, ref in ((out.cpu(), want), (got_state[0].cpu(), want_state)):
+                assert torch.equal(got.isnan(), ref.isnan()), (what, bad)
+                assert torch.equal(got.sign() * got.isinf(), ref.sign() * ref.isinf()), (what, bad)
+                # (fp32 sums: 2e-6 of the largest value a sum of this kind meets, as in the test of the forms; a column's or row's own where one is huge)
+                fine = torch.isfinite(ref)
+                size = ref.abs().where(fine, 0.).amax(-1, keepdim=True).maximum(ref.abs().where(fine, 0.).amax(-2, keepdim=True))
+                assert ((got - ref).abs() <= 2e-6 * size + 2e-8)[fine].all(), (what, bad)
+
+
 # ------------------------------------------------------------------------------------------------- the experts' products
 @pytest.mark.parametrize("tokens, experts, top, k, n, act, by_pair, out_dtype", [
     (1, 1, 1, 8, 16, "none", True, torch.float32), (5, 4, 2, 72, 130, "relu2", True, torch.bfloat16),      # tails of k and of the features

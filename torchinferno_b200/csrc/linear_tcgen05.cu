@@ -10,7 +10,8 @@
 //     S -> k's place               carried = q S                        (scores are weighed, split and put back into tensor memory meanwhile)
 //     v -> q's place               inside = scores v                    (carried is read and scaled before)
 // One launch a run and head keeps no chain between runs but the fold's.  A value that is not finite would meet the weight 0 of the tokens
-// before it: it stays out of the product and is added to its own column from its own token on.
+// before it: it stays out of the product and is added to its own column from its own token on.  Any other infinity, and a number that rounds to
+// one in bf16, makes NaN of what it meets in three terms: a sum or output that is not finite is made again by multiply-adds in order.
 //
 // What bounds it: the threads' activations and conversions (27 instructions an element) between the products, with one block of 16 warps an SM (192 KB
 // of terms): issue slots a third full, tensor cores a fifth.  Blocks of 8 warps took 117 us in all where these take 68.  Figures: linear_attention.cu.
@@ -139,6 +140,15 @@ template <int D, int TV, int ACC> struct LtSums {
   static constexpr uint32_t kColumns = ACC * TV;
 };
 
+// An element of L by multiply-adds: k and v at the run's first token.
+template <typename T>
+__device__ __noinline__ float lt_plain_sum(const T* k, int64_t ldk, const T* v, int64_t ldv, const float* pw, int n, int activation) {
+  float s = 0.f;
+  for (int j = 0; j < n && s == s; ++j)
+    s = fmaf(pw[n - 1 - j] * lt_act(to_f32(k[(size_t)j * ldk]), activation), lt_act(to_f32(v[(size_t)j * ldv]), activation), s);
+  return s;
+}
+
 // grid (heads * column tiles, runs, entries).  How many accumulators there are is the value heads' width's alone, not the tile's, which the step
 // chooses: a request's bits do not depend on its neighbours.
 template <typename T, int D, int TV, int ACC>
@@ -179,11 +189,12 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
     __syncwarp();
   }
   ft_wait(bar, 0, a.error_word, 0x7C0081);
-  const int quarter = warp & 3, d = quarter * 32 + lane;
-  const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16);
-  float* dst = a.run_state + (b.run * a.n_heads + b.own) * (size_t)D * a.value_dim + (size_t)d * a.value_dim + b.col0;
+  const int quarter = warp & 3, part = warp >> 2, d = quarter * 32 + lane;
+  const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + part * (TV / 4);
+  float* dst = a.run_state + (b.run * a.n_heads + b.own) * (size_t)D * a.value_dim + (size_t)d * a.value_dim + b.col0 + part * (TV / 4);
+  uint32_t again = 0;      // columns to be made again
 #pragma unroll
-  for (int c0 = (warp >> 2) * (TV / 4); c0 < (warp >> 2) * (TV / 4) + TV / 4; c0 += 16) {
+  for (int c0 = 0; c0 < TV / 4; c0 += 16) {
     float sum[16];
 #pragma unroll
     for (int i = 0; i < ACC; i += 2) {
@@ -199,10 +210,17 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
     }
     if (D < 128 && d >= D) continue;
 #pragma unroll
+    for (int e = 0; e < 16; ++e) again |= isfinite(sum[e]) ? 0u : 1u << (c0 + e);
+#pragma unroll
     for (int e = 0; e < 16; e += 8) {
       const float o[8] = {sum[e], sum[e + 1], sum[e + 2], sum[e + 3], sum[e + 4], sum[e + 5], sum[e + 6], sum[e + 7]};
       ft_store8(dst + c0 + e, o);
     }
+  }
+  for (; again; again &= again - 1) {
+    const int c = __ffs(again) - 1;
+    dst[c] = lt_plain_sum(k + first * a.ldk + b.head * D + d, a.ldk, v + first * a.ldv + b.head * a.value_dim + b.col0 + part * (TV / 4) + c, a.ldv, pw, b.n,
+                          a.activation);
   }
   ft_release(warp, tmem, S::kColumns);
 }
@@ -213,6 +231,30 @@ template <int D, int TV> struct LtOuts {
   static constexpr uint32_t kSecond = 3 * (kKeyTerm > kStateTerm ? kKeyTerm : kStateTerm);     // k, then S
   static constexpr uint32_t kSmem = 1024 + kFirst + kSecond + 64;
 };
+
+// The columns `again` of token i's outputs by multiply-adds: query is its own row, k and v lie at the run's first token, v, state and dst at the
+// thread's columns.
+template <typename T, int D>
+__device__ __noinline__ void lt_plain_outs(uint32_t again, int i, const T* query, const T* k, int64_t ldk, const T* v, int64_t ldv, const float* state,
+                                           int value_dim, float* dst, const float* pw, int activation) {
+  for (uint32_t left = again; left; left &= left - 1) {
+    const int c = __ffs(left) - 1;
+    float s = 0.f;
+    for (int d = 0; d < D && s == s; ++d) s = fmaf(state[(size_t)d * value_dim + c], lt_act(to_f32(query[d]), activation), s);
+    dst[c] = s * pw[i + 1];
+  }
+  for (int j = 0; j <= i && again; ++j) {
+    float w = 0.f;
+    for (int d = 0; d < D && w == w; ++d) w = fmaf(lt_act(to_f32(query[d]), activation), lt_act(to_f32(k[(size_t)j * ldk + d]), activation), w);
+    w *= pw[i - j];
+    for (uint32_t left = again; left; left &= left - 1) {
+      const int c = __ffs(left) - 1;
+      const float s = fmaf(w, lt_act(to_f32(v[(size_t)j * ldv + c]), activation), dst[c]);
+      dst[c] = s;
+      if (s != s) again ^= 1u << c;      // (it stays NaN)
+    }
+  }
+}
 
 template <typename T, int D, int TV>
 __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, LinRunArgs a) {
@@ -362,6 +404,9 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
 #pragma unroll
     for (int c = 0; c < 16; ++c) sum[c0 + c] += __uint_as_float(x[c]) + __uint_as_float(y[c]);
   }
+  uint32_t again = 0;      // columns to be made again
+#pragma unroll
+  for (int c = 0; c < TV / 4; ++c) again |= isfinite(sum[c]) ? 0u : 1u << c;
   float* dst = a.out + (first + i) * a.heads * a.value_dim + b.head * a.value_dim + b.col0 + part * (TV / 4);
   if (i < b.n) {
 #pragma unroll
@@ -390,6 +435,9 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
       __syncwarp();
     }
   }
+  if (again && i < b.n)
+    lt_plain_outs<T, D>(again, i, q + (first + i) * a.ldq + b.head * D, k + first * a.ldk + b.head * D, a.ldk, values + part * (TV / 4), a.ldv,
+                        state + part * (TV / 4), a.value_dim, dst, pw, a.activation);
   ft_release(warp, tmem, 512);
 }
 
