@@ -1300,6 +1300,34 @@ def test_scan_in_chunks_keeps_a_step_size_that_is_not_finite_from_earlier_tokens
             assert y[changed].isnan().all(), t
 
 
+def test_scan_in_chunks_keeps_infinities_with_their_signs():
+    """An infinite x or step size: its columns of the state as token by token; an infinite B: the rows of its chunk as well."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, head_dim, state, n = 2, 64, 128, 200
+    inner = heads * head_dim
+    xbc, steps = rnd(n, inner + 2 * state, dtype=torch.bfloat16), rnd(n, heads, dtype=torch.bfloat16, seed=1)
+    bias, a_log, skip = dev(rnd(heads, seed=2) - 6.0), dev(0.2 * rnd(heads, seed=3)), dev(rnd(heads, seed=4))      # (nothing decays to zero)
+    held = rnd(1, heads * state * head_dim, seed=5)
+    signs = lambda t: t.sign() * t.isinf()
+    for what, t, column in (("x", 0, 3), ("x", 70, head_dim + 17), ("x", 127, 63), ("x", 128, 40), ("x", n - 1, 0), ("step", 65, 1), ("step", 131, 0), ("B", 0, 9), ("B", 40, 9), ("B", 150, 100)):
+        for bad in (math.inf,) if what == "step" else (math.inf, -math.inf):
+            rows, dt = xbc.clone(), steps.clone()
+            (dt if what == "step" else rows)[t, inner + column if what == "B" else column] = bad
+            results = []
+            for longest in (n, None):      # (in chunks; token by token)
+                y, carried = torch.empty(n, inner, device="cuda"), dev(held.clone())
+                ops.ssd_scan(dev(rows), dev(dt), 0, bias, a_log, skip, carried, dev(torch.tensor([0, n], dtype=torch.int32)), dev(torch.zeros(1, dtype=torch.int32)),
+                             y, 1, heads=heads, groups=1, state_dim=state, head_dim=head_dim, max_q_len=longest)
+                results.append((carried.view(heads, state, head_dim).cpu(), y.cpu()))
+            (got, y), (want, want_y) = results
+            if what == "B":
+                rows = slice(t, min(n, t // 128 * 128 + 128))
+                assert (signs(y[rows]) != 0).all() and torch.equal(signs(y[rows]), signs(want_y[rows])), (what, t, bad)
+            else:
+                assert torch.equal(got.isnan(), want.isnan()) and torch.equal(signs(got), signs(want)) and int(got.isinf().sum()) == state * (head_dim if what == "step" else 1), (what, t, bad)
+
+
 def test_scan_in_chunks_of_an_infinite_state():
     """One infinite element of a request's state: its column is infinite from then on, as in the token-by-token walk."""
     need_gpu()

@@ -62,6 +62,21 @@ __device__ __forceinline__ float st_power(float ah, float al, float bh, float bl
   return fmaf(p, lost + (al - bl), p);
 }
 
+// The terms of W numbers; an infinity has nothing in the lower two, where it would meet its opposite or a zero.
+template <int W>
+__device__ __forceinline__ void st_split(const float (&v)[W], uint32_t (&t)[3][W / 2]) {
+  float largest = 0.f;
+#pragma unroll
+  for (int e = 0; e < W; ++e) largest = fmaxf(largest, fabsf(v[e]));
+  if (largest < 3e38f) {
+#pragma unroll
+    for (int e = 0; e < W / 2; ++e) ft_split2(v[2 * e], v[2 * e + 1], t[0][e], t[1][e], t[2][e]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < W / 2; ++e) ft_split2_finite(v[2 * e], v[2 * e + 1], t[0][e], t[1][e], t[2][e]);
+  }
+}
+
 // A warp fills in the steps of one item: four tokens a lane, F summed in double precision (tokens behind the chunk's: no step, the sum stays).
 template <bool SUMS>
 __device__ __forceinline__ void st_steps(StSteps& s, const ScanArgs& a, const StBlock& b, int h, int lane) {
@@ -159,10 +174,14 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_sums_tcgen05_kernel(ScanArg
       const int p = tid + i * kStThreads, r = p >> 3;
       const float w = steps[it].w[r];
       const uint32_t raw[4] = {x.v[i].x, x.v[i].y, x.v[i].z, x.v[i].w};
-      uint32_t t[3][4];
+      float wx[8];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        ft_split2(__uint_as_float(raw[e] << 16) * w, __uint_as_float(raw[e] & 0xffff0000u) * w, t[0][e], t[1][e], t[2][e]);
+      for (int e = 0; e < 4; ++e) {
+        wx[2 * e] = __uint_as_float(raw[e] << 16) * w;
+        wx[2 * e + 1] = __uint_as_float(raw[e] & 0xffff0000u) * w;
+      }
+      uint32_t t[3][4];
+      st_split(wx, t);
 #pragma unroll
       for (int u = 0; u < 3; ++u) *reinterpret_cast<uint4*>(tile + u * kStSub + ft_place(r, p & 7, kQ)) = make_uint4(t[u][0], t[u][1], t[u][2], t[u][3]);
     }
@@ -264,16 +283,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
       const int p = tid + i * kStThreads;
       const float v[8] = {held[i][0].x, held[i][0].y, held[i][0].z, held[i][0].w, held[i][1].x, held[i][1].y, held[i][1].z, held[i][1].w};
       uint32_t t[3][4];
-      float largest = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) largest = fmaxf(largest, fabsf(v[e]));
-      if (largest < 3e38f) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ft_split2(v[2 * e], v[2 * e + 1], t[0][e], t[1][e], t[2][e]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ft_split2_finite(v[2 * e], v[2 * e + 1], t[0][e], t[1][e], t[2][e]);
-      }
+      st_split(v, t);
 #pragma unroll
       for (int u = 0; u < 3; ++u) *reinterpret_cast<uint4*>(tile + u * S::kTerm + ft_place(p >> 3, p & 7, N)) = make_uint4(t[u][0], t[u][1], t[u][2], t[u][3]);
     }
@@ -397,9 +407,12 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
       for (int c0 = 0; c0 < 32; c0 += 16) {
         uint32_t t[3][8] = {};
         if (part <= quarter) {
+          float half[16];
 #pragma unroll
-          for (int c = 0; c < 16; c += 2) ft_split2(s[c0 + c], s[c0 + c + 1], t[0][c / 2], t[1][c / 2], t[2][c / 2]);
+          for (int c = 0; c < 16; ++c) half[c] = s[c0 + c];
+          st_split(half, t);
         }
+        __syncwarp();
 #pragma unroll
         for (int u = 0; u < 3; ++u) ft_tmem_st8(tmem + lanes + u * 64 + part * 16 + c0 / 2, t[u]);
       }
