@@ -1631,6 +1631,28 @@ def test_latent_single_tokens_on_tensor_cores(heads, rank, rot, entries, sink):
     assert (out - plain).abs().max() <= (2.0 ** -16 + 640 * 2.0 ** -23) * plain.abs().max() and int(error) == 0
 
 
+@pytest.mark.parametrize("heads, rank, rot, entries", [(17, 512, 224, 3), (5, 512, 256, 150), (16, 384, 384, 2)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_latent_single_tokens_of_the_widest_rows_on_tensor_cores(heads, rank, rot, entries, shift):
+    """Rows too wide for the sixteen warps' shared memory, and queries off their 16-byte boundaries, take the kernel of four warps: its sums are not the CUDA cores'."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    page, width = 16, rank + rot
+    contexts = [(1, 64, 65, 127, 200, 129)[i % 6] + 64 * (i % 2) for i in range(entries)]
+    per = -(-max(contexts) // page)
+    keys = dev(rnd(entries * per, 1, page, width, dtype=torch.bfloat16, scale=0.7))
+    table = dev(torch.randperm(entries * per, generator=torch.Generator().manual_seed(4)).int().view(entries, per))
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    room = torch.empty(entries * heads * width + shift, device="cuda")
+    folded = room[shift:].view(entries, heads, width)
+    folded.copy_(rnd(entries, heads, width, scale=0.3, seed=1).bfloat16().float())
+    error = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, plain = (ops.latent_attention(folded, keys, torch.empty(entries, heads, rank, device="cuda"), ints(range(entries + 1)), ints(c - 1 for c in contexts),
+                                       ints(range(entries)), table, entries, 1, heads, rank, rot, 0.11, error, max_kv_len=max(contexts), force_simt=simt) for simt in (False, True))
+    assert (out - plain).abs().max() <= (2.0 ** -16 + 900 * 2.0 ** -23) * plain.abs().max() and int(error) == 0
+    assert not torch.equal(out, plain)
+
+
 @pytest.mark.parametrize("tokens, experts, kept, top, groups, keep", [(1, 1, 1, 1, 1, 1), (31, 40, 33, 3, 4, 2), (64, 300, 300, 8, 1, 1), (65, 64, 64, 2, 8, 3)])
 def test_choices_and_sorting_in_one_launch(tokens, experts, kept, top, groups, keep):
     """Some choices name no expert (``kept`` of ``experts`` are ones): their place is -1."""

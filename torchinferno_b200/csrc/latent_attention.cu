@@ -346,15 +346,14 @@ static inline size_t latent_mma_smem(int width, int mt) {
          + 4 * ((size_t)2 * kMmaWarps * mt * 16);                                                          // fp32: maxima and sums per warp
 }
 
-constexpr int kMmaTiles = 2;        // m-tiles of 16 rows a block owns (rows are (token, head) pairs of one entry, heads fastest)
-
-// R64 = rank / 64: every warp owns 16 * R64 value columns.
-template <int R64>
+// MT: m-tiles of 16 rows a block owns (rows are (token, head) pairs of one entry, heads fastest); two, and one for the single tokens that
+// latent_decode_kernel does not take.  R64 = rank / 64: every warp owns 16 * R64 value columns.
+template <int MT, int R64>
 __global__ void __launch_bounds__(kMmaWarps * 32)
 latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat16* __restrict__ pool, float* __restrict__ out,
                             LatentAttnArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int MT = kMmaTiles, RB = MT * 16;
+  constexpr int RB = MT * 16;
   const int w = a.width, wp = w + 8, pp = kMmaKeys + 8;
   __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);       // [RB][wp]
   __nv_bfloat16* k_s = q_s + RB * wp;                                     // [2][64][wp]
@@ -368,7 +367,8 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
   const int row0 = a.q_start[entry] - a.row_base;
   const int q_len = a.q_start[entry + 1] - a.row_base - row0;
   const int total_rows = q_len * a.heads;
-  const int r0 = blockIdx.x * RB;                                         // first (token, head) row of the block
+  const int split = a.partial ? blockIdx.x : 0;
+  const int r0 = a.partial ? blockIdx.z * RB : blockIdx.x * RB;           // first (token, head) row of the block
   if (r0 >= total_rows || q_len > a.longest) return;
   const int nrows = min(RB, total_rows - r0);
   const int kv0 = a.kv_start[entry];
@@ -376,7 +376,12 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
   const int* table = a.block_table + (size_t)a.slots[entry] * a.table_stride;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
 
-  const int tile_lo = 0, tile_hi = last_pos / kMmaKeys;
+  int tile_lo = 0, tile_hi = last_pos / kMmaKeys;
+  if (a.partial) {      // (blocks_per_split counts runs of 32 keys; a tile is two of them)
+    const int tiles_per_split = (a.blocks_per_split + 1) / 2;
+    tile_lo = split * tiles_per_split;
+    tile_hi = min(tile_hi, tile_lo + tiles_per_split - 1);
+  }
   const int pieces_per_key = w / 8;
   auto fetch = [&](int stage, int tile) {      // a warp takes every fourth key, its lanes the 16-byte pieces of the row
     __nv_bfloat16* dst = k_s + (size_t)stage * kMmaKeys * wp;
@@ -561,12 +566,22 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
     for (int h = 0; h < 2; ++h) {
       const int r = mt * 16 + g + h * 8;
       if (r >= nrows) continue;
-      float* dst = out + ((size_t)row0 * a.heads + r0 + r) * a.rank;
-      const float inv = latent_inverse(m_run[mt][h], l_run[mt][h], a.sink, (r0 + r) % a.heads);
+      if (a.partial) {      // (one token per entry: the block's rows are heads)
+        float* p = a.partial + (((size_t)row0 * a.heads + r0 + r) * a.n_splits + split) * (2 + a.rank);
+        if (warp == 0 && t4 == 0) { p[0] = m_run[mt][h]; p[1] = l_run[mt][h]; }
 #pragma unroll
-      for (int n = 0; n < 2 * R64; ++n) {
-        dst[col0 + n * 8 + 2 * t4] = o[mt][n][2 * h] * inv;
-        dst[col0 + n * 8 + 2 * t4 + 1] = o[mt][n][2 * h + 1] * inv;
+        for (int n = 0; n < 2 * R64; ++n) {
+          p[2 + col0 + n * 8 + 2 * t4] = o[mt][n][2 * h];
+          p[2 + col0 + n * 8 + 2 * t4 + 1] = o[mt][n][2 * h + 1];
+        }
+      } else {
+        float* dst = out + ((size_t)row0 * a.heads + r0 + r) * a.rank;
+        const float inv = latent_inverse(m_run[mt][h], l_run[mt][h], a.sink, (r0 + r) % a.heads);
+#pragma unroll
+        for (int n = 0; n < 2 * R64; ++n) {
+          dst[col0 + n * 8 + 2 * t4] = o[mt][n][2 * h] * inv;
+          dst[col0 + n * 8 + 2 * t4 + 1] = o[mt][n][2 * h + 1] * inv;
+        }
       }
     }
 }
@@ -787,22 +802,25 @@ static int launch_latent_merge(float* out, const LatentAttnArgs& a, int n_entrie
 }
 
 template <int R64>
+static int launch_latent_decode(const float* folded, const void* pool, float* out, const LatentAttnArgs& a, int n_entries, cudaStream_t stream) {
+  const size_t smem = latent_decode_smem(a.width);
+  const cudaError_t e = cudaFuncSetAttribute(latent_decode_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  TIB_LAUNCH_DEPENDENT(latent_decode_kernel<R64>, dim3(a.partial ? a.n_splits : 1, n_entries, ceil_div(a.heads, 16)), kLdThreads, smem, stream,
+                       folded, (const __nv_bfloat16*)pool, out, a);
+  return a.partial ? launch_latent_merge(out, a, n_entries, stream) : TIB_OK;
+}
+
+template <int MT, int R64>
 static int launch_latent_mma(const float* folded, const void* pool, float* out, const LatentAttnArgs& a, int n_entries, int max_q_len,
                              cudaStream_t stream) {
-  if (max_q_len == 1) {
-    const size_t smem = latent_decode_smem(a.width);
-    const cudaError_t e = cudaFuncSetAttribute(latent_decode_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    TIB_LAUNCH_DEPENDENT(latent_decode_kernel<R64>, dim3(a.partial ? a.n_splits : 1, n_entries, ceil_div(a.heads, 16)), kLdThreads, smem, stream,
-                         folded, (const __nv_bfloat16*)pool, out, a);
-    return a.partial ? launch_latent_merge(out, a, n_entries, stream) : TIB_OK;
-  }
-  const size_t smem = latent_mma_smem(a.width, kMmaTiles);
-  const cudaError_t e = cudaFuncSetAttribute(latent_attention_mma_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr int RB = MT * 16;
+  const size_t smem = latent_mma_smem(a.width, MT);
+  const cudaError_t e = cudaFuncSetAttribute((latent_attention_mma_kernel<MT, R64>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  TIB_LAUNCH_DEPENDENT(latent_attention_mma_kernel<R64>, dim3(ceil_div(max_q_len * a.heads, kMmaTiles * 16), n_entries), kMmaWarps * 32, smem, stream,
-                       folded, (const __nv_bfloat16*)pool, out, a);
-  return TIB_OK;
+  const dim3 grid(a.partial ? a.n_splits : ceil_div(max_q_len * a.heads, RB), n_entries, a.partial ? ceil_div(a.heads, RB) : 1);
+  TIB_LAUNCH_DEPENDENT((latent_attention_mma_kernel<MT, R64>), grid, kMmaWarps * 32, smem, stream, folded, (const __nv_bfloat16*)pool, out, a);
+  return a.partial ? launch_latent_merge(out, a, n_entries, stream) : TIB_OK;
 }
 
 template <typename T, int DPL>
@@ -898,16 +916,24 @@ TIB_API int tib_latent_attention(const float* folded, const void* pool, float* o
   const int width = rank + rot;
   if (dtype == TIB_BF16 && !force_simt && width % 16 == 0 && rank % 64 == 0 && (page_stride % 8) == 0 && ((uintptr_t)pool & 15) == 0) {
     const int r64 = rank / 64;
-    const size_t smem = max_q_len == 1 ? latent_decode_smem(width) : latent_mma_smem(width, kMmaTiles);
-    if (smem <= 227 * 1024 && (r64 <= 4 || r64 == 6 || r64 == 8) && (((uintptr_t)folded | (uintptr_t)out) & 15) == 0 && ((uintptr_t)partial & 7) == 0) {
+    // Single tokens take the kernel of sixteen warps, whose scores need 17 KB beside the rows, up to rows of 720; wider ones (768 at most),
+    // and queries or rows off their boundaries, the portions' kernel with one m-tile.
+    const bool single = max_q_len == 1, decode = single && latent_decode_smem(width) <= 227 * 1024 &&
+                                                 (((uintptr_t)folded | (uintptr_t)out) & 15) == 0 && ((uintptr_t)partial & 7) == 0;
+    if (latent_mma_smem(width, single ? 1 : 2) <= 227 * 1024 && (r64 <= 4 || r64 == 6 || r64 == 8)) {
+#define TIB_LAT_TENSOR(R64)                                                                          \
+  (decode ? launch_latent_decode<R64>(folded, pool, out, a, n_entries, stream)                       \
+   : single ? launch_latent_mma<1, R64>(folded, pool, out, a, n_entries, max_q_len, stream)          \
+            : launch_latent_mma<2, R64>(folded, pool, out, a, n_entries, max_q_len, stream))
       switch (r64) {
-        case 1: return launch_latent_mma<1>(folded, pool, out, a, n_entries, max_q_len, stream);
-        case 2: return launch_latent_mma<2>(folded, pool, out, a, n_entries, max_q_len, stream);
-        case 3: return launch_latent_mma<3>(folded, pool, out, a, n_entries, max_q_len, stream);
-        case 4: return launch_latent_mma<4>(folded, pool, out, a, n_entries, max_q_len, stream);
-        case 6: return launch_latent_mma<6>(folded, pool, out, a, n_entries, max_q_len, stream);
-        default: return launch_latent_mma<8>(folded, pool, out, a, n_entries, max_q_len, stream);
+        case 1: return TIB_LAT_TENSOR(1);
+        case 2: return TIB_LAT_TENSOR(2);
+        case 3: return TIB_LAT_TENSOR(3);
+        case 4: return TIB_LAT_TENSOR(4);
+        case 6: return TIB_LAT_TENSOR(6);
+        default: return TIB_LAT_TENSOR(8);
       }
+#undef TIB_LAT_TENSOR
     }
   }
   const int dpl = (rank + 31) / 32;
