@@ -949,6 +949,16 @@ def test_fp32_product_in_three_terms(m, n, k, monkeypatch):
     assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf()) and not torch.isfinite(out[:, 7]).any()
 
 
+def test_fp32_products_of_expanded_weights():
+    """One row of weights for all features, and rows that overlap: what the kernel on multiply-adds makes of them."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    x, row = dev(rnd(5, 2048)), dev(rnd(2048 + 4 * 2047))
+    for w in (row[:2048].expand(2048, 2048), row.as_strided((2048, 2048), (4, 1))):
+        out = ops.gemm_f32(x, w, torch.empty(5, 2048, device="cuda"))
+        assert torch.equal(out[:, :512], ops.gemm_f32(x, w[:512].contiguous(), torch.empty(5, 512, device="cuda")))
+
+
 # ------------------------------------------------- linear attention in runs and token by token
 @pytest.mark.parametrize("lens, heads, key_dim, value_dim", [
     ([1, 1, 1], 3, 128, 128), ([32, 5, 9], 2, 64, 96),                        # token by token, to its longest portion

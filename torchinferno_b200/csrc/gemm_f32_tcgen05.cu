@@ -330,8 +330,10 @@ using namespace tib;
 // than the other kernel's one, are paid back on few rows too: a block of 512 x 512 weights on 20
 // tokens took 143 us there and 182 here, one of 1,024 x 1,024 and 1,024 x 2,112 on 40 139 and 150, one of 1,536 x 1,536 and 1,536 x 6,400 on
 // 100 503 and 299.
+// (Weights whose rows overlap or are one and the same are none of a tensor map's.)
 TIB_API int tib_gemm_f32_tcgen05_takes(const void* x, const void* w, int N, int K, int64_t ldx, int64_t ldw) {
-  return N >= 512 && K >= 512 && (int64_t)N * K >= (1 << 22) && K % kFtK == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+  return N >= 512 && K >= 512 && (int64_t)N * K >= (1 << 22) && K % kFtK == 0 && ldx % 4 == 0 && ldw % 4 == 0 && ldw >= K &&
+         (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
 }
 
 // x: [M, K] (row stride ldx), w: [N, K] (row stride ldw), out: [M, N] (row stride ldo), all fp32.  scratch: bf16, 3 K numbers for each
