@@ -949,6 +949,49 @@ def test_fp32_product_in_three_terms(m, n, k, monkeypatch):
     assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf()) and not torch.isfinite(out[:, 7]).any()
 
 
+def test_calls_of_different_sizes_from_several_threads():
+    """The shared memory that a kernel may take is the function's, not the thread's: one kernel at several sizes from several threads at once."""
+    need_gpu()
+    import threading
+    from torchinferno_b200.kernels import ops
+    w = dev(rnd(2048, 2048))
+    heads, dim = 4, 128
+    chunk = ops.linear_attention_chunk(dim, dim)
+    powers = dev((torch.tensor([0.9] * heads, dtype=torch.float64)[:, None] ** torch.arange(chunk + 1, dtype=torch.float64)).float().contiguous())
+
+    def product(m):
+        x = dev(rnd(m, 2048, seed=m))
+        return lambda: ops.gemm_f32(x, w, torch.empty(m, 2048, device="cuda"))
+
+    def linear(entries):      # (a block's columns, and its shared memory, go by the number of portions)
+        n = 40 * entries
+        rows, state = dev(rnd(n, 3 * heads * dim, seed=entries)), dev(rnd(entries, heads, dim, dim))
+        starts, slots = dev(40 * torch.arange(entries + 1, dtype=torch.int32)), dev(torch.arange(entries, dtype=torch.int32))
+        q, k, v = rows.chunk(3, 1)
+        return lambda: ops.linear_attention(q, k, v, torch.empty(n, heads * dim, device="cuda"), state.clone(), powers, starts, slots, entries, heads, dim, dim,
+                                            silu=True, max_q_len=40)
+
+    calls = [product(m) for m in (8, 48, 80, 300)] + [linear(entries) for entries in (8, 40)]
+    want, faults = [call() for call in calls], []
+    torch.cuda.synchronize()
+
+    def work(call, ref):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(300):
+                    out = call()
+                assert torch.equal(out, ref)
+        except Exception as error:
+            faults.append(error)
+
+    threads = [threading.Thread(target=work, args=pair) for pair in zip(calls, want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not faults, faults
+
+
 def test_fp32_products_of_expanded_weights():
     """One row of weights for all features, and rows that overlap: what the kernel on multiply-adds makes of them."""
     need_gpu()

@@ -250,7 +250,7 @@ static int launch_attention_rows(const void* q, const void* pool, void* out, Att
   if (smem > 227 * 1024) return TIB_E_SMEM;
   auto kern = paged_attention_simt_kernel<T, DPL, R, VEC>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
     if (e != cudaSuccess) return (int)e;
   }
   dim3 grid(ceil_div(max_q_len, a.q_tile), n_entries, a.kv_heads * chunks);

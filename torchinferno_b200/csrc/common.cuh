@@ -40,6 +40,10 @@ enum TibRequestRecord : int {
   TIB_REC_WORDS = 8,        // (two words spare)
 };
 
+// What a block may have of shared memory, static and dynamic.  A kernel whose dynamic part depends on the call is allowed all of it (the limit is
+// the function's, one for all threads: set to each call's size, it could be lowered between another thread's setting and its launch).
+constexpr int kMostSmem = 227 * 1024;
+
 // kernel<<<grid, block, smem, stream>>>(args) as a programmatic dependent launch (see launch_dependent below)
 #define TIB_LAUNCH_DEPENDENT(kernel, grid, block, smem, stream, ...)                                              \
   do {                                                                                                            \

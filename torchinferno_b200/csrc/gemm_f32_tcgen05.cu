@@ -369,7 +369,7 @@ TIB_API int tib_gemm_f32_tcgen05(const float* x, const float* w, float* out, int
     int rc = ft_weight_map(&map_w, w, N, K, ldw);
     if (rc == TIB_OK) rc = make_map(&map, scratch, 3 * rows, K, K, best);
     if (rc != TIB_OK) return rc;
-    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
     if (e != cudaSuccess) return (int)e;
     const int64_t blocks = ceil_div64((int64_t)rows * K / 4, 256);
     TIB_LAUNCH_DEPENDENT(split_rows_kernel, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, a.x, ldx, rows, K, (__nv_bfloat16*)scratch);

@@ -804,7 +804,7 @@ static int launch_latent_merge(float* out, const LatentAttnArgs& a, int n_entrie
 template <int R64>
 static int launch_latent_decode(const float* folded, const void* pool, float* out, const LatentAttnArgs& a, int n_entries, cudaStream_t stream) {
   const size_t smem = latent_decode_smem(a.width);
-  const cudaError_t e = cudaFuncSetAttribute(latent_decode_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = cudaFuncSetAttribute(latent_decode_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   if (e != cudaSuccess) return (int)e;
   TIB_LAUNCH_DEPENDENT(latent_decode_kernel<R64>, dim3(a.partial ? a.n_splits : 1, n_entries, ceil_div(a.heads, 16)), kLdThreads, smem, stream,
                        folded, (const __nv_bfloat16*)pool, out, a);
@@ -816,7 +816,7 @@ static int launch_latent_mma(const float* folded, const void* pool, float* out, 
                              cudaStream_t stream) {
   constexpr int RB = MT * 16;
   const size_t smem = latent_mma_smem(a.width, MT);
-  const cudaError_t e = cudaFuncSetAttribute((latent_attention_mma_kernel<MT, R64>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = cudaFuncSetAttribute((latent_attention_mma_kernel<MT, R64>), cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   if (e != cudaSuccess) return (int)e;
   const dim3 grid(a.partial ? a.n_splits : ceil_div(max_q_len * a.heads, RB), n_entries, a.partial ? ceil_div(a.heads, RB) : 1);
   TIB_LAUNCH_DEPENDENT((latent_attention_mma_kernel<MT, R64>), grid, kMmaWarps * 32, smem, stream, folded, (const __nv_bfloat16*)pool, out, a);
@@ -830,7 +830,7 @@ static int launch_latent_attention(const float* folded, const void* pool, float*
   if (smem > 227 * 1024) return TIB_E_SMEM;
   auto kern = latent_attention_kernel<T, DPL>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
     if (e != cudaSuccess) return (int)e;
   }
   dim3 grid(a.partial ? a.n_splits : ceil_div(max_q_len, a.q_tile), n_entries, ceil_div(a.heads, a.head_chunk));

@@ -441,14 +441,14 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   if (dtype == TIB_F32) {
     auto kern = linear_attention_kernel<float>;
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
       if (e != cudaSuccess) return (int)e;
     }
     TIB_LAUNCH_DEPENDENT(kern, grid, 256, smem, stream, (const float*)q, (const float*)k, (const float*)v, a);
   } else if (dtype == TIB_BF16) {
     auto kern = linear_attention_kernel<__nv_bfloat16>;
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
       if (e != cudaSuccess) return (int)e;
     }
     TIB_LAUNCH_DEPENDENT(kern, grid, 256, smem, stream, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
