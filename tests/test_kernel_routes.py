@@ -1,7 +1,13 @@
-"""The host's rules on which kernel a call takes: no GPU needed, only the library."""
+"""What can be said of the kernels without a GPU: the host's rules on which one a call takes, and rules that their sources keep."""
+import re
 from ctypes import c_int, c_int64, c_void_p
+from pathlib import Path
 
 import pytest
+
+import torchinferno_b200
+
+CSRC = Path(torchinferno_b200.__file__).parent / "csrc"
 
 
 @pytest.mark.parametrize("n, k, ldx, ldw, x, w, takes", [
@@ -13,3 +19,12 @@ import pytest
 def test_which_32_bit_products_run_on_tensor_cores(n, k, ldx, ldw, x, w, takes):
     from torchinferno_b200.kernels.library import load_library
     assert bool(load_library().tib_gemm_f32_tcgen05_takes(c_void_p(x), c_void_p(w), c_int(n), c_int(k), c_int64(ldx), c_int64(ldw))) == takes
+
+
+def test_a_timeout_code_names_one_kernel():
+    """The first digit behind 0x7C00 belongs to one file, as the list in tcgen05.cuh says."""
+    listed = {digit: name for digits, name in re.findall(r"((?:[0-9A-F], )*[0-9A-F]) (\w+?_\w+)", (CSRC / "tcgen05.cuh").read_text().split("first digit of xx:")[1].split("// Bounded")[0])
+              for digit in digits.split(", ")}
+    used = {(code, path.stem) for path in CSRC.glob("*.cu") for code in re.findall(r"0x7C00([0-9A-F])[0-9A-F]\b", path.read_text())}
+    assert used and {code for code, _ in used} == set(listed)
+    assert all(listed[code] == name for code, name in used), used

@@ -126,7 +126,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     const uint32_t dst = tmem_base + ((uint32_t)(quarter * 32) << 16) + part * 8;
     for (int it = 0; it < total; ++it) {
       if (!mbar_wait(w_full_bar(ws), wphase)) {
-        if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0071);
+        if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0091);
         break;
       }
       const unsigned char* src = smem_gen + (size_t)ws * kFtW + (part >> 1) * (kFtW / 2) + r * 128;
@@ -141,7 +141,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       if (lane == 0) mbar_arrive(w_empty_bar(ws));
       if (it >= 2) {      // (the products of two steps ago are done)
         if (!mbar_wait(x_empty_bar(before), bphase)) {
-          if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0076);
+          if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0096);
           break;
         }
         if (++before == a.x_stages) {
@@ -178,7 +178,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             ok = mbar_wait(x_empty_bar(xs), xphase);
           }
           if (!ok) {
-            if (a.error_word) atomicExch(a.error_word, 0x7C0072);
+            if (a.error_word) atomicExch(a.error_word, 0x7C0092);
             break;
           }
           mbar_expect_tx(x_full_bar(xs), 3 * xplane);
@@ -207,7 +207,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         const int ab = chunk & 1;
         const bool free = mbar_wait(acc_empty_bar(ab), ((chunk >> 1) & 1) ^ 1) && (ks > 0 || mbar_wait(small_empty_bar, (tile & 1) ^ 1));
         if (!__all_sync(0xffffffffu, free)) {
-          if (a.error_word && leader) atomicExch(a.error_word, 0x7C0074);
+          if (a.error_word && leader) atomicExch(a.error_word, 0x7C0094);
           ok = false;
           break;
         }
@@ -215,7 +215,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         for (int kc = 0; kc < kFtChunk && ks + kc < k_steps && ok; ++kc, ++it) {
           const uint32_t xs = xring + s * 3 * xplane, wt = tmem_base + (it & 1) * kFtTermCols;
           if (!__all_sync(0xffffffffu, mbar_wait(x_full_bar(s), phase))) {
-            if (a.error_word && leader) atomicExch(a.error_word, 0x7C0073);
+            if (a.error_word && leader) atomicExch(a.error_word, 0x7C0093);
             ok = false;
             break;
           }
@@ -251,7 +251,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       for (int ks = 0; ks < k_steps; ks += kFtChunk, ++chunk) {
         const int b = chunk & 1;
         if (!mbar_wait(acc_full_bar(b), (chunk >> 1) & 1)) {
-          if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0075);
+          if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0095);
           ok = false;
           break;
         }

@@ -132,7 +132,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
           const int s = it % kT2Stages;
           const uint32_t phase = (it / kT2Stages) & 1;
           if (!mbar_wait(empty_bar(s), phase ^ 1)) {
-            if (error_word) atomicExch(error_word, 0x7C0041);
+            if (error_word) atomicExch(error_word, 0x7C0051);
             ok = false;
             break;
           }
@@ -153,7 +153,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         const int b = j & 1;
         const uint32_t tmem_acc = tmem_base + b * kT2AccStride;
         if (!t2_wait_cluster(acc_empty_bar(b), ((j >> 1) & 1) ^ 1)) {   // both epilogues have drained this accumulator
-          if (error_word) atomicExch(error_word, 0x7C0044);
+          if (error_word) atomicExch(error_word, 0x7C0054);
           ok = false;
           break;
         }
@@ -162,7 +162,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
           const int s = it % kT2Stages;
           const uint32_t phase = (it / kT2Stages) & 1;
           if (!t2_wait_cluster(full_bar(s), phase)) {
-            if (error_word) atomicExch(error_word, 0x7C0042);
+            if (error_word) atomicExch(error_word, 0x7C0052);
             ok = false;
             break;
           }
@@ -184,7 +184,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       const int b = j & 1;
       const int row = m0 + quarter * 32 + lane;
       if (!mbar_wait(acc_full_bar(b), (j >> 1) & 1)) {
-        if (error_word && lane == 0) atomicExch(error_word, 0x7C0043);
+        if (error_word && lane == 0) atomicExch(error_word, 0x7C0053);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");

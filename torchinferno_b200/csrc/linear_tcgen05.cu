@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
     if (leader) umma_commit(bar);
     __syncwarp();
   }
-  ft_wait(bar, 0, a.error_word, 0x7C0081);
+  ft_wait(bar, 0, a.error_word, 0x7C00A1);
   const int quarter = warp & 3, part = warp >> 2, d = quarter * 32 + lane;
   const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + part * (TV / 4);
   float* dst = a.run_state + (b.run * a.n_heads + b.own) * (size_t)D * a.value_dim + (size_t)d * a.value_dim + b.col0 + part * (TV / 4);
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     held[i][0] = src[0];
     held[i][1] = src[1];
   }
-  ft_wait(bar, 0, a.error_word, 0x7C0082);
+  ft_wait(bar, 0, a.error_word, 0x7C00A2);
 #pragma unroll
   for (int i = 0; i < SV; ++i) {
     const int p = tid + i * kLtThreads;
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     }
     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
   }
-  ft_wait(bar + 8, 0, a.error_word, 0x7C0083);
+  ft_wait(bar + 8, 0, a.error_word, 0x7C00A3);
   float sum[TV / 4];
   const float decay = pw[i + 1];
 #pragma unroll
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     if (leader) umma_commit(bar + 16);
     __syncwarp();
   }
-  ft_wait(bar + 16, 0, a.error_word, 0x7C0084);
+  ft_wait(bar + 16, 0, a.error_word, 0x7C00A4);
 #pragma unroll
   for (int c0 = 0; c0 < TV / 4; c0 += 16) {
     uint32_t x[16], y[16];

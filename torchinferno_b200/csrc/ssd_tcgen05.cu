@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_sums_tcgen05_kernel(ScanArg
     }
     if (it + 1 < b.items) put(it + 1);
     if (it + 2 < b.items) x.ask(rows + b.head(a, it + 2) * a.P + b.column(it + 2), a.ld_xbc, b.n);
-    ft_wait(bar, it & 1, a.error_word, 0x7C0085);
+    ft_wait(bar, it & 1, a.error_word, 0x7C00B1);
     const int h = b.head(a, it);
     float sum[16];
 #pragma unroll
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
         if (leader) umma_commit(bar);
         __syncwarp();
       }
-      ft_wait(bar, (k0 >> 2) & 1, a.error_word, 0x7C0086);
+      ft_wait(bar, (k0 >> 2) & 1, a.error_word, 0x7C00B2);
       if (part <= quarter) {
 #pragma unroll
         for (int k = 0; k < 4; k += 2)
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
       }
       asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
     }
-    ft_wait(bar + 8, it & 1, a.error_word, 0x7C0087);
+    ft_wait(bar + 8, it & 1, a.error_word, 0x7C00B3);
     float sum[16];
     const auto add_up = [&](float (&sum)[16]) {      // the five accumulators of the warp's columns, small terms first
 #pragma unroll
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
       __syncwarp();
     }
     if (it + 1 < b.items) put(it + 1);
-    ft_wait(bar + 16, it & 1, a.error_word, 0x7C0088);
+    ft_wait(bar + 16, it & 1, a.error_word, 0x7C00B4);
     {
       float own[16];
       add_up(own);

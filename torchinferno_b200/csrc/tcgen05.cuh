@@ -23,6 +23,9 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
+// The codes that a wait leaves in the error word when it runs out, 0x7C00xx, name its kernel by the first digit of xx:
+//   0, 1 gemm_tcgen05   2 attention_tcgen05   3 attention_decode_tma   4 gemm_decode    5 gemm_tcgen05_2cta   6 moe_tcgen05
+//   7 latent_prefill    8 window_tcgen05      9 gemm_f32_tcgen05       A linear_tcgen05   B ssd_tcgen05
 // Bounded wait: false when the limit was reached (the caller records it and gives up).  Each try blocks
 // in hardware for up to about a microsecond (the suspend-time hint), so a waiting role takes no issue
 // slots from the warps that share its scheduler; 2^18 tries bound the whole wait to a fraction of a second.
