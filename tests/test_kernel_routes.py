@@ -28,3 +28,14 @@ def test_a_timeout_code_names_one_kernel():
     used = {(code, path.stem) for path in CSRC.glob("*.cu") for code in re.findall(r"0x7C00([0-9A-F])[0-9A-F]\b", path.read_text())}
     assert used and {code for code, _ in used} == set(listed)
     assert all(listed[code] == name for code, name in used), used
+
+
+@pytest.mark.parametrize("path", sorted(CSRC.glob("*.cu")), ids=lambda p: p.stem)
+def test_dependents_are_let_in_once_tensor_memory_is_taken(path):
+    """A kernel that takes tensor memory lets the next kernel's blocks in only behind that: one that was placed first, had the columns and waited for
+    this kernel's end would never get it.  The products of few rows take half of the columns at most, so that two blocks have room."""
+    for kernel in re.split(r"(?=__global__ void)", path.read_text())[1:]:
+        taken = [m.start() for m in re.finditer(r"ft_setup\(|tcgen05\.alloc", kernel)]
+        let_in = kernel.find("pdl_trigger()")
+        if taken and let_in >= 0 and path.stem not in ("gemm_decode", "gemm_tcgen05"):
+            assert let_in > taken[0], kernel.split("(", 3)[:3]

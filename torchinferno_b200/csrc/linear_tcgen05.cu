@@ -160,12 +160,12 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
   unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   pdl_wait();
-  pdl_trigger();
   LtBlock b;
   if (!lt_block<TV>(a, b)) return;
   const uint32_t bar = base + 3 * (S::kKeyTerm + S::kValueTerm);
   if (threadIdx.x <= kLinRun) pw[threadIdx.x] = a.powers[b.head * (kLinRun + 1) + threadIdx.x];
   const uint32_t tmem = ft_setup(bar, 1, bar + 8, reinterpret_cast<volatile uint32_t*>(smem + (bar + 8 - base)), warp, S::kColumns);
+  pdl_trigger();
   const size_t first = (size_t)(b.row0 + b.t0);
   LtRows<T, D> keys_of;
   LtRows<T, TV> values_of;
@@ -266,7 +266,6 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
   unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   pdl_wait();
-  pdl_trigger();
   LtBlock b;
   if (!lt_block<TV>(a, b)) return;
   const uint32_t bar = base + S::kFirst + S::kSecond;
@@ -274,6 +273,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
   if (tid == 0) odd = 0;
   // tensor memory: scores (two accumulators), later their three terms; carried, later inside
   const uint32_t tmem = ft_setup(bar, 3, bar + 24, reinterpret_cast<volatile uint32_t*>(smem + (bar + 24 - base)), warp, 512);
+  pdl_trigger();
   const size_t first = (size_t)(b.row0 + b.t0);
   const uint32_t one = base, two = base + S::kFirst;
   {

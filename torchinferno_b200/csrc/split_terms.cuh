@@ -88,6 +88,8 @@ __device__ __forceinline__ void ft_store8(float* dst, const float (&v)[8]) {    
 }
 
 // Barriers that one commit completes, and `columns` columns of tensor memory; called by the whole block, with a barrier of the block behind it.
+// pdl_trigger() comes after it: a block of the next kernel that is placed before this one has its columns could take them, and wait for this
+// kernel's end with them.
 __device__ __forceinline__ uint32_t ft_setup(uint32_t bar0, int bars, uint32_t slot, volatile uint32_t* slot_ptr, int warp, uint32_t columns) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < bars; ++i) mbar_init(bar0 + 8 * i, 1);

@@ -154,7 +154,6 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_sums_tcgen05_kernel(ScanArg
   unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   pdl_wait();
-  pdl_trigger();
   StBlock b;
   if (!st_block(a, per_block, b)) return;
   const uint32_t bar = base + S::kB + 2 * S::kX, xs = base + S::kB;
@@ -164,6 +163,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_sums_tcgen05_kernel(ScanArg
   StX x;
   x.ask(rows + b.head(a, 0) * a.P + b.column(0), a.ld_xbc, b.n);
   const uint32_t tmem = ft_setup(bar, 1, bar + 8, reinterpret_cast<volatile uint32_t*>(smem + (bar + 8 - base)), warp, 512);
+  pdl_trigger();
   if (warp < b.items) st_steps<true>(steps[warp], a, b, b.head(a, warp), lane);
   cp_async_wait<0>();
   __syncthreads();
@@ -253,7 +253,6 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
   unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   pdl_wait();
-  pdl_trigger();
   StBlock b;
   if (!st_block(a, per_block, b)) return;
   const size_t first = (size_t)(b.row0 + b.t0);
@@ -307,6 +306,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
   if (tid < kStItems) odd[tid] = 0;
   const uint32_t bar = base + S::kBars;
   const uint32_t tmem = ft_setup(bar, 3, bar + 24, reinterpret_cast<volatile uint32_t*>(smem + S::kBars + 24), warp, 512);
+  pdl_trigger();
   if (warp < b.items) st_steps<false>(steps[warp], a, b, b.head(a, warp), lane);
   put(0);
   cp_async_wait<0>();
