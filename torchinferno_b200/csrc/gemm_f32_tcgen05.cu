@@ -196,7 +196,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       }
     }
   } else if (warp == 17) {
-    const uint32_t leader = ft_elect(), idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFtM >> 4) << 24);
+    const uint32_t leader = umma_leader(), idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFtM >> 4) << 24);
     const uint32_t n1 = (uint32_t)(a.rows >> 4) << 18;      // (an instruction's columns, in sixteens)
     int s = 0;
     uint32_t phase = 0, chunk = 0, it = 0, tile = 0;
@@ -222,12 +222,12 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
           for (int k = 0; k < kFtK / 16; ++k) {
-            const uint64_t x0 = umma_desc_k128(xs + k * 32), x1 = umma_desc_k128(xs + xplane + k * 32);
+            const uint32_t x0 = umma_low_k128(xs + k * 32), x1 = umma_low_k128(xs + xplane + k * 32);
             const uint32_t w0 = wt + k * 8, w1 = w0 + kFtK / 2, w2 = w1 + kFtK / 2;
-            ft_mma(leader, small, w0, x1, idesc0 | 2 * n1, (ks | kc | k) != 0);
-            ft_mma(leader, small, w1, x0, idesc0 | 2 * n1, 1);
-            ft_mma(leader, small + a.rows, w2, x0, idesc0 | n1, 1);
-            ft_mma(leader, large, w0, x0, idesc0 | n1, (kc | k) != 0);
+            umma_warp_tmem(leader, small, w0, x1, idesc0 | 2 * n1, (ks | kc | k) != 0);
+            umma_warp_tmem(leader, small, w1, x0, idesc0 | 2 * n1, 1);
+            umma_warp_tmem(leader, small + a.rows, w2, x0, idesc0 | n1, 1);
+            umma_warp_tmem(leader, large, w0, x0, idesc0 | n1, (kc | k) != 0);
           }
           if (leader) umma_commit(x_empty_bar(s));
           if (++s == a.x_stages) {

@@ -100,19 +100,19 @@ __device__ __forceinline__ void lt_products(uint32_t leader, uint32_t d, uint32_
   const uint32_t last = d + (ACC - 1) * columns;
 #pragma unroll
   for (int k = 0; k < STEPS; ++k) {
-    ft_mma_shared(leader, last, a(0, k), b(2, k), idesc, k != 0);
-    ft_mma_shared(leader, last, a(1, k), b(1, k), idesc, 1);
-    ft_mma_shared(leader, last, a(2, k), b(0, k), idesc, 1);
+    umma_warp(leader, last, a(0, k), b(2, k), idesc, k != 0);
+    umma_warp(leader, last, a(1, k), b(1, k), idesc, 1);
+    umma_warp(leader, last, a(2, k), b(0, k), idesc, 1);
   }
 #pragma unroll
   for (int k = 0; k < STEPS; ++k) {
-    ft_mma_shared(leader, last, a(0, k), b(1, k), idesc, 1);
-    ft_mma_shared(leader, last, a(1, k), b(0, k), idesc, 1);
+    umma_warp(leader, last, a(0, k), b(1, k), idesc, 1);
+    umma_warp(leader, last, a(1, k), b(0, k), idesc, 1);
   }
 #pragma unroll
   for (int k = 0; k < STEPS; ++k) {
     const int share = k * ACC / STEPS;
-    ft_mma_shared(leader, d + share * columns, a(0, k), b(0, k), idesc, share == ACC - 1 || k % (STEPS / ACC) != 0);
+    umma_warp(leader, d + share * columns, a(0, k), b(0, k), idesc, share == ACC - 1 || k % (STEPS / ACC) != 0);
   }
 }
 
@@ -179,12 +179,12 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_sums_kernel(const T* __
   values_of.put(smem + 3 * S::kKeyTerm, a.activation, [](int, float (&)[8]) {});
   ft_hand_over();
   if (warp == 0) {
-    const uint32_t leader = ft_elect();
+    const uint32_t leader = umma_leader();
     // both operands have the tokens as rows (of heads of 64 the upper half of the 128 rows is the next tile's, and never stored)
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(TV >> 3) << 17) | (8u << 24);
     const uint32_t keys = base, values = base + 3 * S::kKeyTerm;
-    lt_products<kLinRun / 16, ACC>(leader, tmem, TV, idesc, [&](int p, int s) { return umma_desc_mn128(keys + p * S::kKeyTerm + s * 2048, kLtSub); },
-                              [&](int p, int s) { return umma_desc_mn128(values + p * S::kValueTerm + s * 2048, kLtSub); });
+    lt_products<kLinRun / 16, ACC>(leader, tmem, TV, idesc, [&](int p, int s) { return umma_low_mn128(keys + p * S::kKeyTerm + s * 2048, kLtSub); },
+                              [&](int p, int s) { return umma_low_mn128(values + p * S::kValueTerm + s * 2048, kLtSub); });
     if (leader) umma_commit(bar);
     __syncwarp();
   }
@@ -284,10 +284,10 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
     rows_k.put(smem + S::kFirst, a.activation, [](int, float (&)[8]) {});
   }
   ft_hand_over();
-  const uint32_t leader = warp == 0 ? ft_elect() : 0;
+  const uint32_t leader = warp == 0 ? umma_leader() : 0;
   if (warp == 0) {
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kLinRun >> 3) << 17) | (8u << 24);
-    const auto at = [](uint32_t tile, int p, int s) { return umma_desc_k128(tile + p * S::kKeyTerm + (s >> 2) * kLtSub + (s & 3) * 32); };
+    const auto at = [](uint32_t tile, int p, int s) { return umma_low_k128(tile + p * S::kKeyTerm + (s >> 2) * kLtSub + (s & 3) * 32); };
     lt_products<D / 16, 2>(leader, tmem, 128, idesc, [&](int p, int s) { return at(one, p, s); }, [&](int p, int s) { return at(two, p, s); });
     if (leader) umma_commit(bar);
     __syncwarp();
@@ -314,8 +314,8 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
   constexpr uint32_t idesc_v = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(TV >> 3) << 17) | (8u << 24);
   if (warp == 0) {
     lt_products<D / 16, 2>(leader, carried, TV, idesc_v,
-                        [&](int p, int s) { return umma_desc_k128(one + p * S::kKeyTerm + (s >> 2) * kLtSub + (s & 3) * 32); },
-                        [&](int p, int s) { return umma_desc_mn128(two + p * S::kStateTerm + s * 2048, D * 128); });
+                        [&](int p, int s) { return umma_low_k128(one + p * S::kKeyTerm + (s >> 2) * kLtSub + (s & 3) * 32); },
+                        [&](int p, int s) { return umma_low_mn128(two + p * S::kStateTerm + s * 2048, D * 128); });
     if (leader) umma_commit(bar + 8);
     __syncwarp();
   }
@@ -376,21 +376,21 @@ __global__ void __launch_bounds__(kLtThreads, 1) lin_run_outs_kernel(const T* __
   ft_hand_over();
   if (warp == 0) {
     // (the weighted scores: tensor memory, 64 columns a term)
-    const auto b_at = [&](int p, int s) { return umma_desc_mn128(one + p * S::kValueTerm + s * 2048, kLtSub); };
+    const auto b_at = [&](int p, int s) { return umma_low_mn128(one + p * S::kValueTerm + s * 2048, kLtSub); };
     const uint32_t d0 = carried, d1 = carried + TV;
 #pragma unroll
     for (int s = 0; s < kLinRun / 16; ++s) {
-      ft_mma(leader, d1, tmem + s * 8, b_at(2, s), idesc_v, s != 0);
-      ft_mma(leader, d1, tmem + 64 + s * 8, b_at(1, s), idesc_v, 1);
-      ft_mma(leader, d1, tmem + 128 + s * 8, b_at(0, s), idesc_v, 1);
+      umma_warp_tmem(leader, d1, tmem + s * 8, b_at(2, s), idesc_v, s != 0);
+      umma_warp_tmem(leader, d1, tmem + 64 + s * 8, b_at(1, s), idesc_v, 1);
+      umma_warp_tmem(leader, d1, tmem + 128 + s * 8, b_at(0, s), idesc_v, 1);
     }
 #pragma unroll
     for (int s = 0; s < kLinRun / 16; ++s) {
-      ft_mma(leader, d1, tmem + s * 8, b_at(1, s), idesc_v, 1);
-      ft_mma(leader, d1, tmem + 64 + s * 8, b_at(0, s), idesc_v, 1);
+      umma_warp_tmem(leader, d1, tmem + s * 8, b_at(1, s), idesc_v, 1);
+      umma_warp_tmem(leader, d1, tmem + 64 + s * 8, b_at(0, s), idesc_v, 1);
     }
 #pragma unroll
-    for (int s = 0; s < kLinRun / 16; ++s) ft_mma(leader, s < kLinRun / 32 ? d0 : d1, tmem + s * 8, b_at(0, s), idesc_v, s != 0);
+    for (int s = 0; s < kLinRun / 16; ++s) umma_warp_tmem(leader, s < kLinRun / 32 ? d0 : d1, tmem + s * 8, b_at(0, s), idesc_v, s != 0);
     if (leader) umma_commit(bar + 16);
     __syncwarp();
   }

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_sums_tcgen05_kernel(ScanArg
   };
   put(0);
   if (b.items > 1) x.ask(rows + b.head(a, 1) * a.P + b.column(1), a.ld_xbc, b.n);
-  const uint32_t leader = warp == 0 ? ft_elect() : 0;
+  const uint32_t leader = warp == 0 ? umma_leader() : 0;
   const int quarter = warp & 3, part = warp >> 2, state_row = quarter * 32 + lane;
   for (int it = 0; it < b.items; ++it) {
     ft_hand_over();
@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_sums_tcgen05_kernel(ScanArg
 #pragma unroll
       for (int k = 0; k < kQ / 16; ++k) {
         const uint64_t rows_b = umma_desc_mn128(base + k * 2048, kStSub);
-        ft_mma_shared(leader, tmem, rows_b, umma_desc_mn128(tile + kStSub + k * 2048, kStSub), idesc | ((128u >> 3) << 17), k != 0);
-        ft_mma_shared(leader, tmem + 128 + (k >> 1) * 64, rows_b, umma_desc_mn128(tile + k * 2048, kStSub), idesc | ((64u >> 3) << 17), (k & 1) != 0);
+        umma_warp(leader, tmem, rows_b, umma_desc_mn128(tile + kStSub + k * 2048, kStSub), idesc | ((128u >> 3) << 17), k != 0);
+        umma_warp(leader, tmem + 128 + (k >> 1) * 64, rows_b, umma_desc_mn128(tile + k * 2048, kStSub), idesc | ((64u >> 3) << 17), (k & 1) != 0);
       }
       if (leader) umma_commit(bar);
       __syncwarp();
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
   if (warp < b.items) st_steps<false>(steps[warp], a, b, b.head(a, warp), lane);
   put(0);
   cp_async_wait<0>();
-  const uint32_t leader = warp == 0 ? ft_elect() : 0;
+  const uint32_t leader = warp == 0 ? umma_leader() : 0;
   // token i: a lane; the warp's fourth of the tokens before it, then of the columns
   const int quarter = warp & 3, part = warp >> 2, i = quarter * 32 + lane;
   const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kQ >> 3) << 17) | (8u << 24);
 #pragma unroll
         for (int k = k0; k < k0 + 4; ++k)
-          ft_mma_shared(leader, tmem + (k - k0) * 128, c_at(k), umma_desc_k128(base + S::kB + (k >> 2) * kStSub + (k & 3) * 32), idesc, 0);
+          umma_warp(leader, tmem + (k - k0) * 128, c_at(k), umma_desc_k128(base + S::kB + (k >> 2) * kStSub + (k & 3) * 32), idesc, 0);
         if (leader) umma_commit(bar);
         __syncwarp();
       }
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
       for (int u = 2; u >= 0; --u)
 #pragma unroll
         for (int k = 0; k < STEPS; ++k)
-          ft_mma_shared(leader, u == 0 ? wide + k * 4 / STEPS * 64 : small, c_at(k), umma_desc_mn128(base + S::kState + u * S::kTerm + k * 2048, N * 128), idesc_v,
+          umma_warp(leader, u == 0 ? wide + k * 4 / STEPS * 64 : small, c_at(k), umma_desc_mn128(base + S::kState + u * S::kTerm + k * 2048, N * 128), idesc_v,
                         u == 0 ? k % (STEPS / 4) != 0 : !(u == 2 && k == 0));
       if (leader) umma_commit(bar + 8);
       __syncwarp();
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_outs_tcgen05_kernel(ScanArg
 #pragma unroll
         for (int k = 0; k < kQ / 16; ++k) {
           const uint32_t to = u == 0 ? wide + k / 2 * 64 : small;
-          ft_mma(leader, to, tmem + u * 64 + k * 8, umma_desc_mn128(base + tile + k * 2048, kStSub), idesc_v, u == 0 ? k % 2 != 0 : !(u == 2 && k == 0));
+          umma_warp_tmem(leader, to, tmem + u * 64 + k * 8, umma_desc_mn128(base + tile + k * 2048, kStSub), idesc_v, u == 0 ? k % 2 != 0 : !(u == 2 && k == 0));
         }
       if (leader) umma_commit(bar + 16);
       __syncwarp();

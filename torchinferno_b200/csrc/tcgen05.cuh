@@ -91,12 +91,6 @@ __device__ __forceinline__ void umma_f16_idesc(uint32_t tmem_d, uint64_t adesc, 
                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
                ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// The same product with the A operand in tensor memory (lane = row, two bf16 of consecutive k per 32-bit column).
-__device__ __forceinline__ void umma_f16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
                "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n"
@@ -129,8 +123,9 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 }
 
 // ----- products issued by a whole warp.  The warp walks its loop together and one lane, elected once, issues: operands then stay in uniform
-// registers.  (Measured, cycles an instruction while the tensor core is not the limit: 37 to 46, a lone lane 52 to 55; a phase that is over costs
-// the lone lane's wait 233, this one some 60.)
+// registers.  Measured, cycles an instruction: of 128 x 16 x 16 products one behind the other, which take the tensor core 10, 8 where a lone lane
+// takes 45; in the loops of attention and of the experts' products, with their waits and commits counted in, 37 to 46 where it takes 52 to 55.  A
+// phase that is over costs the lone lane's wait 233, this one some 60.
 __device__ __forceinline__ uint32_t umma_leader() {
   uint32_t one;
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
@@ -150,11 +145,23 @@ __device__ __forceinline__ void umma_warp(uint32_t leader, uint32_t tmem_d, uint
                "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
                ::"r"(tmem_d), "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(leader), "r"(kUmmaDescHigh) : "memory");
 }
-// The same with the A operand in tensor memory.
+// The same with the A operand in tensor memory (lane = row, two bf16 of consecutive k per 32-bit column).
 __device__ __forceinline__ void umma_warp_tmem(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n.reg .pred p, q;\n.reg .b64 b;\nmov.b64 b, {%2, %6};\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
                "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n"
                ::"r"(tmem_d), "r"(tmem_a), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(leader), "r"(kUmmaDescHigh) : "memory");
+}
+
+// Both with whole descriptors (the scan, at its limit of registers, is 1.2 us in 230 faster with them).
+__device__ __forceinline__ void umma_warp(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void umma_warp_tmem(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
