@@ -934,6 +934,10 @@ def test_fp32_product_in_three_terms(m, n, k, monkeypatch):
     # fp32, and the terms left out are below 2 * 2^-24 of a product: 2^-23 (8 + k / 256 + 1) of the products' magnitudes, and one for the small terms.
     bound = 2.0 ** -23 * (10 + k / 256) * (x.double().abs() @ w.double().abs().T)
     assert ((out.double() - x.double() @ w.double().T).abs() <= bound).all() and int(error) == 0
+    # Seen: 1.4e-7 to 2.4e-7 of the result's 2-norm.  Without one of the three small groups of products it would be 1.3e-6 (a1 b1: two numbers of 2^-9
+    # of theirs, evenly spread) or 2.5e-6 (a2 b0, a0 b2: one of 2^-17) or more.
+    exact = x.double() @ w.double().T
+    assert (out.double() - exact).norm() <= 4e-7 * exact.norm()
     for rows in (slice(m // 2, m // 2 + 1), slice(0, max(1, m - 3))):      # a row does not depend on the rows beside it
         few = x[rows].contiguous()
         assert torch.equal(ops.gemm_f32(few, w, torch.empty(len(few), n, device="cuda")), out[rows])
@@ -1039,8 +1043,9 @@ def test_linear_attention_forms_agree_with_the_recurrence(lens, heads, key_dim, 
             s = decay[:, None, None] * s + k[t][:, :, None] * v[t][:, None, :]
             want[t] = torch.einsum("hkv,hk->hv", s, q[t])
         want_state[slots[e]] = s
-    # fp32 throughout: every output is a sum of at most key_dim + 64 products a run, each rounded once (2^-24), and the
-    # sums' magnitude is at most about sqrt(terms) times the outputs'; 2e-6 is 32 roundings of the largest value
+    # Walk and chunks round every product of key_dim + 32 once (2^-24 of the sum).  In runs every number enters with 24 bits, what is left out of a product is
+    # below 2^-24 of it, and the tensor core cuts off at most 2^-23 of a sum at each of an accumulator's 8 instructions; the last sums are fp32.  2e-6 is
+    # 16 such cuts of the largest value.
     assert (as_ref(out) - want.reshape(n, -1)).abs().max() <= 2e-6 * want.abs().max()
     assert (as_ref(got_state) - want_state).abs().max() <= 2e-6 * want_state.abs().max()
 
@@ -1103,6 +1108,35 @@ def test_linear_attention_in_runs_has_the_same_bits_in_tiles_of_either_width():
     for i in range(entries):
         alone, alone_state = run(i, 1)
         assert torch.equal(alone, out[sum(lens[:i]):sum(lens[:i + 1])]) and torch.equal(alone_state[0], state[i])
+
+
+@pytest.mark.parametrize("key_dim", [64, 128])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_linear_attention_in_runs_in_tiles_of_128_columns(key_dim, dtype):
+    """Enough runs and heads that the step takes its value columns 128 at a time (more than 74 tiles)."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, value_dim, lens = 12, 128, [450, 200, 130]
+    n, entries, qk = sum(lens), len(lens), heads * key_dim
+    rows, decay = rnd(n, 2 * qk + heads * value_dim, dtype=dtype), torch.tensor([1 - 2.0 ** -(3 + i % 6) for i in range(heads)], dtype=torch.float64)
+    state, starts = rnd(entries, heads, key_dim, value_dim, seed=5), [sum(lens[:i]) for i in range(entries + 1)]
+    powers = [dev((decay[:, None] ** torch.arange(most + 1, dtype=torch.float64)).float().contiguous())
+              for most in (ops.linear_attention_chunk(key_dim, value_dim), ops.linear_attention_run())]
+    proj, got_state = dev(rows), dev(state.clone())
+    out = ops.linear_attention(proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:], torch.empty(n, heads * value_dim, device="cuda"), got_state, powers[0],
+                               dev(torch.tensor(starts, dtype=torch.int32)), dev(torch.arange(entries, dtype=torch.int32)), entries, heads, key_dim, value_dim,
+                               silu=True, max_q_len=max(lens), run_powers=powers[1])
+    act = rows.double() * torch.sigmoid(rows.double())
+    q, k, v = act[:, :qk].view(n, heads, -1), act[:, qk:2 * qk].view(n, heads, -1), act[:, 2 * qk:].view(n, heads, -1)
+    want, want_state = torch.empty(n, heads, value_dim, dtype=torch.float64), state.double()
+    for e, length in enumerate(lens):
+        s = want_state[e]
+        for t in range(starts[e], starts[e] + length):
+            s = decay[:, None, None] * s + k[t][:, :, None] * v[t][:, None, :]
+            want[t] = torch.einsum("hkv,hk->hv", s, q[t])
+        want_state[e] = s
+    assert (as_ref(out) - want.reshape(n, -1)).abs().max() <= 2e-6 * want.abs().max()
+    assert (as_ref(got_state) - want_state).abs().max() <= 2e-6 * want_state.abs().max()
 
 
 @pytest.mark.parametrize("at_a_time", [1, 2, 3])
@@ -1288,6 +1322,68 @@ def test_scan_in_chunks_agrees_with_the_recurrence(lens, heads, head_dim, state,
     # everything 32-bit enters its products with 24 bits: sums of up to `state` + 128 such terms, 2^-23 of the largest value each
     for out, ref in ((y, want.reshape(n, inner)), (got, want_state)):
         assert (as_ref(out) - ref).abs().max() <= 32 * 2.0 ** -23 * ref.abs().max()
+
+
+@pytest.mark.parametrize("heads, head_dim, state, groups, lens", [
+    (62, 64, 128, 1, [700, 300]), (46, 64, 64, 2, [900, 257, 40]), (22, 128, 128, 1, [1100]), (80, 64, 64, 4, [650, 129])])      # (three or four a block)
+def test_scan_in_chunks_with_several_heads_a_block(heads, head_dim, state, groups, lens):
+    """Steps large enough that a block takes several heads (or 64-column tiles of them) of a group, the last of a group fewer: the recurrence, the bits
+    that a few heads alone have (a block each), and numbers that are not finite in some of a block's heads."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    n, inner, entries = sum(lens), heads * head_dim, len(lens)
+    xbc, dt = rnd(n, inner + 2 * groups * state, dtype=torch.bfloat16), rnd(n, heads, dtype=torch.bfloat16, seed=1)
+    bias, a_log, skip = rnd(heads, seed=2) - 2.0, 0.5 * rnd(heads, seed=3), rnd(heads, seed=4)
+    held, starts = rnd(entries, heads, state, head_dim, seed=5), torch.tensor([sum(lens[:i]) for i in range(entries + 1)], dtype=torch.int32)
+
+    def run(xbc, of):
+        """The heads ``of`` of one group (None: all of them)."""
+        if of is None:
+            rows, own, g = xbc, slice(None), groups
+        else:
+            at, g = of[0] // (heads // groups), 1
+            rows = torch.cat([xbc[:, of[0] * head_dim:(of[-1] + 1) * head_dim]] + [xbc[:, inner + (i * groups + at) * state:inner + (i * groups + at + 1) * state] for i in range(2)], 1)
+            own = slice(of[0], of[-1] + 1)
+        count = heads if of is None else len(of)
+        y, carried = torch.empty(n, count * head_dim, device="cuda"), dev(held[:, own].reshape(entries, -1).contiguous())
+        error = torch.zeros(1, dtype=torch.int32, device="cuda")
+        ops.ssd_scan(dev(rows.contiguous()), dev(dt[:, own].contiguous()), 0, dev(bias[own].contiguous()), dev(a_log[own].contiguous()), dev(skip[own].contiguous()), carried,
+                     dev(starts), dev(torch.arange(entries, dtype=torch.int32)), y, entries, heads=count, groups=g, state_dim=state, head_dim=head_dim,
+                     max_q_len=max(lens), error_word=error)
+        assert int(error) == 0
+        return y.cpu().view(n, count, head_dim), carried.cpu().view(entries, count, state, head_dim)
+
+    y, carried = run(xbc, None)
+    x = xbc[:, :inner].double().view(n, heads, head_dim)
+    b, c = (xbc[:, inner + i * groups * state:inner + (i + 1) * groups * state].double().view(n, groups, state).repeat_interleave(heads // groups, 1)
+            for i in range(2))
+    step = torch.nn.functional.softplus(dt.double() + bias.double(), threshold=1e9)
+    decay = (-a_log.double().exp() * step).exp()
+    want, want_state = torch.empty(n, heads, head_dim, dtype=torch.float64), held.double().clone()
+    for e, length in enumerate(lens):
+        s = want_state[e].clone()
+        for t in range(int(starts[e]), int(starts[e]) + length):
+            s = decay[t][:, None, None] * s + (step[t][:, None] * b[t])[:, :, None] * x[t][:, None, :]
+            want[t] = torch.einsum("hsp,hs->hp", s, c[t]) + skip.double()[:, None] * x[t]
+        want_state[e] = s
+    for got, ref in ((y, want), (carried, want_state)):      # (as where a block takes one head)
+        assert (got.double() - ref).abs().max() <= 32 * 2.0 ** -23 * ref.abs().max()
+    last = heads // groups - 1
+    parts = [[0], [1, 2], [last - 1, last], [heads - 2, heads - 1]]
+    for of in parts:
+        few, few_state = run(xbc, of)
+        assert torch.equal(few, y[:, of]) and torch.equal(few_state, carried[:, of]), of
+    broken = xbc.clone()
+    for h, t, bad in ((1, 5, math.inf), (2, 140, math.nan), (last, 127, -math.inf), (heads - 1, 0, math.nan), (heads - 1, lens[0] - 1, math.inf)):
+        broken[t, h * head_dim + 3 + h % 32] = bad
+    odd, odd_state = run(broken, None)
+    bits = lambda t: t.contiguous().view(torch.int32).where(~t.isnan(), 0)
+    for of in parts:
+        few, few_state = run(broken, of)
+        assert torch.equal(bits(few), bits(odd[:, of])) and torch.equal(bits(few_state), bits(odd_state[:, of])), of
+    keep = torch.ones(n, heads, head_dim, dtype=torch.bool)
+    keep[:lens[0], [1, 2, last, heads - 1]] = False
+    assert torch.equal(odd[keep], y[keep]) and not odd[~keep].isfinite().all()
 
 
 @pytest.mark.parametrize("lens, head_dim, state", [([300, 7, 129], 64, 128), ([140, 70], 32, 64)])
