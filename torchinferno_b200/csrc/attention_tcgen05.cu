@@ -13,8 +13,8 @@
 // Warp 0 is the TMA producer of Q (one 3-D tile copy; dims: head_dim, head, token) and of K, the last
 // warp that of V, page by page through a 2-D view of the layer's pages ([page rows, head_dim]), each
 // into a ring of its own; pages past the block's last query are fetched from an out-of-range
-// coordinate, which fills zeros.  Warp 1 issues the MMAs (the whole warp walks the loop, one lane issues: three portions of 2,048 tokens behind
-// 512, 32 / 8 heads of 128, take 59 us and took 61).  Every mbarrier wait is bounded; on a timeout a code goes to `error_word`
+// coordinate, which fills zeros.  Warp 1 issues the MMAs (the whole warp walks the loop, one lane issues, as in the other kernels; here that gained no
+// more than the noise: 59 us for three portions of 2,048 tokens behind 512, 32 / 8 heads of 128).  Every mbarrier wait is bounded; on a timeout a code goes to `error_word`
 // and all roles fall through to the common exit.
 //
 // Formula as in attention_mma.cu / attention_simt.cu (src/torchinferno/models/llama3/raw_ops.py:44-51).

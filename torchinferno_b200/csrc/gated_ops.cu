@@ -70,7 +70,7 @@ __device__ __forceinline__ void raw8_floats(const Raw8& r, int dtype, float (&v)
 // The same with rows on 16-byte boundaries: a thread takes eight neighbouring columns, everything asked for before the first is used,
 // and a row is cut over several blocks.  Same sums.  What bounds it: for few rows one trip to memory after the launch, for many the
 // bytes.  Eight rows of 4096 element by element, a row a block, took 10 us; by eight in blocks of 64 threads the block of eight
-// single tokens they end went from 121 to 113.
+// single tokens they end went from 121 to 113 (a served model folds this sum into the next norm and launches nothing here).
 __global__ void __launch_bounds__(256)
 add_pair_vec_kernel(float* __restrict__ residual, const void* __restrict__ a, int a_dtype, int64_t lda, const void* __restrict__ b,
                     int b_dtype, int64_t ldb, void* __restrict__ copy, int copy_dtype, int width) {

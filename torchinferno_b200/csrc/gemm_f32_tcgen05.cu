@@ -326,10 +326,16 @@ static int ft_weight_map(CUtensorMap* map, const float* w, int N, int K, int64_t
 using namespace tib;
 
 // Whether a weight's product runs here.  By the weight's sizes and the alignment alone, not by the number of rows: a request's
-// numbers do not depend on what else is in the step.  Four million weights are where the two launches and the scratch, some 8 us of the host more
-// than the other kernel's one, are paid back on few rows too: a block of 512 x 512 weights on 20
-// tokens took 143 us there and 182 here, one of 1,024 x 1,024 and 1,024 x 2,112 on 40 139 and 150, one of 1,536 x 1,536 and 1,536 x 6,400 on
-// 100 503 and 299.
+// numbers do not depend on what else is in the step.  On the device terms are faster from a million weights on, whatever the rows (1,024 x 1,024,
+// us on 8 / 40 / 300 rows: 19 / 19 / 43 by multiply-adds and 16 / 17 / 19 here; 2,048 x 2,048 37 / 50 / 110 and 26 / 27 / 31).  But a product issued
+// call by call costs the host some 8 us more (two launches and the scratch), and a block of such weights on few tokens waits for the host.
+// Blocks call by call, us on 8 / 40 / 100 / 300 tokens, by multiply-adds alone, with the line at 2^22 weights and at 2^20:
+//     1,024 wide, 1,024 inside   133 / 135 / 165 / 284   132 / 135 / 165 / 283   161 / 162 / 162 / 162
+//     1,024 wide, 2,112 inside   135 / 149 / 206 / 361   142 / 144 / 189 / 302   162 / 163 / 162 / 161
+//     1,536 wide, 3,200 inside   191 / 237 / 340 / 599   156 / 158 / 195 / 275   161 / 162 / 168 / 231
+//     1,536 wide, 6,400 inside   253 / 312 / 486 / 856   180 / 188 / 242 / 328   167 / 175 / 214 / 284
+// So no line is best for all: 2^22 costs few tokens 5 % (the second block's 4.3 million of gate and up), where 2^20 would cost them 20 % and gain
+// prompts of a hundred tokens and more 15 to 45 %.
 // (Weights whose rows overlap or are one and the same are none of a tensor map's.)
 TIB_API int tib_gemm_f32_tcgen05_takes(const void* x, const void* w, int N, int K, int64_t ldx, int64_t ldw) {
   return N >= 512 && K >= 512 && (int64_t)N * K >= (1 << 22) && K % kFtK == 0 && ldx % 4 == 0 && ldw % 4 == 0 && ldw >= K &&

@@ -591,7 +591,7 @@ latent_attention_mma_kernel(const float* __restrict__ folded, const __nv_bfloat1
 // 16 keys over a fourth of the row's width, then the softmax of one head, then 16 or 32 value columns: the chain of one tile is some
 // 20 products and four barriers long.  What bounds it is that chain, the lookups before the first tile and, cold, the rows: eight tokens of 16
 // heads over 3,000 cached rows of 576 take 14 us, and took 33 in blocks of four warps that looked every key's page up by itself (16 with
-// queries read from shared memory for every tile).  The layer: 50 us (66); 12 tokens of 32 heads over 2,000 rows of 320: 54 (84).
+// queries read from shared memory for every tile).  The layer: 53 to 55 us (69); 12 tokens of 32 heads over 2,000 rows of 320: 54 (84).
 constexpr int kLdThreads = 512;
 constexpr int kLdScores = kMmaKeys + 4;      // row stride of the scores
 constexpr int kLdSteps = 9;                  // steps of 16 of a fourth of the row's width whose queries a warp keeps

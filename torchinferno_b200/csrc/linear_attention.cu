@@ -217,8 +217,8 @@ linear_attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 // ---------------------------------------------------------------------------------------------------------- runs
 // The walk above is one serial chain of 64 chunks for 2,048 tokens, each with four barriers, on 512 blocks that each see 32 of a
 // run's 128 columns: 980 us for two portions of 1,366 and 682 tokens, 16 heads of 128 x 128, of which the fp32 arithmetic
-// (3.3 GFLOP here) is some 50 us.  In runs of 64 on the fp32 pipe the three launches took 131 us (49 + 27 + 82 cold); in runs of 128 on the
-// tensor cores (linear_tcgen05.cu) they take 68 (26 + 18 + 52), half of the states' traffic with it.  Of 2,048 tokens of 24 heads of 64 x 64
+// (3.3 GFLOP here) is some 50 us.  In runs of 64 on the fp32 pipe the three launches took 131 us in the layer (one by one and cold 49 + 27 + 82); in
+// runs of 128 on the tensor cores (linear_tcgen05.cu) they take 68 (cold 22 + 16 + 44), half of the states' traffic with it.  Of 2,048 tokens of 24 heads of 64 x 64
 // 57 us (74), of 600 of 8 heads of 128 x 64 27 (33).
 // Everything stays fp32 or three bf16 terms of it: activations, decay powers, scores, states and sums.  Error against 64 bits (2-norm, those
 // four cases with one of 4 heads of 64 x 128): outputs 1.0 to 1.3e-7 (1.4 to 1.9 on the fp32 pipe), states 7 to 8.7e-8 (8.6e-8 to 1.0e-7).
@@ -389,11 +389,13 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   if (heads < 1 || key_dim < 1 || value_dim < 1 || chunk < 1 || chunk > 32 || n_entries > 65535) return TIB_E_SIZE;
   // The newer kernels take heads of 64 or 128 keys whose values come in whole tiles, rows and state on 16-byte boundaries.
   // The lines between the three.  Walk and chunks (four portions of 16 heads of 128 x 128): 14, 16 and 23 us at 8, 9 and 16 tokens
-  // against 33, 33 and 35.  Chunks and runs, the whole layer's device time at 64 / 128 / 192 tokens: one portion of 16 heads of 128 x 128
-  // 43 / 68 / 92 us against 57 / 70 / 72, four of them 87 / 148 / 213 against 76 / 83 / 94; one portion of 12 heads of 64 x 64 27 / 41 /
-  // 53 against 32 / 33 / 33.  On the device alone the lines would lie near 100 tokens.  But a prompt's layer is issued call by call, which
-  // takes some 87 us of the host in chunks and 97 in runs (two launches and an allocation more), and what is shorter on the device
-  // than that waits for the host: runs pay a lone portion from some 200 tokens at 128 x 128 and some 400 at 64 x 64.
+  // against 33, 33 and 35.  Chunks and runs, the whole layer's device time at 40 / 64 / 128 / 192 tokens: one portion of 16 heads of 128 x 128
+  // 36 / 41 / 66 / 91 us against 37 / 37 / 39 / 41, four of them 69 / 86 / 152 / 221 against 45 / 47 / 56 / 71; one portion of 12 heads of 64 x 64
+  // 24 / 25 / 39 / 52 against 28 / 28 / 30 / 30.  On the device alone the lines would lie near 50 tokens.  But a prompt's layer is issued call by
+  // call, which takes 81 us of the host in chunks and 91 in runs (two launches and an allocation more), and what is shorter on the device than
+  // that waits for the host.  Call by call, a lone portion in chunks and in runs: 128 x 128 84 and 91 at 160 tokens, 96 and 91 at 192, 121
+  // and 91 at 256; 64 x 64 82 and 91 at 256, 97 and 91 at 384.  Several portions would gain from 64 tokens on, and not know of it: the line
+  // goes by a portion's own length.
   const int64_t size = dtype == TIB_F32 ? 4 : 2;
   const bool aligned = (ldq * size) % 16 == 0 && (ldk * size) % 16 == 0 && (ldv * size) % 16 == 0 &&
                        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)run_state) & 15) == 0;

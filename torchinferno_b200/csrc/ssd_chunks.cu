@@ -17,7 +17,7 @@
 // Heads in whole tiles of 64 columns run the first and the last on tcgen05 (ssd_tcgen05.cu); the kernels here, on mma.sync, take tiles of 32 (heads
 // of 32 or 96 columns).  The walk of ssd_scan_kernel spends five fp32 operations per state element and token twice over (two prompts of 1,366
 // and 682 tokens, 64 heads of 64 with a state of 128: 182 + 32 + 264 us, the fp32 pipe at 40 %), the products took 39 + 32 + 98 us
-// cold here and take 29 + 33 + 65 there.  Error against 64 bits of such a scan: y 9.8e-8 in both, the walk 8.5e-8; with steps of e^-8 and less, where
+// cold here and take 30 + 32 + 66 there.  Error against 64 bits of such a scan: y 9.8e-8 in both, the walk 8.5e-8; with steps of e^-8 and less, where
 // the walk adds a thousand small terms one by one, 1e-7 against 6e-6.  What bounds it: the legacy tensor path with operands from shared memory,
 // and the states' way through the L2 (one of 32 KB a head of 64 and chunk, written twice and read twice).
 #include "state_space.cuh"
