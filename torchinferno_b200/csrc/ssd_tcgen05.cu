@@ -14,7 +14,8 @@
 //
 // What bounds it: the threads' work around the products, 18,600 warp instructions a head and chunk for outputs and 8,000 for sums, at a third of the
 // issue slots with one block of 16 warps an SM (tensor cores 12 %).  Two prompts of 1,366 and 682 tokens, 64 heads of 64, a state of 128: sums 29 us
-// cold, outputs 65 (39 and 99 on mma.sync), the layer 230 (272), two of it for infinities that stay infinite.  Weights of a group of 32 by two powers each, as between groups, made the outputs
+// cold, outputs 65 (39 and 99 on mma.sync), the layer 230 (272), two of it for infinities that stay infinite.
+// Weights of a group of 32 by two powers each, as between groups, made the outputs
 // 55 us, and the scores in two accumulators of four instructions another 3 less, for errors of y of 1.3e-7 and 1.4e-7 where they are 9.8e-8 now and before.
 #include "state_space.cuh"
 #include "split_terms.cuh"
