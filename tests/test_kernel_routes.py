@@ -1,6 +1,7 @@
 """What can be said of the kernels without a GPU: the host's rules on which one a call takes, and rules that their sources keep."""
 import re
-from ctypes import c_int, c_int64, c_void_p
+import struct
+from ctypes import c_char_p, c_int, c_int64, c_void_p
 from pathlib import Path
 
 import pytest
@@ -19,6 +20,28 @@ CSRC = Path(torchinferno_b200.__file__).parent / "csrc"
 def test_which_32_bit_products_run_on_tensor_cores(n, k, ldx, ldw, x, w, takes):
     from torchinferno_b200.kernels.library import load_library
     assert bool(load_library().tib_gemm_f32_tcgen05_takes(c_void_p(x), c_void_p(w), c_int(n), c_int(k), c_int64(ldx), c_int64(ldw))) == takes
+
+
+@pytest.mark.parametrize("name", sorted(set(re.findall(r"\b(?:lib\(\)|library)\.(tib_\w+)\(", (CSRC.parent / "kernels" / "ops.py").read_text()))))
+def test_every_call_of_the_parts_is_packed_by_its_own_types(name):
+    """As many slots as the function has parameters in its source, d for a floating-point number and q for anything else."""
+    from torchinferno_b200.kernels.library import load_library
+    slots = getattr(load_library(), name + "_slots")
+    slots.restype = c_char_p
+    found = [m.group(1) for path in CSRC.glob("*.cu") for m in [re.search(rf"TIB_API int {name}\(([^)]*)\)", path.read_text())] if m]
+    assert len(found) == 1
+    parameters = [p.strip() for p in found[0].split(",") if p.strip()]
+    assert slots().decode() == "".join("d" if re.match(r"(const )?(float|double) \w+$", p) else "q" for p in parameters)
+
+
+def test_packed_calls_pass_their_arguments():
+    from torchinferno_b200.kernels import ops
+    library = ops.lib()
+    assert bool(library.tib_gemm_f32_tcgen05_takes(1 << 40, 1 << 41, 2048, 2048, 2048, 2048))           # (addresses beyond 32 bits)
+    assert not library.tib_gemm_f32_tcgen05_takes((1 << 40) + 4, 1 << 41, 2048, 2048, 2048, 2048)
+    assert library.tib_embedding(0, 0, 0, 1, 8, 8, 0.5, 0, 0, 0, 0, 0) == -5                              # (a refusal comes back as it is)
+    with pytest.raises(struct.error):
+        library.tib_plan_product(1, 2, 3)
 
 
 def test_a_timeout_code_names_one_kernel():

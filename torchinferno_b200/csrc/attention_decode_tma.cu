@@ -604,3 +604,8 @@ TIB_API int tib_decode_attention_tma_rope(const void* qkv, void* pool, void* out
                               block_table, table_stride, n_entries, heads, kv_heads, head_dim, page_size, page_stride, num_pages,
                               window, scale, num_splits, chunk, counters, error_word, true, inv_freq, rot_dim, interleaved, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_decode_attention_tma)
+TIB_PACKED(tib_decode_attention_tma_rope)
+TIB_PACKED(tib_decode_attention_tma_supports)

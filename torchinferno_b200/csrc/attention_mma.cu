@@ -641,3 +641,8 @@ TIB_API int tib_decode_attention_noalloc(const void* q, const void* pool, void* 
   return head_dim <= 64 ? launch_decode<64>(q, pool, scratch_o, scratch_ml, out, a, n_entries, stream)
                         : launch_decode<128>(q, pool, scratch_o, scratch_ml, out, a, n_entries, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_attention_mma_supports)
+TIB_PACKED(tib_decode_attention)
+TIB_PACKED(tib_prefill_attention)

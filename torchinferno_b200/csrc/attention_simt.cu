@@ -306,3 +306,6 @@ TIB_API int tib_paged_attention_simt(const void* q, const void* pool, void* out,
 #undef TIB_ATTN_DISPATCH
   return TIB_E_DTYPE;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_paged_attention_simt)

@@ -483,3 +483,7 @@ TIB_API int tib_prefill_attention_tcgen05(const void* q, const void* pool, void*
   return head_dim == 64 ? launch_fa<64>(q, pool, out, a, n_entries, max_q_len, page_stride, stream)
                         : launch_fa<128>(q, pool, out, a, n_entries, max_q_len, page_stride, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_prefill_attention_tcgen05)
+TIB_PACKED(tib_prefill_attention_tcgen05_supports)

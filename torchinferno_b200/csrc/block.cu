@@ -328,3 +328,9 @@ TIB_API int tib_prenorm_gqa_glu_block(const TibPrenormBlockWeights* w, TibPrenor
   TIB_TIMED(KC_DOWN, project(s->act, w->down, s->out, n, w->hidden, inter, w->down_kn, w->down_few_rows, w->down_features, w->down_splits, w->down_stages, s->error_word, &s->own_launches, stream));
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_kernel_timers)
+TIB_PACKED(tib_kernel_timers_read)
+TIB_PACKED(tib_plan_attention)
+TIB_PACKED(tib_plan_product)

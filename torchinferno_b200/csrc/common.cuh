@@ -9,8 +9,16 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
+#include <type_traits>
+#include <utility>
 
 #define TIB_API extern "C" __attribute__((visibility("default")))
+
+// name_packed(slots) calls name with its arguments from 64-bit slots, name_slots() says how they are packed (see packed_call below).
+#define TIB_PACKED(name)                                                                  \
+  TIB_API int name##_packed(const void* slots) { return tib::packed_call(&name, slots); } \
+  TIB_API const char* name##_slots() { return tib::packed_slots(&name); }
 
 // Element types of activations, weights and cache pages.
 enum TibDtype : int { TIB_F32 = 0, TIB_BF16 = 1 };
@@ -58,6 +66,32 @@ constexpr int kMostSmem = 227 * 1024;
   } while (0)
 
 namespace tib {
+
+// A call with its arguments in 64-bit slots (integers and addresses as they are, floats as doubles), unpacked by the function's own types:
+// the interpreter packs them in one go, without an object for each.
+template <typename T> static inline T packed_slot(const void* slots, size_t i) {
+  const char* at = static_cast<const char*>(slots) + 8 * i;
+  if constexpr (std::is_floating_point_v<T>) {
+    double v;
+    memcpy(&v, at, 8);
+    return static_cast<T>(v);
+  } else {
+    int64_t v;
+    memcpy(&v, at, 8);
+    if constexpr (std::is_pointer_v<T>) return reinterpret_cast<T>(v);
+    else return static_cast<T>(v);
+  }
+}
+template <typename... A, size_t... I> static inline int packed_call(int (*f)(A...), const void* slots, std::index_sequence<I...>) {
+  return f(packed_slot<A>(slots, I)...);
+}
+template <typename... A> static inline int packed_call(int (*f)(A...), const void* slots) {
+  return packed_call(f, slots, std::index_sequence_for<A...>());
+}
+template <typename... A> static inline const char* packed_slots(int (*)(A...)) {      // how to pack them: q an integer or address, d a float
+  static const char kinds[] = {(std::is_floating_point_v<A> ? 'd' : 'q')..., 0};
+  return kinds;
+}
 
 // The two halves of a bf16 pair as floats, by shift and mask: a bf16 is the upper half of the float it stands for, so two
 // integer instructions unpack a pair (measured faster than the conversion function in kernels that only unpack, compute a

@@ -390,3 +390,6 @@ TIB_API int tib_conv_norm_append(const void* proj, int64_t ld, int q_off, int k_
 #undef TIB_CNA
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_conv_norm_append)

@@ -422,3 +422,13 @@ TIB_API int tib_set_dependent_launch(int on) {
   tib::dependent_launch_flag() = on ? 1 : 0;
   return before;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_add_rmsnorm)
+TIB_PACKED(tib_cast)
+TIB_PACKED(tib_decode_inputs)
+TIB_PACKED(tib_embedding)
+TIB_PACKED(tib_rmsnorm)
+TIB_PACKED(tib_scatter_i32)
+TIB_PACKED(tib_set_dependent_launch)
+TIB_PACKED(tib_swiglu)

@@ -423,3 +423,16 @@ TIB_API int tib_add_vector(float* x, const void* delta, int delta_dtype, int64_t
   TIB_LAUNCH_DEPENDENT(add_vector_kernel, rows, row_threads(width), 0, stream, x, delta, delta_dtype, ldd, v, width);
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_add_pair)
+TIB_PACKED(tib_add_vector)
+TIB_PACKED(tib_gelu)
+TIB_PACKED(tib_gelu_gate_table)
+TIB_PACKED(tib_glu_clamp)
+TIB_PACKED(tib_pair_rows)
+TIB_PACKED(tib_relu_squared)
+TIB_PACKED(tib_scale_f32)
+TIB_PACKED(tib_sigmoid_gate)
+TIB_PACKED(tib_softcap_f32)
+TIB_PACKED(tib_unit_norm_add)

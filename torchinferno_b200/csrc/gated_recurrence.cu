@@ -191,3 +191,6 @@ TIB_API int tib_gated_recurrence(const void* proj, int dtype, int64_t ld, int z_
   TIB_LAUNCH_DEPENDENT(gated_recurrence_scan_kernel, grid, threads, a.staged ? (g_off >= 0 ? 3 : 2) * tile : 0, stream, a);
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_gated_recurrence)

@@ -391,3 +391,7 @@ TIB_API int tib_gemm_decode(const void* x, const void* w, void* out, int M, int 
 #undef TIB_DG_F
 #undef TIB_DG_E
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_gemm_decode)
+TIB_PACKED(tib_gemm_decode_supports)

@@ -205,3 +205,6 @@ TIB_API int tib_gemm_f32(const void* x, const void* w, float* out, int M, int N,
   TIB_LAUNCH_CHECK();
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_gemm_f32)

@@ -385,3 +385,7 @@ TIB_API int tib_gemm_f32_tcgen05(const float* x, const float* w, float* out, int
   }
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_gemm_f32_tcgen05)
+TIB_PACKED(tib_gemm_f32_tcgen05_takes)

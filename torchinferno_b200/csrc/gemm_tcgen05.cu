@@ -563,3 +563,9 @@ TIB_API int tib_gemm_tcgen05(const void* x, const void* w, void* out, int M, int
   TIB_LAUNCH_CHECK();
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_gemm_tcgen05)
+TIB_PACKED(tib_gemm_tcgen05_supports)
+TIB_PACKED(tib_gemm_tcgen05_swapab)
+TIB_PACKED(tib_gemm_tcgen05_swapab_supports)

@@ -318,3 +318,7 @@ TIB_API int tib_gemm_tcgen05_2cta(const void* x, const void* w, void* out, int M
   return wide ? launch_2cta<256, float>(x, w, out, M, N, K, ldx, ldw, ldo, error_word, stream)
               : launch_2cta<224, float>(x, w, out, M, N, K, ldx, ldw, ldo, error_word, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_gemm_tcgen05_2cta)
+TIB_PACKED(tib_gemm_tcgen05_2cta_supports)

@@ -170,3 +170,6 @@ TIB_API int tib_hyper_step(float* streams, int64_t stream_stride, int S, int n_o
   }
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_hyper_step)

@@ -356,3 +356,7 @@ TIB_API int tib_norm_conv_step(const void* delta, float* residual, const float* 
   TIB_LAUNCH_DEPENDENT(norm_conv_step_kernel<__nv_bfloat16>, n_rows, threads, 0, stream, (const __nv_bfloat16*)delta, (__nv_bfloat16*)out, a);
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_input_conv)
+TIB_PACKED(tib_norm_conv_step)

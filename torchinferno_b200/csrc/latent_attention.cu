@@ -948,3 +948,8 @@ TIB_API int tib_latent_attention(const float* folded, const void* pool, float* o
 #undef TIB_LAT_DISPATCH
   return TIB_E_DTYPE;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_latent_append)
+TIB_PACKED(tib_latent_attention)
+TIB_PACKED(tib_latent_attention_splits)

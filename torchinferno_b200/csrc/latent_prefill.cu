@@ -483,3 +483,8 @@ TIB_API int tib_latent_prefill(const void* q, int64_t ldq, const void* kv, const
   return value_dim == 128 ? launch_lp<1, 2>(map_q, map_kv, map_r, a, n_heads, n_entries, max_q_len, stream)
                           : launch_lp<1, 1>(map_q, map_kv, map_r, a, n_heads, n_entries, max_q_len, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_latent_gather)
+TIB_PACKED(tib_latent_prefill)
+TIB_PACKED(tib_latent_prefill_supports)

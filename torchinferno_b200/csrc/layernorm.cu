@@ -293,3 +293,7 @@ TIB_API int tib_layernorm_tail(const void* y, int y_dtype, int64_t ldy, const fl
   TIB_LAUNCH_DEPENDENT(layernorm_tail_kernel, n, ln_threads(width), smem, stream, a);
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_layernorm)
+TIB_PACKED(tib_layernorm_tail)

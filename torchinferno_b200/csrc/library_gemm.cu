@@ -146,3 +146,8 @@ TIB_API int tib_blas_gemm_batched(const void* x, const void* w, void* out, int M
   if (out_dtype != TIB_BF16 && out_dtype != TIB_F32) return TIB_E_DTYPE;
   return blas_gemm_bf16_batched(x, w, out, M, N, K, ldx, ldw, ldo, sx, sw, so, batch, w_kn, out_dtype, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_blas_gemm)
+TIB_PACKED(tib_blas_gemm_batched)
+TIB_PACKED(tib_blas_init)

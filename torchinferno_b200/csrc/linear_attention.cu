@@ -461,3 +461,10 @@ TIB_API int tib_linear_attention(const void* q, const void* k, const void* v, in
   *launches += 1;
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_linear_attention)
+TIB_PACKED(tib_linear_attention_chunk)
+TIB_PACKED(tib_linear_attention_run)
+TIB_PACKED(tib_linear_attention_runs_from)
+TIB_PACKED(tib_linear_attention_walk)

@@ -753,3 +753,10 @@ TIB_API int tib_matrix_memory(const void* proj, int64_t ld, int q_off, int k_off
   }
   return dtype == TIB_F32 ? mem_walk_launch<float>(a, n_entries, stream) : mem_walk_launch<__nv_bfloat16>(a, n_entries, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_matrix_memory_max_dim)
+TIB_PACKED(tib_matrix_memory)
+TIB_PACKED(tib_matrix_memory_chunk)
+TIB_PACKED(tib_matrix_memory_takes_chunks)
+TIB_PACKED(tib_matrix_memory_tile)

@@ -573,3 +573,10 @@ TIB_API int tib_moe_combine(const float* y, const int* place, const float* weigh
 #undef TIB_COMBINE_GO
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_moe_combine)
+TIB_PACKED(tib_moe_expert_product)
+TIB_PACKED(tib_moe_group)
+TIB_PACKED(tib_moe_route)
+TIB_PACKED(tib_router_logits)

@@ -1389,3 +1389,11 @@ TIB_API int tib_pooled_window_attention(const void* q, void* out, const int* q_s
 #undef TIB_PWA_DISPATCH
   return TIB_E_DTYPE;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_pool_blocks)
+TIB_PACKED(tib_pooled_window_attention)
+TIB_PACKED(tib_pooled_window_attention_few_rows)
+TIB_PACKED(tib_pooled_window_attention_part_floats)
+TIB_PACKED(tib_pooled_window_attention_splits)
+TIB_PACKED(tib_rotary_kv_append)

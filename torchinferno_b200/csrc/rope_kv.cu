@@ -257,3 +257,6 @@ TIB_API int tib_rope_append(const void* qkv, void* q_out, void* pool, const int*
   TIB_LAUNCH_CHECK();
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_rope_append)

@@ -141,3 +141,7 @@ TIB_API int tib_sample_records(const float* logits, int64_t row_stride, int* rec
   TIB_LAUNCH_CHECK();
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_sample)
+TIB_PACKED(tib_sample_records)

@@ -657,3 +657,8 @@ TIB_API int tib_sigmoid_attention(const void* q, const void* k_pages, const void
 #undef TIB_SA_DISPATCH
   return TIB_E_DTYPE;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_qk_norm_append)
+TIB_PACKED(tib_sigmoid_attention)
+TIB_PACKED(tib_sigmoid_attention_takes_mma)

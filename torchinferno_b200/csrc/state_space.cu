@@ -608,3 +608,10 @@ TIB_API int tib_gated_group_norm(const float* y, const void* z, int z_dtype, int
                          eps, out, out_dtype, width, part);
   return TIB_OK;
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_gated_group_norm)
+TIB_PACKED(tib_short_conv)
+TIB_PACKED(tib_ssd_scan)
+TIB_PACKED(tib_ssd_scan_max_state)
+TIB_PACKED(tib_ssd_scan_run)

@@ -1239,3 +1239,11 @@ TIB_API int tib_talking_heads_attention(const void* q, void* out, const int* q_s
   if (status != TIB_OK) return status;
   return vdim <= 64 ? th_launch_values<64>(out, a, grid, stream) : th_launch_values<128>(out, a, grid, stream);
 }
+
+// The calls the Python parts make (common.cuh).
+TIB_PACKED(tib_row_norm_append)
+TIB_PACKED(tib_talking_heads_attention)
+TIB_PACKED(tib_talking_heads_key_span)
+TIB_PACKED(tib_talking_heads_takes_mma)
+TIB_PACKED(tib_talking_heads_takes_step)
+TIB_PACKED(tib_talking_heads_tiles_per_part)

@@ -193,8 +193,10 @@ def _linear_kn(x: torch.Tensor, weight_kn: torch.Tensor, out_dtype: torch.dtype,
     if out_dtype not in (torch.bfloat16, torch.float32):
         raise ops.KernelError(f"linear: unsupported output dtype {out_dtype}")
     if out is None or out.dtype != out_dtype:
-        out = torch.empty((x.shape[0], weight_kn.shape[1]), dtype=out_dtype, device=x.device)
-    if _backend == "auto":      # (which kernel: decided where the native block call decides it too)
+        shape = (x.shape[0], weight_kn.shape[1])
+        out = x.new_empty(shape) if x.dtype == out_dtype else torch.empty(shape, dtype=out_dtype, device=x.device)
+    # (which kernel: decided where the native block call decides it too, which leaves more rows than `few_rows` to the library)
+    if _backend == "auto" and 0 < x.shape[0] <= few_rows:
         k, n = weight_kn.shape
         kernel = ops.plan_product(x.shape[0], n, k, True, few_rows, features, splits, False, _aligned(x, weight_kn))
         if kernel == ops.PRODUCT_DECODE:

@@ -16,6 +16,7 @@ import torch
 
 from torchinferno_b200.kernels import gemm, ops
 from torchinferno_b200.kernels.gemm import LinearWeight
+from torchinferno_b200.kernels.library import load_library
 
 
 class BlockWeights(Structure):
@@ -41,7 +42,7 @@ _configured = False
 
 def _function():
     global _configured
-    fn = ops.lib().tib_prenorm_gqa_glu_block
+    fn = load_library().tib_prenorm_gqa_glu_block
     if not _configured:
         fn.restype = c_int
         fn.argtypes = [POINTER(BlockWeights), POINTER(BlockStep), c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int,

@@ -8,8 +8,9 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import struct
 from collections.abc import Mapping
-from ctypes import c_float, c_int, c_int64, c_void_p
+from ctypes import c_int
 
 import torch
 
@@ -39,7 +40,7 @@ def set_dependent_launch(on: bool) -> bool:
     """Programmatic dependent launch of the library's small kernels (on by default): a kernel may be placed on
     the SMs while the one before it drains and waits there for its data.  Returns the setting before.  A
     captured graph keeps what was set when it was captured."""
-    return bool(lib().tib_set_dependent_launch(c_int(1 if on else 0)))
+    return bool(lib().tib_set_dependent_launch(1 if on else 0))
 
 
 KERNEL_CLASSES = ("norm", "qkv", "rope_append", "attention_prefill", "attention_decode", "o", "gate_up", "swiglu", "down")
@@ -48,14 +49,14 @@ KERNEL_CLASSES = ("norm", "qkv", "rope_append", "attention_prefill", "attention_
 def set_kernel_timers(on: bool) -> bool:
     """CUDA-event timers around every launch of a natively issued block, by kernel class (off by default; a step
     captured in a graph records nothing).  Returns the setting before."""
-    return bool(lib().tib_kernel_timers(c_int(1 if on else 0)))
+    return bool(lib().tib_kernel_timers(1 if on else 0))
 
 
 def read_kernel_timers(reset: bool = False) -> dict[str, dict[str, float]]:
     """{class: {"ms": total, "launches": n}} of what the timers have recorded; waits for the recorded events."""
     n = len(KERNEL_CLASSES)
     ms, counts = (ctypes.c_double * n)(), (ctypes.c_longlong * n)()
-    lib().tib_kernel_timers_read(ms, counts, c_int(n), c_int(1 if reset else 0))
+    lib().tib_kernel_timers_read(ctypes.addressof(ms), ctypes.addressof(counts), n, 1 if reset else 0)
     return {name: {"ms": float(ms[i]), "launches": int(counts[i])} for i, name in enumerate(KERNEL_CLASSES)}
 
 
@@ -86,8 +87,8 @@ def _check(name: str, status: int) -> None:
     raise KernelError(f"{name}: CUDA error {status} at launch")
 
 
-def _ptr(t: torch.Tensor | None) -> c_void_p:
-    return c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def _need(t: torch.Tensor, name: str, dtype: torch.dtype | None = None) -> None:
@@ -99,44 +100,43 @@ def _need(t: torch.Tensor, name: str, dtype: torch.dtype | None = None) -> None:
         raise KernelError(f"{name} must be {dtype}, got {t.dtype}")
 
 
-def _stream() -> c_void_p:
+def _stream() -> int:
     # (the raw handle of the current stream of the current device: a fraction of the cost of
     # torch.cuda.current_stream(), which is asked for at every launch)
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-_signatures_set = False
+class _Packed:
+    """A function of the CUDA library as a call that takes plain numbers (and addresses): they are packed into 64-bit slots, which
+    the library unpacks by the function's own types (TIB_PACKED in csrc/common.cuh).  A call of 19 arguments takes 1.0 us, where one
+    with an object of ctypes for each took 3.4."""
+    __slots__ = ("call", "pack")
+
+    def __init__(self, library: ctypes.CDLL, name: str) -> None:
+        slots = getattr(library, name + "_slots")
+        slots.restype, slots.argtypes = ctypes.c_char_p, []
+        self.call = getattr(library, name + "_packed")
+        self.call.restype, self.call.argtypes = c_int, [ctypes.c_char_p]
+        self.pack = struct.Struct("=" + slots().decode()).pack
+
+    def __call__(self, *args) -> int:
+        return self.call(self.pack(*args))
 
 
-def lib() -> ctypes.CDLL:
-    global _signatures_set
-    library = load_library()
-    if not _signatures_set:
-        for fn in ("tib_embedding", "tib_add_rmsnorm", "tib_rmsnorm", "tib_swiglu", "tib_cast",
-                   "tib_scatter_i32", "tib_decode_inputs", "tib_sample_records", "tib_rope_append", "tib_paged_attention_simt", "tib_gemm_f32", "tib_gemm_f32_tcgen05", "tib_gemm_f32_tcgen05_takes", "tib_sample",
-                   "tib_attention_mma_supports", "tib_prefill_attention", "tib_decode_attention",
-                   "tib_prefill_attention_tcgen05", "tib_prefill_attention_tcgen05_supports",
-                   "tib_decode_attention_tma", "tib_decode_attention_tma_rope", "tib_decode_attention_tma_supports", "tib_set_dependent_launch",
-                   "tib_kernel_timers", "tib_kernel_timers_read",
-                   "tib_blas_init", "tib_blas_gemm", "tib_gemm_tcgen05_2cta", "tib_gemm_tcgen05_2cta_supports",
-                   "tib_gemm_tcgen05", "tib_gemm_tcgen05_supports",
-                   "tib_gemm_tcgen05_swapab", "tib_gemm_tcgen05_swapab_supports", "tib_gemm_decode", "tib_gemm_decode_supports",
-                   "tib_plan_attention", "tib_plan_product", "tib_blas_gemm_batched",
-                   "tib_add_pair", "tib_unit_norm_add", "tib_sigmoid_gate", "tib_gelu_gate_table", "tib_relu_squared", "tib_gelu",
-                   "tib_scale_f32", "tib_pair_rows", "tib_add_vector", "tib_linear_attention", "tib_linear_attention_chunk", "tib_linear_attention_run", "tib_linear_attention_walk", "tib_linear_attention_runs_from",
-                   "tib_latent_append", "tib_latent_prefill_supports", "tib_latent_gather", "tib_latent_prefill", "tib_latent_attention", "tib_latent_attention_splits", "tib_moe_route", "tib_moe_group", "tib_router_logits",
-                   "tib_moe_expert_product", "tib_moe_combine", "tib_glu_clamp", "tib_layernorm", "tib_layernorm_tail",
-                   "tib_qk_norm_append", "tib_sigmoid_attention", "tib_sigmoid_attention_takes_mma", "tib_gated_recurrence",
-                   "tib_softcap_f32", "tib_short_conv", "tib_ssd_scan", "tib_ssd_scan_max_state", "tib_ssd_scan_run", "tib_gated_group_norm",
-                   "tib_rotary_kv_append", "tib_pool_blocks", "tib_pooled_window_attention", "tib_hyper_step",
-                   "tib_pooled_window_attention_splits", "tib_pooled_window_attention_part_floats", "tib_pooled_window_attention_few_rows",
-                   "tib_input_conv", "tib_norm_conv_step", "tib_row_norm_append", "tib_talking_heads_attention",
-                   "tib_talking_heads_takes_mma", "tib_talking_heads_takes_step", "tib_talking_heads_key_span",
-                   "tib_talking_heads_tiles_per_part", "tib_conv_norm_append", "tib_matrix_memory", "tib_matrix_memory_tile",
-                   "tib_matrix_memory_chunk", "tib_matrix_memory_max_dim", "tib_matrix_memory_takes_chunks"):
-            getattr(library, fn).restype = c_int
-        _signatures_set = True
-    return library
+class _Library:
+    """The CUDA library's functions by name, as packed calls."""
+
+    def __getattr__(self, name: str) -> _Packed:
+        found = _Packed(load_library(), name)
+        setattr(self, name, found)      # (asked for once)
+        return found
+
+
+_library = _Library()
+
+
+def lib() -> _Library:
+    return _library
 
 
 # ---------------------------------------------------------------------------
@@ -154,9 +154,9 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor, *, scal
         if position_table.dim() != 2 or position_table.shape[1] != hidden or positions.numel() != n:
             raise KernelError("embedding: the table of positions does not fit")
     _check("embedding", lib().tib_embedding(
-        _ptr(ids), _ptr(table), _ptr(out), c_int(n), c_int(hidden), c_int(vocab), c_float(scale),
+        _ptr(ids), _ptr(table), _ptr(out), n, hidden, vocab, scale,
         _ptr(positions if position_table is not None else None), _ptr(position_table),
-        c_int(position_table.shape[0] if position_table is not None else 0), c_int(_code(table.dtype)), _stream()))
+        position_table.shape[0] if position_table is not None else 0, _code(table.dtype), _stream()))
     return out
 
 
@@ -179,8 +179,8 @@ def add_rmsnorm(delta: torch.Tensor | None, residual: torch.Tensor, weight: torc
     if out.shape != (n_out, hidden) or weight.numel() != hidden:
         raise KernelError(f"add_rmsnorm: out {tuple(out.shape)} / weight {tuple(weight.shape)} do not fit {(n_out, hidden)}")
     _check("add_rmsnorm", lib().tib_add_rmsnorm(_ptr(delta), _ptr(residual), _ptr(rows), _ptr(weight), _ptr(out),
-                                                c_int(n_out), c_int(hidden), c_float(eps),
-                                                c_int(_code(out.dtype)), _stream()))
+                                                n_out, hidden, eps,
+                                                _code(out.dtype), _stream()))
     return out
 
 
@@ -198,8 +198,8 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
     n_rows = x.numel() // hidden if hidden else 0
     if out.shape != x.shape or weight.numel() != hidden:
         raise KernelError("rmsnorm: shapes do not fit")
-    _check("rmsnorm", lib().tib_rmsnorm(_ptr(x), c_int64(ldx), _ptr(weight), _ptr(out), c_int(n_rows), c_int(hidden),
-                                        c_float(eps), c_int(_code(x.dtype)), _stream()))
+    _check("rmsnorm", lib().tib_rmsnorm(_ptr(x), ldx, _ptr(weight), _ptr(out), n_rows, hidden,
+                                        eps, _code(x.dtype), _stream()))
     return out
 
 
@@ -210,8 +210,8 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, interleaved: bool = False) 
     n, two_i = gate_up.shape
     if two_i % 2 or out.shape != (n, two_i // 2):
         raise KernelError("swiglu: shapes do not fit")
-    _check("swiglu", lib().tib_swiglu(_ptr(gate_up), _ptr(out), c_int(n), c_int(two_i // 2),
-                                      c_int(_code(gate_up.dtype)), c_int(int(interleaved)), _stream()))
+    _check("swiglu", lib().tib_swiglu(_ptr(gate_up), _ptr(out), n, two_i // 2,
+                                      _code(gate_up.dtype), int(interleaved), _stream()))
     return out
 
 
@@ -219,8 +219,8 @@ def cast(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     _need(x, "x"), _need(out, "out")
     if x.numel() != out.numel():
         raise KernelError("cast: sizes differ")
-    _check("cast", lib().tib_cast(_ptr(x), _ptr(out), c_int64(x.numel()), c_int(_code(x.dtype)),
-                                  c_int(_code(out.dtype)), _stream()))
+    _check("cast", lib().tib_cast(_ptr(x), _ptr(out), x.numel(), _code(x.dtype),
+                                  _code(out.dtype), _stream()))
     return out
 
 
@@ -255,9 +255,9 @@ def rope_append(qkv: torch.Tensor, q_out: torch.Tensor, pool: torch.Tensor | Non
         table_stride = block_table.stride(0)
     _check("rope_append", lib().tib_rope_append(
         _ptr(qkv), _ptr(q_out), _ptr(pool), _ptr(positions), _ptr(token_slot), _ptr(block_table),
-        c_int(table_stride), _ptr(inv_freq), c_int(n), c_int(heads), c_int(kv_heads), c_int(head_dim),
-        c_int(rot), c_int(int(interleaved)), c_int(page_size), c_int64(page_stride), c_int(num_pages),
-        c_int(int(write_kv)), _ptr(error_word), c_int(_code(qkv.dtype)), _stream()))
+        table_stride, _ptr(inv_freq), n, heads, kv_heads, head_dim,
+        rot, int(interleaved), page_size, page_stride, num_pages,
+        int(write_kv), _ptr(error_word), _code(qkv.dtype), _stream()))
     return q_out
 
 
@@ -277,9 +277,9 @@ def paged_attention_simt(q: torch.Tensor, pool: torch.Tensor, out: torch.Tensor,
         raise KernelError("paged_attention: entry arrays are shorter than n_entries")
     _check("paged_attention_simt", lib().tib_paged_attention_simt(
         _ptr(q), _ptr(pool), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(block_table),
-        c_int(block_table.stride(0)), c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(kv_heads),
-        c_int(head_dim), c_int(pool.shape[3]), c_int64(pool.stride(0)), c_int(pool.shape[0]), c_int(window),
-        c_float(scale), _ptr(error_word), c_int(_code(q.dtype)), _stream()))
+        block_table.stride(0), n_entries, max_q_len, heads, kv_heads,
+        head_dim, pool.shape[3], pool.stride(0), pool.shape[0], window,
+        scale, _ptr(error_word), _code(q.dtype), _stream()))
     return out
 
 
@@ -300,18 +300,18 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error_word: to
     if k != k2 or out.shape != (m, n):
         raise KernelError(f"gemm_f32: shapes {tuple(x.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
     if x.dtype == w.dtype == torch.float32 and n * k >= F32_TERMS_WEIGHTS and m and lib().tib_gemm_f32_tcgen05_takes(
-            _ptr(x), _ptr(w), c_int(n), c_int(k), c_int64(x.stride(0)), c_int64(w.stride(0))):
+            _ptr(x), _ptr(w), n, k, x.stride(0), w.stride(0)):
         rows = min(m, max(128, F32_TERMS_BYTES // (6 * k)))
         scratch = torch.empty(3 * rows * k, dtype=torch.bfloat16, device=x.device)
         launches = c_int(0)
-        _check("gemm_f32", lib().tib_gemm_f32_tcgen05(_ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k), c_int64(x.stride(0)),
-                                                      c_int64(w.stride(0)), c_int64(out.stride(0)), _ptr(scratch), c_int(rows),
-                                                      _ptr(error_word), ctypes.byref(launches), _stream()))
+        _check("gemm_f32", lib().tib_gemm_f32_tcgen05(_ptr(x), _ptr(w), _ptr(out), m, n, k, x.stride(0),
+                                                      w.stride(0), out.stride(0), _ptr(scratch), rows,
+                                                      _ptr(error_word), ctypes.addressof(launches), _stream()))
         count_launches(launches.value - 1)
         return out
-    _check("gemm_f32", lib().tib_gemm_f32(_ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k),
-                                          c_int64(x.stride(0)), c_int64(w.stride(0)), c_int64(out.stride(0)),
-                                          c_int(_code(x.dtype)), c_int(_code(w.dtype)), _stream()))
+    _check("gemm_f32", lib().tib_gemm_f32(_ptr(x), _ptr(w), _ptr(out), m, n, k,
+                                          x.stride(0), w.stride(0), out.stride(0),
+                                          _code(x.dtype), _code(w.dtype), _stream()))
     return out
 
 
@@ -333,8 +333,8 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: torch.Tensor | 
             raise KernelError("sample: a per-row array is shorter than the number of rows")
     if out.numel() < n:
         raise KernelError("sample: out is too short")
-    _check("sample", lib().tib_sample(_ptr(logits), c_int64(logits.stride(0)), _ptr(temperature), _ptr(seeds),
-                                      _ptr(positions), _ptr(out), c_int(n), c_int(vocab), _stream()))
+    _check("sample", lib().tib_sample(_ptr(logits), logits.stride(0), _ptr(temperature), _ptr(seeds),
+                                      _ptr(positions), _ptr(out), n, vocab, _stream()))
     return out
 
 
@@ -343,8 +343,8 @@ def scatter_i32(dst: torch.Tensor, index: torch.Tensor, value: torch.Tensor) -> 
     _need(dst, "dst", torch.int32), _need(index, "index", torch.int32), _need(value, "value", torch.int32)
     if index.numel() != value.numel():
         raise KernelError("scatter_i32: index and value differ in length")
-    _check("scatter_i32", lib().tib_scatter_i32(_ptr(dst), _ptr(index), _ptr(value), c_int(index.numel()),
-                                                c_int64(dst.numel()), _stream()))
+    _check("scatter_i32", lib().tib_scatter_i32(_ptr(dst), _ptr(index), _ptr(value), index.numel(),
+                                                dst.numel(), _stream()))
     return dst
 
 
@@ -370,8 +370,8 @@ def sample_records(logits: torch.Tensor, out: torch.Tensor, records: torch.Tenso
         _need(history, "history", torch.int32)
     if out.numel() < n or record_slots.numel() < n or (history is not None and history.numel() < n):
         raise KernelError("sample: a per-row array is shorter than the number of rows")
-    _check("sample", lib().tib_sample_records(_ptr(logits), c_int64(logits.stride(0)), _ptr(records), _ptr(record_slots),
-                                              c_int(records.shape[0]), _ptr(out), _ptr(history), c_int(n), c_int(vocab), _stream()))
+    _check("sample", lib().tib_sample_records(_ptr(logits), logits.stride(0), _ptr(records), _ptr(record_slots),
+                                              records.shape[0], _ptr(out), _ptr(history), n, vocab, _stream()))
     return out
 
 
@@ -383,13 +383,13 @@ def decode_inputs(records: torch.Tensor, slots: torch.Tensor, token_ids: torch.T
         _need(t, name, torch.int32)
         if t.numel() < n:
             raise KernelError(f"decode_inputs: {name} is shorter than slots")
-    _check("decode_inputs", lib().tib_decode_inputs(_ptr(records), _ptr(slots), c_int(records.shape[0]), _ptr(token_ids),
-                                                    _ptr(positions), c_int(n), _stream()))
+    _check("decode_inputs", lib().tib_decode_inputs(_ptr(records), _ptr(slots), records.shape[0], _ptr(token_ids),
+                                                    _ptr(positions), n, _stream()))
 
 
 def attention_mma_supports(head_dim: int, group: int) -> bool:
     """Whether the tensor-core attention kernels are built for this head size and group size."""
-    return bool(lib().tib_attention_mma_supports(c_int(head_dim), c_int(group)))
+    return bool(lib().tib_attention_mma_supports(head_dim, group))
 
 
 def _check_attention_args(q, pool, out, q_start, kv_start, slots, block_table, n_entries, heads, kv_heads, head_dim):
@@ -412,9 +412,9 @@ def prefill_attention(q: torch.Tensor, pool: torch.Tensor, out: torch.Tensor, q_
     _check_attention_args(q, pool, out, q_start, kv_start, slots, block_table, n_entries, heads, kv_heads, head_dim)
     _check("prefill_attention", lib().tib_prefill_attention(
         _ptr(q), _ptr(pool), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(block_table),
-        c_int(block_table.stride(0)), c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(kv_heads), c_int(head_dim),
-        c_int(pool.shape[3]), c_int64(pool.stride(0)), c_int(pool.shape[0]), c_int(window), c_float(scale),
-        c_int(int(skip_single)), _stream()))
+        block_table.stride(0), n_entries, max_q_len, heads, kv_heads, head_dim,
+        pool.shape[3], pool.stride(0), pool.shape[0], window, scale,
+        int(skip_single), _stream()))
     return out
 
 
@@ -440,9 +440,9 @@ def plan_attention(head_dim: int, group: int, page_size: int, packed: bool, n_en
     """(kernel for the portions of prompts, kernel for the single tokens) of a bfloat16 step, as the CUDA library
     chooses them: the one place where that is decided, for the part-by-part sequence and the native block alike."""
     prefill, decode = c_int(0), c_int(0)
-    _check("plan_attention", lib().tib_plan_attention(c_int(head_dim), c_int(group), c_int(page_size), c_int(int(packed)),
-                                                      c_int(n_entries), c_int(n_single), c_int(n_multi), c_int(allow),
-                                                      ctypes.byref(prefill), ctypes.byref(decode)))
+    _check("plan_attention", lib().tib_plan_attention(head_dim, group, page_size, int(packed),
+                                                      n_entries, n_single, n_multi, allow,
+                                                      ctypes.addressof(prefill), ctypes.addressof(decode)))
     return prefill.value, decode.value
 
 
@@ -450,8 +450,8 @@ def plan_product(rows: int, n: int, k: int, kn: bool, few_rows: int, features: i
                  aligned: bool) -> int:
     """The kernel a bf16 product of ``rows`` rows goes to (PRODUCT_*), chosen in the same place for both ways of
     running a block."""
-    return int(lib().tib_plan_product(c_int(rows), c_int(n), c_int(k), c_int(int(kn)), c_int(few_rows), c_int(features),
-                                      c_int(splits), c_int(int(swiglu)), c_int(int(aligned))))
+    return int(lib().tib_plan_product(rows, n, k, int(kn), few_rows, features,
+                                      splits, int(swiglu), int(aligned)))
 
 
 def decode_num_splits(n_entries: int, heads: int, kv_heads: int, max_kv_len: int | None = None,
@@ -524,16 +524,16 @@ def decode_attention(q: torch.Tensor, pool: torch.Tensor, out: torch.Tensor, q_s
     if tma:
         _check("decode_attention_tma", lib().tib_decode_attention_tma(
             _ptr(q), _ptr(pool), _ptr(out), _ptr(scratch_o), _ptr(scratch_ml), _ptr(q_start), _ptr(kv_start), _ptr(slots),
-            _ptr(block_table), c_int(block_table.stride(0)), c_int(n_entries), c_int(heads), c_int(kv_heads), c_int(head_dim),
-            c_int(pool.shape[3]), c_int64(pool.stride(0)), c_int(pool.shape[0]), c_int(window), c_float(scale),
-            c_int(num_splits), c_int(chunk), _ptr(_split_counters(q.device, n_entries * kv_heads) if num_splits > 1 else None),
+            _ptr(block_table), block_table.stride(0), n_entries, heads, kv_heads, head_dim,
+            pool.shape[3], pool.stride(0), pool.shape[0], window, scale,
+            num_splits, chunk, _ptr(_split_counters(q.device, n_entries * kv_heads) if num_splits > 1 else None),
             _ptr(error_word), _stream()))
         return out
     _check("decode_attention", lib().tib_decode_attention(
         _ptr(q), _ptr(pool), _ptr(out), _ptr(scratch_o), _ptr(scratch_ml), _ptr(q_start), _ptr(kv_start), _ptr(slots),
-        _ptr(block_table), c_int(block_table.stride(0)), c_int(n_entries), c_int(heads), c_int(kv_heads), c_int(head_dim),
-        c_int(pool.shape[3]), c_int64(pool.stride(0)), c_int(pool.shape[0]), c_int(window), c_float(scale),
-        c_int(num_splits), c_int(chunk), _stream()))
+        _ptr(block_table), block_table.stride(0), n_entries, heads, kv_heads, head_dim,
+        pool.shape[3], pool.stride(0), pool.shape[0], window, scale,
+        num_splits, chunk, _stream()))
     return out
 
 
@@ -576,10 +576,10 @@ def decode_attention_rope(qkv: torch.Tensor, pool: torch.Tensor, out: torch.Tens
         scratch_o, scratch_ml = scratch, scratch[n_entries * heads * num_splits * head_dim:]
     _check("decode_attention_tma_rope", lib().tib_decode_attention_tma_rope(
         _ptr(qkv), _ptr(pool), _ptr(out), _ptr(scratch_o), _ptr(scratch_ml), _ptr(q_start), _ptr(kv_start), _ptr(slots),
-        _ptr(block_table), c_int(block_table.stride(0)), c_int(n_entries), c_int(heads), c_int(kv_heads), c_int(head_dim),
-        c_int(pool.shape[3]), c_int64(pool.stride(0)), c_int(pool.shape[0]), c_int(window), c_float(scale),
-        c_int(num_splits), c_int(0), _ptr(_split_counters(qkv.device, n_entries * kv_heads) if num_splits > 1 else None),
-        _ptr(error_word), _ptr(inv_freq), c_int(rot), c_int(int(interleaved)), _stream()))
+        _ptr(block_table), block_table.stride(0), n_entries, heads, kv_heads, head_dim,
+        pool.shape[3], pool.stride(0), pool.shape[0], window, scale,
+        num_splits, 0, _ptr(_split_counters(qkv.device, n_entries * kv_heads) if num_splits > 1 else None),
+        _ptr(error_word), _ptr(inv_freq), rot, int(interleaved), _stream()))
     return out
 
 
@@ -599,7 +599,7 @@ def _split_counters(device: torch.device, n: int) -> torch.Tensor | None:
 
 
 def decode_attention_tma_supports(head_dim: int, group: int, page_size: int) -> bool:
-    return bool(lib().tib_decode_attention_tma_supports(c_int(head_dim), c_int(group), c_int(page_size)))
+    return bool(lib().tib_decode_attention_tma_supports(head_dim, group, page_size))
 
 
 _blas_workspace: dict[int, torch.Tensor] = {}
@@ -612,7 +612,7 @@ def library_gemm_ready(device: torch.device) -> None:
     if index not in _blas_workspace:
         buffer = torch.empty(BLAS_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
         with torch.cuda.device(index):
-            status = lib().tib_blas_init(_ptr(buffer), ctypes.c_size_t(buffer.numel()))
+            status = lib().tib_blas_init(_ptr(buffer), buffer.numel())
         if status:
             raise KernelError(f"library_gemm: cuBLAS could not be set up (status {status})")
         _blas_workspace[index] = buffer
@@ -622,23 +622,23 @@ def library_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_kn: bool
     """out[M, N] (bf16 or fp32) = x[M, K] . w^T by cuBLAS, called from the engine's own library: ``w`` is stored
     [N, K], or [K, N] when ``w_kn``.  The library's workspace is a buffer of this module, made at the first call on
     a device (make that call outside a stream capture)."""
-    library_gemm_ready(x.device)
-    m, k = x.shape
-    n = w.shape[1] if w_kn else w.shape[0]
-    if (w.shape[0] if w_kn else w.shape[1]) != k or out.shape != (m, n):
+    if x.device.index not in _blas_workspace:
+        library_gemm_ready(x.device)
+    (m, k), (rows, cols) = x.shape, w.shape
+    n, depth = (cols, rows) if w_kn else (rows, cols)
+    if depth != k or out.shape != (m, n):
         raise KernelError(f"library_gemm: shapes {tuple(x.shape)}, {tuple(w.shape)} (kn={w_kn}), {tuple(out.shape)} do not fit")
-    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
+    (ldx, unit_x), (ldw, unit_w), (ldo, unit_out) = x.stride(), w.stride(), out.stride()
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or unit_x != 1 or unit_w != 1 or unit_out != 1:
         raise KernelError("library_gemm: bf16 operands with unit inner stride are needed")
-    status = lib().tib_blas_gemm(_ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k), c_int64(x.stride(0)),
-                                 c_int64(w.stride(0)), c_int64(out.stride(0)), c_int(1 if w_kn else 0),
-                                 c_int(_code(out.dtype)), _stream())
+    status = lib().tib_blas_gemm(x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, ldx, ldw, ldo, 1 if w_kn else 0, _code(out.dtype), _stream())
     if status:
         raise KernelError(f"library_gemm: status {status} (20000 + n: cuBLAS status n)")
     return out        # (a library kernel: not counted among this library's launches)
 
 
 def gemm_tcgen05_supports(m: int, n: int, k: int) -> bool:
-    return bool(lib().tib_gemm_tcgen05_supports(c_int(m), c_int(n), c_int(k)))
+    return bool(lib().tib_gemm_tcgen05_supports(m, n, k))
 
 
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error_word: torch.Tensor | None = None) -> torch.Tensor:
@@ -650,14 +650,14 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error_word
     (m, k), (n, k2) = x.shape, w.shape
     if k != k2 or out.shape != (m, n):
         raise KernelError(f"gemm_tcgen05: shapes {tuple(x.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
-    _check("gemm_tcgen05", lib().tib_gemm_tcgen05(_ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k),
-                                                  c_int64(x.stride(0)), c_int64(w.stride(0)), c_int64(out.stride(0)),
-                                                  c_int(_code(out.dtype)), _ptr(error_word), _stream()))
+    _check("gemm_tcgen05", lib().tib_gemm_tcgen05(_ptr(x), _ptr(w), _ptr(out), m, n, k,
+                                                  x.stride(0), w.stride(0), out.stride(0),
+                                                  _code(out.dtype), _ptr(error_word), _stream()))
     return out
 
 
 def gemm_tcgen05_2cta_supports(m: int, n: int, k: int) -> bool:
-    return bool(lib().tib_gemm_tcgen05_2cta_supports(c_int(m), c_int(n), c_int(k)))
+    return bool(lib().tib_gemm_tcgen05_2cta_supports(m, n, k))
 
 
 def gemm_tcgen05_2cta(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error_word: torch.Tensor | None = None) -> torch.Tensor:
@@ -669,14 +669,14 @@ def gemm_tcgen05_2cta(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error
     (m, k), (n, k2) = x.shape, w.shape
     if k != k2 or out.shape != (m, n):
         raise KernelError(f"gemm_tcgen05_2cta: shapes {tuple(x.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
-    _check("gemm_tcgen05_2cta", lib().tib_gemm_tcgen05_2cta(_ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k),
-                                                            c_int64(x.stride(0)), c_int64(w.stride(0)), c_int64(out.stride(0)),
-                                                            c_int(_code(out.dtype)), _ptr(error_word), _stream()))
+    _check("gemm_tcgen05_2cta", lib().tib_gemm_tcgen05_2cta(_ptr(x), _ptr(w), _ptr(out), m, n, k,
+                                                            x.stride(0), w.stride(0), out.stride(0),
+                                                            _code(out.dtype), _ptr(error_word), _stream()))
     return out
 
 
 def gemm_tcgen05_swapab_supports(m: int, n: int, k: int) -> bool:
-    return bool(lib().tib_gemm_tcgen05_swapab_supports(c_int(m), c_int(n), c_int(k)))
+    return bool(lib().tib_gemm_tcgen05_swapab_supports(m, n, k))
 
 
 def gemm_tcgen05_swapab(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error_word: torch.Tensor | None = None,
@@ -693,8 +693,8 @@ def gemm_tcgen05_swapab(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, err
     if k != k2 or out.shape != (m, n):
         raise KernelError(f"gemm_tcgen05_swapab: shapes {tuple(x.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
     _check("gemm_tcgen05_swapab", lib().tib_gemm_tcgen05_swapab(
-        _ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k), c_int64(x.stride(0)), c_int64(w.stride(0)),
-        c_int64(out.stride(0)), c_int(int(w_kn)), c_int(_code(out.dtype)), c_int(splits), _ptr(error_word), _stream()))
+        _ptr(x), _ptr(w), _ptr(out), m, n, k, x.stride(0), w.stride(0),
+        out.stride(0), int(w_kn), _code(out.dtype), splits, _ptr(error_word), _stream()))
     return out
 
 
@@ -702,7 +702,7 @@ DG_PLAIN, DG_SWIGLU = 0, 1
 
 
 def gemm_decode_supports(m: int, n: int, k: int, features: int = 128, splits: int = 1, epilogue: int = DG_PLAIN) -> bool:
-    return bool(lib().tib_gemm_decode_supports(c_int(m), c_int(n), c_int(k), c_int(features), c_int(splits), c_int(epilogue)))
+    return bool(lib().tib_gemm_decode_supports(m, n, k, features, splits, epilogue))
 
 
 def gemm_decode(x: torch.Tensor, w_kn: torch.Tensor, out: torch.Tensor, *, features: int = 128, splits: int = 1,
@@ -719,14 +719,14 @@ def gemm_decode(x: torch.Tensor, w_kn: torch.Tensor, out: torch.Tensor, *, featu
     if k != k2 or out.shape != (m, n // 2 if epilogue == DG_SWIGLU else n):
         raise KernelError(f"gemm_decode: shapes {tuple(x.shape)} x {tuple(w_kn.shape)} -> {tuple(out.shape)} do not fit")
     _check("gemm_decode", lib().tib_gemm_decode(
-        _ptr(x), _ptr(w_kn), _ptr(out), c_int(m), c_int(n), c_int(k), c_int64(x.stride(0)), c_int64(w_kn.stride(0)),
-        c_int64(out.stride(0)), c_int(_code(out.dtype)), c_int(features), c_int(splits), c_int(epilogue), c_int(stages),
+        _ptr(x), _ptr(w_kn), _ptr(out), m, n, k, x.stride(0), w_kn.stride(0),
+        out.stride(0), _code(out.dtype), features, splits, epilogue, stages,
         _ptr(error_word), _stream()))
     return out
 
 
 def prefill_attention_tcgen05_supports(head_dim: int, group: int, page_size: int) -> bool:
-    return bool(lib().tib_prefill_attention_tcgen05_supports(c_int(head_dim), c_int(group), c_int(page_size)))
+    return bool(lib().tib_prefill_attention_tcgen05_supports(head_dim, group, page_size))
 
 
 def prefill_attention_tcgen05(q: torch.Tensor, pool: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
@@ -738,9 +738,9 @@ def prefill_attention_tcgen05(q: torch.Tensor, pool: torch.Tensor, out: torch.Te
     _check_attention_args(q, pool, out, q_start, kv_start, slots, block_table, n_entries, heads, kv_heads, head_dim)
     _check("prefill_attention_tcgen05", lib().tib_prefill_attention_tcgen05(
         _ptr(q), _ptr(pool), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(block_table),
-        c_int(block_table.stride(0)), c_int(n_entries), c_int(max_q_len), c_int(q.numel() // (heads * head_dim)),
-        c_int(heads), c_int(kv_heads), c_int(head_dim), c_int(pool.shape[3]), c_int64(pool.stride(0)), c_int(pool.shape[0]),
-        c_int(window), c_float(scale), c_int(int(skip_single)), _ptr(error_word), _stream()))
+        block_table.stride(0), n_entries, max_q_len, q.numel() // (heads * head_dim),
+        heads, kv_heads, head_dim, pool.shape[3], pool.stride(0), pool.shape[0],
+        window, scale, int(skip_single), _ptr(error_word), _stream()))
     return out
 
 
@@ -769,9 +769,9 @@ def add_pair(residual: torch.Tensor, a: torch.Tensor, b: torch.Tensor | None = N
     if a.shape[0] != n or (b is not None and b.shape[0] != n):
         raise KernelError("add_pair: row counts differ")
     _check("add_pair", lib().tib_add_pair(
-        _ptr(residual), _ptr(a), c_int(_code(a.dtype)), c_int64(a.stride(0)), _ptr(b),
-        c_int(_code(b.dtype) if b is not None else 0), c_int64(b.stride(0) if b is not None else 0), _ptr(copy),
-        c_int(_code(copy.dtype) if copy is not None else 0), c_int(n), c_int(width), _stream()))
+        _ptr(residual), _ptr(a), _code(a.dtype), a.stride(0), _ptr(b),
+        _code(b.dtype) if b is not None else 0, b.stride(0) if b is not None else 0, _ptr(copy),
+        _code(copy.dtype) if copy is not None else 0, n, width, _stream()))
     return residual
 
 
@@ -788,9 +788,9 @@ def unit_norm_add(residual: torch.Tensor, y: torch.Tensor, weight: torch.Tensor,
         _need(copy, "copy")
         if copy.shape != residual.shape:
             raise KernelError("unit_norm_add: copy does not fit")
-    _check("unit_norm_add", lib().tib_unit_norm_add(_ptr(residual), _ptr(y), c_int(_code(y.dtype)), c_int64(y.stride(0)),
-                                                    _ptr(weight), c_int(n), c_int(width), c_float(eps), c_float(scale),
-                                                    _ptr(copy), c_int(_code(copy.dtype) if copy is not None else 0), _stream()))
+    _check("unit_norm_add", lib().tib_unit_norm_add(_ptr(residual), _ptr(y), _code(y.dtype), y.stride(0),
+                                                    _ptr(weight), n, width, eps, scale,
+                                                    _ptr(copy), _code(copy.dtype) if copy is not None else 0, _stream()))
     return residual
 
 
@@ -810,8 +810,8 @@ def sigmoid_gate(x: torch.Tensor, gate: torch.Tensor, out: torch.Tensor, weight:
     if x.shape[0] != n or gate.shape[0] != n:
         raise KernelError("sigmoid_gate: row counts differ")
     _check("sigmoid_gate", lib().tib_sigmoid_gate(
-        _ptr(x), c_int(_code(x.dtype)), c_int64(x.stride(0)), _ptr(gate), c_int(_code(gate.dtype)), c_int64(gate.stride(0)),
-        _ptr(weight), c_float(eps), _ptr(out), c_int(_code(out.dtype)), c_int(n), c_int(width), c_int(group), _stream()))
+        _ptr(x), _code(x.dtype), x.stride(0), _ptr(gate), _code(gate.dtype), gate.stride(0),
+        _ptr(weight), eps, _ptr(out), _code(out.dtype), n, width, group, _stream()))
     return out
 
 
@@ -823,9 +823,9 @@ def gelu_gate_table(a: torch.Tensor, ids: torch.Tensor, table: torch.Tensor, fir
     if a.shape[0] != n or ids.numel() != n or first < 0 or first + width > table.shape[1]:
         raise KernelError("gelu_gate_table: shapes do not fit")
     _check("gelu_gate_table", lib().tib_gelu_gate_table(
-        _ptr(a), c_int(_code(a.dtype)), c_int64(a.stride(0)), _ptr(ids), _ptr(table), c_int(_code(table.dtype)),
-        c_int64(table.stride(0)), c_int(table.shape[0]), c_int(first), _ptr(out), c_int(_code(out.dtype)), c_int(n),
-        c_int(width), _stream()))
+        _ptr(a), _code(a.dtype), a.stride(0), _ptr(ids), _ptr(table), _code(table.dtype),
+        table.stride(0), table.shape[0], first, _ptr(out), _code(out.dtype), n,
+        width, _stream()))
     return out
 
 
@@ -833,8 +833,8 @@ def relu_squared(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     _need(x, "x"), _need(out, "out")
     if x.numel() != out.numel():
         raise KernelError("relu_squared: sizes differ")
-    _check("relu_squared", lib().tib_relu_squared(_ptr(x), c_int(_code(x.dtype)), _ptr(out), c_int(_code(out.dtype)),
-                                                  c_int64(x.numel()), _stream()))
+    _check("relu_squared", lib().tib_relu_squared(_ptr(x), _code(x.dtype), _ptr(out), _code(out.dtype),
+                                                  x.numel(), _stream()))
     return out
 
 
@@ -843,14 +843,14 @@ def gelu(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     _need(x, "x"), _need(out, "out")
     if x.numel() != out.numel():
         raise KernelError("gelu: sizes differ")
-    _check("gelu", lib().tib_gelu(_ptr(x), c_int(_code(x.dtype)), _ptr(out), c_int(_code(out.dtype)), c_int64(x.numel()), _stream()))
+    _check("gelu", lib().tib_gelu(_ptr(x), _code(x.dtype), _ptr(out), _code(out.dtype), x.numel(), _stream()))
     return out
 
 
 def scale_(x: torch.Tensor, factor: float) -> torch.Tensor:
     """x *= factor (fp32, in place)."""
     _need(x, "x", torch.float32)
-    _check("scale", lib().tib_scale_f32(_ptr(x), c_float(factor), c_int64(x.numel()), _stream()))
+    _check("scale", lib().tib_scale_f32(_ptr(x), factor, x.numel(), _stream()))
     return x
 
 
@@ -860,7 +860,7 @@ def pair_rows(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor) -> torch.Tens
     n, width = x.shape
     if y.shape != x.shape or out.shape != (n, 2 * width):
         raise KernelError("pair_rows: shapes do not fit")
-    _check("pair_rows", lib().tib_pair_rows(_ptr(x), _ptr(y), _ptr(out), c_int(_code(out.dtype)), c_int(n), c_int(width), _stream()))
+    _check("pair_rows", lib().tib_pair_rows(_ptr(x), _ptr(y), _ptr(out), _code(out.dtype), n, width, _stream()))
     return out
 
 
@@ -874,8 +874,8 @@ def add_vector(x: torch.Tensor, v: torch.Tensor, delta: torch.Tensor | None = No
         if delta.shape[0] != x.shape[0]:
             raise KernelError("add_vector: delta does not fit")
     _check("add_vector", lib().tib_add_vector(
-        _ptr(x), _ptr(delta), c_int(_code(delta.dtype) if delta is not None else 0),
-        c_int64(delta.stride(0) if delta is not None else 0), _ptr(v), c_int(x.shape[0]), c_int(x.shape[1]), _stream()))
+        _ptr(x), _ptr(delta), _code(delta.dtype) if delta is not None else 0,
+        delta.stride(0) if delta is not None else 0, _ptr(v), x.shape[0], x.shape[1], _stream()))
     return x
 
 
@@ -891,9 +891,9 @@ def library_gemm_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.stride(2) != 1 or w.stride(2) != 1 or out.stride(2) != 1:
         raise KernelError("library_gemm_batched: bf16 operands with unit inner stride are needed")
     status = lib().tib_blas_gemm_batched(
-        _ptr(x), _ptr(w), _ptr(out), c_int(m), c_int(n), c_int(k), c_int64(x.stride(0)), c_int64(w.stride(1)),
-        c_int64(out.stride(0)), c_int64(x.stride(1)), c_int64(w.stride(0)), c_int64(out.stride(1)), c_int(batch),
-        c_int(1 if w_kn else 0), c_int(_code(out.dtype)), _stream())
+        _ptr(x), _ptr(w), _ptr(out), m, n, k, x.stride(0), w.stride(1),
+        out.stride(0), x.stride(1), w.stride(0), out.stride(1), batch,
+        1 if w_kn else 0, _code(out.dtype), _stream())
     if status:
         raise KernelError(f"library_gemm_batched: status {status} (20000 + n: cuBLAS status n)")
     return out
@@ -902,7 +902,7 @@ def library_gemm_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_
 # ---------------------------------------------------------------------------
 def linear_attention_chunk(key_dim: int, value_dim: int) -> int:
     """Tokens per chunk of the decayed linear attention kernel for these head sizes (0: they do not fit an SM)."""
-    return int(lib().tib_linear_attention_chunk(c_int(key_dim), c_int(value_dim)))
+    return int(lib().tib_linear_attention_chunk(key_dim, value_dim))
 
 
 @functools.lru_cache(maxsize=None)
@@ -914,7 +914,7 @@ def linear_attention_run() -> int:
 @functools.lru_cache(maxsize=None)
 def linear_attention_forms(key_dim: int, value_dim: int) -> tuple[int, int]:
     """(the longest portion that is walked token by token, the shortest that is cut into runs) in heads of these sizes."""
-    return int(lib().tib_linear_attention_walk()), int(lib().tib_linear_attention_runs_from(c_int(key_dim), c_int(value_dim)))
+    return int(lib().tib_linear_attention_walk()), int(lib().tib_linear_attention_runs_from(key_dim, value_dim))
 
 
 # Bytes of run states that a call makes room for at a time: 2,048 tokens of 16 heads of 128 x 128 take 34 MB, and what is above the
@@ -963,10 +963,10 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tor
             run_state = torch.empty(capacity * run_heads * key_dim * value_dim, dtype=torch.float32, device=q.device)
     launches = c_int(0)
     _check("linear_attention", lib().tib_linear_attention(
-        _ptr(q), _ptr(k), _ptr(v), c_int64(q.stride(0)), c_int64(k.stride(0)), c_int64(v.stride(0)), _ptr(out), _ptr(state),
-        _ptr(powers), _ptr(q_start), _ptr(slots), c_int(n_entries), c_int(heads), c_int(key_dim), c_int(value_dim),
-        c_int(chunk), c_int(1 if silu else 0), c_int(_code(q.dtype)), c_int(q.shape[0]), c_int(max_q_len), c_int(forms),
-        c_int(chunked), _ptr(run_powers), _ptr(run_state), c_int64(capacity), c_int(run_heads), ctypes.byref(launches), _ptr(error_word), _stream()))
+        _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(out), _ptr(state),
+        _ptr(powers), _ptr(q_start), _ptr(slots), n_entries, heads, key_dim, value_dim,
+        chunk, 1 if silu else 0, _code(q.dtype), q.shape[0], max_q_len, forms,
+        chunked, _ptr(run_powers), _ptr(run_state), capacity, run_heads, ctypes.addressof(launches), _ptr(error_word), _stream()))
     count_launches(launches.value - 1)      # (_check counted one)
     return out
 
@@ -998,10 +998,10 @@ def latent_append(dkv: torch.Tensor, q: torch.Tensor, folded: torch.Tensor | Non
             raise KernelError(f"latent_append: pages of shape {tuple(keys.shape)} do not fit")
         num_pages, page_size, page_stride, table_stride = keys.shape[0], keys.shape[2], keys.stride(0), block_table.stride(0)
     _check("latent_append", lib().tib_latent_append(
-        _ptr(dkv), c_int64(dkv.stride(0)), _ptr(q), c_int64(q.stride(0)), _ptr(keys), _ptr(folded), _ptr(positions),
-        _ptr(token_slot), _ptr(block_table), c_int(table_stride), _ptr(norm_weight), c_float(eps), _ptr(inv_freq),
-        c_int(inv_freq.numel()), c_int(n), c_int(heads), c_int(dim), c_int(rank), c_int(rot), c_int(page_size),
-        c_int64(page_stride), c_int(num_pages), c_int(int(half_pairs)), _ptr(error_word), c_int(_code(dkv.dtype)), _stream()))
+        _ptr(dkv), dkv.stride(0), _ptr(q), q.stride(0), _ptr(keys), _ptr(folded), _ptr(positions),
+        _ptr(token_slot), _ptr(block_table), table_stride, _ptr(norm_weight), eps, _ptr(inv_freq),
+        inv_freq.numel(), n, heads, dim, rank, rot, page_size,
+        page_stride, num_pages, int(half_pairs), _ptr(error_word), _code(dkv.dtype), _stream()))
 
 
 def latent_attention(folded: torch.Tensor, keys: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor, kv_start: torch.Tensor,
@@ -1035,15 +1035,15 @@ def latent_attention(folded: torch.Tensor, keys: torch.Tensor, out: torch.Tensor
             raise KernelError("latent_attention: sink holds one number per head")
     splits, partial = 1, None
     if max_q_len == 1 and max_kv_len > 0 and n == n_entries:
-        splits = int(lib().tib_latent_attention_splits(c_int(n_entries), c_int(heads), c_int(max_kv_len)))
+        splits = int(lib().tib_latent_attention_splits(n_entries, heads, max_kv_len))
         if splits > 1:
             partial = torch.empty((n, heads, splits, 2 + rank), dtype=torch.float32, device=folded.device)
     _check("latent_attention", lib().tib_latent_attention(
         _ptr(folded), _ptr(keys), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(block_table),
-        c_int(block_table.stride(0)), c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(rank), c_int(rot),
-        c_int(keys.shape[2]), c_int64(keys.stride(0)), c_int(keys.shape[0]), c_float(scale), _ptr(sink), _ptr(partial), c_int(splits),
-        c_int(max_kv_len), c_int(int(force_simt)), _ptr(error_word), c_int(_code(keys.dtype)),
-        _ptr(merged if splits > 1 else None), c_int(first_row), _stream()))
+        block_table.stride(0), n_entries, max_q_len, heads, rank, rot,
+        keys.shape[2], keys.stride(0), keys.shape[0], scale, _ptr(sink), _ptr(partial), splits,
+        max_kv_len, int(force_simt), _ptr(error_word), _code(keys.dtype),
+        _ptr(merged if splits > 1 else None), first_row, _stream()))
     if partial is not None:
         count_launches(1)
     return out if merged is None or splits == 1 else merged
@@ -1054,7 +1054,7 @@ LATENT_TILE = 128      # an entry's keys made for the step are padded to a multi
 
 def latent_prefill_supports(dim: int, value_dim: int, rank: int, rot: int) -> bool:
     """Whether prompt portions of these head sizes may run on keys and values made for the step (bfloat16)."""
-    return bool(lib().tib_latent_prefill_supports(c_int(dim), c_int(value_dim), c_int(rank), c_int(rot)))
+    return bool(lib().tib_latent_prefill_supports(dim, value_dim, rank, rot))
 
 
 def latent_gather(keys: torch.Tensor, block_table: torch.Tensor, q_start: torch.Tensor, kv_start: torch.Tensor, slots: torch.Tensor,
@@ -1073,9 +1073,9 @@ def latent_gather(keys: torch.Tensor, block_table: torch.Tensor, q_start: torch.
     if q_start.numel() < n_entries + 1 or kv_start.numel() < n_entries or slots.numel() < n_entries:
         raise KernelError("latent_gather: entry arrays are shorter than n_entries")
     _check("latent_gather", lib().tib_latent_gather(
-        _ptr(keys), c_int64(keys.stride(0)), c_int(keys.shape[2]), c_int(keys.shape[0]), _ptr(block_table), c_int(block_table.stride(0)),
-        _ptr(q_start), _ptr(kv_start), _ptr(slots), c_int(n_entries), c_int(max_kv_len), _ptr(latent), _ptr(rotated), c_int(latent.shape[0]),
-        c_int(rank), c_int(rot), _ptr(error_word), _stream()))
+        _ptr(keys), keys.stride(0), keys.shape[2], keys.shape[0], _ptr(block_table), block_table.stride(0),
+        _ptr(q_start), _ptr(kv_start), _ptr(slots), n_entries, max_kv_len, _ptr(latent), _ptr(rotated), latent.shape[0],
+        rank, rot, _ptr(error_word), _stream()))
 
 
 def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
@@ -1104,10 +1104,10 @@ def latent_prefill(q: torch.Tensor, kv: torch.Tensor, rotated: torch.Tensor, out
         if sink.numel() != heads:
             raise KernelError("latent_prefill: sink holds one number per head")
     _check("latent_prefill", lib().tib_latent_prefill(
-        _ptr(q), c_int64(q.stride(0)), _ptr(kv), _ptr(rotated), c_int(kv.shape[0]), _ptr(q_start), _ptr(kv_start), c_int(n_entries),
-        c_int(max_q_len), c_int(shortest), c_int(n), c_int(heads), c_int(first_head), c_int(kv.shape[1] // (dim + value_dim)),
-        c_int(dim), c_int(value_dim), c_int(rot), c_float(scale), _ptr(sink), _ptr(gate),
-        c_int64(gate.stride(0) if gate is not None else 0), c_int(int(gate_per_head)), _ptr(out), _ptr(error_word), _stream()))
+        _ptr(q), q.stride(0), _ptr(kv), _ptr(rotated), kv.shape[0], _ptr(q_start), _ptr(kv_start), n_entries,
+        max_q_len, shortest, n, heads, first_head, kv.shape[1] // (dim + value_dim),
+        dim, value_dim, rot, scale, _ptr(sink), _ptr(gate),
+        gate.stride(0) if gate is not None else 0, int(gate_per_head), _ptr(out), _ptr(error_word), _stream()))
     return out
 
 
@@ -1125,8 +1125,8 @@ def router_logits(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: tor
         _need(bias, "bias", torch.float32)
         if bias.numel() != w.shape[0]:
             raise KernelError("router_logits: the bias holds one number per row")
-    _check("router_logits", lib().tib_router_logits(_ptr(x), c_int(_code(x.dtype)), c_int64(x.stride(0)), _ptr(w), _ptr(bias), _ptr(out),
-                                                    c_int64(out.stride(0)), c_int(x.shape[0]), c_int(w.shape[0]), c_int(x.shape[1]),
+    _check("router_logits", lib().tib_router_logits(_ptr(x), _code(x.dtype), x.stride(0), _ptr(w), _ptr(bias), _ptr(out),
+                                                    out.stride(0), x.shape[0], w.shape[0], x.shape[1],
                                                     _stream()))
     return out
 
@@ -1159,10 +1159,10 @@ def moe_route(logits: torch.Tensor, experts: int, top: int, ids: torch.Tensor, w
     if together:
         _moe_sorted_arrays(ids, *sort)
     kept, offsets, order, place = sort if together else (0, None, None, None)
-    _check("moe_route", lib().tib_moe_route(_ptr(logits), c_int64(logits.stride(0)), c_int(n), c_int(experts), c_int(top),
-                                            c_int(int(sigmoid_scores)), c_int(int(normalize)), c_float(norm_eps),
-                                            _ptr(correction), c_int(groups), c_int(keep), _ptr(ids), _ptr(weights),
-                                            c_int(kept), _ptr(offsets), _ptr(order), _ptr(place), _stream()))
+    _check("moe_route", lib().tib_moe_route(_ptr(logits), logits.stride(0), n, experts, top,
+                                            int(sigmoid_scores), int(normalize), norm_eps,
+                                            _ptr(correction), groups, keep, _ptr(ids), _ptr(weights),
+                                            kept, _ptr(offsets), _ptr(order), _ptr(place), _stream()))
     if sort is not None and not together:
         moe_group(ids, *sort)
 
@@ -1180,7 +1180,7 @@ def _moe_sorted_arrays(ids: torch.Tensor, experts: int, offsets: torch.Tensor, o
 def moe_group(ids: torch.Tensor, experts: int, offsets: torch.Tensor, order: torch.Tensor, place: torch.Tensor) -> None:
     """Sort the (token, choice) pairs by expert on the device: offsets [experts + 1], order[sorted] = pair, place[pair] = sorted."""
     pairs = _moe_sorted_arrays(ids, experts, offsets, order, place)
-    _check("moe_group", lib().tib_moe_group(_ptr(ids), c_int(pairs), c_int(experts), _ptr(offsets), _ptr(order), _ptr(place), _stream()))
+    _check("moe_group", lib().tib_moe_group(_ptr(ids), pairs, experts, _ptr(offsets), _ptr(order), _ptr(place), _stream()))
 
 
 def moe_expert_product(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, offsets: torch.Tensor, order: torch.Tensor, top: int,
@@ -1201,9 +1201,9 @@ def moe_expert_product(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, offset
         if row_scale.numel() != pairs:
             raise KernelError("moe_expert_product: row_scale must hold one factor per pair")
     _check("moe_expert_product", lib().tib_moe_expert_product(
-        _ptr(x), c_int(_code(x.dtype)), c_int64(x.stride(0)), _ptr(w), c_int(_code(w.dtype)), _ptr(y), c_int(_code(y.dtype)),
-        c_int64(y.stride(0)), _ptr(offsets), _ptr(order), c_int(pairs), c_int(experts), c_int(top), c_int(int(x_by_pair)),
-        c_int(n), c_int(k), c_int(MOE_ACT[act]), c_float(limit), c_float(alpha), _ptr(row_scale), _ptr(error_word), _stream()))
+        _ptr(x), _code(x.dtype), x.stride(0), _ptr(w), _code(w.dtype), _ptr(y), _code(y.dtype),
+        y.stride(0), _ptr(offsets), _ptr(order), pairs, experts, top, int(x_by_pair),
+        n, k, MOE_ACT[act], limit, alpha, _ptr(row_scale), _ptr(error_word), _stream()))
     return y
 
 
@@ -1242,9 +1242,9 @@ def moe_combine(y: torch.Tensor, place: torch.Tensor, weights: torch.Tensor | No
             raise KernelError("moe_combine: the input rows must have the output's type and row count")
         ldx = x.stride(0)
     _check("moe_combine", lib().tib_moe_combine(
-        _ptr(y), _ptr(place), _ptr(weights), c_int(top), _ptr(shared), c_int(_code(shared.dtype) if shared is not None else 0),
-        _ptr(gate), c_int64(ld_gate), _ptr(out), c_int(_code(out.dtype)), c_int(n), c_int(width), _ptr(ids),
-        c_int(identity_from), _ptr(x if ids is not None else None), c_int64(ldx), _stream()))
+        _ptr(y), _ptr(place), _ptr(weights), top, _ptr(shared), _code(shared.dtype) if shared is not None else 0,
+        _ptr(gate), ld_gate, _ptr(out), _code(out.dtype), n, width, _ptr(ids),
+        identity_from, _ptr(x if ids is not None else None), ldx, _stream()))
     return out
 
 
@@ -1254,8 +1254,8 @@ def glu_clamp(gate_up: torch.Tensor, out: torch.Tensor, limit: float, alpha: flo
     n, width = out.shape
     if gate_up.shape != (n, 2 * width):
         raise KernelError("glu_clamp: gate_up must be [rows, 2 * width]")
-    _check("glu_clamp", lib().tib_glu_clamp(_ptr(gate_up), c_int(_code(gate_up.dtype)), _ptr(out), c_int(_code(out.dtype)), c_int(n),
-                                            c_int(width), c_float(limit), c_float(alpha), _stream()))
+    _check("glu_clamp", lib().tib_glu_clamp(_ptr(gate_up), _code(gate_up.dtype), _ptr(out), _code(out.dtype), n,
+                                            width, limit, alpha, _stream()))
     return out
 
 
@@ -1271,8 +1271,8 @@ def layernorm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: fl
         _need(rows, "rows", torch.int32)
     if out.shape != (n, width) or weight.numel() != width or bias.numel() != width:
         raise KernelError("layernorm: shapes do not fit")
-    _check("layernorm", lib().tib_layernorm(_ptr(x), c_int(_code(x.dtype)), c_int64(x.stride(0)), _ptr(rows), _ptr(weight), _ptr(bias),
-                                            c_float(eps), _ptr(out), c_int(_code(out.dtype)), c_int(n), c_int(width), _stream()))
+    _check("layernorm", lib().tib_layernorm(_ptr(x), _code(x.dtype), x.stride(0), _ptr(rows), _ptr(weight), _ptr(bias),
+                                            eps, _ptr(out), _code(out.dtype), n, width, _stream()))
     return out
 
 
@@ -1307,9 +1307,9 @@ def layernorm_tail(residual: torch.Tensor, eps: float, *, y: torch.Tensor | None
         if out.shape != (n, width) or wb.numel() != width or bb.numel() != width or wb.dtype != torch.float32 or bb.dtype != torch.float32:
             raise KernelError("layernorm_tail: out or its norm do not fit")
     _check("layernorm_tail", lib().tib_layernorm_tail(
-        _ptr(y), c_int(_code(y.dtype) if y is not None else 0), c_int64(y.stride(0) if y is not None else 0), _ptr(wa), _ptr(ba),
-        _ptr(residual), _ptr(history), c_int64(slice_elems), _ptr(coef), c_int(count), _ptr(wb), _ptr(bb), _ptr(out),
-        c_int(_code(out.dtype) if out is not None else 0), c_int(n), c_int(width), c_float(eps), _stream()))
+        _ptr(y), _code(y.dtype) if y is not None else 0, y.stride(0) if y is not None else 0, _ptr(wa), _ptr(ba),
+        _ptr(residual), _ptr(history), slice_elems, _ptr(coef), count, _ptr(wb), _ptr(bb), _ptr(out),
+        _code(out.dtype) if out is not None else 0, n, width, eps, _stream()))
 
 
 # ---------------------------------------------------------------------------
@@ -1343,11 +1343,11 @@ def qk_norm_append(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_out
         if t is not None and (t.dtype != torch.float32 or t.numel() != dim or not t.is_contiguous() or not t.is_cuda):
             raise KernelError(f"qk_norm_append: {name} must be {dim} fp32 numbers")
     _check("qk_norm_append", lib().tib_qk_norm_append(
-        _ptr(proj), c_int64(proj.stride(0)), c_int(q_off), c_int(k_off if write else -1), c_int(v_off), _ptr(q_out),
+        _ptr(proj), proj.stride(0), q_off, k_off if write else -1, v_off, _ptr(q_out),
         _ptr(keys), _ptr(values), _ptr(positions), _ptr(token_slot if write else None), _ptr(block_table if write else None),
-        c_int(table_stride), _ptr(inv_freq), c_int(n), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim), c_int(rot_dim),
-        c_int(int(interleaved)), c_float(eps), c_int(page_size), c_int64(page_stride), c_int(num_pages), _ptr(q_weight),
-        _ptr(k_weight), c_float(temp_coef), c_int(temp_every), _ptr(error_word), c_int(_code(proj.dtype)), _stream()))
+        table_stride, _ptr(inv_freq), n, heads, kv_heads, dim, vdim, rot_dim,
+        int(interleaved), eps, page_size, page_stride, num_pages, _ptr(q_weight),
+        _ptr(k_weight), temp_coef, temp_every, _ptr(error_word), _code(proj.dtype), _stream()))
     return q_out
 
 
@@ -1376,7 +1376,7 @@ def sigmoid_attention(q: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
         _rows_of(gate, "gate", heads)
     partial = None
     if (max_q_len == 1 and q.dtype == torch.bfloat16 and not force_simt
-            and lib().tib_sigmoid_attention_takes_mma(c_int(dim), c_int(vdim))):
+            and lib().tib_sigmoid_attention_takes_mma(dim, vdim)):
         if splits is None:
             seen = min(x for x in (chunk or None, window or None, max_kv_len, 1 << 30) if x)
             tiles = -(-seen // 64) + 1
@@ -1388,11 +1388,11 @@ def sigmoid_attention(q: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
     splits = splits if partial is not None else 0
     _check("sigmoid_attention", lib().tib_sigmoid_attention(
         _ptr(q), _ptr(keys), _ptr(values), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(block_table),
-        c_int(block_table.stride(0)), c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim),
-        c_int(page_size), c_int64(keys.stride(0)), c_int(keys.shape[0]), c_int(chunk), c_int(window), c_float(scale),
-        _ptr(head_bias), _ptr(gate), c_int(_code(gate.dtype) if gate is not None else 0),
-        c_int64(gate.stride(0) if gate is not None else 0), _ptr(error_word), c_int(_code(q.dtype)), c_int(int(force_simt)),
-        c_int(splits), _ptr(partial), _stream()))
+        block_table.stride(0), n_entries, max_q_len, heads, kv_heads, dim, vdim,
+        page_size, keys.stride(0), keys.shape[0], chunk, window, scale,
+        _ptr(head_bias), _ptr(gate), _code(gate.dtype) if gate is not None else 0,
+        gate.stride(0) if gate is not None else 0, _ptr(error_word), _code(q.dtype), int(force_simt),
+        splits, _ptr(partial), _stream()))
     return out
 
 
@@ -1418,9 +1418,9 @@ def gated_recurrence(proj: torch.Tensor, z_off: int, u_off: int, g_off: int, bia
         scratch = torch.empty((2, n_entries, runs, width), dtype=torch.float32, device=out.device)
         run_a, run_b = scratch[0], scratch[1]
     status = lib().tib_gated_recurrence(
-        _ptr(proj), c_int(_code(proj.dtype)), c_int64(proj.stride(0)), c_int(z_off), c_int(u_off), c_int(g_off), _ptr(bias_z),
-        _ptr(bias_u), _ptr(state), _ptr(q_start), _ptr(slots), _ptr(out), c_int(_code(out.dtype)), _ptr(run_a), _ptr(run_b),
-        c_int(n_entries), c_int(max_q_len), c_int(width), c_int(run_len), _stream())
+        _ptr(proj), _code(proj.dtype), proj.stride(0), z_off, u_off, g_off, _ptr(bias_z),
+        _ptr(bias_u), _ptr(state), _ptr(q_start), _ptr(slots), _ptr(out), _code(out.dtype), _ptr(run_a), _ptr(run_b),
+        n_entries, max_q_len, width, run_len, _stream())
     _check("gated_recurrence", status)
     if runs > 1:
         count_launches(1)
@@ -1432,7 +1432,7 @@ def softcap_(x: torch.Tensor, cap: float) -> torch.Tensor:
     _need(x, "x", torch.float32)
     if not cap > 0:
         raise KernelError("softcap: the cap is positive")
-    _check("softcap", lib().tib_softcap_f32(_ptr(x), c_float(cap), c_int64(x.numel()), _stream()))
+    _check("softcap", lib().tib_softcap_f32(_ptr(x), cap, x.numel(), _stream()))
     return x
 
 
@@ -1452,9 +1452,9 @@ def short_conv(rows: torch.Tensor, col: int, weight: torch.Tensor, bias: torch.T
             or state_off < 0 or state_off + (taps - 1) * channels > state.shape[1] or (bias is not None and bias.numel() != channels)):
         raise KernelError("short_conv: shapes do not fit")
     _check("short_conv", lib().tib_short_conv(
-        _ptr(rows), c_int(_code(rows.dtype)), c_int64(rows.stride(0)), c_int(col), _ptr(weight), _ptr(bias), _ptr(state),
-        c_int64(state.stride(0)), c_int64(state_off), _ptr(q_start), _ptr(slots), _ptr(out), c_int(_code(out.dtype)), c_int(channels),
-        c_int(taps), c_int(int(silu)), c_int(n_entries), c_int(max_q_len), _stream()))
+        _ptr(rows), _code(rows.dtype), rows.stride(0), col, _ptr(weight), _ptr(bias), _ptr(state),
+        state.stride(0), state_off, _ptr(q_start), _ptr(slots), _ptr(out), _code(out.dtype), channels,
+        taps, int(silu), n_entries, max_q_len, _stream()))
     return out
 
 
@@ -1499,10 +1499,10 @@ def ssd_scan(xbc: torch.Tensor, dt_rows: torch.Tensor, dt_col: int, dt_bias: tor
         run_state = torch.empty((capacity, heads * state_dim * head_dim), dtype=torch.float32, device=xbc.device)
         run_decay = torch.empty((capacity, heads), dtype=torch.float32, device=xbc.device)
     _check("ssd_scan", lib().tib_ssd_scan(
-        _ptr(xbc), c_int(_code(xbc.dtype)), c_int64(xbc.stride(0)), _ptr(dt_rows), c_int(_code(dt_rows.dtype)),
-        c_int64(dt_rows.stride(0)), c_int(dt_col), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), c_int64(state.stride(0)),
-        _ptr(q_start), _ptr(slots), _ptr(y), c_int(heads), c_int(groups), c_int(state_dim), c_int(head_dim), c_int(n_entries),
-        c_int(n_tokens), c_int(n_tokens if max_q_len is None else max_q_len), _ptr(run_state), _ptr(run_decay), c_int64(capacity),
+        _ptr(xbc), _code(xbc.dtype), xbc.stride(0), _ptr(dt_rows), _code(dt_rows.dtype),
+        dt_rows.stride(0), dt_col, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), state.stride(0),
+        _ptr(q_start), _ptr(slots), _ptr(y), heads, groups, state_dim, head_dim, n_entries,
+        n_tokens, n_tokens if max_q_len is None else max_q_len, _ptr(run_state), _ptr(run_decay), capacity,
         _ptr(error_word), _stream()))
     return y
 
@@ -1517,8 +1517,8 @@ def gated_group_norm(y: torch.Tensor, z_rows: torch.Tensor, z_col: int, weight: 
     if out.shape != y.shape or weight.numel() != width or z_rows.shape[0] != n or z_col < 0 or z_col + width > z_rows.shape[1]:
         raise KernelError("gated_group_norm: shapes do not fit")
     _check("gated_group_norm", lib().tib_gated_group_norm(
-        _ptr(y), _ptr(z_rows), c_int(_code(z_rows.dtype)), c_int64(z_rows.stride(0)), c_int(z_col), _ptr(weight), c_float(eps),
-        _ptr(out), c_int(_code(out.dtype)), c_int(n), c_int(width), c_int(parts), c_int(int(gate_last)), _stream()))
+        _ptr(y), _ptr(z_rows), _code(z_rows.dtype), z_rows.stride(0), z_col, _ptr(weight), eps,
+        _ptr(out), _code(out.dtype), n, width, parts, int(gate_last), _stream()))
     return out
 
 
@@ -1526,11 +1526,14 @@ def gated_group_norm(y: torch.Tensor, z_rows: torch.Tensor, z_col: int, weight: 
 # Attention over a window and pooled blocks (csrc/pooled_window_attention.cu).
 def _pages(keys: torch.Tensor, values: torch.Tensor, kv_heads: int, dim: int, vdim: int, name: str) -> tuple[int, int, int]:
     """(num_pages, page_size, page_stride) of one layer's [pages, kv_heads, page_size, dim / vdim] views."""
-    if (keys.shape[1:] != (kv_heads, keys.shape[2], dim) or values.shape[1:] != (kv_heads, keys.shape[2], vdim)
-            or keys.stride(0) != values.stride(0) or not keys[0].is_contiguous() or not values[0].is_contiguous()
-            or keys.dtype != values.dtype):
+    shape, strides, value_strides = keys.shape, keys.stride(), values.stride()
+    # (contiguous pages by their strides where these say so: a view of one costs as much as a launch)
+    if (len(shape) != 4 or shape[1:] != (kv_heads, shape[2], dim) or values.shape[1:] != (kv_heads, shape[2], vdim)
+            or strides[0] != value_strides[0] or keys.dtype != values.dtype
+            or not (shape[0] and strides[1:] == (shape[2] * dim, dim, 1) or keys[0].is_contiguous())
+            or not (shape[0] and value_strides[1:] == (shape[2] * vdim, vdim, 1) or values[0].is_contiguous())):
         raise KernelError(f"{name}: keys / values are not one layer's pages")
-    return keys.shape[0], keys.shape[2], keys.stride(0)
+    return shape[0], shape[2], strides[0]
 
 
 def rotary_kv_append(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_out: torch.Tensor, keys: torch.Tensor,
@@ -1558,10 +1561,10 @@ def rotary_kv_append(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_o
             raise KernelError("rotary_kv_append: turns do not fit")
     num_pages, page_size, page_stride = _pages(keys, values, kv_heads, dim, vdim, "rotary_kv_append")
     _check("rotary_kv_append", lib().tib_rotary_kv_append(
-        _ptr(proj), c_int64(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off), _ptr(q_bias), _ptr(k_bias), _ptr(v_bias),
-        _ptr(q_out), _ptr(keys), _ptr(values), _ptr(positions), _ptr(token_slot), _ptr(block_table), c_int(block_table.stride(0)),
-        _ptr(freq), _ptr(value_freq), c_float(amplitude), c_int(n), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim),
-        c_int(rot_dim), c_int(page_size), c_int64(page_stride), c_int(num_pages), _ptr(turns), _ptr(error_word), c_int(_code(proj.dtype)), _stream()))
+        _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(q_bias), _ptr(k_bias), _ptr(v_bias),
+        _ptr(q_out), _ptr(keys), _ptr(values), _ptr(positions), _ptr(token_slot), _ptr(block_table), block_table.stride(0),
+        _ptr(freq), _ptr(value_freq), amplitude, n, heads, kv_heads, dim, vdim,
+        rot_dim, page_size, page_stride, num_pages, _ptr(turns), _ptr(error_word), _code(proj.dtype), _stream()))
     return q_out
 
 
@@ -1577,10 +1580,10 @@ def pool_blocks(keys: torch.Tensor, values: torch.Tensor, block_table: torch.Ten
         raise KernelError("pool_blocks: the two caches differ in type")
     _need(positions, "positions", torch.int32), _need(token_slot, "token_slot", torch.int32)
     _check("pool_blocks", lib().tib_pool_blocks(
-        _ptr(keys), _ptr(values), _ptr(block_table), c_int(block_table.stride(0)), c_int(page_size), c_int64(page_stride),
-        c_int(num_pages), _ptr(block_keys), _ptr(block_values), _ptr(block_block_table), c_int(block_block_table.stride(0)),
-        c_int(b_page_size), c_int64(b_stride), c_int(b_pages), _ptr(positions), _ptr(token_slot), c_int(positions.numel()),
-        c_int(kv_heads), c_int(dim), c_int(vdim), c_int(pool), _ptr(error_word), c_int(_code(keys.dtype)), _stream()))
+        _ptr(keys), _ptr(values), _ptr(block_table), block_table.stride(0), page_size, page_stride,
+        num_pages, _ptr(block_keys), _ptr(block_values), _ptr(block_block_table), block_block_table.stride(0),
+        b_page_size, b_stride, b_pages, _ptr(positions), _ptr(token_slot), positions.numel(),
+        kv_heads, dim, vdim, pool, _ptr(error_word), _code(keys.dtype), _stream()))
 
 
 @functools.lru_cache(maxsize=None)
@@ -1649,9 +1652,9 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
             and value_freq is None and dim % 8 == 0 and vdim % 8 == 0 and dim <= 128 and vdim <= 128
             and heads // kv_heads <= 16):
         n_splits = splits if splits is not None else int(lib().tib_pooled_window_attention_splits(
-            c_int(n_entries), c_int(heads), c_int(kv_heads), c_int(min(window + keep, max_kv_len) + (max_kv_len // pool if pool else 0))))
+            n_entries, heads, kv_heads, min(window + keep, max_kv_len) + (max_kv_len // pool if pool else 0)))
         if n_splits > 1:
-            floats = int(lib().tib_pooled_window_attention_part_floats(c_int(vdim)))
+            floats = int(lib().tib_pooled_window_attention_part_floats(vdim))
             partial = torch.empty((n_splits, n, heads, floats), dtype=torch.float32, device=q.device)
         else:
             n_splits = 1
@@ -1662,13 +1665,13 @@ def pooled_window_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
     launches = c_int(0)
     _check("pooled_window_attention", lib().tib_pooled_window_attention(
         _ptr(q), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(keys), _ptr(values), _ptr(block_table),
-        c_int(block_table.stride(0)), c_int(page_size), c_int64(page_stride), c_int(num_pages),
+        block_table.stride(0), page_size, page_stride, num_pages,
         _ptr(block_keys if pool > 0 else None), _ptr(block_values if pool > 0 else None),
-        _ptr(block_block_table if pool > 0 else None), c_int(b_table_stride), c_int(b_page_size), c_int64(b_stride), c_int(b_pages),
-        c_int(n_entries), c_int(max_q_len), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim), c_int(window), c_int(keep), c_int(pool),
-        c_float(scale), _ptr(temp), _ptr(sink), _ptr(value_freq), _ptr(turns), _ptr(gate), c_int(_code(gate.dtype) if gate is not None else 0),
-        c_int64(ld_gate), _ptr(rel_bias), c_int(rel_bias.shape[1] if rel_bias is not None else 0), _ptr(partial),
-        c_int(n_splits), c_int(n), c_int(few_rows), ctypes.byref(launches), _ptr(error_word), c_int(_code(q.dtype)), c_int(int(force_simt)),
+        _ptr(block_block_table if pool > 0 else None), b_table_stride, b_page_size, b_stride, b_pages,
+        n_entries, max_q_len, heads, kv_heads, dim, vdim, window, keep, pool,
+        scale, _ptr(temp), _ptr(sink), _ptr(value_freq), _ptr(turns), _ptr(gate), _code(gate.dtype) if gate is not None else 0,
+        ld_gate, _ptr(rel_bias), rel_bias.shape[1] if rel_bias is not None else 0, _ptr(partial),
+        n_splits, n, few_rows, ctypes.addressof(launches), _ptr(error_word), _code(q.dtype), int(force_simt),
         _stream()))
     count_launches(launches.value - 1)      # (_check counted one)
     return out
@@ -1719,10 +1722,10 @@ def hyper_step(streams: torch.Tensor, *, y: torch.Tensor | None = None, mix: tor
     elif rows is not None:
         raise KernelError("hyper_step: rows only make sense with a read")
     _check("hyper_step", lib().tib_hyper_step(
-        _ptr(streams), c_int64(streams.stride(0)), c_int(count), c_int(n_out), c_int(width), _ptr(y),
-        c_int(_code(y.dtype) if y is not None else 0), c_int64(y.stride(0) if y is not None else 0), _ptr(mix),
-        _ptr(out_weights), _ptr(in_weights), _ptr(rows), c_int(norm), c_float(alpha), _ptr(weight), _ptr(bias), _ptr(out),
-        c_int(_code(out.dtype) if out is not None else 0), _stream()))
+        _ptr(streams), streams.stride(0), count, n_out, width, _ptr(y),
+        _code(y.dtype) if y is not None else 0, y.stride(0) if y is not None else 0, _ptr(mix),
+        _ptr(out_weights), _ptr(in_weights), _ptr(rows), norm, alpha, _ptr(weight), _ptr(bias), _ptr(out),
+        _code(out.dtype) if out is not None else 0, _stream()))
     return out
 
 
@@ -1753,8 +1756,8 @@ def input_conv(x: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, state: 
         raise KernelError("input_conv: entry arrays are shorter than n_entries")
     stride = _conv_state(state, state_off, taps, width, "input_conv")
     _check("input_conv", lib().tib_input_conv(
-        _ptr(x), _ptr(out), _ptr(weight), _ptr(state), c_int64(stride), c_int64(state_off), _ptr(q_start), _ptr(slots),
-        c_int(n_entries), c_int(max_q_len), c_int(width), c_int(taps), c_int(_code(x.dtype)), _stream()))
+        _ptr(x), _ptr(out), _ptr(weight), _ptr(state), stride, state_off, _ptr(q_start), _ptr(slots),
+        n_entries, max_q_len, width, taps, _code(x.dtype), _stream()))
     return out
 
 
@@ -1774,8 +1777,8 @@ def norm_conv_step(delta: torch.Tensor | None, residual: torch.Tensor, norm_weig
             raise KernelError("norm_conv_step: delta does not fit")
     stride = _conv_state(state, state_off, taps, width, "norm_conv_step")
     _check("norm_conv_step", lib().tib_norm_conv_step(
-        _ptr(delta), _ptr(residual), _ptr(norm_weight), c_float(eps), _ptr(weight), _ptr(state), c_int64(stride),
-        c_int64(state_off), _ptr(slots), _ptr(out), c_int(n), c_int(width), c_int(taps), c_int(_code(out.dtype)), _stream()))
+        _ptr(delta), _ptr(residual), _ptr(norm_weight), eps, _ptr(weight), _ptr(state), stride,
+        state_off, _ptr(slots), _ptr(out), n, width, taps, _code(out.dtype), _stream()))
     return out
 
 
@@ -1802,10 +1805,10 @@ def row_norm_append(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, q_ou
             raise KernelError("row_norm_append: a bias or a weight does not fit")
     num_pages, page_size, page_stride = _pages(keys, values, kv_heads, dim, vdim, "row_norm_append")
     _check("row_norm_append", lib().tib_row_norm_append(
-        _ptr(proj), c_int64(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off), _ptr(q_bias), _ptr(k_bias), _ptr(v_bias),
-        _ptr(q_weight), _ptr(k_weight), c_float(eps), _ptr(q_out), _ptr(keys), _ptr(values), _ptr(positions), _ptr(token_slot),
-        _ptr(block_table), c_int(block_table.stride(0)), c_int(n), c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim),
-        c_int(page_size), c_int64(page_stride), c_int(num_pages), _ptr(error_word), c_int(_code(proj.dtype)), _stream()))
+        _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(q_bias), _ptr(k_bias), _ptr(v_bias),
+        _ptr(q_weight), _ptr(k_weight), eps, _ptr(q_out), _ptr(keys), _ptr(values), _ptr(positions), _ptr(token_slot),
+        _ptr(block_table), block_table.stride(0), n, heads, kv_heads, dim, vdim,
+        page_size, page_stride, num_pages, _ptr(error_word), _code(proj.dtype), _stream()))
     return q_out
 
 
@@ -1853,22 +1856,22 @@ def talking_heads_attention(q: torch.Tensor, out: torch.Tensor, q_start: torch.T
     def call(form, first=0, last=0, scores=None, lse=None, key_span=0, part_ml=None, part_o=None, counters=None, tiles=0, parts=0):
         _check("talking_heads_attention", lib().tib_talking_heads_attention(
             _ptr(q), _ptr(out), _ptr(q_start), _ptr(kv_start), _ptr(slots), _ptr(positions), _ptr(keys), _ptr(values), _ptr(block_table),
-            c_int(block_table.stride(0)), c_int(page_size), c_int64(page_stride), c_int(num_pages), c_int(n_entries), c_int(max_q_len),
-            c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim), c_int(window), c_float(scale), c_float(softcap), _ptr(bias),
-            c_int(bias.shape[1] if bias is not None else 0), _ptr(talk), _ptr(talk_hi), _ptr(talk_lo), _ptr(gate),
-            c_int(_code(gate.dtype) if gate is not None else 0), c_int64(ld_gate), c_int(form), c_int(first), c_int(last),
-            _ptr(scores), _ptr(lse), c_int(key_span), _ptr(part_ml), _ptr(part_o), _ptr(counters), c_int(tiles), c_int(parts),
-            _ptr(error_word), c_int(_code(q.dtype)), _stream()))
+            block_table.stride(0), page_size, page_stride, num_pages, n_entries, max_q_len,
+            heads, kv_heads, dim, vdim, window, scale, softcap, _ptr(bias),
+            bias.shape[1] if bias is not None else 0, _ptr(talk), _ptr(talk_hi), _ptr(talk_lo), _ptr(gate),
+            _code(gate.dtype) if gate is not None else 0, ld_gate, form, first, last,
+            _ptr(scores), _ptr(lse), key_span, _ptr(part_ml), _ptr(part_o), _ptr(counters), tiles, parts,
+            _ptr(error_word), _code(q.dtype), _stream()))
 
-    if q.dtype != torch.bfloat16 or force_simt or not lib().tib_talking_heads_takes_mma(c_int(heads), c_int(dim), c_int(vdim)):
+    if q.dtype != torch.bfloat16 or force_simt or not lib().tib_talking_heads_takes_mma(heads, dim, vdim):
         call(0)
         return out
     if max_kv_len < 1:
         raise KernelError("talking_heads_attention: the tensor-core forms need a bound on the longest context")
-    key_span = int(lib().tib_talking_heads_key_span(c_int(window), c_int(max_kv_len)))
+    key_span = int(lib().tib_talking_heads_key_span(window, max_kv_len))
     if (max_q_len == 1 and n == n_entries and not force_portions
-            and lib().tib_talking_heads_takes_step(c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim))):
-        tiles = tiles_per_part or int(lib().tib_talking_heads_tiles_per_part(c_int(n_entries), c_int(kv_heads), c_int(key_span)))
+            and lib().tib_talking_heads_takes_step(heads, kv_heads, dim, vdim)):
+        tiles = tiles_per_part or int(lib().tib_talking_heads_tiles_per_part(n_entries, kv_heads, key_span))
         parts = -(-key_span // (64 * tiles))
         scores = torch.empty((n, heads, key_span), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((n, parts, heads, 2), dtype=torch.float32, device=q.device)
@@ -1937,11 +1940,11 @@ def conv_norm_append(proj: torch.Tensor, q_off: int, k_off: int, q_out: torch.Te
         stride = state.stride(0)
     num_pages, page_size, page_stride = _pages(keys, values, kv_heads, dim, dim, "conv_norm_append")
     _check("conv_norm_append", lib().tib_conv_norm_append(
-        _ptr(proj), c_int64(proj.stride(0)), c_int(q_off), c_int(k_off), _ptr(q_conv), _ptr(k_conv), c_int(taps), _ptr(q_weight),
-        _ptr(k_weight), c_float(eps), _ptr(freq), c_int(freq.numel()), _ptr(q_out), _ptr(keys), _ptr(values), _ptr(positions),
-        _ptr(block_table), c_int(block_table.stride(0)), _ptr(q_start), _ptr(slots), c_int(n_entries), _ptr(state if taps > 1 else None),
-        c_int64(stride), c_int64(state_off), c_int(n), c_int(max_q_len), c_int(heads), c_int(kv_heads), c_int(dim), c_int(page_size),
-        c_int64(page_stride), c_int(num_pages), _ptr(error_word), c_int(_code(proj.dtype)), _stream()))
+        _ptr(proj), proj.stride(0), q_off, k_off, _ptr(q_conv), _ptr(k_conv), taps, _ptr(q_weight),
+        _ptr(k_weight), eps, _ptr(freq), freq.numel(), _ptr(q_out), _ptr(keys), _ptr(values), _ptr(positions),
+        _ptr(block_table), block_table.stride(0), _ptr(q_start), _ptr(slots), n_entries, _ptr(state if taps > 1 else None),
+        stride, state_off, n, max_q_len, heads, kv_heads, dim, page_size,
+        page_stride, num_pages, _ptr(error_word), _code(proj.dtype), _stream()))
     return q_out
 
 
@@ -1988,7 +1991,7 @@ def matrix_memory(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g_off:
         raise KernelError("matrix_memory: shapes or types do not fit")
     if q_start.numel() < n_entries + 1 or slots.numel() < n_entries:
         raise KernelError("matrix_memory: entry arrays are shorter than n_entries")
-    takes_chunks = proj.dtype == torch.bfloat16 and bool(library.tib_matrix_memory_takes_chunks(c_int(dim), c_int(vdim)))
+    takes_chunks = proj.dtype == torch.bfloat16 and bool(library.tib_matrix_memory_takes_chunks(dim, vdim))
     chunks = takes_chunks and max_q_len > MATRIX_MEMORY_WALK if walk is None else not walk
     if logits is not None:
         _rows_of(logits, "logits")
@@ -2010,12 +2013,12 @@ def matrix_memory(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g_off:
         run_keep = torch.empty((capacity, heads), dtype=torch.float32, device=dev)
         count_launches(3)
     _check("matrix_memory", library.tib_matrix_memory(
-        _ptr(proj), c_int64(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off), c_int(g_off), c_float(q_scale), _ptr(logits),
-        c_int64(logits.stride(0) if logits is not None else 0), _ptr(x), c_int64(x.stride(0)), _ptr(gate_weight), c_int(x.shape[1]), _ptr(gate_bias), c_float(cap), _ptr(state),
-        c_int64(state.stride(0)), _ptr(q_start), _ptr(slots), _ptr(norm_weight if fused else None), c_float(eps), _ptr(y),
-        _ptr(out if fused else None), c_int(heads), c_int(dim), c_int(vdim), c_int(n_entries), c_int(n), c_int(max_q_len),
-        c_int(int(chunks)), _ptr(cum), _ptr(log_in), _ptr(top), _ptr(top0), _ptr(run_state), _ptr(run_n), _ptr(run_keep),
-        c_int64(capacity), c_int(_code(proj.dtype)), _stream()))
+        _ptr(proj), proj.stride(0), q_off, k_off, v_off, g_off, q_scale, _ptr(logits),
+        logits.stride(0) if logits is not None else 0, _ptr(x), x.stride(0), _ptr(gate_weight), x.shape[1], _ptr(gate_bias), cap, _ptr(state),
+        state.stride(0), _ptr(q_start), _ptr(slots), _ptr(norm_weight if fused else None), eps, _ptr(y),
+        _ptr(out if fused else None), heads, dim, vdim, n_entries, n, max_q_len,
+        int(chunks), _ptr(cum), _ptr(log_in), _ptr(top), _ptr(top0), _ptr(run_state), _ptr(run_n), _ptr(run_keep),
+        capacity, _code(proj.dtype), _stream()))
     if not fused:
         gated_group_norm(y, proj, g_off, norm_weight, eps, out, heads, gate_last=True)
     return out
