@@ -134,6 +134,164 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, T* __restrict__ 
   }
 }
 
+// The same for bf16 rows on 16-byte boundaries, eight elements a load and store.  A token is one warp's (WARPS 1: four tokens a block, no barrier of
+// the block but the table's) or, in small steps, a block's, and a thread asks for its next pieces before it works on the last.  The sum of squares adds
+// eight neighbours a thread.  What bounds it is one trip to memory behind the page's lookup: 2,500 tokens of 16 heads, 512 + 64 numbers, in place
+// 7.2 us where the kernel above takes 16.4 (in the running layer); eight tokens 3.3 behind the product before, 4.3 above.
+template <int WARPS>
+__global__ void __launch_bounds__(128)
+latent_append_pieces_kernel(const __nv_bfloat16* __restrict__ dkv, __nv_bfloat16* q, __nv_bfloat16* __restrict__ pool,
+                            float* __restrict__ folded, LatentAppendArgs a, int n_tokens) {
+  constexpr int TOKENS = 4 / WARPS, THREADS = 32 * WARPS;
+  __shared__ float scratch[33];
+  __shared__ float cos_s[TOKENS][kAppendFreq / TOKENS], sin_s[TOKENS][kAppendFreq / TOKENS];
+  const int own = WARPS == 1 ? threadIdx.x >> 5 : 0, tid = WARPS == 1 ? threadIdx.x & 31 : threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
+  const size_t t = (size_t)blockIdx.x * TOKENS + own;
+  const bool live = t < n_tokens;
+  const int width = a.rank + a.rot, rank8 = a.rank / 8, rot8 = a.rot / 8;
+  const __nv_bfloat16* src = dkv + (live ? t : 0) * a.ld_dkv;
+  __nv_bfloat16* dst = nullptr;
+  uint4 first = make_uint4(0u, 0u, 0u, 0u), second = first;      // (the latent's pieces tid and tid + THREADS)
+  int pos = 0;
+  if (live) {
+    pos = a.positions[t];
+    if (tid < rank8) first = *reinterpret_cast<const uint4*>(src + tid * 8);
+    if (tid + THREADS < rank8) second = *reinterpret_cast<const uint4*>(src + (tid + THREADS) * 8);
+    if (pool) {
+      const int page = a.block_table[(size_t)a.token_slot[t] * a.table_stride + pos / a.page_size];
+      if (page >= 0 && page < a.num_pages) dst = pool + (size_t)page * a.page_stride + (size_t)(pos % a.page_size) * width;
+      else if (a.error_word && tid == 0) atomicExch(a.error_word, 0x20000 + (int)(t & 0xffff));
+    }
+    for (int i = tid; i < a.n_freq; i += THREADS) {
+      const float angle = (float)pos * a.inv_freq[i];
+      cos_s[own][i] = cosf(angle);
+      sin_s[own][i] = sinf(angle);
+    }
+  }
+  const auto widen = [](const uint4& raw, float (&v)[8]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  };
+  const auto narrow = [](const float (&v)[8]) { return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7])); };
+  const auto piece = [&](int p) { return p == tid ? first : p == tid + THREADS ? second : *reinterpret_cast<const uint4*>(src + p * 8); };
+  float ss = 0.f;
+  if (live)
+    for (int p = tid; p < rank8; p += THREADS) {
+      float v[8];
+      widen(piece(p), v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+    }
+  if (WARPS == 1) {
+    ss = warp_sum(ss);
+    __syncwarp();      // (the table is the warp's own)
+  } else {
+    ss = block_sum(ss, scratch);      // (its barriers publish the table too)
+  }
+  if (!live) return;
+  const float inv = 1.f / sqrtf(ss / (float)a.rank + a.eps);
+  if (dst)
+    for (int p = tid; p < rank8; p += THREADS) {
+      float v[8];
+      widen(piece(p), v);
+      const float4 g0 = *reinterpret_cast<const float4*>(a.norm_weight + p * 8), g1 = *reinterpret_cast<const float4*>(a.norm_weight + p * 8 + 4);
+      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * g[e];
+      *reinterpret_cast<uint4*>(dst + p * 8) = narrow(v);
+    }
+  // job 0: the shared key part; jobs 1 .. heads: every head's rotated query part
+  const auto from_of = [&](int job) { return job == 0 ? src + a.rank : q + t * a.ld_q + (size_t)(job - 1) * (a.dim + a.rot) + a.dim; };
+  const auto put = [&](int job, int p, const float (&v)[8]) {
+    if (job == 0) {
+      if (dst) *reinterpret_cast<uint4*>(dst + a.rank + p * 8) = narrow(v);
+    } else if (a.in_place) {
+      *reinterpret_cast<uint4*>(q + t * a.ld_q + (size_t)(job - 1) * (a.dim + a.rot) + a.dim + p * 8) = narrow(v);
+    } else {
+      float4* to = reinterpret_cast<float4*>(folded + (t * a.heads + (job - 1)) * (size_t)width + a.rank + p * 8);
+      to[0] = make_float4(v[0], v[1], v[2], v[3]);
+      to[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+  };
+  const float* cs = cos_s[own];
+  const float* sn = sin_s[own];
+  constexpr int AHEAD = 4;      // pieces on their way a thread
+  if (a.half_pairs) {
+    // piece p with its partner at p + n_freq / 8; what lies behind both halves passes unchanged
+    const int half8 = a.n_freq / 8, units = rot8 - half8, total = (a.heads + 1) * units;
+    for (int e0 = tid; e0 < total; e0 += THREADS * AHEAD) {
+      uint4 lo[AHEAD], hi[AHEAD];
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const int e = e0 + u * THREADS, job = e / units, p = e - job * units;
+        if (e >= total) continue;
+        const __nv_bfloat16* from = from_of(job);
+        lo[u] = *reinterpret_cast<const uint4*>(from + (p < half8 ? p : p + half8) * 8);
+        if (p < half8) hi[u] = *reinterpret_cast<const uint4*>(from + (p + half8) * 8);
+      }
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const int e = e0 + u * THREADS, job = e / units, p = e - job * units;
+        if (e >= total) continue;
+        float x[8], y[8];
+        widen(lo[u], x);
+        if (p >= half8) {
+          put(job, p + half8, x);
+          continue;
+        }
+        widen(hi[u], y);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float l = x[k], h = y[k], c = cs[p * 8 + k], s = sn[p * 8 + k];
+          x[k] = rope_lo(l, h, c, s);
+          y[k] = rope_hi(l, h, c, s);
+        }
+        put(job, p, x);
+        put(job, p + half8, y);
+      }
+    }
+    return;
+  }
+  const int total = (a.heads + 1) * rot8;
+  for (int e0 = tid; e0 < total; e0 += THREADS * AHEAD) {
+    uint4 raw[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int e = e0 + u * THREADS, job = e / rot8, p = e - job * rot8;
+      if (e < total) raw[u] = *reinterpret_cast<const uint4*>(from_of(job) + p * 8);
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int e = e0 + u * THREADS, job = e / rot8, p = e - job * rot8;
+      if (e >= total) continue;
+      float v[8];
+      widen(raw[u], v);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = p * 4 + k;
+        if (i >= a.n_freq) continue;
+        const float lo = v[2 * k], hi = v[2 * k + 1];
+        v[2 * k] = rope_lo(lo, hi, cs[i], sn[i]);
+        v[2 * k + 1] = rope_hi(lo, hi, cs[i], sn[i]);
+      }
+      put(job, p, v);
+    }
+  }
+}
+
+// Rows, pages and heads in whole pieces on 16-byte boundaries, and a table that fits.
+static bool latent_append_takes_pieces(const LatentAppendArgs& a, const void* dkv, const void* q, const void* pool, const float* folded, int table) {
+  return a.rank % 8 == 0 && a.rot % 8 == 0 && a.dim % 8 == 0 && a.ld_dkv % 8 == 0 && a.ld_q % 8 == 0 && (!pool || a.page_stride % 8 == 0) && a.n_freq <= table &&
+         (!a.half_pairs || a.n_freq % 8 == 0) &&
+         (((uintptr_t)dkv | (uintptr_t)q | (uintptr_t)pool | (uintptr_t)folded | (uintptr_t)a.norm_weight) & 15) == 0;
+}
+
 // ---------------------------------------------------------------- attention
 constexpr int kLatWarps = 4;
 constexpr int kLatRowsPerWarp = 4;
@@ -862,7 +1020,17 @@ TIB_API int tib_latent_append(const void* dkv, int64_t ld_dkv, void* q, int64_t 
   a.dim = dim; a.ld_dkv = ld_dkv; a.ld_q = ld_q; a.page_size = page_size; a.num_pages = num_pages;
   a.page_stride = page_stride; a.eps = eps; a.error_word = error_word; a.half_pairs = half_pairs;
   a.in_place = folded == nullptr;
-  const int threads = n_tokens <= 2 * 148 ? 512 : 128;      // (few tokens: a token's elements over more warps)
+  const bool few = n_tokens <= 2 * 148;
+  const int threads = few ? 512 : 128;      // (few tokens: a token's elements over more warps)
+  if (dtype == TIB_BF16 && latent_append_takes_pieces(a, dkv, q, pool, folded, few ? kAppendFreq : kAppendFreq / 4)) {
+    if (few)
+      TIB_LAUNCH_DEPENDENT(latent_append_pieces_kernel<4>, n_tokens, 128, 0, stream, (const __nv_bfloat16*)dkv, (__nv_bfloat16*)q, (__nv_bfloat16*)pool,
+                           folded, a, n_tokens);
+    else
+      TIB_LAUNCH_DEPENDENT(latent_append_pieces_kernel<1>, ceil_div(n_tokens, 4), 128, 0, stream, (const __nv_bfloat16*)dkv, (__nv_bfloat16*)q,
+                           (__nv_bfloat16*)pool, folded, a, n_tokens);
+    return TIB_OK;
+  }
   if (dtype == TIB_F32)
     TIB_LAUNCH_DEPENDENT(latent_append_kernel<float>, n_tokens, threads, 0, stream, (const float*)dkv, (float*)q,
                          (float*)pool, folded, a);

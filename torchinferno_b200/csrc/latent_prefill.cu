@@ -15,7 +15,7 @@
 //                    the columns of S they come from.  A head's sink and the output gate are applied at the end.
 //
 // What bounds it: the tensor core (two products, the second twice) at two stages of 80 KB of keys and values.  Two prompts of 1,667
-// and 833 tokens, 16 heads of 128 + 64 over a rank of 512: gather 12 us, product 15, attention 68 (cold), where the folded form took 20 for
+// and 833 tokens, 16 heads of 128 + 64 over a rank of 512: gather 3 us, product 14, attention 45, where the folded form took 20 for
 // folding, 1,094 for the attention, 21 for a cast, 12 for unfolding and 20 for the gate.
 #include "tcgen05.cuh"
 #include <math_constants.h>
@@ -53,7 +53,9 @@ __device__ __forceinline__ int lp_first_row(const int* q_start, const int* kv_st
   return sum;
 }
 
-// grid (runs of 32 rows, entries), 256 threads: a warp copies four rows, 16 bytes a lane.
+// grid (runs of eight rows, entries), 256 threads: 16 bytes a lane, a warp a row (longer runs of rows a block, four rows a warp one after the other:
+// 12 us where this takes 3.1 on the call of the header).
+constexpr int kGatherRows = 8;
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const uint4* __restrict__ pool, int64_t page_stride, int page_size, int num_pages, const int* __restrict__ block_table,
                      int table_stride, const int* __restrict__ q_start, const int* __restrict__ kv_start, const int* __restrict__ slots,
@@ -61,30 +63,30 @@ latent_gather_kernel(const uint4* __restrict__ pool, int64_t page_stride, int pa
   pdl_wait();
   pdl_trigger();
   const int entry = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = blockIdx.x * kGatherRows + warp, slot = slots[entry];
   const int keys = kv_start[entry] + q_start[entry + 1] - q_start[entry];
   const int padded = (keys + kLpTile - 1) / kLpTile * kLpTile;
-  const int r0 = blockIdx.x * 32 + warp * 4;
-  if (r0 >= padded) return;
+  if (r >= padded) return;
+  const int page = r < keys ? block_table[(size_t)slot * table_stride + r / page_size] : -1;
   const int first = lp_first_row(q_start, kv_start, entry, lane);
-  const int* table = block_table + (size_t)slots[entry] * table_stride;
-  int page[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) page[i] = r0 + i < keys ? table[(r0 + i) / page_size] : -1;
   const int pieces = rank8 + rot8;
+  const bool have = page >= 0 && page < num_pages;
+  if (r < keys && !have && error_word && lane == 0) atomicExch(error_word, 0x30000 + entry);
+  if (first + r >= rows) {      // (the entries need more rows than there are: reported, nothing is written behind the last one)
+    if (error_word && lane == 0) atomicExch(error_word, 0x60000 + entry);
+    return;
+  }
+  const uint4* src = pool + (size_t)(have ? page : 0) * page_stride + (size_t)(r % page_size) * pieces;
+  constexpr int AHEAD = 4;
+  for (int c0 = lane; c0 < pieces; c0 += 32 * AHEAD) {
+    uint4 v[AHEAD];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + i;
-    const bool have = page[i] >= 0 && page[i] < num_pages;
-    if (r < keys && !have && error_word && lane == 0) atomicExch(error_word, 0x30000 + entry);
-    if (first + r >= rows) {      // (the entries need more rows than there are: reported, nothing is written behind the last one)
-      if (error_word && lane == 0) atomicExch(error_word, 0x60000 + entry);
-      continue;
-    }
-    const uint4* src = pool + (size_t)(have ? page[i] : 0) * page_stride + (size_t)(r % page_size) * pieces;
-    for (int c = lane; c < pieces; c += 32) {
-      const uint4 v = have ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-      if (c < rank8) latent[(size_t)(first + r) * rank8 + c] = v;
-      else rotated[(size_t)(first + r) * rot8 + c - rank8] = v;
+    for (int u = 0; u < AHEAD; ++u) v[u] = have && c0 + 32 * u < pieces ? src[c0 + 32 * u] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int c = c0 + 32 * u;
+      if (c < rank8) latent[(size_t)(first + r) * rank8 + c] = v[u];
+      else if (c < pieces) rotated[(size_t)(first + r) * rot8 + c - rank8] = v[u];
     }
   }
 }
@@ -446,7 +448,7 @@ TIB_API int tib_latent_gather(const void* pool, int64_t page_stride, int page_si
   if (!pool || !block_table || !q_start || !kv_start || !slots || !latent || !rotated || page_size < 1 || rows < 0) return TIB_E_ARG;
   if (rank % 8 || rot % 8 || page_stride % 8 || (((uintptr_t)pool | (uintptr_t)latent | (uintptr_t)rotated) & 15)) return TIB_E_ALIGN;
   if (n_entries > 65535) return TIB_E_SIZE;
-  TIB_LAUNCH_DEPENDENT(latent_gather_kernel, dim3(ceil_div(max_kv_len, kLpTile) * (kLpTile / 32), n_entries), 256, 0, stream, (const uint4*)pool,
+  TIB_LAUNCH_DEPENDENT(latent_gather_kernel, dim3(ceil_div(max_kv_len, kLpTile) * (kLpTile / kGatherRows), n_entries), 256, 0, stream, (const uint4*)pool,
                        page_stride / 8, page_size, num_pages, block_table, table_stride, q_start, kv_start, slots, (uint4*)latent,
                        (uint4*)rotated, rows, rank / 8, rot / 8, error_word);
   return TIB_OK;
