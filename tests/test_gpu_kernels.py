@@ -1892,3 +1892,53 @@ def test_latent_rows_in_pieces_are_those_element_by_element(tokens, heads, dim, 
     got, want = keys[..., :rank].double(), want_keys[..., :rank].double()
     assert ((got - want).abs() <= 2.0 ** -7 * want.abs()).all()      # (a rounding to the neighbouring bf16 number: at most 2^-7 of the value)
     assert (got != want).double().mean() < 0.01
+
+
+@pytest.mark.parametrize("tokens, rows, k", [(2859, 7, 260), (1187, 37, 64), (331, 61, 1028), (157, 129, 2056)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_router_logits_of_six_rows_a_warp_have_the_bits_of_one(tokens, rows, k, dtype):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    x, w, bias = dev(rnd(tokens, (k + 7) // 8 * 8, dtype=dtype))[:, :k], dev(rnd(rows, k, seed=1)), dev(rnd(rows, seed=2))
+    out = ops.router_logits(x, w, torch.empty(tokens, rows, device="cuda"), bias)
+    parts = [ops.router_logits(x[i:i + 100], w, torch.empty(len(x[i:i + 100]), rows, device="cuda"), bias) for i in range(0, tokens, 100)]
+    assert tokens * rows >= 20000 > 100 * rows and torch.equal(out, torch.cat(parts))
+
+
+@pytest.mark.parametrize("experts, top", [(1, 1), (31, 4), (32, 32), (33, 3), (64, 6), (65, 8), (256, 8)])
+@pytest.mark.parametrize("sigmoid, normalize, corrected", [(False, True, False), (True, False, True)])
+def test_choices_of_few_experts_are_the_general_forms(experts, top, sigmoid, normalize, corrected):
+    """The same logits beside experts that are never chosen (more than 256 take the general form); equal logits among them."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    tokens, wide = 67, 300
+    z = rnd(tokens, experts)
+    z[::3, 1::2] = z[::3, 0:2 * (experts // 2):2]                      # (pairs of equals)
+    beside = torch.full((tokens, wide - experts), -float("inf"))
+    correction = 0.1 * rnd(experts, seed=1) if corrected else None
+    results = []
+    for logits, extra in ((z, 0), (torch.cat([z, beside], dim=1), wide - experts)):
+        ids, weights = torch.empty(tokens, top, dtype=torch.int32, device="cuda"), torch.empty(tokens, top, device="cuda")
+        c = None if correction is None else dev(torch.cat([correction, torch.full((extra,), -100.0)]))
+        ops.moe_route(dev(logits), logits.shape[1], top, ids, weights, sigmoid_scores=sigmoid, normalize=normalize, norm_eps=1e-20, correction=c)
+        results.append((ids, weights))
+    assert torch.equal(results[0][0], results[1][0])
+    # (the softmax's sum takes the same numbers in the same lanes; zeros change nothing)
+    assert torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("pairs, experts", [(1, 1), (1023, 32), (1025, 3), (8191, 256), (16384, 60), (16385, 60), (9000, 257)])
+def test_pairs_are_sorted_by_expert(pairs, experts):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    ids = torch.randint(-1, experts + 1, (pairs,), generator=torch.Generator().manual_seed(pairs), dtype=torch.int32)      # (some have no expert here)
+    offsets, order, place = (torch.full((n,), -9, dtype=torch.int32, device="cuda") for n in (experts + 1, pairs, pairs))
+    ops.moe_group(dev(ids), experts, offsets, order, place)
+    inside = (ids >= 0) & (ids < experts)
+    counts = torch.bincount(ids[inside].long(), minlength=experts)
+    assert offsets.tolist() == [0] + counts.cumsum(0).tolist()
+    order, place = order.cpu().long(), place.cpu().long()
+    assert (place[~inside] == -1).all()
+    held = order[:int(inside.sum())]
+    assert torch.equal(held.sort().values, inside.nonzero().flatten())                       # every pair once
+    assert torch.equal(place[held], torch.arange(len(held))) and (ids[held].long().diff() >= 0).all()

@@ -28,9 +28,9 @@ namespace tib {
 // token: the order of every sum is fixed by k and the alignment alone, so a token's logits do not depend on what else is
 // in the step.  (The general fp32 product gives a product
 // this narrow to a single block.)
-// A block takes TOK tokens, so that a row of w read from the L2 serves several of them.  With 16-byte aligned
+// A block takes four tokens, so that a row of w read from the L2 serves several of them.  With 16-byte aligned
 // rows (VEC) a lane takes eight consecutive k at a time: 16 bytes of a bf16 token row, 32 bytes of w.
-constexpr int kRouterTokens = 4, kRouterMany = 8;      // tokens of a block: of a small step or odd rows, of a large one
+constexpr int kRouterTokens = 4;
 
 __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
   const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
@@ -43,61 +43,139 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
 }
 
-// In a large step a warp works R rows of w at a time (rows e, e + all the warps of the token group, ...), whose pieces stay in
-// registers while the group's tokens pass by, so a token's elements are widened once for R rows: 2,048 tokens, 33 rows of 2,048
-// 36 us with one row and four tokens, 28 with five and eight.  With few tokens one row and four tokens stay ahead (8 tokens:
-// 15 against 21), since there the number of warps counts.
-template <typename TX, bool VEC, int TOK, int R>
+template <typename TX, bool VEC>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ out, int64_t ldo, int tokens, int rows, int K) {
   pdl_wait();
   pdl_trigger();
+  constexpr int TOK = kRouterTokens;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int t0 = blockIdx.x * TOK;
   const int nt = min(TOK, tokens - t0);
   const int K8 = VEC ? (K / 8) * 8 : 0;
-  const int stride = nwarps * gridDim.y;
-  for (int e0 = warp + blockIdx.y * nwarps; e0 < rows; e0 += stride * R) {
-    float acc[R][TOK];
+  for (int e = warp + blockIdx.y * nwarps; e < rows; e += nwarps * gridDim.y) {
+    float acc[TOK];
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int i = 0; i < TOK; ++i) acc[r][i] = 0.f;
+    for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
     if (VEC) {
       // (small steps wait for loads: 12 us for eight tokens of 2,048 with one round's in flight, 7.4 with four rounds')
-#pragma unroll(R == 1 && TOK == kRouterTokens ? 4 : 1)
+#pragma unroll 4
       for (int k = lane * 8; k < K8; k += 256) {
-        float wv[R][8];
-#pragma unroll
-        for (int r = 0; r < R; ++r) load8(w + (size_t)min(e0 + r * stride, rows - 1) * K + k, wv[r]);      // (a row too many is not stored)
+        float wv[8];
+        load8(w + (size_t)e * K + k, wv);
 #pragma unroll
         for (int i = 0; i < TOK; ++i) {
           float xv[8];
           load8(x + (size_t)(t0 + min(i, nt - 1)) * ldx + k, xv);
 #pragma unroll
-          for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[r][i] = fmaf(xv[j], wv[r][j], acc[r][i]);
+          for (int j = 0; j < 8; ++j) acc[i] = fmaf(xv[j], wv[j], acc[i]);
         }
       }
     }
+    for (int k = K8 + lane; k < K; k += 32) {
+      const float wv = w[(size_t)e * K + k];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int e = e0 + r * stride;
-      if (e >= rows) break;
-      for (int k = K8 + lane; k < K; k += 32) {
-        const float wv = w[(size_t)e * K + k];
+      for (int i = 0; i < TOK; ++i)
+        if (i < nt) acc[i] = fmaf(to_f32(x[(size_t)(t0 + i) * ldx + k]), wv, acc[i]);
+    }
 #pragma unroll
-        for (int i = 0; i < TOK; ++i)
-          if (i < nt) acc[r][i] = fmaf(to_f32(x[(size_t)(t0 + i) * ldx + k]), wv, acc[r][i]);
-      }
+    for (int i = 0; i < TOK; ++i) {
+      const float v = warp_sum(acc[i]);
+      if (lane == 0 && i < nt) out[(size_t)(t0 + i) * ldo + e] = bias ? v + bias[e] : v;
+    }
+  }
+}
+
+// The same sums for large steps with 16-byte aligned rows: a warp works six rows of w on eight tokens, two tokens an instruction (packed fp32), so a
+// piece of w serves eight tokens and an element is widened for six rows; what it loads and widens is a third of its instructions.  (A lane's sums
+// run over k in the kernel above's order, and the sum over lanes is its butterfly, whose two halves of a pair add the same two numbers.)  What bounds
+// it: the loads of a step wait for one another's registers (two blocks of six warps an SM), then the fp32 pipe.  2,048 tokens of 2,048: 33 rows 14.4
+// us, 61 (of 1,536) 20.5, 129 41.0; with five rows of whole warps of eight and scalar products 20.2, 30.2, 72.6; rows and tokens through shared memory 27 to 50.
+constexpr int kRouterRows = 6, kRouterMany = 8, kRouterWarps = 6;
+
+__device__ __forceinline__ void load8_pairs(const float* a, const float* b, f32x2 (&v)[8]) {
+  float x[8], y[8];
+  load8(a, x);
+  load8(b, y);
 #pragma unroll
-      for (int i = 0; i < TOK; ++i) {
-        const float v = warp_sum(acc[r][i]);
-        if (lane == 0 && i < nt) out[(size_t)(t0 + i) * ldo + e] = bias ? v + bias[e] : v;
+  for (int j = 0; j < 8; ++j) v[j] = f2_pack(x[j], y[j]);
+}
+__device__ __forceinline__ void load8_pairs(const __nv_bfloat16* a, const __nv_bfloat16* b, f32x2 (&v)[8]) {
+  const uint4 p = *reinterpret_cast<const uint4*>(a), q = *reinterpret_cast<const uint4*>(b);
+  const uint32_t x[4] = {p.x, p.y, p.z, p.w}, y[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = f2_pack(__uint_as_float(x[i] << 16), __uint_as_float(y[i] << 16));
+    v[2 * i + 1] = f2_pack(__uint_as_float(x[i] & 0xffff0000u), __uint_as_float(y[i] & 0xffff0000u));
+  }
+}
+
+// grid (runs of kRouterMany tokens, runs of rows: kRouterRows a warp)
+template <typename TX>
+__global__ void __launch_bounds__(kRouterWarps * 32)
+router_logits_many_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restrict__ w, const float* __restrict__ bias,
+                          float* __restrict__ out, int64_t ldo, int tokens, int rows, int K) {
+  constexpr int TOK = kRouterMany, R = kRouterRows;
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, e0 = (blockIdx.y * warps + (threadIdx.x >> 5)) * R;
+  const int t0 = blockIdx.x * TOK, nt = min(TOK, tokens - t0), K8 = K / 8 * 8;
+  if (e0 >= rows) return;
+  const float* row[R];
+  const TX* token[TOK];
+#pragma unroll
+  for (int r = 0; r < R; ++r) row[r] = w + (size_t)min(e0 + r, rows - 1) * K;      // (a row or token too many is not stored)
+#pragma unroll
+  for (int i = 0; i < TOK; ++i) token[i] = x + (size_t)(t0 + min(i, nt - 1)) * ldx;
+  f32x2 acc[R][TOK / 2];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < TOK / 2; ++i) acc[r][i] = f2_pack(0.f, 0.f);
+#pragma unroll 1
+  for (int k = lane * 8; k < K8; k += 256) {
+    float wv[R][8];
+#pragma unroll
+    for (int r = 0; r < R; ++r) load8(row[r] + k, wv[r]);
+#pragma unroll
+    for (int i = 0; i < TOK / 2; ++i) {
+      f32x2 xv[8];
+      load8_pairs(token[2 * i] + k, token[2 * i + 1] + k, xv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r][i] = f2_fma(xv[j], f2_pack(wv[r][j], wv[r][j]), acc[r][i]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int e = e0 + r;
+    if (e >= rows) break;
+    float own[TOK];
+#pragma unroll
+    for (int i = 0; i < TOK / 2; ++i) f2_unpack(acc[r][i], own[2 * i], own[2 * i + 1]);
+    for (int k = K8 + lane; k < K; k += 32) {
+      const float wv = w[(size_t)e * K + k];
+#pragma unroll
+      for (int i = 0; i < TOK; ++i)
+        if (i < nt) own[i] = fmaf(to_f32(x[(size_t)(t0 + i) * ldx + k]), wv, own[i]);
+    }
+    // the sums over the lanes: at each of three steps a lane hands on the half of its tokens that its partner keeps
+#pragma unroll
+    for (int half = TOK / 2; half > 0; half /= 2) {
+      const bool upper = lane & (4 * half);
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const float give = upper ? own[i] : own[i + half], keep = upper ? own[i + half] : own[i];
+        own[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * half);
       }
     }
+    float v = own[0];
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    const int i = lane >> 2;
+    if ((lane & 3) == 0 && i < nt) out[(size_t)(t0 + i) * ldo + e] = bias ? v + bias[e] : v;
   }
 }
 
@@ -200,12 +278,91 @@ __device__ __forceinline__ void moe_route_token(const MoeRouteArgs& r, int t, un
   if (normalize) for (int k = lane + 32; k < top; k += 32) weights[(size_t)t * top + k] /= (chosen_sum + norm_eps);
 }
 
+// The same choices and weights, to the bit, of at most 32 S experts without groups and at most 32 choices: a lane works its S scores out once and
+// keeps them, and lane k the k-th choice, so that nothing is read back from memory.  2,048 tokens, 4 of 32: 6.8 us behind the logits, 12.2 in the form above.
+template <int S>
+__device__ __forceinline__ void moe_route_token_few(const MoeRouteArgs& r, int t) {
+  const int lane = threadIdx.x & 31;
+  const float* z = r.logits + (size_t)t * r.ld;
+  float logit[S], score[S], rank[S];
+  float mx = -CUDART_INF_F;
+#pragma unroll
+  for (int i = 0; i < S; ++i) {
+    const int e = lane + 32 * i;
+    logit[i] = e < r.experts ? z[e] : -CUDART_INF_F;
+    if (e < r.experts) mx = fmaxf(mx, logit[i]);
+  }
+  if (!r.sigmoid_scores) {
+    mx = warp_max(mx);
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < S; ++i) {
+      score[i] = expf(logit[i] - mx);
+      if (lane + 32 * i < r.experts) sum += score[i];
+    }
+    sum = warp_sum(sum);
+#pragma unroll
+    for (int i = 0; i < S; ++i) score[i] = score[i] / sum;
+  } else {
+#pragma unroll
+    for (int i = 0; i < S; ++i) score[i] = 1.f / (1.f + expf(-logit[i]));
+  }
+#pragma unroll
+  for (int i = 0; i < S; ++i) rank[i] = score[i] + (r.correction && lane + 32 * i < r.experts ? r.correction[lane + 32 * i] : 0.f);
+  unsigned left = 0u;      // of the lane's experts
+#pragma unroll
+  for (int i = 0; i < S; ++i) left |= lane + 32 * i < r.experts ? 1u << i : 0u;
+  float chosen_sum = 0.f, weight = 0.f;
+  int id = -1;
+  for (int k = 0; k < r.top; ++k) {
+    float best = -CUDART_INF_F, best_s = 0.f;
+    int best_e = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < S; ++i)
+      if ((left >> i & 1u) && (rank[i] > best || best_e == 0x7fffffff)) { best = rank[i]; best_s = score[i]; best_e = lane + 32 * i; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const float os = __shfl_xor_sync(0xffffffffu, best_s, o);
+      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
+      if (oe != 0x7fffffff && (best_e == 0x7fffffff || ob > best || (ob == best && oe < best_e))) { best = ob; best_s = os; best_e = oe; }
+    }
+    if ((best_e & 31) == lane && best_e < r.experts) left &= ~(1u << (best_e >> 5));
+    chosen_sum += best_s;
+    if (lane == k && best_e < r.experts) { id = best_e; weight = best_s; }
+  }
+  if (lane < r.top) {
+    r.ids[(size_t)t * r.top + lane] = id;
+    r.weights[(size_t)t * r.top + lane] = r.normalize ? weight / (chosen_sum + r.norm_eps) : weight;
+  }
+}
+
+// S: scores a lane keeps, 0: the general form.
+static int route_scores_a_lane(const MoeRouteArgs& r) {
+  if ((r.groups > 1 && r.keep < r.groups) || r.top > 32) return 0;
+  return r.experts <= 32 ? 1 : r.experts <= 64 ? 2 : r.experts <= 256 ? 8 : 0;
+}
+template <int S> __device__ __forceinline__ void moe_route_one(const MoeRouteArgs& r, int t, unsigned char* kept) {
+  if constexpr (S > 0) moe_route_token_few<S>(r, t);
+  else moe_route_token(r, t, kept);
+}
+#define TIB_ROUTE_PICK(S_OF, kernel, ...)                                                        \
+  do {                                                                                           \
+    switch (S_OF) {                                                                              \
+      case 1: TIB_LAUNCH_DEPENDENT(kernel<1>, __VA_ARGS__); break;                               \
+      case 2: TIB_LAUNCH_DEPENDENT(kernel<2>, __VA_ARGS__); break;                               \
+      case 8: TIB_LAUNCH_DEPENDENT(kernel<8>, __VA_ARGS__); break;                               \
+      default: TIB_LAUNCH_DEPENDENT(kernel<0>, __VA_ARGS__);                                     \
+    }                                                                                            \
+  } while (0)
+
+template <int S>
 __global__ void __launch_bounds__(128) moe_route_kernel(MoeRouteArgs r) {
   pdl_wait();
   pdl_trigger();
   __shared__ unsigned char kept_s[4][kRouteMaxGroups];
   const int warp = threadIdx.x >> 5, t = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (t < r.tokens) moe_route_token(r, t, kept_s[warp]);
+  if (t < r.tokens) moe_route_one<S>(r, t, kept_s[warp]);
 }
 
 // ------------------------------------------------------------------- group
@@ -249,25 +406,87 @@ __device__ __forceinline__ void moe_group_pairs(const int* ids, int pairs, int e
   }
 }
 
+// Up to kGroupPairs pairs a thread and kGroupExperts experts: every warp counts its own pairs, whose place among the warp's stays in a register, so
+// that ids are read once and no two warps meet in an atomic.  8,192 pairs over 32 experts behind the choices: 6.5 us, 7.8 with one set of counts and ids read twice.
+constexpr int kGroupPairs = 16, kGroupExperts = 256;
+__device__ __forceinline__ void moe_group_warps(const int* ids, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ order,
+                                               int* __restrict__ place) {
+  __shared__ int count[32][kGroupExperts];      // of a warp's pairs, then where the warp's begin
+  __shared__ int total[kGroupExperts];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int id[kGroupPairs], at[kGroupPairs];
+#pragma unroll
+  for (int j = 0; j < kGroupPairs; ++j) {
+    const int p = tid + j * 1024;
+    id[j] = p < pairs ? ids[p] : -1;
+  }
+  for (int e = lane; e < experts; e += 32) count[warp][e] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < kGroupPairs; ++j)
+    if (id[j] >= 0 && id[j] < experts) at[j] = atomicAdd(&count[warp][id[j]], 1);
+  __syncthreads();
+  if (tid < experts) {
+    int sum = 0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) {
+      const int own = count[w][tid];
+      count[w][tid] = sum;
+      sum += own;
+    }
+    total[tid] = sum;
+  }
+  __syncthreads();
+  if (tid < 32) {      // a warp's running sums, 32 experts at a time
+    int run = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + tid, own = e < experts ? total[e] : 0;
+      int upto = own;
+#pragma unroll
+      for (int step = 1; step < 32; step *= 2) {
+        const int below = __shfl_up_sync(0xffffffffu, upto, step);
+        if (tid >= step) upto += below;
+      }
+      if (e < experts) { offsets[e] = run + upto - own; total[e] = run + upto - own; }
+      run += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (tid == 0) offsets[experts] = run;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kGroupPairs; ++j) {
+    const int p = tid + j * 1024;
+    if (p >= pairs) break;
+    int s = -1;
+    if (id[j] >= 0 && id[j] < experts) {
+      s = total[id[j]] + count[warp][id[j]] + at[j];
+      order[s] = p;
+    }
+    place[p] = s;
+  }
+}
+
 __global__ void __launch_bounds__(1024)
 moe_group_kernel(const int* __restrict__ ids, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ order,
                  int* __restrict__ place) {
   pdl_wait();
   pdl_trigger();
-  moe_group_pairs(ids, pairs, experts, offsets, order, place);
+  if (pairs <= kGroupPairs * 1024 && experts <= kGroupExperts) moe_group_warps(ids, pairs, experts, offsets, order, place);
+  else moe_group_pairs(ids, pairs, experts, offsets, order, place);
 }
 
 // Both for a step of few tokens, in one launch: a warp per token makes its choices, then the block sorts the pairs.  (Eight tokens x 4
 // of 32: 7.4 us cold, where the two kernels took 5.0 and 3.5 and the second's launch; beyond 64 tokens, two rounds of the block's
 // warps, one block's arithmetic is slower than the grid's.)
 constexpr int kRouteGroupTokens = 64;
+template <int S>
 __global__ void __launch_bounds__(1024)
 moe_route_group_kernel(MoeRouteArgs r, int kept_experts, int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ place) {
   pdl_wait();
   pdl_trigger();
   __shared__ unsigned char kept_s[32][kRouteMaxGroups];
   const int warp = threadIdx.x >> 5;
-  for (int t = warp; t < r.tokens; t += 32) moe_route_token(r, t, kept_s[warp]);
+  for (int t = warp; t < r.tokens; t += 32) moe_route_one<S>(r, t, kept_s[warp]);
   __syncthreads();
   moe_group_pairs(r.ids, r.tokens * r.top, kept_experts, offsets, order, place);
 }
@@ -452,26 +671,29 @@ TIB_API int tib_router_logits(const void* x, int x_dtype, int64_t ldx, const flo
   if (tokens > 0x7fffffff / 2) return TIB_E_SIZE;
   const int64_t xbytes = x_dtype == TIB_F32 ? 4 : 2;
   const bool vec = K % 4 == 0 && (ldx * xbytes) % 16 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-  const bool many = vec && tokens >= kRouterMany * 148;      // (a block an SM at least)
+  // The kernel of large steps from 20,000 logits on: below, a warp a row and four tokens fill the GPU better (33 rows: 400 tokens 8.7 us against 11.5,
+  // 800 13.9 against 12.3; 61: 400 tokens 9.9 and 10.3; 129: 100 8.8 and 11.6, 200 13.8 and 12.3).
+  if (vec && (int64_t)tokens * rows >= 20000) {
+    const int passes = ceil_div(rows, kRouterWarps * kRouterRows), warps = ceil_div(rows, kRouterRows * passes);
+    const dim3 grid(ceil_div(tokens, kRouterMany), passes);
+    if (x_dtype == TIB_F32)
+      TIB_LAUNCH_DEPENDENT(router_logits_many_kernel<float>, grid, warps * 32, 0, stream, (const float*)x, ldx, w, bias, out, ldo, tokens, rows, K);
+    else if (x_dtype == TIB_BF16)
+      TIB_LAUNCH_DEPENDENT(router_logits_many_kernel<__nv_bfloat16>, grid, warps * 32, 0, stream, (const __nv_bfloat16*)x, ldx, w, bias, out, ldo, tokens,
+                           rows, K);
+    else
+      return TIB_E_DTYPE;
+    return TIB_OK;
+  }
   int slices = 1;      // few tokens: the rows of w are spread over several blocks a token
-  const int groups = ceil_div(tokens, many ? kRouterMany : kRouterTokens);
-  while (groups * slices < 2 * 148 && slices * 8 < rows && !many) slices *= 2;
-  dim3 grid(groups, slices);
-  // rows a warp works at a time in a large step: as few passes over the rows as five at a time need, shared out evenly
-  const int passes = ceil_div(rows, 8 * 5), together = ceil_div(rows, 8 * passes);
-#define TIB_ROUTER_R(TX, VEC, TOK, R) \
-  TIB_LAUNCH_DEPENDENT((router_logits_kernel<TX, VEC, TOK, R>), grid, 256, 0, stream, (const TX*)x, ldx, w, bias, out, ldo, tokens, rows, K)
-#define TIB_ROUTER_GO(TX, VEC)                                                    \
-  do {                                                                            \
-    if (!many) TIB_ROUTER_R(TX, VEC, kRouterTokens, 1);                           \
-    else if (together <= 1) TIB_ROUTER_R(TX, true, kRouterMany, 1);               \
-    else if (together <= 3) TIB_ROUTER_R(TX, true, kRouterMany, 3);               \
-    else TIB_ROUTER_R(TX, true, kRouterMany, 5);                                  \
-  } while (0)
+  const int groups = ceil_div(tokens, kRouterTokens);
+  while (groups * slices < 2 * 148 && slices * 8 < rows) slices *= 2;
+  const dim3 grid(groups, slices);
+#define TIB_ROUTER_GO(TX, VEC) \
+  TIB_LAUNCH_DEPENDENT((router_logits_kernel<TX, VEC>), grid, 256, 0, stream, (const TX*)x, ldx, w, bias, out, ldo, tokens, rows, K)
   if (x_dtype == TIB_F32) { if (vec) TIB_ROUTER_GO(float, true); else TIB_ROUTER_GO(float, false); }
   else if (x_dtype == TIB_BF16) { if (vec) TIB_ROUTER_GO(__nv_bfloat16, true); else TIB_ROUTER_GO(__nv_bfloat16, false); }
 #undef TIB_ROUTER_GO
-#undef TIB_ROUTER_R
   else
     return TIB_E_DTYPE;
   return TIB_OK;
@@ -495,10 +717,10 @@ TIB_API int tib_moe_route(const float* logits, int64_t ld, int tokens, int exper
   if (offsets) {      // choices and sorting in one launch
     if (!order || !place) return TIB_E_ARG;
     if (tokens > kRouteGroupTokens || sorted_experts < 1 || sorted_experts > 1024) return TIB_E_SIZE;
-    TIB_LAUNCH_DEPENDENT(moe_route_group_kernel, 1, 1024, 0, stream, r, sorted_experts, offsets, order, place);
+    TIB_ROUTE_PICK(route_scores_a_lane(r), moe_route_group_kernel, 1, 1024, 0, stream, r, sorted_experts, offsets, order, place);
     return TIB_OK;
   }
-  TIB_LAUNCH_DEPENDENT(moe_route_kernel, ceil_div(tokens, 4), 128, 0, stream, r);
+  TIB_ROUTE_PICK(route_scores_a_lane(r), moe_route_kernel, ceil_div(tokens, 4), 128, 0, stream, r);
   return TIB_OK;
 }
 
