@@ -226,6 +226,9 @@ TUNE_ROWS = ((1, 4), (8, 8), (16, 16), (32, 32), (64, 64))      # (rows measured
 # (see _stored_choices): the kernels a checkpoint runs on a GPU model do not change from one process to the next.
 TUNE_MARGIN = 1.04
 TUNE_MEMBERS = 32
+# A walk is at least this many products long, over a few weights again and again: two events are 2 us apart in steps of 2, and of a
+# single product the pick would be chance (a layer of latent attention on 8 tokens took 47 to 53 us by what was picked).
+TUNE_PRODUCTS = 32
 _flush: dict[torch.device, torch.Tensor] = {}     # larger than the L2; made once per tuning pass
 
 
@@ -383,8 +386,10 @@ def _walk_time(group: "list[LinearWeight]", rows: int, config: tuple[int, int] |
             else:
                 ops.gemm_decode(x, w.tensor, out, features=config[0], splits=config[1])
 
+        rounds = -(-TUNE_PRODUCTS // len(group))
+
         def walk() -> None:
-            for w in group:
+            for w in group * rounds:
                 ops.add_rmsnorm(delta, residual, norm_weight, 1e-5, normed)
                 product(w)
         walk()                                                            # (first launches: attributes, handles)
@@ -405,7 +410,7 @@ def _walk_time(group: "list[LinearWeight]", rows: int, config: tuple[int, int] |
             if i >= 2:
                 best = min(best, begin.elapsed_time(end))
         del graph
-    return best * 1e3 / len(group)
+    return best * 1e3 / (len(group) * rounds)
 
 
 def _linear_bf16(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
