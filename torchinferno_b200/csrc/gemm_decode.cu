@@ -12,7 +12,8 @@
 //     meet in distributed shared memory, as in gemm_tcgen05.cu.
 //   * warp 0 / one lane: TMA producer into a ring of stages; it requests its first ring of weights before
 //     `griddepcontrol.wait`, while the kernel before this one is still running (the weights do not depend on it).
-//     warp 1 / one lane: MMA issue and TMEM ownership.  warps 2..5: epilogue; with tiles of 256 features four such
+//     warp 1: MMA issue (the whole warp walks the loop and one lane issues: with a lone lane a stage of the ring took twice as long, which
+//     is what counts once x has come and the ring is full: a block on 8 tokens of the 8B sizes 113.9 -> 109.8 us) and TMEM ownership.  warps 2..5: epilogue; with tiles of 256 features four such
 //     sets of four warps (a warp reaches only its quarter of the lanes of tensor memory, so the sets share the work
 //     by accumulator and by odd and even rows): the epilogue is not overlapped with anything when a block has one tile.
 //   * Epilogues: plain (bf16 or fp32 rows), or SwiGLU: the matrix holds gate and up columns interleaved
@@ -72,7 +73,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   unsigned char* smem_gen = smem_raw + (base - smem_u32(smem_raw));        // generic pointer to `base`
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - base));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t splits = FT == 128 ? cluster_size() : 1u, rank = FT == 128 ? cluster_rank() : 0u;
   const int cluster_id = blockIdx.x / splits, clusters = gridDim.x / splits;
   const int n_tiles = (N + FT - 1) / FT;
@@ -101,7 +102,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot_ptr;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot_ptr, 0);
   if (splits > 1) cluster_sync_all();   // every block of the cluster runs and has its barriers: peers may touch them
   auto load_w = [&](uint32_t dst, int t, int kb, uint32_t bar) {
 #pragma unroll
@@ -141,40 +142,41 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // D fp32, A and B bf16, A MN-major (bit 15), B K-major, N = NPAD, M = 128
-      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(NPAD >> 3) << 17) |
-                                 ((uint32_t)(128 >> 4) << 24);
-      bool ok = true;
-      int j = 0, s = 0;
-      uint32_t phase = 0;
-      for (int t = cluster_id; t < n_tiles && ok; t += clusters, ++j) {
-        const int b = j & 1;
-        if (!mbar_wait(acc_empty_bar(b), ((j >> 1) & 1) ^ 1)) {
-          if (error_word) atomicExch(error_word, 0x7C0044);
+    // D fp32, A and B bf16, A MN-major (bit 15), B K-major, N = NPAD, M = 128
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(NPAD >> 3) << 17) |
+                               ((uint32_t)(128 >> 4) << 24);
+    const uint32_t leader = umma_leader();
+    bool ok = true;
+    int j = 0, s = 0;
+    uint32_t phase = 0;
+    for (int t = cluster_id; t < n_tiles && ok; t += clusters, ++j) {
+      const int b = j & 1;
+      if (!mbar_wait_warp(acc_empty_bar(b), ((j >> 1) & 1) ^ 1)) {
+        if (error_word && leader) atomicExch(error_word, 0x7C0044);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      for (int kb = kb0; kb < kb1; ++kb, phase ^= (s + 1 == kStages), s = (s + 1 == kStages ? 0 : s + 1)) {
+        if (!mbar_wait_warp(full_bar(s), phase)) {
+          if (error_word && leader) atomicExch(error_word, 0x7C0042);
+          ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        for (int kb = kb0; kb < kb1; ++kb, phase ^= (s + 1 == kStages), s = (s + 1 == kStages ? 0 : s + 1)) {
-          if (!mbar_wait(full_bar(s), phase)) {
-            if (error_word) atomicExch(error_word, 0x7C0042);
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          const uint32_t w_src = base + s * kStage, x_src = w_src + kWBytes;
+        const uint32_t w_src = base + s * kStage, x_src = w_src + kWBytes;
 #pragma unroll
-          for (int k = 0; k < kDgBK / 16; ++k) {
-            const uint64_t bdesc = umma_desc_k128(x_src + k * 32);
+        for (int k = 0; k < kDgBK / 16; ++k) {
+          const uint32_t b_low = umma_low_k128(x_src + k * 32);
 #pragma unroll
-            for (int h = 0; h < H; ++h)
-              umma_f16_idesc(tmem_base + (b * H + h) * NPAD, umma_desc_mn128(w_src + h * 16384 + k * 16 * 128, 8192), bdesc, idesc,
-                             (kb > kb0) || (k > 0));
-          }
-          umma_commit(empty_bar(s));
+          for (int h = 0; h < H; ++h)
+            umma_warp(leader, tmem_base + (b * H + h) * NPAD, umma_low_mn128(w_src + h * 16384 + k * 16 * 128, 8192), b_low, idesc,
+                      (kb > kb0) || (k > 0));
         }
-        umma_commit(acc_full_bar(b));
+        if (leader) umma_commit(empty_bar(s));
+        __syncwarp();
       }
+      if (leader) umma_commit(acc_full_bar(b));
+      __syncwarp();
     }
   } else {
     pdl_wait();                                        // `out` may be memory the kernel before still reads
