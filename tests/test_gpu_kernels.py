@@ -1942,3 +1942,24 @@ def test_pairs_are_sorted_by_expert(pairs, experts):
     held = order[:int(inside.sum())]
     assert torch.equal(held.sort().values, inside.nonzero().flatten())                       # every pair once
     assert torch.equal(place[held], torch.arange(len(held))) and (ids[held].long().diff() >= 0).all()
+
+
+@pytest.mark.parametrize("n, k, many", [(512, 8192, 700), (2048, 4096, 2100), (2050, 2112, 1500), (8190, 2048, 300)])
+def test_fp32_product_in_parts_of_k_has_one_order(n, k, many):
+    """Parts that blocks of their own sum, and parts that one block sums one after the other: the same bits."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    x, w = dev(rnd(many, k)), dev(rnd(n, k, seed=3))
+    apart = [ops.lib().tib_gemm_f32_tcgen05_partial(m, n, k, m) for m in (8, 130, many)]
+    assert apart[0] > 0                                                    # (few rows: blocks of their own)
+    out = ops.gemm_f32(x, w, torch.empty(many, n, device="cuda"))
+    for m in (8, 130):
+        assert torch.equal(ops.gemm_f32(x[:m], w, torch.empty(m, n, device="cuda")), out[:m])
+    whole = torch.empty(130, n, device="cuda")
+    scratch = torch.empty(3 * 130 * k, dtype=torch.bfloat16, device="cuda")
+    launches = torch.zeros(1, dtype=torch.int32)
+    assert ops.lib().tib_gemm_f32_tcgen05(x.data_ptr(), w.data_ptr(), whole.data_ptr(), 130, n, k, k, k, n, scratch.data_ptr(), 130, 0, 0, 0,
+                                          launches.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0      # (no room for the parts' sums)
+    assert torch.equal(whole, out[:130]) and int(launches) == 2
+    exact = x[:130].double() @ w.double().T
+    assert (whole.double() - exact).norm() <= 4e-7 * exact.norm()          # (the bound of the products in one part)

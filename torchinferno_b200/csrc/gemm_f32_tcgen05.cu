@@ -20,8 +20,8 @@
 // What bounds it: the warp that issues the MMAs, which waits once and issues 16 instructions a step of 64 k (0.95 us at 80 rows, of which 0.5 are
 // products), and for the last round of tiles the SMs that have none.  A wait for the rows, one for each half of the weights' terms and one
 // commit each made it 1.15 us; a lane issuing alone takes 45 cycles an instruction instead of 8.  301 rows, us, against gemm_f32.cu's fused
-// multiply-adds: 16,384 x 2,048 123 (536), 2,048 x 8,192 98 (431), 2,048 x 2,048 33 (111); 8 rows: 31 (68), 84 (146), 26 (39).
-// Error against 64 bits (2-norm): 1.4e-7 at 2,048 k and 2.0e-7 at 8,192, where multiply-adds in order have 8.1e-7 and 1.6e-6; numbers of one
+// multiply-adds: 16,384 x 2,048 119 (536), 2,048 x 8,192 72 (431), 2,048 x 2,048 25 (111); 8 rows: 30 (68), 33 (146), 17 (39).
+// Error against 64 bits (2-norm): 1.4e-7 at 2,048 k and 1.5e-7 at 8,192, where multiply-adds in order have 8.1e-7 and 1.6e-6; numbers of one
 // sign 1.6e-7 (6.3e-7); sums over 256 k 2.4e-7, for a tenth off the time.
 // An output that is not finite is worked out again with fused multiply-adds in order (an infinity's terms make NaN of it).
 #include "split_terms.cuh"
@@ -66,9 +66,40 @@ struct FtArgs {
   int64_t ldx, ldw, ldo;
   int M, N, K;
   int rows;               // rows of a tile (a multiple of 16, at most kFtRows)
+  int parts;              // of k, each summed by itself
+  float* partial;         // [parts][M][N]: the parts' sums go there, a block takes any part of any tile; null: a block takes all parts of a tile, one after the other
   int w_stages, x_stages;
   int* error_word;
 };
+
+// A thread's sums of one feature into out (fetched and added to where `onto`); LAST: what is not finite is made again.
+template <bool LAST>
+__device__ __forceinline__ void ft_put(float (&sum)[kFtGroups][16], float* out, int64_t ld, bool onto, int m0, int feature, int half, const FtArgs& a) {
+  if (feature >= a.N) return;
+#pragma unroll
+  for (int g = 0; g < kFtGroups; ++g) {
+    const int j0 = (2 * g + half) * 16, left = min(a.rows - j0, a.M - m0 - j0);
+    if (left <= 0) break;
+    float* to = out + (size_t)(m0 + j0) * ld + feature;
+    if (onto) {
+#pragma unroll
+      for (int c0 = 0; c0 < 16; c0 += 8) {
+        float before[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) before[c] = c0 + c < left ? to[(c0 + c) * ld] : 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) sum[g][c0 + c] = before[c] + sum[g][c0 + c];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      if (c >= left) break;
+      float v = sum[g][c];
+      if (LAST && !isfinite(v)) v = ft_plain_sum(a.x + (size_t)(m0 + j0 + c) * a.ldx, a.w + (size_t)feature * a.ldw, a.K);
+      to[c * ld] = v;
+    }
+  }
+}
 
 __global__ void __launch_bounds__(kFtThreads, 1)
 gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, FtArgs a) {
@@ -115,8 +146,29 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 
   const int m_tiles = (a.M + a.rows - 1) / a.rows, f_tiles = (a.N + kFtM - 1) / kFtM, num_tiles = m_tiles * f_tiles;
   const int k_steps = a.K / kFtK;
-  const int own = (int)blockIdx.x < num_tiles ? (num_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;      // tiles of this block
-  const int total = own * k_steps;
+  // This block's pieces of work: parts of tiles, steps first .. end - 1 of k.
+  struct Piece { int tile, part, first, end; };
+  const int of_tile = a.partial ? 1 : a.parts, stride = (int)gridDim.x, all = a.partial ? num_tiles * a.parts : num_tiles;
+  const int pieces = (int)blockIdx.x < all ? (all - (int)blockIdx.x + stride - 1) / stride * of_tile : 0;
+  const auto piece_of = [&](int i) {
+    Piece u;
+    if (a.partial) {
+      const int at = (int)blockIdx.x + i * stride;
+      u.tile = at / a.parts;
+      u.part = at - u.tile * a.parts;
+    } else {
+      u.tile = (int)blockIdx.x + i / a.parts * stride;
+      u.part = i % a.parts;
+    }
+    u.first = k_steps * u.part / a.parts;
+    u.end = k_steps * (u.part + 1) / a.parts;
+    return u;
+  };
+  int total = 0;
+  for (int i = 0; i < pieces; ++i) {
+    const Piece u = piece_of(i);
+    total += u.end - u.first;
+  }
 
   if (warp < 16) {
     // lane: a feature; the warp's 16 of the step's 64 k (which come as two copies of 32 k: rows of 128 bytes, swizzled)
@@ -167,9 +219,10 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       int ws = 0, xs = 0;
       uint32_t wphase = 1, xphase = 1;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int m0 = t % m_tiles * a.rows, f0 = t / m_tiles * kFtM;
-        for (int ks = 0; ks < k_steps; ++ks) {
+      for (int i = 0; i < pieces && ok; ++i) {
+        const Piece u = piece_of(i);
+        const int m0 = u.tile % m_tiles * a.rows, f0 = u.tile / m_tiles * kFtM;
+        for (int ks = u.first; ks < u.end; ++ks) {
           ok = mbar_wait(w_empty_bar(ws), wphase);
           if (ok) {
             mbar_expect_tx(w_full_bar(ws), kFtW);
@@ -199,20 +252,21 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     const uint32_t leader = umma_leader(), idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFtM >> 4) << 24);
     const uint32_t n1 = (uint32_t)(a.rows >> 4) << 18;      // (an instruction's columns, in sixteens)
     int s = 0;
-    uint32_t phase = 0, chunk = 0, it = 0, tile = 0;
+    uint32_t phase = 0, chunk = 0, it = 0;
     bool ok = true;
     const uint32_t small = tmem_base + kFtSums + 2 * kFtRows;      // (behind each other: a.rows columns a group)
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile) {
-      for (int ks = 0; ks < k_steps && ok; ks += kFtChunk, ++chunk) {
+    for (int i = 0; i < pieces && ok; ++i) {
+      const Piece u = piece_of(i);
+      for (int ks = u.first; ks < u.end && ok; ks += kFtChunk, ++chunk) {
         const int ab = chunk & 1;
-        const bool free = mbar_wait(acc_empty_bar(ab), ((chunk >> 1) & 1) ^ 1) && (ks > 0 || mbar_wait(small_empty_bar, (tile & 1) ^ 1));
+        const bool free = mbar_wait(acc_empty_bar(ab), ((chunk >> 1) & 1) ^ 1) && (ks > u.first || mbar_wait(small_empty_bar, (i & 1) ^ 1));
         if (!__all_sync(0xffffffffu, free)) {
           if (a.error_word && leader) atomicExch(a.error_word, 0x7C0094);
           ok = false;
           break;
         }
         const uint32_t large = tmem_base + kFtSums + ab * kFtRows;
-        for (int kc = 0; kc < kFtChunk && ks + kc < k_steps && ok; ++kc, ++it) {
+        for (int kc = 0; kc < kFtChunk && ks + kc < u.end && ok; ++kc, ++it) {
           const uint32_t xs = xring + s * 3 * xplane, wt = tmem_base + (it & 1) * kFtTermCols;
           if (!__all_sync(0xffffffffu, mbar_wait(x_full_bar(s), phase))) {
             if (a.error_word && leader) atomicExch(a.error_word, 0x7C0093);
@@ -224,7 +278,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
           for (int k = 0; k < kFtK / 16; ++k) {
             const uint32_t x0 = umma_low_k128(xs + k * 32), x1 = umma_low_k128(xs + xplane + k * 32);
             const uint32_t w0 = wt + k * 8, w1 = w0 + kFtK / 2, w2 = w1 + kFtK / 2;
-            umma_warp_tmem(leader, small, w0, x1, idesc0 | 2 * n1, (ks | kc | k) != 0);
+            umma_warp_tmem(leader, small, w0, x1, idesc0 | 2 * n1, (ks - u.first | kc | k) != 0);
             umma_warp_tmem(leader, small, w1, x0, idesc0 | 2 * n1, 1);
             umma_warp_tmem(leader, small + a.rows, w2, x0, idesc0 | n1, 1);
             umma_warp_tmem(leader, large, w0, x0, idesc0 | n1, (kc | k) != 0);
@@ -242,13 +296,14 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     const int quarter = warp & 3, half = (warp - 18) >> 2;      // 32 features; groups of 16 rows half, half + 2, ...
     uint32_t chunk = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+    for (int i = 0; i < pieces && ok; ++i) {
+      const Piece u = piece_of(i);
       float sum[kFtGroups][16];
 #pragma unroll
       for (int g = 0; g < kFtGroups; ++g)
 #pragma unroll
         for (int c = 0; c < 16; ++c) sum[g][c] = 0.f;
-      for (int ks = 0; ks < k_steps; ks += kFtChunk, ++chunk) {
+      for (int ks = u.first; ks < u.end; ks += kFtChunk, ++chunk) {
         const int b = chunk & 1;
         if (!mbar_wait(acc_full_bar(b), (chunk >> 1) & 1)) {
           if (a.error_word && lane == 0) atomicExch(a.error_word, 0x7C0095);
@@ -256,7 +311,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const bool last = ks + kFtChunk >= k_steps;
+        const bool last = ks + kFtChunk >= u.end;
         const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + kFtSums;
 #pragma unroll
         for (int g = 0; g < kFtGroups; ++g) {
@@ -289,17 +344,15 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         }
       }
       if (!ok) break;
-      const int m0 = t % m_tiles * a.rows, feature = t / m_tiles * kFtM + quarter * 32 + lane;
-#pragma unroll
-      for (int g = 0; g < kFtGroups; ++g)
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const int j = (2 * g + half) * 16 + c;
-          if (j >= a.rows || m0 + j >= a.M || feature >= a.N) continue;
-          float v = sum[g][c];
-          if (!isfinite(v)) v = ft_plain_sum(a.x + (size_t)(m0 + j) * a.ldx, a.w + (size_t)feature * a.ldw, a.K);
-          a.out[(size_t)(m0 + j) * a.ldo + feature] = v;
-        }
+      const int m0 = u.tile % m_tiles * a.rows, feature = u.tile / m_tiles * kFtM + quarter * 32 + lane;
+      const bool last = u.part == a.parts - 1;
+      if (a.partial || !last) {      // (a part's sum: by itself, or on top of the parts' before it, whose sums are all asked for first)
+        float* dst = a.partial ? a.partial + (size_t)u.part * a.M * a.N : a.out;
+        const int64_t ld = a.partial ? a.N : a.ldo;
+        ft_put<false>(sum, dst, ld, !a.partial && u.part > 0, m0, feature, half, a);
+      } else {
+        ft_put<true>(sum, a.out, a.ldo, u.part > 0, m0, feature, half, a);
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -308,6 +361,64 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
   }
+}
+
+// The parts' sums, in their order: four outputs a thread.
+__global__ void __launch_bounds__(256) add_parts_kernel(FtArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t outputs = (int64_t)a.M * a.N, first = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+  float v[4], next[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = first + i * 256 < outputs ? a.partial[first + i * 256] : 0.f;
+  for (int p = 1; p < a.parts; ++p) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) next[i] = first + i * 256 < outputs ? a.partial[p * outputs + first + i * 256] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = v[i] + next[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int64_t e = first + i * 256;
+    if (e >= outputs) break;
+    const int64_t row = e / a.N, f = e - row * a.N;
+    a.out[row * a.ldo + f] = isfinite(v[i]) ? v[i] : ft_plain_sum(a.x + row * a.ldx, a.w + f * a.ldw, a.K);
+  }
+}
+
+// Into how many parts of k a product is summed, each by itself: by the weight's sizes alone, so that a row's bits do not depend on how many rows
+// there are.  A weight of few features leaves SMs without a tile (2,048 features, 301 rows: 64 to 112 tiles), and these parts are work for them:
+// 2,048 x 8,192 in four, us on 8 / 100 / 301 / 1,000 / 2,048 rows, 85 / 89 / 96 / 200 / 367 in one and 33 / 39 / 72 / 194 / 383; 2,048 x 2,048 in two
+// 26 / 28 / 31 / 58 / 94 and 17 / 20 / 25 / 59 / 98 (with many rows the parts only cost their ends); 3,072 x 2,048 27 / 28 / 32 / 83 / 150 and
+// 17 / 21 / 32 / 84 / 156.
+static int ft_parts(int N, int K) {
+  const int f_tiles = ceil_div(N, kFtM), k_steps = K / kFtK;
+  return f_tiles <= 32 && k_steps >= 64 ? 4 : f_tiles <= 64 && k_steps >= 32 ? 2 : 1;
+}
+
+// Rows of a tile, and whether the parts go to blocks of their own: whole rounds of work over the SMs times its steps' cost (0.65 us with 16
+// rows, 0.76 with 48, 0.95 with 80: in units of 1 / 210 us), and for parts of their own the launch that adds them (3 us, and their way through the L2).
+struct FtPlan { int rows; bool apart; };
+static FtPlan ft_plan(int rows, int N, int K, bool may_part) {
+  const int parts = ft_parts(N, K), k_steps = K / kFtK;
+  FtPlan plan = {kFtRows, false};
+  double least = 1e30;
+  for (int tiles = ceil_div(rows, kFtRows); tiles <= ceil_div(rows, 16); ++tiles) {
+    const int r = ceil_div(ceil_div(rows, tiles), 16) * 16;
+    const int64_t n = (int64_t)ceil_div(rows, r) * ceil_div(N, kFtM);
+    const double step = 120 + r, whole = (double)ceil_div64(n, 148) * k_steps * step;
+    const double bytes = 8.0 * parts * rows * N;
+    const double apart = parts > 1 && may_part && bytes <= 128e6 ? (double)ceil_div64(n * parts, 148) * ceil_div(k_steps, parts) * step + 210 * (3 + bytes / 4e6) : 1e30;
+    if (whole < least) {
+      least = whole;
+      plan = {r, false};
+    }
+    if (apart < least) {
+      least = apart;
+      plan = {r, true};
+    }
+  }
+  return plan;
 }
 
 // Rows of 32-bit weights in boxes of 128 x 32.
@@ -334,6 +445,7 @@ using namespace tib;
 //     1,024 wide, 2,112 inside   135 / 149 / 206 / 361   142 / 144 / 189 / 302   162 / 163 / 162 / 161
 //     1,536 wide, 3,200 inside   191 / 237 / 340 / 599   156 / 158 / 195 / 275   161 / 162 / 168 / 231
 //     1,536 wide, 6,400 inside   253 / 312 / 486 / 856   180 / 188 / 242 / 328   167 / 175 / 214 / 284
+// (measured when no product was summed in parts and the host took some 30 us more a block).
 // So no line is best for all: 2^22 costs few tokens 5 % (the second block's 4.3 million of gate and up), where 2^20 would cost them 20 % and gain
 // prompts of a hundred tokens and more 15 to 45 %.
 // (Weights whose rows overlap or are one and the same are none of a tensor map's.)
@@ -342,31 +454,33 @@ TIB_API int tib_gemm_f32_tcgen05_takes(const void* x, const void* w, int N, int 
          (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
 }
 
+// Rows of N numbers that a product of M rows, made scratch_rows at a time, takes for its parts' sums (0: none).
+TIB_API int tib_gemm_f32_tcgen05_partial(int M, int N, int K, int scratch_rows) {
+  if (M < 1 || N < 1 || K < kFtK || scratch_rows < 1) return 0;
+  int most = 0;
+  for (int rows : {M < scratch_rows ? M : scratch_rows, M % scratch_rows})
+    if (rows > 0 && ft_plan(rows, N, K, true).apart && ft_parts(N, K) * rows > most) most = ft_parts(N, K) * rows;
+  return most;
+}
+
 // x: [M, K] (row stride ldx), w: [N, K] (row stride ldw), out: [M, N] (row stride ldo), all fp32.  scratch: bf16, 3 K numbers for each
-// of scratch_rows rows, on a 16-byte boundary; the product is made for that many rows at a time.  launches: takes the number of kernels launched.
+// of scratch_rows rows, on a 16-byte boundary; the product is made for that many rows at a time.  partial: partial_rows rows of N numbers, as many as
+// tib_gemm_f32_tcgen05_partial says (fewer, or none: the same bits, a block taking all parts of a tile).  launches: takes the number of kernels launched.
 TIB_API int tib_gemm_f32_tcgen05(const float* x, const float* w, float* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
-                                 void* scratch, int scratch_rows, int* error_word, int* launches, cudaStream_t stream) {
+                                 void* scratch, int scratch_rows, float* partial, int partial_rows, int* error_word, int* launches, cudaStream_t stream) {
   *launches = 0;
   if (M == 0) return TIB_OK;
   if (!x || !w || !out || !scratch || M < 0 || scratch_rows < 1 || ((uintptr_t)scratch & 15)) return TIB_E_ARG;
   if (!tib_gemm_f32_tcgen05_takes(x, w, N, K, ldx, ldw) || (int64_t)scratch_rows * 3 > 0x7fffffff - 256) return TIB_E_SIZE;
+  const int parts = ft_parts(N, K);
   for (int first = 0; first < M; first += scratch_rows) {
     const int rows = M - first < scratch_rows ? M - first : scratch_rows;
-    // Rows of a tile: whole rounds of tiles over the SMs times a step's cost (0.65 us with 16 rows, 0.76 with 48, 0.95 with 80).
-    int best = kFtRows;
-    double least = 1e30;
-    for (int tiles = ceil_div(rows, kFtRows); tiles <= ceil_div(rows, 16); ++tiles) {
-      const int r = ceil_div(ceil_div(rows, tiles), 16) * 16;
-      const double step = 120 + r;
-      const double cost = (double)ceil_div64((int64_t)ceil_div(rows, r) * ceil_div(N, kFtM), 148) * step;
-      if (cost < least) {
-        least = cost;
-        best = r;
-      }
-    }
+    const FtPlan plan = ft_plan(rows, N, K, partial && (int64_t)parts * rows <= partial_rows);
+    const int best = plan.rows;
     FtArgs a;
     a.x = x + (size_t)first * ldx; a.w = w; a.out = out + (size_t)first * ldo;
     a.ldx = ldx; a.ldw = ldw; a.ldo = ldo; a.M = rows; a.N = N; a.K = K; a.rows = best; a.error_word = error_word;
+    a.parts = parts; a.partial = plan.apart ? partial : nullptr;
     const int x_stage = 3 * best * kFtK * 2;
     a.x_stages = best > 48 ? 4 : 6;
     a.w_stages = (220 * 1024 - a.x_stages * x_stage) / (int)kFtW < 6 ? (220 * 1024 - a.x_stages * x_stage) / (int)kFtW : 6;
@@ -379,13 +493,18 @@ TIB_API int tib_gemm_f32_tcgen05(const float* x, const float* w, float* out, int
     if (e != cudaSuccess) return (int)e;
     const int64_t blocks = ceil_div64((int64_t)rows * K / 4, 256);
     TIB_LAUNCH_DEPENDENT(split_rows_kernel, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, a.x, ldx, rows, K, (__nv_bfloat16*)scratch);
-    const int64_t tiles = (int64_t)ceil_div(rows, best) * ceil_div(N, kFtM);
+    const int64_t tiles = (int64_t)ceil_div(rows, best) * ceil_div(N, kFtM) * (plan.apart ? parts : 1);
     TIB_LAUNCH_DEPENDENT(gemm_f32_tcgen05_kernel, (int)(tiles < 148 ? tiles : 148), kFtThreads, smem, stream, map_w, map, a);
     *launches += 2;
+    if (plan.apart) {
+      TIB_LAUNCH_DEPENDENT(add_parts_kernel, (unsigned)ceil_div64((int64_t)rows * N, 1024), 256, 0, stream, a);
+      ++*launches;
+    }
   }
   return TIB_OK;
 }
 
 // The calls the Python parts make (common.cuh).
 TIB_PACKED(tib_gemm_f32_tcgen05)
+TIB_PACKED(tib_gemm_f32_tcgen05_partial)
 TIB_PACKED(tib_gemm_f32_tcgen05_takes)

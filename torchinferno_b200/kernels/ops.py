@@ -303,9 +303,11 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, error_word: to
             _ptr(x), _ptr(w), n, k, x.stride(0), w.stride(0)):
         rows = min(m, max(128, F32_TERMS_BYTES // (6 * k)))
         scratch = torch.empty(3 * rows * k, dtype=torch.bfloat16, device=x.device)
+        need = lib().tib_gemm_f32_tcgen05_partial(m, n, k, rows)
+        partial = torch.empty(need * n, dtype=torch.float32, device=x.device) if need else None
         launches = c_int(0)
         _check("gemm_f32", lib().tib_gemm_f32_tcgen05(_ptr(x), _ptr(w), _ptr(out), m, n, k, x.stride(0),
-                                                      w.stride(0), out.stride(0), _ptr(scratch), rows,
+                                                      w.stride(0), out.stride(0), _ptr(scratch), rows, _ptr(partial), need,
                                                       _ptr(error_word), ctypes.addressof(launches), _stream()))
         count_launches(launches.value - 1)
         return out
