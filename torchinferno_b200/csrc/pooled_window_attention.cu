@@ -187,13 +187,21 @@ __global__ void __launch_bounds__(1024) pwa_append_pairs_kernel(const __nv_bfloa
 
 // The same bits again for large steps whose heads come in whole pieces of 16 bytes: a thread owns 16 elements of a head (eight and their
 // eight partners, or 16 neighbours that are not turned) and asks for them before the token's angles are worked out and its page is
-// found, so that a token is two trips to memory long.  2,048 tokens of 16 + 8 + 8 heads of 128: 14 us, 20 with two elements a thread at a time.
-__global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloat16* __restrict__ proj, __nv_bfloat16* __restrict__ q_out, PwaAppendArgs a) {
+// found, so that a token is two trips to memory long.  A block takes two tokens, whose biases and frequencies are fetched once: half as many rounds of
+// blocks, each as long as one trip.  2,048 tokens of 16 + 8 + 8 heads of 128: 10.1 us (one token a block 12.6; two elements a thread at a time 20 cold).
+constexpr int kPwaPair = 2;      // tokens of a block
+__global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloat16* __restrict__ proj, __nv_bfloat16* __restrict__ q_out, PwaAppendArgs a, int n_tokens) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float2 turn_s[kPwaTurns], vturn_s[kPwaTurns];      // (cosine, sine)
-  const int t = blockIdx.x, pos = a.positions[t], slot = a.cache.keys ? a.token_slot[t] : 0;
-  const __nv_bfloat16* row = proj + (size_t)t * a.ld;
+  __shared__ float2 turn_s[kPwaPair][kPwaTurns], vturn_s[kPwaPair][kPwaTurns];      // (cosine, sine)
+  const int t0 = blockIdx.x * kPwaPair, own = min(kPwaPair, n_tokens - t0);
+  int pos[kPwaPair], slot[kPwaPair];
+#pragma unroll
+  for (int u = 0; u < kPwaPair; ++u) {
+    pos[u] = a.positions[t0 + min(u, own - 1)];
+    slot[u] = a.cache.keys ? a.token_slot[t0 + min(u, own - 1)] : 0;
+  }
+  const __nv_bfloat16* row = proj + (size_t)t0 * a.ld;
   const int half = a.rot_dim / 2, vhalf = a.vfreq ? a.vdim / 2 : 0;
   const int units = a.dim / 16, vunits = a.vdim / 16, qk = (a.heads + a.kv_heads) * units, total = qk + a.kv_heads * vunits;
   struct Unit { const __nv_bfloat16* src; const float* bias; int head, i, k; bool value; };      // elements i .. i + 7 and k .. k + 7 of a head
@@ -217,11 +225,15 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
     }
     return u;
   };
-  struct Pieces { uint4 lo, hi; float4 bias[4]; };
+  struct Pieces { uint4 lo[kPwaPair], hi[kPwaPair]; float4 bias[4]; };
   auto ask = [&](const Unit& u) {
     Pieces p;
-    p.lo = *reinterpret_cast<const uint4*>(u.src + u.i);
-    p.hi = *reinterpret_cast<const uint4*>(u.src + u.k);
+#pragma unroll
+    for (int w = 0; w < kPwaPair; ++w) {
+      const __nv_bfloat16* src = u.src + (w < own ? (size_t)w * a.ld : 0);
+      p.lo[w] = *reinterpret_cast<const uint4*>(src + u.i);
+      p.hi[w] = *reinterpret_cast<const uint4*>(src + u.k);
+    }
     if (u.bias) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
@@ -231,14 +243,17 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
     }
     return p;
   };
-  int page = -1, in_page = 0;
-  auto put = [&](const Unit& u, const Pieces& p) {
+  int pages[kPwaPair], in_pages[kPwaPair];
+#pragma unroll
+  for (int u = 0; u < kPwaPair; ++u) pages[u] = -1, in_pages[u] = 0;
+  auto put_one = [&](const Unit& u, const Pieces& p, int w) {
+    const int page = pages[w], in_page = in_pages[w], t = t0 + w;
     __nv_bfloat16* dst;
     if (!u.value && u.head < a.heads) dst = q_out + ((size_t)t * a.heads + u.head) * a.dim;
     else if (page < 0) return;
     else if (u.value) dst = reinterpret_cast<__nv_bfloat16*>(a.cache.values) + (size_t)page * a.cache.page_stride + ((size_t)u.head * a.cache.page_size + in_page) * a.vdim;
     else dst = reinterpret_cast<__nv_bfloat16*>(a.cache.keys) + (size_t)page * a.cache.page_stride + ((size_t)(u.head - a.heads) * a.cache.page_size + in_page) * a.dim;
-    const uint32_t l[4] = {p.lo.x, p.lo.y, p.lo.z, p.lo.w}, h[4] = {p.hi.x, p.hi.y, p.hi.z, p.hi.w};
+    const uint32_t l[4] = {p.lo[w].x, p.lo[w].y, p.lo[w].z, p.lo[w].w}, h[4] = {p.hi[w].x, p.hi[w].y, p.hi[w].z, p.hi[w].w};
     float lo[8], hi[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -253,7 +268,7 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
       }
     }
     if (u.k - u.i != 8 || u.i < (u.value ? vhalf : half)) {      // turned (partners eight apart: a half of eight, which its index tells apart)
-      const float2* turns = (u.value ? vturn_s : turn_s) + u.i;
+      const float2* turns = (u.value ? vturn_s[w] : turn_s[w]) + u.i;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float2 turn = turns[j];
@@ -272,6 +287,11 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
     *reinterpret_cast<uint4*>(dst + u.i) = out[0];
     *reinterpret_cast<uint4*>(dst + u.k) = out[1];
   };
+  auto put = [&](const Unit& u, const Pieces& p) {
+#pragma unroll
+    for (int w = 0; w < kPwaPair; ++w)
+      if (w < own) put_one(u, p, w);
+  };
   Unit mine;
   Pieces held;
   const bool any = (int)threadIdx.x < total;
@@ -280,18 +300,23 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
     held = ask(mine);
   }
   if (a.cache.keys) {
-    const int* table = a.cache.block_table + (size_t)slot * a.cache.table_stride;
-    page = pwa_page(a.cache, table, pos, a.error_word, 0x30000 + (t & 0xffff));
-    in_page = pos % a.cache.page_size;
+#pragma unroll
+    for (int u = 0; u < kPwaPair; ++u) {
+      if (u >= own) break;
+      const int* table = a.cache.block_table + (size_t)slot[u] * a.cache.table_stride;
+      pages[u] = pwa_page(a.cache, table, pos[u], a.error_word, 0x30000 + ((t0 + u) & 0xffff));
+      in_pages[u] = pos[u] % a.cache.page_size;
+    }
   }
-  for (int i = threadIdx.x; i < half + vhalf; i += blockDim.x) {
-    const bool key = i < half;
-    const float angle = (float)pos * (key ? a.freq[i] : a.vfreq[i - half]);
+  for (int i = threadIdx.x; i < (half + vhalf) * own; i += blockDim.x) {
+    const int w = i >= half + vhalf ? 1 : 0, j = i - w * (half + vhalf);
+    const bool key = j < half;
+    const float angle = (float)(w ? pos[1] : pos[0]) * (key ? a.freq[j] : a.vfreq[j - half]);
     const float c = cosf(angle), sn = sinf(angle);
-    if (key) turn_s[i] = make_float2(c * a.amplitude, sn * a.amplitude);
+    if (key) turn_s[w][j] = make_float2(c * a.amplitude, sn * a.amplitude);
     else {
-      vturn_s[i - half] = make_float2(c, sn);
-      if (a.turns) a.turns[(size_t)t * vhalf + i - half] = make_float2(c, sn);
+      vturn_s[w][j - half] = make_float2(c, sn);
+      if (a.turns) a.turns[(size_t)(t0 + w) * vhalf + j - half] = make_float2(c, sn);
     }
   }
   __syncthreads();
@@ -1264,8 +1289,8 @@ TIB_API int tib_rotary_kv_append(const void* proj, int64_t ld, int q_off, int k_
     if (n_tokens > 2 * 148 && dim % 16 == 0 && vdim % 16 == 0 && rot_dim % 16 == 0 && vhalf % 8 == 0 && ld % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 &&
         v_off % 8 == 0 && page_stride % 8 == 0 && (bits & 15) == 0) {
       const int pieces = ((heads + kv_heads) * dim + kv_heads * vdim) / 16;
-      TIB_LAUNCH_DEPENDENT(pwa_append_pieces_kernel, n_tokens, pieces >= 256 ? 256 : pieces <= 128 ? 128 : (pieces + 31) / 32 * 32, 0, stream,
-                           (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a);
+      TIB_LAUNCH_DEPENDENT(pwa_append_pieces_kernel, ceil_div(n_tokens, kPwaPair), pieces >= 256 ? 256 : pieces <= 128 ? 128 : (pieces + 31) / 32 * 32, 0, stream,
+                           (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a, n_tokens);
       return TIB_OK;
     }
     // few tokens: a thread for every two elements, so that a token is one round of loads and not five or six one after the other
