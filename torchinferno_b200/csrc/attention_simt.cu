@@ -18,9 +18,11 @@
 
 namespace tib {
 
-// What bounds it: loads from shared memory.  A warp works on its rows together, so that a key's four numbers, read at once, serve all of them, and a
-// value's, and the next block's keys and values are on their way meanwhile.  Row by row and number by number, two loads a multiply-add, two portions
-// of 200 and 101 tokens, 32 / 8 heads of 64, took 117 us, 45 now; a block of 1,536 on 12 single tokens at 300, 32 heads of 128: 415 and 213.
+// What bounds it: chains of loads and shuffles with four blocks of 16 rows an SM (128 registers a thread).  A warp works on its rows together, so
+// that a key's four numbers, read at once, serve all of them, and a value's, the next block's keys and values are on their way meanwhile, and the
+// rows' maxima and sums cross the lanes side by side.  Row by row and number by number, two loads a multiply-add, two portions of 200 and 101
+// tokens, 32 / 8 heads of 64, took 117 us, 37 now (44 with one row's maximum and sum after the other's and divisions for every piece's place);
+// 12 single tokens at 300, 32 heads of 128: 40 (55).  Five blocks an SM, at 96 registers: 45 and 58.
 constexpr int kAttnWarps = 4;
 constexpr int kAttnKeys = 32;                              // keys per step = lanes
 
@@ -60,6 +62,8 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ pool,
   float* v_s = k_s + kAttnKeys * kd;           // [32][d]
   float* p_s = v_s + kAttnKeys * d;            // [ROWS][32]: a row's weights
 
+  pdl_wait();
+  pdl_trigger();
   const int entry = blockIdx.y;
   const int group = a.heads / a.kv_heads;
   const int chunks = (group + a.group_chunk - 1) / a.group_chunk;
@@ -106,25 +110,29 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ pool,
 
   // Keys and values of block b.  Keys past last_pos are not yet written (or belong to nobody): they are filled with zeros and
   // always masked.
-  auto row_of = [&](int b, int e, int& j, int& dd) -> const T* {
-    j = e / pieces;
-    dd = (e - j * pieces) * W;
+  const int shift = (a.page_size & (a.page_size - 1)) == 0 ? 31 - __clz(a.page_size) : -1;      // (a division is 20 instructions)
+  auto row_of = [&](int b, int j, int dd) -> const T* {
     const int kp = b * kAttnKeys + j;
     if (kp > last_pos || kp < first_key) return nullptr;
-    const int page = table[kp / a.page_size];
-    if (page >= 0 && page < a.num_pages) return pool + (size_t)page * a.page_stride + ((size_t)kvh * a.page_size + (kp % a.page_size)) * d + dd;
+    const int at = shift >= 0 ? kp >> shift : kp / a.page_size, page = table[at];
+    if (page >= 0 && page < a.num_pages) return pool + (size_t)page * a.page_stride + ((size_t)kvh * a.page_size + (kp - at * a.page_size)) * d + dd;
     if (a.error_word) atomicExch(a.error_word, 0x10000 + entry);
     return nullptr;
   };
   const size_t values = (size_t)a.kv_heads * a.page_size * d;
   constexpr int AHEAD = VEC ? 2 * DPL : 1;              // pieces a thread holds: the next block's are on their way under this one's work
   float4 k_next[AHEAD], v_next[AHEAD];
+  int own_j[AHEAD], own_dd[AHEAD];                      // the thread's pieces of every block
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i) {
+    const int e = threadIdx.x + i * kAttnWarps * 32;
+    own_j[i] = e / pieces;
+    own_dd[i] = (e - own_j[i] * pieces) * W;
+  }
   auto ask = [&](int b) {
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
-      const int e = threadIdx.x + i * kAttnWarps * 32;
-      int j, dd;
-      const T* from = e < kAttnKeys * pieces ? row_of(b, e, j, dd) : nullptr;
+      const T* from = own_j[i] < kAttnKeys ? row_of(b, own_j[i], own_dd[i]) : nullptr;
       k_next[i] = v_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (from) {
         k_next[i] = attn_load4(from);
@@ -138,16 +146,15 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ pool,
     if constexpr (VEC) {
 #pragma unroll
       for (int i = 0; i < AHEAD; ++i) {
-        const int e = threadIdx.x + i * kAttnWarps * 32, j = e / pieces, dd = (e - j * pieces) * W;
-        if (e >= kAttnKeys * pieces) break;
-        *reinterpret_cast<float4*>(k_s + j * kd + dd) = k_next[i];
-        *reinterpret_cast<float4*>(v_s + j * d + dd) = v_next[i];
+        if (own_j[i] >= kAttnKeys) break;
+        *reinterpret_cast<float4*>(k_s + own_j[i] * kd + own_dd[i]) = k_next[i];
+        *reinterpret_cast<float4*>(v_s + own_j[i] * d + own_dd[i]) = v_next[i];
       }
       if (b < b_hi) ask(b + 1);
     } else {
       for (int e = threadIdx.x; e < kAttnKeys * pieces; e += blockDim.x) {
-        int j, dd;
-        const T* from = row_of(b, e, j, dd);
+        const int j = e / pieces, dd = (e - j * pieces) * W;
+        const T* from = row_of(b, j, dd);
         k_s[j * kd + dd] = from ? to_f32(*from) : 0.f;
         v_s[j * d + dd] = from ? to_f32(from[values]) : 0.f;
       }
@@ -162,7 +169,7 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ pool,
     const float* qr = q_s + warp * R * d;
     const float* kr = k_s + lane * kd;
     if constexpr (VEC) {
-#pragma unroll 2
+#pragma unroll 4
       for (int dd = 0; dd < d; dd += 4) {
         const float4 kv = *reinterpret_cast<const float4*>(kr + dd);
 #pragma unroll
@@ -179,25 +186,42 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ pool,
         for (int i = 0; i < R; ++i) s[i] = fmaf(qr[i * d + dd], kv, s[i]);
       }
     }
-    bool live[R];                                     // the block holds a key the row may read
+    // The rows' softmax side by side, so that their chains of shuffles run together; a row that may read no key of the block keeps what it has.
+    bool live[R], allowed[R];
+    float top[R], p[R], sum[R];
     float* pw = p_s + warp * R * kAttnKeys;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const int r = warp * R + i, qpos = pos0 + r / gc;
+      const int r = warp * R + i, qpos = pos0 + r / gc, kp = b * kAttnKeys + lane;
       const int lo = a.window > 0 ? max(0, qpos - a.window + 1) : 0;
       live[i] = r < nrows && b * kAttnKeys <= qpos && b * kAttnKeys + kAttnKeys - 1 >= lo;
-      if (!live[i]) continue;                         // uniform in the warp
-      const int kp = b * kAttnKeys + lane;
-      const bool allowed = kp <= qpos && kp >= lo;
-      const float score = allowed ? s[i] * a.scale : -CUDART_INF_F;
-      const float m_new = fmaxf(m[i], warp_max(score));   // finite: the block holds an allowed key
-      const float alpha = m[i] == -CUDART_INF_F ? 0.f : expf(m[i] - m_new);
-      const float p = allowed ? expf(score - m_new) : 0.f;
-      l[i] = l[i] * alpha + warp_sum(p);
-      m[i] = m_new;
+      allowed[i] = kp <= qpos && kp >= lo;
+      s[i] = allowed[i] ? s[i] * a.scale : -CUDART_INF_F;
+      top[i] = s[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < R; ++i) top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], o));
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      top[i] = fmaxf(m[i], top[i]);                   // (finite where the row is live: the block holds an allowed key)
+      p[i] = allowed[i] ? expf(s[i] - top[i]) : 0.f;
+      sum[i] = p[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < R; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (!live[i]) continue;                         // (uniform in the warp)
+      const float alpha = m[i] == -CUDART_INF_F ? 0.f : expf(m[i] - top[i]);
+      l[i] = l[i] * alpha + sum[i];
+      m[i] = top[i];
 #pragma unroll
       for (int j = 0; j < DPL; ++j) acc[i][j] *= alpha;
-      pw[i * kAttnKeys + lane] = p;
+      pw[i * kAttnKeys + lane] = p[i];
     }
     __syncwarp();
 #pragma unroll 2
@@ -254,8 +278,7 @@ static int launch_attention_rows(const void* q, const void* pool, void* out, Att
     if (e != cudaSuccess) return (int)e;
   }
   dim3 grid(ceil_div(max_q_len, a.q_tile), n_entries, a.kv_heads * chunks);
-  kern<<<grid, kAttnWarps * 32, smem, stream>>>((const T*)q, (const T*)pool, (T*)out, a);
-  TIB_LAUNCH_CHECK();
+  TIB_LAUNCH_DEPENDENT(kern, grid, kAttnWarps * 32, smem, stream, (const T*)q, (const T*)pool, (T*)out, a);
   return TIB_OK;
 }
 
