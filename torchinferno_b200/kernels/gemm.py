@@ -325,7 +325,7 @@ def tune_few_rows() -> dict[tuple, tuple[int, int, int]]:
         groups.setdefault((w.out_features, w.in_features, w.tensor.device, w.epilogue), []).append(w)
     _undecided.clear()
     if groups:
-        ops.lib()                 # (loads, and at the first call builds, the library the decisions are kept beside)
+        ops.load_library()        # (and at the first call builds: the decisions are kept beside it)
     try:
         for key, group in groups.items():
             if key not in _tuned:
