@@ -225,13 +225,11 @@ TUNE_ROWS = ((1, 4), (8, 8), (16, 16), (32, 32), (64, 64))      # (rows measured
 # So parity in the walk is a gain in the layer, and the line is drawn a little above it; what is decided is kept
 # (see _stored_choices): the kernels a checkpoint runs on a GPU model do not change from one process to the next.
 TUNE_MARGIN = 1.04
-# The few-rows kernel with the activation in its epilogue may take this much up to 8 and 16 rows: it applies it to the fp32 sums, where the
-# library's product is rounded to bfloat16 first (blocks' errors against 64 bits 0.0017 or 0.0018, and 0.0022 or 0.0023 so, for 1 or 2 us in 50
-# at few rows; at 12 rows of 4,096 x 3,008 it would be 6 in 44).
-TUNE_MARGIN_SWIGLU = {1: 2.0, 8: 2.0, 16: 1.25}
 TUNE_MEMBERS = 32
 # A walk is at least this many products long, over a few weights again and again: two events are 2 us apart in steps of 2, and of a
-# single product the pick would be chance (a layer of latent attention on 8 tokens took 47 to 53 us by what was picked).
+# single product the pick would be chance (a layer of latent attention on 8 tokens took 47 to 53 us by what was picked).  Weights with the
+# SwiGLU epilogue are walked once, from memory: again and again from the L2 they look better with the library, whose product is rounded to
+# bfloat16 before the activation (blocks' errors against 64 bits 0.0022 and 0.0023 for 0.0017 and 0.0018).
 TUNE_PRODUCTS = 32
 _flush: dict[torch.device, torch.Tensor] = {}     # larger than the L2; made once per tuning pass
 
@@ -255,7 +253,7 @@ def _choice_key(n: int, k: int, device: torch.device, members: int, epilogue: st
     mark = stamp.read_text().strip()[:16] if stamp.is_file() else "?"
     measured = min(members, TUNE_MEMBERS)
     where = "from memory" if measured * n * k * 2 > (256 << 20) else f"{measured} weights"
-    return f"{torch.cuda.get_device_name(device)}|{mark}|margins {TUNE_MARGIN} {sorted(TUNE_MARGIN_SWIGLU.values())}|{n}x{k}|{epilogue}|{where}"
+    return f"{torch.cuda.get_device_name(device)}|{mark}|margin {TUNE_MARGIN}|{n}x{k}|{epilogue}|{where}"
 
 
 def _stored_choices() -> dict[str, list[int]]:
@@ -346,8 +344,7 @@ def tune_few_rows() -> dict[tuple, tuple[int, int, int]]:
                         for rows, stands_for in TUNE_ROWS:      # (rising: the first row count at which the library wins ends it)
                             times = {"few_rows": _walk_time(members, rows, best, epilogue), "library": _walk_time(members, rows, None, epilogue)}
                             tuning_times[(n, k, device, epilogue, rows)] = times
-                            margin = TUNE_MARGIN_SWIGLU.get(rows, TUNE_MARGIN) if epilogue == "swiglu" else TUNE_MARGIN
-                            if not times["few_rows"] <= margin * times["library"]:
+                            if not times["few_rows"] <= TUNE_MARGIN * times["library"]:
                                 break
                             rows_taken = stands_for
                         _tuned[key] = (min(rows_taken, LinearWeight.FEW_ROWS), *best)
@@ -391,7 +388,7 @@ def _walk_time(group: "list[LinearWeight]", rows: int, config: tuple[int, int] |
             else:
                 ops.gemm_decode(x, w.tensor, out, features=config[0], splits=config[1])
 
-        rounds = -(-TUNE_PRODUCTS // len(group))
+        rounds = 1 if epilogue == "swiglu" else -(-TUNE_PRODUCTS // len(group))
 
         def walk() -> None:
             for w in group * rounds:
