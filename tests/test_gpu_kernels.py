@@ -1963,3 +1963,33 @@ def test_fp32_product_in_parts_of_k_has_one_order(n, k, many):
     assert torch.equal(whole, out[:130]) and int(launches) == 2
     exact = x[:130].double() @ w.double().T
     assert (whole.double() - exact).norm() <= 4e-7 * exact.norm()          # (the bound of the products in one part)
+
+
+@pytest.mark.parametrize("lens", [[129, 641], [512, 100, 513]])      # (chunks of a request: fewer than four, four, and one more)
+def test_scan_of_many_states_folds_each_request_as_alone(lens):
+    """Where states are enough for five blocks an SM a thread has four chunks on their way instead of eight: the same chain, to the bit."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, head_dim, state, n = 64, 64, 128, sum(lens)
+    blocks = heads * head_dim * state // 1024
+    assert blocks * len(lens) >= 5 * 148 > blocks
+    inner = heads * head_dim
+    xbc, dt = dev(rnd(n, inner + 2 * state, dtype=torch.bfloat16)), dev(rnd(n, heads, dtype=torch.bfloat16, seed=1))
+    bias, a_log, skip = dev(rnd(heads, seed=2)), dev(0.2 * rnd(heads, seed=3)), dev(rnd(heads, seed=4))
+    held = rnd(len(lens), heads * state * head_dim, seed=5)
+
+    def scan(first, lens, held):
+        rows = slice(first, first + sum(lens))
+        y, carried = torch.empty(sum(lens), inner, device="cuda"), dev(held.clone())
+        starts = dev(torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32))
+        ops.ssd_scan(xbc[rows], dt[rows], 0, bias, a_log, skip, carried, starts, dev(torch.arange(len(lens), dtype=torch.int32)), y, len(lens),
+                     heads=heads, groups=1, state_dim=state, head_dim=head_dim, max_q_len=max(lens))
+        return y, carried
+
+    y, carried = scan(0, lens, held)
+    for i, length in enumerate(lens):
+        if length <= 128:      # (alone it would not go in chunks)
+            continue
+        first = sum(lens[:i])
+        own, own_state = scan(first, [length], held[i:i + 1])
+        assert torch.equal(own, y[first:first + length]) and torch.equal(own_state, carried[i:i + 1])

@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_sums_kernel(ScanArgs a) {
 }
 
 // grid (state elements / 1024, entries), four elements a thread: run_state turns from a chunk's sum into the state at its start.
+template <int AHEAD>      // chunks whose sums a thread has on their way
 __global__ void __launch_bounds__(256) ssd_fold_kernel(ScanArgs a) {
   pdl_wait();
   pdl_trigger();
@@ -184,7 +185,6 @@ __global__ void __launch_bounds__(256) ssd_fold_kernel(ScanArgs a) {
   const float* decays = a.run_decay + run0 * a.heads + h;
   float4* slot = reinterpret_cast<float4*>(a.state + (size_t)a.slots[entry] * a.state_stride + e);
   float4 s = *slot;
-  constexpr int AHEAD = 8;
   for (int r = 0; r < runs; r += AHEAD) {
     float4 sum[AHEAD];
     float decay[AHEAD];
@@ -391,7 +391,12 @@ __global__ void __launch_bounds__(kSsdThreads, 2) ssd_outs_kernel(ScanArgs a) {
 }
 
 int ssd_fold(const ScanArgs& a, int n_entries, cudaStream_t stream) {
-  TIB_LAUNCH_DEPENDENT(ssd_fold_kernel, dim3((unsigned)ceil_div64((int64_t)a.heads * a.N * a.P, 1024), n_entries), 256, 0, stream, a);
+  const dim3 grid((unsigned)ceil_div64((int64_t)a.heads * a.N * a.P, 1024), n_entries);
+  // Four chunks' sums on their way a thread where there are five blocks an SM and more, which fill the memory with fewer registers a thread, else eight
+  // (layers on 600 to 2,600 tokens, us with four and eight: 192 blocks 148 and 142, 512 103 and 102, 640 108 and 108, 1,024 174 and 177, 1,536 174
+  // and 179, 2,560 303 and 311; two prompts of 1,366 and 682 tokens, 64 heads of 64: the fold 14.5 -> 11.4 behind the sums, with twelve 17, with two 19).
+  if ((int64_t)grid.x * grid.y >= 5 * 148) TIB_LAUNCH_DEPENDENT(ssd_fold_kernel<4>, grid, 256, 0, stream, a);
+  else TIB_LAUNCH_DEPENDENT(ssd_fold_kernel<8>, grid, 256, 0, stream, a);
   return TIB_OK;
 }
 
