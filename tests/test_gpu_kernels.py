@@ -1865,7 +1865,8 @@ def test_sums_of_two_outputs(rows, width, wide, dtypes, shift):
     (1, 1, 8, 8, 8, 4, False, True), (3, 2, 64, 520, 16, 5, False, False), (5, 3, 16, 1032, 24, 8, True, True), (2, 16, 128, 512, 64, 32, True, False),
     (296, 2, 8, 72, 16, 8, True, False), (297, 3, 8, 264, 16, 8, True, True), (301, 5, 24, 512, 64, 32, False, True), (299, 2, 16, 264, 8, 0, False, False)])
 def test_latent_rows_in_pieces_are_those_element_by_element(tokens, heads, dim, rank, rot, n_freq, half_pairs, in_place):
-    """Rotated parts to the bit; the latent within a bf16 rounding, since the sum of squares is added in another order."""
+    """To the bit, whichever kernel stores a row: the sum of squares is added in one order.  Without a cache nothing is stored; a token whose page is
+    out of range is reported, and its neighbours are stored."""
     need_gpu()
     from torchinferno_b200.kernels import ops
     page, width, slots = 16, rank + rot, 3
@@ -1876,22 +1877,27 @@ def test_latent_rows_in_pieces_are_those_element_by_element(tokens, heads, dim, 
     token_slot = dev(torch.tensor([t % slots for t in range(tokens)], dtype=torch.int32))
     dkv_rows, q_rows = rnd(tokens, width, dtype=torch.bfloat16), rnd(tokens, heads * (dim + rot), dtype=torch.bfloat16, seed=1)
     weight, freq = dev(1 + 0.1 * rnd(rank, seed=2)), dev(rnd(n_freq, seed=3).abs())
+    bad = table.clone()
+    bad[tokens % slots, 0] = 1 << 20      # (the first page of one slot)
+    last = int(table.max()) + 1
     results = []
     for shift in (8, 7):      # (rows off their 16-byte boundaries are taken element by element)
         dkv = dev(torch.zeros(tokens, width + 8, dtype=torch.bfloat16))
         dkv[:, shift:shift + width] = dev(dkv_rows)
-        q = dev(q_rows.clone())
-        keys = torch.full((int(table.max()) + 1, 1, page, width), -7.0, dtype=torch.bfloat16, device="cuda")
-        folded = None if in_place else torch.full((tokens, heads, width), -7.0, device="cuda")
-        ops.latent_append(dkv[:, shift:shift + width], q, folded, keys, positions, token_slot, table, weight, 1e-6, freq, heads, dim, rank, rot,
-                          half_pairs=half_pairs)
-        results.append((keys, q, folded))
-    (keys, q, folded), (want_keys, want_q, want_folded) = results
-    assert torch.equal(q, want_q) and (in_place or torch.equal(folded, want_folded))
-    assert torch.equal(keys[..., rank:], want_keys[..., rank:])
-    got, want = keys[..., :rank].double(), want_keys[..., :rank].double()
-    assert ((got - want).abs() <= 2.0 ** -7 * want.abs()).all()      # (a rounding to the neighbouring bf16 number: at most 2^-7 of the value)
-    assert (got != want).double().mean() < 0.01
+        for pages in (table, bad, None):
+            q = dev(q_rows.clone())
+            keys = None if pages is None else torch.full((last, 1, page, width), -7.0, dtype=torch.bfloat16, device="cuda")
+            folded = None if in_place else torch.full((tokens, heads, width), -7.0, device="cuda")
+            error = torch.zeros(1, dtype=torch.int32, device="cuda")
+            ops.latent_append(dkv[:, shift:shift + width], q, folded, keys, positions, token_slot, pages, weight, 1e-6, freq, heads, dim, rank, rot,
+                              half_pairs=half_pairs, error_word=error)
+            results.append((keys, q, folded))
+            assert (int(error) >> 16 == 2) == (pages is bad and bool((token_slot == tokens % slots).any()))
+    for got, want in zip(results[:3], results[3:]):
+        for x, y in zip(got, want):
+            assert (x is None and y is None) or torch.equal(x, y)
+    for cached in results[1:3]:      # (the queries do not depend on the cache)
+        assert torch.equal(cached[1], results[0][1]) and (in_place or torch.equal(cached[2], results[0][2]))
 
 
 @pytest.mark.parametrize("tokens, rows, k", [(2859, 7, 260), (1187, 37, 64), (331, 61, 1028), (157, 129, 2056)])

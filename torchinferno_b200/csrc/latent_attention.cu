@@ -134,16 +134,32 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, T* __restrict__ 
   }
 }
 
+// The latent's sum of squares in the order of the kernel above with THREADS threads (its thread t adds elements t, t + THREADS, ..., then come the sums
+// over lanes and over warps), so that a row's bits do not depend on which kernel stores it.  Eight of those threads are one holder's here, whose pieces are
+// p, p + THREADS / 8, ... and make the terms of one element each: of a warp's tree the steps 16 and 8 lanes apart run between four neighbouring holders, the others
+// in registers.  v: a holder's eight sums; returns the sum of the warp that it and its three neighbours stand for.
+__device__ __forceinline__ float squares_of_a_warp(float (&v)[8]) {
+#pragma unroll
+  for (int step = 2; step > 0; step /= 2)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] += __shfl_xor_sync(0xffffffffu, v[e], step);
+#pragma unroll
+  for (int step = 4; step > 0; step /= 2)
+#pragma unroll
+    for (int e = 0; e < step; ++e) v[e] += v[e + step];
+  return v[0];
+}
+
 // The same for bf16 rows on 16-byte boundaries, eight elements a load and store.  A token is one warp's (WARPS 1: four tokens a block, no barrier of
-// the block but the table's) or, in small steps, a block's, and a thread asks for its next pieces before it works on the last.  The sum of squares adds
-// eight neighbours a thread.  What bounds it is one trip to memory behind the page's lookup: 2,500 tokens of 16 heads, 512 + 64 numbers, in place
+// the block but the table's) or, in small steps, a block's, and a thread asks for its next pieces before it works on the last.  Same bits.
+// What bounds it is one trip to memory behind the page's lookup: 2,500 tokens of 16 heads, 512 + 64 numbers, in place
 // 7.2 us where the kernel above takes 16.4 (in the running layer); eight tokens 3.3 behind the product before, 4.3 above.
 template <int WARPS>
 __global__ void __launch_bounds__(128)
 latent_append_pieces_kernel(const __nv_bfloat16* __restrict__ dkv, __nv_bfloat16* q, __nv_bfloat16* __restrict__ pool,
                             float* __restrict__ folded, LatentAppendArgs a, int n_tokens) {
   constexpr int TOKENS = 4 / WARPS, THREADS = 32 * WARPS;
-  __shared__ float scratch[33];
+  __shared__ float scratch[16];
   __shared__ float cos_s[TOKENS][kAppendFreq / TOKENS], sin_s[TOKENS][kAppendFreq / TOKENS];
   const int own = WARPS == 1 ? threadIdx.x >> 5 : 0, tid = WARPS == 1 ? threadIdx.x & 31 : threadIdx.x;
   pdl_wait();
@@ -180,19 +196,40 @@ latent_append_pieces_kernel(const __nv_bfloat16* __restrict__ dkv, __nv_bfloat16
   };
   const auto narrow = [](const float (&v)[8]) { return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7])); };
   const auto piece = [&](int p) { return p == tid ? first : p == tid + THREADS ? second : *reinterpret_cast<const uint4*>(src + p * 8); };
-  float ss = 0.f;
-  if (live)
-    for (int p = tid; p < rank8; p += THREADS) {
-      float v[8];
-      widen(piece(p), v);
+  float ss;
+  {
+    float v[8], x[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+    for (int e = 0; e < 8; ++e) v[e] = 0.f;
+    const auto square = [&](const uint4& raw) {
+      widen(raw, x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = fmaf(x[e], x[e], v[e]);
+    };
+    if (WARPS == 1) {      // (128 threads there: 16 holders, the lower half of the warp, which takes its own piece and the upper half's in turn)
+      for (int p0 = 0; p0 < rank8; p0 += THREADS) {      // (uniform: rank8 is)
+        const uint4 raw = live && p0 + tid < rank8 ? piece(p0 + tid) : make_uint4(0u, 0u, 0u, 0u);
+        square(raw);
+        square(make_uint4(__shfl_down_sync(0xffffffffu, raw.x, 16), __shfl_down_sync(0xffffffffu, raw.y, 16), __shfl_down_sync(0xffffffffu, raw.z, 16),
+                          __shfl_down_sync(0xffffffffu, raw.w, 16)));
+      }
+      float warp = squares_of_a_warp(v);      // (of four: lanes 0, 4, 8 and 12 hold them)
+      warp += __shfl_xor_sync(0xffffffffu, warp, 8);
+      warp += __shfl_xor_sync(0xffffffffu, warp, 4);
+      ss = __shfl_sync(0xffffffffu, warp, 0);
+      __syncwarp();      // (the table is the warp's own)
+    } else {               // (512 threads there: 64 holders, the block's first two warps)
+      if (tid < 64) {
+        for (int p = tid; p < rank8; p += 64) square(piece(p));
+        const float warp = squares_of_a_warp(v);
+        if ((tid & 3) == 0) scratch[tid >> 2] = warp;
+      }
+      __syncthreads();      // (the table too)
+      float warp = scratch[tid & 15];
+#pragma unroll
+      for (int step = 8; step > 0; step /= 2) warp += __shfl_xor_sync(0xffffffffu, warp, step);
+      ss = warp;
     }
-  if (WARPS == 1) {
-    ss = warp_sum(ss);
-    __syncwarp();      // (the table is the warp's own)
-  } else {
-    ss = block_sum(ss, scratch);      // (its barriers publish the table too)
   }
   if (!live) return;
   const float inv = 1.f / sqrtf(ss / (float)a.rank + a.eps);
