@@ -5,6 +5,7 @@ from ctypes import c_char_p, c_int, c_int64, c_void_p
 from pathlib import Path
 
 import pytest
+import torch
 
 import torchinferno_b200
 
@@ -42,6 +43,42 @@ def test_packed_calls_pass_their_arguments():
     assert library.tib_embedding(0, 0, 0, 1, 8, 8, 0.5, 0, 0, 0, 0, 0) == -5                              # (a refusal comes back as it is)
     with pytest.raises(struct.error):
         library.tib_plan_product(1, 2, 3)
+
+
+@pytest.mark.parametrize("members, size, products, distinct", [
+    (1, 4, 32, 32), (1, 64, 32, 16), (3, 64, 32, 16), (16, 64, 32, 16), (20, 64, 32, 20), (1, 1000, 5, 2), (1, 1024, 4, 1), (2, 8192, 2, 2), (40, 4, 40, 40)])
+def test_a_measured_walk_reads_every_weight_from_memory(members, size, products, distinct, monkeypatch):
+    """Members first, copies of them behind; none is read again before TUNE_COLD bytes of them were read, or at all; the copies are smaller than that together."""
+    from torchinferno_b200.kernels import gemm
+    monkeypatch.setattr(gemm, "TUNE_COLD", 1024)
+    monkeypatch.setattr(gemm, "TUNE_BYTES", 4096)
+    own = [torch.full((size // 2, 1), float(i), dtype=torch.bfloat16) for i in range(members)]
+    walk = gemm._walk_weights(own)
+    places = [w.data_ptr() for w in walk]
+    assert len(walk) == products and len(set(places)) == distinct and places[:members] == [w.data_ptr() for w in own]
+    assert all(torch.equal(w, own[i % distinct % members]) for i, w in enumerate(walk))
+    assert all(p not in places[i + 1:i + distinct] for i, p in enumerate(places))
+    assert (distinct == products or distinct * size >= 1024) and (distinct - members) * size < 1024
+
+
+def test_a_stored_choice_names_how_it_was_measured(monkeypatch):
+    from torchinferno_b200.kernels import gemm
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda device: "a GPU")
+    keys = [gemm._choice_key(2048, 1024, torch.device("cuda", 0), epilogue) for epilogue in ("none", "swiglu")]
+    for name in ("TUNE_PRODUCTS", "TUNE_BYTES", "TUNE_COLD", "TUNE_MARGIN", "TUNE_SWIGLU_US"):
+        with monkeypatch.context() as patch:
+            patch.setattr(gemm, name, 2 * getattr(gemm, name))
+            keys.append(gemm._choice_key(2048, 1024, torch.device("cuda", 0), "none"))
+    assert len(set(keys)) == 7
+
+
+@pytest.mark.parametrize("few_rows, library, none, swiglu", [
+    (10.0, 10.0, True, True), (10.4, 10.0, True, True), (10.5, 10.0, False, True), (12.0, 10.0, False, True), (12.1, 10.0, False, False),
+    (103.0, 100.0, True, True), (104.1, 100.0, False, False), (float("nan"), 10.0, False, False)])
+def test_the_line_between_the_few_rows_kernel_and_the_library(few_rows, library, none, swiglu):
+    """4 % for all weights; 2 us for those whose activation is then made of fp32 sums."""
+    from torchinferno_b200.kernels import gemm
+    assert (gemm._few_rows_wins(few_rows, library, "none"), gemm._few_rows_wins(few_rows, library, "swiglu")) == (none, swiglu)
 
 
 def test_a_timeout_code_names_one_kernel():

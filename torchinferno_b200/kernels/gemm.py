@@ -225,12 +225,19 @@ TUNE_ROWS = ((1, 4), (8, 8), (16, 16), (32, 32), (64, 64))      # (rows measured
 # So parity in the walk is a gain in the layer, and the line is drawn a little above it; what is decided is kept
 # (see _stored_choices): the kernels a checkpoint runs on a GPU model do not change from one process to the next.
 TUNE_MARGIN = 1.04
+# A product with the SwiGLU epilogue activates its fp32 sums, where the library's is rounded to bfloat16 first: blocks on few tokens have
+# errors of 0.0017 to 0.0018 against 64 bits with the one and 0.0021 to 0.0023 with the other.  For that it may take 2 us longer.  (At 8 rows, us,
+# fused / library: 6,400 x 1,536 10.4 / 9.2, 2,048 x 1,280 9.2 / 7.8; beyond the line 8,192 x 2,560 14.9 / 12.5, 2,048 x 3,072 16.4 / 10.5, a layer of
+# which takes 49 and 42.)
+TUNE_SWIGLU_US = 2.0
 TUNE_MEMBERS = 32
-# A walk is at least this many products long, over a few weights again and again: two events are 2 us apart in steps of 2, and of a
-# single product the pick would be chance (a layer of latent attention on 8 tokens took 47 to 53 us by what was picked).  Weights with the
-# SwiGLU epilogue are walked once, from memory: again and again from the L2 they look better with the library, whose product is rounded to
-# bfloat16 before the activation (blocks' errors against 64 bits 0.0022 and 0.0023 for 0.0017 and 0.0018).
+# A walk is at least TUNE_PRODUCTS products or TUNE_BYTES of weights long (150 us): two events are 2 us apart in steps of 2, and of a single
+# small product the pick would be chance.  Every weight in it comes from memory, as in a decode step, where the other layers' weights have
+# passed through the L2 since: a shape with few weights gets copies (less than TUNE_COLD bytes), which are walked once each or, where TUNE_COLD bytes
+# lie between two readings of one, in rotation.
 TUNE_PRODUCTS = 32
+TUNE_BYTES = 1 << 30
+TUNE_COLD = 256 << 20
 _flush: dict[torch.device, torch.Tensor] = {}     # larger than the L2; made once per tuning pass
 
 
@@ -243,17 +250,14 @@ def _choice_file():
     return None if path is None else Path(path).parent / "gemm_choice.json"
 
 
-def _choice_key(n: int, k: int, device: torch.device, members: int, epilogue: str) -> str:
-    """What a stored decision holds for: the GPU model, the build of the kernels, the line, the shape, and whether
-    the measured weights together exceed the L2 (a model of two layers is timed out of the L2, one of thirty-two
-    out of memory, and the two may well decide differently)."""
+def _choice_key(n: int, k: int, device: torch.device, epilogue: str) -> str:
+    """What a stored decision holds for: the GPU model, the build of the kernels, the line, the shape, and how it was
+    measured (see TUNE_PRODUCTS)."""
     from pathlib import Path
     from torchinferno_b200.kernels.library import library_path
     stamp = Path(library_path()).parent / "stamp.txt"
     mark = stamp.read_text().strip()[:16] if stamp.is_file() else "?"
-    measured = min(members, TUNE_MEMBERS)
-    where = "from memory" if measured * n * k * 2 > (256 << 20) else f"{measured} weights"
-    return f"{torch.cuda.get_device_name(device)}|{mark}|margin {TUNE_MARGIN}|{n}x{k}|{epilogue}|{where}"
+    return f"{torch.cuda.get_device_name(device)}|{mark}|margin {TUNE_MARGIN} {TUNE_SWIGLU_US}|{n}x{k}|{epilogue}|walk {TUNE_PRODUCTS} {TUNE_BYTES >> 20} {TUNE_COLD >> 20}"
 
 
 def _stored_choices() -> dict[str, list[int]]:
@@ -311,13 +315,13 @@ def tune_few_rows() -> dict[tuple, tuple[int, int, int]]:
     the decisions made so far by (out, in, device, epilogue).
 
     Under the "measured" choice, weights of one shape are measured together, once per shape and GPU model, the way
-    a decode step runs them: a CUDA graph walks over them (different weights one after the other, so nothing
-    comes from L2), each product behind a small kernel, as in a layer (under programmatic dependent launch the
+    a decode step runs them: a CUDA graph walks over them and over copies (so that every product's weight comes
+    from memory: _walk_weights), each product behind a small kernel, as in a layer (under programmatic dependent launch the
     few-rows kernel fetches its first weights while that kernel runs, and a measurement of the product alone
     would not show it).  First the kernel's own configurations are timed at 8 rows and the fastest is kept; then
     the graph is timed with either kernel at rising row counts, and the few-rows kernel gets the shape up to
-    the last count at which it takes less than TUNE_MARGIN of the library's time.  The outcome is stored and later
-    processes read it."""
+    the last count at which it takes less than TUNE_MARGIN of the library's time (or, with the SwiGLU epilogue, up to
+    TUNE_SWIGLU_US more than it).  The outcome is stored and later processes read it."""
     groups: dict[tuple, list[LinearWeight]] = {}
     for w in list(_undecided):
         groups.setdefault((w.out_features, w.in_features, w.tensor.device, w.epilogue), []).append(w)
@@ -333,20 +337,21 @@ def tune_few_rows() -> dict[tuple, tuple[int, int, int]]:
                     takes = _few_rows_choice == "swapab" and bool(configs)
                     _tuned[key] = (LinearWeight.FEW_ROWS, *configs[0]) if takes else (0, 128, 0)
                 else:
-                    name, stored = _choice_key(n, k, device, len(group), epilogue), _stored_choices()
+                    name, stored = _choice_key(n, k, device, epilogue), _stored_choices()
                     if name in stored and len(stored[name]) == 3:
                         _tuned[key] = tuple(stored[name])
                     else:
-                        members = group[:TUNE_MEMBERS]
+                        members = _walk_weights([w.tensor for w in group[:TUNE_MEMBERS]])
                         timed = {c: _walk_time(members, 8, c, epilogue) for c in configs}
                         best = min(timed, key=timed.get)
                         rows_taken = 0
                         for rows, stands_for in TUNE_ROWS:      # (rising: the first row count at which the library wins ends it)
                             times = {"few_rows": _walk_time(members, rows, best, epilogue), "library": _walk_time(members, rows, None, epilogue)}
                             tuning_times[(n, k, device, epilogue, rows)] = times
-                            if not times["few_rows"] <= TUNE_MARGIN * times["library"]:
+                            if not _few_rows_wins(times["few_rows"], times["library"], epilogue):
                                 break
                             rows_taken = stands_for
+                        del members      # (the copies: the next shape makes its own)
                         _tuned[key] = (min(rows_taken, LinearWeight.FEW_ROWS), *best)
                         _store_choice(name, _tuned[key])
             for w in group:
@@ -358,12 +363,26 @@ def tune_few_rows() -> dict[tuple, tuple[int, int, int]]:
     return dict(_tuned)
 
 
-def _walk_time(group: "list[LinearWeight]", rows: int, config: tuple[int, int] | None, epilogue: str) -> float:
-    """Microseconds per (small kernel + product) of a captured walk over ``group``'s weights with the few-rows
+def _few_rows_wins(few_rows: float, library: float, epilogue: str) -> bool:
+    return few_rows <= max(TUNE_MARGIN * library, library + (TUNE_SWIGLU_US if epilogue == "swiglu" else 0.0))
+
+
+def _walk_weights(members: list[torch.Tensor]) -> list[torch.Tensor]:
+    """The weights of a walk (see TUNE_PRODUCTS) in their order: the members, then copies of them, then, with TUNE_COLD bytes together,
+    the same again."""
+    size = members[0].numel() * members[0].element_size()
+    products = max(len(members), min(TUNE_PRODUCTS, -(-TUNE_BYTES // size)))
+    distinct = list(members)
+    while len(distinct) < products and len(distinct) * size < TUNE_COLD:
+        distinct.append(members[len(distinct) % len(members)].clone())
+    return (distinct * -(-products // len(distinct)))[:products]
+
+
+def _walk_time(weights: list[torch.Tensor], rows: int, config: tuple[int, int] | None, epilogue: str) -> float:
+    """Microseconds per (small kernel + product) of a captured walk over ``weights`` ([in, out], of one shape) with the few-rows
     kernel in ``config`` (tile width, K split), or with the library (None); with the SwiGLU epilogue the library's
     product is followed by the SwiGLU kernel, as it is in a layer."""
-    first = group[0]
-    n, k, device = first.out_features, first.in_features, first.tensor.device
+    (k, n), device = weights[0].shape, weights[0].device
     ops.library_gemm_ready(device)
     with torch.cuda.device(device):
         x = torch.zeros((rows, k), dtype=torch.bfloat16, device=device)
@@ -376,22 +395,20 @@ def _walk_time(group: "list[LinearWeight]", rows: int, config: tuple[int, int] |
         act = torch.empty((rows, n // 2), dtype=torch.bfloat16, device=device)
         flush = _flush.get(device)
         if flush is None:
-            flush = _flush[device] = torch.empty(256 << 20, dtype=torch.uint8, device=device)      # larger than the L2
+            flush = _flush[device] = torch.empty(TUNE_COLD, dtype=torch.uint8, device=device)
 
-        def product(w: LinearWeight) -> None:
+        def product(w: torch.Tensor) -> None:
             if config is None:
-                ops.library_gemm(x, w.tensor, out, w_kn=True)
+                ops.library_gemm(x, w, out, w_kn=True)
                 if epilogue == "swiglu":
                     ops.swiglu(out, act, interleaved=True)
             elif epilogue == "swiglu":
-                ops.gemm_decode(x, w.tensor, act, features=config[0], splits=config[1], epilogue=ops.DG_SWIGLU)
+                ops.gemm_decode(x, w, act, features=config[0], splits=config[1], epilogue=ops.DG_SWIGLU)
             else:
-                ops.gemm_decode(x, w.tensor, out, features=config[0], splits=config[1])
-
-        rounds = 1 if epilogue == "swiglu" else -(-TUNE_PRODUCTS // len(group))
+                ops.gemm_decode(x, w, out, features=config[0], splits=config[1])
 
         def walk() -> None:
-            for w in group * rounds:
+            for w in weights:
                 ops.add_rmsnorm(delta, residual, norm_weight, 1e-5, normed)
                 product(w)
         walk()                                                            # (first launches: attributes, handles)
@@ -412,7 +429,7 @@ def _walk_time(group: "list[LinearWeight]", rows: int, config: tuple[int, int] |
             if i >= 2:
                 best = min(best, begin.elapsed_time(end))
         del graph
-    return best * 1e3 / (len(group) * rounds)
+    return best * 1e3 / len(weights)
 
 
 def _linear_bf16(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
