@@ -193,6 +193,29 @@ def test_the_choice_of_a_shape_with_one_weight_is_measured_from_memory(epilogue,
     assert len(read) >= 64 and all(len(set(read[i:i + 32])) == 32 for i in range(len(read) - 31))
 
 
+@pytest.mark.parametrize("choice", ["measured", "swapab", "library"])
+def test_pairs_of_odd_eights_bind_and_run(choice):
+    """A SwiGLU weight whose outputs are no whole eights: the few-rows kernel does not take it with its epilogue."""
+    need_gpu()
+    from torchinferno_b200.kernels import gemm
+    n, k = 1096, 1088
+    w, x = rnd(n, k, dtype=torch.bfloat16, scale=0.05), rnd(8, k, dtype=torch.bfloat16, seed=1)
+    gemm.set_few_rows_choice(choice)
+    try:
+        weight = gemm.LinearWeight(dev(w), few_rows_tcgen05=None, epilogue="swiglu")
+        gemm._tuned.pop((n, k, weight.tensor.device, "swiglu"), None)
+        gemm.tune_few_rows()
+        got = as_ref(gemm.linear_swiglu(dev(x), weight))
+    finally:
+        gemm._tuned.pop((n, k, weight.tensor.device, "swiglu"), None)
+        gemm.set_few_rows_choice("measured")
+    both = x.double() @ w.double().T
+    gate, up = both[:, 0::2], both[:, 1::2]
+    want = gate * torch.sigmoid(gate) * up
+    # (gate, up and the result are rounded to bfloat16: 2^-9 each, times the slopes of the silu and the product, at most 1.1 and 1)
+    assert (got - want).norm() <= 4 * 2.0 ** -9 * want.norm()
+
+
 def test_few_rows_kernel_is_chosen_by_measurement_and_either_choice_is_right():
     """Weights that leave their few-rows kernel open get it from tune_few_rows (the hand-written kernel up to 0, 4, 8,
     16, 32 or 64 rows, with the tile width and K split that measured fastest): one decision per shape, kept for the

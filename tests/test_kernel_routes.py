@@ -45,6 +45,17 @@ def test_packed_calls_pass_their_arguments():
         library.tib_plan_product(1, 2, 3)
 
 
+@pytest.mark.parametrize("n, k", [(1096, 1088), (1104, 1088), (24584, 1024), (28672, 4096)])
+@pytest.mark.parametrize("epilogue", ["none", "swiglu"])
+def test_what_is_measured_is_what_the_kernel_takes(n, k, epilogue):
+    """Every tile width and K split that is timed is one the kernel takes with the weight's own epilogue (outputs of pairs in whole eights)."""
+    from torchinferno_b200.kernels import gemm, ops
+    code = ops.DG_SWIGLU if epilogue == "swiglu" else ops.DG_PLAIN
+    found = gemm._candidates(n, k, epilogue)
+    assert all(ops.gemm_decode_supports(8, n, k, *config, code) for config in found)
+    assert bool(found) == (epilogue == "none" or n % 16 == 0)
+
+
 @pytest.mark.parametrize("members, size, products, distinct", [
     (1, 4, 32, 32), (1, 64, 32, 16), (3, 64, 32, 16), (16, 64, 32, 16), (20, 64, 32, 20), (1, 1000, 5, 2), (1, 1024, 4, 1), (2, 8192, 2, 2), (40, 4, 40, 40)])
 def test_a_measured_walk_reads_every_weight_from_memory(members, size, products, distinct, monkeypatch):

@@ -294,14 +294,14 @@ def decisions() -> dict[tuple, tuple[int, int, int]]:
 def _candidates(n: int, k: int, epilogue: str) -> list[tuple[int, int]]:
     """(tile width, K split) worth timing for a [k, n] weight: 256 features a tile only where that still gives about
     a hundred blocks, splits that leave every block a few k slices and the grid neither tiny nor many rounds deep."""
-    out = []
-    if n >= 256 * 96 and ops.gemm_decode_supports(8, n, k, 256, 1, ops.DG_SWIGLU if epilogue == "swiglu" else ops.DG_PLAIN):
+    out, code = [], ops.DG_SWIGLU if epilogue == "swiglu" else ops.DG_PLAIN
+    if n >= 256 * 96 and ops.gemm_decode_supports(8, n, k, 256, 1, code):
         out.append((256, 1))
     tiles = -(-n // 128)
     for splits in range(1, 9):
         if epilogue == "swiglu" and splits > 1:
             break
-        if not ops.gemm_decode_supports(8, n, k, 128, splits, ops.DG_PLAIN) or k // 64 < 4 * splits:
+        if not ops.gemm_decode_supports(8, n, k, 128, splits, code) or k // 64 < 4 * splits:
             continue
         if splits > 1 and (tiles * splits < 64 or tiles * splits > 4 * 148):
             continue
@@ -334,8 +334,11 @@ def tune_few_rows() -> dict[tuple, tuple[int, int, int]]:
                 n, k, device, epilogue = key
                 configs = _candidates(n, k, epilogue) if group[0].transposed else []
                 if _few_rows_choice != "measured" or not configs:
-                    takes = _few_rows_choice == "swapab" and bool(configs)
-                    _tuned[key] = (LinearWeight.FEW_ROWS, *configs[0]) if takes else (0, 128, 0)
+                    if _few_rows_choice == "swapab" and group[0].transposed:      # (without its epilogue where that does not fit)
+                        configs = configs or _candidates(n, k, "none")
+                        _tuned[key] = (LinearWeight.FEW_ROWS, *configs[0]) if configs else (0, 128, 0)
+                    else:
+                        _tuned[key] = (0, 128, 0)
                 else:
                     name, stored = _choice_key(n, k, device, epilogue), _stored_choices()
                     if name in stored and len(stored[name]) == 3:
