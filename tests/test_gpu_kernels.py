@@ -1949,6 +1949,27 @@ def test_router_logits_of_six_rows_a_warp_have_the_bits_of_one(tokens, rows, k, 
     assert tokens * rows >= 20000 > 100 * rows and torch.equal(out, torch.cat(parts))
 
 
+# (two and four blocks on the fullest SM and bf16 rows, more than one and fp32 rows: the form with fewer registers; the last the form of large steps)
+@pytest.mark.parametrize("tokens, rows, dtype", [(501, 16, torch.bfloat16), (1180, 16, torch.bfloat16), (2049, 9, torch.bfloat16), (603, 9, torch.bfloat16),
+                                                 (1183, 16, torch.float32), (1301, 7, torch.float32), (1184, 9, torch.float32)])
+def test_router_logits_have_the_bits_of_a_few_tokens_alone(tokens, rows, dtype):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    x, w = dev(rnd(tokens, 1032, dtype=dtype)), dev(rnd(rows, 1032, seed=1))
+    out = ops.router_logits(x, w, torch.empty(tokens, rows, device="cuda"))
+    parts = [ops.router_logits(x[i:i + 100], w, torch.empty(len(x[i:i + 100]), rows, device="cuda")) for i in range(0, tokens, 100)]
+    assert tokens * rows < 20000 and torch.equal(out, torch.cat(parts))
+
+
+def test_router_logits_of_more_rows_than_a_grid_is_high():
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    x, w = dev(rnd(1, 4)), dev(rnd(36 * 65535 + 1, 4, seed=1))
+    out = ops.router_logits(x, w, torch.empty(1, len(w), device="cuda"))
+    want = x.double() @ w.double().T
+    assert (out.double() - want).abs().max() <= 4 * 2.0 ** -24 * (x.abs().double() @ w.abs().double().T).max()      # (four products, rounded as they are added)
+
+
 @pytest.mark.parametrize("experts, top", [(1, 1), (31, 4), (32, 32), (33, 3), (64, 6), (65, 8), (256, 8)])
 @pytest.mark.parametrize("sigmoid, normalize, corrected", [(False, True, False), (True, False, True)])
 def test_choices_of_few_experts_are_the_general_forms(experts, top, sigmoid, normalize, corrected):

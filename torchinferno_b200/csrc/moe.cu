@@ -43,7 +43,11 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
 }
 
-template <typename TX, bool VEC>
+// DENSE: fewer registers (bf16 rows 64 for 74, four blocks an SM for three; fp32 rows 50 for 60), by one clamp of an index, which has the compiler keep fewer
+// addresses and loads.  With one block an SM the more loads are ahead; beyond that it goes by how the blocks fall into rounds.  16 rows of 4,096, bf16, us,
+// dense and not, by blocks on the fullest SM: one 6.0 and 5.5 (200 tokens), two 6.6 and 8.5 (500), three 10.7 and 8.6 (600), four 10.9 and 15.9 (1,180); fp32
+// rows of 2,048, 16 of them: one 6.0 and 4.7, two 7.7 and 7.3, 24 of them 7.7 and 8.4, 12 of them 6.5 and 7.8, four 12.7 and 12.8.
+template <typename TX, bool VEC, bool DENSE>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ out, int64_t ldo, int tokens, int rows, int K) {
@@ -54,7 +58,7 @@ router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restr
   const int t0 = blockIdx.x * TOK;
   const int nt = min(TOK, tokens - t0);
   const int K8 = VEC ? (K / 8) * 8 : 0;
-  for (int e = warp + blockIdx.y * nwarps; e < rows; e += nwarps * gridDim.y) {
+  const auto work = [&](int e, int row) {
     float acc[TOK];
 #pragma unroll
     for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
@@ -63,7 +67,7 @@ router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restr
 #pragma unroll 4
       for (int k = lane * 8; k < K8; k += 256) {
         float wv[8];
-        load8(w + (size_t)e * K + k, wv);
+        load8(w + (size_t)row * K + k, wv);
 #pragma unroll
         for (int i = 0; i < TOK; ++i) {
           float xv[8];
@@ -84,6 +88,12 @@ router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restr
       const float v = warp_sum(acc[i]);
       if (lane == 0 && i < nt) out[(size_t)(t0 + i) * ldo + e] = bias ? v + bias[e] : v;
     }
+  };
+  if constexpr (DENSE) {
+    const int stride = nwarps * gridDim.y;
+    for (int e = warp + blockIdx.y * nwarps; e < rows; e += stride) work(e, min(e, rows - 1));
+  } else {
+    for (int e = warp + blockIdx.y * nwarps; e < rows; e += nwarps * gridDim.y) work(e, e);
   }
 }
 
@@ -673,8 +683,10 @@ TIB_API int tib_router_logits(const void* x, int x_dtype, int64_t ldx, const flo
   const bool vec = K % 4 == 0 && (ldx * xbytes) % 16 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
   // The kernel of large steps from 20,000 logits on: below, a warp a row and four tokens fill the GPU better (33 rows: 400 tokens 8.7 us against 11.5,
   // 800 13.9 against 12.3; 61: 400 tokens 9.9 and 10.3; 129: 100 8.8 and 11.6, 200 13.8 and 12.3).
-  if (vec && (int64_t)tokens * rows >= 20000) {
-    const int passes = ceil_div(rows, kRouterWarps * kRouterRows), warps = ceil_div(rows, kRouterRows * passes);
+  // fp32 tokens in their thousands from 10,400 on (2,048 wide, 12 rows, 1,300 tokens 11.1 against 18.5; 4 rows, 3,000 10.6 and 12.4; 6 rows, 1,300 10.6 and 9.8).
+  const int passes = ceil_div(rows, kRouterWarps * kRouterRows);      // (of a grid's second dimension)
+  if (vec && (int64_t)tokens * rows >= (x_dtype == TIB_F32 && tokens >= 1184 ? 10400 : 20000) && passes <= 65535) {
+    const int warps = ceil_div(rows, kRouterRows * passes);
     const dim3 grid(ceil_div(tokens, kRouterMany), passes);
     if (x_dtype == TIB_F32)
       TIB_LAUNCH_DEPENDENT(router_logits_many_kernel<float>, grid, warps * 32, 0, stream, (const float*)x, ldx, w, bias, out, ldo, tokens, rows, K);
@@ -689,11 +701,17 @@ TIB_API int tib_router_logits(const void* x, int x_dtype, int64_t ldx, const flo
   const int groups = ceil_div(tokens, kRouterTokens);
   while (groups * slices < 2 * 148 && slices * 8 < rows) slices *= 2;
   const dim3 grid(groups, slices);
-#define TIB_ROUTER_GO(TX, VEC) \
-  TIB_LAUNCH_DEPENDENT((router_logits_kernel<TX, VEC>), grid, 256, 0, stream, (const TX*)x, ldx, w, bias, out, ldo, tokens, rows, K)
+  // Blocks an SM, of which a slice's last one may be half empty: which form is ahead depends on how they fall into rounds (see DENSE).
+  const int first_rows = rows < 8 * slices ? rows : 8 * slices;
+  const int most = ceil_div64((int64_t)groups * ceil_div(first_rows, 8), 148), least = ceil_div64((int64_t)groups * ceil_div(first_rows, 4), 2 * 148);
+  const bool dense = vec && (x_dtype == TIB_F32 ? most > 1 : most % 2 == 0 || least % 2 == 0);
+#define TIB_ROUTER_D(TX, VEC, DENSE) \
+  TIB_LAUNCH_DEPENDENT((router_logits_kernel<TX, VEC, DENSE>), grid, 256, 0, stream, (const TX*)x, ldx, w, bias, out, ldo, tokens, rows, K)
+#define TIB_ROUTER_GO(TX, VEC) do { if (VEC && dense) TIB_ROUTER_D(TX, VEC, VEC); else TIB_ROUTER_D(TX, VEC, false); } while (0)
   if (x_dtype == TIB_F32) { if (vec) TIB_ROUTER_GO(float, true); else TIB_ROUTER_GO(float, false); }
   else if (x_dtype == TIB_BF16) { if (vec) TIB_ROUTER_GO(__nv_bfloat16, true); else TIB_ROUTER_GO(__nv_bfloat16, false); }
 #undef TIB_ROUTER_GO
+#undef TIB_ROUTER_D
   else
     return TIB_E_DTYPE;
   return TIB_OK;
