@@ -1992,7 +1992,7 @@ def test_choices_of_few_experts_are_the_general_forms(experts, top, sigmoid, nor
     assert torch.equal(results[0][1], results[1][1])
 
 
-@pytest.mark.parametrize("pairs, experts", [(1, 1), (1023, 32), (1025, 3), (8191, 256), (16384, 60), (16385, 60), (9000, 257)])
+@pytest.mark.parametrize("pairs, experts", [(1, 1), (1023, 32), (1025, 3), (8191, 256), (8192, 32), (8192, 31), (9001, 256), (16384, 60), (16385, 60), (9000, 257)])
 def test_pairs_are_sorted_by_expert(pairs, experts):
     need_gpu()
     from torchinferno_b200.kernels import ops

@@ -417,10 +417,16 @@ __device__ __forceinline__ void moe_group_pairs(const int* ids, int pairs, int e
 }
 
 // Up to kGroupPairs pairs a thread and kGroupExperts experts: every warp counts its own pairs, whose place among the warp's stays in a register, so
-// that ids are read once and no two warps meet in an atomic.  8,192 pairs over 32 experts behind the choices: 6.5 us, 7.8 with one set of counts and ids read twice.
+// that ids are read once and no two warps meet in an atomic, at the price of 32 counts an expert to add up.  A kernel of its own, since twice the registers
+// make a small call longer; us, one set of counts / a set a warp: 64 pairs over 32 experts 1.7 / 2.6, 4,096 over 32 4.1 / 4.6, 8,192 over 24, 32 and 64
+// 6.2 / 6.3, 6.5 / 6.5 (behind the choices 7.8 / 6.5) and 7.5 / 7.3, 16,384 over 16, 32 and 256 8.7 / 9.4, 11.4 / 10.8 and 15.3 / 13.9.
 constexpr int kGroupPairs = 16, kGroupExperts = 256;
-__device__ __forceinline__ void moe_group_warps(const int* ids, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ order,
-                                               int* __restrict__ place) {
+static bool group_by_warps(int pairs, int experts) { return pairs >= 8192 && pairs <= kGroupPairs * 1024 && experts >= 32 && experts <= kGroupExperts; }
+
+__global__ void __launch_bounds__(1024)
+moe_group_warps_kernel(const int* __restrict__ ids, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ place) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ int count[32][kGroupExperts];      // of a warp's pairs, then where the warp's begin
   __shared__ int total[kGroupExperts];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -481,8 +487,7 @@ moe_group_kernel(const int* __restrict__ ids, int pairs, int experts, int* __res
                  int* __restrict__ place) {
   pdl_wait();
   pdl_trigger();
-  if (pairs <= kGroupPairs * 1024 && experts <= kGroupExperts) moe_group_warps(ids, pairs, experts, offsets, order, place);
-  else moe_group_pairs(ids, pairs, experts, offsets, order, place);
+  moe_group_pairs(ids, pairs, experts, offsets, order, place);
 }
 
 // Both for a step of few tokens, in one launch: a warp per token makes its choices, then the block sorts the pairs.  (Eight tokens x 4
@@ -745,7 +750,8 @@ TIB_API int tib_moe_route(const float* logits, int64_t ld, int tokens, int exper
 TIB_API int tib_moe_group(const int* ids, int pairs, int experts, int* offsets, int* order, int* place, cudaStream_t stream) {
   if (!ids || !offsets || !order || !place) return TIB_E_ARG;
   if (experts < 1 || experts > 1024 || pairs < 0) return TIB_E_SIZE;
-  TIB_LAUNCH_DEPENDENT(moe_group_kernel, 1, 1024, 0, stream, ids, pairs, experts, offsets, order, place);
+  if (group_by_warps(pairs, experts)) TIB_LAUNCH_DEPENDENT(moe_group_warps_kernel, 1, 1024, 0, stream, ids, pairs, experts, offsets, order, place);
+  else TIB_LAUNCH_DEPENDENT(moe_group_kernel, 1, 1024, 0, stream, ids, pairs, experts, offsets, order, place);
   return TIB_OK;
 }
 
