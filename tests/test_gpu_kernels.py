@@ -1949,6 +1949,24 @@ def test_router_logits_of_six_rows_a_warp_have_the_bits_of_one(tokens, rows, k, 
     assert tokens * rows >= 20000 > 100 * rows and torch.equal(out, torch.cat(parts))
 
 
+@pytest.mark.parametrize("entries, dim", [(28, 128), (37, 100), (30, 32)])      # (448 to 592 blocks of heads of 65 to 128: the form with four blocks an SM)
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_attention_on_cuda_cores_of_many_single_tokens_has_the_bits_of_a_few(entries, dim, dtype):
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    heads, page, contexts = 16, 16, [1 + 37 * i % 90 for i in range(entries)]
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    pool = dev(rnd(6 * entries, 2, heads, page, dim, dtype=dtype))
+    table, q = ints(torch.randperm(6 * entries, generator=torch.Generator().manual_seed(2)).tolist()).view(entries, 6), dev(rnd(entries, heads * dim, dtype=dtype, seed=1))
+
+    def run(first, last):
+        n = last - first
+        return ops.paged_attention_simt(q[first:last], pool, torch.empty(n, heads * dim, dtype=dtype, device="cuda"), ints(range(n + 1)),
+                                        ints(c - 1 for c in contexts[first:last]), ints(range(first, last)), table, n, 1, heads, heads, dim, scale=dim ** -0.5)
+
+    assert torch.equal(run(0, entries), torch.cat([run(0, 15), run(15, entries)]))
+
+
 # (two and four blocks on the fullest SM and bf16 rows, more than one and fp32 rows: the form with fewer registers; the last the form of large steps)
 @pytest.mark.parametrize("tokens, rows, dtype", [(501, 16, torch.bfloat16), (1180, 16, torch.bfloat16), (2049, 9, torch.bfloat16), (603, 9, torch.bfloat16),
                                                  (1183, 16, torch.float32), (1301, 7, torch.float32), (1184, 9, torch.float32)])
