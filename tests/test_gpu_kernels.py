@@ -1649,18 +1649,29 @@ def test_append_with_one_table_of_angles_agrees_with_the_plain_kernel(tokens, he
         assert torch.equal(got, plain)      # (the same turns and sums in fp32, each rounded once to bfloat16)
 
 
-# (297 tokens are the fewest that go in pieces of 16 bytes; halves of eight elements, heads that are turned whole or not at all, more pieces than threads)
+# (297 tokens are the fewest that go in pieces of 16 bytes, 2,049 go two a block; halves of eight elements, heads that are turned whole or not at all, more
+# pieces than threads; three requests that begin on odd rows, so that a block holds tokens of two)
+@pytest.mark.parametrize("tokens", [297, 2049])
+@pytest.mark.parametrize("missing", [False, True])
 @pytest.mark.parametrize("heads, kv_heads, dim, vdim, rot, turned, bias", [
     (3, 1, 64, 64, 64, True, True), (5, 2, 32, 16, 16, True, False), (24, 8, 128, 128, 32, True, True), (2, 2, 48, 80, 0, False, True), (4, 4, 256, 256, 128, True, False)])
-def test_append_in_pieces_agrees_with_the_plain_kernel(heads, kv_heads, dim, vdim, rot, turned, bias):
+def test_append_in_pieces_agrees_with_the_plain_kernel(tokens, missing, heads, kv_heads, dim, vdim, rot, turned, bias):
+    """``missing``: the first page of the request that begins on a block's second token is out of range: it is reported, the first token is stored."""
     need_gpu()
     from torchinferno_b200.kernels import ops
-    tokens, page = 297, 8
-    total, pages = heads * dim + kv_heads * (dim + vdim), -(-tokens // page) + 1
+    page, lens, pasts = 8, [tokens // 3 | 1, tokens // 4 * 2, 0], [5, 800, 30]
+    lens[2] = tokens - lens[0] - lens[1]
+    total, per = heads * dim + kv_heads * (dim + vdim), -(-max(n + p for n, p in zip(lens, pasts)) // page)
+    pages = 3 * per
     rows, biases = rnd(tokens, total, dtype=torch.bfloat16), [dev(rnd(w, seed=i)) if bias else None for i, w in enumerate((heads * dim, kv_heads * dim, kv_heads * vdim))]
     freq = dev(1e4 ** (-torch.arange(rot // 2) / max(rot // 2, 1)))
     vfreq = dev(1e4 ** (-torch.arange(vdim // 2) / (vdim // 2))) if turned else None
-    table = dev(torch.randperm(pages, generator=torch.Generator().manual_seed(3)).int().view(1, pages))
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(3)).int().view(3, per)
+    if missing:
+        table[1, pasts[1] // page] = pages
+    positions = torch.cat([p + torch.arange(n) for n, p in zip(lens, pasts)]).int()
+    token_slot = torch.cat([torch.full((n,), i) for i, n in enumerate(lens)]).int()
+    assert lens[0] % 2 == 1 and pasts[1] % page == 0
     results = []
     for shift in (8, 1):      # (columns off their boundaries take the plain kernel)
         wide = torch.zeros(tokens, total + 8, dtype=torch.bfloat16)
@@ -1668,9 +1679,11 @@ def test_append_in_pieces_agrees_with_the_plain_kernel(heads, kv_heads, dim, vdi
         keys, values = page_views(pages, kv_heads, page, dim, vdim, torch.bfloat16)
         q = torch.empty(tokens, heads * dim, dtype=torch.bfloat16, device="cuda")
         turns = torch.empty(tokens, vdim // 2, 2, device="cuda") if turned else None
+        error = torch.zeros(1, dtype=torch.int32, device="cuda")
         ops.rotary_kv_append(dev(wide), shift, shift + heads * dim, shift + (heads + kv_heads) * dim, q, keys, values,
-                             dev(torch.arange(tokens, dtype=torch.int32)), torch.zeros(tokens, dtype=torch.int32, device="cuda"), table, freq, vfreq, heads,
-                             kv_heads, dim, vdim, rot_dim=rot, amplitude=1.25, q_bias=biases[0], k_bias=biases[1], v_bias=biases[2], turns=turns)
+                             dev(positions), dev(token_slot), dev(table), freq, vfreq, heads,
+                             kv_heads, dim, vdim, rot_dim=rot, amplitude=1.25, q_bias=biases[0], k_bias=biases[1], v_bias=biases[2], turns=turns, error_word=error)
+        assert (int(error) != 0) == missing
         results.append((q, keys, values) + ((turns,) if turned else ()))
     for got, plain in zip(*results):
         assert torch.equal(got, plain)      # (the same turns and sums in fp32, each rounded once to bfloat16)

@@ -187,17 +187,17 @@ __global__ void __launch_bounds__(1024) pwa_append_pairs_kernel(const __nv_bfloa
 
 // The same bits again for large steps whose heads come in whole pieces of 16 bytes: a thread owns 16 elements of a head (eight and their
 // eight partners, or 16 neighbours that are not turned) and asks for them before the token's angles are worked out and its page is
-// found, so that a token is two trips to memory long.  A block takes two tokens, whose biases and frequencies are fetched once: half as many rounds of
-// blocks, each as long as one trip.  2,048 tokens of 16 + 8 + 8 heads of 128: 10.1 us (one token a block 12.6; two elements a thread at a time 20 cold).
-constexpr int kPwaPair = 2;      // tokens of a block
+// found, so that a token is two trips to memory long.  With two tokens a block their biases and frequencies are fetched once and there are half as many
+// rounds of blocks, each a little longer.  2,048 tokens of 16 + 8 + 8 heads of 128: 10.1 us (one token a block 12.6; two elements a thread at a time 20 cold).
+template <int PAIR>      // tokens of a block
 __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloat16* __restrict__ proj, __nv_bfloat16* __restrict__ q_out, PwaAppendArgs a, int n_tokens) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float2 turn_s[kPwaPair][kPwaTurns], vturn_s[kPwaPair][kPwaTurns];      // (cosine, sine)
-  const int t0 = blockIdx.x * kPwaPair, own = min(kPwaPair, n_tokens - t0);
-  int pos[kPwaPair], slot[kPwaPair];
+  __shared__ float2 turn_s[PAIR][kPwaTurns], vturn_s[PAIR][kPwaTurns];      // (cosine, sine)
+  const int t0 = blockIdx.x * PAIR, own = PAIR == 1 ? 1 : min(PAIR, n_tokens - t0);
+  int pos[PAIR], slot[PAIR];
 #pragma unroll
-  for (int u = 0; u < kPwaPair; ++u) {
+  for (int u = 0; u < PAIR; ++u) {
     pos[u] = a.positions[t0 + min(u, own - 1)];
     slot[u] = a.cache.keys ? a.token_slot[t0 + min(u, own - 1)] : 0;
   }
@@ -225,12 +225,12 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
     }
     return u;
   };
-  struct Pieces { uint4 lo[kPwaPair], hi[kPwaPair]; float4 bias[4]; };
+  struct Pieces { uint4 lo[PAIR], hi[PAIR]; float4 bias[4]; };
   auto ask = [&](const Unit& u) {
     Pieces p;
 #pragma unroll
-    for (int w = 0; w < kPwaPair; ++w) {
-      const __nv_bfloat16* src = u.src + (w < own ? (size_t)w * a.ld : 0);
+    for (int w = 0; w < PAIR; ++w) {
+      const __nv_bfloat16* src = u.src + (w > 0 && w < own ? (size_t)w * a.ld : 0);
       p.lo[w] = *reinterpret_cast<const uint4*>(src + u.i);
       p.hi[w] = *reinterpret_cast<const uint4*>(src + u.k);
     }
@@ -243,9 +243,9 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
     }
     return p;
   };
-  int pages[kPwaPair], in_pages[kPwaPair];
+  int pages[PAIR], in_pages[PAIR];
 #pragma unroll
-  for (int u = 0; u < kPwaPair; ++u) pages[u] = -1, in_pages[u] = 0;
+  for (int u = 0; u < PAIR; ++u) pages[u] = -1, in_pages[u] = 0;
   auto put_one = [&](const Unit& u, const Pieces& p, int w) {
     const int page = pages[w], in_page = in_pages[w], t = t0 + w;
     __nv_bfloat16* dst;
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
   };
   auto put = [&](const Unit& u, const Pieces& p) {
 #pragma unroll
-    for (int w = 0; w < kPwaPair; ++w)
+    for (int w = 0; w < PAIR; ++w)
       if (w < own) put_one(u, p, w);
   };
   Unit mine;
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
   }
   if (a.cache.keys) {
 #pragma unroll
-    for (int u = 0; u < kPwaPair; ++u) {
+    for (int u = 0; u < PAIR; ++u) {
       if (u >= own) break;
       const int* table = a.cache.block_table + (size_t)slot[u] * a.cache.table_stride;
       pages[u] = pwa_page(a.cache, table, pos[u], a.error_word, 0x30000 + ((t0 + u) & 0xffff));
@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(256) pwa_append_pieces_kernel(const __nv_bfloa
     }
   }
   for (int i = threadIdx.x; i < (half + vhalf) * own; i += blockDim.x) {
-    const int w = i >= half + vhalf ? 1 : 0, j = i - w * (half + vhalf);
+    const int w = PAIR > 1 && i >= half + vhalf ? 1 : 0, j = i - w * (half + vhalf);
     const bool key = j < half;
-    const float angle = (float)(w ? pos[1] : pos[0]) * (key ? a.freq[j] : a.vfreq[j - half]);
+    const float angle = (float)(w ? pos[PAIR - 1] : pos[0]) * (key ? a.freq[j] : a.vfreq[j - half]);
     const float c = cosf(angle), sn = sinf(angle);
     if (key) turn_s[w][j] = make_float2(c * a.amplitude, sn * a.amplitude);
     else {
@@ -1289,8 +1289,15 @@ TIB_API int tib_rotary_kv_append(const void* proj, int64_t ld, int q_off, int k_
     if (n_tokens > 2 * 148 && dim % 16 == 0 && vdim % 16 == 0 && rot_dim % 16 == 0 && vhalf % 8 == 0 && ld % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 &&
         v_off % 8 == 0 && page_stride % 8 == 0 && (bits & 15) == 0) {
       const int pieces = ((heads + kv_heads) * dim + kv_heads * vdim) / 16;
-      TIB_LAUNCH_DEPENDENT(pwa_append_pieces_kernel, ceil_div(n_tokens, kPwaPair), pieces >= 256 ? 256 : pieces <= 128 ? 128 : (pieces + 31) / 32 * 32, 0, stream,
-                           (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a, n_tokens);
+      const int threads = pieces >= 256 ? 256 : pieces <= 128 ? 128 : (pieces + 31) / 32 * 32, a_round = 1024 / threads * 148;
+      // Two tokens a block from the second round of blocks on; where a block goes over its tokens' pieces twice, only where that halves the rounds, the
+      // last of them half full at least.  us, one token / two: 16 + 8 + 8 heads of 128, 592 tokens 3.3 / 3.5, 700 4.8 / 4.4, 1,184 5.6 / 4.7, 5,000
+      // 19.3 / 15.7; 24 + 6 + 6 of 128, 700 tokens 4.9 / 5.2, 1,184 5.9 / 5.5, 1,500 7.2 / 8.0, 2,048 9.1 / 8.6; 4 + 1 + 1 of 64, 1,184 2.7 / 3.1, 1,500 4.2 / 3.6.
+      const int rounds = ceil_div(n_tokens, a_round), paired = ceil_div(ceil_div(n_tokens, 2), a_round);
+      if (rounds > 4 || (pieces <= 256 ? rounds > 1 : rounds >= 2 * paired && 2 * (int64_t)n_tokens >= 3 * a_round))
+        TIB_LAUNCH_DEPENDENT(pwa_append_pieces_kernel<2>, ceil_div(n_tokens, 2), threads, 0, stream, (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a, n_tokens);
+      else
+        TIB_LAUNCH_DEPENDENT(pwa_append_pieces_kernel<1>, n_tokens, threads, 0, stream, (const __nv_bfloat16*)proj, (__nv_bfloat16*)q_out, a, n_tokens);
       return TIB_OK;
     }
     // few tokens: a thread for every two elements, so that a token is one round of loads and not five or six one after the other
