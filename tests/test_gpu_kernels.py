@@ -961,7 +961,7 @@ def test_aligned_fp32_product_has_the_plain_kernels_bits(m, n, k):
 
 
 # (edges of the tiles: 128 features, 16 to 80 rows, 64 k a step and 128 a sum)
-@pytest.mark.parametrize("m, n, k", [(1, 8192, 512), (16, 7297, 576), (17, 512, 8192), (80, 6560, 640), (81, 2000, 2112), (161, 4100, 1024), (330, 7400, 576)])
+@pytest.mark.parametrize("m, n, k", [(1, 8192, 512), (16, 7297, 576), (17, 512, 8192), (80, 6560, 640), (81, 2000, 2112), (161, 4100, 1024), (330, 7400, 576), (2600, 2050, 4160)])
 def test_fp32_product_in_three_terms(m, n, k, monkeypatch):
     need_gpu()
     from torchinferno_b200.kernels import ops

@@ -20,7 +20,7 @@
 // What bounds it: the warp that issues the MMAs, which waits once and issues 16 instructions a step of 64 k (0.95 us at 80 rows, of which 0.5 are
 // products), and for the last round of tiles the SMs that have none.  A wait for the rows, one for each half of the weights' terms and one
 // commit each made it 1.15 us; a lane issuing alone takes 45 cycles an instruction instead of 8.  301 rows, us, against gemm_f32.cu's fused
-// multiply-adds: 16,384 x 2,048 119 (536), 2,048 x 8,192 72 (431), 2,048 x 2,048 25 (111); 8 rows: 30 (68), 33 (146), 17 (39).
+// multiply-adds: 16,384 x 2,048 117 (536), 2,048 x 8,192 66 (431), 2,048 x 2,048 25 (111); 8 rows: 30 (68), 33 (146), 20 (39).
 // Error against 64 bits (2-norm): 1.4e-7 at 2,048 k and 1.5e-7 at 8,192, where multiply-adds in order have 8.1e-7 and 1.6e-6; numbers of one
 // sign 1.6e-7 (6.3e-7); sums over 256 k 2.4e-7, for a tenth off the time.
 // An output that is not finite is worked out again with fused multiply-adds in order (an infinity's terms make NaN of it).
@@ -72,33 +72,40 @@ struct FtArgs {
   int* error_word;
 };
 
-// A thread's sums of one feature into out (fetched and added to where `onto`); LAST: what is not finite is made again.
-template <bool LAST>
-__device__ __forceinline__ void ft_put(float (&sum)[kFtGroups][16], float* out, int64_t ld, bool onto, int m0, int feature, int half, const FtArgs& a) {
+// A thread's sums of one feature into out, fetched and added to where `onto`; where `last`, what is not finite is made again, in a second pass over what was
+// stored (a call with the sums still in registers would spill them).
+__device__ __forceinline__ void ft_put(float (&sum)[kFtGroups][16], float* out, int64_t ld, bool onto, bool last, int m0, int feature, int half, const FtArgs& a) {
   if (feature >= a.N) return;
+  bool finite = true;
 #pragma unroll
   for (int g = 0; g < kFtGroups; ++g) {
     const int j0 = (2 * g + half) * 16, left = min(a.rows - j0, a.M - m0 - j0);
     if (left <= 0) break;
     float* to = out + (size_t)(m0 + j0) * ld + feature;
     if (onto) {
+      float before[16];
 #pragma unroll
-      for (int c0 = 0; c0 < 16; c0 += 8) {
-        float before[8];
+      for (int c = 0; c < 16; ++c) before[c] = c < left ? to[c * ld] : 0.f;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) before[c] = c0 + c < left ? to[(c0 + c) * ld] : 0.f;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) sum[g][c0 + c] = before[c] + sum[g][c0 + c];
-      }
+      for (int c = 0; c < 16; ++c) sum[g][c] = before[c] + sum[g][c];
     }
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
       if (c >= left) break;
-      float v = sum[g][c];
-      if (LAST && !isfinite(v)) v = ft_plain_sum(a.x + (size_t)(m0 + j0 + c) * a.ldx, a.w + (size_t)feature * a.ldw, a.K);
-      to[c * ld] = v;
+      finite = finite && isfinite(sum[g][c]);
+      to[c * ld] = sum[g][c];
     }
   }
+  if (!last || finite) return;
+#pragma unroll 1
+  for (int g = 0; g < kFtGroups; ++g)
+#pragma unroll 1
+    for (int c = 0; c < 16; ++c) {
+      const int row = (2 * g + half) * 16 + c;
+      if (row >= a.rows || m0 + row >= a.M) break;
+      float* to = out + (size_t)(m0 + row) * ld + feature;
+      if (!isfinite(*to)) *to = ft_plain_sum(a.x + (size_t)(m0 + row) * a.ldx, a.w + (size_t)feature * a.ldw, a.K);
+    }
 }
 
 __global__ void __launch_bounds__(kFtThreads, 1)
@@ -346,13 +353,8 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       if (!ok) break;
       const int m0 = u.tile % m_tiles * a.rows, feature = u.tile / m_tiles * kFtM + quarter * 32 + lane;
       const bool last = u.part == a.parts - 1;
-      if (a.partial || !last) {      // (a part's sum: by itself, or on top of the parts' before it, whose sums are all asked for first)
-        float* dst = a.partial ? a.partial + (size_t)u.part * a.M * a.N : a.out;
-        const int64_t ld = a.partial ? a.N : a.ldo;
-        ft_put<false>(sum, dst, ld, !a.partial && u.part > 0, m0, feature, half, a);
-      } else {
-        ft_put<true>(sum, a.out, a.ldo, u.part > 0, m0, feature, half, a);
-      }
+      // (a part's sum: by itself, or on top of the parts' before it)
+      ft_put(sum, a.partial ? a.partial + (size_t)u.part * a.M * a.N : a.out, a.partial ? a.N : a.ldo, !a.partial && u.part > 0, !a.partial && last, m0, feature, half, a);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -387,13 +389,14 @@ __global__ void __launch_bounds__(256) add_parts_kernel(FtArgs a) {
 }
 
 // Into how many parts of k a product is summed, each by itself: by the weight's sizes alone, so that a row's bits do not depend on how many rows
-// there are.  A weight of few features leaves SMs without a tile (2,048 features, 301 rows: 64 to 112 tiles), and these parts are work for them:
-// 2,048 x 8,192 in four, us on 8 / 100 / 301 / 1,000 / 2,048 rows, 85 / 89 / 96 / 200 / 367 in one and 33 / 39 / 72 / 194 / 383; 2,048 x 2,048 in two
-// 26 / 28 / 31 / 58 / 94 and 17 / 20 / 25 / 59 / 98 (with many rows the parts only cost their ends); 3,072 x 2,048 27 / 28 / 32 / 83 / 150 and
-// 17 / 21 / 32 / 84 / 156.
+// there are.  A weight of few features leaves SMs without a tile (2,048 features, 301 rows: 64 to 112 tiles), and these parts are work for them, while with
+// many rows they cost their ends; us on 8 / 100 / 301 / 1,000 / 2,048 rows, weights in the L2: 2,048 x 8,192 in one 91 / 89 / 95 / 205 / 372, in four 34 / 38 /
+// 66 / 195 / 415; 2,048 x 4,096 50 / 50 / 52 / 104 / 184 and 17 / 24 / 40 / 102 / 195; 4,096 x 4,096 55 / 52 / 60 / 177 / 368, in two 30 / 38 / 61 / 178 / 366
+// (in four 22 / 39 / 68 / 190 / 400); 3,072 x 4,096 55 / 52 / 54 / 152 / 290 and 33 / 33 / 54 / 150 / 288; 2,048 x 2,048 32 / 32 / 32 / 59 / 94 and 20 / 22 /
+// 27 / 58 / 95; 3,072 x 2,048 32 / 31 / 33 / 84 / 152 and 21 / 26 / 34 / 83 / 150; 8,192 x 2,048 33 / 35 / 65 / 182 / 380 and 23 / 36 / 68 / 183 / 380.
 static int ft_parts(int N, int K) {
   const int f_tiles = ceil_div(N, kFtM), k_steps = K / kFtK;
-  return f_tiles <= 32 && k_steps >= 64 ? 4 : f_tiles <= 64 && k_steps >= 32 ? 2 : 1;
+  return f_tiles <= 16 && k_steps >= 64 ? 4 : f_tiles <= 64 && k_steps >= 32 ? 2 : 1;
 }
 
 // Rows of a tile, and whether the parts go to blocks of their own: whole rounds of work over the SMs times its steps' cost (0.65 us with 16
