@@ -1537,7 +1537,8 @@ def test_scan_in_chunks_of_an_infinite_state():
         assert (chunks[fine] - walk[fine]).abs().max() <= 32 * 2.0 ** -23 * walk[fine].abs().max()      # (the bound of the finite states' test)
 
 
-@pytest.mark.parametrize("lens, channels, taps", [([1, 2, 3], 8, 4), ([16, 17, 1], 1032, 3), ([50, 2], 520, 2), ([40], 16, 4)])
+# (the last: more segments of eight tokens than a grid is high or deep)
+@pytest.mark.parametrize("lens, channels, taps", [([1, 2, 3], 8, 4), ([16, 17, 1], 1032, 3), ([50, 2], 520, 2), ([40], 16, 4), ([7, 9], 512, 4), ([8, 524300], 8, 4)])
 def test_short_convolution_by_eight_channels_has_the_plain_kernels_bits(lens, channels, taps):
     need_gpu()
     from torchinferno_b200.kernels import ops

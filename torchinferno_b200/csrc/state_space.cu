@@ -120,8 +120,8 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(ConvArgs a) {
   pdl_trigger();
   constexpr int CARRIED = TAPS - 1, SEG = kConvVecSegment;
   static_assert(SEG >= kConvMaxTaps - 1, "a segment is at least as long as what it looks back");
-  const int entry = blockIdx.z, seg = blockIdx.y;
-  const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
+  const int runs = (a.channels + 511) / 512, seg = blockIdx.x / runs, entry = blockIdx.y;      // (segments of 512 channels each, in the grid's long dimension)
+  const int c = ((blockIdx.x - seg * runs) * 128 + threadIdx.x) * 4;
   const int row0 = a.q_start[entry], len = a.q_start[entry + 1] - row0;
   const int t0 = seg * SEG;
   if (c >= a.channels || t0 >= len) return;
@@ -516,17 +516,17 @@ TIB_API int tib_short_conv(const void* in, int in_dtype, int64_t ld, int col, co
   a.in = in; a.in_dtype = in_dtype; a.ld = ld; a.col = col; a.weight = weight; a.bias = bias; a.state = state;
   a.state_stride = state_stride; a.state_off = state_off; a.q_start = q_start; a.slots = slots; a.out = out;
   a.out_dtype = out_dtype; a.channels = channels; a.taps = taps; a.silu = silu;
-  const int vec_segments = ceil_div(max_q_len, kConvVecSegment);
+  const int segments = ceil_div(max_q_len, kConvSegment);
+  if (segments > 65535) return TIB_E_SIZE;
+  const int64_t vec_blocks = (int64_t)ceil_div(max_q_len, kConvVecSegment) * ceil_div(channels, 512);
   if (in_dtype == TIB_BF16 && out_dtype == TIB_BF16 && taps >= 2 && taps <= 4 && channels % 8 == 0 && ld % 8 == 0 && col % 8 == 0 &&
-      (((uintptr_t)in | (uintptr_t)out | (uintptr_t)weight | (uintptr_t)bias) & 15) == 0 && vec_segments <= 65535) {
-    const dim3 grid(ceil_div(channels, 512), vec_segments, n_entries);
+      (((uintptr_t)in | (uintptr_t)out | (uintptr_t)weight | (uintptr_t)bias) & 15) == 0 && vec_blocks <= 0x7fffffff) {
+    const dim3 grid((unsigned)vec_blocks, n_entries);
     if (taps == 4) TIB_LAUNCH_DEPENDENT(short_conv_vec_kernel<4>, grid, 128, 0, stream, a);
     else if (taps == 3) TIB_LAUNCH_DEPENDENT(short_conv_vec_kernel<3>, grid, 128, 0, stream, a);
     else TIB_LAUNCH_DEPENDENT(short_conv_vec_kernel<2>, grid, 128, 0, stream, a);
     return TIB_OK;
   }
-  const int segments = ceil_div(max_q_len, kConvSegment);
-  if (segments > 65535) return TIB_E_SIZE;
   TIB_LAUNCH_DEPENDENT(short_conv_kernel, dim3(ceil_div(channels, kConvChannels), segments, n_entries), kConvChannels, 0, stream, a);
   return TIB_OK;
 }
