@@ -1811,6 +1811,35 @@ def test_merged_latent_rows_in_bfloat16_are_the_fp32_rows_rounded_once(contexts,
     assert rows is merged
 
 
+# (runs of 32 keys: 50, 63, 24, 25, 9 and 8 of them: the merge has nine to 24 on their way at once; a context of one run beside them)
+@pytest.mark.parametrize("contexts, heads, rank, rot", [([1600, 33], 3, 64, 16), ([2010], 16, 512, 64), ([768, 1, 700], 2, 96, 0), ([800], 5, 40, 8), ([288, 90], 4, 64, 64), ([256, 17], 3, 512, 64)])
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("simt", [False, True])
+def test_latent_single_tokens_over_many_runs(contexts, heads, rank, rot, sink, simt):
+    """Against the formula in 64 bits."""
+    need_gpu()
+    from torchinferno_b200.kernels import ops
+    n, page, width, scale = len(contexts), 16, rank + rot, 0.11
+    per = -(-max(contexts) // page)
+    keys, table = rnd(n * per, 1, page, width, dtype=torch.bfloat16, scale=0.7), torch.randperm(n * per, generator=torch.Generator().manual_seed(4)).int().view(n, per)
+    folded, sinks = rnd(n, heads, width, scale=0.3, seed=1).bfloat16().float(), rnd(heads, seed=2) if sink else None      # (no rounding of the queries)
+    ints = lambda v: dev(torch.tensor(list(v), dtype=torch.int32))
+    assert ops.lib().tib_latent_attention_splits(n, heads, max(contexts)) == -(-max(contexts) // 32)
+    out = as_ref(ops.latent_attention(dev(folded), dev(keys), torch.empty(n, heads, rank, device="cuda"), ints(range(n + 1)), ints(c - 1 for c in contexts),
+                                      ints(range(n)), dev(table), n, 1, heads, rank, rot, scale, max_kv_len=max(contexts), force_simt=simt,
+                                      sink=None if sinks is None else dev(sinks)))
+    for i, c in enumerate(contexts):
+        rows = keys[table[i].long(), 0].reshape(-1, width)[:c].double()
+        scores = scale * folded[i].double() @ rows.T
+        beside = scores if sinks is None else torch.cat([scores, sinks.double()[:, None]], 1)
+        want = (beside.softmax(1)[:, :c]) @ rows[:, :rank]
+        # a score's error: its `width` products rounded as they are added; a weight's twice that, and two bf16 terms of it (2^-17) on tensor cores;
+        # the sums over c keys and up to 64 runs in fp32
+        wrong = width * 2.0 ** -24 * scale * (folded[i].double().abs() @ rows.abs().T).max()
+        bound = (2 * wrong + 2.0 ** -16 + (c + 64 + 8) * 2.0 ** -24) * rows[:, :rank].abs().max()
+        assert (out[i] - want).abs().max() <= bound
+
+
 # (rows wider than the queries' registers hold, in whole and odd steps; heads beyond a block's 16; contexts split and, with many entries, whole)
 @pytest.mark.parametrize("heads, rank, rot, entries", [(17, 512, 128, 3), (5, 512, 80, 150), (16, 384, 16, 2), (33, 64, 16, 160), (4, 192, 112, 1)])
 @pytest.mark.parametrize("sink", [False, True])

@@ -482,12 +482,14 @@ latent_attention_kernel(const float* __restrict__ folded, const T* __restrict__ 
 }
 
 // grid (heads, tokens): out = sum_s w_s acc_s / sum_s w_s l_s with w_s = exp(m_s - max m); a run without keys has m = -inf and sums
-// of zero.  One warp makes the weights (summed in the order of the runs), while every thread's first kMergeAhead runs of its column are on their way,
-// then adds them in their order.  (Asked for behind the weights, eight at a time, 18 runs were three more trips to memory: 4.7 us
-// behind the attention, 4.1 now.  One thread making the weights, a cast of the rows behind this kernel and 128 threads in the append made the layer
-// 86 us on eight tokens of 16 heads over 3,000 cached ones; 71 now.)
+// of zero.  One warp makes the weights (summed in the order of the runs), then every thread adds its column in their order, with eight runs' loads in
+// flight.  AHEAD: the first kMergeAhead of them are on their way under the weights.  (18 runs, three more trips to memory behind the weights, took 4.7 us behind
+// the attention, 4.1 so; 47 runs on a token of 24 heads over a rank of 256 11.7 with the attention and 10.7.  With few runs, or with many of many rows, its
+// code, which a block runs once from end to end, costs more than it saves: two runs on 64 tokens of 16 heads 15.7 and 16.5, 64 runs on two tokens 15.5 and 16.0.)
+// (One thread making the weights, a cast of the rows behind this kernel and 128 threads in the append made the layer 86 us on eight tokens of 16 heads over
+// 3,000 cached ones, 71 without; 53 with the layer's other kernels as they are now.)
 constexpr int kMergeAhead = 24;
-template <typename TO>
+template <typename TO, bool AHEAD>
 __global__ void __launch_bounds__(512)
 latent_merge_kernel(const float* __restrict__ partial, TO* __restrict__ out, const float* __restrict__ sink, int heads, int n_splits, int rank) {
   pdl_wait();
@@ -498,7 +500,7 @@ latent_merge_kernel(const float* __restrict__ partial, TO* __restrict__ out, con
   const float* p = partial + row * n_splits * (2 + rank);
   float first[kMergeAhead];      // (of column threadIdx.x)
 #pragma unroll
-  for (int s = 0; s < kMergeAhead; ++s) first[s] = s < n_splits && (int)threadIdx.x < rank ? p[(size_t)s * (2 + rank) + 2 + threadIdx.x] : 0.f;
+  for (int s = 0; s < kMergeAhead && AHEAD; ++s) first[s] = s < n_splits && (int)threadIdx.x < rank ? p[(size_t)s * (2 + rank) + 2 + threadIdx.x] : 0.f;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     float m[2], l[2], mx = -CUDART_INF_F;
@@ -522,9 +524,9 @@ latent_merge_kernel(const float* __restrict__ partial, TO* __restrict__ out, con
     if (lane == 0) inv_total = latent_inverse(mx, total, sink, blockIdx.x);
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < rank; c += blockDim.x) {
+  for (int c = threadIdx.x; c < rank; c += blockDim.x) {      // (once: a rank is at most the block's 512 threads)
     float acc = 0.f;
-    const bool held = c == (int)threadIdx.x;
+    const bool held = AHEAD && c == (int)threadIdx.x;
     if (held) {
 #pragma unroll
       for (int s = 0; s < kMergeAhead; ++s)
@@ -1000,10 +1002,14 @@ latent_decode_kernel(const float* __restrict__ folded, const __nv_bfloat16* __re
 static int launch_latent_merge(float* out, const LatentAttnArgs& a, int n_entries, cudaStream_t stream) {
   const dim3 grid(a.heads, n_entries);
   const int threads = a.rank >= 512 ? 512 : (a.rank + 31) / 32 * 32;
-  if (a.merged)
-    TIB_LAUNCH_DEPENDENT(latent_merge_kernel<__nv_bfloat16>, grid, threads, 0, stream, (const float*)a.partial, a.merged, a.sink, a.heads, a.n_splits, a.rank);
-  else
-    TIB_LAUNCH_DEPENDENT(latent_merge_kernel<float>, grid, threads, 0, stream, (const float*)a.partial, out, a.sink, a.heads, a.n_splits, a.rank);
+  const bool ahead = a.n_splits > 8 && (a.n_splits <= 50 || (int64_t)a.heads * n_entries * a.rank <= 8192);
+#define TIB_MERGE(TO, AHEAD, to) \
+  TIB_LAUNCH_DEPENDENT((latent_merge_kernel<TO, AHEAD>), grid, threads, 0, stream, (const float*)a.partial, to, a.sink, a.heads, a.n_splits, a.rank)
+  if (a.merged && ahead) TIB_MERGE(__nv_bfloat16, true, a.merged);
+  else if (a.merged) TIB_MERGE(__nv_bfloat16, false, a.merged);
+  else if (ahead) TIB_MERGE(float, true, out);
+  else TIB_MERGE(float, false, out);
+#undef TIB_MERGE
   return TIB_OK;
 }
 
