@@ -443,14 +443,12 @@ using namespace tib;
 // numbers do not depend on what else is in the step.  On the device terms are faster from a million weights on, whatever the rows (1,024 x 1,024,
 // us on 8 / 40 / 300 rows: 19 / 19 / 43 by multiply-adds and 16 / 17 / 19 here; 2,048 x 2,048 37 / 50 / 110 and 26 / 27 / 31).  But a product issued
 // call by call costs the host some 8 us more (two launches and the scratch), and a block of such weights on few tokens waits for the host.
-// Blocks call by call, us on 8 / 40 / 100 / 300 tokens, by multiply-adds alone, with the line at 2^22 weights and at 2^20:
-//     1,024 wide, 1,024 inside   133 / 135 / 165 / 284   132 / 135 / 165 / 283   161 / 162 / 162 / 162
-//     1,024 wide, 2,112 inside   135 / 149 / 206 / 361   142 / 144 / 189 / 302   162 / 163 / 162 / 161
-//     1,536 wide, 3,200 inside   191 / 237 / 340 / 599   156 / 158 / 195 / 275   161 / 162 / 168 / 231
-//     1,536 wide, 6,400 inside   253 / 312 / 486 / 856   180 / 188 / 242 / 328   167 / 175 / 214 / 284
-// (measured when no product was summed in parts and the host took some 30 us more a block).
-// So no line is best for all: 2^22 costs few tokens 5 % (the second block's 4.3 million of gate and up), where 2^20 would cost them 20 % and gain
-// prompts of a hundred tokens and more 15 to 45 %.
+// Blocks call by call (8 / 4 heads of 128), us on 8 / 40 / 100 / 300 tokens, by multiply-adds alone, with the line at 2^22 weights and at 2^20:
+//     1,024 wide, 1,024 inside   119 / 123 / 155 / 277   118 / 123 / 155 / 277   143 / 144 / 145 / 145
+//     1,024 wide, 2,112 inside   127 / 146 / 196 / 354   127 / 132 / 169 / 285   149 / 149 / 150 / 150
+//     1,536 wide, 3,200 inside   173 / 214 / 299 / 528   137 / 139 / 173 / 281   149 / 150 / 150 / 191
+//     1,536 wide, 6,400 inside   242 / 292 / 448 / 798   138 / 147 / 197 / 331   150 / 151 / 153 / 238
+// So no line is best for all: 2^20 would cost few tokens 10 to 20 % and gain prompts of a hundred tokens and more 6 to 48 %.
 // (Weights whose rows overlap or are one and the same are none of a tensor map's.)
 TIB_API int tib_gemm_f32_tcgen05_takes(const void* x, const void* w, int N, int K, int64_t ldx, int64_t ldw) {
   return N >= 512 && K >= 512 && (int64_t)N * K >= (1 << 22) && K % kFtK == 0 && ldx % 4 == 0 && ldw % 4 == 0 && ldw >= K &&

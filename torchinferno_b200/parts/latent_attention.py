@@ -241,7 +241,8 @@ class _Plan:
 
 
 # What the folded form's launches, and those of both forms in one step, take the host that issues a prompt's layer call by call beyond
-# the unfolded form's, in us (130 a layer unfolded, 145 folded, some 240 with both).
+# the unfolded form's, in us (100 a layer unfolded, 117 folded, 206 with both; the differences were the same when a call took the interpreter longer:
+# 126, 144 and 245).
 FOLDED_HOST_US, BOTH_FORMS_US = 15.0, 110.0
 
 
