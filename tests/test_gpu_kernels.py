@@ -180,17 +180,23 @@ def test_gemm_tcgen05_swapab(m, n, k, splits, w_kn):
 
 @pytest.mark.parametrize("epilogue", ["none", "swiglu"])
 def test_the_choice_of_a_shape_with_one_weight_is_measured_from_memory(epilogue, monkeypatch):
-    """32 products in a row never read one weight twice (a hybrid model's only layer of a shape finds its weight in memory, not in the L2)."""
+    """32 captured products in a row never read one weight twice (a hybrid model's only layer of a shape finds its weight in memory, not in the L2)."""
     need_gpu()
     from torchinferno_b200.kernels import gemm, ops
     read, product = [], ops.library_gemm
     monkeypatch.setattr(gemm, "_stored_choices", dict)
     monkeypatch.setattr(gemm, "_store_choice", lambda name, choice: None)
-    monkeypatch.setattr(ops, "library_gemm", lambda x, w, *args, **options: (read.append(w.data_ptr()), product(x, w, *args, **options))[1])
+
+    def library_gemm(x, w, *args, **options):
+        if torch.cuda.is_current_stream_capturing():
+            read.append(w.data_ptr())
+        return product(x, w, *args, **options)
+
+    monkeypatch.setattr(ops, "library_gemm", library_gemm)
     weight = gemm.LinearWeight(dev(rnd(1104, 1088, dtype=torch.bfloat16)), few_rows_tcgen05=None, epilogue=epilogue)
     gemm.tune_few_rows()
     gemm._tuned.pop((1104, 1088, weight.tensor.device, epilogue))
-    assert len(read) >= 64 and all(len(set(read[i:i + 32])) == 32 for i in range(len(read) - 31))
+    assert len(read) >= 32 and all(len(set(read[i:i + 32])) == 32 for i in range(len(read) - 31))
 
 
 @pytest.mark.parametrize("choice", ["measured", "swapab", "library"])
