@@ -100,8 +100,9 @@ router_logits_kernel(const TX* __restrict__ x, int64_t ldx, const float* __restr
 // The same sums for large steps with 16-byte aligned rows: a warp works six rows of w on eight tokens, two tokens an instruction (packed fp32), so a
 // piece of w serves eight tokens and an element is widened for six rows; what it loads and widens is a third of its instructions.  (A lane's sums
 // run over k in the kernel above's order, and the sum over lanes is its butterfly, whose two halves of a pair add the same two numbers.)  What bounds
-// it: the loads of a step wait for one another's registers (two blocks of six warps an SM), then the fp32 pipe.  2,048 tokens of 2,048: 33 rows 14.4
-// us, 61 (of 1,536) 20.5, 129 41.0; with five rows of whole warps of eight and scalar products 20.2, 30.2, 72.6; rows and tokens through shared memory 27 to 50.
+// it: the loads of a step wait for one another's registers (two blocks of six warps an SM), then the fp32 pipe.  2,048 tokens of 2,048, one call after another,
+// everything in the L2: 17 rows 8.6 us, 33 12.4; 1,300 tokens, 129 rows 27, 513 88 (33 rows in a running layer, behind the kernel that wrote the tokens, 20);
+// five rows of whole warps of eight and scalar products 13.6, 19.8, 72 and 246 (24 in the layer); rows and tokens through shared memory 27 to 50 in the layer.
 constexpr int kRouterRows = 6, kRouterMany = 8, kRouterWarps = 6;
 
 __device__ __forceinline__ void load8_pairs(const float* a, const float* b, f32x2 (&v)[8]) {
