@@ -72,6 +72,22 @@ def test_a_measured_walk_reads_every_weight_from_memory(members, size, products,
     assert (distinct == products or distinct * size >= 1024) and (distinct - members) * size < 1024
 
 
+def test_a_walk_without_room_for_copies_reads_what_there_is(monkeypatch):
+    from torchinferno_b200.kernels import gemm
+    clone, made = torch.Tensor.clone, []
+
+    def limited(self):
+        if len(made) == 3:
+            raise torch.OutOfMemoryError("no room")
+        made.append(self)
+        return clone(self)
+
+    own = [torch.zeros(8, 8, dtype=torch.bfloat16) for _ in range(2)]
+    monkeypatch.setattr(torch.Tensor, "clone", limited)
+    walk = gemm._walk_weights(own)
+    assert len(walk) == gemm.TUNE_PRODUCTS and len({w.data_ptr() for w in walk}) == 5 and walk[0] is own[0] and walk[5] is own[0]
+
+
 def test_a_stored_choice_names_how_it_was_measured(monkeypatch):
     from torchinferno_b200.kernels import gemm
     monkeypatch.setattr(torch.cuda, "get_device_name", lambda device: "a GPU")

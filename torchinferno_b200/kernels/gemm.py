@@ -344,6 +344,8 @@ def tune_few_rows() -> dict[tuple, tuple[int, int, int]]:
                     if name in stored and len(stored[name]) == 3:
                         _tuned[key] = tuple(stored[name])
                     else:
+                        if device not in _flush:      # (before the copies, which do without where there is no room)
+                            _flush[device] = torch.empty(TUNE_COLD, dtype=torch.uint8, device=device)
                         members = _walk_weights([w.tensor for w in group[:TUNE_MEMBERS]])
                         timed = {c: _walk_time(members, 8, c, epilogue) for c in configs}
                         best = min(timed, key=timed.get)
@@ -377,7 +379,10 @@ def _walk_weights(members: list[torch.Tensor]) -> list[torch.Tensor]:
     products = max(len(members), min(TUNE_PRODUCTS, -(-TUNE_BYTES // size)))
     distinct = list(members)
     while len(distinct) < products and len(distinct) * size < TUNE_COLD:
-        distinct.append(members[len(distinct) % len(members)].clone())
+        try:
+            distinct.append(members[len(distinct) % len(members)].clone())
+        except torch.OutOfMemoryError:      # (a model that leaves no room is measured over fewer)
+            break
     return (distinct * -(-products // len(distinct)))[:products]
 
 
@@ -396,9 +401,7 @@ def _walk_time(weights: list[torch.Tensor], rows: int, config: tuple[int, int] |
         norm_weight = torch.ones(width, dtype=torch.float32, device=device)
         out = torch.empty((rows, n), dtype=torch.bfloat16, device=device)
         act = torch.empty((rows, n // 2), dtype=torch.bfloat16, device=device)
-        flush = _flush.get(device)
-        if flush is None:
-            flush = _flush[device] = torch.empty(TUNE_COLD, dtype=torch.uint8, device=device)
+        flush = _flush[device]
 
         def product(w: torch.Tensor) -> None:
             if config is None:
