@@ -243,7 +243,7 @@ def test_few_rows_kernel_is_chosen_by_measurement_and_either_choice_is_right():
     later = LinearWeight(dev(ws[0]), few_rows_tcgen05=None)
     assert gemm.tune_few_rows()[key] == decisions[key] and later.few_rows == open_weights[0].few_rows
     gemm._tuned.pop(key)                                                   # a new process reads what this one stored
-    again = [LinearWeight(dev(w), few_rows_tcgen05=None) for w in ws]      # (as many weights of the shape as were measured)
+    again = [LinearWeight(dev(w), few_rows_tcgen05=None) for w in ws]
     assert gemm.tune_few_rows()[key] == decisions[key] and again[0].splits == splits
     forced = [LinearWeight(dev(ws[0]), few_rows_tcgen05=True), LinearWeight(dev(ws[0]), few_rows_tcgen05=False)]
     assert [w.few_rows for w in forced] == [LinearWeight.FEW_ROWS, 0] and LinearWeight.FEW_ROWS == 64
